@@ -9,11 +9,13 @@ rebuilt only when a source or header is newer than it.
 
 from __future__ import annotations
 
+import concurrent.futures
 import os
 import pathlib
 import shutil
 import subprocess
 import sys
+import tempfile
 
 PACKAGE_DIR = pathlib.Path(__file__).resolve().parent
 CSRC = PACKAGE_DIR / "csrc"
@@ -24,7 +26,7 @@ LIB_PATH = PACKAGE_DIR / LIB_NAME
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
     "-O3", "-std=c++17", "-lineinfo",
-    "-shared", "-Xcompiler", "-fPIC",
+    "-Xcompiler", "-fPIC",
     "-Xcompiler", "-Wall",
 ]
 
@@ -49,19 +51,27 @@ def _stale() -> bool:
 
 
 def build(force: bool = False, verbose: bool = False) -> pathlib.Path:
+    """Compile the sources side by side (one nvcc per file) and link them."""
+
     if not force and not _stale():
         return LIB_PATH
-    cmd = [_nvcc(), *NVCC_FLAGS, "-I", str(INCLUDE)]
-    if verbose:
-        cmd += ["-Xptxas", "-v"]
-    cmd += [str(src) for src in sources()]
-    tmp = LIB_PATH.with_suffix(".so.tmp")
-    cmd += ["-o", str(tmp), "-lcudart", "-lcuda"]
-    proc = subprocess.run(cmd, capture_output=True, text=True)
-    if verbose or proc.returncode != 0:
-        sys.stderr.write(proc.stdout + proc.stderr)
-    if proc.returncode != 0:
-        raise RuntimeError(f"nvcc failed with exit code {proc.returncode}")
+    nvcc = _nvcc()
+    common = [*NVCC_FLAGS, "-I", str(INCLUDE)] + (["-Xptxas", "-v"] if verbose else [])
+
+    def run(cmd: list[str]) -> None:
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if verbose or proc.returncode != 0:
+            sys.stderr.write(proc.stdout + proc.stderr)
+        if proc.returncode != 0:
+            raise RuntimeError(f"nvcc failed with exit code {proc.returncode}")
+
+    with tempfile.TemporaryDirectory() as work:
+        objects = [str(pathlib.Path(work) / (src.stem + ".o")) for src in sources()]
+        jobs = [[nvcc, *common, "-c", str(src), "-o", obj] for src, obj in zip(sources(), objects)]
+        with concurrent.futures.ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            list(pool.map(run, jobs))
+        tmp = LIB_PATH.with_suffix(".so.tmp")
+        run([nvcc, *common, "-shared", *objects, "-o", str(tmp), "-lcudart", "-lcuda"])
     os.replace(tmp, LIB_PATH)
     return LIB_PATH
 

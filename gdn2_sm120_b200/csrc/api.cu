@@ -1,6 +1,7 @@
 // extern "C" entry points of libgdn2_b200.so: argument validation + kernel launches.
 // No allocation, no synchronisation, no exceptions cross this boundary.
 
+#include <atomic>
 #include <cstdio>
 #include <cstring>
 #include <initializer_list>
@@ -116,6 +117,23 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
     entry->devices |= bit;
   }
   return cudaSuccess;
+}
+
+// The attribute never changes: one query per device, then a table (a query costs about a microsecond).
+int multiprocessors(int* count) {
+  static std::atomic<int> known[64];
+  int device = 0;
+  cudaError_t err = cudaGetDevice(&device);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  std::atomic<int>& slot = known[device & 63];
+  int n = device < 64 ? slot.load(std::memory_order_relaxed) : 0;
+  if (n == 0) {
+    err = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device);
+    if (err != cudaSuccess || n <= 0) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+    if (device < 64) slot.store(n, std::memory_order_relaxed);
+  }
+  *count = n;
+  return GDN2_OK;
 }
 
 int check_launch() {

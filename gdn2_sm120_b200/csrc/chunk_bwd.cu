@@ -39,8 +39,16 @@ constexpr int64_t kStateElems = int64_t(kDim) * kDim;
 // =============================================================================================
 // reverse scan
 // =============================================================================================
-constexpr int kBScanThreads = 512;
-constexpr int kRsDot = 2064;   // dO^T tile: padded row-group stride (16-byte chunk stores, 4 tokens each)
+// Warp-specialised like the forward scan (chunk_fwd.cu), for the same reason: the MMAs of a chunk are issued
+// back to back by one warp, the rest runs beside them.
+//   warp 0       tiled TMA loads, each buffer refilled as soon as its MMA has read it
+//   warp 1       MMAs, per chunk:  dR^T += dS^T Kt^T | dS'^T += dO^T Qg | dS'^T -= dR^T Y | dZ^T = dR^T T |
+//                dR'^T = dO'^T Aqk of the next chunk, the dependences between accumulators waited for
+//   warps 2..9   decay: dS' <- dS diag(d) into the other of two buffers; the cotangent checkpoints, staged
+//   warps 10..17 dO of the next chunk (the one before it in time) into tensor memory, dZ out (staged)
+// Tensor memory (columns): dS 2 x 128, dR 2 x 64, dZ 64, dO 64 = all 512.
+constexpr int kBScanThreads = 576;
+constexpr int kBScanDecay0 = 2, kBScanDo0 = 10;  // first warps of the groups
 constexpr int kCsZ = 144, kRsZ = 32 * kCsZ;  // dZ tile: the padded strides of the VJP kernel's [dZ ; dO] stack
 
 struct BScanSmem {
@@ -50,263 +58,349 @@ struct BScanSmem {
   alignas(1024) uint8_t yt[32768];   // Yt[k][j]: 2 slabs of 128 lines
   alignas(1024) uint8_t at[16384];   // At[j][i]: 2 slabs of 64 lines
   alignas(1024) uint8_t tt[16384];   // Tt[j][i]: 2 slabs of 64 lines
-  alignas(128) uint8_t dot[16 * kRsDot];  // dO^T tile X[r = v][c = i], tf32, blocked (built from dO)
+  alignas(128) uint8_t d_out[16384]; // raw dO of the chunk, [64][128] 16-bit rows
   alignas(128) uint8_t dz[kBlobDZ];  // dZ staging, natural tile X[r = j][c = v] with the padded strides
-  alignas(16) float d[kDim];
-  alignas(8) uint64_t bar_ak, bar_qy, bar_mma1, bar_mma2;
+  alignas(128) float ck[2][32 * kDim];  // 32 rows of the cotangent per half of the decay group
+  alignas(16) float d[2][kDim];
+  alignas(8) uint64_t full_o, full_d[2];
+  uint64_t go_a;      // At, dO written:               1 load + 8 warps
+  uint64_t full_k, full_y;
+  uint64_t go_q;      // Q, decayed cotangent:         1 load + 8 warps
+  uint64_t go_z;      // Tt, dZ of the last step read: 1 load + 8 warps
+  uint64_t do_read;   // dO is in registers:                                 8 warps
+  uint64_t a_done, k_done, z_done, do_done, s_done;  // MMA commits
+  volatile int failed;
   uint32_t tmem_base;
 };
+static_assert(sizeof(BScanSmem) <= 232448, "reverse scan exceeds the 227 KiB shared-memory limit");
 
 struct BScanParams {
-  const uint8_t* ws;        // workspace of the training forward (D; the tiles come through tensor maps)
-  uint8_t* sc;              // scratch: receives dZ
-  const void* d_out;        // [B,T,H,128]
-  const float* ds_final;    // [B,H,128,128] or null
-  float* d_bnd;             // [B, n_chunks+1, H,128,128]
-  float* ds_init;           // [B,H,128,128] or null
+  const uint8_t* d;         // chunk-end decays, 512 bytes per unit
+  uint8_t* dz;              // dZ tiles
+  const float* ds_final;    // [sequences,H,128,128] or null
+  float* d_bnd;             // cotangents at the chunk starts, one slot more than chunks per sequence
+  float* ds_init;           // [sequences,H,128,128] or null
   int* status;
-  int64_t T, H, n_chunks, n_ch;
+  int H;
+};
+struct BScanMaps {
+  CUtensorMap at, tt, kn, q, yt, d_out;
 };
 
-template <typename T>
+template <typename T, typename Seqs>
 __global__ void __launch_bounds__(kBScanThreads, 1)
-chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ CUtensorMap tm_at,
-                      const __grid_constant__ CUtensorMap tm_tt, const __grid_constant__ CUtensorMap tm_kn,
-                      const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_yt) {
+chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   BScanSmem& sm = *reinterpret_cast<BScanSmem*>(smem_raw);
-  const WsLayout ws{p.n_ch, true};
-  const ScratchLayout sc{p.n_ch};
-  BoundedWaiter waiter(p.status);
-  // a wait that ran out earlier (forward or backward) left garbage behind: results become NaN
-  const bool upstream_failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
+  BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
-  // 16 warps.  TMEM phases: warp & 3 = lane quadrant, warp >> 2 = quarter of the columns.
-  // dO^T tile builder: warp = 4-token group tg, lane = 4-channel group.
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int q4 = warp & 3, part = warp >> 2;
-  const int tg = warp;
-  const int64_t bh = blockIdx.x;
-  const int64_t b = bh / p.H, h = bh % p.H;
-  constexpr uint32_t kColS = 0, kColR = 128, kColZ = 192;
+  const int s = int(blockIdx.x) / p.H, h = int(blockIdx.x) - s * p.H;
+  const SeqInfo sq = seqs.at(s);
+  const int n_chunks = sq.n_chunks;
+  constexpr uint32_t kColS = 0, kColR = 256, kColZ = 384, kColDo = 448;
+  // step `it` of the reverse scan works on chunk n_chunks - 1 - it
+  auto chunk_of = [&](int it) { return n_chunks - 1 - it; };
+  auto ch_of = [&](int it) { return int64_t(sq.chunk0 + chunk_of(it)) * p.H + h; };
 
-  if (warp == 0) {
-    tmem_alloc(&sm.tmem_base, 256);
+  if (warp == 1) {
+    tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(&sm.bar_ak, 1);
-    mbar_init(&sm.bar_qy, 1);
-    mbar_init(&sm.bar_mma1, 1);
-    mbar_init(&sm.bar_mma2, 1);
+    uint64_t* one[] = {&sm.full_o, &sm.full_d[0], &sm.full_d[1], &sm.full_k, &sm.full_y, &sm.a_done, &sm.k_done,
+                       &sm.z_done, &sm.do_done, &sm.s_done};
+#pragma unroll
+    for (int i = 0; i < 10; ++i) mbar_init(one[i], 1);
+    mbar_init(&sm.go_a, 1 + 8);
+    mbar_init(&sm.go_q, 1 + 8);
+    mbar_init(&sm.go_z, 1 + 8);
+    mbar_init(&sm.do_read, 8);
+    // a wait that ran out earlier (forward or backward) left garbage behind: results become NaN
+    sm.failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
     fence_mbar_init();
   }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tb = sm.tmem_base;
-  const uint32_t lane_base = 32u * q4;
-  const int vrow = 32 * q4 + lane;
-  const int k0 = 32 * part, j0 = 16 * part;
-
-  auto ch_of = [&](int64_t c) { return (b * p.n_chunks + c) * p.H + h; };
-  auto load_ak = [&](int64_t c) {
-    const int ch = int(ch_of(c));
-    mbar_arrive_expect_tx(&sm.bar_ak, uint32_t(kTileAt + kTileKn + kTileTt - 2 * 4096));
-    // At and Tt are zero for j >= 32, i < 32: three 32-row boxes each, the fourth quadrant stays zero
-    tma_load_3d(sm.at, &tm_at, 0, 0, ch, &sm.bar_ak);
-    tma_load_3d(sm.at + 8192, &tm_at, 32, 0, ch, &sm.bar_ak);
-    tma_load_3d(sm.at + 8192 + 4096, &tm_at, 32, 32, ch, &sm.bar_ak);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) tma_load_3d(sm.kn + s * 8192, &tm_kn, 32 * s, 0, ch, &sm.bar_ak);
-    tma_load_3d(sm.tt, &tm_tt, 0, 0, ch, &sm.bar_ak);
-    tma_load_3d(sm.tt + 8192, &tm_tt, 32, 0, ch, &sm.bar_ak);
-    tma_load_3d(sm.tt + 8192 + 4096, &tm_tt, 32, 32, ch, &sm.bar_ak);
-  };
-  auto load_qy = [&](int64_t c) {
-    const int64_t ch = ch_of(c);
-    mbar_arrive_expect_tx(&sm.bar_qy, uint32_t(kTileQ + kTileYt + kBlobD));
-#pragma unroll
-    for (int s = 0; s < 4; ++s) tma_load_3d(sm.q + s * 8192, &tm_q, 32 * s, 0, int(ch), &sm.bar_qy);
-#pragma unroll
-    for (int s = 0; s < 2; ++s) tma_load_3d(sm.yt + s * 16384, &tm_yt, 32 * s, 0, int(ch), &sm.bar_qy);
-    bulk_g2s(sm.d, p.ws + ws.off_d() + ch * kBlobD, uint32_t(kBlobD), &sm.bar_qy);
-  };
-  // dO of one chunk: 4 tokens x 4 channels per thread, still packed
-  auto load_do = [&](int64_t c, typename Raw4<T>::type (&raw)[4]) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      // past the end of a ragged sequence there is no cotangent: read the chunk's first token instead
-      // (always there) and drop the value, so that no branch separates the loads
-      const int64_t t = c * kChunk + 4 * tg + e;
-      const typename Raw4<T>::type x =
-          load4_raw<T>(p.d_out, ((b * p.T + (t < p.T ? t : c * kChunk)) * p.H + h) * kDim + 4 * lane);
-      raw[e] = (t < p.T) ? x : typename Raw4<T>::type{};
-    }
-  };
-
   // lines 32..63 of the first slab of At and Tt (j >= 32, i < 32) are never loaded: zero, once
   for (int e = tid; e < 4096 / 16; e += kBScanThreads) {
     reinterpret_cast<float4*>(sm.at + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     reinterpret_cast<float4*>(sm.tt + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
   fence_async_smem();
-  typename Raw4<T>::type do_raw[4] = {};
-  if (p.n_chunks > 0) {
-    if (tid == 0) {
-      load_ak(p.n_chunks - 1);
-      load_qy(p.n_chunks - 1);
-    }
-    load_do(p.n_chunks - 1, do_raw);
-  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tb = sm.tmem_base;
 
-  // ---- dS^T <- dS_T^T (32 key rows of column v per thread); also becomes the last boundary slot ----
-  {
-    const float* src = (p.ds_final != nullptr) ? p.ds_final + bh * kStateElems + vrow : nullptr;
-    float* slot = p.d_bnd + ((b * (p.n_chunks + 1) + p.n_chunks) * p.H + h) * kStateElems + vrow;
-    uint32_t r[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
-#pragma unroll
-    for (int j = 0; j < 32; ++j) slot[(k0 + j) * kDim] = __uint_as_float(r[j]);
-    tmem_st32(tmem_addr(tb, lane_base, kColS + k0), r);
-    tmem_wait_st();
-  }
-
-  uint32_t it = 0;
-  for (int64_t c = p.n_chunks - 1; c >= 0; --c, ++it) {
-    const uint32_t par = it & 1u;
-    if (it > 0) {
-      // previous iteration's second MMA group read dO^T, Qt, Yt and dR^T
-      waiter.wait(&sm.bar_mma2, par ^ 1u);
-      tc_fence_after();
-      if (tid == 0) load_qy(c);
-    }
-    // ---- dO^T tile: one 16-byte chunk (4 tokens) per channel ------------------------------------------
-    {
-      float dv[4][4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) unpack4<T>(do_raw[e], dv[e]);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        *reinterpret_cast<float4*>(sm.dot + blk_off<4>(4 * lane + f, 4 * tg, kRsDot, 128)) =
-            make_float4(dv[0][f], dv[1][f], dv[2][f], dv[3][f]);
-      }
-    }
-    if (it > 0) {
-      // cotangent at the start of chunk c + 1 (= end of chunk c); off the MMA's critical path
-      float* slot = p.d_bnd + ((b * (p.n_chunks + 1) + c + 1) * p.H + h) * kStateElems + vrow;
-      uint32_t r[32];
-      tmem_ld32(tmem_addr(tb, lane_base, kColS + k0), r);
-      tmem_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) slot[(k0 + j) * kDim] = __uint_as_float(r[j]);
-    }
-    fence_async_smem();
-    waiter.wait(&sm.bar_ak, par);
-    if (tid == 0) bulk_wait_read_all();  // the previous dZ tile has left its staging buffer
+  auto arrive = [&](uint64_t* bar) {  // one arrival per warp, after its tensor-memory accesses
     tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- loads
+    const uint32_t leader = elect_leader();
+    auto load_o = [&](int it) {
+      mbar_arrive_expect_tx(&sm.full_o, 16384u, leader);
+      tma_load_3d(sm.d_out, &tm.d_out, 0, h, int(sq.row0) + chunk_of(it) * kChunk, &sm.full_o, leader);
+    };
+    // At and Tt are zero for j >= 32, i < 32: three 32-row boxes each, the fourth quadrant stays zero
+    auto load_tri = [&](uint8_t* dst, const CUtensorMap* map, int it, uint64_t* bar) {
+      const int ch = int(ch_of(it));
+      mbar_arrive_expect_tx(bar, uint32_t(kTileAt - 4096), leader);
+      tma_load_4d(dst, map, 0, 0, 0, ch, bar, leader);
+      tma_load_4d(dst + 8192, map, 0, 0, 1, ch, bar, leader);
+      tma_load_4d(dst + 8192 + 4096, map, 0, 32, 1, ch, bar, leader);
+    };
+    auto load_tile = [&](uint8_t* dst, const CUtensorMap* map, int it, uint64_t* bar) {
+      mbar_arrive_expect_tx(bar, 32768u, leader);
+      tma_load_4d(dst, map, 0, 0, 0, int(ch_of(it)), bar, leader);
+    };
+    auto load_d = [&](int it) {
+      mbar_arrive_expect_tx(&sm.full_d[it & 1], uint32_t(kBlobD), leader);
+      bulk_g2s(sm.d[it & 1], p.d + ch_of(it) * kBlobD, uint32_t(kBlobD), &sm.full_d[it & 1], leader);
+    };
+    load_o(0);
+    load_tri(sm.at, &tm.at, 0, &sm.go_a);
+    load_tile(sm.kn, &tm.kn, 0, &sm.full_k);
+    load_d(0);
+    load_tile(sm.q, &tm.q, 0, &sm.go_q);
+    load_tile(sm.yt, &tm.yt, 0, &sm.full_y);
+    load_tri(sm.tt, &tm.tt, 0, &sm.go_z);
+    if (n_chunks > 1) load_d(1);
+    for (int it = 1; it < n_chunks; ++it) {
+      const uint32_t par = uint32_t(it - 1) & 1u;
+      waiter.wait(&sm.do_read, par);
+      load_o(it);
+      waiter.wait(&sm.a_done, par);
+      load_tri(sm.at, &tm.at, it, &sm.go_a);
+      waiter.wait(&sm.k_done, par);
+      load_tile(sm.kn, &tm.kn, it, &sm.full_k);
+      waiter.wait(&sm.do_done, par);
+      load_tile(sm.q, &tm.q, it, &sm.go_q);
+      waiter.wait(&sm.s_done, par);
+      load_tile(sm.yt, &tm.yt, it, &sm.full_y);
+      if (it + 1 < n_chunks) load_d(it + 1);  // the decay of step it - 1 has run: its slot is free
+      waiter.wait(&sm.z_done, par);
+      load_tri(sm.tt, &tm.tt, it, &sm.go_z);
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMAs
+    // (the terminal cotangent must be in tensor memory: barrier 1, decay group and this warp)
+    asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+    tc_fence_after();
+    const uint32_t leader = elect_leader();
+    const uint32_t a0 = smem_u32(sm.at), kn0 = smem_u32(sm.kn), tt0 = smem_u32(sm.tt);
+    const uint32_t q0 = smem_u32(sm.q), y0 = smem_u32(sm.yt);
+    const uint32_t id64 = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
+    const uint32_t id_pos = idesc(128, 128, kFmtTF32, kMajorK, kMajorMN);
+    const uint32_t id_neg = idesc(128, 128, kFmtTF32, kMajorK, kMajorK, 1, 0);
+    const uint32_t d_o = tb + kColDo, z = tb + kColZ;
+    // dR^T = dO^T Aqk   (A: dO columns, K = 64 tokens; B: At[j][i] read K-major)
+    auto issue_a = [&](int it) {
+      const uint32_t r = tb + kColR + 64u * (uint32_t(it) & 1u);
+      waiter.wait(&sm.go_a, uint32_t(it) & 1u);
       tc_fence_after();
-      const uint32_t d0 = smem_u32(sm.dot), a0 = smem_u32(sm.at), kn0 = smem_u32(sm.kn);
-      const uint32_t id64 = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
-      // dR^T = dO^T Aqk   (A: dO^T [v x i], B: At[j][i] read K-major)
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ss(tb + kColR, smem_desc(d0 + ks * 256, 128, kRsDot), smem_desc_sw128_k(a0, 8192, ks), id64,
-                    ks > 0 ? 1u : 0u);
+        mma_tf32_ts(r, d_o + ks * 8, smem_desc_sw128_k(a0, 8192, ks), id64, ks > 0 ? 1u : 0u, leader);
       }
+      mma_commit(&sm.a_done, leader);
+    };
+    issue_a(0);
+    for (int it = 0; it < n_chunks; ++it) {
+      const uint32_t par = uint32_t(it) & 1u;
+      const uint32_t s_old = tb + kColS + 128u * par, s_new = tb + kColS + 128u * (par ^ 1u);
+      const uint32_t r = tb + kColR + 64u * par;
       // dR^T += dS^T Kt^T (A: cotangent columns, K = 128 keys; B: Kn[j][k] read K-major)
+      waiter.wait(&sm.full_k, par);
+      if (it > 0) waiter.wait(&sm.s_done, par ^ 1u);
+      tc_fence_after();
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {
-        mma_tf32_ts(tb + kColR, tb + kColS + ks * 8, smem_desc_sw128_k(kn0, 8192, ks), id64, 1u);
+        mma_tf32_ts(r, s_old + ks * 8, smem_desc_sw128_k(kn0, 8192, ks), id64, 1u, leader);
       }
-      // dZ^T = dR^T T     (A: the accumulator just produced, K = 64 tokens; B: Tt[j][i] read K-major)
-      const uint32_t tt0 = smem_u32(sm.tt);
-#pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ts(tb + kColZ, tb + kColR + ks * 8, smem_desc_sw128_k(tt0, 8192, ks), id64, ks > 0 ? 1u : 0u);
-      }
-      mma_commit(&sm.bar_mma1);
-    }
-    // the next chunk's dO is on its way while the tensor cores work
-    if (c > 0) load_do(c - 1, do_raw);
-    waiter.wait(&sm.bar_mma1, par);
-    tc_fence_after();
-    if (tid == 0 && c > 0) load_ak(c - 1);  // At / Kn are free again
-
-    // ---- dZ out: 16 token columns of value row v into the staging tile X[r = j][c = v] ----------------
-    {
-      uint8_t* col = sm.dz + (vrow >> 2) * kCsZ + (vrow & 3) * 4;
-      uint32_t r[16];
-      tmem_ld16(tmem_addr(tb, lane_base, kColZ + j0), r);
-      tmem_wait_ld();
-#pragma unroll
-      for (int jj = 0; jj < 16; ++jj) {
-        const int j = j0 + jj;
-        *reinterpret_cast<float*>(col + (j >> 3) * kRsZ + (j & 7) * 16) =
-            (upstream_failed || waiter.dead) ? poison_nan() : to_tf32(__uint_as_float(r[jj]));
-      }
-    }
-    // ---- decay: dS^T <- dS^T diag(d) -------------------------------------------------------------------
-    waiter.wait(&sm.bar_qy, par);
-    {
-      uint32_t r[32];
-      tmem_ld32(tmem_addr(tb, lane_base, kColS + k0), r);
-      tmem_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * sm.d[k0 + j]);
-      tmem_st32(tmem_addr(tb, lane_base, kColS + k0), r);
-      tmem_wait_st();
-    }
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+      mma_commit(&sm.k_done, leader);
+      // dS'^T += dO^T Qg  (K = 64 tokens; B: Q[i][k] read MN-major)
+      waiter.wait(&sm.go_q, par);
       tc_fence_after();
-      bulk_s2g(p.sc + sc.off_dz() + ch_of(c) * kBlobDZ, sm.dz, uint32_t(kBlobDZ));
-      bulk_commit();
-      const uint32_t d0 = smem_u32(sm.dot), q0 = smem_u32(sm.q), y0 = smem_u32(sm.yt);
-      const uint32_t id_pos = idesc(128, 128, kFmtTF32, kMajorK, kMajorMN);
-      const uint32_t id_neg = idesc(128, 128, kFmtTF32, kMajorK, kMajorK, 1, 0);
-      // dS^T += dO^T Qg   (K = 64 tokens; B: Q[i][k] read MN-major)
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ss(tb + kColS, smem_desc(d0 + ks * 256, 128, kRsDot), smem_desc_sw128_mn(q0, 8192, ks), id_pos, 1u);
+        mma_tf32_ts(s_new, d_o + ks * 8, smem_desc_sw128_mn(q0, 8192, ks), id_pos, 1u, leader);
       }
-      // dS^T -= dR^T Y    (A: dR^T columns, K = 64 tokens; B: Yt[k][j] read K-major)
+      mma_commit(&sm.do_done, leader);
+      // dS'^T -= dR^T Y   (A: dR^T columns, K = 64 tokens; B: Yt[k][j] read K-major)
+      waiter.wait(&sm.full_y, par);
+      waiter.wait(&sm.k_done, par);
+      tc_fence_after();
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ts(tb + kColS, tb + kColR + ks * 8, smem_desc_sw128_k(y0, 16384, ks), id_neg, 1u);
+        mma_tf32_ts(s_new, r + ks * 8, smem_desc_sw128_k(y0, 16384, ks), id_neg, 1u, leader);
       }
-      mma_commit(&sm.bar_mma2);
+      mma_commit(&sm.s_done, leader);
+      // dZ^T = dR^T T     (A: dR^T columns, K = 64 tokens; B: Tt[j][i] read K-major)
+      waiter.wait(&sm.go_z, par);
+      tc_fence_after();
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        mma_tf32_ts(z, r + ks * 8, smem_desc_sw128_k(tt0, 8192, ks), id64, ks > 0 ? 1u : 0u, leader);
+      }
+      mma_commit(&sm.z_done, leader);
+      if (it + 1 < n_chunks) issue_a(it + 1);
     }
-  }
-
-  // ---- cotangent of the initial state: slot 0 and d_initial_state ------------------------------------
-  if (p.n_chunks > 0) {
-    waiter.wait(&sm.bar_mma2, (it - 1) & 1u);
-    tc_fence_after();
-  }
-  {
-    float* slot = p.d_bnd + ((b * (p.n_chunks + 1)) * p.H + h) * kStateElems + vrow;
-    float* init = (p.ds_init != nullptr) ? p.ds_init + bh * kStateElems + vrow : nullptr;
-    uint32_t r[32];
-    tmem_ld32(tmem_addr(tb, lane_base, kColS + k0), r);
-    tmem_wait_ld();
-    const bool failed = upstream_failed || waiter.dead;
+  } else if (warp < kBScanDo0) {
+    // ---------------------------------------------------------------- decay of the cotangent
+    // thread = value row of the transposed cotangent (TMEM lane) x one half of the 128 key columns
+    const int q4 = warp & 3, half = (warp - kBScanDecay0) >> 2;
+    const int vrow = 32 * q4 + lane, k0 = 64 * half;
+    const uint32_t lane_base = 32u * q4;
+    const int64_t state = (int64_t(sq.sid) * p.H + h) * kStateElems;
+    const bool sender = lane == 0 && ((warp - kBScanDecay0) & 3) == 0;  // sends this half's staged rows
+    uint32_t lo[32], hi[32];
+    auto half_barrier = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory"); };
+    auto load_state = [&](uint32_t col) {
+      tmem_ld32(tmem_addr(tb, lane_base, col + k0), lo);
+      tmem_ld32(tmem_addr(tb, lane_base, col + k0 + 32), hi);
+      tmem_wait_ld();
+    };
+    auto store_state = [&](uint32_t col) {
+      tmem_st32(tmem_addr(tb, lane_base, col + k0), lo);
+      tmem_st32(tmem_addr(tb, lane_base, col + k0 + 32), hi);
+      tmem_wait_st();
+    };
+    // 32 key rows of the cotangent at the end of chunk c, 16 KiB, through the staging buffer of this half
+    auto send_rows = [&](const uint32_t (&x)[32], int c, int kr) {
+      if (sender) bulk_wait_read_all();  // the previous rows have left the buffer
+      half_barrier();
+      float* dst = sm.ck[half] + vrow;
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float x = failed ? poison_nan() : __uint_as_float(r[j]);
+      for (int j = 0; j < 32; ++j) dst[j * kDim] = __uint_as_float(x[j]);
+      fence_async_smem();
+      half_barrier();
+      if (sender) {
+        bulk_s2g(p.d_bnd + ((int64_t(sq.slot0 + c + 1) * p.H + h) * kDim + kr) * kDim, sm.ck[half], 32u * kDim * 4u);
+        bulk_commit();
+      }
+    };
+    {
+      const float* src = (p.ds_final != nullptr) ? p.ds_final + state + vrow : nullptr;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) {
+        lo[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
+        hi[j] = (src != nullptr) ? __float_as_uint(src[(k0 + 32 + j) * kDim]) : 0u;
+      }
+      store_state(kColS);
+      tc_fence_before();
+      asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+    }
+    for (int it = 0; it < n_chunks; ++it) {
+      const uint32_t par = uint32_t(it) & 1u;
+      if (it > 0) {
+        waiter.wait(&sm.s_done, par ^ 1u);
+        tc_fence_after();
+        load_state(kColS + 128u * par);
+      }
+      waiter.wait(&sm.full_d[par], uint32_t(it >> 1) & 1u);
+#pragma unroll
+      for (int j4 = 0; j4 < 8; ++j4) {
+        const float4 da = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 4 * j4]);
+        const float4 db = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 32 + 4 * j4]);
+        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * da.x);
+        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * da.y);
+        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * da.z);
+        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * da.w);
+        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * db.x);
+        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * db.y);
+        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * db.z);
+        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * db.w);
+      }
+      store_state(kColS + 128u * (par ^ 1u));
+      arrive(&sm.go_q);
+      // the cotangent at the end of this chunk, off the chain: it is still in its buffer, which this group
+      // alone overwrites, one step later
+      load_state(kColS + 128u * par);
+      send_rows(lo, chunk_of(it), k0);
+      send_rows(hi, chunk_of(it), k0 + 32);
+    }
+    // ---- cotangent of the initial state: slot 0 and d_initial_state ----------------------------------
+    waiter.wait(&sm.s_done, uint32_t(n_chunks - 1) & 1u);
+    tc_fence_after();
+    load_state(kColS + 128u * (uint32_t(n_chunks) & 1u));
+    float* slot = p.d_bnd + (int64_t(sq.slot0) * p.H + h) * kStateElems + vrow;
+    float* init = (p.ds_init != nullptr) ? p.ds_init + state + vrow : nullptr;
+    const bool failed = sm.failed != 0;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      const float x = failed ? poison_nan() : __uint_as_float(j < 32 ? lo[j & 31] : hi[j & 31]);
       slot[(k0 + j) * kDim] = x;
       if (init != nullptr) init[(k0 + j) * kDim] = x;
     }
+    if (sender) bulk_wait_all();  // the last staged rows are in global memory before the CTA retires
+  } else {
+    // ---------------------------------------------------------------- dO in, dZ out
+    // thread = value row (TMEM lane) x one half of the 64 tokens
+    const int q4 = warp & 3, half = (warp - kBScanDo0) >> 2;
+    const int vrow = 32 * q4 + lane, i0 = 32 * half;
+    const uint32_t lane_base = 32u * q4;
+    const bool sender = tid == kBScanDo0 * 32;
+    auto group_barrier = [&] { asm volatile("bar.sync 4, 256;" ::: "memory"); };
+    const T* src = reinterpret_cast<const T*>(sm.d_out) + i0 * kDim + vrow;
+    auto build_do = [&](int it) {
+      waiter.wait(&sm.full_o, uint32_t(it) & 1u);
+      uint32_t x[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(to_float(src[j * kDim]));
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sm.do_read);
+      const int n_valid = sq.len - chunk_of(it) * kChunk;
+      if (n_valid < kChunk) {  // past the end of the sequence there is no cotangent
+#pragma unroll
+        for (int j = 0; j < 32; ++j) x[j] = (i0 + j < n_valid) ? x[j] : 0u;
+      }
+      if (it > 0) {
+        waiter.wait(&sm.do_done, uint32_t(it - 1) & 1u);
+        tc_fence_after();
+      }
+      tmem_st32(tmem_addr(tb, lane_base, kColDo + i0), x);
+      tmem_wait_st();
+      arrive(&sm.go_a);
+    };
+    arrive(&sm.go_z);  // no earlier step holds up the first dZ
+    build_do(0);
+    uint8_t* col = sm.dz + (vrow >> 2) * kCsZ + (vrow & 3) * 4;
+    for (int it = 0; it < n_chunks; ++it) {
+      if (it + 1 < n_chunks) build_do(it + 1);
+      waiter.wait(&sm.z_done, uint32_t(it) & 1u);
+      tc_fence_after();
+      uint32_t r[32];
+      tmem_ld32(tmem_addr(tb, lane_base, kColZ + i0), r);
+      tmem_wait_ld();
+      if (it + 1 < n_chunks) arrive(&sm.go_z);
+      // dZ out: 32 token columns of value row v into the staging tile X[r = j][c = v], one bulk store
+      const bool failed = sm.failed != 0;
+      if (sender) bulk_wait_read_all();  // the previous tile has left the staging buffer
+      group_barrier();
+#pragma unroll
+      for (int jj = 0; jj < 32; ++jj) {
+        const int j = i0 + jj;
+        *reinterpret_cast<float*>(col + (j >> 3) * kRsZ + (j & 7) * 16) =
+            failed ? poison_nan() : to_tf32(__uint_as_float(r[jj]));
+      }
+      fence_async_smem();
+      group_barrier();
+      if (sender) {
+        bulk_s2g(p.dz + ch_of(it) * kBlobDZ, sm.dz, uint32_t(kBlobDZ));
+        bulk_commit();
+      }
+    }
+    if (sender) bulk_wait_all();  // the last dZ tile is in global memory before the CTA retires
   }
-  if (tid == 0) bulk_wait_all();  // the last dZ tile is in global memory before the CTA retires
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tb, 256);
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tb, 512);
+  }
 }
 
 
@@ -371,13 +465,13 @@ __device__ __forceinline__ uint32_t d6_col(int I) { return (I == 3) ? 0u : (I ==
 
 struct VjpParams {
   const void *q, *k, *v, *g, *beta, *w, *d_out;
-  const uint8_t* ws;    // workspace of the training forward (Rn)
   const uint8_t* sc;    // scratch: dZ written by the reverse scan
   const float* bnd;     // [B, n_chunks+1, H,128,128] forward states
   const float* d_bnd;   // same shape, cotangents
   void *dq, *dk, *dv, *dg, *dbeta, *dw;
   int* status;
-  int64_t T, H, n_chunks, n_ch;
+  int64_t n_ch;
+  int H;
   float scale;
 };
 // tensor maps of the seven sequence tensors the VJP kernel reads (for L2 prefetches only)
@@ -444,18 +538,17 @@ __device__ __forceinline__ void tmem_ld8f(uint32_t taddr, float (&x)[8]) {
 
 // kF32Grads: dq, dk, dv, dbeta, dw leave as fp32 instead of the sequence dtype (the values before
 // their final rounding; used by tests to judge the arithmetic apart from the 16-bit cast).
-// kRagged: the sequence length is not a multiple of 64 and the last chunk of every (batch, head) is
-// partial; only this instantiation carries the guards (they cost the others 6 %).
-template <typename T, typename G, bool kF32Grads = false, bool kRagged = false>
+// kRagged: some sequence length is not a multiple of 64, its last chunk is partial; only this
+// instantiation carries the guards (they cost the others 6 %).
+template <typename T, typename G, typename Seqs, bool kF32Grads = false, bool kRagged = false>
 __global__ void __launch_bounds__(kVjpThreads, 1)
-chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s0,
+chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ CUtensorMap tm_s0,
                      const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_rn,
                      const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
                      const __grid_constant__ CUtensorMap tm_dbeta, const __grid_constant__ VjpInputMaps tm_in) {
   using O = typename std::conditional<kF32Grads, float, T>::type;  // element type of dq, dk, dv, dbeta, dw
   extern __shared__ __align__(1024) uint8_t smem[];
   VjpMisc& ms = *reinterpret_cast<VjpMisc*>(smem + kOffMisc);
-  const WsLayout ws{p.n_ch, true};
   const ScratchLayout sc{p.n_ch};
   BoundedWaiter waiter(p.status);
   // a wait that ran out earlier (forward or reverse scan) left garbage behind: gradients become NaN
@@ -481,6 +574,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   __syncthreads();
   tc_fence_after();
   const uint32_t tb = ms.tmem_base;
+  const uint32_t leader = elect_leader();
   uint32_t mma_phase = 0;
   constexpr uint32_t kColD2 = 64, kColD3 = 128, kColD4 = 256, kColD5 = 320;
 
@@ -493,46 +587,43 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   // memory, and land during its final chain.
   // The chain keeps the dO rows of the stack and the dS_1 buffer for its own tiles, so the copies come in
   // two parts: S_0, R and dZ before the chain, the dS_1 half after it (bar_s expects both from the start).
-  auto s0_slot_of = [&](int64_t ch_) {
-    const int64_t h_ = ch_ % p.H, c_ = (ch_ / p.H) % p.n_chunks, b_ = ch_ / (p.H * p.n_chunks);
-    return int((b_ * (p.n_chunks + 1) + c_) * p.H + h_);
+  // unit -> head, first token row, tokens that exist, checkpoint slot of the chunk start
+  // (all 31-bit numbers, the launcher checks: 32-bit divisions, a fraction of the 64-bit routine)
+  struct Place { int h, row, valid, slot; };
+  auto locate = [&](int64_t ch_) {
+    const int chunk = int(uint32_t(ch_) / uint32_t(p.H));
+    const SeqInfo sq = seqs.at(seqs.find(chunk));
+    const int c_ = chunk - sq.chunk0, h_ = int(ch_) - chunk * p.H;
+    return Place{h_, int(sq.row0) + c_ * kChunk, min(kChunk, sq.len - c_ * kChunk), (sq.slot0 + c_) * p.H + h_};
   };
-  auto issue_loads = [&](int64_t ch_) {
+  auto issue_loads = [&](int64_t ch_, int slot_) {
     mbar_arrive_expect_tx(&ms.bar_s, uint32_t(65536 + 32768));
-#pragma unroll
-    for (int sl = 0; sl < 4; ++sl) tma_load_3d(smem + kOffS0 + sl * 16384, &tm_s0, 32 * sl, 0, s0_slot_of(ch_), &ms.bar_s);
+    tma_load_4d(smem + kOffS0, &tm_s0, 0, 0, 0, slot_, &ms.bar_s);
     mbar_arrive_expect_tx(&ms.bar_a, uint32_t(kBlobDZ + kBlobRn));
-#pragma unroll
-    for (int sl = 0; sl < 4; ++sl) tma_load_3d(smem + kOffRn + sl * 8192, &tm_rn, 32 * sl, 0, int(ch_), &ms.bar_a);
+    tma_load_4d(smem + kOffRn, &tm_rn, 0, 0, 0, int(ch_), &ms.bar_a);
     bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + ch_ * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
   };
-  auto issue_ds1 = [&](int64_t ch_) {
-#pragma unroll
-    for (int sl = 0; sl < 2; ++sl) {
-      tma_load_3d(smem + kOffDs1 + sl * 16384, &tm_ds, 32 * sl, 0, s0_slot_of(ch_) + int(p.H), &ms.bar_s);
-    }
+  auto issue_ds1 = [&](int slot_) {
+    tma_load_4d(smem + kOffDs1, &tm_ds, 0, 0, 0, slot_ + p.H, &ms.bar_s);
   };
   if (tid == 0 && int64_t(blockIdx.x) < p.n_ch) {
-    issue_loads(blockIdx.x);
-    issue_ds1(blockIdx.x);
+    const int slot_ = locate(blockIdx.x).slot;
+    issue_loads(blockIdx.x, slot_);
+    issue_ds1(slot_);
   }
 
   uint32_t iter = 0;
   for (int64_t ch = blockIdx.x; ch < p.n_ch; ch += gridDim.x, ++iter) {
   const uint32_t par = iter & 1u;
-  // (unit numbers fit 31 bits, the launcher checks: 32-bit divisions, a fraction of the 64-bit routine)
-  const uint32_t bc32 = uint32_t(ch) / uint32_t(p.H);
-  const int64_t h = uint32_t(ch) - bc32 * uint32_t(p.H);
-  const int64_t b = bc32 / uint32_t(p.n_chunks);
-  const int64_t c = bc32 - uint32_t(b) * uint32_t(p.n_chunks);
-  const int64_t t0 = c * kChunk;
-  auto seq_idx = [&](int tok) { return ((b * p.T + t0 + tok) * p.H + h) * int64_t(kDim); };
-  // tokens of this chunk that exist: 64 except in the last chunk of a ragged sequence, whose missing
-  // tokens read as zeros (the identity step) and whose gradients are not stored
-  const int n_valid = kRagged ? int(min(int64_t(kChunk), p.T - t0)) : kChunk;
+  const Place at = locate(ch);
+  const int h = at.h;
+  auto seq_idx = [&](int tok) { return (int64_t(at.row + tok) * p.H + h) * int64_t(kDim); };
+  // tokens of this chunk that exist: 64 except in the last chunk of a sequence, whose missing tokens read
+  // as zeros (the identity step) and whose gradients are not stored
+  const int n_valid = kRagged ? at.valid : kChunk;
   auto there = [&](int tok) { return !kRagged || tok < n_valid; };            // does token `tok` of the chunk exist
   auto clamped = [&](int tok) { return kRagged ? min(tok, n_valid - 1) : tok; };  // a token that does
-  const int ds1_slot = int((b * (p.n_chunks + 1) + c + 1) * p.H + h);
+  const int ds1_slot = at.slot + p.H;
   // dd[k] += sum over the 64 value columns of half `hf` of dS_1[k][v] S_0[k][v], both read from their
   // shared-memory tiles.  The two tiles are swizzled alike (a line = 32 values of one key row, its
   // 16-byte pieces permuted by the row), so equal positions hold equal (k, v) and the order inside a
@@ -603,7 +694,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   __syncthreads();
   // ---- first MMA batch: M4 (first half) dKt^T = dS_1[:, v < 64] R[:, v < 64]^T ;
   //      M2 [-dL ; dA] = [dZ ; dO] R^T ;  M3 [-dE ; dQg]^T = S_0 [dZ ; dO]^T ------------------------------
-  if (tid == 0) {
+  if (warp == 0) {
     tc_fence_after();
     const uint32_t st = smem_u32(smem + kOffStack), rn = smem_u32(smem + kOffRn);
     const uint32_t s0 = smem_u32(smem + kOffS0), d1 = smem_u32(smem + kOffDs1);
@@ -612,25 +703,24 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
       mma_tf32_ss(tb + kColD4, smem_desc_sw128_k(d1, 16384, ks), smem_desc_sw128_k(rn, 8192, ks), id64,
-                  ks > 0 ? 1u : 0u);
+                  ks > 0 ? 1u : 0u, leader);
     }
-    mma_commit(&ms.bar_r);  // the dS_1 buffer may be refilled once these have run
+    mma_commit(&ms.bar_r, leader);  // the dS_1 buffer may be refilled once these have run
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
       mma_tf32_ss(tb + kColD2, smem_desc(st + ks * 2 * kCsN, kCsN, kRsN), smem_desc_sw128_k(rn, 8192, ks), id64,
-                  ks > 0 ? 1u : 0u);
+                  ks > 0 ? 1u : 0u, leader);
     }
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
       mma_tf32_ss(tb + kColD3, smem_desc_sw128_k(s0, 16384, ks), smem_desc(st + ks * 2 * kCsN, kCsN, kRsN), id128,
-                  ks > 0 ? 1u : 0u);
+                  ks > 0 ? 1u : 0u, leader);
     }
-    mma_commit(&ms.bar_m);
+    mma_commit(&ms.bar_m, leader);
     // the second 64 value columns of dS_1 replace the first as soon as their product has run
     waiter.wait(&ms.bar_r, 0);
-    mbar_arrive_expect_tx(&ms.bar_d, 32768u);
-#pragma unroll
-    for (int sl = 0; sl < 2; ++sl) tma_load_3d(smem + kOffDs1 + sl * 16384, &tm_ds, 64 + 32 * sl, 0, ds1_slot, &ms.bar_d);
+    mbar_arrive_expect_tx(&ms.bar_d, 32768u, leader);
+    tma_load_4d(smem + kOffDs1, &tm_ds, 0, 0, 2, ds1_slot, &ms.bar_d, leader);
   }
   // ---- under the tensor cores: log-decay prefixes, dv = dZ w, dw = dZ v, and the raw inputs of the
   // Gram operands.  Every load is issued before the first store: the outputs may alias the inputs as
@@ -694,15 +784,15 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   dd_half(1);
   tc_fence_before();
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0) {
     tc_fence_after();
     const uint32_t rn = smem_u32(smem + kOffRn), d1 = smem_u32(smem + kOffDs1);
     const uint32_t id64 = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      mma_tf32_ss(tb + kColD4, smem_desc_sw128_k(d1, 16384, ks), smem_desc_sw128_k(rn, 8192, 8 + ks), id64, 1u);
+      mma_tf32_ss(tb + kColD4, smem_desc_sw128_k(d1, 16384, ks), smem_desc_sw128_k(rn, 8192, 8 + ks), id64, 1u, leader);
     }
-    mma_commit(&ms.bar_r);
+    mma_commit(&ms.bar_r, leader);
   }
   waiter.wait(&ms.bar_m, mma_phase & 1u);
   ++mma_phase;
@@ -794,7 +884,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  if (tid == 0) {
+  if (warp == 0) {
     tc_fence_after();
     const uint32_t s2 = smem_u32(smem + kOffStack2);
     const uint32_t dlt = smem_u32(smem + kOffDLt), dat = smem_u32(smem + kOffDAt);
@@ -805,9 +895,10 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
     for (int I = 0; I < 4; ++I) {
       const uint32_t kit = smem_u32(smem + kit_offset(I));
       const uint32_t rs = uint32_t(kit_rs(I));
+#pragma unroll
       for (int ks = 0; ks < 2 * (I + 1); ++ks) {
         mma_tf32_ss(tb + kColD5 + 32 * I, smem_desc(kit + ks * 256, 128, rs),
-                    smem_desc(s2 + 4 * I * 2048 + ks * 256, 128, 2048), id32, ks > 0 ? 1u : 0u);
+                    smem_desc(s2 + 4 * I * 2048 + ks * 256, 128, 2048), id32, ks > 0 ? 1u : 0u, leader);
       }
     }
     // (dK^I)^T = Ea^T[:, block I] dL[block I, :] + Qa^T[:, block I] dA[block I, :]
@@ -821,29 +912,28 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
           mma_tf32_ss(tb + d6_col(I), smem_desc(a_base + ks * 256, 128, kRsT),
-                      smem_desc(b_base + ks * 2 * kCsS, kCsS, kRsS), idn, (pt | ks) ? 1u : 0u);
+                      smem_desc(b_base + ks * 2 * kCsS, kCsS, kRsS), idn, (pt | ks) ? 1u : 0u, leader);
         }
       }
     }
-    mma_commit(&ms.bar_m);
+    mma_commit(&ms.bar_m, leader);
   }
   waiter.wait(&ms.bar_m, mma_phase & 1u);
   ++mma_phase;
   tc_fence_after();
   // shared memory (all but the small arrays of VjpMisc) is dead from here on: fetch the next chunk-head
-  if (tid == 0 && ch + gridDim.x < p.n_ch) issue_loads(ch + gridDim.x);
+  if (tid == 0 && ch + gridDim.x < p.n_ch) issue_loads(ch + gridDim.x, locate(ch + gridDim.x).slot);
   // The sequence tensors of the next chunk-head are read with per-thread loads, whose rate is set by the
   // bytes in flight over the latency: have its seven [64][128] tiles brought into L2 while the chain runs.
   if (tid == 64 && ch + gridDim.x < p.n_ch) {
-    const int64_t ch_ = ch + gridDim.x;
-    const int h_ = int(ch_ % p.H), t_ = int((ch_ / p.H) % p.n_chunks) * kChunk, b_ = int(ch_ / (p.H * p.n_chunks));
-    tma_prefetch_l2_4d(&tm_in.d_out, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.g, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.w, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.v, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.k, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.q, 0, h_, t_, b_);
-    tma_prefetch_l2_4d(&tm_in.beta, 0, h_, t_, b_);
+    const Place nx = locate(ch + gridDim.x);
+    tma_prefetch_l2_3d(&tm_in.d_out, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.g, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.w, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.v, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.k, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.q, 0, nx.h, nx.row);
+    tma_prefetch_l2_3d(&tm_in.beta, 0, nx.h, nx.row);
   }
   // hand k, q and the log-decay prefix to the chain, which walks the tokens of one channel: these threads
   // hold them as 4 x 4 patches (the same values, and for G the same summation order, as the tiles above)
@@ -999,19 +1089,31 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  // The rows behind a partial chunk belong to somebody else: its gradients leave row by row, those of a
+  // whole chunk by TMA.  (bulk_wait_read_all above and the barriers of phase A guard the tiles' reuse.)
+  if (!kF32Grads && kRagged && n_valid < kChunk) {
+    for (int e = tid; e < n_valid * 16; e += kVjpThreads) {
+      const int tok = e >> 4, piece = e & 15;
+      const int64_t idx = seq_idx(tok) + 8 * piece;
+      const int off = tok * 256 + piece * 16;
+      *reinterpret_cast<uint4*>(static_cast<T*>(p.dq) + idx) = *reinterpret_cast<const uint4*>(smem + kOffTileQ + off);
+      *reinterpret_cast<uint4*>(static_cast<T*>(p.dk) + idx) = *reinterpret_cast<const uint4*>(smem + kOffTileK + off);
+      *reinterpret_cast<uint4*>(static_cast<T*>(p.dbeta) + idx) =
+          *reinterpret_cast<const uint4*>(smem + beta_tile_offset(tok >> 4) + (tok & 15) * 256 + piece * 16);
+    }
+  }
   if (tid == 0) {
-    if (!kF32Grads) {
-      // (the boxes are clipped at token T - 1: rows of a partial last chunk that do not exist are dropped)
-      tma_store_4d(&tm_dq, 0, int(h), int(t0), int(b), smem + kOffTileQ);
-      tma_store_4d(&tm_dk, 0, int(h), int(t0), int(b), smem + kOffTileK);
+    if (!kF32Grads && !(kRagged && n_valid < kChunk)) {
+      tma_store_3d(&tm_dq, 0, h, at.row, smem + kOffTileQ);
+      tma_store_3d(&tm_dk, 0, h, at.row, smem + kOffTileK);
 #pragma unroll
-      for (int bq = 0; bq < 4; ++bq) {  // (a box that starts past token T - 1 is dropped whole)
-        tma_store_4d(&tm_dbeta, 0, int(h), int(t0) + 16 * bq, int(b), smem + beta_tile_offset(bq));
+      for (int bq = 0; bq < 4; ++bq) {
+        tma_store_3d(&tm_dbeta, 0, h, at.row + 16 * bq, smem + beta_tile_offset(bq));
       }
       bulk_commit();
     }
     // the G tile is dead: the dS_1 half of the next chunk-head may land on it
-    if (ch + gridDim.x < p.n_ch) issue_ds1(ch + gridDim.x);
+    if (ch + gridDim.x < p.n_ch) issue_ds1(locate(ch + gridDim.x).slot);
   }
   }  // chunk-head loop
   if (tid == 0) bulk_wait_all();  // the last dq / dk tiles are in global memory before the CTA retires
@@ -1021,106 +1123,137 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ CUtensorMap tm_s
 }  // namespace
 
 // ---- launcher ---------------------------------------------------------------------------------------
+namespace {
+
+struct BackwardCall {
+  const void *q, *k, *v, *g, *beta, *w, *d_out;
+  const float *ds_final, *bnd;
+  float* d_bnd;
+  const uint8_t* workspace;
+  uint8_t* scratch;
+  void *dq, *dk, *dv, *dg, *dbeta, *dw;
+  float* ds_init;
+  int64_t rows, H;  // token rows of the sequence tensors, heads
+  int dtype, g_dtype;
+  float scale;
+  int grads_f32;
+  bool ragged;      // some last chunk is partial
+};
+
+struct VjpMaps {
+  CUtensorMap s0, ds, rn, dq, dk, dbeta;
+  VjpInputMaps in;
+};
+
+template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
+int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStream_t stream) {
+  auto kernel = chunk_bwd_vjp_kernel<T, G, Seqs, kF32Grads, kRagged>;
+  cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kVjpSmemBytes);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  int sm_count = 0;
+  if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
+  const unsigned grid = unsigned(p.n_ch < int64_t(sm_count) ? p.n_ch : int64_t(sm_count));
+  kernel<<<grid, kVjpThreads, kVjpSmemBytes, stream>>>(p, seqs, m.s0, m.ds, m.rn, m.dq, m.dk, m.dbeta, m.in);
+  return check_launch();
+}
+
+template <typename Seqs>
+int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream) {
+  if (a.grads_f32 && !(a.dtype == GDN2_BF16 && a.g_dtype == GDN2_FP32)) return GDN2_ERR_UNSUPPORTED;
+  const int64_t n_ch = int64_t(seqs.total_chunks()) * a.H;
+  const int64_t n_slots = (int64_t(seqs.total_chunks()) + seqs.count()) * a.H;
+  if (n_ch <= 0 || n_slots > int64_t(0x7fffffff) || a.rows > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
+  const WsLayout ws{n_ch, true};
+  const ScratchLayout sc{n_ch};
+  // the status word is the one the forward cleared: a forward failure stays visible to backward
+  int* status = reinterpret_cast<int*>(const_cast<uint8_t*>(a.workspace) + ws.off_status());
+
+  profile_mark(3, stream);
+  // the reverse scan's operands: the forward's tiles, each in the swizzle of the role backward reads it in
+  BScanMaps tm;
+  if (!encode_tile_map(&tm.at, a.workspace + ws.off_at(), n_ch, kChunk, kChunk, false, 32, 1) ||
+      !encode_tile_map(&tm.tt, a.workspace + ws.off_tt(), n_ch, kChunk, kChunk, false, 32, 1) ||
+      !encode_tile_map(&tm.kn, a.workspace + ws.off_kn(), n_ch, kChunk, kDim, false) ||
+      !encode_tile_map(&tm.q, a.workspace + ws.off_q(), n_ch, kChunk, kDim, true) ||
+      !encode_tile_map(&tm.yt, a.workspace + ws.off_yt(), n_ch, kDim, kChunk, false) ||
+      !encode_sequence_map(&tm.d_out, a.d_out, a.rows, a.H, a.dtype)) {
+    return GDN2_ERR_LAUNCH;
+  }
+  const BScanParams sp{a.workspace + ws.off_d(), a.scratch + sc.off_dz(), a.ds_final, a.d_bnd, a.ds_init, status,
+                       int(a.H)};
+  {
+    const int smem = int(sizeof(BScanSmem));
+    auto kernel = a.dtype == GDN2_BF16 ? chunk_bwd_scan_kernel<__nv_bfloat16, Seqs>
+                                       : chunk_bwd_scan_kernel<__half, Seqs>;
+    cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+    kernel<<<unsigned(seqs.count() * a.H), kBScanThreads, smem, stream>>>(sp, seqs, tm);
+  }
+  int st = check_launch();
+  if (st != GDN2_OK) return st;
+  profile_mark(4, stream);
+
+  // dq, dk and dbeta leave the VJP kernel through tiled TMA stores; the maps of the inputs serve prefetches
+  VjpMaps m;
+  const int grad_dtype = a.grads_f32 ? GDN2_FP32 : a.dtype;
+  if (!encode_tile_map(&m.s0, reinterpret_cast<const uint8_t*>(a.bnd), n_slots, kDim, kDim, false) ||
+      !encode_tile_map(&m.ds, reinterpret_cast<const uint8_t*>(a.d_bnd), n_slots, kDim, kDim, false, 0, 2) ||
+      !encode_tile_map(&m.rn, a.workspace + ws.off_rn(), n_ch, kChunk, kDim, false) ||
+      !encode_sequence_map(&m.dq, a.dq, a.rows, a.H, grad_dtype) ||
+      !encode_sequence_map(&m.dk, a.dk, a.rows, a.H, grad_dtype) ||
+      !encode_sequence_map(&m.dbeta, a.dbeta, a.rows, a.H, grad_dtype, 16) ||
+      !encode_sequence_map(&m.in.q, a.q, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&m.in.k, a.k, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&m.in.v, a.v, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&m.in.g, a.g, a.rows, a.H, a.g_dtype) ||
+      !encode_sequence_map(&m.in.beta, a.beta, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&m.in.w, a.w, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&m.in.d_out, a.d_out, a.rows, a.H, a.dtype)) {
+    return GDN2_ERR_LAUNCH;
+  }
+  const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.bnd, a.d_bnd, a.dq, a.dk, a.dv, a.dg,
+                     a.dbeta, a.dw, status, n_ch, int(a.H), a.scale};
+  constexpr bool kPacked = std::is_same<Seqs, PackedSeqs>::value;
+  if constexpr (!kPacked) {
+    if (a.grads_f32) {
+      st = a.ragged ? launch_vjp<__nv_bfloat16, float, Seqs, true, true>(vp, seqs, m, stream)
+                    : launch_vjp<__nv_bfloat16, float, Seqs, true, false>(vp, seqs, m, stream);
+    } else if (!a.ragged) {
+      GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, { st = launch_vjp<T, G, Seqs, false, false>(vp, seqs, m, stream); });
+    }
+  }
+  if (!a.grads_f32 && (kPacked || a.ragged)) {
+    GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, { st = launch_vjp<T, G, Seqs, false, true>(vp, seqs, m, stream); });
+  }
+  profile_mark(5, stream);
+  return st;
+}
+
+}  // namespace
+
 int launch_chunk_backward(const void* q, const void* k, const void* v, const void* g, const void* beta,
                           const void* w, const void* d_out, const float* ds_final, const float* bnd,
                           float* d_bnd, const uint8_t* workspace, uint8_t* scratch, void* dq, void* dk, void* dv, void* dg,
                           void* dbeta, void* dw, float* ds_init, int64_t B, int64_t T, int64_t H,
                           int64_t full_tokens, int dtype, int g_dtype, float scale, int grads_f32,
                           cudaStream_t stream) {
-  if (grads_f32 && !(dtype == GDN2_BF16 && g_dtype == GDN2_FP32)) return GDN2_ERR_UNSUPPORTED;
   const int64_t n_chunks = full_tokens / kChunk;
-  const int64_t n_ch = B * n_chunks * H;
-  if (n_ch <= 0 || n_ch > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  const WsLayout ws{n_ch, true};
-  // the status word is the one the forward cleared: a forward failure stays visible to backward
-  int* status = reinterpret_cast<int*>(const_cast<uint8_t*>(workspace) + ws.off_status());
-  cudaError_t err;
+  if (B * T > int64_t(0x7fffffff) || B * n_chunks * H > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
+  const UniformSeqs seqs{T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
+  const BackwardCall a{q, k, v, g, beta, w, d_out, ds_final, bnd, d_bnd, workspace, scratch, dq, dk, dv, dg, dbeta,
+                       dw, ds_init, B * T, H, dtype, g_dtype, scale, grads_f32, full_tokens > T};
+  return launch_backward(seqs, a, stream);
+}
 
-  profile_mark(3, stream);
-  // the reverse scan's operands: the forward's tiles, each in the swizzle of the role backward reads it in
-  CUtensorMap tm_at, tm_tt, tm_kn, tm_q, tm_yt;
-  if (!encode_tile_map(&tm_at, workspace + ws.off_at(), n_ch, kChunk, kChunk, false, 32) ||
-      !encode_tile_map(&tm_tt, workspace + ws.off_tt(), n_ch, kChunk, kChunk, false, 32) ||
-      !encode_tile_map(&tm_kn, workspace + ws.off_kn(), n_ch, kChunk, kDim, false) ||
-      !encode_tile_map(&tm_q, workspace + ws.off_q(), n_ch, kChunk, kDim, true) ||
-      !encode_tile_map(&tm_yt, workspace + ws.off_yt(), n_ch, kDim, kChunk, false)) {
-    return GDN2_ERR_LAUNCH;
-  }
-  BScanParams sp{workspace, scratch, d_out, ds_final, d_bnd, ds_init, status, T, H, n_chunks, n_ch};
-  const int scan_smem = int(sizeof(BScanSmem));
-  if (dtype == GDN2_BF16) {
-    auto kernel = chunk_bwd_scan_kernel<__nv_bfloat16>;
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), scan_smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<unsigned(B * H), kBScanThreads, scan_smem, stream>>>(sp, tm_at, tm_tt, tm_kn, tm_q, tm_yt);
-  } else {
-    auto kernel = chunk_bwd_scan_kernel<__half>;
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), scan_smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<unsigned(B * H), kBScanThreads, scan_smem, stream>>>(sp, tm_at, tm_tt, tm_kn, tm_q, tm_yt);
-  }
-  int st = check_launch();
-  if (st != GDN2_OK) return st;
-  profile_mark(4, stream);
-
-  int device = 0, sm_count = 0;
-  err = cudaGetDevice(&device);
-  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
-  if (err != cudaSuccess || sm_count <= 0) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  CUtensorMap tm_s0, tm_ds;
-  const int64_t n_slots = B * (n_chunks + 1) * H;
-  if ((reinterpret_cast<uintptr_t>(bnd) & 15u) != 0 || (reinterpret_cast<uintptr_t>(d_bnd) & 15u) != 0 ||
-      !encode_tile_map(&tm_s0, reinterpret_cast<const uint8_t*>(bnd), n_slots, kDim, kDim, false) ||
-      !encode_tile_map(&tm_ds, reinterpret_cast<const uint8_t*>(d_bnd), n_slots, kDim, kDim, false)) {
-    return GDN2_ERR_LAUNCH;
-  }
-  // dq and dk leave the VJP kernel as [64][128] tiles through tiled TMA stores (rows b * T + t in 31 bits)
-  CUtensorMap tm_dq, tm_dk;
-  if (B * T > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  if ((reinterpret_cast<uintptr_t>(dq) & 15u) != 0 || (reinterpret_cast<uintptr_t>(dk) & 15u) != 0 ||
-      !encode_sequence_map(&tm_dq, dq, B, T, H, grads_f32 ? GDN2_FP32 : dtype) ||
-      !encode_sequence_map(&tm_dk, dk, B, T, H, grads_f32 ? GDN2_FP32 : dtype)) {
-    return GDN2_ERR_LAUNCH;
-  }
-  CUtensorMap tm_dbeta;
-  if ((reinterpret_cast<uintptr_t>(dbeta) & 15u) != 0 ||
-      !encode_sequence_map(&tm_dbeta, dbeta, B, T, H, grads_f32 ? GDN2_FP32 : dtype, 16)) {
-    return GDN2_ERR_LAUNCH;
-  }
-  CUtensorMap tm_rn;
-  if (!encode_tile_map(&tm_rn, workspace + ws.off_rn(), n_ch, kChunk, kDim, false)) return GDN2_ERR_LAUNCH;
-  VjpInputMaps tm_in;
-  {
-    const void* bases[7] = {q, k, v, g, beta, w, d_out};
-    CUtensorMap* maps[7] = {&tm_in.q, &tm_in.k, &tm_in.v, &tm_in.g, &tm_in.beta, &tm_in.w, &tm_in.d_out};
-    for (int i = 0; i < 7; ++i) {
-      if ((reinterpret_cast<uintptr_t>(bases[i]) & 15u) != 0 ||
-          !encode_sequence_map(maps[i], bases[i], B, T, H, i == 3 ? g_dtype : dtype)) {
-        return GDN2_ERR_LAUNCH;
-      }
-    }
-  }
-  VjpParams vp{q, k, v, g, beta, w, d_out, workspace, scratch, bnd, d_bnd, dq, dk, dv, dg, dbeta, dw,
-               status, T, H, n_chunks, n_ch, scale};
-  const unsigned vjp_grid = unsigned(n_ch < int64_t(sm_count) ? n_ch : int64_t(sm_count));
-  const bool ragged = full_tokens > T;  // the last chunk of every (batch, head) is partial
-  if (grads_f32) {
-    auto kernel = ragged ? chunk_bwd_vjp_kernel<__nv_bfloat16, float, true, true>
-                         : chunk_bwd_vjp_kernel<__nv_bfloat16, float, true, false>;
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kVjpSmemBytes);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<vjp_grid, kVjpThreads, kVjpSmemBytes, stream>>>(vp, tm_s0, tm_ds, tm_rn, tm_dq, tm_dk, tm_dbeta, tm_in);
-  } else {
-    GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-      auto kernel = ragged ? chunk_bwd_vjp_kernel<T, G, false, true> : chunk_bwd_vjp_kernel<T, G, false, false>;
-      err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kVjpSmemBytes);
-      if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-      kernel<<<vjp_grid, kVjpThreads, kVjpSmemBytes, stream>>>(vp, tm_s0, tm_ds, tm_rn, tm_dq, tm_dk, tm_dbeta, tm_in);
-    });
-  }
-  st = check_launch();
-  profile_mark(5, stream);
-  return st;
+// `table` as for launch_packed_chunk_forward.
+int launch_packed_chunk_backward(const PackedSeqs& table, const void* q, const void* k, const void* v, const void* g,
+                                 const void* beta, const void* w, const void* d_out, const float* ds_final,
+                                 const float* bnd, float* d_bnd, const uint8_t* workspace, uint8_t* scratch, void* dq,
+                                 void* dk, void* dv, void* dg, void* dbeta, void* dw, float* ds_init, int64_t rows,
+                                 int64_t H, int dtype, int g_dtype, float scale, cudaStream_t stream) {
+  const BackwardCall a{q, k, v, g, beta, w, d_out, ds_final, bnd, d_bnd, workspace, scratch, dq, dk, dv, dg, dbeta,
+                       dw, ds_init, rows, H, dtype, g_dtype, scale, 0, true};
+  return launch_backward(table, a, stream);
 }
 
 }  // namespace gdn2

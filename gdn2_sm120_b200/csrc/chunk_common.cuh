@@ -14,11 +14,9 @@
 //   Kn   [token j (64)][key k (128)]     32 KiB   k * gamma_end / gamma        fwd MN-major, bwd K-major
 //   Yt   [key k (128)][token i (64)]     32 KiB   Y^T, Y = (I+L)^-1 E          fwd MN-major, bwd K-major
 //   At   [token j (64)][token i (64)]    16 KiB   tril(Q_gamma Kbar^T)^T       fwd MN-major, bwd K-major
-//   Tt   [token j (64)][token i (64)]    16 KiB   ((I+L)^-1)^T                 bwd K-major (training only)
+//   Tt   [token j (64)][token i (64)]    16 KiB   ((I+L)^-1)^T                 fwd MN-major, bwd K-major
 //        (both are zero where j > i: the quadrant j >= 32, i < 32 is neither written nor read, the
 //        consumers keep those lines of their shared-memory tile at zero; 12 KiB move)
-//   U    [token j (64)][value v (128)]   32 KiB   U = (I+L)^-1 (w*v)           forward only: copied into
-//                                                                               tensor memory by threads
 //   D    float[128]                      512 B    gamma_end
 //
 //   Rn   [token j (64)][value v (128)]   32 KiB   R = U - Y S_0   forward scan -> VJP kernel (K-major)
@@ -30,8 +28,9 @@
 // Buffers (caller-provided, struct of arrays, each array n_ch entries long):
 //   workspace  D, a 256-byte status block, and for a training call what backward consumes:
 //              Rn, Q, Kn, Yt, At, Tt
-//   scratch    dead when the call returns: forward U (and Q, Kn, Yt, At for an inference call);
-//              backward dZ
+//   scratch    dead when the call returns: the forward tiles of an inference call (Q, Kn, Yt, At, Tt in
+//              144 KiB per unit; a training call has them in its workspace and leaves its forward
+//              scratch alone); backward dZ
 #pragma once
 
 #include <cuda.h>
@@ -45,11 +44,13 @@ namespace gdn2 {
 
 constexpr int kChunk = GDN2_CHUNK;  // 64
 
-constexpr int64_t kTileQ = 32768, kTileKn = 32768, kTileYt = 32768, kTileU = 32768;
+constexpr int64_t kTileQ = 32768, kTileKn = 32768, kTileYt = 32768;
 constexpr int64_t kTileAt = 16384, kTileTt = 16384, kBlobD = 512;
 constexpr int64_t kBlobRn = 32768, kBlobDZ = 8 * 4608;
 constexpr int64_t kStatusBytes = 256;
-constexpr int64_t kFwdTilesBytes = kTileQ + kTileKn + kTileYt + kTileAt;  // the tiles both scans read
+// forward scratch per unit, a size callers know: 144 KiB for an inference call (its tiles take 128 of
+// them), 32 KiB for a training call
+constexpr int64_t kFwdScratchInference = 147456, kFwdScratchTraining = 32768;
 
 // workspace: what a training forward leaves for backward (inference: D and the status block only)
 struct WsLayout {
@@ -70,34 +71,34 @@ struct WsLayout {
 // scratch of one call
 struct ScratchLayout {
   int64_t n_ch;
-  __host__ __device__ int64_t off_u() const { return 0; }
   // inference calls only (a training call keeps these in its workspace)
-  __host__ __device__ int64_t off_q() const { return n_ch * kTileU; }
+  __host__ __device__ int64_t off_q() const { return 0; }
   __host__ __device__ int64_t off_kn() const { return off_q() + n_ch * kTileQ; }
   __host__ __device__ int64_t off_yt() const { return off_kn() + n_ch * kTileKn; }
   __host__ __device__ int64_t off_at() const { return off_yt() + n_ch * kTileYt; }
+  __host__ __device__ int64_t off_tt() const { return off_at() + n_ch * kTileAt; }
   __host__ __device__ int64_t total_forward(bool training) const {
-    return training ? n_ch * kTileU : n_ch * (kTileU + kFwdTilesBytes);
+    return n_ch * (training ? kFwdScratchTraining : kFwdScratchInference);
   }
   __host__ __device__ int64_t off_dz() const { return 0; }
   __host__ __device__ int64_t total_backward() const { return n_ch * kBlobDZ; }
 };
+static_assert(kTileQ + kTileKn + kTileYt + kTileAt + kTileTt <= kFwdScratchInference, "tiles exceed the scratch");
 
 // where the forward tile arrays of a call live
 struct ForwardTiles {
-  uint8_t *q, *kn, *yt, *at, *tt, *u;
+  uint8_t *q, *kn, *yt, *at, *tt;
 };
 inline ForwardTiles forward_tiles(uint8_t* workspace, uint8_t* scratch, int64_t n_ch, bool training) {
   const WsLayout ws{n_ch, training};
   const ScratchLayout sc{n_ch};
   ForwardTiles t;
-  t.u = scratch + sc.off_u();
   if (training) {
     t.q = workspace + ws.off_q(); t.kn = workspace + ws.off_kn(); t.yt = workspace + ws.off_yt();
     t.at = workspace + ws.off_at(); t.tt = workspace + ws.off_tt();
   } else {
     t.q = scratch + sc.off_q(); t.kn = scratch + sc.off_kn(); t.yt = scratch + sc.off_yt();
-    t.at = scratch + sc.off_at(); t.tt = nullptr;
+    t.at = scratch + sc.off_at(); t.tt = scratch + sc.off_tt();
   }
   return t;
 }
@@ -108,20 +109,71 @@ enum : int { kStatusOk = 0, kStatusBarrierTimeout = 1 };
 __device__ __forceinline__ float poison_nan() { return __int_as_float(0x7fc00000); }
 
 // A wait that gives up: after `limit` failed polls the thread records kStatusBarrierTimeout in the
-// status word and every later wait of the thread returns immediately.  The kernel then runs to its
-// end (shared resources such as TMEM are always released) and writes NaN instead of results, so the
-// failure shows in the outputs themselves and not only in the status word.
+// status word (and in the CTA's flag when it has one, for the roles of a warp-specialised kernel) and
+// every later wait of the thread returns immediately.  The kernel then runs to its end (shared
+// resources such as TMEM are always released) and writes NaN instead of results, so the failure shows
+// in the outputs themselves and not only in the status word.
 struct BoundedWaiter {
   bool dead = false;
   int* status;
   uint32_t limit;
-  __device__ explicit BoundedWaiter(int* s, uint32_t max_polls = (1u << 20)) : status(s), limit(max_polls) {}
+  volatile int* cta_flag;
+  __device__ explicit BoundedWaiter(int* s, uint32_t max_polls = (1u << 20), volatile int* flag = nullptr)
+      : status(s), limit(max_polls), cta_flag(flag) {}
   __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
     if (dead) return;
     if (!tc::mbar_wait(bar, parity, limit)) {
       dead = true;
+      if (cta_flag != nullptr) *cta_flag = 1;
       if (status != nullptr) atomicExch(status, kStatusBarrierTimeout);
     }
+  }
+};
+
+// ---- which tokens a chunk consists of -------------------------------------------------------------
+// A sequence is a run of token rows of the [rows][H][128] tensors (rows = batch * time, or the packed
+// length) cut into 64-token chunks; the last one may be partial.  Chunks are numbered through all
+// sequences, `chunk0` is a sequence's first one; unit = chunk * H + h.  The state checkpoints have one
+// slot more than chunks per sequence: slot of chunk c = (chunk0 + order + c) * H + h.
+struct SeqInfo {
+  int64_t row0;   // first token row
+  int len;        // tokens
+  int chunk0;     // number of its first chunk
+  int n_chunks;
+  int slot0;      // chunk0 + position of the sequence in the list
+  int sid;        // row of its state in the [sequences][H][128][128] state tensors
+};
+// A batch of equally long sequences: everything follows from the sizes.
+struct UniformSeqs {
+  int64_t stride;  // token rows from one sequence to the next
+  int len, n_chunks, n;
+  __host__ __device__ int count() const { return n; }
+  __host__ __device__ int total_chunks() const { return n * n_chunks; }
+  __device__ __forceinline__ SeqInfo at(int s) const {
+    return SeqInfo{s * stride, len, s * n_chunks, n_chunks, s * (n_chunks + 1), s};
+  }
+  __device__ __forceinline__ int find(int chunk) const { return int(uint32_t(chunk) / uint32_t(n_chunks)); }
+};
+// Packed sequences of several lengths, a table in kernel-parameter space (no copy to the device).  The
+// host lists the longest first: the scans walk a sequence serially and the long ones must not start last.
+constexpr int kMaxPacked = 256;  // sequences per launch (4 KiB of parameters); longer lists take several
+struct PackedSeqs {
+  struct Entry { int row0, len, chunk0, sid; };
+  int n, chunks;
+  Entry e[kMaxPacked];
+  __host__ __device__ int count() const { return n; }
+  __host__ __device__ int total_chunks() const { return chunks; }
+  __device__ __forceinline__ SeqInfo at(int s) const {
+    const Entry x = e[s];
+    return SeqInfo{x.row0, x.len, x.chunk0, (x.len + kChunk - 1) / kChunk, x.chunk0 + s, x.sid};
+  }
+  __device__ __forceinline__ int find(int chunk) const {  // last entry with chunk0 <= chunk
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (e[mid].chunk0 <= chunk) lo = mid; else hi = mid - 1;
+    }
+    return lo;
   }
 };
 
@@ -253,42 +305,36 @@ inline bool encode_cached(CUtensorMap* tm, int rank, CUtensorMapDataType type, c
   return true;
 }
 
-// A contiguous [B, T, H, 128] sequence tensor seen as (channel, head, token, batch): a box
-// (128, 1, 64, 1) is one head's 64-token chunk, landing in shared memory as dense [64][128] rows
-// (`box_rows` tokens instead of 64 when given).  Tokens are a dimension of their own so that the last,
-// partial chunk of a ragged sequence reads zeros beyond token T - 1 (and a store is clipped there).
-inline bool encode_sequence_map(CUtensorMap* tm, const void* base, int64_t batch, int64_t time, int64_t heads,
-                                int dtype, int box_rows = kChunk) {
+// A contiguous [rows, H, 128] sequence tensor (rows = batch * time, or the packed length) seen as
+// (channel, head, row): a box (128, 1, 64) is one head's 64-token chunk, landing in shared memory as dense
+// [64][128] rows (`box_rows` tokens instead of 64 when given).  A partial chunk reads on into the rows of
+// the next sequence (zeros past the end of the tensor): the kernels mask what is not theirs.
+inline bool encode_sequence_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t heads, int dtype,
+                                int box_rows = kChunk) {
   const cuuint64_t es = (dtype == GDN2_FP32) ? 4 : 2;
   const CUtensorMapDataType type = (dtype == GDN2_FP32)   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : (dtype == GDN2_BF16) ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                           : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  const cuuint64_t dims[4] = {cuuint64_t(kDim), cuuint64_t(heads), cuuint64_t(time), cuuint64_t(batch)};
-  const cuuint64_t strides[3] = {cuuint64_t(kDim) * es, cuuint64_t(heads) * kDim * es,
-                                 cuuint64_t(time) * heads * kDim * es};  // bytes, dimensions 1..3
+  const cuuint64_t dims[4] = {cuuint64_t(kDim), cuuint64_t(heads), cuuint64_t(rows), 1};
+  const cuuint64_t strides[3] = {cuuint64_t(kDim) * es, cuuint64_t(heads) * kDim * es, 0};  // bytes, dimensions 1..2
   const cuuint32_t box[4] = {cuuint32_t(kDim), 1, cuuint32_t(box_rows), 1};
-  return encode_cached(tm, 4, type, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+  return encode_cached(tm, 3, type, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-// An array of n_ch row-major fp32 tiles [rows][cols] seen as (col, row, unit): a box (32, rows, 1) is a
-// slab of 32 columns of one tile, `rows` lines of 128 bytes in shared memory.  mn_major chooses the
+// An array of n_ch row-major fp32 tiles [rows][cols] seen as (column within a slab, row, slab of 32
+// columns, unit).  A slab lands in shared memory as `rows` lines of 128 bytes; mn_major chooses the
 // swizzle: 128-byte with 32-byte atoms (the tile is read as an MN-major operand, contraction over its
-// rows) or plain 128-byte (K-major operand, contraction over its columns).
-// (`box_rows` < rows: boxes of that many rows, for tiles whose zero quadrant is never moved.)
+// rows) or plain 128-byte (K-major operand, contraction over its columns).  A box takes `box_slabs` slabs
+// of `box_rows` rows (0: all of them): one copy instruction brings a whole tile.  Tiles whose zero
+// quadrant is never moved go in boxes of one slab and half the rows.
 inline bool encode_tile_map(CUtensorMap* tm, const uint8_t* base, int64_t n_ch, int rows, int cols, bool mn_major,
-                            int box_rows = 0) {
-  const cuuint64_t dims[4] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(n_ch), 1};
-  const cuuint64_t strides[3] = {cuuint64_t(cols) * 4, cuuint64_t(rows) * cols * 4, 0};
-  const cuuint32_t box[4] = {32, cuuint32_t(box_rows > 0 ? box_rows : rows), 1, 1};
-  return encode_cached(tm, 3, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box,
+                            int box_rows = 0, int box_slabs = 0) {
+  const cuuint64_t dims[4] = {32, cuuint64_t(rows), cuuint64_t(cols / 32), cuuint64_t(n_ch)};
+  const cuuint64_t strides[3] = {cuuint64_t(cols) * 4, 128, cuuint64_t(rows) * cols * 4};
+  const cuuint32_t box[4] = {32, cuuint32_t(box_rows > 0 ? box_rows : rows),
+                             cuuint32_t(box_slabs > 0 ? box_slabs : cols / 32), 1};
+  return encode_cached(tm, 4, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box,
                        mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B);
-}
-// The same array, whole tiles without swizzle (box (cols, rows, 1); cols <= 256): for tiles that threads read.
-inline bool encode_plain_tile_map(CUtensorMap* tm, const uint8_t* base, int64_t n_ch, int rows, int cols) {
-  const cuuint64_t dims[4] = {cuuint64_t(cols), cuuint64_t(rows), cuuint64_t(n_ch), 1};
-  const cuuint64_t strides[3] = {cuuint64_t(cols) * 4, cuuint64_t(rows) * cols * 4, 0};
-  const cuuint32_t box[4] = {cuuint32_t(cols), cuuint32_t(rows), 1, 1};
-  return encode_cached(tm, 3, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

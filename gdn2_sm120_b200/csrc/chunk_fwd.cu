@@ -56,36 +56,32 @@ struct PrepSmem {
   //           after the Gram products: fp32 scratch for L, T, A_qk and the block products
   alignas(128) uint8_t gram_a[16 * kRsN];               // 73728
   // region 2: tf32 Gram B operands K^I X[r = j < 16 (I + 1)][c = k]: 2 (I + 1) row groups each;
-  //           after the Gram products: E^T at +0 and Z^T at +kTileT, tiles X[r = channel][c = j]
+  //           after the Gram products: E^T, tile X[r = channel][c = j]
   alignas(128) uint8_t gram_b[20 * kRsN];               // 92160
-  alignas(128) uint8_t tmat[32768];    // T tile X[r = i][c = j], tf32, RS 2048 (rows 64..127: filler of the M = 128
-                                       // product, whose output rows nobody reads; v of the next unit is staged there)
-  alignas(128) uint8_t stage_w[16384]; // w of the next unit
+  alignas(128) uint8_t tmat[16384];    // T tile X[r = i][c = j], tf32, RS 2048
   float part[16][kDim];                // per 4-token group partial sums -> exclusive prefixes
   float gend[kDim];
   float nrm[16][2][4][2];              // fused prologue: per (warp, token group, token) sums of q^2, k^2 over 64 channels
   alignas(8) uint64_t bar[2];          // MMA commits
-  alignas(8) uint64_t bar_ld[2];       // raw inputs of the next unit: {g, k, q} and {beta, v, w}
+  alignas(8) uint64_t bar_ld[2];       // raw inputs of the next unit: {g, k, q} and {beta}
   uint32_t tmem_base;
 };
 // landing zones of the raw [64][128] input tiles of the next unit, in places that are dead by then:
 // g, k, q over the fp32 scratch in region 1 (free once T is written, just before the last MMAs);
-// beta behind E^T / Z^T in region 2, v in the filler rows of the T tile, w in its own buffer (free as
-// soon as the Gram products are done, half a unit earlier)
+// beta behind E^T in region 2 (free as soon as the Gram products are done, half a unit earlier)
 constexpr int kStageK = 32768, kStageQ = 49152;                     // region 1: g at 0 (16 or 32 KiB)
-constexpr int kStageBeta = 2 * kTileT;                              // region 2, behind the two transposed tiles
-constexpr int kStageV = 16384;                                      // T tile, rows 64..127
+constexpr int kStageBeta = 2 * kTileT;                              // region 2, behind the transposed tile
 constexpr uint32_t kStageTile16 = kChunk * kDim * 2;                // a 16-bit input tile
 static_assert(kStageQ + kStageTile16 <= 16 * kRsN && kStageBeta + kStageTile16 <= 20 * kRsN, "staging exceeds its region");
 static_assert(kStageBeta % 128 == 0, "TMA destinations are 128-byte aligned");
 
 struct PrepParams {
-  const void *q, *k, *v, *g, *beta, *w;
   uint8_t* ws;   // workspace (D, status)
   ForwardTiles tiles;  // the tile arrays (in the workspace for a training call, else in the scratch)
-  int64_t T, H, n_chunks, n_ch;
+  int64_t n_ch;
+  int H;
   float scale;
-  int training;  // also write T^T, which only backward consumes
+  int training;  // layout of the workspace
   int prologue;  // kPrologueNorm | kPrologueGate: the inputs are raw projections / gate pre-activations
 };
 
@@ -94,18 +90,16 @@ __device__ __forceinline__ int gram_col(int I) { return (I == 0) ? 0 : (I == 1) 
 
 // kPro: the instantiation that can apply the layer prologue to raw inputs (p.prologue says which parts);
 // the plain instantiation carries none of that code.
-template <typename T, typename G, bool kPro = false>
+template <typename T, typename G, typename Seqs, bool kPro = false>
 __global__ void __launch_bounds__(kPrepThreads, 1)
-chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
+chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ CUtensorMap tm_g,
                   const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
-                  const __grid_constant__ CUtensorMap tm_beta, const __grid_constant__ CUtensorMap tm_v,
-                  const __grid_constant__ CUtensorMap tm_w) {
+                  const __grid_constant__ CUtensorMap tm_beta) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   const WsLayout ws{p.n_ch, p.training != 0};
   int* status = reinterpret_cast<int*>(p.ws + ws.off_status());
   BoundedWaiter waiter(status);
-  const bool training = p.training != 0;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -127,33 +121,38 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
   const int kc0 = 4 * c4;
   const int q4 = warp & 3, part = warp >> 2;  // TMEM lane quadrant of this warp, and its share of the columns
 
-  // unit -> TMA coordinates (channel 0, head, first token of the chunk, batch row).  The last chunk of a
-  // ragged sequence reaches past token T - 1: the loads fill those rows with zeros, which is the identity
-  // step of the recurrence (no decay, no key, no query, no value).
-  const int heads = int(p.H), chunks = int(p.n_chunks), n_ch = int(p.n_ch);
+  // unit -> TMA coordinates (channel 0, head, first token row of the chunk)
+  const int heads = p.H, n_ch = int(p.n_ch);
   constexpr uint32_t kStageTileG = kChunk * kDim * sizeof(G);
-  auto issue_gkq = [&](int ch_) {
-    const int h_ = ch_ % heads, bc = ch_ / heads, b_ = bc / chunks, t_ = (bc % chunks) * kChunk;
+  auto locate = [&](int ch_, int& h_, int& row_, int& valid_) {
+    const int chunk = int(uint32_t(ch_) / uint32_t(heads));
+    h_ = ch_ - chunk * heads;
+    const SeqInfo sq = seqs.at(seqs.find(chunk));
+    const int t_ = (chunk - sq.chunk0) * kChunk;
+    row_ = int(sq.row0) + t_;
+    valid_ = min(kChunk, sq.len - t_);
+  };
+  auto issue_gkq = [&](int h_, int row_) {
     mbar_arrive_expect_tx(&sm.bar_ld[0], kStageTileG + 2 * kStageTile16);
-    tma_load_4d(sm.gram_a, &tm_g, 0, h_, t_, b_, &sm.bar_ld[0]);
-    tma_load_4d(sm.gram_a + kStageK, &tm_k, 0, h_, t_, b_, &sm.bar_ld[0]);
-    tma_load_4d(sm.gram_a + kStageQ, &tm_q, 0, h_, t_, b_, &sm.bar_ld[0]);
+    tma_load_3d(sm.gram_a, &tm_g, 0, h_, row_, &sm.bar_ld[0]);
+    tma_load_3d(sm.gram_a + kStageK, &tm_k, 0, h_, row_, &sm.bar_ld[0]);
+    tma_load_3d(sm.gram_a + kStageQ, &tm_q, 0, h_, row_, &sm.bar_ld[0]);
   };
-  auto issue_bvw = [&](int ch_) {
-    const int h_ = ch_ % heads, bc = ch_ / heads, b_ = bc / chunks, t_ = (bc % chunks) * kChunk;
-    mbar_arrive_expect_tx(&sm.bar_ld[1], 3 * kStageTile16);
-    tma_load_4d(sm.gram_b + kStageBeta, &tm_beta, 0, h_, t_, b_, &sm.bar_ld[1]);
-    tma_load_4d(sm.tmat + kStageV, &tm_v, 0, h_, t_, b_, &sm.bar_ld[1]);
-    tma_load_4d(sm.stage_w, &tm_w, 0, h_, t_, b_, &sm.bar_ld[1]);
+  auto issue_beta = [&](int h_, int row_) {
+    mbar_arrive_expect_tx(&sm.bar_ld[1], kStageTile16);
+    tma_load_3d(sm.gram_b + kStageBeta, &tm_beta, 0, h_, row_, &sm.bar_ld[1]);
   };
+  int h_next = 0, row_next = 0, valid_next = kChunk;
+  if (int(blockIdx.x) < n_ch) locate(int(blockIdx.x), h_next, row_next, valid_next);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (tid == 0 && int(blockIdx.x) < n_ch) {
-    issue_gkq(int(blockIdx.x));
-    issue_bvw(int(blockIdx.x));
+    issue_gkq(h_next, row_next);
+    issue_beta(h_next, row_next);
   }
   const uint32_t tb = sm.tmem_base;
+  const uint32_t leader = elect_leader();
   // this thread's 8- or 16-byte piece of row 4 tg + e of a staged [64][128] tile
   auto staged = [&](const uint8_t* tile, int e, int elem_bytes) {
     return tile + ((4 * tg + e) * kDim + kc0) * elem_bytes;
@@ -162,9 +161,11 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
   uint32_t par = 0;
   for (int ch = int(blockIdx.x); ch < n_ch; ch += int(gridDim.x), par ^= 1u) {
   const int ch_next = ch + int(gridDim.x);
-  // tokens of this chunk that exist (64 except in the last chunk of a ragged sequence); only the fused
-  // prologue needs to know: its activations do not map the zero fill to the identity step
-  const int n_valid = kPro ? min(kChunk, int(p.T) - ((ch / heads) % chunks) * kChunk) : kChunk;
+  // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
+  // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
+  const int n_valid = valid_next;
+  const bool partial = n_valid < kChunk;
+  if (ch_next < n_ch) locate(ch_next, h_next, row_next, valid_next);
   // ---- the raw inputs were brought in while the previous unit was finishing; the log-decay is
   // consumed first: the prefix sums below need it alone ------------------------------------------------
   float Gc[4][4], kk[4][4], qq[4][4], bb[4][4];
@@ -189,7 +190,8 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
       unpack4<G>(rg[e], gv);
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        if (pro_gate) gv[f] = (4 * tg + e < n_valid) ? prologue_log_decay(gv[f]) : 0.f;
+        if (pro_gate) gv[f] = prologue_log_decay(gv[f]);
+        if (partial && 4 * tg + e >= n_valid) gv[f] = 0.f;
         Gc[e][f] = (e ? Gc[e - 1][f] : 0.f) + gv[f];
       }
     }
@@ -218,8 +220,6 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
       }
     }
     waiter.wait(&sm.bar_ld[1], par);
-    // v and w stay where they landed until Z is built, after the Gram products: nothing overwrites their
-    // landing zones before the next unit's copies, which are issued after that
     RawT rb[4];
 #pragma unroll
     for (int e = 0; e < 4; ++e) rb[e] = *reinterpret_cast<const RawT*>(staged(sm.gram_b + kStageBeta, e, 2));
@@ -239,7 +239,11 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
       }
       if (pro_gate) {
 #pragma unroll
-        for (int f = 0; f < 4; ++f) bb[e][f] = (4 * tg + e < n_valid) ? prologue_sigmoid(bb[e][f]) : 0.f;
+        for (int f = 0; f < 4; ++f) bb[e][f] = prologue_sigmoid(bb[e][f]);
+      }
+      if (partial && 4 * tg + e >= n_valid) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) kk[e][f] = qq[e][f] = bb[e][f] = 0.f;
       }
     }
   }
@@ -327,7 +331,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
   __syncthreads();
 
   // ---- Gram products on the tensor cores: P_I = [E_a ; Q_a] (K^I)^T -----------------------------
-  if (tid == 0) {
+  if (warp == 0) {
     tc_fence_after();
     // the four anchored copies K^0 .. K^3 are stacked (16 + 32 + 48 + 64 = 160 rows) and their products
     // sit side by side in TMEM, so one N = 160 instruction per k-step reads the A tile once for all four
@@ -336,41 +340,23 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
       mma_tf32_ss(tb, smem_desc(a0 + ks * 2 * kCsN, kCsN, kRsN), smem_desc(b0 + ks * 2 * kCsN, kCsN, kRsN), id,
-                  ks > 0 ? 1u : 0u);
+                  ks > 0 ? 1u : 0u, leader);
     }
-    mma_commit(&sm.bar[0]);
+    mma_commit(&sm.bar[0], leader);
   }
   waiter.wait(&sm.bar[0], par);
   tc_fence_after();
-  // the Gram operands are dead: region 1 becomes fp32 scratch, region 2 receives E^T and Z^T
+  // the Gram operands are dead: region 1 becomes fp32 scratch, region 2 receives E^T
   float* Ln = reinterpret_cast<float*>(sm.gram_a);           // [64][kLd]   L
   float* Tn = Ln + 64 * kLd;                                  // [64][kLd]   T
   float* Tc = Tn + 64 * kLd;                                  // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
   float* Wt = Tc + 64 * kLd;                                  // [3][16][kLdW] block products, transposed
   static_assert((3 * 64 * kLd + 3 * 16 * kLdW) * 4 <= 16 * kRsN, "fp32 scratch exceeds the Gram A region");
   uint8_t* et_tile = sm.gram_b;                               // E^T  X[r = k][c = j], tf32, RS kRsT
-  uint8_t* zt_tile = sm.gram_b + kTileT;                      // Z^T  X[r = v][c = j], tf32, RS kRsT
-  {
-    // Z = w * v from the staged inputs (kept out of registers until now)
-    float zz[4][4];
-    const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float vv[4], ww[4];
-      unpack4<T>(*reinterpret_cast<const typename Raw4<T>::type*>(staged(sm.tmat + kStageV, e, 2)), vv);
-      unpack4<T>(*reinterpret_cast<const typename Raw4<T>::type*>(staged(sm.stage_w, e, 2)), ww);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        if (pro_gate) ww[f] = (4 * tg + e < n_valid) ? prologue_sigmoid(ww[f]) : 0.f;
-        zz[e][f] = to_tf32_operand(vv[f] * ww[f]);
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const uint32_t off = blk_off<4>(kc0 + f, 4 * tg, kRsT, 128);
-      *reinterpret_cast<float4*>(et_tile + off) = make_float4(ebar[0][f], ebar[1][f], ebar[2][f], ebar[3][f]);
-      *reinterpret_cast<float4*>(zt_tile + off) = make_float4(zz[0][f], zz[1][f], zz[2][f], zz[3][f]);
-    }
+  for (int f = 0; f < 4; ++f) {
+    *reinterpret_cast<float4*>(et_tile + blk_off<4>(kc0 + f, 4 * tg, kRsT, 128)) =
+        make_float4(ebar[0][f], ebar[1][f], ebar[2][f], ebar[3][f]);
   }
   {
     // pull L (rows 0..63) into fp32 scratch and A_qk (rows 64..127) into the workspace;
@@ -415,9 +401,8 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
   }
   tc_fence_before();
   __syncthreads();
-  // every thread has read v and w of this unit, the Gram operands are dead: beta, v, w of the next unit
-  // start to arrive
-  if (tid == 0 && ch_next < n_ch) issue_bvw(ch_next);
+  // the Gram operands are dead: beta of the next unit starts to arrive
+  if (tid == 0 && ch_next < n_ch) issue_beta(h_next, row_next);
 
   // ---- T = (I + L)^-1, blocked: 16x16 diagonal blocks by substitution, the rest by block products.
   // T is kept in both orientations (Tn row-major, Tc column-major) and the block products W transposed,
@@ -532,7 +517,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
     Tc[cc * kLd + 48 + r] = -s1;
   }
   __syncthreads();
-  // T as tf32 tile X[r = i][c = j] in shared memory (MMA operand); T^T[j][i] goes to the workspace when training
+  // T as tf32 tile X[r = i][c = j] in shared memory (MMA operand), and T^T[j][i] for the scans
   {
     for (int e = tid; e < 64 * 16; e += kPrepThreads) {
       const int i = e & 63, c4t = e >> 6;  // consecutive threads -> consecutive rows -> contiguous 16-byte chunks
@@ -540,7 +525,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
       *reinterpret_cast<float4*>(sm.tmat + blk_off<4>(i, 4 * c4t, 2048, 128)) =
           make_float4(to_tf32_operand(tn.x), to_tf32_operand(tn.y), to_tf32_operand(tn.z), to_tf32_operand(tn.w));
     }
-    if (training) {
+    {
       float* tile_tt = reinterpret_cast<float*>(p.tiles.tt + int64_t(ch) * kTileTt);
       for (int e = tid; e < 64 * 16; e += kPrepThreads) {
         const int j = e >> 4, c4t = e & 15;  // consecutive threads -> consecutive 16-byte pieces of a row
@@ -555,55 +540,35 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
   tc_fence_before();
   __syncthreads();
 
-  // ---- Y = T E (rows 0..63 of an M = 128 product) and U^T = Z^T T^T ----------------------------------
-  if (tid == 0) {
+  // ---- Y^T = E^T T^T ------------------------------------------------------------------------------------
+  if (warp == 0) {
     tc_fence_after();
     // region 1 (fp32 scratch) is dead: g, k, q of the next unit land there under the MMAs and the epilogue
-    if (ch_next < n_ch) issue_gkq(ch_next);
-    const uint32_t t0a = smem_u32(sm.tmat), e0 = smem_u32(et_tile), z0 = smem_u32(zt_tile);
-    const uint32_t id_y = idesc(128, 128, kFmtTF32, kMajorK, kMajorK);
-    const uint32_t id_u = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
+    if (tid == 0 && ch_next < n_ch) issue_gkq(h_next, row_next);
+    const uint32_t t0a = smem_u32(sm.tmat), e0 = smem_u32(et_tile);
+    const uint32_t id_y = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      mma_tf32_ss(tb + 0, smem_desc(t0a + ks * 256, 128, 2048), smem_desc(e0 + ks * 256, 128, kRsT), id_y,
-                  ks > 0 ? 1u : 0u);
+      mma_tf32_ss(tb, smem_desc(e0 + ks * 256, 128, kRsT), smem_desc(t0a + ks * 256, 128, 2048), id_y,
+                  ks > 0 ? 1u : 0u, leader);
     }
-#pragma unroll
-    for (int ks = 0; ks < 8; ++ks) {
-      mma_tf32_ss(tb + 128, smem_desc(z0 + ks * 256, 128, kRsT), smem_desc(t0a + ks * 256, 128, 2048), id_u,
-                  ks > 0 ? 1u : 0u);
-    }
-    mma_commit(&sm.bar[1]);
+    mma_commit(&sm.bar[1], leader);
   }
   waiter.wait(&sm.bar[1], par);
   tc_fence_after();
   {
-    // Both accumulators leave transposed: a register holds one column, the 32 lanes of a warp hold 32
-    // consecutive rows of it, which are 128 consecutive bytes of the row-major tile.
-    // Y (lanes 0..63 = tokens i): Yt[k][i]; the four warps of quadrants 0 and 1 take 32 key columns each
-    if (q4 < 2) {
-      const int i = 32 * q4 + lane;
-      float* tile_yt = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + i;
+    // lanes = key channels k, columns = tokens i: each warp takes 16 tokens of its quadrant, a lane 64
+    // consecutive bytes of row k of Yt[k][i]
+    const int kr = 32 * q4 + lane, c0 = 16 * part;
+    float* row_yt = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + c0;
+    uint32_t r[16];
+    tmem_ld16(tmem_addr(tb, 32 * q4, c0), r);
+    tmem_wait_ld();
+    float y[16];
 #pragma unroll
-      for (int c0 = 32 * part; c0 < 32 * part + 32; c0 += 16) {
-        uint32_t r[16];
-        tmem_ld16(tmem_addr(tb, 32 * q4, c0), r);
-        tmem_wait_ld();
-#pragma unroll
-        for (int j = 0; j < 16; ++j) tile_yt[(c0 + j) * kChunk] = to_tf32_operand(__uint_as_float(r[j]));
-      }
-    }
-    // U^T (lanes = values v; kept in full fp32): U[j][v]; each warp of a quadrant takes 16 tokens
-    {
-      const int row = 32 * q4 + lane;
-      const int c0 = 16 * part;
-      float* tile_u = reinterpret_cast<float*>(p.tiles.u + int64_t(ch) * kTileU) + row;
-      uint32_t r[16];
-      tmem_ld16(tmem_addr(tb, 32 * q4, 128 + c0), r);
-      tmem_wait_ld();
-#pragma unroll
-      for (int j = 0; j < 16; ++j) tile_u[(c0 + j) * kDim] = __uint_as_float(r[j]);
-    }
+    for (int j = 0; j < 16; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
+    store_global_32b(row_yt, make_float4(y[0], y[1], y[2], y[3]), make_float4(y[4], y[5], y[6], y[7]));
+    store_global_32b(row_yt + 8, make_float4(y[8], y[9], y[10], y[11]), make_float4(y[12], y[13], y[14], y[15]));
   }
   }  // units of this CTA
   tc_fence_before();
@@ -614,255 +579,461 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ CUtensorMap tm_g,
 // ---------------------------------------------------------------------------------------------
 // scan kernel
 // ---------------------------------------------------------------------------------------------
-constexpr int kScanThreads = 512;
+// Warp-specialised.  What bounds a scan of few heads is the latency of one chunk, which walks the chain
+// S -> R -> S; in phases that all warps go through together a chunk took 3.8-5 us (every phase waited for
+// the tensor cores and the tensor cores for every phase).  Here the MMAs of a chunk are issued back to
+// back by one warp and everything else runs beside them:
+//   warp 0       tiled TMA loads, each buffer refilled as soon as its MMA has read it (one lane)
+//   warp 1       MMAs, per chunk:  R^T -= S^T Y^T | O^T = S^T Qg^T | S'^T += R^T Kt | O^T += R^T Aqk^T |
+//                R'^T = Z'^T T^T of the next chunk.  MMAs of one shape on one accumulator run in order; every
+//                other dependence (R -> S', S' -> R') is waited for, with independent MMAs in the queue meanwhile
+//   warps 2..9   decay: S' <- S diag(d) into the other of two state buffers while R is formed (the output
+//                still reads S); training: the chunk-start state, staged and sent by bulk stores
+//   warps 10..17 Z = w v of the next chunk into tensor memory; training: R out
+//   warps 18..21 O out (staged, one TMA store)
+//   warp 22      loads of v and w, whose buffer frees at another time than the others
+// A passed mbarrier wait costs ~150 clocks, so what an MMA group needs arrives on one barrier: the bytes of
+// its tiles, the threads that wrote its other operand and those that freed its accumulator.
+// Tensor memory (columns): S 2 x 128, R 2 x 64, O 64, Z 64 = all 512.
+constexpr int kScanThreads = 736;
+constexpr int kScanDecay0 = 2, kScanZ0 = 10, kScanOut0 = 18, kScanVw = 22;  // first warps of the groups
 
 struct ScanSmem {
-  // swizzled operand tiles, slabs of 32 columns (tc05.cuh): Yt and At and Kn are read MN-major, Q K-major
+  // swizzled operand tiles, slabs of 32 columns (tc05.cuh): Q is read K-major, the others MN-major
   alignas(1024) uint8_t yt[32768];   // Yt[k][i]: 2 slabs of 128 lines
   alignas(1024) uint8_t q[32768];    // Q[i][k]:  4 slabs of 64 lines
   alignas(1024) uint8_t kn[32768];   // Kn[j][k]: 4 slabs of 64 lines
   alignas(1024) uint8_t at[16384];   // At[j][i]: 2 slabs of 64 lines
-  alignas(1024) float u[kChunk * kDim];  // U[j][v], plain rows: threads copy it into tensor memory
-  alignas(128) float ck[kDim * kDim];    // training: the chunk-start state [k][v] on its way out (one bulk
-                                         // store per chunk: 64 KiB of per-thread stores would hold up the chain)
-  alignas(16) float d[kDim];
-  alignas(8) uint64_t bar_yqa, bar_ut, bar_kt, bar_mma1, bar_mma2;
+  alignas(1024) uint8_t tt[16384];   // Tt[j][i]: 2 slabs of 64 lines
+  alignas(128) uint8_t v[16384];     // raw v, w of the chunk, [64][128] 16-bit rows
+  alignas(128) uint8_t w[16384];
+  alignas(128) uint8_t o[16384];     // output rows [64][128] on their way out (one TMA store: 64-byte pieces
+                                     // stored by threads at the stride of a token row drain at 2 bytes per clock)
+  alignas(128) float ck[2][32 * kDim];  // training: 32 rows of the chunk-start state per half of the decay group
+  alignas(16) float d[2][kDim];
+  alignas(8) uint64_t full_vw, full_d[2];
+  uint64_t go_u;      // Tt, Z written (and the R before the last read):          1 load + 8 warps
+  uint64_t go_r;      // Yt, Q, the state of the last chunk, its O read:          2 loads + 1 commit + 4 warps
+  uint64_t go_s;      // Kn, At, decayed state, R:                                2 loads + 8 warps + 1 commit
+  uint64_t vw_read;   // v, w are in registers:                                   8 warps
+  uint64_t u_done, r_done, q_done, s_done, o_done, all_done;  // MMA commits
+  volatile int failed;
   uint32_t tmem_base;
 };
+static_assert(sizeof(ScanSmem) <= 232448, "forward scan exceeds the 227 KiB shared-memory limit");
 
 struct ScanParams {
-  const uint8_t* ws;   // workspace (D)
-  const float* s_in;   // [B,H,128,128] or null
-  void* out;           // [B,T,H,128]
-  float* s_out;        // [B,H,128,128] or null
-  float* bnd;          // [B, n_chunks+1, H,128,128] or null
+  const uint8_t* d;    // chunk-end decays, 512 bytes per unit
+  const float* s_in;   // [sequences,H,128,128] or null
+  void* out;           // [rows,H,128]
+  float* s_out;        // [sequences,H,128,128] or null
+  float* bnd;          // chunk-start states, one slot more than chunks per sequence, or null
+  float* rn;           // residual tiles (training) or null
   int* status;
-  int64_t T, H, n_chunks, n_ch;
-  uint8_t* ws_out;     // same workspace, writable (training: residual tiles)
-  int training;
+  int H;
+  int activate_w;      // w holds pre-activations
+};
+struct ScanMaps {
+  CUtensorMap yt, q, kn, at, tt, v, w, out;
 };
 
-template <typename T>
+template <typename T, typename Seqs>
 __global__ void __launch_bounds__(kScanThreads, 1)
-chunk_scan_kernel(const ScanParams p, const __grid_constant__ CUtensorMap tm_yt,
-                  const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_kn,
-                  const __grid_constant__ CUtensorMap tm_at, const __grid_constant__ CUtensorMap tm_u) {
+chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ ScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   ScanSmem& sm = *reinterpret_cast<ScanSmem*>(smem_raw);
-  const WsLayout ws{p.n_ch, p.training != 0};
-  BoundedWaiter waiter(p.status);
-  // a wait that ran out in the prep kernel left garbage tiles: results become NaN from the start
-  const bool upstream_failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
+  BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
-  // 16 warps: warp & 3 = TMEM lane quadrant (a warp reaches only the 32 lanes of its quadrant),
-  // warp >> 2 = its quarter of the columns of whatever accumulator is being moved
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int q4 = warp & 3, part = warp >> 2;
-  const int64_t bh = blockIdx.x;
-  const int64_t b = bh / p.H, h = bh % p.H;
-  constexpr uint32_t kColS = 0, kColR = 128, kColO = 192;
+  const int s = int(blockIdx.x) / p.H, h = int(blockIdx.x) - s * p.H;
+  const SeqInfo sq = seqs.at(s);
+  const int n_chunks = sq.n_chunks;
+  constexpr uint32_t kColS = 0, kColR = 256, kColO = 384, kColZ = 448;
+  auto ch_of = [&](int c) { return int64_t(sq.chunk0 + c) * p.H + h; };
 
-  if (warp == 0) {
-    tmem_alloc(&sm.tmem_base, 256);
+  if (warp == 1) {
+    tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(&sm.bar_yqa, 1);
-    mbar_init(&sm.bar_ut, 1);
-    mbar_init(&sm.bar_kt, 1);
-    mbar_init(&sm.bar_mma1, 1);
-    mbar_init(&sm.bar_mma2, 1);
+    mbar_init(&sm.full_vw, 1);
+    mbar_init(&sm.full_d[0], 1);
+    mbar_init(&sm.full_d[1], 1);
+    mbar_init(&sm.go_u, 1 + 8);
+    mbar_init(&sm.go_r, 2 + 1 + 4);
+    mbar_init(&sm.go_s, 2 + 8 + 1);
+    mbar_init(&sm.vw_read, 8);
+    mbar_init(&sm.u_done, 1); mbar_init(&sm.r_done, 1); mbar_init(&sm.q_done, 1);
+    mbar_init(&sm.s_done, 1); mbar_init(&sm.o_done, 1); mbar_init(&sm.all_done, 1);
+    mbar_arrive(&sm.go_r);  // no earlier chunk holds up the first one
+    // a wait that ran out in the prep kernel left garbage tiles: results become NaN from the start
+    sm.failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
     fence_mbar_init();
   }
+  // lines 32..63 of the first slab of At and Tt (j >= 32, i < 32) are never loaded: zero, once
+  for (int e = tid; e < 4096 / 16; e += kScanThreads) {
+    reinterpret_cast<float4*>(sm.at + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+    reinterpret_cast<float4*>(sm.tt + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  fence_async_smem();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tb = sm.tmem_base;
-  const uint32_t lane_base = 32u * q4;
-  const int vrow = 32 * q4 + lane;   // value row of the transposed state = TMEM lane
-  const int k0 = 32 * part;          // this thread's quarter of the 128 key columns
-  const int i0 = 16 * part;          // ... and of the 64 token columns
-
-  auto ch_of = [&](int64_t c) { return (b * p.n_chunks + c) * p.H + h; };
-  auto load_yqa = [&](int64_t c) {
-    const int ch = int(ch_of(c));
-    mbar_arrive_expect_tx(&sm.bar_yqa, uint32_t(kTileYt + kTileQ + kTileAt - 4096));
-#pragma unroll
-    for (int s = 0; s < 2; ++s) tma_load_3d(sm.yt + s * 16384, &tm_yt, 32 * s, 0, ch, &sm.bar_yqa);
-#pragma unroll
-    for (int s = 0; s < 4; ++s) tma_load_3d(sm.q + s * 8192, &tm_q, 32 * s, 0, ch, &sm.bar_yqa);
-    // At is zero for j >= 32, i < 32: three 32-row boxes, the fourth quadrant of the tile stays zero
-    tma_load_3d(sm.at, &tm_at, 0, 0, ch, &sm.bar_yqa);
-    tma_load_3d(sm.at + 8192, &tm_at, 32, 0, ch, &sm.bar_yqa);
-    tma_load_3d(sm.at + 8192 + 4096, &tm_at, 32, 32, ch, &sm.bar_yqa);
-  };
-  auto load_ut = [&](int64_t c) {
-    mbar_arrive_expect_tx(&sm.bar_ut, uint32_t(kTileU));
-    tma_load_3d(sm.u, &tm_u, 0, 0, int(ch_of(c)), &sm.bar_ut);
-  };
-  auto load_kt = [&](int64_t c) {
-    const int64_t ch = ch_of(c);
-    mbar_arrive_expect_tx(&sm.bar_kt, uint32_t(kTileKn + kBlobD));
-#pragma unroll
-    for (int s = 0; s < 4; ++s) tma_load_3d(sm.kn + s * 8192, &tm_kn, 32 * s, 0, int(ch), &sm.bar_kt);
-    bulk_g2s(sm.d, p.ws + ws.off_d() + ch * kBlobD, uint32_t(kBlobD), &sm.bar_kt);
-  };
-
-  // lines 32..63 of the first slab of At (j >= 32, i < 32) are never loaded: zero, once
-  for (int e = tid; e < 4096 / 16; e += kScanThreads) {
-    reinterpret_cast<float4*>(sm.at + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  fence_async_smem();
-  if (tid == 0) {
-    load_ut(0);
-    load_yqa(0);
-    load_kt(0);
-  }
-
-  // ---- S^T <- S_0^T : thread (v, part) gathers 32 key rows of column v of the key-major state ------
-  {
-    const float* src = (p.s_in != nullptr) ? p.s_in + bh * int64_t(kDim) * kDim + vrow : nullptr;
-    uint32_t r[32];
-#pragma unroll
-    for (int j = 0; j < 32; ++j) r[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
-    tmem_st32(tmem_addr(tb, lane_base, kColS + k0), r);
-    tmem_wait_st();
-  }
-
-  for (int64_t c = 0; c < p.n_chunks; ++c) {
-    const uint32_t par = uint32_t(c & 1);
-    const int64_t t0 = c * kChunk;
-    if (c > 0) {
-      // the previous state update must have finished reading R^T and the Kt buffer
-      waiter.wait(&sm.bar_mma2, par ^ 1u);
-      tc_fence_after();
-      if (tid == 0) load_kt(c);
-    }
-    // ---- R^T <- U^T (16 token columns of row v of the U^T tile into TMEM) ---------------------------
-    waiter.wait(&sm.bar_ut, par);
-    {
-      uint32_t r[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(sm.u[(i0 + j) * kDim + vrow]);
-      tmem_st16(tmem_addr(tb, lane_base, kColR + i0), r);
-      tmem_wait_st();
-    }
-    waiter.wait(&sm.bar_yqa, par);
-    if (tid == 0) bulk_wait_read_all();  // the previous checkpoint has left its staging buffer
+  auto arrive = [&](uint64_t* bar) {  // one arrival per warp, after its tensor-memory accesses
     tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
+    __syncwarp();
+    if (lane == 0) mbar_arrive(bar);
+  };
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- loads
+    const uint32_t leader = elect_leader();
+    // Tt and At are zero for j >= 32, i < 32: three 32-row boxes, the fourth quadrant of the tile stays zero
+    auto load_tri = [&](uint8_t* dst, const CUtensorMap* map, int ch, uint64_t* bar) {
+      tma_load_4d(dst, map, 0, 0, 0, ch, bar, leader);
+      tma_load_4d(dst + 8192, map, 0, 0, 1, ch, bar, leader);
+      tma_load_4d(dst + 8192 + 4096, map, 0, 32, 1, ch, bar, leader);
+    };
+    auto load_t = [&](int c) {
+      mbar_arrive_expect_tx(&sm.go_u, uint32_t(kTileTt - 4096), leader);
+      load_tri(sm.tt, &tm.tt, int(ch_of(c)), &sm.go_u);
+    };
+    auto load_y = [&](int c) {
+      mbar_arrive_expect_tx(&sm.go_r, uint32_t(kTileYt), leader);
+      tma_load_4d(sm.yt, &tm.yt, 0, 0, 0, int(ch_of(c)), &sm.go_r, leader);
+    };
+    auto load_d = [&](int c) {
+      mbar_arrive_expect_tx(&sm.full_d[c & 1], uint32_t(kBlobD), leader);
+      bulk_g2s(sm.d[c & 1], p.d + ch_of(c) * kBlobD, uint32_t(kBlobD), &sm.full_d[c & 1], leader);
+    };
+    auto load_k = [&](int c) {
+      mbar_arrive_expect_tx(&sm.go_s, uint32_t(kTileKn), leader);
+      tma_load_4d(sm.kn, &tm.kn, 0, 0, 0, int(ch_of(c)), &sm.go_s, leader);
+    };
+    auto load_q = [&](int c) {
+      mbar_arrive_expect_tx(&sm.go_r, uint32_t(kTileQ), leader);
+      tma_load_4d(sm.q, &tm.q, 0, 0, 0, int(ch_of(c)), &sm.go_r, leader);
+    };
+    auto load_a = [&](int c) {
+      mbar_arrive_expect_tx(&sm.go_s, uint32_t(kTileAt - 4096), leader);
+      load_tri(sm.at, &tm.at, int(ch_of(c)), &sm.go_s);
+    };
+    load_t(0);
+    load_y(0);
+    load_d(0);
+    load_q(0);
+    load_k(0);
+    load_a(0);
+    if (n_chunks > 1) load_d(1);
+    for (int c = 1; c < n_chunks; ++c) {
+      const uint32_t par = uint32_t(c - 1) & 1u;
+      waiter.wait(&sm.u_done, par);
+      load_t(c);
+      waiter.wait(&sm.r_done, par);
+      load_y(c);
+      waiter.wait(&sm.q_done, par);
+      load_q(c);
+      waiter.wait(&sm.s_done, par);
+      load_k(c);
+      if (c + 1 < n_chunks) load_d(c + 1);  // the decay of chunk c - 1 has run: its slot is free
+      waiter.wait(&sm.o_done, par);
+      load_a(c);
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMAs
+    // (the initial state must be in tensor memory: barrier 1, decay group and this warp)
+    asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+    tc_fence_after();
+    const uint32_t leader = elect_leader();
+    const uint32_t y0 = smem_u32(sm.yt), q0 = smem_u32(sm.q), a0 = smem_u32(sm.at);
+    const uint32_t kn0 = smem_u32(sm.kn), t0 = smem_u32(sm.tt);
+    const uint32_t id_neg_mn = idesc(128, 64, kFmtTF32, kMajorK, kMajorMN, 1, 0);
+    const uint32_t id_pos_mn = idesc(128, 64, kFmtTF32, kMajorK, kMajorMN);
+    const uint32_t id_pos_k = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
+    const uint32_t id_s = idesc(128, 128, kFmtTF32, kMajorK, kMajorMN);
+    // R^T = Z^T T^T    (A = Z columns, K = 64 tokens; B = Tt[j][i] read MN-major)
+    auto issue_u = [&](int c) {
+      const uint32_t r = tb + kColR + 64u * (uint32_t(c) & 1u);
+      waiter.wait(&sm.go_u, uint32_t(c) & 1u);
       tc_fence_after();
-      if (c + 1 < p.n_chunks) load_ut(c + 1);  // every thread has consumed the U^T tile
-      const uint32_t y0 = smem_u32(sm.yt), q0 = smem_u32(sm.q), a0 = smem_u32(sm.at);
-      const uint32_t id_neg_mn = idesc(128, 64, kFmtTF32, kMajorK, kMajorMN, 1, 0);
-      const uint32_t id_pos_k = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
-      const uint32_t id_pos_mn = idesc(128, 64, kFmtTF32, kMajorK, kMajorMN);
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        mma_tf32_ts(r, tb + kColZ + ks * 8, smem_desc_sw128_mn(t0, 8192, ks), id_pos_mn, ks > 0 ? 1u : 0u, leader);
+      }
+      mma_commit(&sm.u_done, leader);
+    };
+    issue_u(0);
+    for (int c = 0; c < n_chunks; ++c) {
+      const uint32_t par = uint32_t(c) & 1u;
+      const uint32_t s_old = tb + kColS + 128u * par, s_new = tb + kColS + 128u * (par ^ 1u);
+      const uint32_t r = tb + kColR + 64u * par;
+      waiter.wait(&sm.go_r, par);
+      tc_fence_after();
       // R^T -= S^T Y^T   (A = state columns, K = 128 keys; B = Yt[k][i] read MN-major)
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {
-        mma_tf32_ts(tb + kColR, tb + kColS + ks * 8, smem_desc_sw128_mn(y0, 16384, ks), id_neg_mn, 1u);
+        mma_tf32_ts(r, s_old + ks * 8, smem_desc_sw128_mn(y0, 16384, ks), id_neg_mn, 1u, leader);
       }
+      mma_commit(&sm.r_done, leader);
+      mma_commit(&sm.go_s, leader);
       // O^T = S^T Qg^T   (B = Q[i][k] read K-major)
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {
-        mma_tf32_ts(tb + kColO, tb + kColS + ks * 8, smem_desc_sw128_k(q0, 8192, ks), id_pos_k, ks > 0 ? 1u : 0u);
+        mma_tf32_ts(tb + kColO, s_old + ks * 8, smem_desc_sw128_k(q0, 8192, ks), id_pos_k, ks > 0 ? 1u : 0u, leader);
       }
-      // O^T += R^T Aqk^T  (A = residual columns, K = 64 tokens; B = At[j][i] read MN-major)
+      mma_commit(&sm.q_done, leader);
+      waiter.wait(&sm.go_s, par);
+      tc_fence_after();
+      // S'^T += R^T Kt   (K = 64 tokens; B = Kn[j][k] read MN-major)
 #pragma unroll
       for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ts(tb + kColO, tb + kColR + ks * 8, smem_desc_sw128_mn(a0, 8192, ks), id_pos_mn, 1u);
+        mma_tf32_ts(s_new, r + ks * 8, smem_desc_sw128_mn(kn0, 8192, ks), id_s, 1u, leader);
       }
-      mma_commit(&sm.bar_mma1);
+      mma_commit(&sm.s_done, leader);
+      if (c + 1 < n_chunks) mma_commit(&sm.go_r, leader);
+      // O^T += R^T Aqk^T (B = At[j][i] read MN-major)
+#pragma unroll
+      for (int ks = 0; ks < 8; ++ks) {
+        mma_tf32_ts(tb + kColO, r + ks * 8, smem_desc_sw128_mn(a0, 8192, ks), id_pos_mn, 1u, leader);
+      }
+      mma_commit(&sm.o_done, leader);
+      if (c + 1 < n_chunks) issue_u(c + 1);
     }
-    waiter.wait(&sm.bar_mma1, par);
-    tc_fence_after();
-    if (tid == 0 && c + 1 < p.n_chunks) load_yqa(c + 1);  // the three MMAs no longer read Y, Q, A
-
-    // ---- training: keep the residual R = U - Y S_0 for backward -------------------------------------
-    {
-      uint32_t rr[16], ro[16];
-      if (p.training) tmem_ld16(tmem_addr(tb, lane_base, kColR + i0), rr);
-      tmem_ld16(tmem_addr(tb, lane_base, kColO + i0), ro);
+    mma_commit(&sm.all_done, leader);
+  } else if (warp < kScanZ0) {
+    // ---------------------------------------------------------------- decay of the state
+    // thread = value row of the transposed state (TMEM lane) x one half of the 128 key columns
+    const int q4 = warp & 3, half = (warp - kScanDecay0) >> 2;
+    const int vrow = 32 * q4 + lane, k0 = 64 * half;
+    const uint32_t lane_base = 32u * q4;
+    const int64_t state = (int64_t(sq.sid) * p.H + h) * int64_t(kDim * kDim);
+    const bool sender = lane == 0 && ((warp - kScanDecay0) & 3) == 0;  // sends this half's staged rows
+    uint32_t lo[32], hi[32];
+    auto half_barrier = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory"); };
+    auto load_state = [&](uint32_t col) {
+      tmem_ld32(tmem_addr(tb, lane_base, col + k0), lo);
+      tmem_ld32(tmem_addr(tb, lane_base, col + k0 + 32), hi);
       tmem_wait_ld();
-      if (p.training) {
-        // row-major R[j][v]: the 32 lanes of a warp fill one 128-byte line per token
-        float* rn = reinterpret_cast<float*>(p.ws_out + ws.off_rn() + ch_of(c) * kBlobRn) + vrow;
-#pragma unroll
-        for (int j = 0; j < 16; ++j) rn[(i0 + j) * kDim] = to_tf32(__uint_as_float(rr[j]));
-      }
-      // ---- output rows of this chunk: o[t0 + i][v] ---------------------------------------------------
-      T* out = static_cast<T*>(p.out);
-      const bool failed = upstream_failed || waiter.dead;
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        if (t0 + i0 + j < p.T) {  // the last chunk of a ragged sequence has fewer than 64 tokens
-          out[((b * p.T + t0 + i0 + j) * p.H + h) * kDim + vrow] =
-              from_float<T>(failed ? poison_nan() : __uint_as_float(ro[j]));
-        }
-      }
-    }
-    // ---- checkpoint the chunk-start state, then decay the accumulator: S^T <- S^T diag(d) ----------
-    waiter.wait(&sm.bar_kt, par);
-    {
-      uint32_t r[32];
-      tmem_ld32(tmem_addr(tb, lane_base, kColS + k0), r);
-      tmem_wait_ld();
-      if (p.bnd != nullptr) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) sm.ck[(k0 + j) * kDim + vrow] = __uint_as_float(r[j]);
-        fence_async_smem();
-      }
-#pragma unroll
-      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * sm.d[k0 + j]);
-      tmem_st32(tmem_addr(tb, lane_base, kColS + k0), r);
+    };
+    auto store_state = [&](uint32_t col) {
+      tmem_st32(tmem_addr(tb, lane_base, col + k0), lo);
+      tmem_st32(tmem_addr(tb, lane_base, col + k0 + 32), hi);
       tmem_wait_st();
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (tid == 0) {
-      tc_fence_after();
-      if (p.bnd != nullptr) {
-        bulk_s2g(p.bnd + ((b * (p.n_chunks + 1) + c) * p.H + h) * int64_t(kDim) * kDim, sm.ck,
-                 uint32_t(kDim * kDim * sizeof(float)));
+    };
+    // 32 key rows of the chunk-start state, 16 KiB, through the staging buffer of this half
+    auto send_rows = [&](const uint32_t (&x)[32], int c, int kr) {
+      if (sender) bulk_wait_read_all();  // the previous rows have left the buffer
+      half_barrier();
+      float* dst = sm.ck[half] + vrow;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) dst[j * kDim] = __uint_as_float(x[j]);
+      fence_async_smem();
+      half_barrier();
+      if (sender) {
+        bulk_s2g(p.bnd + ((int64_t(sq.slot0 + c) * p.H + h) * kDim + kr) * kDim, sm.ck[half], 32u * kDim * 4u);
         bulk_commit();
       }
-      const uint32_t kn0 = smem_u32(sm.kn);
-      const uint32_t id_s = idesc(128, 128, kFmtTF32, kMajorK, kMajorMN);
-      // S^T += R^T Kt   (K = 64 tokens; B = Kn[j][k] read MN-major)
+    };
+    {
+      const float* src = (p.s_in != nullptr) ? p.s_in + state + vrow : nullptr;
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ts(tb + kColS, tb + kColR + ks * 8, smem_desc_sw128_mn(kn0, 8192, ks), id_s, 1u);
+      for (int j = 0; j < 32; ++j) {
+        lo[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
+        hi[j] = (src != nullptr) ? __float_as_uint(src[(k0 + 32 + j) * kDim]) : 0u;
       }
-      mma_commit(&sm.bar_mma2);
+      store_state(kColS);
+      tc_fence_before();
+      asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
     }
-  }
-
-  // ---- final state ---------------------------------------------------------------------------------
-  if (p.n_chunks > 0) {
-    waiter.wait(&sm.bar_mma2, uint32_t((p.n_chunks - 1) & 1));
-    tc_fence_after();
-  }
-  {
-    float* fin = (p.s_out != nullptr) ? p.s_out + bh * int64_t(kDim) * kDim + vrow : nullptr;
-    float* ck = (p.bnd != nullptr)
-                    ? p.bnd + ((b * (p.n_chunks + 1) + p.n_chunks) * p.H + h) * int64_t(kDim) * kDim + vrow
-                    : nullptr;
-    uint32_t r[32];
-    tmem_ld32(tmem_addr(tb, lane_base, kColS + k0), r);
-    tmem_wait_ld();
-    const bool failed = upstream_failed || waiter.dead;
+    for (int c = 0; c < n_chunks; ++c) {
+      const uint32_t par = uint32_t(c) & 1u;
+      if (c > 0) {
+        waiter.wait(&sm.s_done, par ^ 1u);
+        tc_fence_after();
+        load_state(kColS + 128u * par);
+      }
+      if (p.bnd != nullptr) send_rows(lo, c, k0);
+      waiter.wait(&sm.full_d[par], uint32_t(c >> 1) & 1u);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) {
-      const float x = failed ? poison_nan() : __uint_as_float(r[j]);
+      for (int j4 = 0; j4 < 8; ++j4) {
+        const float4 da = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 4 * j4]);
+        const float4 db = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 32 + 4 * j4]);
+        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * da.x);
+        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * da.y);
+        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * da.z);
+        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * da.w);
+        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * db.x);
+        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * db.y);
+        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * db.z);
+        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * db.w);
+      }
+      // (the other buffer: its readers, R and O of chunk c - 1, ran before the update that s_done stands for)
+      store_state(kColS + 128u * (par ^ 1u));
+      arrive(&sm.go_s);
+      if (p.bnd != nullptr) {
+        // the other rows, off the chain: the chunk-start state is still in its buffer, which this group alone
+        // overwrites, one chunk later.  They leave by plain stores: the copy engine has 200 KB of a chunk to
+        // move as it is (with these rows staged too, a chunk waited 2000 clocks for its buffer)
+        tmem_ld32(tmem_addr(tb, lane_base, kColS + 128u * par + k0 + 32), hi);
+        tmem_wait_ld();
+        float* ck = p.bnd + ((int64_t(sq.slot0 + c) * p.H + h) * kDim + k0 + 32) * kDim + vrow;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) ck[j * kDim] = __uint_as_float(hi[j]);
+      }
+    }
+    // ---- final state ---------------------------------------------------------------------------------
+    waiter.wait(&sm.s_done, uint32_t(n_chunks - 1) & 1u);
+    tc_fence_after();
+    load_state(kColS + 128u * (uint32_t(n_chunks) & 1u));
+    float* fin = (p.s_out != nullptr) ? p.s_out + state + vrow : nullptr;
+    float* ck = (p.bnd != nullptr) ? p.bnd + (int64_t(sq.slot0 + n_chunks) * p.H + h) * int64_t(kDim * kDim) + vrow
+                                   : nullptr;
+    const bool failed = sm.failed != 0;
+#pragma unroll
+    for (int j = 0; j < 64; ++j) {
+      const float x = failed ? poison_nan() : __uint_as_float(j < 32 ? lo[j & 31] : hi[j & 31]);
       if (fin != nullptr) fin[(k0 + j) * kDim] = x;
       if (ck != nullptr) ck[(k0 + j) * kDim] = x;
     }
+    if (sender) bulk_wait_all();  // the last staged rows are in global memory before the CTA retires
+  } else if (warp < kScanOut0) {
+    // ---------------------------------------------------------------- Z = w v
+    // thread = value row (TMEM lane) x one half of the 64 tokens
+    const int q4 = warp & 3, half = (warp - kScanZ0) >> 2;
+    const int vrow = 32 * q4 + lane, i0 = 32 * half;
+    const uint32_t lane_base = 32u * q4;
+    const T* vs = reinterpret_cast<const T*>(sm.v) + i0 * kDim + vrow;
+    const T* wsrc = reinterpret_cast<const T*>(sm.w) + i0 * kDim + vrow;
+    uint32_t x[32];
+    // R of chunk c for backward, row-major R[j][v]: the 32 lanes of a warp fill one 128-byte line per token
+    auto load_residual = [&](int c) {
+      tmem_ld32(tmem_addr(tb, lane_base, kColR + 64u * (uint32_t(c) & 1u) + i0), x);
+      tmem_wait_ld();
+    };
+    auto store_residual = [&](int c) {
+      float* rn = p.rn + ch_of(c) * (kBlobRn / 4) + i0 * kDim + vrow;
+#pragma unroll
+      for (int j = 0; j < 32; ++j) rn[j * kDim] = to_tf32(__uint_as_float(x[j]));
+    };
+    for (int c = 0; c < n_chunks; ++c) {
+      waiter.wait(&sm.full_vw, uint32_t(c) & 1u);
+      const int n_valid = sq.len - c * kChunk;
+      // 16 tokens at a time: all 32 with their activations in flight would not fit the registers
+#pragma unroll
+      for (int part = 0; part < 2; ++part) {
+        T vr[16];
+        float z[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+          z[j] = to_float(wsrc[(16 * part + j) * kDim]);
+          vr[j] = vs[(16 * part + j) * kDim];
+        }
+        if (part == 1) {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&sm.vw_read);
+        }
+        if (p.activate_w) {
+#pragma unroll
+          for (int j = 0; j < 16; j += 2) prologue_sigmoid2(z[j], z[j + 1]);
+        }
+        uint32_t zr[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) zr[j] = __float_as_uint(to_tf32_operand(to_float(vr[j]) * z[j]));
+        if (n_valid < kChunk) {  // rows past the end of the sequence are somebody else's
+#pragma unroll
+          for (int j = 0; j < 16; ++j) zr[j] = (i0 + 16 * part + j < n_valid) ? zr[j] : 0u;
+        }
+        if (part == 0 && c > 0) {
+          waiter.wait(&sm.u_done, uint32_t(c - 1) & 1u);  // and with it everything of chunk c - 2
+          tc_fence_after();
+        }
+        tmem_st16(tmem_addr(tb, lane_base, kColZ + i0 + 16 * part), zr);
+      }
+      tmem_wait_st();
+      if (p.rn != nullptr && c > 1) load_residual(c - 2);  // before its columns take the R of this chunk
+      arrive(&sm.go_u);
+      if (p.rn != nullptr && c > 1) store_residual(c - 2);
+    }
+    if (p.rn != nullptr) {
+      waiter.wait(&sm.all_done, 0);
+      tc_fence_after();
+      for (int c = max(0, n_chunks - 2); c < n_chunks; ++c) {
+        load_residual(c);
+        store_residual(c);
+      }
+    }
+  } else if (warp < kScanVw) {
+    // ---------------------------------------------------------------- O out
+    // thread = value row (TMEM lane)
+    const int q4 = warp & 3;
+    const int vrow = 32 * q4 + lane;
+    const uint32_t lane_base = 32u * q4;
+    const bool sender = tid == kScanOut0 * 32;
+    auto group_barrier = [&] { asm volatile("bar.sync 4, 128;" ::: "memory"); };
+    arrive(&sm.go_r);  // no earlier chunk holds up the first output
+    for (int c = 0; c < n_chunks; ++c) {
+      waiter.wait(&sm.o_done, uint32_t(c) & 1u);
+      tc_fence_after();
+      uint32_t a[32], b[32];
+      tmem_ld32(tmem_addr(tb, lane_base, kColO), a);
+      tmem_ld32(tmem_addr(tb, lane_base, kColO + 32), b);
+      tmem_wait_ld();
+      if (c + 1 < n_chunks) arrive(&sm.go_r);
+      const bool failed = sm.failed != 0;
+      if (sender) bulk_wait_read_all();  // the previous chunk's rows have left the buffer
+      group_barrier();
+      T* tile = reinterpret_cast<T*>(sm.o) + vrow;
+      if (failed) {
+#pragma unroll
+        for (int j = 0; j < 32; ++j) a[j] = b[j] = __float_as_uint(poison_nan());
+      }
+#pragma unroll
+      for (int j = 0; j < 32; j += 2) {
+        const typename Pair<T>::type x = Pair<T>::make(__uint_as_float(a[j]), __uint_as_float(a[j + 1]));
+        const typename Pair<T>::type y = Pair<T>::make(__uint_as_float(b[j]), __uint_as_float(b[j + 1]));
+        tile[j * kDim] = x.x;
+        tile[(j + 1) * kDim] = x.y;
+        tile[(j + 32) * kDim] = y.x;
+        tile[(j + 33) * kDim] = y.y;
+      }
+      fence_async_smem();
+      group_barrier();
+      const int row = int(sq.row0) + c * kChunk, n_valid = min(kChunk, sq.len - c * kChunk);
+      if (n_valid == kChunk) {
+        if (sender) {
+          tma_store_3d(&tm.out, 0, h, row, sm.o);
+          bulk_commit();
+        }
+      } else {  // the rows behind a partial chunk (the last one) belong to somebody else
+        for (int e = tid - kScanOut0 * 32; e < n_valid * 16; e += 128) {
+          *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + (int64_t(row + (e >> 4)) * p.H + h) * kDim + 8 * (e & 15)) =
+              *reinterpret_cast<const uint4*>(sm.o + e * 16);
+        }
+      }
+    }
+    if (sender) bulk_wait_all();  // the last rows are in global memory before the CTA retires
+  } else {
+    // ---------------------------------------------------------------- v and w
+    const uint32_t leader = elect_leader();
+    auto load_vw = [&](int c) {
+      const int row = int(sq.row0) + c * kChunk;
+      mbar_arrive_expect_tx(&sm.full_vw, 2u * 16384u, leader);
+      tma_load_3d(sm.v, &tm.v, 0, h, row, &sm.full_vw, leader);
+      tma_load_3d(sm.w, &tm.w, 0, h, row, &sm.full_vw, leader);
+    };
+    load_vw(0);
+    for (int c = 1; c < n_chunks; ++c) {
+      waiter.wait(&sm.vw_read, uint32_t(c - 1) & 1u);
+      load_vw(c);
+    }
   }
-  if (tid == 0) bulk_wait_all();  // the last staged checkpoint is in global memory before the CTA retires
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tb, 256);
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tb, 512);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -916,74 +1087,103 @@ int64_t chunk_status_offset(int64_t batch, int64_t full_tokens, int64_t heads) {
   return ws.off_status();
 }
 
+namespace {
+
+struct ForwardCall {
+  const void *q, *k, *v, *g, *beta, *w;
+  const float* s_in;
+  void* out;
+  float *s_out, *bnd;
+  uint8_t *workspace, *scratch;
+  int64_t rows, H;  // token rows of the sequence tensors, heads
+  int training, dtype, g_dtype;
+  float scale;
+  int prologue;
+};
+
+template <typename Seqs>
+int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) {
+  const int64_t n_ch = int64_t(seqs.total_chunks()) * a.H;
+  // units, token rows and the grids of the scans are 31-bit numbers
+  if (n_ch <= 0 || n_ch > int64_t(0x7fffffff) || a.rows > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
+  const WsLayout ws{n_ch, a.training != 0};
+  int* status = reinterpret_cast<int*>(a.workspace + ws.off_status());
+  cudaError_t err = cudaMemsetAsync(status, 0, kStatusBytes, stream);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+
+  const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
+  CUtensorMap tm_g, tm_k, tm_q, tm_beta;
+  ScanMaps tm;
+  // the sequence tensors, and the scan's operands: the prep kernel's tiles in the swizzle of their role
+  if (!encode_sequence_map(&tm_g, a.g, a.rows, a.H, a.g_dtype) ||
+      !encode_sequence_map(&tm_k, a.k, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm_q, a.q, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm_beta, a.beta, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm.v, a.v, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm.w, a.w, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm.out, a.out, a.rows, a.H, a.dtype) ||
+      !encode_tile_map(&tm.yt, tiles.yt, n_ch, kDim, kChunk, true) ||
+      !encode_tile_map(&tm.q, tiles.q, n_ch, kChunk, kDim, false) ||
+      !encode_tile_map(&tm.kn, tiles.kn, n_ch, kChunk, kDim, true) ||
+      !encode_tile_map(&tm.at, tiles.at, n_ch, kChunk, kChunk, true, 32, 1) ||
+      !encode_tile_map(&tm.tt, tiles.tt, n_ch, kChunk, kChunk, true, 32, 1)) {
+    return GDN2_ERR_LAUNCH;
+  }
+  int sm_count = 0;
+  if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
+
+  profile_mark(0, stream);
+  const unsigned prep_grid = unsigned(n_ch < int64_t(sm_count) ? n_ch : int64_t(sm_count));
+  const PrepParams pp{a.workspace, tiles, n_ch, int(a.H), a.scale, a.training, a.prologue};
+  GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
+    auto kernel = a.prologue != 0 ? chunk_prep_kernel<T, G, Seqs, true> : chunk_prep_kernel<T, G, Seqs, false>;
+    const int smem = int(sizeof(PrepSmem));
+    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+    kernel<<<prep_grid, kPrepThreads, smem, stream>>>(pp, seqs, tm_g, tm_k, tm_q, tm_beta);
+  });
+  int st = check_launch();
+  if (st != GDN2_OK) return st;
+  profile_mark(1, stream);
+
+  const ScanParams sp{a.workspace + ws.off_d(), a.s_in, a.out, a.s_out, a.bnd,
+                      a.training ? reinterpret_cast<float*>(a.workspace + ws.off_rn()) : nullptr,
+                      status, int(a.H), (a.prologue & kPrologueGate) != 0};
+  const int smem = int(sizeof(ScanSmem));
+  const unsigned grid = unsigned(seqs.count() * a.H);
+  auto kernel = a.dtype == GDN2_BF16 ? chunk_scan_kernel<__nv_bfloat16, Seqs> : chunk_scan_kernel<__half, Seqs>;
+  err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  kernel<<<grid, kScanThreads, smem, stream>>>(sp, seqs, tm);
+  st = check_launch();
+  profile_mark(2, stream);
+  return st;
+}
+
+}  // namespace
+
 int launch_chunk_forward(const void* q, const void* k, const void* v, const void* g, const void* beta,
                          const void* w, const float* s_in, void* out, float* s_out, float* bnd,
                          uint8_t* workspace, uint8_t* scratch, int64_t B, int64_t T, int64_t H,
                          int64_t full_tokens, int training, int dtype, int g_dtype, float scale,
                          int prologue, cudaStream_t stream) {
   const int64_t n_chunks = full_tokens / kChunk;
-  const int64_t n_ch = B * n_chunks * H;
-  if (n_ch <= 0 || n_ch > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  const WsLayout ws{n_ch, training != 0};
-  int* status = reinterpret_cast<int*>(workspace + ws.off_status());
-  cudaError_t err = cudaMemsetAsync(status, 0, kStatusBytes, stream);
-  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  if (B * T > int64_t(0x7fffffff) || B * n_chunks * H > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
+  const UniformSeqs seqs{T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
+  const ForwardCall a{q, k, v, g, beta, w, s_in, out, s_out, bnd, workspace, scratch, B * T, H,
+                      training, dtype, g_dtype, scale, prologue};
+  return launch_forward(seqs, a, stream);
+}
 
-  // the prep kernel addresses its inputs through tensor maps: 16-byte aligned bases
-  if (B * T > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  const void* seq[6] = {g, k, q, beta, v, w};
-  CUtensorMap tm[6];
-  for (int i = 0; i < 6; ++i) {
-    if ((reinterpret_cast<uintptr_t>(seq[i]) & 15u) != 0 ||
-        !encode_sequence_map(&tm[i], seq[i], B, T, H, i == 0 ? g_dtype : dtype)) {
-      return GDN2_ERR_LAUNCH;
-    }
-  }
-  int device = 0, sm_count = 0;
-  err = cudaGetDevice(&device);
-  if (err == cudaSuccess) err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
-  if (err != cudaSuccess || sm_count <= 0) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  const unsigned prep_grid = unsigned(n_ch < int64_t(sm_count) ? n_ch : int64_t(sm_count));
-
-  profile_mark(0, stream);
-  const ForwardTiles tiles = forward_tiles(workspace, scratch, n_ch, training != 0);
-  PrepParams pp{q, k, v, g, beta, w, workspace, tiles, T, H, n_chunks, n_ch, scale, training, prologue};
-  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    auto kernel = prologue != 0 ? chunk_prep_kernel<T, G, true> : chunk_prep_kernel<T, G, false>;
-    const int smem = int(sizeof(PrepSmem));
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<prep_grid, kPrepThreads, smem, stream>>>(pp, tm[0], tm[1], tm[2], tm[3], tm[4], tm[5]);
-  });
-  int st = check_launch();
-  if (st != GDN2_OK) return st;
-  profile_mark(1, stream);
-
-  // the scan's operands: the same tiles, in the swizzle of the role the forward reads them in
-  CUtensorMap tm_yt, tm_q, tm_kn, tm_at, tm_u;
-  if (!encode_tile_map(&tm_yt, tiles.yt, n_ch, kDim, kChunk, true) ||
-      !encode_tile_map(&tm_q, tiles.q, n_ch, kChunk, kDim, false) ||
-      !encode_tile_map(&tm_kn, tiles.kn, n_ch, kChunk, kDim, true) ||
-      !encode_tile_map(&tm_at, tiles.at, n_ch, kChunk, kChunk, true, 32) ||
-      !encode_plain_tile_map(&tm_u, tiles.u, n_ch, kChunk, kDim)) {
-    return GDN2_ERR_LAUNCH;
-  }
-  ScanParams sp{workspace, s_in, out, s_out, bnd, status, T, H, n_chunks, n_ch, workspace, training};
-  const int smem = int(sizeof(ScanSmem));
-  if (dtype == GDN2_BF16) {
-    auto kernel = chunk_scan_kernel<__nv_bfloat16>;
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<unsigned(B * H), kScanThreads, smem, stream>>>(sp, tm_yt, tm_q, tm_kn, tm_at, tm_u);
-  } else {
-    auto kernel = chunk_scan_kernel<__half>;
-    err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<unsigned(B * H), kScanThreads, smem, stream>>>(sp, tm_yt, tm_q, tm_kn, tm_at, tm_u);
-  }
-  st = check_launch();
-  profile_mark(2, stream);
-  return st;
+// `table` lists the sequences of at least one chunk, longest first; `rows` is the packed length.
+int launch_packed_chunk_forward(const PackedSeqs& table, const void* q, const void* k, const void* v, const void* g,
+                                const void* beta, const void* w, const float* s_in, void* out, float* s_out,
+                                float* bnd, uint8_t* workspace, uint8_t* scratch, int64_t rows, int64_t H,
+                                int training, int dtype, int g_dtype, float scale, int prologue,
+                                cudaStream_t stream) {
+  const ForwardCall a{q, k, v, g, beta, w, s_in, out, s_out, bnd, workspace, scratch, rows, H,
+                      training, dtype, g_dtype, scale, prologue};
+  return launch_forward(table, a, stream);
 }
 
 }  // namespace gdn2

@@ -36,6 +36,17 @@ __device__ __forceinline__ float from_float<float>(float x) {
   return x;
 }
 
+// two values converted at once (one instruction for both)
+template <typename T> struct Pair;
+template <> struct Pair<__nv_bfloat16> {
+  using type = __nv_bfloat162;
+  __device__ static __forceinline__ type make(float lo, float hi) { return __floats2bfloat162_rn(lo, hi); }
+};
+template <> struct Pair<__half> {
+  using type = __half2;
+  __device__ static __forceinline__ type make(float lo, float hi) { return __floats2half2_rn(lo, hi); }
+};
+
 template <typename T>
 __device__ __forceinline__ float ldf(const void* base, int64_t index) {
   return to_float(static_cast<const T*>(base)[index]);
@@ -77,6 +88,15 @@ __device__ __forceinline__ float prologue_sigmoid(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-x)));
   return r;
 }
+// Two at a time with one reciprocal, 1 / (a b): three special-function results instead of four.  The
+// arguments are held to -43 so that the product stays finite (a sigmoid is 2e-19 there).
+__device__ __forceinline__ void prologue_sigmoid2(float& x, float& y) {
+  const float a = 1.f + __expf(-fmaxf(x, -43.f)), b = 1.f + __expf(-fmaxf(y, -43.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
+  x = r * b;
+  y = r * a;
+}
 // log-decay g = -softplus(x) = -log(1 + e^x).  Small e^x: the series e - e^2/2 + e^3/3 (its first
 // dropped term is below 2^-26 of the sum there; lg2 of a number next to 1 would lose the digits);
 // softplus(x) equals x to fp32 precision beyond 20.
@@ -90,6 +110,7 @@ __device__ __forceinline__ float prologue_log_decay(float x) {
 // ---- host-side status helpers ---------------------------------------------------
 void record_cuda_error(cudaError_t err);  // defined in api.cu
 int check_launch();                       // cudaGetLastError -> status
+int multiprocessors(int* count);          // SMs of the current device, looked up once per device (api.cu)
 cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);  // once per (kernel, device) opt-in (api.cu)
 void profile_mark(int index, cudaStream_t stream);  // records timing event `index` when profiling is on (api.cu)
 
