@@ -53,6 +53,9 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_gate_prologue_vjp": [_P] * 17 + [_I64] * 3 + [_INT, _INT, _P],
     "gdn2_chunk_forward_static": [_P] * 9 + [_I64] * 4 + [_INT, _INT, _F32, _P],
     "gdn2_chunk_static_read_status": [_P],
+    "gdn2_packed_sizes": [_P] + [_I64] * 3 + [_P] * 3,
+    "gdn2_packed_forward": [_P] * 14 + [_I64] * 3 + [_INT] * 3 + [_F32, _INT, _P],
+    "gdn2_packed_backward": [_P] * 22 + [_I64] * 3 + [_INT, _INT, _F32, _P],
     "gdn2_profile_enable": [_INT],
     "gdn2_profile_chunk_kernels": [_P] * 4,
 }
@@ -119,11 +122,11 @@ _KERNELS_PER_CALL = {"gdn2_chunk_forward": 2, "gdn2_chunk_forward_fused": 2, "gd
                      "gdn2_chunk_forward_static": 2}
 
 
-def check(status: int, what: str) -> None:
+def check(status: int, what: str, kernels: int | None = None) -> None:
     """Turn a negative gdn2_status into a RuntimeError; count successful launches."""
 
     if status == 0:
-        LAUNCHES[0] += _KERNELS_PER_CALL.get(what, 1)
+        LAUNCHES[0] += _KERNELS_PER_CALL.get(what, 1) if kernels is None else kernels
         return
     handle = lib()
     text = handle.gdn2_status_string(status).decode()
@@ -132,8 +135,9 @@ def check(status: int, what: str) -> None:
     raise RuntimeError(f"{what} failed with status {status}: {text}{suffix}")
 
 
-def call(name: str, device: torch.device, *args) -> None:
-    """Invoke entry point ``name`` with ``device`` current; raise on a non-zero status."""
+def call(name: str, device: torch.device, *args, kernels: int | None = None) -> None:
+    """Invoke entry point ``name`` with ``device`` current; raise on a non-zero status.  ``kernels``:
+    what a successful call launches, where that is not a property of the entry point."""
 
     fn = getattr(lib(), name)
     with torch.cuda.device(device):
@@ -146,7 +150,7 @@ def call(name: str, device: torch.device, *args) -> None:
             status = fn(*args)
             end.record()
             KERNEL_EVENTS.setdefault(name, []).append((begin, end))
-    check(status, name)
+    check(status, name, kernels)
 
 
 _capability_ok: dict[int, bool] = {}

@@ -1239,7 +1239,7 @@ int launch_chunk_backward(const void* q, const void* k, const void* v, const voi
                           cudaStream_t stream) {
   const int64_t n_chunks = full_tokens / kChunk;
   if (B * T > int64_t(0x7fffffff) || B * n_chunks * H > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  const UniformSeqs seqs{T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
+  const UniformSeqs seqs{0, T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
   const BackwardCall a{q, k, v, g, beta, w, d_out, ds_final, bnd, d_bnd, workspace, scratch, dq, dk, dv, dg, dbeta,
                        dw, ds_init, B * T, H, dtype, g_dtype, scale, grads_f32, full_tokens > T};
   return launch_backward(seqs, a, stream);

@@ -1169,7 +1169,7 @@ int launch_chunk_forward(const void* q, const void* k, const void* v, const void
                          int prologue, cudaStream_t stream) {
   const int64_t n_chunks = full_tokens / kChunk;
   if (B * T > int64_t(0x7fffffff) || B * n_chunks * H > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
-  const UniformSeqs seqs{T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
+  const UniformSeqs seqs{0, T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
   const ForwardCall a{q, k, v, g, beta, w, s_in, out, s_out, bnd, workspace, scratch, B * T, H,
                       training, dtype, g_dtype, scale, prologue};
   return launch_forward(seqs, a, stream);

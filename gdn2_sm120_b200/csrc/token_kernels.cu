@@ -19,6 +19,7 @@
 // exactly one thread (which is why an exact in-place state update is race-free).
 
 #include "common.cuh"
+#include "seqs.cuh"
 #include "tc05.cuh"
 
 namespace gdn2 {
@@ -43,7 +44,7 @@ struct TokenFwdParams {
   void* out;
   float* s_out;
   float* bnd;
-  int64_t T, H, t_begin, t_end, n_slots;
+  int H;
   float scale;
   int prologue;  // kPrologueNorm | kPrologueGate: raw projections / gate pre-activations are activated here
 };
@@ -61,8 +62,9 @@ __device__ __forceinline__ float4 ld_red4(const float (*red)[kTokVT], int col) {
 
 // kPro (here and in the two decode kernels below): the instantiation that can apply the layer prologue
 // to raw inputs; the plain instantiation carries none of that code.
-template <typename T, typename G, bool kPro = false>
-__global__ void __launch_bounds__(kTokThreads) token_forward_kernel(const TokenFwdParams p) {
+template <typename T, typename G, typename Seqs, bool kPro = false>
+__global__ void __launch_bounds__(kTokThreads)
+token_forward_kernel(const TokenFwdParams p, const __grid_constant__ Seqs seqs) {
   __shared__ float s_a[2][kDim], s_e[2][kDim], s_k[2][kDim], s_q[2][kDim];
   __shared__ float s_z[2][kTokVT];
   __shared__ __align__(16) float s_red[2][2][4][kTokVT];  // [buffer][erase|output][warp][column]
@@ -71,14 +73,15 @@ __global__ void __launch_bounds__(kTokThreads) token_forward_kernel(const TokenF
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cg = tid & 7, rg = tid >> 3;
   const int vt = int(blockIdx.x % kTokTiles);
-  const int64_t bh = blockIdx.x / kTokTiles;
-  const int64_t b = bh / p.H, h = bh % p.H;
+  const int sh = int(blockIdx.x / kTokTiles), s_ = sh / p.H, h = sh - s_ * p.H;
+  const SeqInfo sq = seqs.at(s_);
+  const int64_t bh = int64_t(sq.sid) * p.H + h;
   const int col0 = vt * kTokVT + cg * 4;
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
 
-  auto stage = [&](int64_t t, int buf) {
-    const int64_t idx = ((b * p.T + t) * p.H + h) * kDim;
+  auto stage = [&](int t, int buf) {
+    const int64_t idx = ((sq.row0 + t) * p.H + h) * kDim;
     const float kv = ldf<T>(p.k, idx + tid);
     float gv = ldf<G>(p.g, idx + tid), bv = ldf<T>(p.beta, idx + tid);
     const float qv = ldf<T>(p.q, idx + tid);
@@ -120,16 +123,13 @@ __global__ void __launch_bounds__(kTokThreads) token_forward_kernel(const TokenF
     for (int i = 0; i < kRowsPerThread; ++i) store4(base + (rg + 16 * i) * kDim + col0, vec, S[i]);
   };
 
-  if (p.t_begin < p.t_end) {
-    stage(p.t_begin, 0);
-  }
+  if (sq.len > 0) stage(0, 0);
   __syncthreads();
 
-  for (int64_t t = p.t_begin; t < p.t_end; ++t) {
-    const int64_t rel = t - p.t_begin;
-    const int buf = int(rel & 1);
-    if (p.bnd != nullptr && (rel % kTokenInterval) == 0) {
-      store_tile(p.bnd + ((b * p.n_slots + rel / kTokenInterval) * p.H + h) * kStateElems);
+  for (int t = 0; t < sq.len; ++t) {
+    const int buf = t & 1;
+    if (p.bnd != nullptr && (t % kTokenInterval) == 0) {
+      store_tile(p.bnd + (int64_t(sq.slot0 + t / kTokenInterval) * p.H + h) * kStateElems);
     }
     // reciprocal norms of this token's raw q and k (1 when the inputs are already normalised)
     float iq = 1.f, ik = 1.f;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(kTokThreads) token_forward_kernel(const TokenF
     if (lane < 8) {
       *reinterpret_cast<float4*>(&s_red[buf][0][warp][cg * 4]) = make_float4(r[0], r[1], r[2], r[3]);
     }
-    if (t + 1 < p.t_end) stage(t + 1, buf ^ 1);
+    if (t + 1 < sq.len) stage(t + 1, buf ^ 1);
     __syncthreads();
 
     const float4 rs = ld_red4(s_red[buf][0], cg * 4);
@@ -186,12 +186,12 @@ __global__ void __launch_bounds__(kTokThreads) token_forward_kernel(const TokenF
     if (tid < kTokVT) {
       const float ov = s_red[buf][1][0][tid] + s_red[buf][1][1][tid] + s_red[buf][1][2][tid] +
                        s_red[buf][1][3][tid];
-      stf<T>(p.out, ((b * p.T + t) * p.H + h) * kDim + vt * kTokVT + tid, ov);
+      stf<T>(p.out, ((sq.row0 + t) * p.H + h) * kDim + vt * kTokVT + tid, ov);
     }
   }
 
   if (p.bnd != nullptr) {
-    store_tile(p.bnd + ((b * p.n_slots + (p.n_slots - 1)) * p.H + h) * kStateElems);
+    store_tile(p.bnd + (int64_t(sq.slot0 + sq.n_chunks) * p.H + h) * kStateElems);
   }
   if (p.s_out != nullptr) {
     store_tile(p.s_out + bh * kStateElems);
@@ -443,12 +443,13 @@ struct DstateScanParams {
   const float* ds_final;
   float* d_bnd;
   float* ds_init;
-  int64_t T, H, t_begin, t_end, n_slots;
+  int H;
   float scale;
 };
 
-template <typename T, typename G>
-__global__ void __launch_bounds__(kTokThreads) token_dstate_scan_kernel(const DstateScanParams p) {
+template <typename T, typename G, typename Seqs>
+__global__ void __launch_bounds__(kTokThreads)
+token_dstate_scan_kernel(const DstateScanParams p, const __grid_constant__ Seqs seqs) {
   __shared__ float s_a[2][kDim], s_e[2][kDim], s_k[2][kDim], s_q[2][kDim];
   __shared__ float s_do[2][kTokVT];
   __shared__ __align__(16) float s_red[2][4][kTokVT];
@@ -456,12 +457,13 @@ __global__ void __launch_bounds__(kTokThreads) token_dstate_scan_kernel(const Ds
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cg = tid & 7, rg = tid >> 3;
   const int vt = int(blockIdx.x % kTokTiles);
-  const int64_t bh = blockIdx.x / kTokTiles;
-  const int64_t b = bh / p.H, h = bh % p.H;
+  const int sh = int(blockIdx.x / kTokTiles), s_ = sh / p.H, h = sh - s_ * p.H;
+  const SeqInfo sq = seqs.at(s_);
+  const int64_t bh = int64_t(sq.sid) * p.H + h;
   const int col0 = vt * kTokVT + cg * 4;
 
-  auto stage = [&](int64_t t, int buf) {
-    const int64_t idx = ((b * p.T + t) * p.H + h) * kDim;
+  auto stage = [&](int t, int buf) {
+    const int64_t idx = ((sq.row0 + t) * p.H + h) * kDim;
     const float kv = ldf<T>(p.k, idx + tid);
     s_a[buf][tid] = expf(ldf<G>(p.g, idx + tid));
     s_e[buf][tid] = ldf<T>(p.beta, idx + tid) * kv;
@@ -486,12 +488,12 @@ __global__ void __launch_bounds__(kTokThreads) token_dstate_scan_kernel(const Ds
     for (int i = 0; i < kRowsPerThread; ++i) store4(base + (rg + 16 * i) * kDim + col0, vec, dS[i]);
   };
 
-  store_tile(p.d_bnd + ((b * p.n_slots + (p.n_slots - 1)) * p.H + h) * kStateElems);
-  if (p.t_begin < p.t_end) stage(p.t_end - 1, 0);
+  store_tile(p.d_bnd + (int64_t(sq.slot0 + sq.n_chunks) * p.H + h) * kStateElems);
+  if (sq.len > 0) stage(sq.len - 1, 0);
   __syncthreads();
 
   int buf = 0;
-  for (int64_t t = p.t_end - 1; t >= p.t_begin; --t, buf ^= 1) {
+  for (int t = sq.len - 1; t >= 0; --t, buf ^= 1) {
     // dS' = dS + (scale q) do^T ; partial du = dS'^T k
     float du[4] = {0.f, 0.f, 0.f, 0.f};
     float dov[4];
@@ -514,8 +516,8 @@ __global__ void __launch_bounds__(kTokThreads) token_dstate_scan_kernel(const Ds
     if (lane < 8) {
       *reinterpret_cast<float4*>(&s_red[buf][warp][cg * 4]) = make_float4(du[0], du[1], du[2], du[3]);
     }
-    if (t - 1 >= p.t_begin) stage(t - 1, buf ^ 1);
     __syncthreads();
+    if (t > 0) stage(t - 1, buf ^ 1);  // (behind the barrier: its buffer was read up to the end of the last step)
     const float4 ds = ld_red4(s_red[buf], cg * 4);
     const float dus[4] = {ds.x, ds.y, ds.z, ds.w};
     // dS <- a * (dS' - e du^T)
@@ -525,10 +527,10 @@ __global__ void __launch_bounds__(kTokThreads) token_dstate_scan_kernel(const Ds
 #pragma unroll
       for (int c = 0; c < 4; ++c) dS[i][c] = a * fmaf(-e, dus[c], dS[i][c]);
     }
-    const int64_t rel = t - p.t_begin;
-    if ((rel % kTokenInterval) == 0) {
-      store_tile(p.d_bnd + ((b * p.n_slots + rel / kTokenInterval) * p.H + h) * kStateElems);
+    if ((t % kTokenInterval) == 0) {
+      store_tile(p.d_bnd + (int64_t(sq.slot0 + t / kTokenInterval) * p.H + h) * kStateElems);
     }
+    __syncthreads();  // the next token is staged
   }
   if (p.ds_init != nullptr) store_tile(p.ds_init + bh * kStateElems);
 }
@@ -559,7 +561,7 @@ struct ChunkVjpParams {
   const void *q, *k, *v, *g, *beta, *w, *d_out;
   const float *bnd, *d_bnd;
   void *dq, *dk, *dv, *dg, *dbeta, *dw;
-  int64_t T, H, t_begin, t_end, n_slots;
+  int H;
   float scale;
 };
 
@@ -593,21 +595,21 @@ __device__ __forceinline__ void block_sum8(float (&x)[8], float (*red)[4][kVjpVT
   rb ^= 1;
 }
 
-template <typename T, typename G>
-__global__ void __launch_bounds__(kVjpThreads) token_chunk_vjp_kernel(const ChunkVjpParams p) {
+template <typename T, typename G, typename Seqs>
+__global__ void __launch_bounds__(kVjpThreads)
+token_chunk_vjp_kernel(const ChunkVjpParams p, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   VjpSmem<T>& sm = *reinterpret_cast<VjpSmem<T>*>(smem_raw);
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int64_t n_spans = p.n_slots - 1;
-  const int64_t h = blockIdx.x % p.H;
-  const int64_t j = (blockIdx.x / p.H) % n_spans;
-  const int64_t b = blockIdx.x / (p.H * n_spans);
-  const int64_t t0 = p.t_begin + j * kTokenInterval;
-  const int n = int(min(int64_t(kTokenInterval), p.t_end - t0));
+  const int span = int(blockIdx.x) / p.H, h = int(blockIdx.x) - span * p.H;
+  const SeqInfo sq = seqs.at(seqs.find(span));
+  const int j = span - sq.chunk0;
+  const int64_t row0 = sq.row0 + j * kTokenInterval;
+  const int n = min(kTokenInterval, sq.len - j * kTokenInterval);
 
   for (int t = 0; t < n; ++t) {
-    const int64_t idx = ((b * p.T + t0 + t) * p.H + h) * kDim + tid;
+    const int64_t idx = ((row0 + t) * p.H + h) * kDim + tid;
     sm.q[t][tid] = static_cast<const T*>(p.q)[idx];
     sm.k[t][tid] = static_cast<const T*>(p.k)[idx];
     sm.beta[t][tid] = static_cast<const T*>(p.beta)[idx];
@@ -622,8 +624,8 @@ __global__ void __launch_bounds__(kVjpThreads) token_chunk_vjp_kernel(const Chun
 #pragma unroll
   for (int t = 0; t < kTokenInterval; ++t) adq[t] = adk[t] = ade[t] = adg[t] = 0.f;
 
-  const float* s_src = p.bnd + ((b * p.n_slots + j) * p.H + h) * kStateElems + tid * kDim;
-  const float* ds_src = p.d_bnd + ((b * p.n_slots + j + 1) * p.H + h) * kStateElems + tid * kDim;
+  const float* s_src = p.bnd + (int64_t(sq.slot0 + j) * p.H + h) * kStateElems + tid * kDim;
+  const float* ds_src = p.d_bnd + (int64_t(sq.slot0 + j + 1) * p.H + h) * kStateElems + tid * kDim;
   int rb = 0;
 
   for (int pass = 0; pass < kVjpPasses; ++pass) {
@@ -710,7 +712,7 @@ __global__ void __launch_bounds__(kVjpThreads) token_chunk_vjp_kernel(const Chun
 #pragma unroll
   for (int t = 0; t < kTokenInterval; ++t) {
     if (t < n) {
-      const int64_t idx = ((b * p.T + t0 + t) * p.H + h) * kDim + tid;
+      const int64_t idx = ((row0 + t) * p.H + h) * kDim + tid;
       const float kv = to_float(sm.k[t][tid]);
       const float bv = to_float(sm.beta[t][tid]);
       stf<T>(p.dq, idx, p.scale * adq[t]);
@@ -724,11 +726,58 @@ __global__ void __launch_bounds__(kVjpThreads) token_chunk_vjp_kernel(const Chun
   }
 }
 
-inline int64_t slots_for(int64_t t_begin, int64_t t_end) {
-  return (t_end - t_begin + kTokenInterval - 1) / kTokenInterval + 1;
-}
+inline int64_t spans_for(int64_t tokens) { return (tokens + kTokenInterval - 1) / kTokenInterval; }
 
 inline bool grid_fits(int64_t blocks) { return blocks > 0 && blocks <= int64_t(0x7fffffff); }
+
+// batch rows' token ranges [t_begin, t_end); false when a grid or a slot number would not fit 31 bits
+bool uniform_spans(int64_t B, int64_t T, int64_t H, int64_t t_begin, int64_t t_end, UniformSeqs* seqs) {
+  const int64_t spans = spans_for(t_end - t_begin);
+  if (t_end - t_begin > int64_t(0x7fffffff) || !grid_fits(B * H * kTokTiles) ||
+      B * (spans + 1) * H > int64_t(0x7fffffff)) {
+    return false;
+  }
+  *seqs = UniformSeqs{t_begin, T, int(t_end - t_begin), int(spans), int(B)};
+  return true;
+}
+
+template <typename Seqs>
+int run_token_forward(const Seqs& seqs, const TokenFwdParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+  const int64_t blocks = int64_t(seqs.count()) * p.H * kTokTiles;
+  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
+  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+    if (p.prologue != 0) {
+      token_forward_kernel<T, G, Seqs, true><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
+    } else {
+      token_forward_kernel<T, G, Seqs, false><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
+    }
+  });
+  return check_launch();
+}
+
+template <typename Seqs>
+int run_dstate_scan(const Seqs& seqs, const DstateScanParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+  const int64_t blocks = int64_t(seqs.count()) * p.H * kTokTiles;
+  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
+  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+    token_dstate_scan_kernel<T, G, Seqs><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
+  });
+  return check_launch();
+}
+
+template <typename Seqs>
+int run_chunk_vjp(const Seqs& seqs, const ChunkVjpParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+  const int64_t blocks = int64_t(seqs.total_chunks()) * p.H;
+  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
+  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+    auto kernel = token_chunk_vjp_kernel<T, G, Seqs>;
+    const int smem = int(sizeof(VjpSmem<T>));
+    const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+    kernel<<<unsigned(blocks), kVjpThreads, smem, stream>>>(p, seqs);
+  });
+  return check_launch();
+}
 
 }  // namespace
 
@@ -759,13 +808,18 @@ int launch_token_forward(const void* q, const void* k, const void* v, const void
     });
     return check_launch();
   }
-  TokenFwdParams p{q, k, v, g, beta, w, s_in, out, s_out, bnd,
-                   T, H, t_begin, t_end, slots_for(t_begin, t_end), scale, prologue};
-  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    if (prologue != 0) token_forward_kernel<T, G, true><<<unsigned(blocks), kTokThreads, 0, stream>>>(p);
-    else token_forward_kernel<T, G, false><<<unsigned(blocks), kTokThreads, 0, stream>>>(p);
-  });
-  return check_launch();
+  UniformSeqs seqs;
+  if (!uniform_spans(B, T, H, t_begin, t_end, &seqs)) return GDN2_ERR_TOO_LARGE;
+  return run_token_forward(seqs, TokenFwdParams{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), scale, prologue},
+                           dtype, g_dtype, stream);
+}
+
+int launch_packed_token_forward(const PackedSpans& table, const void* q, const void* k, const void* v, const void* g,
+                                const void* beta, const void* w, const float* s_in, void* out, float* s_out,
+                                float* bnd, int64_t H, int dtype, int g_dtype, float scale, int prologue,
+                                cudaStream_t stream) {
+  return run_token_forward(table, TokenFwdParams{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), scale, prologue},
+                           dtype, g_dtype, stream);
 }
 
 int launch_token_t1_zero(const void* q, const void* k, const void* v, const void* w, void* out,
@@ -789,14 +843,10 @@ int launch_token_dstate_scan(const void* q, const void* k, const void* g, const 
                              float* ds_init, int64_t B, int64_t T, int64_t H, int64_t t_begin,
                              int64_t t_end, int dtype, int g_dtype, float scale,
                              cudaStream_t stream) {
-  const int64_t blocks = B * H * kTokTiles;
-  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
-  DstateScanParams p{q, k, g, beta, d_out, ds_final, d_bnd, ds_init,
-                     T, H, t_begin, t_end, slots_for(t_begin, t_end), scale};
-  GDN2_DISPATCH_TYPES(
-      dtype, g_dtype,
-      (token_dstate_scan_kernel<T, G><<<unsigned(blocks), kTokThreads, 0, stream>>>(p)));
-  return check_launch();
+  UniformSeqs seqs;
+  if (!uniform_spans(B, T, H, t_begin, t_end, &seqs)) return GDN2_ERR_TOO_LARGE;
+  return run_dstate_scan(seqs, DstateScanParams{q, k, g, beta, d_out, ds_final, d_bnd, ds_init, int(H), scale}, dtype,
+                         g_dtype, stream);
 }
 
 int launch_token_chunk_vjp(const void* q, const void* k, const void* v, const void* g,
@@ -805,23 +855,22 @@ int launch_token_chunk_vjp(const void* q, const void* k, const void* v, const vo
                            void* dbeta, void* dw, int64_t B, int64_t T, int64_t H,
                            int64_t t_begin, int64_t t_end, int dtype, int g_dtype, float scale,
                            cudaStream_t stream) {
-  const int64_t n_slots = slots_for(t_begin, t_end);
-  const int64_t blocks = B * (n_slots - 1) * H;
-  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
-  ChunkVjpParams p{q, k, v, g, beta, w, d_out, bnd, d_bnd, dq, dk, dv, dg, dbeta, dw,
-                   T, H, t_begin, t_end, n_slots, scale};
-  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    auto kernel = token_chunk_vjp_kernel<T, G>;
-    const int smem = int(sizeof(VjpSmem<T>));
-    cudaError_t err =
-        ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != cudaSuccess) {
-      record_cuda_error(err);
-      return GDN2_ERR_LAUNCH;
-    }
-    kernel<<<unsigned(blocks), kVjpThreads, smem, stream>>>(p);
-  });
-  return check_launch();
+  UniformSeqs seqs;
+  if (!uniform_spans(B, T, H, t_begin, t_end, &seqs)) return GDN2_ERR_TOO_LARGE;
+  return run_chunk_vjp(seqs, ChunkVjpParams{q, k, v, g, beta, w, d_out, bnd, d_bnd, dq, dk, dv, dg, dbeta, dw, int(H),
+                                            scale}, dtype, g_dtype, stream);
+}
+
+int launch_packed_token_backward(const PackedSpans& table, const void* q, const void* k, const void* v, const void* g,
+                                 const void* beta, const void* w, const void* d_out, const float* ds_final,
+                                 const float* bnd, float* d_bnd, void* dq, void* dk, void* dv, void* dg, void* dbeta,
+                                 void* dw, float* ds_init, int64_t H, int dtype, int g_dtype, float scale,
+                                 cudaStream_t stream) {
+  int st = run_dstate_scan(table, DstateScanParams{q, k, g, beta, d_out, ds_final, d_bnd, ds_init, int(H), scale},
+                           dtype, g_dtype, stream);
+  if (st != GDN2_OK || table.chunks == 0) return st;
+  return run_chunk_vjp(table, ChunkVjpParams{q, k, v, g, beta, w, d_out, bnd, d_bnd, dq, dk, dv, dg, dbeta, dw, int(H),
+                                             scale}, dtype, g_dtype, stream);
 }
 
 }  // namespace gdn2

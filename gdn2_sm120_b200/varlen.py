@@ -6,30 +6,29 @@ the reference); callers that batch ragged sequences need them next to the operat
 ``chunk_gdn2_varlen``    several sequences packed along the time axis of ``[1, total, H, 128]``
                          tensors, delimited by ``cu_seqlens`` (``[N + 1]`` cumulative lengths, as
                          in flash-attention style APIs), each with its own initial / final state
-                         (``[N, H, 128, 128]``).  Every sequence is an independent recurrence, so
-                         the implementation walks over the sequences and runs the same
-                         shape-dispatched kernels on each slice of the packed buffers (a slice of
-                         consecutive tokens of a batch-1 tensor is itself a contiguous
-                         ``[1, L, H, 128]`` tensor: nothing is copied on the way in).  One
-                         ``autograd.Function`` spans the whole call, so backward writes every
+                         (``[N, H, 128, 128]``).  Every sequence is an independent recurrence; the
+                         kernels of all of them are launched together (csrc/packed.cu), each
+                         sequence on the kernels its length calls for.  One
+                         ``autograd.Function`` spans the whole call, and backward writes every
                          sequence's gradients straight into the packed gradient tensors.
 ``expand_grouped_heads`` key-shaped tensors given for fewer heads than the value-shaped ones
                          (every group of value heads shares one q / k / g / beta head) expanded
                          to the value heads; gradients of the shared heads are summed by autograd.
 
-The kernels themselves are unchanged: one launch sequence per packed sequence, which is efficient
-for long sequences (prefill, training on documents) and launch-bound for many very short ones.
+A batch goes to the library in groups of consecutive sequences: at most 256 of them (their table
+travels in the kernels' parameters) and no more than the scratch budget of ``chunk_kernels`` holds.
 """
 
 from __future__ import annotations
 
+import ctypes
 import math
+from dataclasses import dataclass
 
 import torch
 
-from . import _validate
-from .backward import backward_from_aux
-from .ops import _aux_from_tensors, _aux_tensors, _forward_with_aux, _prologue_flags
+from . import _lib, _validate, chunk_kernels
+from .ops import _prologue_flags
 from .prologue import gate_prologue
 
 _DIM = 128
@@ -49,77 +48,139 @@ def _bounds(cu_seqlens, total: int) -> tuple[int, ...]:
     return tuple(values)
 
 
-def _packed_forward(seq, state, bounds, scale: float, prepare_backward: bool, prologue: int = 0):
-    """Forward over every packed sequence; returns output, final states and the saved checkpoints."""
+_MAX_SEQUENCES = 256
+
+
+@dataclass(frozen=True)
+class _Group:
+    """Consecutive sequences ``first .. last - 1`` handed to the library in one call."""
+
+    first: int
+    last: int
+    bounds: ctypes.Array   # int64[last - first + 1], rows of the packed tensors
+    chunks: int
+    chunk_slots: int
+    span_slots: int
+
+
+def _plan_groups(bounds: tuple[int, ...], heads: int, training: bool) -> list[_Group]:
+    per_unit = chunk_kernels.scratch_bytes(1, 64, 1, False)
+    if training:
+        per_unit = chunk_kernels.scratch_bytes(1, 64, 1, True) + 2 * 65536
+    most = max(1, chunk_kernels.SCRATCH_BUDGET_BYTES // (per_unit * heads))
+    groups, first, chunks = [], 0, 0
+    for i in range(len(bounds) - 1):
+        own = chunk_kernels.supported_tokens(bounds[i + 1] - bounds[i]) // 64
+        if i > first and (i - first == _MAX_SEQUENCES or chunks + own > most):
+            groups.append((first, i))
+            first, chunks = i, 0
+        chunks += own
+    groups.append((first, len(bounds) - 1))
+    out, sizes = [], [ctypes.c_int64() for _ in range(3)]
+    for lo, hi in groups:
+        part = (ctypes.c_int64 * (hi - lo + 1))(*bounds[lo:hi + 1])
+        status = _lib.lib().gdn2_packed_sizes(part, hi - lo, bounds[-1], heads, *(ctypes.byref(x) for x in sizes))
+        if status != 0:
+            raise RuntimeError(f"gdn2_packed_sizes failed with status {status}")
+        out.append(_Group(lo, hi, part, *(x.value for x in sizes)))
+    return out
+
+
+def _states(slots: int, heads: int, device):
+    if not slots:
+        return None
+    return torch.empty((slots, heads, _DIM, _DIM), device=device, dtype=torch.float32)
+
+
+def _bytes(size: int, device):
+    return torch.empty(size, device=device, dtype=torch.uint8)
+
+
+def _packed_forward(seq, state, bounds, scale: float, training: bool, prologue: int = 0):
+    """Forward over every packed sequence; returns output, final states and what backward needs: the
+    groups and, for each, ``(workspace, chunk checkpoints, span checkpoints)``."""
 
     q = seq[0]
-    n_seq, heads = len(bounds) - 1, q.shape[2]
+    n_seq, total, heads, device = len(bounds) - 1, q.shape[1], q.shape[2], q.device
     output = torch.empty_like(seq[2])
-    final_state = torch.empty((n_seq, heads, _DIM, _DIM), device=q.device, dtype=torch.float32)
-    saved, layouts = [], []
-    for i, (start, stop) in enumerate(zip(bounds, bounds[1:])):
-        state_i = None if state is None else state[i:i + 1]
-        if stop == start:   # an empty sequence leaves its state as it is
-            if state_i is None:
-                final_state[i].zero_()
-            else:
-                final_state[i:i + 1].copy_(state_i)
-            layouts.append((0, 0, 0, 0))
-            continue
-        piece = tuple(t[:, start:stop] for t in seq)
-        out_i, final_i, aux = _forward_with_aux(piece, state_i, scale, prepare_backward, prologue)
-        output[:, start:stop].copy_(out_i)
-        final_state[i:i + 1].copy_(final_i)
-        tensors, layout = _aux_tensors(aux)
-        saved.extend(tensors)
-        layouts.append(layout)
-    return output, final_state, saved, tuple(layouts)
+    final_state = torch.empty((n_seq, heads, _DIM, _DIM), device=device, dtype=torch.float32)
+    if total == 0:
+        final_state.zero_() if state is None else final_state.copy_(state)
+        return output, final_state, [], []
+    saved, groups = [], _plan_groups(bounds, heads, training)
+    scale = _validate.float32_scale(scale)
+    for group in groups:
+        tokens = 64 * group.chunks
+        workspace = scratch = chunk_states = span_states = None
+        if tokens:
+            size = chunk_kernels.workspace_bytes(1, tokens, heads, training)
+            scratch_size = chunk_kernels.scratch_bytes(1, tokens, heads, False, training=training)
+            slots = group.chunk_slots if training else 0
+            chunk_kernels.check_memory(size + scratch_size + slots * heads * _DIM * _DIM * 4, device, "packed forward")
+            workspace, scratch = _bytes(size, device), _bytes(scratch_size, device)
+        if training:
+            chunk_states = _states(group.chunk_slots, heads, device)
+            span_states = _states(group.span_slots, heads, device)
+        part = slice(group.first, group.last)
+        _lib.call("gdn2_packed_forward", device, *(x.data_ptr() for x in seq),
+                  None if state is None else state[part].data_ptr(), output.data_ptr(), final_state[part].data_ptr(),
+                  _lib.ptr(chunk_states), _lib.ptr(span_states), _lib.ptr(workspace), _lib.ptr(scratch), group.bounds,
+                  group.last - group.first, total, heads, int(training), _lib.dtype_code(q.dtype),
+                  _lib.dtype_code(seq[3].dtype), scale, prologue, _lib.stream_ptr(device),
+                  kernels=2 * (group.chunks > 0) + (group.span_slots > 0))
+        saved.append((workspace, chunk_states, span_states))
+    return output, final_state, groups, saved
 
 
 class _ChunkGDN2Varlen(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, g, beta, w, initial_state, bounds, scale: float):
         seq = tuple(_validate.detached(x) for x in (q, k, v, g, beta, w))
-        output, final_state, saved, layouts = _packed_forward(seq, _validate.detached(initial_state), bounds,
-                                                              scale, True)
-        ctx.save_for_backward(q, k, v, g, beta, w, *saved)
+        output, final_state, ctx.groups, saved = _packed_forward(seq, _validate.detached(initial_state), bounds, scale,
+                                                                 True)
+        ctx.present = [tuple(x is not None for x in item) for item in saved]
+        ctx.save_for_backward(q, k, v, g, beta, w, *(x for item in saved for x in item if x is not None))
         ctx.set_materialize_grads(False)
-        ctx.bounds, ctx.layouts, ctx.scale = bounds, layouts, scale
+        ctx.n_seq, ctx.scale = len(bounds) - 1, scale
         ctx.has_initial_state = initial_state is not None
         return output, final_state
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, d_output, d_final_state):
-        q, k, v, g, beta, w, *saved = ctx.saved_tensors
+        q, k, v, g, beta, w, *rest = ctx.saved_tensors
         seq = tuple(_validate.detached(x) for x in (q, k, v, g, beta, w))
-        n_seq, heads = len(ctx.bounds) - 1, q.shape[2]
-        if d_output is None:
-            d_output = torch.zeros_like(v)
-        elif not d_output.is_contiguous():
-            d_output = d_output.contiguous()
-        if d_final_state is not None and not d_final_state.is_contiguous():
-            d_final_state = d_final_state.contiguous()
+        total, heads, device = q.shape[1], q.shape[2], q.device
+        d_output = torch.zeros_like(v) if d_output is None else _dense(d_output)
+        d_final_state = None if d_final_state is None else _dense(d_final_state)
         grads = tuple(torch.empty_like(x) for x in seq)
-        d_state = torch.empty((n_seq, heads, _DIM, _DIM), device=q.device, dtype=torch.float32)
-        scale = _validate.float32_scale(ctx.scale)
-        cursor = 0
-        for i, (start, stop) in enumerate(zip(ctx.bounds, ctx.bounds[1:])):
-            layout = ctx.layouts[i]
-            d_final_i = None if d_final_state is None else d_final_state[i:i + 1]
-            if stop == start:
-                if d_final_i is None:
-                    d_state[i].zero_()
-                else:
-                    d_state[i:i + 1].copy_(d_final_i)
-                continue
-            count = layout[0] + layout[1] + layout[2]
-            aux = _aux_from_tensors(saved[cursor:cursor + count], layout)
-            cursor += count
-            backward_from_aux(*(t[:, start:stop] for t in seq), aux, d_output[:, start:stop], d_final_i, scale,
-                              grads_out=tuple(gr[:, start:stop] for gr in grads),
-                              d_initial_state_out=d_state[i:i + 1])
+        d_state = torch.empty((ctx.n_seq, heads, _DIM, _DIM), device=device, dtype=torch.float32)
+        if total == 0:
+            d_state.zero_() if d_final_state is None else d_state.copy_(d_final_state)
+        scale, rest = _validate.float32_scale(ctx.scale), iter(rest)
+        for group, present in zip(ctx.groups, ctx.present):
+            workspace, chunk_states, span_states = (next(rest) if there else None for there in present)
+            scratch = d_chunk_states = None
+            if group.chunks:
+                scratch = _bytes(chunk_kernels.scratch_bytes(1, 64 * group.chunks, heads, True), device)
+                d_chunk_states = torch.empty_like(chunk_states)
+            d_span_states = None if span_states is None else torch.empty_like(span_states)
+            part = slice(group.first, group.last)
+            _lib.call("gdn2_packed_backward", device, *(x.data_ptr() for x in seq), d_output.data_ptr(),
+                      None if d_final_state is None else d_final_state[part].data_ptr(), _lib.ptr(chunk_states),
+                      _lib.ptr(d_chunk_states), _lib.ptr(span_states), _lib.ptr(d_span_states), _lib.ptr(workspace),
+                      _lib.ptr(scratch), *(x.data_ptr() for x in grads), d_state[part].data_ptr(), group.bounds,
+                      group.last - group.first, total, heads, _lib.dtype_code(q.dtype), _lib.dtype_code(g.dtype),
+                      scale, _lib.stream_ptr(device),
+                      kernels=2 * (group.chunks > 0) + 2 * (group.span_slots > 0))
         return (*grads, d_state if ctx.has_initial_state else None, None, None)
+
+
+def _dense(tensor):
+    """Contiguous and 16-byte aligned, as the kernels' copies need it (nearly always already so)."""
+
+    tensor = tensor if tensor.is_contiguous() else tensor.contiguous()
+    return tensor if tensor.data_ptr() % 16 == 0 else tensor.clone()
 
 
 def chunk_gdn2_varlen(

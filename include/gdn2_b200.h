@@ -163,9 +163,9 @@ int gdn2_token_chunk_vjp(const void* q, const void* k, const void* v, const void
  *              same tiles): 160 KiB per 64-token chunk and head.  It must then stay alive and
  *              unmodified until that call has run.
  *   scratch    gdn2_chunk_scratch_bytes(batch, full_tokens, heads, kind).  Tiles that only live
- *              inside one call.  kind 0: forward of an inference call (U and the WY tiles, 144 KiB
- *              per chunk-head); kind 2: forward of a training call (U alone, 32 KiB per chunk-head:
- *              the other tiles are in its workspace); kind 1: backward (dZ, 36 KiB per chunk-head).
+ *              inside one call.  kind 0: forward of an inference call (the WY tiles; 144 KiB per
+ *              chunk-head); kind 2: forward of a training call (32 KiB per chunk-head, reserved: its
+ *              tiles are in the workspace); kind 1: backward (dZ, 36 KiB per chunk-head).
  *              Dead when the call's kernels have run, so one scratch buffer serves every call on a
  *              stream; a large batch can be processed as several calls over batch slices that share it.
  * The kernels address tiles, sequence tensors and state checkpoints through tensor maps, which the
@@ -323,6 +323,39 @@ int gdn2_gate_prologue_vjp(const void* q_raw, const void* k_raw, const void* g_r
                            const void* dq, const void* dk, const void* dg, const void* dbeta, const void* dw,
                            void* dq_raw, void* dk_raw, void* dg_raw, void* dbeta_raw, void* dw_raw,
                            int64_t batch, int64_t time, int64_t heads, int dtype, int g_dtype, void* stream);
+
+/*
+ * Packed variable-length sequences: forward and backward of n_seq independent sequences laid out one
+ * after another in [total, H, 128] tensors, in as many launches as one sequence takes.  Sequence i has the
+ * rows bounds[i] .. bounds[i + 1] - 1 (`bounds` is read on the host; n_seq + 1 non-decreasing values
+ * within [0, total]; n_seq <= GDN2_PACKED_MAX_SEQUENCES) and row i of the [n_seq, H, 128, 128] states.
+ * Sequences of 64 tokens and more run on the chunk kernels, shorter ones on the token kernels, an empty
+ * one hands its state through; results equal those of a separate call for each.  No counterpart in the
+ * reference (README.md:128-130, 297-299 list packed sequences as not yet covered).
+ *   gdn2_packed_sizes  number of 64-token chunks, and of chunk and span checkpoint slots
+ *   workspace, scratch sized by gdn2_chunk_workspace_bytes(1, 64 * chunks, H, training) and
+ *                      gdn2_chunk_scratch_bytes(1, 64 * chunks, H, kind); NULL when chunks == 0
+ *   chunk_boundaries   fp32 [chunk_slots, H, 128, 128], span_boundaries fp32 [span_slots, H, 128, 128]:
+ *                      the checkpoints of a training call (NULL otherwise); d_*: same shapes, scratch
+ * All pointers 16-byte aligned.  `training`, `prologue`, types and failures as for gdn2_chunk_forward.
+ */
+#define GDN2_PACKED_MAX_SEQUENCES 256
+int gdn2_packed_sizes(const int64_t* bounds, int64_t n_seq, int64_t total, int64_t heads, int64_t* chunks,
+                      int64_t* chunk_slots, int64_t* span_slots);
+int gdn2_packed_forward(const void* q, const void* k, const void* v, const void* g,
+                        const void* beta, const void* w, const float* initial_state,
+                        void* out, float* final_state, float* chunk_boundaries, float* span_boundaries,
+                        void* workspace, void* scratch, const int64_t* bounds, int64_t n_seq, int64_t total,
+                        int64_t heads, int training, int dtype, int g_dtype, float scale, int prologue,
+                        void* stream);
+int gdn2_packed_backward(const void* q, const void* k, const void* v, const void* g,
+                         const void* beta, const void* w, const void* d_out, const float* d_final_state,
+                         const float* chunk_boundaries, float* d_chunk_boundaries,
+                         const float* span_boundaries, float* d_span_boundaries,
+                         const void* workspace, void* scratch,
+                         void* dq, void* dk, void* dv, void* dg, void* dbeta, void* dw,
+                         float* d_initial_state, const int64_t* bounds, int64_t n_seq, int64_t total,
+                         int64_t heads, int dtype, int g_dtype, float scale, void* stream);
 
 /*
  * Per-kernel timing of the chunk entry points.  While enabled, gdn2_chunk_forward and
