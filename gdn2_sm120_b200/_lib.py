@@ -10,6 +10,8 @@ fails, an exception is raised.
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 import pathlib
 import threading
@@ -95,6 +97,28 @@ def lib() -> ctypes.CDLL:
                 fn.restype = _RESTYPES.get(name, ctypes.c_int)
             _handle = handle
     return _handle
+
+
+_host_module = None
+
+
+def host():
+    """The native host path (csrc/host.cpp), bound to the library; raise if it has not been built."""
+
+    global _host_module
+    if _host_module is not None:
+        return _host_module
+    handle = lib()
+    path = _PACKAGE_DIR / "_host.so"
+    if not path.exists():
+        raise RuntimeError(f"{path} is missing: build it with `python -m gdn2_sm120_b200.build`")
+    loader = importlib.machinery.ExtensionFileLoader("_host", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+    loader.exec_module(module)
+    addresses = {name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in _PROTOTYPES}
+    module.bind(addresses, check, LAUNCHES, torch.cuda.OutOfMemoryError)
+    _host_module = module
+    return module
 
 
 def dtype_code(dtype: torch.dtype) -> int:

@@ -13,7 +13,7 @@ import math
 
 import torch
 
-from . import _validate
+from . import _lib, _validate, chunk_kernels
 from .backward import backward_from_aux
 from .chunk import ChunkForwardAux, _token_slots, chunk_forward
 from .prologue import gate_prologue
@@ -104,20 +104,40 @@ class _ChunkGDN2(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, q, k, v, g, beta, w, initial_state, scale: float, prepare_backward: bool):
+        ctx.set_materialize_grads(False)
+        ctx.has_initial_state = initial_state is not None
+        ctx.scale = scale
+        done = None
+        if prepare_backward and q.is_cuda and _lib.KERNEL_EVENTS is None:
+            done = _lib.host().train_forward(q, k, v, g, beta, w, initial_state, scale,
+                                             chunk_kernels.SCRATCH_BUDGET_BYTES)
+        ctx.native = done is not None
+        if ctx.native:
+            output, final_state, workspace, boundaries = done
+            if workspace is None:
+                ctx.save_for_backward(q, k, v, g, beta, w, boundaries)
+                ctx.aux_layout = (0, 1, 0, 0)
+            else:
+                ctx.save_for_backward(q, k, v, g, beta, w, boundaries, workspace)
+                ctx.aux_layout = (1, 0, 1, chunk_kernels.supported_tokens(q.shape[1]))
+            return output, final_state
         seq = tuple(_validate.detached(x) for x in (q, k, v, g, beta, w))
         state = _validate.detached(initial_state)
         output, final_state, aux = _forward_with_aux(seq, state, scale, prepare_backward)
         tensors, ctx.aux_layout = _aux_tensors(aux)
         ctx.save_for_backward(q, k, v, g, beta, w, *tensors)
-        ctx.set_materialize_grads(False)
-        ctx.has_initial_state = initial_state is not None
-        ctx.scale = scale
         return output, final_state
 
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, d_output, d_final_state):
         q, k, v, g, beta, w, *saved = ctx.saved_tensors
+        if ctx.native and _lib.KERNEL_EVENTS is None:
+            workspace = saved[1] if len(saved) > 1 else None
+            grads = _lib.host().train_backward(q, k, v, g, beta, w, d_output, d_final_state, workspace, saved[0],
+                                               ctx.scale)
+            if grads is not None:
+                return (*grads[:6], grads[6] if ctx.has_initial_state else None, None, None)
         if q.shape[1] == 0:
             empty = tuple(torch.empty_like(x) for x in (q, k, v, g, beta, w))
             d_state = None
@@ -170,6 +190,12 @@ def chunk_gdn2(
     and one behind its backward (``prologue.gate_prologue``).  Returns ``(o, S_T)`` or ``(o, None)``.
     """
 
+    if _lib.KERNEL_EVENTS is None and isinstance(q, torch.Tensor) and q.is_cuda:
+        done = _lib.host().forward(q, k, v, g, beta, w, initial_state, scale, None, None, False,
+                                   _prologue_flags(use_qk_l2norm_in_kernel, use_gate_in_kernel), True,
+                                   chunk_kernels.SCRATCH_BUDGET_BYTES)
+        if done is not None:  # inference, nothing unusual about the arguments
+            return done if output_final_state else (done[0], None)
     output_scale = float(scale) if scale is not None else 1.0 / math.sqrt(_DIM)
     if not math.isfinite(output_scale):
         raise ValueError("scale must be finite")
@@ -216,6 +242,12 @@ def recurrent_gdn2(
     With the two ``use_*_in_kernel`` keywords (default off) the inputs are raw projections / gate
     pre-activations and the decode and prefill kernels apply the prologue as they load them."""
 
+    if _lib.KERNEL_EVENTS is None and isinstance(q, torch.Tensor) and q.is_cuda:
+        done = _lib.host().forward(q, k, v, g, beta, w, initial_state, scale, out, final_state_out,
+                                   inplace_final_state, _prologue_flags(use_qk_l2norm_in_kernel, use_gate_in_kernel),
+                                   False, chunk_kernels.SCRATCH_BUDGET_BYTES)
+        if done is not None:
+            return done
     return token_forward(q, k, v, g, beta, w, initial_state, scale=scale, out=out,
                          final_state_out=final_state_out, inplace_final_state=inplace_final_state,
                          prologue=_prologue_flags(use_qk_l2norm_in_kernel, use_gate_in_kernel))

@@ -20,6 +20,8 @@ from . import _lib, _validate
 
 
 def _launch_forward(q, k, g, beta, w, normalize_qk, activate_gates):
+    # beta / w / v share the value-shaped layout checks of the primitive; v is not touched here
+    _validate.sequence_inputs(q, k, w, g, beta, w, need_alignment=True)
     batch, time, heads, _ = q.shape
     rows = (batch, time, heads)
     outs = [torch.empty_like(t) if on else t for t, on in
@@ -45,8 +47,14 @@ def _launch_forward(q, k, g, beta, w, normalize_qk, activate_gates):
 class _GatePrologue(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, g, beta, w, normalize_qk: bool, activate_gates: bool):
-        raw = tuple(_validate.detached(t) for t in (q, k, g, beta, w))
-        outs, inv_q, inv_k = _launch_forward(*raw, normalize_qk, activate_gates)
+        done = None
+        if _lib.KERNEL_EVENTS is None:
+            done = _lib.host().prologue_forward(q, k, g, beta, w, normalize_qk, activate_gates)
+        if done is not None:
+            *outs, inv_q, inv_k = done
+        else:
+            raw = tuple(_validate.detached(t) for t in (q, k, g, beta, w))
+            outs, inv_q, inv_k = _launch_forward(*raw, normalize_qk, activate_gates)
         ctx.normalize_qk, ctx.activate_gates = normalize_qk, activate_gates
         saved = [q, k, g, beta, w]
         if normalize_qk:
@@ -63,6 +71,11 @@ class _GatePrologue(torch.autograd.Function):
         q, k, g, beta, w, *inv = ctx.saved_tensors
         n, a = ctx.normalize_qk, ctx.activate_gates
         batch, time, heads, _ = q.shape
+        if _lib.KERNEL_EVENTS is None:
+            done = _lib.host().prologue_backward(q, k, g, beta, w, *(inv if n else (None, None)), dq, dk, dg, dbeta, dw,
+                                                 n, a)
+            if done is not None:
+                return (*done, None, None)
 
         def ready(grad, like):
             if grad is None:
@@ -98,9 +111,8 @@ def gate_prologue(q, k, g, beta, w, *, normalize_qk: bool = True, activate_gates
 
     if not (normalize_qk or activate_gates):
         return q, k, g, beta, w
-    # beta / w / v share the value-shaped layout checks of the primitive; v is not touched here
-    _validate.sequence_inputs(q, k, w, g, beta, w, need_alignment=True)
-    wants_grad = torch.is_grad_enabled() and any(t.requires_grad for t in (q, k, g, beta, w))
+    wants_grad = torch.is_grad_enabled() and any(
+        isinstance(t, torch.Tensor) and t.requires_grad for t in (q, k, g, beta, w))
     if wants_grad:
         return _GatePrologue.apply(q, k, g, beta, w, bool(normalize_qk), bool(activate_gates))
     raw = tuple(_validate.detached(t) for t in (q, k, g, beta, w))
