@@ -38,42 +38,53 @@ namespace {
 // ---------------------------------------------------------------------------------------------
 // prep kernel
 // ---------------------------------------------------------------------------------------------
-// 512 threads: warp = 4-token group tg (0..15), lane = 4-channel group c4 (0..31).  A thread owns
-// 4 tokens x 4 channels: one 16-byte chunk of every natural tile row (tokens x channels) and one
-// 16-byte chunk (4 tokens) per channel of every transposed tile (channels x tokens).
-// Shared-memory tiles written this way use padded strides so that the 8 lanes of a store phase hit
-// 8 different 16-byte bank groups: natural tiles CS = 144 (chunk stride), transposed tiles RS = 2064.
-constexpr int kPrepThreads = 512;
+// Persistent, two CTAs of 256 threads per SM.  A unit is a chain of a dozen phases of about a microsecond,
+// each waiting for the one before (loads, exponentials, tensor cores, the blocked inverse, stores): with one
+// CTA per SM the issue slots were 35 % busy and a unit took 10.5 us.  Two CTAs fill each other's waits; for
+// that a CTA has to live in 113 KB, so the Gram operands are built and multiplied in two halves of 64
+// channels, and everything else shares their place.
+//
+// A thread owns 4 tokens x 4 channels of each half: token group tg = 2 warp + lane / 16, channel group
+// cl = lane % 16: one 16-byte chunk of every tile row (tokens x channels).  The Gram tiles use a padded chunk
+// stride (CS = 144), so that the 8 lanes of a store phase hit 8 different 16-byte bank groups.
+constexpr int kPrepThreads = 256;
+constexpr int kHalf = 64;         // channels per half
 constexpr int kLd = 68;           // leading dimension of the fp32 64x64 scratch matrices (16-byte rows, banks shift by 4)
 constexpr int kLdW = 20;          // leading dimension of the transposed 16x16 block products
-constexpr int kCsN = 144;         // natural tiles: byte stride between 16-byte column chunks
-constexpr int kRsN = 32 * kCsN;   // natural tiles of 128 fp32 columns: byte stride between 8-row groups (4608)
-constexpr int kRsT = 2064;        // transposed tiles (64 fp32 columns): byte stride between 8-row groups
-constexpr int kTileT = 16 * kRsT; // 33024 bytes
+constexpr int kCsN = 144;         // Gram tiles: byte stride between 16-byte column chunks
+constexpr int kRsN = 16 * kCsN;   // Gram tiles of 64 fp32 columns: byte stride between 8-row groups (2304)
+constexpr float kLog2e = 1.4426950408889634f;
+
+// One region, by phase (bytes):
+//   inputs       g at 0 (16 or 32 KiB), then k, q, beta (16 KiB each), dense [64][128] rows by TMA
+//   Gram halves  A operand [E_anchored ; Q_anchored] X[r = 128][c = k], B operands K^I X[r = j < 16 (I + 1)][c = k]
+//   E            E[j][k], tf32, MN-major operand: 4 swizzled slabs of 32 channels x 64 lines (tc05.cuh), the
+//                second half's two slabs first: they replace Gram operands that have been multiplied, the first
+//                half's are behind the Gram operands and written with them
+//   inverse      fp32 T, T^T, L, block products.  The tf32 T tile replaces L.
+// The next unit's g and q arrive over T, T^T and the block products under the last MMA, k and beta after it.
+constexpr int kOffGramA = 0, kOffGramB = 16 * kRsN;                     // 36864 + 46080
+constexpr int kOffTn = 0, kOffTc = kOffTn + 64 * kLd * 4;               // 17408 each
+constexpr int kOffLn = kOffTc + 64 * kLd * 4, kOffTmat = kOffLn;
+constexpr int kOffWt = kOffLn + 64 * kLd * 4;
+constexpr int kOffE = 67584;                                            // 32768
+constexpr int kOffInG = 0, kOffInK = kOffLn, kOffInQ = kOffInK + 16384, kOffInBeta = kOffInQ + 16384;
+constexpr int kPrepRegion = kOffE + 32768;                              // 100352
+static_assert(kOffWt + 2 * 16 * kLdW * 4 <= kOffInBeta && kOffGramB + 20 * kRsN <= kOffE + 16384, "prep region");
+static_assert(kOffInG + 32768 <= kOffInK && kOffInQ >= kOffTmat + 16384 && kOffInBeta + 16384 <= kPrepRegion, "prep inputs");
+static_assert(kOffInK % 128 == 0 && kOffE % 1024 == 0, "alignment of TMA destinations and swizzled slabs");
 
 struct PrepSmem {
-  // region 1: tf32 Gram A operand [E_anchored ; Q_anchored] X[r = 128][c = k];
-  //           after the Gram products: fp32 scratch for L, T, A_qk and the block products
-  alignas(128) uint8_t gram_a[16 * kRsN];               // 73728
-  // region 2: tf32 Gram B operands K^I X[r = j < 16 (I + 1)][c = k]: 2 (I + 1) row groups each;
-  //           after the Gram products: E^T, tile X[r = channel][c = j]
-  alignas(128) uint8_t gram_b[20 * kRsN];               // 92160
-  alignas(128) uint8_t tmat[16384];    // T tile X[r = i][c = j], tf32, RS 2048
+  alignas(1024) uint8_t region[kPrepRegion];
   float part[16][kDim];                // per 4-token group partial sums -> exclusive prefixes
   float gend[kDim];
-  float nrm[16][2][4][2];              // fused prologue: per (warp, token group, token) sums of q^2, k^2 over 64 channels
+  float nrm[16][4][2];                 // fused prologue: reciprocal norms of q, k per token
   alignas(8) uint64_t bar[2];          // MMA commits
-  alignas(8) uint64_t bar_ld[2];       // raw inputs of the next unit: {g, k, q} and {beta}
+  alignas(8) uint64_t bar_ld[2];       // raw inputs: {g, q} and {k, beta}
   uint32_t tmem_base;
 };
-// landing zones of the raw [64][128] input tiles of the next unit, in places that are dead by then:
-// g, k, q over the fp32 scratch in region 1 (free once T is written, just before the last MMAs);
-// beta behind E^T in region 2 (free as soon as the Gram products are done, half a unit earlier)
-constexpr int kStageK = 32768, kStageQ = 49152;                     // region 1: g at 0 (16 or 32 KiB)
-constexpr int kStageBeta = 2 * kTileT;                              // region 2, behind the transposed tile
+static_assert(sizeof(PrepSmem) <= 115712, "two prep CTAs must fit an SM");
 constexpr uint32_t kStageTile16 = kChunk * kDim * 2;                // a 16-bit input tile
-static_assert(kStageQ + kStageTile16 <= 16 * kRsN && kStageBeta + kStageTile16 <= 20 * kRsN, "staging exceeds its region");
-static_assert(kStageBeta % 128 == 0, "TMA destinations are 128-byte aligned");
 
 struct PrepParams {
   uint8_t* ws;   // workspace (D, status)
@@ -91,12 +102,13 @@ __device__ __forceinline__ int gram_col(int I) { return (I == 0) ? 0 : (I == 1) 
 // kPro: the instantiation that can apply the layer prologue to raw inputs (p.prologue says which parts);
 // the plain instantiation carries none of that code.
 template <typename T, typename G, typename Seqs, bool kPro = false>
-__global__ void __launch_bounds__(kPrepThreads, 1)
+__global__ void __launch_bounds__(kPrepThreads, 2)
 chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ CUtensorMap tm_g,
                   const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
                   const __grid_constant__ CUtensorMap tm_beta) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
+  uint8_t* const R = sm.region;
   const WsLayout ws{p.n_ch, p.training != 0};
   int* status = reinterpret_cast<int*>(p.ws + ws.off_status());
   BoundedWaiter waiter(status);
@@ -114,76 +126,65 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     mbar_init(&sm.bar_ld[1], 1);
     fence_mbar_init();
   }
+  const int tg = 2 * warp + (lane >> 4), cl = lane & 15;
+  const int mb = tg >> 2;                     // 16-token block of this thread's tokens
+  const int q4 = warp & 3, part = warp >> 2;  // TMEM lane quadrant of this warp, and its half of the columns
 
-  // a warp holds two neighbouring token groups x 16 channel groups: a store of one token row per lane
-  // then touches 16 lines of a blocked tile (two 16-byte pieces each) instead of 32
-  const int tg = 2 * (warp >> 1) + (lane >> 4), c4 = 16 * (warp & 1) + (lane & 15);
-  const int kc0 = 4 * c4;
-  const int q4 = warp & 3, part = warp >> 2;  // TMEM lane quadrant of this warp, and its share of the columns
-
-  // unit -> TMA coordinates (channel 0, head, first token row of the chunk)
+  // unit -> head, first token row of the chunk, tokens that exist
   const int heads = p.H, n_ch = int(p.n_ch);
-  constexpr uint32_t kStageTileG = kChunk * kDim * sizeof(G);
-  auto locate = [&](int ch_, int& h_, int& row_, int& valid_) {
+  struct Place { int h, row, valid; };
+  auto locate = [&](int ch_) {
     const int chunk = int(uint32_t(ch_) / uint32_t(heads));
-    h_ = ch_ - chunk * heads;
     const SeqInfo sq = seqs.at(seqs.find(chunk));
     const int t_ = (chunk - sq.chunk0) * kChunk;
-    row_ = int(sq.row0) + t_;
-    valid_ = min(kChunk, sq.len - t_);
+    return Place{ch_ - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
   };
-  auto issue_gkq = [&](int h_, int row_) {
-    mbar_arrive_expect_tx(&sm.bar_ld[0], kStageTileG + 2 * kStageTile16);
-    tma_load_3d(sm.gram_a, &tm_g, 0, h_, row_, &sm.bar_ld[0]);
-    tma_load_3d(sm.gram_a + kStageK, &tm_k, 0, h_, row_, &sm.bar_ld[0]);
-    tma_load_3d(sm.gram_a + kStageQ, &tm_q, 0, h_, row_, &sm.bar_ld[0]);
+  auto issue_gq = [&](const Place& at) {
+    mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)) + kStageTile16);
+    tma_load_3d(R + kOffInG, &tm_g, 0, at.h, at.row, &sm.bar_ld[0]);
+    tma_load_3d(R + kOffInQ, &tm_q, 0, at.h, at.row, &sm.bar_ld[0]);
   };
-  auto issue_beta = [&](int h_, int row_) {
-    mbar_arrive_expect_tx(&sm.bar_ld[1], kStageTile16);
-    tma_load_3d(sm.gram_b + kStageBeta, &tm_beta, 0, h_, row_, &sm.bar_ld[1]);
+  auto issue_kb = [&](const Place& at) {
+    mbar_arrive_expect_tx(&sm.bar_ld[1], 2 * kStageTile16);
+    tma_load_3d(R + kOffInK, &tm_k, 0, at.h, at.row, &sm.bar_ld[1]);
+    tma_load_3d(R + kOffInBeta, &tm_beta, 0, at.h, at.row, &sm.bar_ld[1]);
   };
-  int h_next = 0, row_next = 0, valid_next = kChunk;
-  if (int(blockIdx.x) < n_ch) locate(int(blockIdx.x), h_next, row_next, valid_next);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   if (tid == 0 && int(blockIdx.x) < n_ch) {
-    issue_gkq(h_next, row_next);
-    issue_beta(h_next, row_next);
+    const Place at = locate(int(blockIdx.x));
+    issue_gq(at);
+    issue_kb(at);
   }
   const uint32_t tb = sm.tmem_base;
   const uint32_t leader = elect_leader();
-  // this thread's 8- or 16-byte piece of row 4 tg + e of a staged [64][128] tile
-  auto staged = [&](const uint8_t* tile, int e, int elem_bytes) {
-    return tile + ((4 * tg + e) * kDim + kc0) * elem_bytes;
+  // this thread's 8- or 16-byte piece of row 4 tg + e, half hf, of a [64][128] input tile
+  auto staged = [&](int tile, int e, int hf, int elem_bytes) {
+    return R + tile + ((4 * tg + e) * kDim + kHalf * hf + 4 * cl) * elem_bytes;
   };
+  const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
+  const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
+  using RawG = typename Raw4<G>::type;
+  using RawT = typename Raw4<T>::type;
 
   uint32_t par = 0;
   for (int ch = int(blockIdx.x); ch < n_ch; ch += int(gridDim.x), par ^= 1u) {
   const int ch_next = ch + int(gridDim.x);
   // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
   // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
-  const int n_valid = valid_next;
+  const int n_valid = locate(ch).valid;
   const bool partial = n_valid < kChunk;
-  if (ch_next < n_ch) locate(ch_next, h_next, row_next, valid_next);
-  // ---- the raw inputs were brought in while the previous unit was finishing; the log-decay is
-  // consumed first: the prefix sums below need it alone ------------------------------------------------
-  float Gc[4][4], kk[4][4], qq[4][4], bb[4][4];
-  {
-    using RawG = typename Raw4<G>::type;
-    using RawT = typename Raw4<T>::type;
+  // ---- inputs into registers: log-decay sums of this thread's tokens (in units of ln 2: a decay is one ex2),
+  // k, q and beta still packed
+  float Gc[2][4][4];
+  RawT rk[2][4], rq[2][4], rb[2][4];
+  waiter.wait(&sm.bar_ld[0], par);
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
     RawG rg[4];
-    RawT rk[4], rq[4];
-    waiter.wait(&sm.bar_ld[0], par);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) rg[e] = *reinterpret_cast<const RawG*>(staged(sm.gram_a, e, sizeof(G)));
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      rk[e] = *reinterpret_cast<const RawT*>(staged(sm.gram_a + kStageK, e, 2));
-      rq[e] = *reinterpret_cast<const RawT*>(staged(sm.gram_a + kStageQ, e, 2));
-    }
-    const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
-    const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
+    for (int e = 0; e < 4; ++e) rg[e] = *reinterpret_cast<const RawG*>(staged(kOffInG, e, hf, sizeof(G)));
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       float gv[4];
@@ -192,221 +193,250 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       for (int f = 0; f < 4; ++f) {
         if (pro_gate) gv[f] = prologue_log_decay(gv[f]);
         if (partial && 4 * tg + e >= n_valid) gv[f] = 0.f;
-        Gc[e][f] = (e ? Gc[e - 1][f] : 0.f) + gv[f];
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) sm.part[tg][kc0 + f] = Gc[3][f];
-    if (pro_norm) {
-      // sums of q^2 and k^2 of this thread's four tokens over its four channels, then over the 16 lanes
-      // that hold the other channels of the same tokens in this warp (the other 64 channels are in the
-      // neighbouring warp: combined after the barrier)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        float kf[4], qf[4];
-        unpack4<T>(rk[e], kf);
-        unpack4<T>(rq[e], qf);
-        float sq = qf[0] * qf[0] + qf[1] * qf[1] + qf[2] * qf[2] + qf[3] * qf[3];
-        float sk = kf[0] * kf[0] + kf[1] * kf[1] + kf[2] * kf[2] + kf[3] * kf[3];
-#pragma unroll
-        for (int off = 1; off < 16; off <<= 1) {
-          sq += __shfl_xor_sync(0xffffffffu, sq, off);
-          sk += __shfl_xor_sync(0xffffffffu, sk, off);
-        }
-        if ((lane & 15) == 0) {
-          sm.nrm[warp][lane >> 4][e][0] = sq;
-          sm.nrm[warp][lane >> 4][e][1] = sk;
-        }
-      }
-    }
-    waiter.wait(&sm.bar_ld[1], par);
-    RawT rb[4];
-#pragma unroll
-    for (int e = 0; e < 4; ++e) rb[e] = *reinterpret_cast<const RawT*>(staged(sm.gram_b + kStageBeta, e, 2));
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      unpack4<T>(rk[e], kk[e]);
-      unpack4<T>(rq[e], qq[e]);
-      unpack4<T>(rb[e], bb[e]);
-      if (pro_norm) {
-        const float inv_q = rsqrtf(sm.nrm[warp][lane >> 4][e][0] + sm.nrm[warp ^ 1][lane >> 4][e][0] + kPrologueEps);
-        const float inv_k = rsqrtf(sm.nrm[warp][lane >> 4][e][1] + sm.nrm[warp ^ 1][lane >> 4][e][1] + kPrologueEps);
-#pragma unroll
-        for (int f = 0; f < 4; ++f) { qq[e][f] *= inv_q; kk[e][f] *= inv_k; }
-      }
-      if (pro_gate) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) bb[e][f] = prologue_sigmoid(bb[e][f]);
-      }
-      if (partial && 4 * tg + e >= n_valid) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) kk[e][f] = qq[e][f] = bb[e][f] = 0.f;
+        Gc[hf][e][f] = e ? fmaf(gv[f], kLog2e, Gc[hf][e - 1][f]) : gv[f] * kLog2e;
       }
     }
   }
+  waiter.wait(&sm.bar_ld[1], par);
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      rk[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInK, e, hf, 2));
+      rq[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInQ, e, hf, 2));
+      rb[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInBeta, e, hf, 2));
+      if (partial && 4 * tg + e >= n_valid) rk[hf][e] = rq[hf][e] = rb[hf][e] = RawT{};
+    }
+  }
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    *reinterpret_cast<float4*>(&sm.part[tg][kHalf * hf + 4 * cl]) =
+        make_float4(Gc[hf][3][0], Gc[hf][3][1], Gc[hf][3][2], Gc[hf][3][3]);
+  }
+  if (pro_norm) {
+    // sums of q^2 and k^2: this thread's channels, then the 16 lanes that hold the others of the same tokens
+    // (as two sums, channels 0..63 and 64..127)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      float sq[2], sk[2];
+#pragma unroll
+      for (int hf = 0; hf < 2; ++hf) {
+        float kf[4], qf[4];
+        unpack4<T>(rk[hf][e], kf);
+        unpack4<T>(rq[hf][e], qf);
+        sq[hf] = qf[0] * qf[0] + qf[1] * qf[1] + qf[2] * qf[2] + qf[3] * qf[3];
+        sk[hf] = kf[0] * kf[0] + kf[1] * kf[1] + kf[2] * kf[2] + kf[3] * kf[3];
+#pragma unroll
+        for (int off = 1; off < 16; off <<= 1) {
+          sq[hf] += __shfl_xor_sync(0xffffffffu, sq[hf], off);
+          sk[hf] += __shfl_xor_sync(0xffffffffu, sk[hf], off);
+        }
+      }
+      if (cl == 0) {
+        sm.nrm[tg][e][0] = rsqrtf(sq[0] + sq[1] + kPrologueEps);
+        sm.nrm[tg][e][1] = rsqrtf(sk[0] + sk[1] + kPrologueEps);
+      }
+    }
+  }
+  __syncthreads();
   if (tid < kDim) {
+    float x[16];
+#pragma unroll
+    for (int t = 0; t < 16; ++t) x[t] = sm.part[t][tid];
     float run = 0.f;
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
-      const float x = sm.part[t][tid];
       sm.part[t][tid] = run;
-      run += x;
+      run += x[t];
     }
     sm.gend[tid] = run;
+    reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(run);
   }
   __syncthreads();
-
-  // ---- per-thread decay table: everything except three exponentials per element comes from here ----
-  const int mb = tg >> 2;  // 16-token block of this thread's tokens
-  float a_mb[4], a_nx[4], e_amb[4], c_nx[4], t_end[4], t_far[2][4];
+  // k and beta of token e, half hf (normalised / activated when the inputs are raw)
+  auto key = [&](int hf, int e, float (&x)[4]) {
+    unpack4<T>(rk[hf][e], x);
+    if (pro_norm) {
+      const float inv = sm.nrm[tg][e][1];
 #pragma unroll
-  for (int f = 0; f < 4; ++f) {
-    const int kc = kc0 + f;
-    a_mb[f] = sm.part[4 * mb][kc];
-    a_nx[f] = (mb < 3) ? sm.part[4 * (mb + 1)][kc] : sm.gend[kc];
-    e_amb[f] = __expf(a_mb[f]);
-    c_nx[f] = __expf(a_nx[f] - a_mb[f]);  // decay over the whole 16-token block (<= 1)
-    t_end[f] = __expf(sm.gend[kc] - a_nx[f]);
-    // blocks further than the next one: exp(a_I - a_next), I = mb + 2, mb + 3
-    t_far[0][f] = (mb + 2 < 4) ? __expf(sm.part[4 * (mb + 2)][kc] - a_nx[f]) : 0.f;
-    t_far[1][f] = (mb + 3 < 4) ? __expf(sm.part[4 * (mb + 3)][kc] - a_nx[f]) : 0.f;
-  }
-
-  float* tile_q = reinterpret_cast<float*>(p.tiles.q + int64_t(ch) * kTileQ);
-  float* tile_kn = reinterpret_cast<float*>(p.tiles.kn + int64_t(ch) * kTileKn);
-  float ebar[4][4];
-#pragma unroll
-  for (int e = 0; e < 4; ++e) {
-    const int i = 4 * tg + e;
-    float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4];
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const float Gi = Gc[e][f] + sm.part[tg][kc0 + f];
-      const float anchored = __expf(Gi - a_mb[f]);   // <= 1
-      const float own = __expf(a_mb[f] - Gi);        // >= 1, bounded by the 16-token contract
-      const float nb = own * c_nx[f];                // exp(a_nx - G_i) <= 1: decay from token i to the next block start
-      const float bk = bb[e][f] * kk[e][f];
-      const float sq = p.scale * qq[e][f];
-      ea[f] = to_tf32_operand(bk * anchored);
-      qa[f] = to_tf32_operand(sq * anchored);
-      ebar[e][f] = to_tf32_operand(bk * anchored * e_amb[f]);
-      qgam[f] = to_tf32_operand(sq * anchored * e_amb[f]);
-      kown[f] = to_tf32_operand(kk[e][f] * own);
-      knb[f] = kk[e][f] * nb;
-      ktail[f] = to_tf32_operand(knb[f] * t_end[f]);
+      for (int f = 0; f < 4; ++f) x[f] *= inv;
     }
-    // Gram A operand rows i (erase) and 64 + i (query), tf32, K-major, padded chunk stride
-    *reinterpret_cast<float4*>(sm.gram_a + (i >> 3) * kRsN + c4 * kCsN + (i & 7) * 16) =
-        make_float4(ea[0], ea[1], ea[2], ea[3]);
-    *reinterpret_cast<float4*>(sm.gram_a + ((64 + i) >> 3) * kRsN + c4 * kCsN + (i & 7) * 16) =
-        make_float4(qa[0], qa[1], qa[2], qa[3]);
-    // Gram B operands: token i is a column of every row block I >= its own
-    const uint32_t row_off = (i >> 3) * kRsN + c4 * kCsN + (i & 7) * 16;
-    *reinterpret_cast<float4*>(sm.gram_b + gram_b_offset(mb) + row_off) =
-        make_float4(kown[0], kown[1], kown[2], kown[3]);
-    if (mb + 1 < 4) {
-      *reinterpret_cast<float4*>(sm.gram_b + gram_b_offset(mb + 1) + row_off) =
-          make_float4(to_tf32_operand(knb[0]), to_tf32_operand(knb[1]), to_tf32_operand(knb[2]), to_tf32_operand(knb[3]));
-    }
+  };
+  auto gate = [&](int hf, int e, float (&x)[4]) {
+    unpack4<T>(rb[hf][e], x);
+    if (pro_gate) {
 #pragma unroll
-    for (int far = 0; far < 2; ++far) {
-      if (mb + 2 + far < 4) {
-        *reinterpret_cast<float4*>(sm.gram_b + gram_b_offset(mb + 2 + far) + row_off) =
-            make_float4(to_tf32_operand(knb[0] * t_far[far][0]), to_tf32_operand(knb[1] * t_far[far][1]),
-                        to_tf32_operand(knb[2] * t_far[far][2]), to_tf32_operand(knb[3] * t_far[far][3]));
+      for (int f = 0; f < 4; f += 2) prologue_sigmoid2(x[f], x[f + 1]);
+    }
+  };
+
+  // ---- Gram products P_I = [E_a ; Q_a] (K^I)^T on the tensor cores, 64 channels at a time ------------------
+  float* const tile_q = reinterpret_cast<float*>(p.tiles.q + int64_t(ch) * kTileQ);
+  float* const tile_kn = reinterpret_cast<float*>(p.tiles.kn + int64_t(ch) * kTileKn);
+  // E[i][channels of this thread]: 16 bytes of line i of a slab, 32-byte pieces permuted by the line
+  auto store_e = [&](int hf, int i, const float (&x)[4]) {
+    uint8_t* slab = R + kOffE + (hf == 0 ? 16384 : 0) + (cl >> 3) * 8192;
+    *reinterpret_cast<float4*>(slab + i * 128 + ((((cl & 7) >> 1) ^ (i & 3)) << 5) + (cl & 1) * 16) =
+        make_float4(x[0], x[1], x[2], x[3]);
+  };
+  float e_second[4][4];
+#pragma unroll
+  for (int hf = 0; hf < 2; ++hf) {
+    const int kc0 = kHalf * hf + 4 * cl;
+    // decay table of this thread's channels: everything except two exponentials per element comes from here
+    float pre[4], e_amb[4], c_nx[4], t_end[4], t_far[2][4];
+    {
+      const float* end = &sm.gend[kc0];
+      const float* nx = mb + 1 < 4 ? &sm.part[4 * mb + 4][kc0] : end;
+      const float* f0 = mb + 2 < 4 ? &sm.part[4 * mb + 8][kc0] : end;
+      const float* f1 = mb + 3 < 4 ? &sm.part[4 * mb + 12][kc0] : end;
+      float a_mb[4], a_nx[4], a_end[4], a_f0[4], a_f1[4];
+      load4(&sm.part[tg][kc0], true, pre);
+      load4(&sm.part[4 * mb][kc0], true, a_mb);
+      load4(nx, true, a_nx);
+      load4(end, true, a_end);
+      load4(f0, true, a_f0);
+      load4(f1, true, a_f1);
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        pre[f] -= a_mb[f];                             // sum from the start of the 16-token block
+        e_amb[f] = exp2_approx(a_mb[f]);
+        c_nx[f] = exp2_approx(a_nx[f] - a_mb[f]);      // decay over the whole 16-token block (<= 1)
+        t_end[f] = exp2_approx(a_end[f] - a_nx[f]);
+        t_far[0][f] = exp2_approx(a_f0[f] - a_nx[f]);  // blocks further than the next one: exp(a_I - a_next)
+        t_far[1][f] = exp2_approx(a_f1[f] - a_nx[f]);
       }
     }
-    // token-major tiles Q[i][k] and Kn[i][k]: the 16 lanes of a token write 256 consecutive bytes
-    *reinterpret_cast<float4*>(tile_q + i * kDim + kc0) = make_float4(qgam[0], qgam[1], qgam[2], qgam[3]);
-    *reinterpret_cast<float4*>(tile_kn + i * kDim + kc0) = make_float4(ktail[0], ktail[1], ktail[2], ktail[3]);
-  }
-  if (tid < kDim) {
-    reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = __expf(sm.gend[tid]);
-  }
-  fence_async_smem();
-  tc_fence_before();
-  __syncthreads();
-
-  // ---- Gram products on the tensor cores: P_I = [E_a ; Q_a] (K^I)^T -----------------------------
-  if (warp == 0) {
-    tc_fence_after();
-    // the four anchored copies K^0 .. K^3 are stacked (16 + 32 + 48 + 64 = 160 rows) and their products
-    // sit side by side in TMEM, so one N = 160 instruction per k-step reads the A tile once for all four
-    const uint32_t id = idesc(128, 160, kFmtTF32, kMajorK, kMajorK);
-    const uint32_t a0 = smem_u32(sm.gram_a), b0 = smem_u32(sm.gram_b);
+    if (hf == 1) waiter.wait(&sm.bar[0], 0);  // the first half's operands have been multiplied
 #pragma unroll
-    for (int ks = 0; ks < 16; ++ks) {
-      mma_tf32_ss(tb, smem_desc(a0 + ks * 2 * kCsN, kCsN, kRsN), smem_desc(b0 + ks * 2 * kCsN, kCsN, kRsN), id,
-                  ks > 0 ? 1u : 0u, leader);
+    for (int e = 0; e < 4; ++e) {
+      const int i = 4 * tg + e;
+      float kk[4], bb[4], qq[4];
+      key(hf, e, kk);
+      gate(hf, e, bb);
+      unpack4<T>(rq[hf][e], qq);
+      if (pro_norm) {
+        const float inv = sm.nrm[tg][e][0];
+#pragma unroll
+        for (int f = 0; f < 4; ++f) qq[f] *= inv;
+      }
+      float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4], eb[4];
+#pragma unroll
+      for (int f = 0; f < 4; ++f) {
+        const float Gi = Gc[hf][e][f] + pre[f];
+        const float anchored = exp2_approx(Gi);        // <= 1
+        const float own = exp2_approx(-Gi);            // >= 1, bounded by the 16-token contract
+        const float nb = own * c_nx[f];                // exp(a_nx - G_i) <= 1: decay from token i to the next block start
+        const float bk = bb[f] * kk[f];
+        const float sq = p.scale * qq[f];
+        ea[f] = to_tf32_operand(bk * anchored);
+        qa[f] = to_tf32_operand(sq * anchored);
+        eb[f] = to_tf32_operand(bk * anchored * e_amb[f]);
+        qgam[f] = to_tf32_operand(sq * anchored * e_amb[f]);
+        kown[f] = to_tf32_operand(kk[f] * own);
+        knb[f] = kk[f] * nb;
+        ktail[f] = to_tf32_operand(knb[f] * t_end[f]);
+      }
+      // Gram A operand rows i (erase) and 64 + i (query), tf32, K-major, padded chunk stride
+      const uint32_t row_off = (i >> 3) * kRsN + cl * kCsN + (i & 7) * 16;
+      *reinterpret_cast<float4*>(R + kOffGramA + row_off) = make_float4(ea[0], ea[1], ea[2], ea[3]);
+      *reinterpret_cast<float4*>(R + kOffGramA + 8 * kRsN + row_off) = make_float4(qa[0], qa[1], qa[2], qa[3]);
+      // Gram B operands: token i is a column of every row block I >= its own
+      *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb) + row_off) =
+          make_float4(kown[0], kown[1], kown[2], kown[3]);
+      if (mb + 1 < 4) {
+        *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb + 1) + row_off) =
+            make_float4(to_tf32_operand(knb[0]), to_tf32_operand(knb[1]), to_tf32_operand(knb[2]), to_tf32_operand(knb[3]));
+      }
+#pragma unroll
+      for (int far = 0; far < 2; ++far) {
+        if (mb + 2 + far < 4) {
+          *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb + 2 + far) + row_off) =
+              make_float4(to_tf32_operand(knb[0] * t_far[far][0]), to_tf32_operand(knb[1] * t_far[far][1]),
+                          to_tf32_operand(knb[2] * t_far[far][2]), to_tf32_operand(knb[3] * t_far[far][3]));
+        }
+      }
+      if (hf == 0) {
+        store_e(0, i, eb);
+      } else {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) e_second[e][f] = eb[f];
+      }
+      // token-major tiles Q[i][k] and Kn[i][k]: the 16 lanes of a token write 256 consecutive bytes
+      *reinterpret_cast<float4*>(tile_q + i * kDim + kc0) = make_float4(qgam[0], qgam[1], qgam[2], qgam[3]);
+      *reinterpret_cast<float4*>(tile_kn + i * kDim + kc0) = make_float4(ktail[0], ktail[1], ktail[2], ktail[3]);
     }
-    mma_commit(&sm.bar[0], leader);
-  }
-  waiter.wait(&sm.bar[0], par);
-  tc_fence_after();
-  // the Gram operands are dead: region 1 becomes fp32 scratch, region 2 receives E^T
-  float* Ln = reinterpret_cast<float*>(sm.gram_a);           // [64][kLd]   L
-  float* Tn = Ln + 64 * kLd;                                  // [64][kLd]   T
-  float* Tc = Tn + 64 * kLd;                                  // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
-  float* Wt = Tc + 64 * kLd;                                  // [3][16][kLdW] block products, transposed
-  static_assert((3 * 64 * kLd + 3 * 16 * kLdW) * 4 <= 16 * kRsN, "fp32 scratch exceeds the Gram A region");
-  uint8_t* et_tile = sm.gram_b;                               // E^T  X[r = k][c = j], tf32, RS kRsT
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) {
+      tc_fence_after();
+      // the four anchored copies K^0 .. K^3 are stacked (16 + 32 + 48 + 64 = 160 rows) and their products
+      // sit side by side in TMEM, so one N = 160 instruction per k-step reads the A tile once for all four
+      const uint32_t id = idesc(128, 160, kFmtTF32, kMajorK, kMajorK);
+      const uint32_t a0 = smem_u32(R + kOffGramA), b0 = smem_u32(R + kOffGramB);
 #pragma unroll
-  for (int f = 0; f < 4; ++f) {
-    *reinterpret_cast<float4*>(et_tile + blk_off<4>(kc0 + f, 4 * tg, kRsT, 128)) =
-        make_float4(ebar[0][f], ebar[1][f], ebar[2][f], ebar[3][f]);
+      for (int ks = 0; ks < 8; ++ks) {
+        mma_tf32_ss(tb, smem_desc(a0 + ks * 2 * kCsN, kCsN, kRsN), smem_desc(b0 + ks * 2 * kCsN, kCsN, kRsN), id,
+                    (hf | ks) > 0 ? 1u : 0u, leader);
+      }
+      mma_commit(&sm.bar[0], leader);
+    }
   }
+  waiter.wait(&sm.bar[0], 1);
+  tc_fence_after();
+  // the Gram operands are dead: the region becomes fp32 scratch and the second half of E
+  float* Tn = reinterpret_cast<float*>(R + kOffTn);           // [64][kLd]   T
+  float* Tc = reinterpret_cast<float*>(R + kOffTc);           // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
+  float* Ln = reinterpret_cast<float*>(R + kOffLn);           // [64][kLd]   L
+  float* Wt = reinterpret_cast<float*>(R + kOffWt);           // [2][16][kLdW] block products, transposed
+#pragma unroll
+  for (int e = 0; e < 4; ++e) store_e(1, 4 * tg + e, e_second[e]);
   {
     // pull L (rows 0..63) into fp32 scratch and A_qk (rows 64..127) into the workspace;
-    // the four warps of a quadrant take 16 columns each
+    // the two warps of a quadrant take 32 columns each
     const int r = 32 * q4 + lane;  // TMEM lane = row of [E_a ; Q_a]
     const int i = r & 63;
     const int I_lo = (q4 & 1) * 2;
     const int my_I = I_lo + (lane >> 4);
-    const int c0 = 16 * part;
     float* tile_at = reinterpret_cast<float*>(p.tiles.at + int64_t(ch) * kTileAt);
-    uint32_t lo[16], hi[16];
-    const bool need_lo = c0 < 16 * (I_lo + 1), need_hi = c0 < 16 * (I_lo + 2);
-    if (need_lo) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo) + c0), lo);
-    if (need_hi) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo + 1) + c0), hi);
-    tmem_wait_ld();
-    float vals[16];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
-      const bool mine_lo = (my_I == I_lo);
-      const float x = mine_lo ? (need_lo ? __uint_as_float(lo[j]) : 0.f) : (need_hi ? __uint_as_float(hi[j]) : 0.f);
-      const int col = c0 + j;
-      vals[j] = (r < 64) ? ((col < i) ? x : 0.f) : ((col <= i) ? to_tf32_operand(x) : 0.f);
-    }
-    if (r < 64) {
+    for (int sub = 0; sub < 2; ++sub) {
+      const int c0 = 32 * part + 16 * sub;
+      uint32_t lo[16], hi[16];
+      const bool need_lo = c0 < 16 * (I_lo + 1), need_hi = c0 < 16 * (I_lo + 2);
+      if (need_lo) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo) + c0), lo);
+      if (need_hi) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo + 1) + c0), hi);
+      tmem_wait_ld();
+      float vals[16];
 #pragma unroll
-      for (int j4 = 0; j4 < 4; ++j4) {
-        *reinterpret_cast<float4*>(Ln + i * kLd + c0 + 4 * j4) =
-            make_float4(vals[4 * j4], vals[4 * j4 + 1], vals[4 * j4 + 2], vals[4 * j4 + 3]);
+      for (int j = 0; j < 16; ++j) {
+        const bool mine_lo = (my_I == I_lo);
+        const float x = mine_lo ? (need_lo ? __uint_as_float(lo[j]) : 0.f) : (need_hi ? __uint_as_float(hi[j]) : 0.f);
+        const int col = c0 + j;
+        vals[j] = (r < 64) ? ((col < i) ? x : 0.f) : ((col <= i) ? to_tf32_operand(x) : 0.f);
       }
-    } else {
-      // A_qk leaves transposed, At[j][i]: the 32 lanes of a warp (rows i) fill one 128-byte line per column j;
-      // the quadrant j >= 32, i < 32 is zero and stays unwritten (nobody reads it)
-      if (!(c0 >= 32 && i < 32)) {
+      if (r < 64) {
+#pragma unroll
+        for (int j4 = 0; j4 < 4; ++j4) {
+          *reinterpret_cast<float4*>(Ln + i * kLd + c0 + 4 * j4) =
+              make_float4(vals[4 * j4], vals[4 * j4 + 1], vals[4 * j4 + 2], vals[4 * j4 + 3]);
+        }
+      } else if (!(c0 >= 32 && i < 32)) {
+        // A_qk leaves transposed, At[j][i]: the 32 lanes of a warp (rows i) fill one 128-byte line per column j;
+        // the quadrant j >= 32, i < 32 is zero and stays unwritten (nobody reads it)
 #pragma unroll
         for (int j = 0; j < 16; ++j) tile_at[(c0 + j) * kChunk + i] = vals[j];
       }
     }
   }
-  for (int e = tid; e < 64 * kLd / 4; e += kPrepThreads) {
-    reinterpret_cast<float4*>(Tn)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-    reinterpret_cast<float4*>(Tc)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
   tc_fence_before();
   __syncthreads();
-  // the Gram operands are dead: beta of the next unit starts to arrive
-  if (tid == 0 && ch_next < n_ch) issue_beta(h_next, row_next);
 
   // ---- T = (I + L)^-1, blocked: 16x16 diagonal blocks by substitution, the rest by block products.
   // T is kept in both orientations (Tn row-major, Tc column-major) and the block products W transposed,
-  // so that both factors of every inner product are read as 16-byte vectors along the summed index.
+  // so that both factors of every inner product are read as 16-byte vectors along the summed index.  Blocks
+  // above the diagonal are not stored, except the two that the 32 x 32 products read as zeros.
   auto ld4 = [](const float* ptr) { return *reinterpret_cast<const float4*>(ptr); };
   if (tid < 64) {
     const int I = tid >> 4, cc = tid & 15;
@@ -431,145 +461,156 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       *reinterpret_cast<float4*>(Tc + (16 * I + cc) * kLd + 16 * I + 4 * r4) =
           make_float4(x[4 * r4], x[4 * r4 + 1], x[4 * r4 + 2], x[4 * r4 + 3]);
     }
+  } else if (tid < 192) {
+    const int e = tid & 63, r = e >> 2, c4 = 4 * (e & 3);
+    *reinterpret_cast<float4*>((tid < 128 ? Tc + (16 + r) * kLd : Tn + (32 + r) * kLd + 48) + c4) =
+        make_float4(0.f, 0.f, 0.f, 0.f);
   }
   __syncthreads();
+  // inner product of 4 `quads` values, in four independent chains (latency-bound otherwise)
+  auto dot = [&](const float* a, const float* b, int quads) {
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int m4 = 0; m4 < quads; ++m4) {
+      const float4 x = ld4(a + 4 * m4), y = ld4(b + 4 * m4);
+      acc.x = fmaf(x.x, y.x, acc.x); acc.y = fmaf(x.y, y.y, acc.y);
+      acc.z = fmaf(x.z, y.z, acc.z); acc.w = fmaf(x.w, y.w, acc.w);
+    }
+    return (acc.x + acc.y) + (acc.z + acc.w);
+  };
   // Two levels of 2 x 2 blocking instead of one block row at a time (four barriers fewer):
   // level 1: the 16 x 16 blocks (1,0) and (3,2) complete the two 32 x 32 diagonal inverses P and Q,
   // level 2: T[32.., ..32) = -Q (L[32.., ..32) P).
   // level 1, W = L_IJ T_JJ for (I, J) = (1, 0), (3, 2)
   {
-    const int pair = tid >> 8, r = (tid >> 4) & 15, cc = tid & 15;
-    const int J = 2 * pair, I = J + 1;
-    const float* lrow = Ln + (16 * I + r) * kLd + 16 * J;
-    const float* tcol = Tc + (16 * J + cc) * kLd + 16 * J;
-    // four independent chains (one per vector component): the sum is latency-bound otherwise
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int r = tid >> 4, cc = tid & 15;
+    float w[2];
 #pragma unroll
-    for (int m4 = 0; m4 < 4; ++m4) {
-      const float4 a = ld4(lrow + 4 * m4), b = ld4(tcol + 4 * m4);
-      acc.x = fmaf(a.x, b.x, acc.x); acc.y = fmaf(a.y, b.y, acc.y);
-      acc.z = fmaf(a.z, b.z, acc.z); acc.w = fmaf(a.w, b.w, acc.w);
+    for (int pair = 0; pair < 2; ++pair) {
+      const int J = 2 * pair, I = J + 1;
+      w[pair] = dot(Ln + (16 * I + r) * kLd + 16 * J, Tc + (16 * J + cc) * kLd + 16 * J, 4);
     }
-    Wt[(pair * 16 + cc) * kLdW + r] = (acc.x + acc.y) + (acc.z + acc.w);
+#pragma unroll
+    for (int pair = 0; pair < 2; ++pair) Wt[(pair * 16 + cc) * kLdW + r] = w[pair];
   }
   __syncthreads();
   // level 1, T_IJ = -T_II W
   {
-    const int pair = tid >> 8, r = (tid >> 4) & 15, cc = tid & 15;
-    const int J = 2 * pair, I = J + 1;
-    const float* trow = Tn + (16 * I + r) * kLd + 16 * I;
-    const float* wcol = Wt + (pair * 16 + cc) * kLdW;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int r = tid >> 4, cc = tid & 15;
+    float s[2];
 #pragma unroll
-    for (int m4 = 0; m4 < 4; ++m4) {
-      const float4 a = ld4(trow + 4 * m4), b = ld4(wcol + 4 * m4);
-      acc.x = fmaf(a.x, b.x, acc.x); acc.y = fmaf(a.y, b.y, acc.y);
-      acc.z = fmaf(a.z, b.z, acc.z); acc.w = fmaf(a.w, b.w, acc.w);
+    for (int pair = 0; pair < 2; ++pair) {
+      const int I = 2 * pair + 1;
+      s[pair] = dot(Tn + (16 * I + r) * kLd + 16 * I, Wt + (pair * 16 + cc) * kLdW, 4);
     }
-    const float s = (acc.x + acc.y) + (acc.z + acc.w);
-    Tn[(16 * I + r) * kLd + 16 * J + cc] = -s;
-    Tc[(16 * J + cc) * kLd + 16 * I + r] = -s;
+#pragma unroll
+    for (int pair = 0; pair < 2; ++pair) {
+      const int J = 2 * pair, I = J + 1;
+      Tn[(16 * I + r) * kLd + 16 * J + cc] = -s[pair];
+      Tc[(16 * J + cc) * kLd + 16 * I + r] = -s[pair];
+    }
   }
   __syncthreads();
   // level 2, W2 = L[32.., ..32) P, stored transposed over the (now dead) first 32 rows of L
-  // A thread forms two entries of a column (rows r and r + 16): the column of the right factor is the
-  // expensive read (a different 16-byte piece per lane, four shared-memory wavefronts), the row of the
-  // left factor is a broadcast; the column is read once for both.
+  // A thread forms four entries of a column (rows r, r + 8, r + 16, r + 24): the column of the right factor is
+  // the expensive read (a different 16-byte piece per lane, four shared-memory wavefronts), the rows of the
+  // left factor are broadcasts; the column is read once for all.
+  auto four_rows = [&](const float* rows, const float* col, float (&out)[4]) {
+    float4 acc[4];
+#pragma unroll
+    for (int x = 0; x < 4; ++x) acc[x] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int m4 = 0; m4 < 8; ++m4) {
+      const float4 b = ld4(col + 4 * m4);
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const float4 a = ld4(rows + 8 * x * kLd + 4 * m4);
+        acc[x].x = fmaf(a.x, b.x, acc[x].x); acc[x].y = fmaf(a.y, b.y, acc[x].y);
+        acc[x].z = fmaf(a.z, b.z, acc[x].z); acc[x].w = fmaf(a.w, b.w, acc[x].w);
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) out[x] = (acc[x].x + acc[x].y) + (acc[x].z + acc[x].w);
+  };
   float* W2t = Ln;  // W2t[c][r] = W2[r][c], leading dimension kLd
   {
     const int r = tid >> 5, cc = tid & 31;
-    const float* lrow = Ln + (32 + r) * kLd;
-    const float* pcol = Tc + cc * kLd;
-    float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
+    float w[4];
+    // rows 32.. of L are read here, W2t lives in rows 0..31, which nobody reads any more
+    four_rows(Ln + (32 + r) * kLd, Tc + cc * kLd, w);
 #pragma unroll
-    for (int m4 = 0; m4 < 8; ++m4) {
-      const float4 b = ld4(pcol + 4 * m4);
-      const float4 a0 = ld4(lrow + 4 * m4), a1 = ld4(lrow + 16 * kLd + 4 * m4);
-      acc0.x = fmaf(a0.x, b.x, acc0.x); acc0.y = fmaf(a0.y, b.y, acc0.y);
-      acc0.z = fmaf(a0.z, b.z, acc0.z); acc0.w = fmaf(a0.w, b.w, acc0.w);
-      acc1.x = fmaf(a1.x, b.x, acc1.x); acc1.y = fmaf(a1.y, b.y, acc1.y);
-      acc1.z = fmaf(a1.z, b.z, acc1.z); acc1.w = fmaf(a1.w, b.w, acc1.w);
-    }
-    // rows 32.. of L are read above by other threads; W2t lives in rows 0..31, which nobody reads any more
-    W2t[cc * kLd + r] = (acc0.x + acc0.y) + (acc0.z + acc0.w);
-    W2t[cc * kLd + r + 16] = (acc1.x + acc1.y) + (acc1.z + acc1.w);
+    for (int x = 0; x < 4; ++x) W2t[cc * kLd + r + 8 * x] = w[x];
   }
   __syncthreads();
   // level 2, T[32 + r][c] = -sum_m Q[r][m] W2[m][c]
   {
     const int r = tid >> 5, cc = tid & 31;
-    const float* qrow = Tn + (32 + r) * kLd + 32;
-    const float* wcol = W2t + cc * kLd;
-    float4 acc0 = make_float4(0.f, 0.f, 0.f, 0.f), acc1 = acc0;
+    float s[4];
+    four_rows(Tn + (32 + r) * kLd + 32, W2t + cc * kLd, s);
 #pragma unroll
-    for (int m4 = 0; m4 < 8; ++m4) {
-      const float4 b = ld4(wcol + 4 * m4);
-      const float4 a0 = ld4(qrow + 4 * m4), a1 = ld4(qrow + 16 * kLd + 4 * m4);
-      acc0.x = fmaf(a0.x, b.x, acc0.x); acc0.y = fmaf(a0.y, b.y, acc0.y);
-      acc0.z = fmaf(a0.z, b.z, acc0.z); acc0.w = fmaf(a0.w, b.w, acc0.w);
-      acc1.x = fmaf(a1.x, b.x, acc1.x); acc1.y = fmaf(a1.y, b.y, acc1.y);
-      acc1.z = fmaf(a1.z, b.z, acc1.z); acc1.w = fmaf(a1.w, b.w, acc1.w);
+    for (int x = 0; x < 4; ++x) {
+      Tn[(32 + r + 8 * x) * kLd + cc] = -s[x];
+      Tc[cc * kLd + 32 + r + 8 * x] = -s[x];
     }
-    const float s0 = (acc0.x + acc0.y) + (acc0.z + acc0.w), s1 = (acc1.x + acc1.y) + (acc1.z + acc1.w);
-    Tn[(32 + r) * kLd + cc] = -s0;
-    Tc[cc * kLd + 32 + r] = -s0;
-    Tn[(48 + r) * kLd + cc] = -s1;
-    Tc[cc * kLd + 48 + r] = -s1;
   }
   __syncthreads();
-  // T as tf32 tile X[r = i][c = j] in shared memory (MMA operand), and T^T[j][i] for the scans
+  // T as tf32 tile X[r = i][c = j] over L (MMA operand), and T^T[j][i] for the scans
   {
-    for (int e = tid; e < 64 * 16; e += kPrepThreads) {
-      const int i = e & 63, c4t = e >> 6;  // consecutive threads -> consecutive rows -> contiguous 16-byte chunks
-      const float4 tn = ld4(Tn + i * kLd + 4 * c4t);
-      *reinterpret_cast<float4*>(sm.tmat + blk_off<4>(i, 4 * c4t, 2048, 128)) =
+    float* tile_tt = reinterpret_cast<float*>(p.tiles.tt + int64_t(ch) * kTileTt);
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int e = tid + x * kPrepThreads, i = e & 63, c4t = e >> 6;  // consecutive rows: contiguous 16-byte chunks
+      const float4 tn = (c4t >> 2) <= (i >> 4) ? ld4(Tn + i * kLd + 4 * c4t) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(R + kOffTmat + blk_off<4>(i, 4 * c4t, 2048, 128)) =
           make_float4(to_tf32_operand(tn.x), to_tf32_operand(tn.y), to_tf32_operand(tn.z), to_tf32_operand(tn.w));
     }
-    {
-      float* tile_tt = reinterpret_cast<float*>(p.tiles.tt + int64_t(ch) * kTileTt);
-      for (int e = tid; e < 64 * 16; e += kPrepThreads) {
-        const int j = e >> 4, c4t = e & 15;  // consecutive threads -> consecutive 16-byte pieces of a row
-        if (j >= 32 && c4t < 8) continue;    // the zero quadrant j >= 32, i < 32 stays unwritten
-        const float4 tc = ld4(Tc + j * kLd + 4 * c4t);
-        *reinterpret_cast<float4*>(tile_tt + j * kChunk + 4 * c4t) =
-            make_float4(to_tf32_operand(tc.x), to_tf32_operand(tc.y), to_tf32_operand(tc.z), to_tf32_operand(tc.w));
-      }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const int e = tid + x * kPrepThreads, j = e >> 4, c4t = e & 15;  // consecutive 16-byte pieces of a row
+      if (j >= 32 && c4t < 8) continue;    // the zero quadrant j >= 32, i < 32 stays unwritten
+      const float4 tc = (j >> 4) <= (c4t >> 2) ? ld4(Tc + j * kLd + 4 * c4t) : make_float4(0.f, 0.f, 0.f, 0.f);
+      *reinterpret_cast<float4*>(tile_tt + j * kChunk + 4 * c4t) =
+          make_float4(to_tf32_operand(tc.x), to_tf32_operand(tc.y), to_tf32_operand(tc.z), to_tf32_operand(tc.w));
     }
   }
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
 
-  // ---- Y^T = E^T T^T ------------------------------------------------------------------------------------
+  // ---- Y^T = E^T T^T (A = E[j][k] read MN-major) ------------------------------------------------------------------------------------
   if (warp == 0) {
     tc_fence_after();
-    // region 1 (fp32 scratch) is dead: g, k, q of the next unit land there under the MMAs and the epilogue
-    if (tid == 0 && ch_next < n_ch) issue_gkq(h_next, row_next);
-    const uint32_t t0a = smem_u32(sm.tmat), e0 = smem_u32(et_tile);
-    const uint32_t id_y = idesc(128, 64, kFmtTF32, kMajorK, kMajorK);
+    const uint32_t t0a = smem_u32(R + kOffTmat), e0 = smem_u32(R + kOffE);
+    const uint32_t id_y = idesc(128, 64, kFmtTF32, kMajorMN, kMajorK);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      mma_tf32_ss(tb, smem_desc(e0 + ks * 256, 128, kRsT), smem_desc(t0a + ks * 256, 128, 2048), id_y,
+      mma_tf32_ss(tb, smem_desc_sw128_mn(e0, 8192, ks), smem_desc(t0a + ks * 256, 128, 2048), id_y,
                   ks > 0 ? 1u : 0u, leader);
     }
     mma_commit(&sm.bar[1], leader);
   }
+  if (tid == 32 && ch_next < n_ch) issue_gq(locate(ch_next));
   waiter.wait(&sm.bar[1], par);
   tc_fence_after();
+  if (tid == 32 && ch_next < n_ch) issue_kb(locate(ch_next));
   {
-    // lanes = key channels k, columns = tokens i: each warp takes 16 tokens of its quadrant, a lane 64
+    // lanes = key channels k, columns = tokens i: each warp takes 32 tokens of its quadrant, a lane 128
     // consecutive bytes of row k of Yt[k][i]
-    const int kr = 32 * q4 + lane, c0 = 16 * part;
+    const int kr = (32 * q4 + lane + kHalf) & (kDim - 1), c0 = 32 * part;  // (the second half's slabs come first)
     float* row_yt = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + c0;
-    uint32_t r[16];
-    tmem_ld16(tmem_addr(tb, 32 * q4, c0), r);
+    uint32_t r[32];
+    tmem_ld32(tmem_addr(tb, 32 * q4, c0), r);
     tmem_wait_ld();
-    float y[16];
+    float y[32];
 #pragma unroll
-    for (int j = 0; j < 16; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
-    store_global_32b(row_yt, make_float4(y[0], y[1], y[2], y[3]), make_float4(y[4], y[5], y[6], y[7]));
-    store_global_32b(row_yt + 8, make_float4(y[8], y[9], y[10], y[11]), make_float4(y[12], y[13], y[14], y[15]));
+    for (int j = 0; j < 32; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
+#pragma unroll
+    for (int j = 0; j < 32; j += 8) {
+      store_global_32b(row_yt + j, make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]),
+                       make_float4(y[j + 4], y[j + 5], y[j + 6], y[j + 7]));
+    }
   }
+  tc_fence_before();  // the next unit's products replace these accumulators, behind two barriers
   }  // units of this CTA
   tc_fence_before();
   __syncthreads();
@@ -1133,7 +1174,7 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
 
   profile_mark(0, stream);
-  const unsigned prep_grid = unsigned(n_ch < int64_t(sm_count) ? n_ch : int64_t(sm_count));
+  const unsigned prep_grid = unsigned(n_ch < 2 * int64_t(sm_count) ? n_ch : 2 * int64_t(sm_count));
   const PrepParams pp{a.workspace, tiles, n_ch, int(a.H), a.scale, a.training, a.prologue};
   GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
     auto kernel = a.prologue != 0 ? chunk_prep_kernel<T, G, Seqs, true> : chunk_prep_kernel<T, G, Seqs, false>;

@@ -73,6 +73,12 @@ __device__ __forceinline__ void store4(float* p, bool vec, const float (&x)[4]) 
   }
 }
 
+__device__ __forceinline__ float exp2_approx(float x) {  // one special-function result
+  float r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
 // ---- layer prologue (optional, fused into the forward kernels) ------------------------------
 // bit flags of the `prologue` argument of the *_fused entry points
 constexpr int kPrologueNorm = GDN2_PROLOGUE_NORMALIZE_QK;   // q, k are raw projections: L2-normalise them
