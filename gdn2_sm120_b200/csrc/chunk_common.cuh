@@ -247,10 +247,16 @@ inline bool encode_cached(CUtensorMap* tm, int rank, CUtensorMapDataType type, c
   if (encode == nullptr) return false;
   const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
   // OOB_FILL_NONE: the part of a load box outside the tensor reads as zero
-  if (encode(tm, type, cuuint32_t(rank), const_cast<void*>(base), dims, strides, box, elem_strides,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
-    return false;
+  auto attempt = [&] {
+    return encode(tm, type, cuuint32_t(rank), const_cast<void*>(base), dims, strides, box, elem_strides,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  if (!attempt()) {
+    // a driver call needs the device's context in this thread, and a thread whose first CUDA call this is (an
+    // autograd thread served from an allocator's cache) has none yet
+    int device = 0;
+    if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess || !attempt()) return false;
   }
   std::lock_guard<std::mutex> lock(mutex);
   slot.used = true; slot.key = key; slot.map = *tm;
