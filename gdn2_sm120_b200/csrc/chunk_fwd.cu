@@ -27,6 +27,8 @@
 //   T = (I + L)^-1,  Y = T (beta k exp(G)),  U = T (w v)
 //   Qg = scale q exp(G),  Kt = k exp(G_end - G),  d = exp(G_end)
 
+#include <type_traits>
+
 #include "chunk_common.cuh"
 
 namespace gdn2 {
@@ -41,46 +43,45 @@ namespace {
 // Persistent, two CTAs of 256 threads per SM.  A unit is a chain of a dozen phases of about a microsecond,
 // each waiting for the one before (loads, exponentials, tensor cores, the blocked inverse, stores): with one
 // CTA per SM the issue slots were 35 % busy and a unit took 10.5 us.  Two CTAs fill each other's waits; for
-// that a CTA has to live in 113 KB, so the Gram operands are built and multiplied in two halves of 64
-// channels, and everything else shares their place.
+// that a CTA has to live in 113 KB and 128 registers per thread, so the Gram operands are built and multiplied
+// 32 channels at a time, and everything else shares their place.  (In two rounds of 64 channels the inputs
+// waiting for the second spilled: 115 KB a unit through L2, as much as the tiles themselves.)
 //
-// A thread owns 4 tokens x 4 channels of each half: token group tg = 2 warp + lane / 16, channel group
-// cl = lane % 16: one 16-byte chunk of every tile row (tokens x channels).  The Gram tiles use a padded chunk
-// stride (CS = 144), so that the 8 lanes of a store phase hit 8 different 16-byte bank groups.
+// A thread owns 2 tokens x 4 channels of each round: tokens 8 warp + lane / 8 and 4 further on, channels
+// 4 (lane % 8): one 16-byte chunk of every tile row.  The eight lanes of a store phase fill one 128-byte line.
 constexpr int kPrepThreads = 256;
-constexpr int kHalf = 64;         // channels per half
+constexpr int kRound = 32, kRounds = kDim / kRound;  // channels per round
 constexpr int kLd = 68;           // leading dimension of the fp32 64x64 scratch matrices (16-byte rows, banks shift by 4)
 constexpr int kLdW = 20;          // leading dimension of the transposed 16x16 block products
-constexpr int kCsN = 144;         // Gram tiles: byte stride between 16-byte column chunks
-constexpr int kRsN = 16 * kCsN;   // Gram tiles of 64 fp32 columns: byte stride between 8-row groups (2304)
 constexpr float kLog2e = 1.4426950408889634f;
 
 // One region, by phase (bytes):
-//   inputs       g at 0 (16 or 32 KiB), then k, q, beta (16 KiB each), dense [64][128] rows by TMA
-//   Gram halves  A operand [E_anchored ; Q_anchored] X[r = 128][c = k], B operands K^I X[r = j < 16 (I + 1)][c = k]
-//   E            E[j][k], tf32, MN-major operand: 4 swizzled slabs of 32 channels x 64 lines (tc05.cuh), the
-//                second half's two slabs first: they replace Gram operands that have been multiplied, the first
-//                half's are behind the Gram operands and written with them
-//   inverse      fp32 T, T^T, L, block products.  The tf32 T tile replaces L.
-// The next unit's g and q arrive over T, T^T and the block products under the last MMA, k and beta after it.
-constexpr int kOffGramA = 0, kOffGramB = 16 * kRsN;                     // 36864 + 46080
+//   inputs       g at 0 (16 or 32 KiB), dense rows; k, q, beta (16 KiB each) by rounds, [round][64][32]
+//   rounds       A operand [E_anchored ; Q_anchored], 128 lines of 32 channels, B operands K^I, 16 (I + 1) lines
+//                each (K-major, 128-byte swizzle); E[j][k], tf32, MN-major operand, 4 swizzled slabs of 32
+//                channels x 64 lines (tc05.cuh) over k and q: slab r is written once rounds r and r + 1 have
+//                been read, hence the order 0, 2, 1, 3
+//   inverse      fp32 T and T^T over the Gram operands, L over beta, block products over the decay table; the
+//                tf32 T tile replaces L
+// The next unit's g arrives over T and T^T under the last MMA, its k, q and beta after it.
+constexpr int kOffGramA = 0, kOffGramB = 16384;                         // + 20480
+constexpr int kOffTable = 36864;                                        // decay table, 13 rows of 128
+constexpr int kOffInG = 0, kOffInK = 47104, kOffInQ = kOffInK + 16384, kOffInBeta = kOffInQ + 16384;
+constexpr int kOffE = kOffInK;
 constexpr int kOffTn = 0, kOffTc = kOffTn + 64 * kLd * 4;               // 17408 each
-constexpr int kOffLn = kOffTc + 64 * kLd * 4, kOffTmat = kOffLn;
-constexpr int kOffWt = kOffLn + 64 * kLd * 4;
-constexpr int kOffE = 67584;                                            // 32768
-constexpr int kOffInG = 0, kOffInK = kOffLn, kOffInQ = kOffInK + 16384, kOffInBeta = kOffInQ + 16384;
-constexpr int kPrepRegion = kOffE + 32768;                              // 100352
-static_assert(kOffWt + 2 * 16 * kLdW * 4 <= kOffInBeta && kOffGramB + 20 * kRsN <= kOffE + 16384, "prep region");
-static_assert(kOffInG + 32768 <= kOffInK && kOffInQ >= kOffTmat + 16384 && kOffInBeta + 16384 <= kPrepRegion, "prep inputs");
-static_assert(kOffInK % 128 == 0 && kOffE % 1024 == 0, "alignment of TMA destinations and swizzled slabs");
+constexpr int kOffLn = kOffInBeta, kOffTmat = kOffLn;
+constexpr int kOffWt = kOffTable;
+constexpr int kPrepRegion = kOffLn + 64 * kLd * 4;                      // 97280
+static_assert(kOffTc + 64 * kLd * 4 <= kOffTable && kOffWt + 2 * 16 * kLdW * 4 <= kOffE && kOffTable + 13 * 512 <= kOffE,
+              "prep region");
+static_assert(kOffE % 1024 == 0 && kOffGramB % 1024 == 0, "swizzled tiles are 1024-byte aligned");
 
 struct PrepSmem {
   alignas(1024) uint8_t region[kPrepRegion];
-  float part[16][kDim];                // per 4-token group partial sums -> exclusive prefixes
+  float part[8][kDim];                 // per 8-token group sums -> exclusive prefixes
   float gend[kDim];
-  float nrm[16][4][2];                 // fused prologue: reciprocal norms of q, k per token
   alignas(8) uint64_t bar[2];          // MMA commits
-  alignas(8) uint64_t bar_ld[2];       // raw inputs: {g, q} and {k, beta}
+  alignas(8) uint64_t bar_ld[2];       // raw inputs: {g} and {k, q, beta}
   uint32_t tmem_base;
 };
 static_assert(sizeof(PrepSmem) <= 115712, "two prep CTAs must fit an SM");
@@ -96,25 +97,24 @@ struct PrepParams {
   int prologue;  // kPrologueNorm | kPrologueGate: the inputs are raw projections / gate pre-activations
 };
 
-__device__ __forceinline__ int gram_b_offset(int I) { return kRsN * ((I == 0) ? 0 : (I == 1) ? 2 : (I == 2) ? 6 : 12); }
 __device__ __forceinline__ int gram_col(int I) { return (I == 0) ? 0 : (I == 1) ? 16 : (I == 2) ? 48 : 96; }
 
-// kPro: the instantiation that can apply the layer prologue to raw inputs (p.prologue says which parts);
-// the plain instantiation carries none of that code.
+struct PrepMaps {
+  CUtensorMap g, k, q, beta;
+};
+
+// kPro: the instantiation that can apply the layer prologue to raw inputs (p.prologue says which parts); the
+// plain instantiation carries none of that code.
 template <typename T, typename G, typename Seqs, bool kPro = false>
 __global__ void __launch_bounds__(kPrepThreads, 2)
-chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ CUtensorMap tm_g,
-                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_q,
-                  const __grid_constant__ CUtensorMap tm_beta) {
+chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ PrepMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
   uint8_t* const R = sm.region;
   const WsLayout ws{p.n_ch, p.training != 0};
   int* status = reinterpret_cast<int*>(p.ws + ws.off_status());
   BoundedWaiter waiter(status);
-
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-
   if (warp == 0) {
     tmem_alloc(&sm.tmem_base, 256);
     tmem_relinquish();
@@ -126,243 +126,233 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     mbar_init(&sm.bar_ld[1], 1);
     fence_mbar_init();
   }
-  const int tg = 2 * warp + (lane >> 4), cl = lane & 15;
-  const int mb = tg >> 2;                     // 16-token block of this thread's tokens
+  const int i0 = 8 * warp + (lane >> 3), cl = lane & 7;  // tokens i0 and i0 + 4
+  const int mb = warp >> 1;                   // 16-token block of this warp's tokens
   const int q4 = warp & 3, part = warp >> 2;  // TMEM lane quadrant of this warp, and its half of the columns
 
-  // unit -> head, first token row of the chunk, tokens that exist
+  // unit -> number of its tiles, head, first token row of the chunk, tokens that exist
   const int heads = p.H, n_ch = int(p.n_ch);
-  struct Place { int h, row, valid; };
-  auto locate = [&](int ch_) {
-    const int chunk = int(uint32_t(ch_) / uint32_t(heads));
+  struct Place { int ch, h, row, valid; };
+  auto locate = [&](int unit) {
+    const int chunk = int(uint32_t(unit) / uint32_t(heads));
     const SeqInfo sq = seqs.at(seqs.find(chunk));
     const int t_ = (chunk - sq.chunk0) * kChunk;
-    return Place{ch_ - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
+    return Place{unit, unit - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
   };
-  auto issue_gq = [&](const Place& at) {
-    mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)) + kStageTile16);
-    tma_load_3d(R + kOffInG, &tm_g, 0, at.h, at.row, &sm.bar_ld[0]);
-    tma_load_3d(R + kOffInQ, &tm_q, 0, at.h, at.row, &sm.bar_ld[0]);
+  auto issue_g = [&](const Place& at) {
+    mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)));
+    tma_load_3d(R + kOffInG, &tm.g, 0, at.h, at.row, &sm.bar_ld[0]);
   };
-  auto issue_kb = [&](const Place& at) {
-    mbar_arrive_expect_tx(&sm.bar_ld[1], 2 * kStageTile16);
-    tma_load_3d(R + kOffInK, &tm_k, 0, at.h, at.row, &sm.bar_ld[1]);
-    tma_load_3d(R + kOffInBeta, &tm_beta, 0, at.h, at.row, &sm.bar_ld[1]);
+  auto issue_kqb = [&](const Place& at) {
+    mbar_arrive_expect_tx(&sm.bar_ld[1], 3 * kStageTile16);
+    tma_load_4d(R + kOffInK, &tm.k, 0, at.row, 0, at.h, &sm.bar_ld[1]);
+    tma_load_4d(R + kOffInQ, &tm.q, 0, at.row, 0, at.h, &sm.bar_ld[1]);
+    tma_load_4d(R + kOffInBeta, &tm.beta, 0, at.row, 0, at.h, &sm.bar_ld[1]);
   };
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  if (tid == 0 && int(blockIdx.x) < n_ch) {
-    const Place at = locate(int(blockIdx.x));
-    issue_gq(at);
-    issue_kb(at);
-  }
   const uint32_t tb = sm.tmem_base;
+  if (tid == 0 && int(blockIdx.x) < n_ch) {
+    const Place at = locate(blockIdx.x);
+    issue_g(at);
+    issue_kqb(at);
+  }
   const uint32_t leader = elect_leader();
-  // this thread's 8- or 16-byte piece of row 4 tg + e, half hf, of a [64][128] input tile
-  auto staged = [&](int tile, int e, int hf, int elem_bytes) {
-    return R + tile + ((4 * tg + e) * kDim + kHalf * hf + 4 * cl) * elem_bytes;
-  };
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
   using RawG = typename Raw4<G>::type;
   using RawT = typename Raw4<T>::type;
 
   uint32_t par = 0;
-  for (int ch = int(blockIdx.x); ch < n_ch; ch += int(gridDim.x), par ^= 1u) {
-  const int ch_next = ch + int(gridDim.x);
+  for (int unit = blockIdx.x; unit < n_ch; unit += gridDim.x, par ^= 1u) {
+  const int unit_next = unit + int(gridDim.x);
   // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
   // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
-  const int n_valid = locate(ch).valid;
+  const Place here = locate(unit);
+  const int ch = here.ch, n_valid = here.valid;
   const bool partial = n_valid < kChunk;
-  // ---- inputs into registers: log-decay sums of this thread's tokens (in units of ln 2: a decay is one ex2),
-  // k, q and beta still packed
-  float Gc[2][4][4];
-  RawT rk[2][4], rq[2][4], rb[2][4];
+  // ---- log-decays, in units of ln 2 (a decay is one ex2): sums from the start of the 16-token block ----------
+  float Gc[kRounds][2][4];
   waiter.wait(&sm.bar_ld[0], par);
 #pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    RawG rg[4];
+  for (int r = 0; r < kRounds; ++r) {
+    float gv[2][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) rg[e] = *reinterpret_cast<const RawG*>(staged(kOffInG, e, hf, sizeof(G)));
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float gv[4];
-      unpack4<G>(rg[e], gv);
+    for (int e = 0; e < 2; ++e) {
+      const int i = i0 + 4 * e;
+      unpack4<G>(*reinterpret_cast<const RawG*>(R + kOffInG + (i * kDim + kRound * r + 4 * cl) * sizeof(G)), gv[e]);
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        if (pro_gate) gv[f] = prologue_log_decay(gv[f]);
-        if (partial && 4 * tg + e >= n_valid) gv[f] = 0.f;
-        Gc[hf][e][f] = e ? fmaf(gv[f], kLog2e, Gc[hf][e - 1][f]) : gv[f] * kLog2e;
+        if (pro_gate) gv[e][f] = prologue_log_decay(gv[e][f]);
+        gv[e][f] = (partial && i >= n_valid) ? 0.f : gv[e][f] * kLog2e;
       }
     }
+    // inclusive sums over the eight tokens of this warp: four lanes of one channel, first tokens, then the others
+    float total[4];
+#pragma unroll
+    for (int f = 0; f < 4; ++f) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        float x = __shfl_up_sync(0xffffffffu, gv[e][f], 8);
+        if (lane >= 8) gv[e][f] += x;
+        x = __shfl_up_sync(0xffffffffu, gv[e][f], 16);
+        if (lane >= 16) gv[e][f] += x;
+      }
+      gv[1][f] += __shfl_sync(0xffffffffu, gv[0][f], 24 + cl);
+      total[f] = gv[1][f];
+#pragma unroll
+      for (int e = 0; e < 2; ++e) Gc[r][e][f] = gv[e][f];
+    }
+    if (lane >= 24) {
+      *reinterpret_cast<float4*>(&sm.part[warp][kRound * r + 4 * cl]) = make_float4(total[0], total[1], total[2], total[3]);
+    }
+  }
+  __syncthreads();
+  // A thread per channel: prefixes of the eight groups, and the decay table, row by row:
+  //   0..3 exp(a_I), a_I = sum up to block I   4..7 exp(a_{I+1} - a_I)   8..11 exp(a_end - a_{I+1})   12 exp(a_3 - a_1)
+  float* const table = reinterpret_cast<float*>(R + kOffTable);
+  if (tid < kDim) {
+    float a[9];
+    a[0] = 0.f;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) a[t + 1] = sm.part[t][tid];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) a[t + 1] += a[t];
+#pragma unroll
+    for (int t = 0; t < 8; ++t) sm.part[t][tid] = a[t] - a[t & ~1];  // from the start of the block
+    sm.gend[tid] = a[8];
+    reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(a[8]);
+#pragma unroll
+    for (int I = 0; I < 4; ++I) {
+      table[I * kDim + tid] = exp2_approx(a[2 * I]);
+      table[(4 + I) * kDim + tid] = exp2_approx(a[2 * I + 2] - a[2 * I]);
+      table[(8 + I) * kDim + tid] = exp2_approx(a[8] - a[2 * I + 2]);
+    }
+    table[12 * kDim + tid] = exp2_approx(a[6] - a[2]);
   }
   waiter.wait(&sm.bar_ld[1], par);
+  RawT rk[2], rq[2], rb[2];
+  auto read_raw = [&](int r) {
 #pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      rk[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInK, e, hf, 2));
-      rq[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInQ, e, hf, 2));
-      rb[hf][e] = *reinterpret_cast<const RawT*>(staged(kOffInBeta, e, hf, 2));
-      if (partial && 4 * tg + e >= n_valid) rk[hf][e] = rq[hf][e] = rb[hf][e] = RawT{};
+    for (int e = 0; e < 2; ++e) {
+      const int at = r * 4096 + (i0 + 4 * e) * 64 + cl * 8;
+      rk[e] = *reinterpret_cast<const RawT*>(R + kOffInK + at);
+      rq[e] = *reinterpret_cast<const RawT*>(R + kOffInQ + at);
+      rb[e] = *reinterpret_cast<const RawT*>(R + kOffInBeta + at);
+      if (partial && i0 + 4 * e >= n_valid) rk[e] = rq[e] = rb[e] = RawT{};
     }
-  }
-#pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    *reinterpret_cast<float4*>(&sm.part[tg][kHalf * hf + 4 * cl]) =
-        make_float4(Gc[hf][3][0], Gc[hf][3][1], Gc[hf][3][2], Gc[hf][3][3]);
-  }
+  };
+  float inv_q[2] = {1.f, 1.f}, inv_k[2] = {1.f, 1.f};
   if (pro_norm) {
-    // sums of q^2 and k^2: this thread's channels, then the 16 lanes that hold the others of the same tokens
-    // (as two sums, channels 0..63 and 64..127)
+    // sums of q^2 and k^2 over the channels: this thread's, then the eight lanes of a token
+    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      float sq[2], sk[2];
+    for (int r = 0; r < kRounds; ++r) {
+      read_raw(r);
 #pragma unroll
-      for (int hf = 0; hf < 2; ++hf) {
-        float kf[4], qf[4];
-        unpack4<T>(rk[hf][e], kf);
-        unpack4<T>(rq[hf][e], qf);
-        sq[hf] = qf[0] * qf[0] + qf[1] * qf[1] + qf[2] * qf[2] + qf[3] * qf[3];
-        sk[hf] = kf[0] * kf[0] + kf[1] * kf[1] + kf[2] * kf[2] + kf[3] * kf[3];
-#pragma unroll
-        for (int off = 1; off < 16; off <<= 1) {
-          sq[hf] += __shfl_xor_sync(0xffffffffu, sq[hf], off);
-          sk[hf] += __shfl_xor_sync(0xffffffffu, sk[hf], off);
-        }
-      }
-      if (cl == 0) {
-        sm.nrm[tg][e][0] = rsqrtf(sq[0] + sq[1] + kPrologueEps);
-        sm.nrm[tg][e][1] = rsqrtf(sk[0] + sk[1] + kPrologueEps);
+      for (int e = 0; e < 2; ++e) {
+        float x[4];
+        unpack4<T>(rq[e], x);
+        sq[e] += (x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]);
+        unpack4<T>(rk[e], x);
+        sk[e] += (x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]);
       }
     }
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int off = 1; off < 8; off <<= 1) {
+        sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], off);
+        sk[e] += __shfl_xor_sync(0xffffffffu, sk[e], off);
+      }
+      inv_q[e] = rsqrtf(sq[e] + kPrologueEps);
+      inv_k[e] = rsqrtf(sk[e] + kPrologueEps);
+    }
   }
+  read_raw(0);
   __syncthreads();
-  if (tid < kDim) {
-    float x[16];
 #pragma unroll
-    for (int t = 0; t < 16; ++t) x[t] = sm.part[t][tid];
-    float run = 0.f;
+  for (int r = 0; r < kRounds; ++r) {
+    float base[4];
+    load4(&sm.part[warp][kRound * r + 4 * cl], true, base);
 #pragma unroll
-    for (int t = 0; t < 16; ++t) {
-      sm.part[t][tid] = run;
-      run += x[t];
+    for (int e = 0; e < 2; ++e) {
+#pragma unroll
+      for (int f = 0; f < 4; ++f) Gc[r][e][f] += base[f];
     }
-    sm.gend[tid] = run;
-    reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(run);
   }
-  __syncthreads();
-  // k and beta of token e, half hf (normalised / activated when the inputs are raw)
-  auto key = [&](int hf, int e, float (&x)[4]) {
-    unpack4<T>(rk[hf][e], x);
-    if (pro_norm) {
-      const float inv = sm.nrm[tg][e][1];
-#pragma unroll
-      for (int f = 0; f < 4; ++f) x[f] *= inv;
-    }
-  };
-  auto gate = [&](int hf, int e, float (&x)[4]) {
-    unpack4<T>(rb[hf][e], x);
-    if (pro_gate) {
-#pragma unroll
-      for (int f = 0; f < 4; f += 2) prologue_sigmoid2(x[f], x[f + 1]);
-    }
-  };
 
-  // ---- Gram products P_I = [E_a ; Q_a] (K^I)^T on the tensor cores, 64 channels at a time ------------------
+  // ---- Gram products P_I = [E_a ; Q_a] (K^I)^T on the tensor cores, 32 channels at a time ------------------
   float* const tile_q = reinterpret_cast<float*>(p.tiles.q + int64_t(ch) * kTileQ);
   float* const tile_kn = reinterpret_cast<float*>(p.tiles.kn + int64_t(ch) * kTileKn);
-  // E[i][channels of this thread]: 16 bytes of line i of a slab, 32-byte pieces permuted by the line
-  auto store_e = [&](int hf, int i, const float (&x)[4]) {
-    uint8_t* slab = R + kOffE + (hf == 0 ? 16384 : 0) + (cl >> 3) * 8192;
-    *reinterpret_cast<float4*>(slab + i * 128 + ((((cl & 7) >> 1) ^ (i & 3)) << 5) + (cl & 1) * 16) =
-        make_float4(x[0], x[1], x[2], x[3]);
-  };
-  float e_second[4][4];
+  // (a loop, with the round's sums shifted into place at its end: unrolled it would be 4 x the code, and the
+  // compiler's moves across the rounds cost more registers than there are)
+#pragma unroll 1
+  for (int r = 0; r < kRounds; ++r) {
+    const int kc0 = kRound * r + 4 * cl;
+    float e_amb[4], c_nx[4], t_end[4], far0[4], far1[4];
+    load4(table + mb * kDim + kc0, true, e_amb);
+    load4(table + (4 + mb) * kDim + kc0, true, c_nx);         // decay over the whole 16-token block (<= 1)
+    load4(table + (8 + mb) * kDim + kc0, true, t_end);
+    load4(table + (mb < 2 ? 5 + mb : 4) * kDim + kc0, true, far0);  // (mb < 2) on to the block after the next one
+    load4(table + 12 * kDim + kc0, true, far1);                     // (mb < 1) ... and the one after that
+    float kk[2][4], bb[2][4], qq[2][4];
 #pragma unroll
-  for (int hf = 0; hf < 2; ++hf) {
-    const int kc0 = kHalf * hf + 4 * cl;
-    // decay table of this thread's channels: everything except two exponentials per element comes from here
-    float pre[4], e_amb[4], c_nx[4], t_end[4], t_far[2][4];
-    {
-      const float* end = &sm.gend[kc0];
-      const float* nx = mb + 1 < 4 ? &sm.part[4 * mb + 4][kc0] : end;
-      const float* f0 = mb + 2 < 4 ? &sm.part[4 * mb + 8][kc0] : end;
-      const float* f1 = mb + 3 < 4 ? &sm.part[4 * mb + 12][kc0] : end;
-      float a_mb[4], a_nx[4], a_end[4], a_f0[4], a_f1[4];
-      load4(&sm.part[tg][kc0], true, pre);
-      load4(&sm.part[4 * mb][kc0], true, a_mb);
-      load4(nx, true, a_nx);
-      load4(end, true, a_end);
-      load4(f0, true, a_f0);
-      load4(f1, true, a_f1);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        pre[f] -= a_mb[f];                             // sum from the start of the 16-token block
-        e_amb[f] = exp2_approx(a_mb[f]);
-        c_nx[f] = exp2_approx(a_nx[f] - a_mb[f]);      // decay over the whole 16-token block (<= 1)
-        t_end[f] = exp2_approx(a_end[f] - a_nx[f]);
-        t_far[0][f] = exp2_approx(a_f0[f] - a_nx[f]);  // blocks further than the next one: exp(a_I - a_next)
-        t_far[1][f] = exp2_approx(a_f1[f] - a_nx[f]);
-      }
+    for (int e = 0; e < 2; ++e) {
+      unpack4<T>(rk[e], kk[e]);
+      unpack4<T>(rb[e], bb[e]);
+      unpack4<T>(rq[e], qq[e]);
     }
-    if (hf == 1) waiter.wait(&sm.bar[0], 0);  // the first half's operands have been multiplied
+    if (r + 1 < kRounds) read_raw(r + 1);
+    if (r > 0) waiter.wait(&sm.bar[0], (r - 1) & 1);  // the last round's operands have been multiplied
+    float eb[2][4];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int i = 4 * tg + e;
-      float kk[4], bb[4], qq[4];
-      key(hf, e, kk);
-      gate(hf, e, bb);
-      unpack4<T>(rq[hf][e], qq);
-      if (pro_norm) {
-        const float inv = sm.nrm[tg][e][0];
+    for (int e = 0; e < 2; ++e) {
+      const int i = i0 + 4 * e;
+      if (pro_gate) {
 #pragma unroll
-        for (int f = 0; f < 4; ++f) qq[f] *= inv;
+        for (int f = 0; f < 4; f += 2) prologue_sigmoid2(bb[e][f], bb[e][f + 1]);
       }
-      float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4], eb[4];
+      float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4];
 #pragma unroll
       for (int f = 0; f < 4; ++f) {
-        const float Gi = Gc[hf][e][f] + pre[f];
-        const float anchored = exp2_approx(Gi);        // <= 1
-        const float own = exp2_approx(-Gi);            // >= 1, bounded by the 16-token contract
-        const float nb = own * c_nx[f];                // exp(a_nx - G_i) <= 1: decay from token i to the next block start
-        const float bk = bb[f] * kk[f];
-        const float sq = p.scale * qq[f];
+        const float anchored = exp2_approx(Gc[0][e][f]);   // <= 1
+        const float own = exp2_approx(-Gc[0][e][f]);       // >= 1, bounded by the 16-token contract
+        const float nb = own * c_nx[f];                    // <= 1: decay from token i to the next block start
+        const float k = kPro ? kk[e][f] * inv_k[e] : kk[e][f];
+        const float bk = bb[e][f] * k;
+        const float sq = p.scale * (kPro ? qq[e][f] * inv_q[e] : qq[e][f]);
         ea[f] = to_tf32_operand(bk * anchored);
         qa[f] = to_tf32_operand(sq * anchored);
-        eb[f] = to_tf32_operand(bk * anchored * e_amb[f]);
+        eb[e][f] = to_tf32_operand(bk * anchored * e_amb[f]);
         qgam[f] = to_tf32_operand(sq * anchored * e_amb[f]);
-        kown[f] = to_tf32_operand(kk[f] * own);
-        knb[f] = kk[f] * nb;
+        kown[f] = to_tf32_operand(k * own);
+        knb[f] = k * nb;
         ktail[f] = to_tf32_operand(knb[f] * t_end[f]);
       }
-      // Gram A operand rows i (erase) and 64 + i (query), tf32, K-major, padded chunk stride
-      const uint32_t row_off = (i >> 3) * kRsN + cl * kCsN + (i & 7) * 16;
-      *reinterpret_cast<float4*>(R + kOffGramA + row_off) = make_float4(ea[0], ea[1], ea[2], ea[3]);
-      *reinterpret_cast<float4*>(R + kOffGramA + 8 * kRsN + row_off) = make_float4(qa[0], qa[1], qa[2], qa[3]);
-      // Gram B operands: token i is a column of every row block I >= its own
-      *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb) + row_off) =
-          make_float4(kown[0], kown[1], kown[2], kown[3]);
-      if (mb + 1 < 4) {
-        *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb + 1) + row_off) =
+      // 16-byte chunk cl of a 128-byte line, permuted by the line (the row numbers of K^I start at multiples
+      // of 16: one permutation for all)
+      const uint32_t at = i * 128 + ((cl ^ (i & 7)) << 4);
+      *reinterpret_cast<float4*>(R + kOffGramA + at) = make_float4(ea[0], ea[1], ea[2], ea[3]);
+      *reinterpret_cast<float4*>(R + kOffGramA + 64 * 128 + at) = make_float4(qa[0], qa[1], qa[2], qa[3]);
+      // token i is a row of every K^I, I >= its own block
+      *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb) * 128 + at) = make_float4(kown[0], kown[1], kown[2], kown[3]);
+      if (mb < 3) {
+        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb + 1) * 128 + at) =
             make_float4(to_tf32_operand(knb[0]), to_tf32_operand(knb[1]), to_tf32_operand(knb[2]), to_tf32_operand(knb[3]));
       }
-#pragma unroll
-      for (int far = 0; far < 2; ++far) {
-        if (mb + 2 + far < 4) {
-          *reinterpret_cast<float4*>(R + kOffGramB + gram_b_offset(mb + 2 + far) + row_off) =
-              make_float4(to_tf32_operand(knb[0] * t_far[far][0]), to_tf32_operand(knb[1] * t_far[far][1]),
-                          to_tf32_operand(knb[2] * t_far[far][2]), to_tf32_operand(knb[3] * t_far[far][3]));
-        }
+      if (mb < 2) {
+        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb + 2) * 128 + at) =
+            make_float4(to_tf32_operand(knb[0] * far0[0]), to_tf32_operand(knb[1] * far0[1]),
+                        to_tf32_operand(knb[2] * far0[2]), to_tf32_operand(knb[3] * far0[3]));
       }
-      if (hf == 0) {
-        store_e(0, i, eb);
-      } else {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) e_second[e][f] = eb[f];
+      if (mb < 1) {
+        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(3) * 128 + at) =
+            make_float4(to_tf32_operand(knb[0] * far1[0]), to_tf32_operand(knb[1] * far1[1]),
+                        to_tf32_operand(knb[2] * far1[2]), to_tf32_operand(knb[3] * far1[3]));
       }
-      // token-major tiles Q[i][k] and Kn[i][k]: the 16 lanes of a token write 256 consecutive bytes
+      // token-major tiles Q[i][k] and Kn[i][k]: the 8 lanes of a token write 128 consecutive bytes
       *reinterpret_cast<float4*>(tile_q + i * kDim + kc0) = make_float4(qgam[0], qgam[1], qgam[2], qgam[3]);
       *reinterpret_cast<float4*>(tile_kn + i * kDim + kc0) = make_float4(ktail[0], ktail[1], ktail[2], ktail[3]);
     }
@@ -376,22 +366,34 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       const uint32_t id = idesc(128, 160, kFmtTF32, kMajorK, kMajorK);
       const uint32_t a0 = smem_u32(R + kOffGramA), b0 = smem_u32(R + kOffGramB);
 #pragma unroll
-      for (int ks = 0; ks < 8; ++ks) {
-        mma_tf32_ss(tb, smem_desc(a0 + ks * 2 * kCsN, kCsN, kRsN), smem_desc(b0 + ks * 2 * kCsN, kCsN, kRsN), id,
-                    (hf | ks) > 0 ? 1u : 0u, leader);
+      for (int ks = 0; ks < 4; ++ks) {
+        mma_tf32_ss(tb, smem_desc_sw128_k(a0, 0, ks), smem_desc_sw128_k(b0, 0, ks), id, (r | ks) > 0 ? 1u : 0u, leader);
       }
       mma_commit(&sm.bar[0], leader);
+    }
+    // E[i][channels of this thread]: 16 bytes of line i of a slab, 32-byte pieces permuted by the line
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int i = i0 + 4 * e, slab = (r >> 1) | ((r & 1) << 1);
+      *reinterpret_cast<float4*>(R + kOffE + slab * 8192 + i * 128 + (((cl >> 1) ^ (i & 3)) << 5) + (cl & 1) * 16) =
+          make_float4(eb[e][0], eb[e][1], eb[e][2], eb[e][3]);
+    }
+#pragma unroll
+    for (int n = 0; n + 1 < kRounds; ++n) {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+#pragma unroll
+        for (int f = 0; f < 4; ++f) Gc[n][e][f] = Gc[n + 1][e][f];
+      }
     }
   }
   waiter.wait(&sm.bar[0], 1);
   tc_fence_after();
-  // the Gram operands are dead: the region becomes fp32 scratch and the second half of E
+  // the Gram operands are dead: the region becomes fp32 scratch
   float* Tn = reinterpret_cast<float*>(R + kOffTn);           // [64][kLd]   T
   float* Tc = reinterpret_cast<float*>(R + kOffTc);           // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
   float* Ln = reinterpret_cast<float*>(R + kOffLn);           // [64][kLd]   L
   float* Wt = reinterpret_cast<float*>(R + kOffWt);           // [2][16][kLdW] block products, transposed
-#pragma unroll
-  for (int e = 0; e < 4; ++e) store_e(1, 4 * tg + e, e_second[e]);
   {
     // pull L (rows 0..63) into fp32 scratch and A_qk (rows 64..127) into the workspace;
     // the two warps of a quadrant take 32 columns each
@@ -589,14 +591,14 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     }
     mma_commit(&sm.bar[1], leader);
   }
-  if (tid == 32 && ch_next < n_ch) issue_gq(locate(ch_next));
+  if (tid == 32 && unit_next < n_ch) issue_g(locate(unit_next));
   waiter.wait(&sm.bar[1], par);
   tc_fence_after();
-  if (tid == 32 && ch_next < n_ch) issue_kb(locate(ch_next));
+  if (tid == 32 && unit_next < n_ch) issue_kqb(locate(unit_next));
   {
     // lanes = key channels k, columns = tokens i: each warp takes 32 tokens of its quadrant, a lane 128
     // consecutive bytes of row k of Yt[k][i]
-    const int kr = (32 * q4 + lane + kHalf) & (kDim - 1), c0 = 32 * part;  // (the second half's slabs come first)
+    const int kr = 32 * ((q4 >> 1) | ((q4 & 1) << 1)) + lane, c0 = 32 * part;  // (slabs in the order 0, 2, 1, 3)
     float* row_yt = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + c0;
     uint32_t r[32];
     tmem_ld32(tmem_addr(tb, 32 * q4, c0), r);
@@ -1153,13 +1155,13 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
 
   const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
-  CUtensorMap tm_g, tm_k, tm_q, tm_beta;
+  PrepMaps tm_prep;
   ScanMaps tm;
   // the sequence tensors, and the scan's operands: the prep kernel's tiles in the swizzle of their role
-  if (!encode_sequence_map(&tm_g, a.g, a.rows, a.H, a.g_dtype) ||
-      !encode_sequence_map(&tm_k, a.k, a.rows, a.H, a.dtype) ||
-      !encode_sequence_map(&tm_q, a.q, a.rows, a.H, a.dtype) ||
-      !encode_sequence_map(&tm_beta, a.beta, a.rows, a.H, a.dtype) ||
+  if (!encode_sequence_map(&tm_prep.g, a.g, a.rows, a.H, a.g_dtype) ||
+      !encode_round_map(&tm_prep.k, a.k, a.rows, a.H, a.dtype) ||
+      !encode_round_map(&tm_prep.q, a.q, a.rows, a.H, a.dtype) ||
+      !encode_round_map(&tm_prep.beta, a.beta, a.rows, a.H, a.dtype) ||
       !encode_sequence_map(&tm.v, a.v, a.rows, a.H, a.dtype) ||
       !encode_sequence_map(&tm.w, a.w, a.rows, a.H, a.dtype) ||
       !encode_sequence_map(&tm.out, a.out, a.rows, a.H, a.dtype) ||
@@ -1181,7 +1183,7 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
     const int smem = int(sizeof(PrepSmem));
     err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
     if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<prep_grid, kPrepThreads, smem, stream>>>(pp, seqs, tm_g, tm_k, tm_q, tm_beta);
+    kernel<<<prep_grid, kPrepThreads, smem, stream>>>(pp, seqs, tm_prep);
   });
   int st = check_launch();
   if (st != GDN2_OK) return st;
