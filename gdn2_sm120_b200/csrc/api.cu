@@ -67,6 +67,8 @@ ProfileSet g_profile[kProfileDevices];
 std::mutex g_profile_mutex;
 }  // namespace
 
+bool profiling() { return g_profile_on; }
+
 void profile_mark(int index, cudaStream_t stream) {
   if (!g_profile_on) return;
   int device = 0;

@@ -305,14 +305,14 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       for (int j4 = 0; j4 < 8; ++j4) {
         const float4 da = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 4 * j4]);
         const float4 db = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 32 + 4 * j4]);
-        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * da.x);
-        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * da.y);
-        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * da.z);
-        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * da.w);
-        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * db.x);
-        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * db.y);
-        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * db.z);
-        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * db.w);
+        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * fabsf(da.x));
+        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * fabsf(da.y));
+        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * fabsf(da.z));
+        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * fabsf(da.w));
+        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * fabsf(db.x));
+        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * fabsf(db.y));
+        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * fabsf(db.z));
+        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * fabsf(db.w));
       }
       store_state(kColS + 128u * (par ^ 1u));
       arrive(&sm.go_q);

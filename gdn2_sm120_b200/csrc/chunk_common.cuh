@@ -18,6 +18,7 @@
 //        (both are zero where j > i: the quadrant j >= 32, i < 32 is neither written nor read, the
 //        consumers keep those lines of their shared-memory tile at zero; 12 KiB move)
 //   D    float[128]                      512 B    gamma_end
+//        (element 0 is negative when its unit was prepared beside a running scan: read magnitudes)
 //
 //   Rn   [token j (64)][value v (128)]   32 KiB   R = U - Y S_0   forward scan -> VJP kernel (K-major)
 //
@@ -46,7 +47,8 @@ namespace gdn2 {
 constexpr int64_t kTileQ = 32768, kTileKn = 32768, kTileYt = 32768;
 constexpr int64_t kTileAt = 16384, kTileTt = 16384, kBlobD = 512;
 constexpr int64_t kBlobRn = 32768, kBlobDZ = 8 * 4608;
-constexpr int64_t kStatusBytes = 256;
+constexpr int64_t kStatusBytes = 256;  // word 0: status
+constexpr int kQueueWord = 16;         // joint launch: next unit to prepare
 // forward scratch per unit, a size callers know: 144 KiB for an inference call (its tiles take 128 of
 // them), 32 KiB for a training call
 constexpr int64_t kFwdScratchInference = 147456, kFwdScratchTraining = 32768;
@@ -121,13 +123,30 @@ struct BoundedWaiter {
       : status(s), limit(max_polls), cta_flag(flag) {}
   __device__ __forceinline__ void wait(uint64_t* bar, uint32_t parity) {
     if (dead) return;
-    if (!tc::mbar_wait(bar, parity, limit)) {
-      dead = true;
-      if (cta_flag != nullptr) *cta_flag = 1;
-      if (status != nullptr) atomicExch(status, kStatusBarrierTimeout);
-    }
+    if (!tc::mbar_wait(bar, parity, limit)) expire();
+  }
+  // for loops that look at something other than an mbarrier: false once `limit` looks were in vain
+  __device__ __forceinline__ bool look_again() {
+    if (limit > 0) --limit;
+    if (limit == 0 && !dead) expire();
+    return limit > 0;
+  }
+  __device__ __forceinline__ void expire() {
+    dead = true;
+    if (cta_flag != nullptr) *cta_flag = 1;
+    if (status != nullptr) atomicExch(status, kStatusBarrierTimeout);
   }
 };
+
+// ---- marks between CTAs of one launch: a float whose sign says that a unit is finished ------------
+__device__ __forceinline__ void store_release(float* p, float x) {
+  asm volatile("st.release.gpu.global.f32 [%0], %1;" ::"l"(p), "f"(x) : "memory");
+}
+__device__ __forceinline__ bool marked(const float* p) {
+  uint32_t x;
+  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+  return (x >> 31) != 0;
+}
 
 // load 8 consecutive sequence elements (16-bit type: one 16-byte load; fp32: two)
 template <typename T>

@@ -82,6 +82,7 @@ struct PrepSmem {
   float gend[kDim];
   alignas(8) uint64_t bar[2];          // MMA commits
   alignas(8) uint64_t bar_ld[2];       // raw inputs: {g} and {k, q, beta}
+  int next[2];                         // joint launch: the unit after this one (two slots: one may still be read)
   uint32_t tmem_base;
 };
 static_assert(sizeof(PrepSmem) <= 115712, "two prep CTAs must fit an SM");
@@ -103,22 +104,24 @@ struct PrepMaps {
   CUtensorMap g, k, q, beta;
 };
 
-// kPro: the instantiation that can apply the layer prologue to raw inputs (p.prologue says which parts); the
-// plain instantiation carries none of that code.
-template <typename T, typename G, typename Seqs, bool kPro = false>
-__global__ void __launch_bounds__(kPrepThreads, 2)
-chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ PrepMaps tm) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
+// The units of one group of 256 threads (`tid` within it): first, first + stride, ..., or in a joint launch
+// `first` and then whatever the queue gives; tensor memory columns tb .. tb + 255.  kPro: the instantiation
+// that can apply the layer prologue to raw inputs (p.prologue says which parts); the plain instantiation
+// carries none of that code.  kJoint: units are taken in the order in which the scans running beside need
+// them (chunk by chunk through all sequences), and a finished one is marked in its D array.
+template <typename T, typename G, typename Seqs, bool kPro, bool kJoint>
+__device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs, const PrepMaps& tm, PrepSmem& sm,
+                                           const int tid, const uint32_t tb, const int first, const int stride,
+                                           const int barrier, int* queue) {
   uint8_t* const R = sm.region;
   const WsLayout ws{p.n_ch, p.training != 0};
   int* status = reinterpret_cast<int*>(p.ws + ws.off_status());
   BoundedWaiter waiter(status);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  if (warp == 0) {
-    tmem_alloc(&sm.tmem_base, 256);
-    tmem_relinquish();
-  }
+  const int warp = tid >> 5, lane = tid & 31;
+  auto sync = [&] {
+    if constexpr (kJoint) asm volatile("bar.sync %0, 256;" ::"r"(barrier) : "memory");
+    else __syncthreads();
+  };
   if (tid == 0) {
     mbar_init(&sm.bar[0], 1);
     mbar_init(&sm.bar[1], 1);
@@ -134,10 +137,18 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
   const int heads = p.H, n_ch = int(p.n_ch);
   struct Place { int ch, h, row, valid; };
   auto locate = [&](int unit) {
-    const int chunk = int(uint32_t(unit) / uint32_t(heads));
-    const SeqInfo sq = seqs.at(seqs.find(chunk));
-    const int t_ = (chunk - sq.chunk0) * kChunk;
-    return Place{unit, unit - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
+    if constexpr (kJoint) {
+      const int per_chunk = seqs.count() * heads, c = int(uint32_t(unit) / uint32_t(per_chunk));
+      const int r = unit - c * per_chunk, s_ = int(uint32_t(r) / uint32_t(heads));
+      const SeqInfo sq = seqs.at(s_);
+      unit = (sq.chunk0 + c) * heads + (r - s_ * heads);
+      return Place{unit, r - s_ * heads, int(sq.row0) + c * kChunk, min(kChunk, sq.len - c * kChunk)};
+    } else {
+      const int chunk = int(uint32_t(unit) / uint32_t(heads));
+      const SeqInfo sq = seqs.at(seqs.find(chunk));
+      const int t_ = (chunk - sq.chunk0) * kChunk;
+      return Place{unit, unit - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
+    }
   };
   auto issue_g = [&](const Place& at) {
     mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)));
@@ -149,12 +160,9 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     tma_load_4d(R + kOffInQ, &tm.q, 0, at.row, 0, at.h, &sm.bar_ld[1]);
     tma_load_4d(R + kOffInBeta, &tm.beta, 0, at.row, 0, at.h, &sm.bar_ld[1]);
   };
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tb = sm.tmem_base;
-  if (tid == 0 && int(blockIdx.x) < n_ch) {
-    const Place at = locate(blockIdx.x);
+  sync();
+  if (tid == 0 && first < n_ch) {
+    const Place at = locate(first);
     issue_g(at);
     issue_kqb(at);
   }
@@ -165,8 +173,13 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
   using RawT = typename Raw4<T>::type;
 
   uint32_t par = 0;
-  for (int unit = blockIdx.x; unit < n_ch; unit += gridDim.x, par ^= 1u) {
-  const int unit_next = unit + int(gridDim.x);
+  for (int unit = first, unit_next; unit < n_ch; unit = unit_next, par ^= 1u) {
+  // a queue and not a stride: an SM that shares its way to L2 with a scan prepares at little more than half
+  // the pace of the others, and the scans wait for the slowest
+  unit_next = unit + stride;
+  if constexpr (kJoint) {
+    if (tid == 32) sm.next[par] = unit_next = stride + atomicAdd(queue, 1);
+  }
   // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
   // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
   const Place here = locate(unit);
@@ -208,7 +221,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       *reinterpret_cast<float4*>(&sm.part[warp][kRound * r + 4 * cl]) = make_float4(total[0], total[1], total[2], total[3]);
     }
   }
-  __syncthreads();
+  sync();
   // A thread per channel: prefixes of the eight groups, and the decay table, row by row:
   //   0..3 exp(a_I), a_I = sum up to block I   4..7 exp(a_{I+1} - a_I)   8..11 exp(a_end - a_{I+1})   12 exp(a_3 - a_1)
   float* const table = reinterpret_cast<float*>(R + kOffTable);
@@ -222,7 +235,8 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 #pragma unroll
     for (int t = 0; t < 8; ++t) sm.part[t][tid] = a[t] - a[t & ~1];  // from the start of the block
     sm.gend[tid] = a[8];
-    reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(a[8]);
+    // (element 0 of D doubles as the mark of a finished unit: see the end of the loop)
+    if (!kJoint || tid > 0) reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(a[8]);
 #pragma unroll
     for (int I = 0; I < 4; ++I) {
       table[I * kDim + tid] = exp2_approx(a[2 * I]);
@@ -271,7 +285,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     }
   }
   read_raw(0);
-  __syncthreads();
+  sync();
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
     float base[4];
@@ -358,7 +372,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     }
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
+    sync();
     if (warp == 0) {
       tc_fence_after();
       // the four anchored copies K^0 .. K^3 are stacked (16 + 32 + 48 + 64 = 160 rows) and their products
@@ -433,7 +447,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     }
   }
   tc_fence_before();
-  __syncthreads();
+  sync();
 
   // ---- T = (I + L)^-1, blocked: 16x16 diagonal blocks by substitution, the rest by block products.
   // T is kept in both orientations (Tn row-major, Tc column-major) and the block products W transposed,
@@ -468,7 +482,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     *reinterpret_cast<float4*>((tid < 128 ? Tc + (16 + r) * kLd : Tn + (32 + r) * kLd + 48) + c4) =
         make_float4(0.f, 0.f, 0.f, 0.f);
   }
-  __syncthreads();
+  sync();
   // inner product of 4 `quads` values, in four independent chains (latency-bound otherwise)
   auto dot = [&](const float* a, const float* b, int quads) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -495,7 +509,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 #pragma unroll
     for (int pair = 0; pair < 2; ++pair) Wt[(pair * 16 + cc) * kLdW + r] = w[pair];
   }
-  __syncthreads();
+  sync();
   // level 1, T_IJ = -T_II W
   {
     const int r = tid >> 4, cc = tid & 15;
@@ -512,7 +526,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       Tc[(16 * J + cc) * kLd + 16 * I + r] = -s[pair];
     }
   }
-  __syncthreads();
+  sync();
   // level 2, W2 = L[32.., ..32) P, stored transposed over the (now dead) first 32 rows of L
   // A thread forms four entries of a column (rows r, r + 8, r + 16, r + 24): the column of the right factor is
   // the expensive read (a different 16-byte piece per lane, four shared-memory wavefronts), the rows of the
@@ -543,7 +557,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 #pragma unroll
     for (int x = 0; x < 4; ++x) W2t[cc * kLd + r + 8 * x] = w[x];
   }
-  __syncthreads();
+  sync();
   // level 2, T[32 + r][c] = -sum_m Q[r][m] W2[m][c]
   {
     const int r = tid >> 5, cc = tid & 31;
@@ -555,7 +569,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
       Tc[cc * kLd + 32 + r + 8 * x] = -s[x];
     }
   }
-  __syncthreads();
+  sync();
   // T as tf32 tile X[r = i][c = j] over L (MMA operand), and T^T[j][i] for the scans
   {
     float* tile_tt = reinterpret_cast<float*>(p.tiles.tt + int64_t(ch) * kTileTt);
@@ -577,7 +591,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
   }
   fence_async_smem();
   tc_fence_before();
-  __syncthreads();
+  sync();
 
   // ---- Y^T = E^T T^T (A = E[j][k] read MN-major) ------------------------------------------------------------------------------------
   if (warp == 0) {
@@ -613,10 +627,37 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
     }
   }
   tc_fence_before();  // the next unit's products replace these accumulators, behind two barriers
-  }  // units of this CTA
+  if constexpr (kJoint) {
+    // every thread's stores, then the mark: the sign of D[0] (a decay is never negative).  The scan reads the
+    // tiles through the copy engine, another proxy than the stores.
+    fence_async_all();
+    sync();
+    unit_next = sm.next[par];
+    if (tid == 0) {
+      float* d = reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD);
+      store_release(d, __uint_as_float(__float_as_uint(exp2_approx(sm.gend[0])) | 0x80000000u));
+    }
+  }
+  }  // units of this group
+}
+
+template <typename T, typename G, typename Seqs, bool kPro = false>
+__global__ void __launch_bounds__(kPrepThreads, 2)
+chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ PrepMaps tm) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  PrepSmem& sm = *reinterpret_cast<PrepSmem*>(smem_raw);
+  if (threadIdx.x < 32) {
+    tmem_alloc(&sm.tmem_base, 256);
+    tmem_relinquish();
+  }
   tc_fence_before();
   __syncthreads();
-  if (warp == 0) tmem_dealloc(tb, 256);
+  tc_fence_after();
+  const uint32_t tb = sm.tmem_base;
+  prep_units<T, G, Seqs, kPro, false>(p, seqs, tm, sm, threadIdx.x, tb, int(blockIdx.x), int(gridDim.x), 0, nullptr);
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x < 32) tmem_dealloc(tb, 256);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -630,16 +671,19 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 //   warp 1       MMAs, per chunk:  R^T -= S^T Y^T | O^T = S^T Qg^T | S'^T += R^T Kt | O^T += R^T Aqk^T |
 //                R'^T = Z'^T T^T of the next chunk.  MMAs of one shape on one accumulator run in order; every
 //                other dependence (R -> S', S' -> R') is waited for, with independent MMAs in the queue meanwhile
-//   warps 2..9   decay: S' <- S diag(d) into the other of two state buffers while R is formed (the output
+//   warp 2       loads of v and w, whose buffer frees at another time than the others
+//   warp 3       joint launch: watches the marks of prepared chunks (a look at one takes most of a microsecond)
+//   warps 4..11  decay: S' <- S diag(d) into the other of two state buffers while R is formed (the output
 //                still reads S); training: the chunk-start state, staged and sent by bulk stores
-//   warps 10..17 Z = w v of the next chunk into tensor memory; training: R out
-//   warps 18..21 O out (staged, one TMA store)
-//   warp 22      loads of v and w, whose buffer frees at another time than the others
+//   warps 12..19 Z = w v of the next chunk into tensor memory; training: R out
+//   warps 20..23 O out (staged, one TMA store); in a joint launch, whose preparing CTAs need the registers, the Z
+//                warps do it (where loads are late, Z waits for them and O behind it: 691 -> 743 us at
+//                B4 T8192 H32 training, so not in a launch of its own)
 // A passed mbarrier wait costs ~150 clocks, so what an MMA group needs arrives on one barrier: the bytes of
 // its tiles, the threads that wrote its other operand and those that freed its accumulator.
 // Tensor memory (columns): S 2 x 128, R 2 x 64, O 64, Z 64 = all 512.
-constexpr int kScanThreads = 736;
-constexpr int kScanDecay0 = 2, kScanZ0 = 10, kScanOut0 = 18, kScanVw = 22;  // first warps of the groups
+constexpr int kScanThreads = 768, kScanThreadsJoint = 640;
+constexpr int kScanVw = 2, kScanWatch = 3, kScanDecay0 = 4, kScanZ0 = 12, kScanOut0 = 20;  // first warps of the groups
 
 struct ScanSmem {
   // swizzled operand tiles, slabs of 32 columns (tc05.cuh): Q is read K-major, the others MN-major
@@ -656,11 +700,12 @@ struct ScanSmem {
   alignas(16) float d[2][kDim];
   alignas(8) uint64_t full_vw, full_d[2];
   uint64_t go_u;      // Tt, Z written (and the R before the last read):          1 load + 8 warps
-  uint64_t go_r;      // Yt, Q, the state of the last chunk, its O read:          2 loads + 1 commit + 4 warps
+  uint64_t go_r;      // Yt, Q, the state of the last chunk, its O read:          2 loads + 1 commit + the warps of O
   uint64_t go_s;      // Kn, At, decayed state, R:                                2 loads + 8 warps + 1 commit
   uint64_t vw_read;   // v, w are in registers:                                   8 warps
   uint64_t u_done, r_done, q_done, s_done, o_done, all_done;  // MMA commits
   volatile int failed;
+  volatile int prepared;  // chunks whose tiles may be loaded
   uint32_t tmem_base;
 };
 static_assert(sizeof(ScanSmem) <= 232448, "forward scan exceeds the 227 KiB shared-memory limit");
@@ -680,15 +725,16 @@ struct ScanMaps {
   CUtensorMap yt, q, kn, at, tt, v, w, out;
 };
 
-template <typename T, typename Seqs>
-__global__ void __launch_bounds__(kScanThreads, 1)
-chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ ScanMaps tm) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  ScanSmem& sm = *reinterpret_cast<ScanSmem*>(smem_raw);
+// One sequence and head, by a whole CTA.  kJoint: the prep groups run beside in the same launch, and a chunk's
+// tiles are loaded once its mark is there.
+template <typename T, typename Seqs, bool kJoint>
+__device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& seqs, const ScanMaps& tm, ScanSmem& sm,
+                                              const int item) {
+  constexpr int kThreads = kJoint ? kScanThreadsJoint : kScanThreads;
   BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int s = int(blockIdx.x) / p.H, h = int(blockIdx.x) - s * p.H;
+  const int s = item / p.H, h = item - s * p.H;
   const SeqInfo sq = seqs.at(s);
   const int n_chunks = sq.n_chunks;
   constexpr uint32_t kColS = 0, kColR = 256, kColO = 384, kColZ = 448;
@@ -703,7 +749,7 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
     mbar_init(&sm.full_d[0], 1);
     mbar_init(&sm.full_d[1], 1);
     mbar_init(&sm.go_u, 1 + 8);
-    mbar_init(&sm.go_r, 2 + 1 + 4);
+    mbar_init(&sm.go_r, 2 + 1 + (kJoint ? 8 : 4));
     mbar_init(&sm.go_s, 2 + 8 + 1);
     mbar_init(&sm.vw_read, 8);
     mbar_init(&sm.u_done, 1); mbar_init(&sm.r_done, 1); mbar_init(&sm.q_done, 1);
@@ -711,10 +757,11 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
     mbar_arrive(&sm.go_r);  // no earlier chunk holds up the first one
     // a wait that ran out in the prep kernel left garbage tiles: results become NaN from the start
     sm.failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
+    sm.prepared = 0;
     fence_mbar_init();
   }
   // lines 32..63 of the first slab of At and Tt (j >= 32, i < 32) are never loaded: zero, once
-  for (int e = tid; e < 4096 / 16; e += kScanThreads) {
+  for (int e = tid; e < 4096 / 16; e += kThreads) {
     reinterpret_cast<float4*>(sm.at + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     reinterpret_cast<float4*>(sm.tt + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -727,6 +774,49 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
+  };
+
+  // O of a chunk out, by whole sets of four warps (one per lane quadrant of tensor memory), each `kTokens` of
+  // the 64 tokens from i0 on
+  auto emit_o = [&](auto tokens, int c, int i0, int group0) {
+    constexpr int kTokens = decltype(tokens)::value, kGroup = 128 * (kChunk / kTokens);
+    const int vrow = 32 * (warp & 3) + lane;
+    const bool sender = tid == group0 * 32;
+    waiter.wait(&sm.o_done, uint32_t(c) & 1u);
+    tc_fence_after();
+    uint32_t x[kTokens];
+#pragma unroll
+    for (int j = 0; j < kTokens; j += 32) {
+      tmem_ld32(tmem_addr(tb, 32u * (warp & 3), kColO + i0 + j), *reinterpret_cast<uint32_t(*)[32]>(&x[j]));
+    }
+    tmem_wait_ld();
+    if (c + 1 < n_chunks) arrive(&sm.go_r);
+    const bool failed = sm.failed != 0;
+    if (sender) bulk_wait_read_all();  // the previous chunk's rows have left the buffer
+    asm volatile("bar.sync 4, %0;" ::"n"(kGroup) : "memory");
+    T* tile = reinterpret_cast<T*>(sm.o) + i0 * kDim + vrow;
+#pragma unroll
+    for (int j = 0; j < kTokens; j += 2) {
+      typename Pair<T>::type y = Pair<T>::make(__uint_as_float(x[j]), __uint_as_float(x[j + 1]));
+      if (failed) y = Pair<T>::make(poison_nan(), poison_nan());
+      tile[j * kDim] = y.x;
+      tile[(j + 1) * kDim] = y.y;
+    }
+    fence_async_smem();
+    asm volatile("bar.sync 4, %0;" ::"n"(kGroup) : "memory");
+    const int row = int(sq.row0) + c * kChunk, n_valid = min(kChunk, sq.len - c * kChunk);
+    if (n_valid == kChunk) {
+      if (sender) {
+        tma_store_3d(&tm.out, 0, h, row, sm.o);
+        bulk_commit();
+      }
+    } else {  // the rows behind a partial chunk (the last one) belong to somebody else
+      for (int e = tid - group0 * 32; e < n_valid * 16; e += kGroup) {
+        *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + (int64_t(row + (e >> 4)) * p.H + h) * kDim + 8 * (e & 15)) =
+            *reinterpret_cast<const uint4*>(sm.o + e * 16);
+      }
+    }
+    if (sender && c + 1 == n_chunks) bulk_wait_all();  // the last rows are in global memory before the CTA retires
   };
 
   if (warp == 0) {
@@ -762,24 +852,33 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       mbar_arrive_expect_tx(&sm.go_s, uint32_t(kTileAt - 4096), leader);
       load_tri(sm.at, &tm.at, int(ch_of(c)), &sm.go_s);
     };
+    auto ready = [&](int c) {
+      if constexpr (kJoint) {
+        // (the watching warp gives up by itself and then lets everything pass)
+        for (uint32_t looks = 0; sm.prepared <= c && looks < (1u << 27); ++looks) __nanosleep(20);
+        __threadfence_block();
+        fence_async_all();
+      }
+    };
+    ready(0);
     load_t(0);
     load_y(0);
     load_d(0);
     load_q(0);
     load_k(0);
     load_a(0);
-    if (n_chunks > 1) load_d(1);
     for (int c = 1; c < n_chunks; ++c) {
       const uint32_t par = uint32_t(c - 1) & 1u;
       waiter.wait(&sm.u_done, par);
+      ready(c);
       load_t(c);
+      load_d(c);  // (the decay of chunk c - 2, which had the slot, has run)
       waiter.wait(&sm.r_done, par);
       load_y(c);
       waiter.wait(&sm.q_done, par);
       load_q(c);
       waiter.wait(&sm.s_done, par);
       load_k(c);
-      if (c + 1 < n_chunks) load_d(c + 1);  // the decay of chunk c - 1 has run: its slot is free
       waiter.wait(&sm.o_done, par);
       load_a(c);
     }
@@ -844,7 +943,7 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       if (c + 1 < n_chunks) issue_u(c + 1);
     }
     mma_commit(&sm.all_done, leader);
-  } else if (warp < kScanZ0) {
+  } else if (warp >= kScanDecay0 && warp < kScanZ0) {
     // ---------------------------------------------------------------- decay of the state
     // thread = value row of the transposed state (TMEM lane) x one half of the 128 key columns
     const int q4 = warp & 3, half = (warp - kScanDecay0) >> 2;
@@ -902,14 +1001,14 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       for (int j4 = 0; j4 < 8; ++j4) {
         const float4 da = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 4 * j4]);
         const float4 db = *reinterpret_cast<const float4*>(&sm.d[par][k0 + 32 + 4 * j4]);
-        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * da.x);
-        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * da.y);
-        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * da.z);
-        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * da.w);
-        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * db.x);
-        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * db.y);
-        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * db.z);
-        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * db.w);
+        lo[4 * j4 + 0] = __float_as_uint(__uint_as_float(lo[4 * j4 + 0]) * fabsf(da.x));
+        lo[4 * j4 + 1] = __float_as_uint(__uint_as_float(lo[4 * j4 + 1]) * fabsf(da.y));
+        lo[4 * j4 + 2] = __float_as_uint(__uint_as_float(lo[4 * j4 + 2]) * fabsf(da.z));
+        lo[4 * j4 + 3] = __float_as_uint(__uint_as_float(lo[4 * j4 + 3]) * fabsf(da.w));
+        hi[4 * j4 + 0] = __float_as_uint(__uint_as_float(hi[4 * j4 + 0]) * fabsf(db.x));
+        hi[4 * j4 + 1] = __float_as_uint(__uint_as_float(hi[4 * j4 + 1]) * fabsf(db.y));
+        hi[4 * j4 + 2] = __float_as_uint(__uint_as_float(hi[4 * j4 + 2]) * fabsf(db.z));
+        hi[4 * j4 + 3] = __float_as_uint(__uint_as_float(hi[4 * j4 + 3]) * fabsf(db.w));
       }
       // (the other buffer: its readers, R and O of chunk c - 1, ran before the update that s_done stands for)
       store_state(kColS + 128u * (par ^ 1u));
@@ -940,29 +1039,29 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       if (ck != nullptr) ck[(k0 + j) * kDim] = x;
     }
     if (sender) bulk_wait_all();  // the last staged rows are in global memory before the CTA retires
-  } else if (warp < kScanOut0) {
-    // ---------------------------------------------------------------- Z = w v
+  } else if (warp >= kScanZ0 && (kJoint || warp < kScanOut0)) {
+    // ---------------------------------------------------------------- Z = w v (and in a joint launch O out)
     // thread = value row (TMEM lane) x one half of the 64 tokens
     const int q4 = warp & 3, half = (warp - kScanZ0) >> 2;
     const int vrow = 32 * q4 + lane, i0 = 32 * half;
     const uint32_t lane_base = 32u * q4;
     const T* vs = reinterpret_cast<const T*>(sm.v) + i0 * kDim + vrow;
     const T* wsrc = reinterpret_cast<const T*>(sm.w) + i0 * kDim + vrow;
-    uint32_t x[32];
+    uint32_t a[32];
     // R of chunk c for backward, row-major R[j][v]: the 32 lanes of a warp fill one 128-byte line per token
     auto load_residual = [&](int c) {
-      tmem_ld32(tmem_addr(tb, lane_base, kColR + 64u * (uint32_t(c) & 1u) + i0), x);
+      tmem_ld32(tmem_addr(tb, lane_base, kColR + 64u * (uint32_t(c) & 1u) + i0), a);
       tmem_wait_ld();
     };
     auto store_residual = [&](int c) {
       float* rn = p.rn + ch_of(c) * (kBlobRn / 4) + i0 * kDim + vrow;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) rn[j * kDim] = to_tf32(__uint_as_float(x[j]));
+      for (int j = 0; j < 32; ++j) rn[j * kDim] = to_tf32(__uint_as_float(a[j]));
     };
-    for (int c = 0; c < n_chunks; ++c) {
+    auto build_z = [&](int c) {
       waiter.wait(&sm.full_vw, uint32_t(c) & 1u);
       const int n_valid = sq.len - c * kChunk;
-      // 16 tokens at a time: all 32 with their activations in flight would not fit the registers
+      // 16 tokens at a time: more with their activations in flight would not fit the registers
 #pragma unroll
       for (int part = 0; part < 2; ++part) {
         T vr[16];
@@ -997,6 +1096,12 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       if (p.rn != nullptr && c > 1) load_residual(c - 2);  // before its columns take the R of this chunk
       arrive(&sm.go_u);
       if (p.rn != nullptr && c > 1) store_residual(c - 2);
+    };
+    if constexpr (kJoint) arrive(&sm.go_r);  // no earlier chunk holds up the first output
+    build_z(0);
+    for (int c = 0; c < n_chunks; ++c) {
+      if (c + 1 < n_chunks) build_z(c + 1);
+      if constexpr (kJoint) emit_o(std::integral_constant<int, 32>{}, c, i0, kScanZ0);
     }
     if (p.rn != nullptr) {
       waiter.wait(&sm.all_done, 0);
@@ -1006,57 +1111,11 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
         store_residual(c);
       }
     }
-  } else if (warp < kScanVw) {
+  } else if (!kJoint && warp >= kScanOut0) {
     // ---------------------------------------------------------------- O out
-    // thread = value row (TMEM lane)
-    const int q4 = warp & 3;
-    const int vrow = 32 * q4 + lane;
-    const uint32_t lane_base = 32u * q4;
-    const bool sender = tid == kScanOut0 * 32;
-    auto group_barrier = [&] { asm volatile("bar.sync 4, 128;" ::: "memory"); };
     arrive(&sm.go_r);  // no earlier chunk holds up the first output
-    for (int c = 0; c < n_chunks; ++c) {
-      waiter.wait(&sm.o_done, uint32_t(c) & 1u);
-      tc_fence_after();
-      uint32_t a[32], b[32];
-      tmem_ld32(tmem_addr(tb, lane_base, kColO), a);
-      tmem_ld32(tmem_addr(tb, lane_base, kColO + 32), b);
-      tmem_wait_ld();
-      if (c + 1 < n_chunks) arrive(&sm.go_r);
-      const bool failed = sm.failed != 0;
-      if (sender) bulk_wait_read_all();  // the previous chunk's rows have left the buffer
-      group_barrier();
-      T* tile = reinterpret_cast<T*>(sm.o) + vrow;
-      if (failed) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) a[j] = b[j] = __float_as_uint(poison_nan());
-      }
-#pragma unroll
-      for (int j = 0; j < 32; j += 2) {
-        const typename Pair<T>::type x = Pair<T>::make(__uint_as_float(a[j]), __uint_as_float(a[j + 1]));
-        const typename Pair<T>::type y = Pair<T>::make(__uint_as_float(b[j]), __uint_as_float(b[j + 1]));
-        tile[j * kDim] = x.x;
-        tile[(j + 1) * kDim] = x.y;
-        tile[(j + 32) * kDim] = y.x;
-        tile[(j + 33) * kDim] = y.y;
-      }
-      fence_async_smem();
-      group_barrier();
-      const int row = int(sq.row0) + c * kChunk, n_valid = min(kChunk, sq.len - c * kChunk);
-      if (n_valid == kChunk) {
-        if (sender) {
-          tma_store_3d(&tm.out, 0, h, row, sm.o);
-          bulk_commit();
-        }
-      } else {  // the rows behind a partial chunk (the last one) belong to somebody else
-        for (int e = tid - kScanOut0 * 32; e < n_valid * 16; e += 128) {
-          *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + (int64_t(row + (e >> 4)) * p.H + h) * kDim + 8 * (e & 15)) =
-              *reinterpret_cast<const uint4*>(sm.o + e * 16);
-        }
-      }
-    }
-    if (sender) bulk_wait_all();  // the last rows are in global memory before the CTA retires
-  } else {
+    for (int c = 0; c < n_chunks; ++c) emit_o(std::integral_constant<int, 64>{}, c, 0, kScanOut0);
+  } else if (warp == kScanVw) {
     // ---------------------------------------------------------------- v and w
     const uint32_t leader = elect_leader();
     auto load_vw = [&](int c) {
@@ -1070,6 +1129,26 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
       waiter.wait(&sm.vw_read, uint32_t(c - 1) & 1u);
       load_vw(c);
     }
+  } else if (kJoint && warp == kScanWatch) {
+    // ---------------------------------------------------------------- marks of prepared chunks
+    for (int c = 0; c < n_chunks;) {
+      const int mine = min(c + lane, n_chunks - 1);
+      const uint32_t missing = ~__ballot_sync(0xffffffffu, marked(reinterpret_cast<const float*>(p.d + ch_of(mine) * kBlobD)));
+      const int there = missing == 0 ? 32 : __ffs(int(missing)) - 1;
+      if (there == 0) {
+        if (!waiter.look_again()) c = n_chunks;
+        __nanosleep(200);
+      } else {
+        c = min(c + there, n_chunks);
+      }
+      // (a wait of a preparer that ran out, or this one's own: results become NaN)
+      if (*static_cast<volatile const int*>(p.status) != kStatusOk) sm.failed = 1;
+      __syncwarp();
+      if (lane == 0 && c > 0) {
+        __threadfence_block();
+        sm.prepared = c;
+      }
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -1077,6 +1156,68 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
     tc_fence_after();
     tmem_dealloc(tb, 512);
   }
+}
+
+template <typename T, typename Seqs>
+__global__ void __launch_bounds__(kScanThreads, 1)
+chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ ScanMaps tm) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  scan_sequence<T, Seqs, false>(p, seqs, tm, *reinterpret_cast<ScanSmem*>(smem_raw), int(blockIdx.x));
+}
+
+// ---------------------------------------------------------------------------------------------
+// prep and scan in one launch
+// ---------------------------------------------------------------------------------------------
+// With few sequences and heads the scan is a serial chain on a few SMs (1.85 us per chunk) while the others
+// idle, and it starts when the last prep unit is done.  Here some CTAs scan and the others prepare, chunk by
+// chunk; the tiles are still in L2 when the scan reads them.  The scans wait for the preparers, which wait
+// for nobody; the launch is cooperative, so that all CTAs are resident together.
+// The two SMs of a pair share their way to L2: with a preparer beside it a scan took 3.3 us per chunk.  So the
+// CTAs come in clusters of two, the first n_scan clusters scan with one CTA and leave the other idle unless
+// (`mates`) the preparation would be the longer part.
+// Registers: 640 threads x 96 at launch; a preparing CTA gives its two groups of 256 threads 112 each and the
+// four warps left 32 (16 * 112 + 4 * 32 = 20 * 96).
+constexpr int kJointRegs = 96;
+struct JointSmem {
+  PrepSmem prep[2];
+};
+template <typename T, typename G, typename Seqs, bool kPro>
+__global__ void __launch_bounds__(kScanThreadsJoint, 1) __cluster_dims__(2, 1, 1)
+chunk_joint_kernel(const PrepParams pp, const ScanParams sp, const __grid_constant__ Seqs seqs,
+                   const __grid_constant__ PrepMaps tm_prep, const __grid_constant__ ScanMaps tm_scan,
+                   const int mates) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  const int n_scan = seqs.count() * sp.H, pair = int(blockIdx.x) >> 1, mate = int(blockIdx.x) & 1;
+  if (pair < n_scan && mate == 0) {
+    scan_sequence<T, Seqs, true>(sp, seqs, tm_scan, *reinterpret_cast<ScanSmem*>(smem_raw), pair);
+    return;
+  }
+  if (pair < n_scan && !mates) return;
+  // number of this CTA among those that prepare: whole pairs first
+  const int n_whole = int(gridDim.x) - 2 * n_scan;
+  const int nr = pair < n_scan ? n_whole + pair : int(blockIdx.x) - 2 * n_scan;
+  const int n_groups = 2 * (n_whole + (mates ? n_scan : 0));
+  JointSmem& sm = *reinterpret_cast<JointSmem*>(smem_raw);
+  const int tid = threadIdx.x;
+  if (tid < 32) {
+    tmem_alloc(&sm.prep[0].tmem_base, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tb = sm.prep[0].tmem_base;
+  if (tid >= 512) {  // (nothing may follow for these warps: code behind a join is compiled for the others' registers)
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
+    return;
+  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
+  const int group = tid >> 8;
+  prep_units<T, G, Seqs, kPro, true>(pp, seqs, tm_prep, sm.prep[group], tid & 255, tb + 256u * group,
+                                     group * (n_groups / 2) + nr, n_groups, 1 + group, sp.status + kQueueWord);
+  tc_fence_before();
+  asm volatile("bar.sync 3, 512;" ::: "memory");
+  if (tid < 32) tmem_dealloc(tb, 512);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1144,6 +1285,52 @@ struct ForwardCall {
   int prologue;
 };
 
+// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation) and 2-3 us per chunk
+// (the scans); together the longer of the two, the first units taking some 35 us and a scan 0.4 us per chunk
+// more beside preparers.  Beyond a quarter of the SMs scanning, the preparation falls behind.
+bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, int sm_count) {
+  return 4 * n_scan <= sm_count && 83 * n_ch > (350 + 4 * n_chunks) * sm_count && !profiling();
+}
+
+template <typename T, typename G, typename Seqs, bool kPro>
+int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, const PrepMaps& tm_prep,
+                 const ScanMaps& tm_scan, int sm_count, cudaStream_t stream) {
+  constexpr int smem = int(sizeof(JointSmem) > sizeof(ScanSmem) ? sizeof(JointSmem) : sizeof(ScanSmem));
+  static_assert(smem <= 232448, "joint kernel exceeds the 227 KiB shared-memory limit");
+  auto kernel = chunk_joint_kernel<T, G, Seqs, kPro>;
+  cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  // the register split of the kernel is only valid for the launch allocation it was written for
+  static const int regs = [&] {
+    cudaFuncAttributes attr;
+    return cudaFuncGetAttributes(&attr, kernel) == cudaSuccess ? attr.numRegs : -1;
+  }();
+  if (regs != kJointRegs) return GDN2_ERR_UNSUPPORTED;  // (the caller then takes two launches)
+  const int n_scan = seqs.count() * sp.H;
+  // clusters of two CTAs; no more preparers than pairs of units
+  const int64_t want = n_scan + (pp.n_ch + 3) / 4;
+  const int clusters = int(want < sm_count / 2 ? want : sm_count / 2);
+  // per chunk the scans take 2 us (3 with a preparer beside them), a unit 9.5 us on one SM
+  const int mates = 95 * n_scan > 20 * (2 * (clusters - n_scan)) || clusters == n_scan;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(unsigned(2 * clusters));
+  config.blockDim = dim3(kScanThreadsJoint);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute together;
+  together.id = cudaLaunchAttributeCooperative;
+  together.val.cooperative = 1;
+  config.attrs = &together;
+  config.numAttrs = 1;
+  err = cudaLaunchKernelEx(&config, kernel, pp, sp, seqs, tm_prep, tm_scan, mates);
+  if (err == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs than the device
+    (void)cudaGetLastError();
+    return GDN2_ERR_UNSUPPORTED;
+  }
+  if (err != cudaSuccess) { (void)cudaGetLastError(); record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  return GDN2_OK;
+}
+
 template <typename Seqs>
 int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) {
   const int64_t n_ch = int64_t(seqs.total_chunks()) * a.H;
@@ -1151,9 +1338,6 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (n_ch <= 0 || n_ch > int64_t(0x7fffffff) || a.rows > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
   const WsLayout ws{n_ch, a.training != 0};
   int* status = reinterpret_cast<int*>(a.workspace + ws.off_status());
-  cudaError_t err = cudaMemsetAsync(status, 0, kStatusBytes, stream);
-  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-
   const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
   PrepMaps tm_prep;
   ScanMaps tm;
@@ -1175,9 +1359,30 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   int sm_count = 0;
   if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
 
+  const PrepParams pp{a.workspace, tiles, n_ch, int(a.H), a.scale, a.training, a.prologue};
+  const ScanParams sp{a.workspace + ws.off_d(), a.s_in, a.out, a.s_out, a.bnd,
+                      a.training ? reinterpret_cast<float*>(a.workspace + ws.off_rn()) : nullptr,
+                      status, int(a.H), (a.prologue & kPrologueGate) != 0};
+  const int64_t n_scan = int64_t(seqs.count()) * a.H;
+  cudaError_t err;
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
+    if (prefer_joint(n_scan, n_ch, seqs.n_chunks, sm_count)) {
+      // the marks of finished units are in D, right before the status block: one fill clears both
+      err = cudaMemsetAsync(a.workspace + ws.off_d(), 0, size_t(n_ch) * kBlobD + kStatusBytes, stream);
+      if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+      int st = GDN2_OK;
+      GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
+        st = a.prologue != 0 ? launch_joint<T, G, Seqs, true>(pp, sp, seqs, tm_prep, tm, sm_count, stream)
+                             : launch_joint<T, G, Seqs, false>(pp, sp, seqs, tm_prep, tm, sm_count, stream);
+      });
+      if (st != GDN2_ERR_UNSUPPORTED) return st;
+    }
+  }
+  err = cudaMemsetAsync(status, 0, kStatusBytes, stream);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+
   profile_mark(0, stream);
   const unsigned prep_grid = unsigned(n_ch < 2 * int64_t(sm_count) ? n_ch : 2 * int64_t(sm_count));
-  const PrepParams pp{a.workspace, tiles, n_ch, int(a.H), a.scale, a.training, a.prologue};
   GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
     auto kernel = a.prologue != 0 ? chunk_prep_kernel<T, G, Seqs, true> : chunk_prep_kernel<T, G, Seqs, false>;
     const int smem = int(sizeof(PrepSmem));
@@ -1189,11 +1394,8 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (st != GDN2_OK) return st;
   profile_mark(1, stream);
 
-  const ScanParams sp{a.workspace + ws.off_d(), a.s_in, a.out, a.s_out, a.bnd,
-                      a.training ? reinterpret_cast<float*>(a.workspace + ws.off_rn()) : nullptr,
-                      status, int(a.H), (a.prologue & kPrologueGate) != 0};
   const int smem = int(sizeof(ScanSmem));
-  const unsigned grid = unsigned(seqs.count() * a.H);
+  const unsigned grid = unsigned(n_scan);
   auto kernel = a.dtype == GDN2_BF16 ? chunk_scan_kernel<__nv_bfloat16, Seqs> : chunk_scan_kernel<__half, Seqs>;
   err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }

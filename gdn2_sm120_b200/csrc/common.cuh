@@ -118,6 +118,7 @@ void record_cuda_error(cudaError_t err);  // defined in api.cu
 int check_launch();                       // cudaGetLastError -> status
 int multiprocessors(int* count);          // SMs of the current device, looked up once per device (api.cu)
 cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);  // once per (kernel, device) opt-in (api.cu)
+bool profiling();  // per-kernel timing is on: the kernels of a call then run one by one (api.cu)
 void profile_mark(int index, cudaStream_t stream);  // records timing event `index` when profiling is on (api.cu)
 
 inline bool valid_seq_dtype(int d) { return d == GDN2_BF16 || d == GDN2_FP16; }
