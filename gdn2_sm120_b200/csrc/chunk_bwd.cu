@@ -517,23 +517,48 @@ __device__ __forceinline__ void store4v<__half>(void* base, int64_t idx, float a
       make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
-// tf32 value of k times its anchored decay, as stored in the (K^I)^T tiles: `decay` alone, or
-// `decay * far` for row blocks beyond the next one.  Tile build and chain both call this, so that the
-// chain multiplies the Gram cotangents by exactly the operand values the tensor cores saw.
-__device__ __forceinline__ float anchored_k(float k, float decay, float far, bool use_far) {
-  return to_tf32(k * (use_far ? decay * far : decay));
+// Two fp32 operations per instruction (each rounded like the scalar one): the VJP kernel's elementwise phases
+// are bound by instruction issue.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
 }
-// the same product for the tile itself, which only the tensor cores read (they drop the low bits themselves)
-__device__ __forceinline__ float anchored_k_operand(float k, float decay, float far, bool use_far) {
-  return to_tf32_operand(k * (use_far ? decay * far : decay));
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return fma2(b, twice(-1.f), a); }
+__device__ __forceinline__ float2 exp2_2(float2 x) { return make_float2(exp2_approx(x.x), exp2_approx(x.y)); }
+__device__ __forceinline__ float2 tf32_2(float2 x) { return make_float2(to_tf32(x.x), to_tf32(x.y)); }
+__device__ __forceinline__ float2 tf32_operand_2(float2 x) { return make_float2(to_tf32_operand(x.x), to_tf32_operand(x.y)); }
+
+// The value of k times its anchored decay, `decay` alone or `decay * far` for row blocks beyond the next one:
+// the chain calls this with the factors of the tile build, so that it multiplies the Gram cotangents by
+// exactly the operand values the tensor cores saw.
+__device__ __forceinline__ float2 anchored_k(float2 k, float2 decay, float2 far, bool use_far) {
+  return mul2(k, use_far ? mul2(decay, far) : decay);
 }
 
-__device__ __forceinline__ void tmem_ld8f(uint32_t taddr, float (&x)[8]) {
+__device__ __forceinline__ void tmem_ld4x2(uint32_t taddr, float2 (&x)[4]) {
   uint32_t r[8];
   tmem_ld8(taddr, r);
   tmem_wait_ld();
 #pragma unroll
-  for (int i = 0; i < 8; ++i) x[i] = __uint_as_float(r[i]);
+  for (int i = 0; i < 4; ++i) x[i] = make_float2(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
 }
 
 // kF32Grads: dq, dk, dv, dbeta, dw leave as fp32 instead of the sequence dtype (the values before
@@ -678,14 +703,12 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
       const int i = 4 * tg + e;
       *reinterpret_cast<float4*>(smem + kOffStack + ((64 + i) >> 3) * kRsN + c4 * kCsN + (i & 7) * 16) =
           make_float4(dv4[e][0], dv4[e][1], dv4[e][2], dv4[e][3]);
-      if (e > 0) {
+      // (log-decays in units of ln 2: a decay is one ex2)
 #pragma unroll
-        for (int f = 0; f < 4; ++f) Gc[e][f] += Gc[e - 1][f];
-      }
+      for (int f = 0; f < 4; ++f) Gc[e][f] = e > 0 ? fmaf(Gc[e][f], kLog2e, Gc[e - 1][f]) : Gc[e][f] * kLog2e;
     }
   }
-#pragma unroll
-  for (int f = 0; f < 4; ++f) ms.part[tg][kc0 + f] = Gc[3][f];
+  *reinterpret_cast<float4*>(&ms.part[tg][kc0]) = make_float4(Gc[3][0], Gc[3][1], Gc[3][2], Gc[3][3]);
   waiter.wait(&ms.bar_a, par);
   waiter.wait(&ms.bar_s, par);
   dd_half(0);
@@ -726,12 +749,13 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   // Gram operands.  Every load is issued before the first store: the outputs may alias the inputs as
   // far as the compiler knows, so a load placed after a store would wait for its round trip.
   if (tid < kDim) {
-    float run = 0.f;
+    float x[16], run = 0.f;  // (all read before the first is written: the reads wait together)
+#pragma unroll
+    for (int t = 0; t < 16; ++t) x[t] = ms.part[t][tid];
 #pragma unroll
     for (int t = 0; t < 16; ++t) {
-      const float x = ms.part[t][tid];
       ms.part[t][tid] = run;
-      run += x;
+      run += x[t];
     }
     ms.gend[tid] = run;
   }
@@ -832,51 +856,55 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   waiter.wait(&ms.bar_r, 1);
   tc_fence_after();
   {
-    float eat[4][4], qat[4][4];
+    auto row4 = [&](const float* row, float (&x)[4]) {
+      const float4 y = *reinterpret_cast<const float4*>(row + kc0);
+      x[0] = y.x; x[1] = y.y; x[2] = y.z; x[3] = y.w;
+    };
+    float base[4], a_blk[4][4], end[4];
+    row4(ms.part[tg], base);
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        const int kc = kc0 + f;
-        const float Gi = Gc[e][f] + ms.part[tg][kc];
-        Gc[e][f] = Gi;
-        const float anchored = __expf(Gi - ms.part[4 * mb][kc]);
-        eat[e][f] = to_tf32_operand(bb[e][f] * kk[e][f] * anchored);
-        qat[e][f] = to_tf32_operand(p.scale * qq[e][f] * anchored);
-      }
-    }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) {
-      const uint32_t off = blk_off<4>(kc0 + f, 4 * tg, kRsT, 128);
-      *reinterpret_cast<float4*>(smem + kOffEat + off) = make_float4(eat[0][f], eat[1][f], eat[2][f], eat[3][f]);
-      *reinterpret_cast<float4*>(smem + kOffQat + off) = make_float4(qat[0][f], qat[1][f], qat[2][f], qat[3][f]);
-    }
-    // (K^I)^T for every row block I >= the token's own block mb, three exponentials per element:
+    for (int I = 0; I < 4; ++I) row4(ms.part[4 * I], a_blk[I]);
+    row4(ms.gend, end);
+    // Ea, Qa: anchored at the start of the token's own block.  (K^I)^T for every row block I >= the own block
+    // mb, two exponentials per element in all:
     //   I = mb      k exp(a_mb - G)                      (own block: >= 1, bounded by the 16-token contract)
     //   I = mb + 1  k exp(a_next - G)                    (a_next = start of the next block)
     //   I > mb + 1  k (exp(a_next - G) exp(a_I - a_next))
-    // The final chain forms the same products with the same expressions (anchored_k below).
+    // The final chain forms the same products with the same expressions (anchored_k above).
 #pragma unroll
     for (int f = 0; f < 4; ++f) {
       const int kc = kc0 + f;
-      const float a_mb = ms.part[4 * mb][kc];
-      const float a_nx = (mb < 3) ? ms.part[4 * (mb + 1)][kc] : ms.gend[kc];
-      const float c_nx = __expf(a_nx - a_mb);  // decay over the whole 16-token block
-      float own[4], nb[4];
+      const float a_mb = mb == 0 ? a_blk[0][f] : mb == 1 ? a_blk[1][f] : mb == 2 ? a_blk[2][f] : a_blk[3][f];
+      const float a_nx = mb == 0 ? a_blk[1][f] : mb == 1 ? a_blk[2][f] : mb == 2 ? a_blk[3][f] : end[f];
+      const float c_nx = exp2_approx(a_nx - a_mb);  // decay over the whole 16-token block
+      float2 k2[2], own[2], nb[2], ea[2], qa[2];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        own[e] = __expf(a_mb - Gc[e][f]);
-        nb[e] = own[e] * c_nx;                 // exp(a_nx - G): the chain forms it the same way
+      for (int x = 0; x < 2; ++x) {
+        const float2 G = add2(make_float2(Gc[2 * x][f], Gc[2 * x + 1][f]), twice(base[f]));
+        Gc[2 * x][f] = G.x;
+        Gc[2 * x + 1][f] = G.y;
+        const float2 to_anchor = minus2(twice(a_mb), G);
+        const float2 anchored = exp2_2(make_float2(-to_anchor.x, -to_anchor.y));
+        k2[x] = make_float2(kk[2 * x][f], kk[2 * x + 1][f]);
+        ea[x] = tf32_operand_2(mul2(mul2(make_float2(bb[2 * x][f], bb[2 * x + 1][f]), k2[x]), anchored));
+        qa[x] = tf32_operand_2(mul2(mul2(twice(p.scale), make_float2(qq[2 * x][f], qq[2 * x + 1][f])), anchored));
+        own[x] = exp2_2(to_anchor);
+        nb[x] = mul2(own[x], twice(c_nx));           // exp(a_nx - G): the chain forms it the same way
       }
+      const uint32_t off = blk_off<4>(kc, 4 * tg, kRsT, 128);
+      *reinterpret_cast<float4*>(smem + kOffEat + off) = make_float4(ea[0].x, ea[0].y, ea[1].x, ea[1].y);
+      *reinterpret_cast<float4*>(smem + kOffQat + off) = make_float4(qa[0].x, qa[0].y, qa[1].x, qa[1].y);
 #pragma unroll
       for (int I = 0; I < 4; ++I) {
         if (I >= mb) {
-          const float far = (I > mb + 1) ? __expf(ms.part[4 * I][kc] - a_nx) : 1.f;
-          float val[4];
+          const float far = (I > mb + 1) ? exp2_approx(a_blk[I][f] - a_nx) : 1.f;
+          float2 val[2];
 #pragma unroll
-          for (int e = 0; e < 4; ++e) val[e] = anchored_k_operand(kk[e][f], (I == mb) ? own[e] : nb[e], far, I > mb + 1);
+          for (int x = 0; x < 2; ++x) {
+            val[x] = tf32_operand_2(anchored_k(k2[x], (I == mb) ? own[x] : nb[x], twice(far), I > mb + 1));
+          }
           *reinterpret_cast<float4*>(smem + kit_offset(I) + blk_off<4>(kc, 4 * tg, kit_rs(I), 128)) =
-              make_float4(val[0], val[1], val[2], val[3]);
+              make_float4(val[0].x, val[0].y, val[1].x, val[1].y);
         }
       }
     }
@@ -963,107 +991,111 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
     const float a_me = ms.part[4 * blk][kc];
     const float a_nx = (blk < 3) ? ms.part[4 * (blk + 1)][kc] : gend;
     // per-thread constants: everything but three exponentials per token comes from these
-    const float e_ame = __expf(a_me);            // exp(G) = exp(G - a_me) e_ame
-    const float c_nx = __expf(a_nx - a_me);      // exp(a_next - G) = exp(a_me - G) c_nx, as in the tile build
-    const float t_end = __expf(gend - a_nx);     // exp(G_end - G) = exp(a_next - G) t_end
-    const float far2 = (blk + 2 < 4) ? __expf(ms.part[4 * (blk + 2)][kc] - a_nx) : 1.f;  // row block blk + 2
-    const float far3 = (blk + 3 < 4) ? __expf(ms.part[4 * (blk + 3)][kc] - a_nx) : 1.f;  // row block blk + 3
+    const float e_ame = exp2_approx(a_me);            // exp(G) = exp(G - a_me) e_ame
+    const float c_nx = exp2_approx(a_nx - a_me);      // exp(a_next - G) = exp(a_me - G) c_nx, as in the tile build
+    const float t_end = exp2_approx(gend - a_nx);     // exp(G_end - G) = exp(a_next - G) t_end
+    const float far2 = (blk + 2 < 4) ? exp2_approx(ms.part[4 * (blk + 2)][kc] - a_nx) : 1.f;  // row block blk + 2
+    const float far3 = (blk + 3 < 4) ? exp2_approx(ms.part[4 * (blk + 3)][kc] - a_nx) : 1.f;  // row block blk + 3
     // dG of a token goes back into the slot of the G tile this thread read its log-decay from (nobody else
     // touches it), and the two halves of the block run as a loop: the kernel is a long stretch of
     // straight-line code that every warp walks once per unit, and what it does not need to hold twice
     // saves instruction fetches
-    float e_part = 0.f, tot = 0.f;
+    // Two tokens per instruction throughout; -k in place of k where the contribution to dG is negative.
+    float2 e_part = twice(0.f), tot = twice(0.f);  // (e_part: negated)
 #pragma unroll 1
     for (int sb = 0; sb < 2; ++sb) {
       const int i0 = 16 * blk + 8 * sb;
-      float Gb[8], kv[8], bv[8], sq[8], P3[8], P2[8], dG[8], x[8], y[8];
+      float2 ea[4], nk[4], kv[4], bv[4], sq[4], nb[4], P3[4], P2[4], dG[4], x[4], y[4];
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const int off = (i0 + t) * kDim + kc;
-        Gb[t] = ldf<float>(smem + kOffTileG, off);
-        kv[t] = ldf<T>(smem + kOffTileK, off);
-        sq[t] = p.scale * ldf<T>(smem + kOffTileQ, off);
-        bv[t] = ldf<T>(smem + beta_tile_offset(blk), (8 * sb + t) * kDim + kc);
+      for (int t = 0; t < 4; ++t) {
+        const int off = (i0 + 2 * t) * kDim + kc, off_b = (8 * sb + 2 * t) * kDim + kc;
+        ea[t] = make_float2(ldf<float>(smem + kOffTileG, off), ldf<float>(smem + kOffTileG, off + kDim));
+        kv[t] = make_float2(ldf<T>(smem + kOffTileK, off), ldf<T>(smem + kOffTileK, off + kDim));
+        sq[t] = mul2(twice(p.scale), make_float2(ldf<T>(smem + kOffTileQ, off), ldf<T>(smem + kOffTileQ, off + kDim)));
+        bv[t] = make_float2(ldf<T>(smem + beta_tile_offset(blk), off_b), ldf<T>(smem + beta_tile_offset(blk), off_b + kDim));
       }
       // row blocks I = blk + d that contain these tokens as columns, nearest first: the own block uses
       // exp(a_me - G), the others exp(a_next - G) (times the block-to-block factor from d = 2 on)
-      tmem_ld8f(tmem_addr(tb, 32 * q4, d6_col(blk) + i0), x);  // dK^blk
-      float nb[8];
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, d6_col(blk) + i0), x);  // dK^blk
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float own = __expf(a_me - Gb[t]);
-        nb[t] = own * c_nx;
-        Gb[t] = __expf(Gb[t] - a_me);  // from here on Gb holds the anchored decay exp(G - a_me)
-        P3[t] = x[t] * own;
-        dG[t] = -anchored_k(kv[t], own, 1.f, false) * x[t];
+      for (int t = 0; t < 4; ++t) {
+        const float2 to_anchor = minus2(twice(a_me), ea[t]);
+        const float2 own = exp2_2(to_anchor);
+        nk[t] = make_float2(-kv[t].x, -kv[t].y);
+        nb[t] = mul2(own, twice(c_nx));
+        ea[t] = exp2_2(make_float2(-to_anchor.x, -to_anchor.y));  // the anchored decay exp(G - a_me)
+        P3[t] = mul2(x[t], own);
+        dG[t] = mul2(tf32_2(anchored_k(nk[t], own, twice(1.f), false)), x[t]);
       }
-      tmem_ld8f(tmem_addr(tb, 32 * q4, kColD4 + i0), x);  // dKt
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, kColD4 + i0), x);  // dKt
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float et = nb[t] * t_end;
-        const float kt = kv[t] * et;
-        P3[t] = fmaf(x[t], et, P3[t]);
-        e_part = fmaf(kt, x[t], e_part);
-        dG[t] = fmaf(-kt, x[t], dG[t]);
+      for (int t = 0; t < 4; ++t) {
+        const float2 et = mul2(nb[t], twice(t_end));
+        const float2 nkt = mul2(nk[t], et);
+        P3[t] = fma2(x[t], et, P3[t]);
+        e_part = fma2(nkt, x[t], e_part);
+        dG[t] = fma2(nkt, x[t], dG[t]);
       }
 #pragma unroll
       for (int d = 1; d < 4; ++d) {
         if (blk + d < 4) {
-          const float far = (d == 2) ? far2 : far3;
-          tmem_ld8f(tmem_addr(tb, 32 * q4, d6_col(blk + d) + i0), x);  // dK^(blk + d)
+          const float2 far = twice((d == 2) ? far2 : far3);
+          tmem_ld4x2(tmem_addr(tb, 32 * q4, d6_col(blk + d) + i0), x);  // dK^(blk + d)
 #pragma unroll
-          for (int t = 0; t < 8; ++t) {
-            const float ex = (d > 1) ? nb[t] * far : nb[t];
-            P3[t] = fmaf(x[t], ex, P3[t]);
-            dG[t] = fmaf(-anchored_k(kv[t], nb[t], far, d > 1), x[t], dG[t]);
+          for (int t = 0; t < 4; ++t) {
+            P3[t] = fma2(x[t], (d > 1) ? mul2(nb[t], far) : nb[t], P3[t]);
+            dG[t] = fma2(tf32_2(anchored_k(nk[t], nb[t], far, d > 1)), x[t], dG[t]);
           }
         }
       }
-      tmem_ld8f(tmem_addr(tb, 32 * q4, kColD3 + i0), x);  // -dE (state part)
-      tmem_ld8f(tmem_addr(tb, 32 * q4, kColD5 + 32 * blk + 8 * sb), y);  // dEa
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, kColD3 + i0), x);  // -dE (state part)
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, kColD5 + 32 * blk + 8 * sb), y);  // dEa
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const float ea = Gb[t], eg = ea * e_ame;
-        const float de = -x[t], dea = y[t];
-        P2[t] = fmaf(de, eg, dea * ea);
-        const float bk = bv[t] * kv[t];
-        dG[t] = fmaf(bk * eg, de, dG[t]);
-        dG[t] = fmaf(to_tf32(bk * ea), dea, dG[t]);
+      for (int t = 0; t < 4; ++t) {
+        const float2 neg_eg = mul2(ea[t], twice(-e_ame));
+        P2[t] = fma2(x[t], neg_eg, mul2(y[t], ea[t]));
+        const float2 bk = mul2(bv[t], kv[t]);
+        dG[t] = fma2(mul2(bk, neg_eg), x[t], dG[t]);
+        dG[t] = fma2(tf32_2(mul2(bk, ea[t])), y[t], dG[t]);
       }
-      tmem_ld8f(tmem_addr(tb, 32 * q4, kColD3 + 64 + i0), x);  // dQg (state part)
-      tmem_ld8f(tmem_addr(tb, 32 * q4, kColD5 + 32 * blk + 16 + 8 * sb), y);  // dQa
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, kColD3 + 64 + i0), x);  // dQg (state part)
+      tmem_ld4x2(tmem_addr(tb, 32 * q4, kColD5 + 32 * blk + 16 + 8 * sb), y);  // dQa
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const int64_t idx = seq_idx(i0 + t) + kc;
-        const float ea = Gb[t], eg = ea * e_ame;
-        const float P1 = failed ? poison_nan() : fmaf(x[t], eg, y[t] * ea);
-        const float dGt = fmaf(to_tf32(sq[t] * ea), y[t], fmaf(sq[t] * eg, x[t], dG[t]));
-        const float dk_t = failed ? poison_nan() : fmaf(bv[t], P2[t], P3[t]);
+      for (int t = 0; t < 4; ++t) {
+        const float2 eg = mul2(ea[t], twice(e_ame));
+        float2 dq = mul2(twice(p.scale), fma2(x[t], eg, mul2(y[t], ea[t])));
+        dG[t] = fma2(tf32_2(mul2(sq[t], ea[t])), y[t], fma2(mul2(sq[t], eg), x[t], dG[t]));
+        float2 dk = fma2(bv[t], P2[t], P3[t]), db = mul2(kv[t], P2[t]);
+        if (failed) dq = dk = db = twice(poison_nan());
+        const int tok = i0 + 2 * t, off = tok * kDim + kc;
         if (kF32Grads) {
-          if (there(i0 + t)) {
-            stf<O>(p.dq, idx, p.scale * P1);
-            stf<O>(p.dk, idx, dk_t);
-          }
+          const int64_t idx = seq_idx(tok) + kc, idx1 = seq_idx(tok + 1) + kc;
+          if (there(tok)) { stf<O>(p.dq, idx, dq.x); stf<O>(p.dk, idx, dk.x); stf<O>(p.dbeta, idx, db.x); }
+          if (there(tok + 1)) { stf<O>(p.dq, idx1, dq.y); stf<O>(p.dk, idx1, dk.y); stf<O>(p.dbeta, idx1, db.y); }
         } else {
           // in place over q and k (this thread's own slots, already read): the tiles leave by TMA stores
-          const int off = (i0 + t) * kDim + kc;
-          stf<T>(smem + kOffTileQ, off, p.scale * P1);
-          stf<T>(smem + kOffTileK, off, dk_t);
-          stf<T>(smem + beta_tile_offset(blk), (8 * sb + t) * kDim + kc, failed ? poison_nan() : kv[t] * P2[t]);
+          const int off_b = (8 * sb + 2 * t) * kDim + kc;
+          stf<T>(smem + kOffTileQ, off, dq.x);
+          stf<T>(smem + kOffTileQ, off + kDim, dq.y);
+          stf<T>(smem + kOffTileK, off, dk.x);
+          stf<T>(smem + kOffTileK, off + kDim, dk.y);
+          stf<T>(smem + beta_tile_offset(blk), off_b, db.x);
+          stf<T>(smem + beta_tile_offset(blk), off_b + kDim, db.y);
         }
-        if (kF32Grads && there(i0 + t)) stf<O>(p.dbeta, idx, failed ? poison_nan() : kv[t] * P2[t]);
-        stf<float>(smem + kOffTileG, (i0 + t) * kDim + kc, dGt);
-        tot += dGt;
+        stf<float>(smem + kOffTileG, off, dG[t].x);
+        stf<float>(smem + kOffTileG, off + kDim, dG[t].y);
+        tot = add2(tot, dG[t]);
       }
     }
-    ms.xe[blk][kc] = e_part;
+    ms.xe[blk][kc] = -(e_part.x + e_part.y);
+    float total = tot.x + tot.y;
     __syncthreads();
     if (blk == 3) {
-      const float end_term = ms.xe[0][kc] + ms.xe[1][kc] + ms.xe[2][kc] + ms.xe[3][kc] + __expf(gend) * dd_k;
+      const float end_term = ms.xe[0][kc] + ms.xe[1][kc] + ms.xe[2][kc] + ms.xe[3][kc] + exp2_approx(gend) * dd_k;
       *reinterpret_cast<float*>(smem + kOffTileG + (63 * kDim + kc) * 4) += end_term;
-      tot += end_term;
+      total += end_term;
     }
-    ms.xt[blk][kc] = tot;
+    ms.xt[blk][kc] = total;
     __syncthreads();
     float run = 0.f;
 #pragma unroll

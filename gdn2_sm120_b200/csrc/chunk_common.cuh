@@ -49,6 +49,7 @@ constexpr int64_t kTileAt = 16384, kTileTt = 16384, kBlobD = 512;
 constexpr int64_t kBlobRn = 32768, kBlobDZ = 8 * 4608;
 constexpr int64_t kStatusBytes = 256;  // word 0: status
 constexpr int kQueueWord = 16;         // joint launch: next unit to prepare
+constexpr float kLog2e = 1.4426950408889634f;  // log-decays are summed in units of ln 2
 // forward scratch per unit, a size callers know: 144 KiB for an inference call (its tiles take 128 of
 // them), 32 KiB for a training call
 constexpr int64_t kFwdScratchInference = 147456, kFwdScratchTraining = 32768;

@@ -53,7 +53,6 @@ constexpr int kPrepThreads = 256;
 constexpr int kRound = 32, kRounds = kDim / kRound;  // channels per round
 constexpr int kLd = 68;           // leading dimension of the fp32 64x64 scratch matrices (16-byte rows, banks shift by 4)
 constexpr int kLdW = 20;          // leading dimension of the transposed 16x16 block products
-constexpr float kLog2e = 1.4426950408889634f;
 
 // One region, by phase (bytes):
 //   inputs       g at 0 (16 or 32 KiB), dense rows; k, q, beta (16 KiB each) by rounds, [round][64][32]
