@@ -22,28 +22,9 @@ namespace {
 constexpr int kRowsPerBlock = 8;  // 8 warps, one row each
 constexpr float kNormEps = 1e-6f;
 
-template <typename T> struct Vec4 { using type = uint2; };
-template <> struct Vec4<float> { using type = float4; };
-
 template <typename T>
-__device__ __forceinline__ void load4f(const void* base, int64_t idx, float (&x)[4]);
-template <>
-__device__ __forceinline__ void load4f<__nv_bfloat16>(const void* base, int64_t idx, float (&x)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(base) + idx);
-  x[0] = __uint_as_float(raw.x << 16); x[1] = __uint_as_float(raw.x & 0xffff0000u);
-  x[2] = __uint_as_float(raw.y << 16); x[3] = __uint_as_float(raw.y & 0xffff0000u);
-}
-template <>
-__device__ __forceinline__ void load4f<__half>(const void* base, int64_t idx, float (&x)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __half*>(base) + idx);
-  const __half2* h = reinterpret_cast<const __half2*>(&raw);
-  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
-  x[0] = a.x; x[1] = a.y; x[2] = b.x; x[3] = b.y;
-}
-template <>
-__device__ __forceinline__ void load4f<float>(const void* base, int64_t idx, float (&x)[4]) {
-  const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx);
-  x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
+__device__ __forceinline__ void load4f(const void* base, int64_t idx, float (&x)[4]) {
+  unpack4<T>(load4_raw<T>(base, idx), x);
 }
 
 template <typename T>
@@ -88,31 +69,42 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) gate_prologue_kernel(const
   const int64_t row = int64_t(blockIdx.x) * kRowsPerBlock + (threadIdx.x >> 5);
   if (row >= p.rows) return;
   const int64_t idx = row * kDim + 4 * lane;
-  float x[4], y[4];
+  // every load before the first store: the outputs may alias the inputs as far as the compiler knows
+  typename Raw4<T>::type q, k, beta, w;
+  typename Raw4<G>::type g;
   if (p.q_raw != nullptr) {
-    load4f<T>(p.q_raw, idx, x);
-    const float inv = rsqrtf(warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) + kNormEps);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) y[c] = x[c] * inv;
-    store4f<T>(p.q, idx, y);
-    if (lane == 0) p.inv_q[row] = inv;
-    load4f<T>(p.k_raw, idx, x);
-    const float invk = rsqrtf(warp_sum(x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3]) + kNormEps);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) y[c] = x[c] * invk;
-    store4f<T>(p.k, idx, y);
-    if (lane == 0) p.inv_k[row] = invk;
+    q = load4_raw<T>(p.q_raw, idx);
+    k = load4_raw<T>(p.k_raw, idx);
   }
   if (p.g_raw != nullptr) {
-    load4f<G>(p.g_raw, idx, x);
+    g = load4_raw<G>(p.g_raw, idx);
+    beta = load4_raw<T>(p.beta_raw, idx);
+    w = load4_raw<T>(p.w_raw, idx);
+  }
+  float x[4], y[4];
+  if (p.q_raw != nullptr) {
+    unpack4<T>(q, x);
+    unpack4<T>(k, y);
+    float sq = x[0] * x[0] + x[1] * x[1] + x[2] * x[2] + x[3] * x[3];
+    float sk = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+    sq = rsqrtf(warp_sum(sq) + kNormEps);
+    sk = rsqrtf(warp_sum(sk) + kNormEps);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) { x[c] *= sq; y[c] *= sk; }
+    store4f<T>(p.q, idx, x);
+    store4f<T>(p.k, idx, y);
+    if (lane == 0) { p.inv_q[row] = sq; p.inv_k[row] = sk; }
+  }
+  if (p.g_raw != nullptr) {
+    unpack4<G>(g, x);
 #pragma unroll
     for (int c = 0; c < 4; ++c) y[c] = -softplusf(x[c]);
     store4f<G>(p.g, idx, y);
-    load4f<T>(p.beta_raw, idx, x);
+    unpack4<T>(beta, x);
 #pragma unroll
     for (int c = 0; c < 4; ++c) y[c] = sigmoidf(x[c]);
     store4f<T>(p.beta, idx, y);
-    load4f<T>(p.w_raw, idx, x);
+    unpack4<T>(w, x);
 #pragma unroll
     for (int c = 0; c < 4; ++c) y[c] = sigmoidf(x[c]);
     store4f<T>(p.w, idx, y);
