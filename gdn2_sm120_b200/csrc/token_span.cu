@@ -16,6 +16,8 @@
 //             and back through the definitions of L, A, E, Q, K, D to q, k, beta and g.
 // Reference counterparts: recurrent.py:108-303, backward_parallel.py:625-718, 1052-1421, backward.py:378-797.
 
+#include <type_traits>
+
 #include "common.cuh"
 #include "seqs.cuh"
 
@@ -39,20 +41,21 @@ struct SpanRows {
   float mt[kSpan][kSpan];  // A[j][i]
 };
 
-template <typename T> struct Quad { using type = uint2; };
-template <> struct Quad<float> { using type = float4; };
+// The token path takes tensors of any element alignment.  Whether four elements can be read at once is asked
+// once for all tensors and not per load: a branch at each load keeps the next one from being issued behind it
+// (8.3k of the 27k clocks of a span).
+template <typename T, bool kVec>
+__device__ __forceinline__ typename Raw4<T>::type load_quad(const void* base, int64_t idx) {
+  if (kVec) return load4_raw<T>(base, idx);
+  typename Raw4<T>::type raw;
+  T* h = reinterpret_cast<T*>(&raw);
+#pragma unroll
+  for (int c = 0; c < 4; ++c) h[c] = static_cast<const T*>(base)[idx + c];
+  return raw;
+}
 template <typename T>
-__device__ __forceinline__ void load_quad(const void* base, int64_t idx, float (&x)[4]) {
-  const T* p = static_cast<const T*>(base) + idx;
-  if ((reinterpret_cast<uintptr_t>(p) & (4 * sizeof(T) - 1)) == 0) {
-    const typename Quad<T>::type raw = *reinterpret_cast<const typename Quad<T>::type*>(p);
-    const T* h = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-    for (int c = 0; c < 4; ++c) x[c] = to_float(h[c]);
-  } else {  // the token path takes tensors of any element alignment
-#pragma unroll
-    for (int c = 0; c < 4; ++c) x[c] = to_float(p[c]);
-  }
+__device__ __forceinline__ bool quads_aligned(const void* base) {
+  return (reinterpret_cast<uintptr_t>(base) & (4 * sizeof(T) - 1)) == 0;
 }
 __device__ __forceinline__ void put4(float* p, const float (&x)[4]) {
   *reinterpret_cast<float4*>(p) = make_float4(x[0], x[1], x[2], x[3]);
@@ -67,19 +70,30 @@ __device__ __forceinline__ void load_rows(SpanRows& sm, const void* q, const voi
                                           int64_t row0, int H, int h, int n, float scale, int prologue, int warp,
                                           int lane) {
   constexpr int kEach = kSpan / kWarps;
+  typename Raw4<G>::type raw_g[kEach];
+  typename Raw4<T>::type raw_b[kEach], raw_k[kEach], raw_q[kEach];
+  auto fetch = [&](auto vec) {
+    constexpr bool kVec = decltype(vec)::value;
+#pragma unroll
+    for (int x = 0; x < kEach; ++x) {
+      // (a token that does not exist: the last one is read in its place, so that no branch separates the loads)
+      const int64_t idx = ((row0 + min(warp + x * kWarps, n - 1)) * H + h) * kDim + 4 * lane;
+      raw_g[x] = load_quad<G, kVec>(g, idx);
+      raw_b[x] = load_quad<T, kVec>(beta, idx);
+      raw_k[x] = load_quad<T, kVec>(k, idx);
+      raw_q[x] = load_quad<T, kVec>(q, idx);
+    }
+  };
+  if (quads_aligned<G>(g) && quads_aligned<T>(beta) && quads_aligned<T>(k) && quads_aligned<T>(q)) fetch(std::true_type{});
+  else fetch(std::false_type{});
   float gv[kEach][4], bv[kEach][4], kk[kEach][4], s[kEach][4];
 #pragma unroll
   for (int x = 0; x < kEach; ++x) {
-    // (a token that does not exist: the last one is read in its place, so that no branch separates the loads)
-    const int64_t idx = ((row0 + min(warp + x * kWarps, n - 1)) * H + h) * kDim + 4 * lane;
-    load_quad<G>(g, idx, gv[x]);
-    load_quad<T>(beta, idx, bv[x]);
-    load_quad<T>(k, idx, kk[x]);
-    load_quad<T>(q, idx, s[x]);
-  }
-#pragma unroll
-  for (int x = 0; x < kEach; ++x) {
     const int t = warp + x * kWarps;
+    unpack4<G>(raw_g[x], gv[x]);
+    unpack4<T>(raw_b[x], bv[x]);
+    unpack4<T>(raw_k[x], kk[x]);
+    unpack4<T>(raw_q[x], s[x]);
     if (kPro && (prologue & kPrologueNorm) != 0) {
       float sk = kk[x][0] * kk[x][0] + kk[x][1] * kk[x][1] + kk[x][2] * kk[x][2] + kk[x][3] * kk[x][3];
       float sq = s[x][0] * s[x][0] + s[x][1] * s[x][1] + s[x][2] * s[x][2] + s[x][3] * s[x][3];
@@ -300,14 +314,21 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
   for (int j0 = 0; j0 < sq.len; j0 += kSpan) {
     const int n = min(kSpan, sq.len - j0);
     const int64_t row0 = sq.row0 + j0;
-    load_rows<T, G, kPro, kWarps>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, p.prologue, t.warp, t.lane);
+    constexpr int kZ = kSpan * kCols / kThreads;
+    float wv[kZ], vv[kZ];  // (issued before anything waits)
 #pragma unroll
-    for (int x = 0; x < kSpan * kCols / kThreads; ++x) {
+    for (int x = 0; x < kZ; ++x) {
       const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
       const int64_t idx = ((row0 + min(i, n - 1)) * p.H + h) * kDim + tile * kCols + c;
-      float wv = ldf<T>(p.w, idx);
-      if (kPro && (p.prologue & kPrologueGate) != 0) wv = prologue_sigmoid(wv);
-      sm.z[i][c] = i < n ? wv * ldf<T>(p.v, idx) : 0.f;
+      wv[x] = ldf<T>(p.w, idx);
+      vv[x] = ldf<T>(p.v, idx);
+    }
+    load_rows<T, G, kPro, kWarps>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, p.prologue, t.warp, t.lane);
+#pragma unroll
+    for (int x = 0; x < kZ; ++x) {
+      const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
+      if (kPro && (p.prologue & kPrologueGate) != 0) wv[x] = prologue_sigmoid(wv[x]);
+      sm.z[i][c] = i < n ? wv[x] * vv[x] : 0.f;
     }
     if (p.bnd != nullptr) store_tile(p.bnd + (int64_t(sq.slot0 + j0 / kSpan) * p.H + h) * kStateElems, t, S);
     __syncthreads();
@@ -425,12 +446,18 @@ token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs se
     const int j0 = span * kSpan, n = min(kSpan, sq.len - j0);
     const int64_t row0 = sq.row0 + j0;
     store_tile(p.d_bnd + (int64_t(sq.slot0 + span + 1) * p.H + h) * kStateElems, t, dS);
+    constexpr int kZ = kSpan * kCols / kThreads;
+    float o[kZ];  // (issued before anything waits)
+#pragma unroll
+    for (int x = 0; x < kZ; ++x) {
+      const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
+      o[x] = ldf<T>(p.d_out, ((row0 + min(i, n - 1)) * p.H + h) * kDim + tile * kCols + c);
+    }
     load_rows<T, G, false, kWarps>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, 0, t.warp, t.lane);
 #pragma unroll
-    for (int x = 0; x < kSpan * kCols / kThreads; ++x) {
+    for (int x = 0; x < kZ; ++x) {
       const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
-      const float o = ldf<T>(p.d_out, ((row0 + min(i, n - 1)) * p.H + h) * kDim + tile * kCols + c);
-      sm.d_out[i][c] = i < n ? o : 0.f;
+      sm.d_out[i][c] = i < n ? o[x] : 0.f;
     }
     __syncthreads();
     gram<kWarps>(sm.rows, t.warp, t.lane);
@@ -545,11 +572,25 @@ token_span_vjp_kernel(const SpanVjpParams p, const __grid_constant__ Seqs seqs) 
       load8(d_src + r * kDim, dS[r]);
     }
   }
+  constexpr int kEach = kSpan / (kVjpThreads / 32);
+  typename Raw4<T>::type raw_o[kEach];
+  auto fetch_o = [&](auto vec) {
+#pragma unroll
+    for (int x = 0; x < kEach; ++x) {
+      const int i = min(warp + x * (kVjpThreads / 32), n - 1);
+      raw_o[x] = load_quad<T, decltype(vec)::value>(p.d_out, ((row0 + i) * p.H + h) * kDim + 4 * lane);
+    }
+  };
+  if (quads_aligned<T>(p.d_out)) fetch_o(std::true_type{});
+  else fetch_o(std::false_type{});
   load_rows<T, G, false, kVjpThreads / 32>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, 0, warp, lane);
-  for (int i = warp; i < kSpan; i += kVjpThreads / 32) {
-    float x[4] = {0.f, 0.f, 0.f, 0.f};
-    if (i < n) load_quad<T>(p.d_out, ((row0 + i) * p.H + h) * kDim + 4 * lane, x);
-    put4(&sm.d_out[i][4 * lane], x);
+#pragma unroll
+  for (int x = 0; x < kEach; ++x) {
+    const int i = warp + x * (kVjpThreads / 32);
+    float o[4];
+    unpack4<T>(raw_o[x], o);
+    if (i >= n) o[0] = o[1] = o[2] = o[3] = 0.f;
+    put4(&sm.d_out[i][4 * lane], o);
   }
   __syncthreads();
   gram<kVjpThreads / 32>(sm.rows, warp, lane);
