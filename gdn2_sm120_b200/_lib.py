@@ -141,7 +141,8 @@ LAUNCHES = [0]
 KERNEL_EVENTS: dict[str, list] | None = None
 
 
-# kernels launched by one successful call of each entry point (default 1)
+# kernels launched by one successful call of each entry point (default 1); a chunk forward of few heads, which
+# runs its two kernels as one launch, still counts as two
 _KERNELS_PER_CALL = {"gdn2_chunk_forward": 2, "gdn2_chunk_forward_fused": 2, "gdn2_chunk_backward": 2, "gdn2_chunk_backward_f32grads": 2,
                      "gdn2_chunk_forward_static": 2}
 

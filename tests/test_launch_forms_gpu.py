@@ -1,0 +1,102 @@
+"""GPU tests of what a dispatch rule chooses between: the joint launch of prep and scan, packed batches that
+take several launches, the token spans' loads of unaligned tensors, and calls from threads that have made no
+CUDA call yet.  The forms run the same arithmetic in the same order, so results are compared bit for bit; one
+unit of each joint case is held against the oracle with the tolerances of test_autograd_gpu.py."""
+
+from __future__ import annotations
+
+import threading
+
+import pytest
+import torch
+
+import gdn2_oracle as oracle
+from gdn2_sm120_b200 import _lib, chunk_gdn2
+from gdn2_sm120_b200.varlen import chunk_gdn2_varlen
+from test_autograd_gpu import _check_unit_alone_and_against_oracle, _device_inputs, _step
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+# (at most SMs / 4 sequences x heads, and enough chunks: the smallest that qualify at 37, 32 and 16 heads, one
+# chunk less, and ragged ends of 1 and 63 tokens)
+@pytest.mark.parametrize("batch,heads,time", [(1, 37, 21 * 64), (2, 16, 26 * 64), (2, 16, 25 * 64), (2, 16, 26 * 64 + 1),
+                                              (1, 16, 70 * 64 + 63)])
+def test_joint_launch_equals_a_unit_alone_and_the_oracle(batch, heads, time):
+    tensors, d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
+    full = _step(tensors, d_out, d_fin)
+    _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
+
+
+@pytest.mark.parametrize("dtype,g_dtype", [(torch.bfloat16, torch.float32), (torch.float16, torch.float16)])
+@pytest.mark.parametrize("raw", [False, True])
+def test_joint_launch_equals_two_launches(dtype, g_dtype, raw):
+    tensors, _, _ = _device_inputs(2, 40 * 64 + 17, 16, seed=7)
+    q, k, v, g, beta, w = [t.to(g_dtype if i == 3 else dtype) for i, t in enumerate(tensors[:6])]
+    flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
+    with torch.no_grad():
+        joint = chunk_gdn2(q, k, v, g, beta, w, tensors[6], output_final_state=True, **flags)
+        _lib.profile_enable(True)  # times the kernels one by one: never joint
+        try:
+            apart = chunk_gdn2(q, k, v, g, beta, w, tensors[6], output_final_state=True, **flags)
+        finally:
+            _lib.profile_enable(False)
+    assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
+
+
+# 255 .. 257 and 513: around one and two launch tables of 256 sequences
+@pytest.mark.parametrize("count", [255, 256, 257, 513])
+def test_packed_batches_around_the_table_size(count):
+    lengths = [(7 * i) % 40 if i % 50 else 64 + i % 70 for i in range(count)]
+    heads, total = 1, sum(lengths)
+    tensors, d_out, _ = _device_inputs(1, total, heads, seed=count)
+    torch.manual_seed(count)
+    states = 0.02 * torch.randn(count, heads, 128, 128, device=DEV)
+    d_fin = 0.01 * torch.randn_like(states)
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    leaves = [t.requires_grad_(True) for t in (*tensors[:6], states)]
+    out, fin = chunk_gdn2_varlen(*leaves[:6], cu, leaves[6], output_final_state=True)
+    grads = torch.autograd.grad((out.float() * d_out.float()).sum() + (fin * d_fin).sum(), leaves)
+    for i in {0, 1, 50, 51, count // 2, count - 2, count - 1}:
+        lo, hi = cu[i], cu[i + 1]
+        if lo == hi:
+            assert torch.equal(fin[i], states[i]) and torch.equal(grads[6][i], d_fin[i])
+            continue
+        single = [t[:, lo:hi].detach().clone() for t in leaves[:6]] + [states[i:i + 1].detach().clone()]
+        o, f, gr = _step(single, d_out[:, lo:hi], d_fin[i:i + 1])
+        assert torch.equal(o, out[:, lo:hi]) and torch.equal(f, fin[i:i + 1])
+        for a, b in zip(gr[:6], grads[:6]):
+            assert torch.equal(a, b[:, lo:hi])
+        assert torch.equal(gr[6], grads[6][i:i + 1])
+
+
+# spans of one token, a whole span, one token more, and several spans
+@pytest.mark.parametrize("time", [2, 16, 17, 48])
+def test_token_spans_of_unaligned_tensors(time):
+    cpu = oracle.make_inputs(2, time, 3, seed=time)
+
+    def shifted(t):  # the same values one element past an aligned address
+        flat = torch.empty(t.numel() + 1, dtype=t.dtype, device=DEV)
+        view = flat[1:].view(t.shape)
+        view.copy_(t)
+        return view
+
+    with torch.no_grad():
+        expected = chunk_gdn2(*[t.to(DEV) for t in cpu], output_final_state=True)
+        got = chunk_gdn2(*[shifted(t) for t in cpu[:6]], cpu[6].to(DEV), output_final_state=True)
+    assert torch.equal(got[0], expected[0]) and torch.equal(got[1], expected[1])
+
+
+def test_training_in_a_thread_without_a_context():
+    tensors, d_out, d_fin = _device_inputs(1, 130, 2, seed=3)
+    expected = _step(tensors, d_out, d_fin)
+    results = []
+    worker = threading.Thread(target=lambda: results.append(_step(tensors, d_out, d_fin)))
+    worker.start()
+    worker.join()
+    assert results and torch.equal(results[0][0], expected[0]) and torch.equal(results[0][1], expected[1])
+    for a, b in zip(results[0][2], expected[2]):
+        assert torch.equal(a, b)
