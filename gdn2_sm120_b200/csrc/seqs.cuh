@@ -27,7 +27,7 @@ struct UniformSeqs {
   int len, n_chunks, n;
   __host__ __device__ int count() const { return n; }
   __host__ __device__ int total_chunks() const { return n * n_chunks; }
-  __device__ __forceinline__ SeqInfo at(int s) const {
+  __host__ __device__ __forceinline__ SeqInfo at(int s) const {
     return SeqInfo{first + s * stride, len, s * n_chunks, n_chunks, s * (n_chunks + 1), s};
   }
   __device__ __forceinline__ int find(int chunk) const { return int(uint32_t(chunk) / uint32_t(n_chunks)); }
@@ -43,7 +43,7 @@ struct PackedSeqsOf {
   Entry e[kMaxPacked];
   __host__ __device__ int count() const { return n; }
   __host__ __device__ int total_chunks() const { return chunks; }
-  __device__ __forceinline__ SeqInfo at(int s) const {
+  __host__ __device__ __forceinline__ SeqInfo at(int s) const {
     const Entry x = e[s];
     return SeqInfo{x.row0, x.len, x.chunk0, (x.len + kSpan - 1) / kSpan, x.chunk0 + s, x.sid};
   }

@@ -210,11 +210,43 @@ __device__ __forceinline__ void matrix_row(const float (*m)[kSpan], int i, float
 }
 
 // ---- forward and reverse state scan: one CTA = (sequence, head, 64 value columns) ---------------------
-// 256 threads; thread = 8 key rows x 4 value columns of the state, in registers from start to end.  Bound by
-// latency where the grid is small (a warp alone on its scheduler issues every fourth clock: hence 8 warps
-// and not 4 on 32 columns, which also halves the Gram products per column), by shared-memory reads and
-// multiply-adds in equal parts where it is large.
+// 256 threads hold the state: thread = 8 key rows x 4 value columns, in registers from start to end (8 warps and
+// not 4 on 32 columns, which also halves the Gram products per column).  Half of a span's work, its rows and
+// Gram products, does not touch the state: with kSplit a second group of 256 threads prepares the next span
+// meanwhile, in the other of two buffers (B4 T48 H16 training: forward 30 -> 24 us, reverse 29 -> 22; B4 T32
+// raw 20 -> 17).  That is the form for grids that leave a CTA its SM alone; larger ones run two CTAs of 256
+// threads per SM, which fill each other's waits as well and need no registers for two groups (B32 T32 H16 raw
+// 105 us, split 121; B16 T48 the same either way).
 constexpr int kThreads = 256, kWarps = kThreads / 32;
+// named barriers: 1, 2 within a group; ready / free of buffer b between the groups
+constexpr int kBarReady = 3, kBarFree = 5;
+__device__ __forceinline__ void bar_sync(int id, int threads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int threads) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(threads) : "memory"); }
+
+// Runs prepare(span, buffer) and advance(span, buffer) for the spans 0 .. n - 1 in order.
+template <bool kSplit, typename Prepare, typename Advance>
+__device__ __forceinline__ void walk_spans(int n, bool preparer, Prepare prepare, Advance advance) {
+  if constexpr (!kSplit) {
+    for (int i = 0; i < n; ++i) {
+      prepare(i, 0);
+      __syncthreads();
+      advance(i, 0);
+      __syncthreads();
+    }
+  } else if (preparer) {
+    for (int i = 0; i < n; ++i) {
+      if (i >= 2) bar_sync(kBarFree + (i & 1), 2 * kThreads);
+      prepare(i, i & 1);
+      bar_arrive(kBarReady + (i & 1), 2 * kThreads);
+    }
+  } else {
+    for (int i = 0; i < n; ++i) {
+      bar_sync(kBarReady + (i & 1), 2 * kThreads);
+      advance(i, i & 1);
+      if (i + 2 < n) bar_arrive(kBarFree + (i & 1), 2 * kThreads);
+    }
+  }
+}
 constexpr int kCols = 64, kTiles = kDim / kCols;
 
 // Warps 0..3 hold columns 0..31 of the tile, warps 4..7 columns 32..63.
@@ -277,9 +309,10 @@ __device__ __forceinline__ void decay_rows(const float* d, const TileThread& t, 
   }
 }
 
+template <bool kSplit>
 struct FwdSmem {
-  SpanRows rows;
-  float z[kSpan][kCols];                 // w v
+  SpanRows rows[kSplit ? 2 : 1];
+  float z[kSplit ? 2 : 1][kSpan][kCols];  // w v
   float u[kSpan][kCols];
   float part[4][kSpan][2][kCols];        // per warp of a column half: E S and Q S
 };
@@ -293,27 +326,30 @@ struct SpanFwdParams {
   int prologue;
 };
 
-template <typename T, typename G, typename Seqs, bool kPro>
-__global__ void __launch_bounds__(kThreads)
+template <typename T, typename G, typename Seqs, bool kPro, bool kSplit>
+__global__ void __launch_bounds__(kSplit ? 2 * kThreads : kThreads)
 token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  FwdSmem& sm = *reinterpret_cast<FwdSmem*>(smem_raw);
-  const int tid = threadIdx.x, tile = int(blockIdx.x) % kTiles;
+  FwdSmem<kSplit>& sm = *reinterpret_cast<FwdSmem<kSplit>*>(smem_raw);
+  const int tid = threadIdx.x % kThreads, tile = int(blockIdx.x) % kTiles;
+  const bool preparer = kSplit && threadIdx.x >= kThreads;
   const TileThread t(tid, tile);
   const int sh = int(blockIdx.x) / kTiles, s_ = sh / p.H, h = sh - s_ * p.H;
   const SeqInfo sq = seqs.at(s_);
   const int64_t state = (int64_t(sq.sid) * p.H + h) * kStateElems;
+  auto sync = [&] { bar_sync(preparer ? 2 : 1, kThreads); };
 
   float S[8][4];
-  if (p.s_in != nullptr) {
+  if (p.s_in != nullptr && !preparer) {
     load_tile(p.s_in + state, t, S);
   } else {
 #pragma unroll
     for (int r = 0; r < 8; ++r) S[r][0] = S[r][1] = S[r][2] = S[r][3] = 0.f;
   }
-  for (int j0 = 0; j0 < sq.len; j0 += kSpan) {
-    const int n = min(kSpan, sq.len - j0);
+  auto prepare = [&](int span, int buf) {
+    const int j0 = span * kSpan, n = min(kSpan, sq.len - j0);
     const int64_t row0 = sq.row0 + j0;
+    SpanRows& rows = sm.rows[buf];
     constexpr int kZ = kSpan * kCols / kThreads;
     float wv[kZ], vv[kZ];  // (issued before anything waits)
 #pragma unroll
@@ -323,19 +359,23 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
       wv[x] = ldf<T>(p.w, idx);
       vv[x] = ldf<T>(p.v, idx);
     }
-    load_rows<T, G, kPro, kWarps>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, p.prologue, t.warp, t.lane);
+    load_rows<T, G, kPro, kWarps>(rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, p.prologue, t.warp, t.lane);
 #pragma unroll
     for (int x = 0; x < kZ; ++x) {
       const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
       if (kPro && (p.prologue & kPrologueGate) != 0) wv[x] = prologue_sigmoid(wv[x]);
-      sm.z[i][c] = i < n ? wv[x] * vv[x] : 0.f;
+      sm.z[buf][i][c] = i < n ? wv[x] * vv[x] : 0.f;
     }
-    if (p.bnd != nullptr) store_tile(p.bnd + (int64_t(sq.slot0 + j0 / kSpan) * p.H + h) * kStateElems, t, S);
-    __syncthreads();
-    gram<kWarps>(sm.rows, t.warp, t.lane);
-    __syncthreads();
-    if (tid < kDim) finish_gram(sm.rows, tid);
-    __syncthreads();
+    sync();
+    gram<kWarps>(rows, t.warp, t.lane);
+    sync();
+    if (tid < kDim) finish_gram(rows, tid);
+  };
+  auto advance = [&](int span, int buf) {
+    const int j0 = span * kSpan, n = min(kSpan, sq.len - j0);
+    const int64_t row0 = sq.row0 + j0;
+    const SpanRows& rows = sm.rows[buf];
+    if (p.bnd != nullptr) store_tile(p.bnd + (int64_t(sq.slot0 + span) * p.H + h) * kStateElems, t, S);
     // E S and Q S: over this thread's rows, then over the four row groups of the warp; four tokens at a time
     // (rows of tokens that do not exist are zero)
 #pragma unroll 1
@@ -345,8 +385,8 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float r[4], o[4], y[4];
-        rows_times_tile(sm.rows.e[i0 + i], t, S, r);
-        rows_times_tile(sm.rows.s[i0 + i], t, S, o);
+        rows_times_tile(rows.e[i0 + i], t, S, r);
+        rows_times_tile(rows.s[i0 + i], t, S, o);
 #pragma unroll
         for (int c = 0; c < 4; ++c) y[c] = (b16 ? o[c] : r[c]) + __shfl_xor_sync(0xffffffffu, b16 ? r[c] : o[c], 16);
 #pragma unroll
@@ -357,27 +397,27 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
         *reinterpret_cast<float2*>(&sm.part[t.rw][i0 + i][b16 ? 1 : 0][t.cc + (b8 ? 2 : 0)]) = make_float2(x[i][0], x[i][1]);
       }
     }
-    __syncthreads();
+    sync();
     if (tid < kCols) {  // a thread per column: (I + L) u = z - E S
       const int col = tid;
       float u[kSpan];
 #pragma unroll
       for (int i = 0; i < kSpan; ++i) {
-        u[i] = i < n ? sm.z[i][col] - ((sm.part[0][i][0][col] + sm.part[1][i][0][col]) +
+        u[i] = i < n ? sm.z[buf][i][col] - ((sm.part[0][i][0][col] + sm.part[1][i][0][col]) +
                                           (sm.part[2][i][0][col] + sm.part[3][i][0][col]))
                      : 0.f;
       }
 #pragma unroll
       for (int i = 0; i < kSpan; ++i) {
         float l[kSpan];
-        matrix_row(sm.rows.l, i, l);
+        matrix_row(rows.l, i, l);
 #pragma unroll
         for (int j = 0; j < i; ++j) u[i] = fmaf(-l[j], u[j], u[i]);
       }
 #pragma unroll
       for (int i = 0; i < kSpan; ++i) sm.u[i][col] = u[i];
     }
-    __syncthreads();
+    sync();
     {
       const int col = tid % kCols;
       float u[kSpan];
@@ -388,7 +428,7 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
         const int i = (tid + x * kThreads) / kCols;
         if (i < n) {
           float m[kSpan];
-          matrix_row(sm.rows.m, i, m);
+          matrix_row(rows.m, i, m);
           float o = (sm.part[0][i][1][col] + sm.part[1][i][1][col]) +
                     (sm.part[2][i][1][col] + sm.part[3][i][1][col]);
 #pragma unroll
@@ -397,22 +437,25 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
         }
       }
     }
-    decay_rows(sm.rows.d, t, S);
+    decay_rows(rows.d, t, S);
 #pragma unroll 1
-    for (int j0 = 0; j0 < n; j0 += 4) {
+    for (int i0 = 0; i0 < n; i0 += 4) {
 #pragma unroll
-      for (int j = j0; j < j0 + 4; ++j) rank_one(sm.rows.k[j], sm.u[j], t, 1.f, S);
+      for (int j = i0; j < i0 + 4; ++j) rank_one(rows.k[j], sm.u[j], t, 1.f, S);
     }
-    __syncthreads();
-  }
+    if (kSplit) sync();  // (u and part are written again)
+  };
+  walk_spans<kSplit>(sq.n_chunks, preparer, prepare, advance);
+  if (preparer) return;
   if (p.bnd != nullptr) store_tile(p.bnd + (int64_t(sq.slot0 + sq.n_chunks) * p.H + h) * kStateElems, t, S);
   if (p.s_out != nullptr) store_tile(p.s_out + state, t, S);
 }
 
 // ---- reverse scan of the state cotangent -------------------------------------------------------------
+template <bool kSplit>
 struct RevSmem {
-  SpanRows rows;
-  float d_out[kSpan][kCols];
+  SpanRows rows[kSplit ? 2 : 1];
+  float d_out[kSplit ? 2 : 1][kSpan][kCols];
   float x[kSpan][kCols];                // d(w v)
   float part[4][kSpan][kCols];          // per warp of a column half: K dS'
 };
@@ -424,28 +467,31 @@ struct SpanRevParams {
   float scale;
 };
 
-template <typename T, typename G, typename Seqs>
-__global__ void __launch_bounds__(kThreads)
+template <typename T, typename G, typename Seqs, bool kSplit>
+__global__ void __launch_bounds__(kSplit ? 2 * kThreads : kThreads)
 token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  RevSmem& sm = *reinterpret_cast<RevSmem*>(smem_raw);
-  const int tid = threadIdx.x, tile = int(blockIdx.x) % kTiles;
+  RevSmem<kSplit>& sm = *reinterpret_cast<RevSmem<kSplit>*>(smem_raw);
+  const int tid = threadIdx.x % kThreads, tile = int(blockIdx.x) % kTiles;
+  const bool preparer = kSplit && threadIdx.x >= kThreads;
   const TileThread t(tid, tile);
   const int sh = int(blockIdx.x) / kTiles, s_ = sh / p.H, h = sh - s_ * p.H;
   const SeqInfo sq = seqs.at(s_);
   const int64_t state = (int64_t(sq.sid) * p.H + h) * kStateElems;
+  auto sync = [&] { bar_sync(preparer ? 2 : 1, kThreads); };
 
   float dS[8][4];
-  if (p.ds_final != nullptr) {
+  if (p.ds_final != nullptr && !preparer) {
     load_tile(p.ds_final + state, t, dS);
   } else {
 #pragma unroll
     for (int r = 0; r < 8; ++r) dS[r][0] = dS[r][1] = dS[r][2] = dS[r][3] = 0.f;
   }
-  for (int span = sq.n_chunks - 1; span >= 0; --span) {
-    const int j0 = span * kSpan, n = min(kSpan, sq.len - j0);
+  // step `it` works on span n_chunks - 1 - it
+  auto prepare = [&](int it, int buf) {
+    const int j0 = (sq.n_chunks - 1 - it) * kSpan, n = min(kSpan, sq.len - j0);
     const int64_t row0 = sq.row0 + j0;
-    store_tile(p.d_bnd + (int64_t(sq.slot0 + span + 1) * p.H + h) * kStateElems, t, dS);
+    SpanRows& rows = sm.rows[buf];
     constexpr int kZ = kSpan * kCols / kThreads;
     float o[kZ];  // (issued before anything waits)
 #pragma unroll
@@ -453,17 +499,21 @@ token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs se
       const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
       o[x] = ldf<T>(p.d_out, ((row0 + min(i, n - 1)) * p.H + h) * kDim + tile * kCols + c);
     }
-    load_rows<T, G, false, kWarps>(sm.rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, 0, t.warp, t.lane);
+    load_rows<T, G, false, kWarps>(rows, p.q, p.k, p.g, p.beta, row0, p.H, h, n, p.scale, 0, t.warp, t.lane);
 #pragma unroll
     for (int x = 0; x < kZ; ++x) {
       const int i = (tid + x * kThreads) / kCols, c = tid % kCols;
-      sm.d_out[i][c] = i < n ? o[x] : 0.f;
+      sm.d_out[buf][i][c] = i < n ? o[x] : 0.f;
     }
-    __syncthreads();
-    gram<kWarps>(sm.rows, t.warp, t.lane);
-    __syncthreads();
-    if (tid < kDim) finish_gram(sm.rows, tid);
-    __syncthreads();
+    sync();
+    gram<kWarps>(rows, t.warp, t.lane);
+    sync();
+    if (tid < kDim) finish_gram(rows, tid);
+  };
+  auto advance = [&](int it, int buf) {
+    const int span = sq.n_chunks - 1 - it, n = min(kSpan, sq.len - span * kSpan);
+    const SpanRows& rows = sm.rows[buf];
+    store_tile(p.d_bnd + (int64_t(sq.slot0 + span + 1) * p.H + h) * kStateElems, t, dS);
 #pragma unroll 1
     for (int i0 = 0; i0 < n; i0 += 4) {
       const bool b16 = (t.lane & 16) != 0, b8 = (t.lane & 8) != 0;
@@ -471,7 +521,7 @@ token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs se
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         float r[4], y[2];
-        rows_times_tile(sm.rows.k[i0 + i], t, dS, r);
+        rows_times_tile(rows.k[i0 + i], t, dS, r);
 #pragma unroll
         for (int c = 0; c < 2; ++c) y[c] = (b16 ? r[c + 2] : r[c]) + __shfl_xor_sync(0xffffffffu, b16 ? r[c] : r[c + 2], 16);
         x[i] = (b8 ? y[1] : y[0]) + __shfl_xor_sync(0xffffffffu, b8 ? y[0] : y[1], 8);
@@ -479,21 +529,21 @@ token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs se
 #pragma unroll
       for (int i = 0; i < 4; ++i) sm.part[t.rw][i0 + i][t.cc + (b16 ? 2 : 0) + (b8 ? 1 : 0)] = x[i];
     }
-    __syncthreads();
+    sync();
     if (tid < kCols) {  // a thread per column: (I + L)^T x = K dS' + A^T do
       const int col = tid;
       float x[kSpan], o[kSpan];
 #pragma unroll
       for (int i = 0; i < kSpan; ++i) {
-        o[i] = sm.d_out[i][col];
+        o[i] = sm.d_out[buf][i][col];
         x[i] = i < n ? (sm.part[0][i][col] + sm.part[1][i][col]) + (sm.part[2][i][col] + sm.part[3][i][col])
                      : 0.f;
       }
 #pragma unroll
       for (int i = kSpan - 1; i >= 0; --i) {
         float l[kSpan], m[kSpan];
-        matrix_row(sm.rows.mt, i, m);
-        matrix_row(sm.rows.lt, i, l);
+        matrix_row(rows.mt, i, m);
+        matrix_row(rows.lt, i, l);
 #pragma unroll
         for (int j = i; j < kSpan; ++j) x[i] = fmaf(m[j], o[j], x[i]);
 #pragma unroll
@@ -502,18 +552,20 @@ token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs se
 #pragma unroll
       for (int i = 0; i < kSpan; ++i) sm.x[i][col] = x[i];
     }
-    __syncthreads();
-    decay_rows(sm.rows.d, t, dS);
+    sync();
+    decay_rows(rows.d, t, dS);
 #pragma unroll 1
     for (int i0 = 0; i0 < n; i0 += 2) {
 #pragma unroll
       for (int i = i0; i < i0 + 2; ++i) {
-        rank_one(sm.rows.s[i], sm.d_out[i], t, 1.f, dS);
-        rank_one(sm.rows.e[i], sm.x[i], t, -1.f, dS);
+        rank_one(rows.s[i], sm.d_out[buf][i], t, 1.f, dS);
+        rank_one(rows.e[i], sm.x[i], t, -1.f, dS);
       }
     }
-    __syncthreads();
-  }
+    if (kSplit) sync();  // (x and part are written again)
+  };
+  walk_spans<kSplit>(sq.n_chunks, preparer, prepare, advance);
+  if (preparer) return;
   store_tile(p.d_bnd + int64_t(sq.slot0 * int64_t(p.H) + h) * kStateElems, t, dS);
   if (p.ds_init != nullptr) store_tile(p.ds_init + state, t, dS);
 }
@@ -884,25 +936,47 @@ int launch(Kernel kernel, int64_t blocks, int threads, int smem, const Params& p
   return check_launch();
 }
 
+// kSplit needs a second span to prepare (a packed batch lists its longest sequence first) and an SM per CTA.
 template <typename Seqs>
+int prefer_split(const Seqs& seqs, int64_t H, bool* split) {
+  int sm_count = 0;
+  if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
+  *split = seqs.count() > 0 && seqs.at(0).len > kSpan && int64_t(seqs.count()) * H * kTiles <= sm_count;
+  return GDN2_OK;
+}
+template <bool kPro, bool kSplit, typename Seqs>
 int run_forward(const Seqs& seqs, const SpanFwdParams& p, int dtype, int g_dtype, cudaStream_t stream) {
   const int64_t blocks = int64_t(seqs.count()) * p.H * kTiles;
   int st = GDN2_OK;
   GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    st = p.prologue != 0
-             ? launch(token_span_forward_kernel<T, G, Seqs, true>, blocks, kThreads, int(sizeof(FwdSmem)), p, seqs, stream)
-             : launch(token_span_forward_kernel<T, G, Seqs, false>, blocks, kThreads, int(sizeof(FwdSmem)), p, seqs, stream);
+    st = launch(token_span_forward_kernel<T, G, Seqs, kPro, kSplit>, blocks, kSplit ? 2 * kThreads : kThreads,
+                int(sizeof(FwdSmem<kSplit>)), p, seqs, stream);
+  });
+  return st;
+}
+template <typename Seqs>
+int run_forward(const Seqs& seqs, const SpanFwdParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+  bool split = false;
+  if (int st = prefer_split(seqs, p.H, &split); st != GDN2_OK) return st;
+  auto run = p.prologue != 0 ? (split ? run_forward<true, true, Seqs> : run_forward<true, false, Seqs>)
+                             : (split ? run_forward<false, true, Seqs> : run_forward<false, false, Seqs>);
+  return run(seqs, p, dtype, g_dtype, stream);
+}
+template <bool kSplit, typename Seqs>
+int run_reverse(const Seqs& seqs, const SpanRevParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+  const int64_t blocks = int64_t(seqs.count()) * p.H * kTiles;
+  int st = GDN2_OK;
+  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+    st = launch(token_span_reverse_kernel<T, G, Seqs, kSplit>, blocks, kSplit ? 2 * kThreads : kThreads,
+                int(sizeof(RevSmem<kSplit>)), p, seqs, stream);
   });
   return st;
 }
 template <typename Seqs>
 int run_reverse(const Seqs& seqs, const SpanRevParams& p, int dtype, int g_dtype, cudaStream_t stream) {
-  const int64_t blocks = int64_t(seqs.count()) * p.H * kTiles;
-  int st = GDN2_OK;
-  GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    st = launch(token_span_reverse_kernel<T, G, Seqs>, blocks, kThreads, int(sizeof(RevSmem)), p, seqs, stream);
-  });
-  return st;
+  bool split = false;
+  if (int st = prefer_split(seqs, p.H, &split); st != GDN2_OK) return st;
+  return (split ? run_reverse<true, Seqs> : run_reverse<false, Seqs>)(seqs, p, dtype, g_dtype, stream);
 }
 template <typename Seqs>
 int run_vjp(const Seqs& seqs, const SpanVjpParams& p, int dtype, int g_dtype, cudaStream_t stream) {

@@ -100,3 +100,12 @@ def test_training_in_a_thread_without_a_context():
     assert results and torch.equal(results[0][0], expected[0]) and torch.equal(results[0][1], expected[1])
     for a, b in zip(results[0][2], expected[2]):
         assert torch.equal(a, b)
+
+
+# 1 to 4 spans, whole and partial; 74 pairs x 2 tiles fill the SMs once, 75 do not
+@pytest.mark.parametrize("time", [16, 17, 33, 63])
+@pytest.mark.parametrize("batch,heads", [(2, 37), (3, 25)])
+def test_token_spans_at_the_grid_where_the_form_changes(batch, heads, time):
+    tensors, d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
+    full = _step(tensors, d_out, d_fin)
+    _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
