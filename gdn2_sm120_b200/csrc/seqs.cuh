@@ -11,6 +11,7 @@
 namespace gdn2 {
 
 constexpr int kChunk = GDN2_CHUNK;  // 64
+constexpr int kStepTokens = 8;      // forward calls of sequences up to this long go token by token
 
 struct SeqInfo {
   int64_t row0;   // first token row

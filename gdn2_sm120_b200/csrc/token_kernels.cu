@@ -1,6 +1,7 @@
-// Token-path kernels for one token: exact fp32 recurrence.
+// Token-path kernels for one token or a few: exact fp32 recurrence.
 //
-//   token_step_kernel         one decode step of few heads (or of states that are not 16-byte aligned)
+//   token_step_kernel         one decode step of few heads (or of states that are not 16-byte aligned), and
+//                             sequences of up to 8 tokens
 //   token_decode_ring_kernel  one decode step of many heads, persistent
 //   token_t1_zero_kernel      T == 1, zero initial state closed form (write-only state)
 //
@@ -14,7 +15,10 @@
 // fp32 state registers per thread, and every state element is read and written by exactly one thread
 // (which is why an exact in-place state update is race-free).
 
+#include <type_traits>
+
 #include "common.cuh"
+#include "seqs.cuh"
 #include "tc05.cuh"
 
 namespace gdn2 {
@@ -42,6 +46,9 @@ struct TokenStepParams {
   const float* s_in;
   void* out;
   float* s_out;
+  float* bnd;    // states before and after the tokens, or null
+  int H;
+  int first;     // sequences of the list before this one are not this launch's
   float scale;
   int prologue;  // kPrologueNorm | kPrologueGate: raw projections / gate pre-activations are activated here
 };
@@ -59,18 +66,27 @@ __device__ __forceinline__ float4 ld_red4(const float (*red)[kTokVT], int col) {
 
 // kPro (here and in the two decode kernels below): the instantiation that can apply the layer prologue
 // to raw inputs; the plain instantiation carries none of that code.
-template <typename T, typename G, bool kPro = false>
-__global__ void __launch_bounds__(kTokThreads) token_step_kernel(const TokenStepParams p) {
-  __shared__ float s_a[kDim], s_e[kDim], s_k[kDim], s_q[kDim];
-  __shared__ float s_z[kTokVT];
+//
+// Up to kTok tokens one after the other, their inputs read at the start; a token costs two barriers and two
+// reductions over the CTA.  kTok = 1 is a decode step (T == 1).
+template <typename T, typename G, typename Seqs, bool kPro, int kTok>
+__global__ void __launch_bounds__(kTokThreads)
+token_step_kernel(const TokenStepParams p, const __grid_constant__ Seqs seqs) {
+  __shared__ float s_a[kTok][kDim], s_e[kTok][kDim], s_k[kTok][kDim], s_q[kTok][kDim];
+  __shared__ float s_z[kTok][kTokVT];
   __shared__ __align__(16) float s_red[2][4][kTokVT];  // [erase|output][warp][column]
-  __shared__ float s_nrm[4][2];                        // fused prologue: per warp sums of q^2, k^2
+  __shared__ float s_nrm[kTok][4][2];                  // fused prologue: per warp sums of q^2, k^2
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cg = tid & 7, rg = tid >> 3;
   const int vt = int(blockIdx.x % kTokTiles);
-  const int64_t bh = blockIdx.x / kTokTiles;  // T == 1: the sequence row is the head's number
-  const int64_t idx = bh * kDim;
+  const int sh = int(blockIdx.x) / kTokTiles;
+  const int s_ = kTok == 1 ? 0 : sh / p.H, h = sh - s_ * p.H;
+  const SeqInfo sq = seqs.at(kTok == 1 ? 0 : p.first + s_);
+  const int n = kTok == 1 ? 1 : sq.len;  // (0: an empty sequence of a packed batch, its state passes through)
+  const int64_t bh = kTok == 1 ? sh : int64_t(sq.sid) * p.H + h;
+  // (T == 1: the sequence row is the head's number)
+  auto row_of = [&](int t) { return kTok == 1 ? bh * kDim : ((sq.row0 + t) * p.H + h) * kDim; };
   const int col0 = vt * kTokVT + cg * 4;
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
@@ -85,85 +101,121 @@ __global__ void __launch_bounds__(kTokThreads) token_step_kernel(const TokenStep
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) S[i][0] = S[i][1] = S[i][2] = S[i][3] = 0.f;
   }
-  {
-    const float kv = ldf<T>(p.k, idx + tid), qv = ldf<T>(p.q, idx + tid);
-    float gv = ldf<G>(p.g, idx + tid), bv = ldf<T>(p.beta, idx + tid);
-    if (pro_gate) { gv = prologue_log_decay(gv); bv = prologue_sigmoid(bv); }
-    s_a[tid] = expf(gv);
-    s_e[tid] = bv * kv;
-    s_k[tid] = kv;
-    s_q[tid] = p.scale * qv;
-    if (tid < kTokVT) {
-      float wv = ldf<T>(p.w, idx + vt * kTokVT + tid);
-      if (pro_gate) wv = prologue_sigmoid(wv);
-      s_z[tid] = wv * ldf<T>(p.v, idx + vt * kTokVT + tid);
-    }
-    if (pro_norm) {
-      float sq = qv * qv, sk = kv * kv;
-#pragma unroll
-      for (int off = 16; off > 0; off >>= 1) {
-        sq += __shfl_xor_sync(0xffffffffu, sq, off);
-        sk += __shfl_xor_sync(0xffffffffu, sk, off);
-      }
-      if (lane == 0) { s_nrm[warp][0] = sq; s_nrm[warp][1] = sk; }
-    }
-  }
-  __syncthreads();
-
-  // reciprocal norms of the raw q and k (1 when the inputs are already normalised)
-  float iq = 1.f, ik = 1.f;
-  if (pro_norm) {
-    iq = rsqrtf(s_nrm[0][0] + s_nrm[1][0] + s_nrm[2][0] + s_nrm[3][0] + kPrologueEps);
-    ik = rsqrtf(s_nrm[0][1] + s_nrm[1][1] + s_nrm[2][1] + s_nrm[3][1] + kPrologueEps);
-  }
-  // X = a * S ; partial r = X^T e over this thread's rows
-  float r[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < kRowsPerThread; ++i) {
-    const float a = s_a[rg + 16 * i], e = kPro ? s_e[rg + 16 * i] * ik : s_e[rg + 16 * i];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      S[i][c] *= a;
-      r[c] = fmaf(S[i][c], e, r[c]);
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    r[c] += __shfl_xor_sync(0xffffffffu, r[c], 8);
-    r[c] += __shfl_xor_sync(0xffffffffu, r[c], 16);
-  }
-  if (lane < 8) *reinterpret_cast<float4*>(&s_red[0][warp][cg * 4]) = make_float4(r[0], r[1], r[2], r[3]);
-  __syncthreads();
-
-  const float4 rs = ld_red4(s_red[0], cg * 4);
-  const float u[4] = {s_z[cg * 4 + 0] - rs.x, s_z[cg * 4 + 1] - rs.y, s_z[cg * 4 + 2] - rs.z, s_z[cg * 4 + 3] - rs.w};
-  // S = X + k u^T ; partial o = S^T (scale q)
-  float o[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-  for (int i = 0; i < kRowsPerThread; ++i) {
-    const float kv = kPro ? s_k[rg + 16 * i] * ik : s_k[rg + 16 * i];
-    const float qv = kPro ? s_q[rg + 16 * i] * iq : s_q[rg + 16 * i];
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      S[i][c] = fmaf(kv, u[c], S[i][c]);
-      o[c] = fmaf(S[i][c], qv, o[c]);
-    }
-  }
-  if (p.s_out != nullptr) {
-    float* dst = p.s_out + bh * kStateElems;
-    const bool vec = (reinterpret_cast<uintptr_t>(p.s_out) & 15) == 0;
+  auto store_state = [&](float* dst) {
+    const bool vec = (reinterpret_cast<uintptr_t>(dst) & 15) == 0;
 #pragma unroll
     for (int i = 0; i < kRowsPerThread; ++i) store4(dst + (rg + 16 * i) * kDim + col0, vec, S[i]);
-  }
+  };
+  constexpr int kBatch = kTok < 4 ? kTok : 4;  // tokens read together (eight take the registers of other CTAs)
+  auto stage = [&](int t0) {
+    T rk[kBatch], rq[kBatch], rb[kBatch], rw[kBatch], rv[kBatch];
+    G rg_[kBatch];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    o[c] += __shfl_xor_sync(0xffffffffu, o[c], 8);
-    o[c] += __shfl_xor_sync(0xffffffffu, o[c], 16);
+    for (int t = 0; t < kBatch; ++t) {  // (a token that does not exist: the last one is read in its place)
+      const int64_t idx = row_of(min(t0 + t, n - 1));
+      rk[t] = static_cast<const T*>(p.k)[idx + tid];
+      rq[t] = static_cast<const T*>(p.q)[idx + tid];
+      rg_[t] = static_cast<const G*>(p.g)[idx + tid];
+      rb[t] = static_cast<const T*>(p.beta)[idx + tid];
+      if (tid < kTokVT) {
+        rw[t] = static_cast<const T*>(p.w)[idx + vt * kTokVT + tid];
+        rv[t] = static_cast<const T*>(p.v)[idx + vt * kTokVT + tid];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < kBatch; ++x) {
+      const int t = t0 + x;
+      if (t >= n) break;
+      const float kv = to_float(rk[x]), qv = to_float(rq[x]);
+      float gv = to_float(rg_[x]), bv = to_float(rb[x]);
+      if (pro_gate) { gv = prologue_log_decay(gv); bv = prologue_sigmoid(bv); }
+      s_a[t][tid] = expf(gv);
+      s_e[t][tid] = bv * kv;
+      s_k[t][tid] = kv;
+      s_q[t][tid] = p.scale * qv;
+      if (tid < kTokVT) {
+        float wv = to_float(rw[x]);
+        if (pro_gate) wv = prologue_sigmoid(wv);
+        s_z[t][tid] = wv * to_float(rv[x]);
+      }
+      if (pro_norm) {
+        float sq_ = qv * qv, sk = kv * kv;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+          sq_ += __shfl_xor_sync(0xffffffffu, sq_, off);
+          sk += __shfl_xor_sync(0xffffffffu, sk, off);
+        }
+        if (lane == 0) { s_nrm[t][warp][0] = sq_; s_nrm[t][warp][1] = sk; }
+      }
+    }
+  };
+  if constexpr (kTok == kBatch) {
+    if (n > 0) stage(0);
+  } else {
+#pragma unroll 1
+    for (int t0 = 0; t0 < n; t0 += kBatch) stage(t0);
   }
-  if (lane < 8) *reinterpret_cast<float4*>(&s_red[1][warp][cg * 4]) = make_float4(o[0], o[1], o[2], o[3]);
+  if (p.bnd != nullptr) store_state(p.bnd + (int64_t(sq.slot0) * p.H + h) * kStateElems);
+  if (n == 0 && p.s_out != nullptr) store_state(p.s_out + bh * kStateElems);
   __syncthreads();
-  if (tid < kTokVT) {
-    stf<T>(p.out, idx + vt * kTokVT + tid, s_red[1][0][tid] + s_red[1][1][tid] + s_red[1][2][tid] + s_red[1][3][tid]);
+
+#pragma unroll 1
+  for (int t = 0; t < n; ++t) {
+    // reciprocal norms of the raw q and k (1 when the inputs are already normalised)
+    float iq = 1.f, ik = 1.f;
+    if (pro_norm) {
+      iq = rsqrtf(s_nrm[t][0][0] + s_nrm[t][1][0] + s_nrm[t][2][0] + s_nrm[t][3][0] + kPrologueEps);
+      ik = rsqrtf(s_nrm[t][0][1] + s_nrm[t][1][1] + s_nrm[t][2][1] + s_nrm[t][3][1] + kPrologueEps);
+    }
+    // X = a * S ; partial r = X^T e over this thread's rows
+    float r[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i) {
+      const float a = s_a[t][rg + 16 * i], e = kPro ? s_e[t][rg + 16 * i] * ik : s_e[t][rg + 16 * i];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        S[i][c] *= a;
+        r[c] = fmaf(S[i][c], e, r[c]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      r[c] += __shfl_xor_sync(0xffffffffu, r[c], 8);
+      r[c] += __shfl_xor_sync(0xffffffffu, r[c], 16);
+    }
+    if (lane < 8) *reinterpret_cast<float4*>(&s_red[0][warp][cg * 4]) = make_float4(r[0], r[1], r[2], r[3]);
+    __syncthreads();
+
+    const float4 rs = ld_red4(s_red[0], cg * 4);
+    const float u[4] = {s_z[t][cg * 4 + 0] - rs.x, s_z[t][cg * 4 + 1] - rs.y,
+                        s_z[t][cg * 4 + 2] - rs.z, s_z[t][cg * 4 + 3] - rs.w};
+    // S = X + k u^T ; partial o = S^T (scale q)
+    float o[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int i = 0; i < kRowsPerThread; ++i) {
+      const float kv = kPro ? s_k[t][rg + 16 * i] * ik : s_k[t][rg + 16 * i];
+      const float qv = kPro ? s_q[t][rg + 16 * i] * iq : s_q[t][rg + 16 * i];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        S[i][c] = fmaf(kv, u[c], S[i][c]);
+        o[c] = fmaf(S[i][c], qv, o[c]);
+      }
+    }
+    if (t + 1 == n) {
+      if (p.s_out != nullptr) store_state(p.s_out + bh * kStateElems);
+      if (p.bnd != nullptr) store_state(p.bnd + (int64_t(sq.slot0 + 1) * p.H + h) * kStateElems);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      o[c] += __shfl_xor_sync(0xffffffffu, o[c], 8);
+      o[c] += __shfl_xor_sync(0xffffffffu, o[c], 16);
+    }
+    if (lane < 8) *reinterpret_cast<float4*>(&s_red[1][warp][cg * 4]) = make_float4(o[0], o[1], o[2], o[3]);
+    __syncthreads();
+    if (tid < kTokVT) {
+      const float ov = s_red[1][0][tid] + s_red[1][1][tid] + s_red[1][2][tid] + s_red[1][3][tid];
+      stf<T>(p.out, row_of(t) + vt * kTokVT + tid, ov);
+    }
   }
 }
 
@@ -408,6 +460,25 @@ __global__ void __launch_bounds__(kTokThreads) token_t1_zero_kernel(const T1Zero
 
 inline bool grid_fits(int64_t blocks) { return blocks > 0 && blocks <= int64_t(0x7fffffff); }
 
+// `most`: 1 (T == 1 without checkpoints), 4 or 8, the most tokens a sequence has
+template <typename Seqs>
+int launch_steps(const TokenStepParams& p, const Seqs& seqs, int64_t blocks, int most, int dtype, int g_dtype,
+                 cudaStream_t stream) {
+  if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
+  auto run = [&](auto tok) {
+    constexpr int kTok = decltype(tok)::value;
+    GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+      if (p.prologue != 0) token_step_kernel<T, G, Seqs, true, kTok><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
+      else token_step_kernel<T, G, Seqs, false, kTok><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
+    });
+    return check_launch();
+  };
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
+    if (most == 1) return run(std::integral_constant<int, 1>{});
+  }
+  return most == 4 ? run(std::integral_constant<int, 4>{}) : run(std::integral_constant<int, kStepTokens>{});
+}
+
 }  // namespace
 
 // ---- launchers (called from api.cu) --------------------------------------------------
@@ -437,16 +508,25 @@ int launch_token_forward(const void* q, const void* k, const void* v, const void
     });
     return check_launch();
   }
-  if (T == 1 && t_end - t_begin == 1 && bnd == nullptr) {
-    const TokenStepParams p{q, k, v, g, beta, w, s_in, out, s_out, scale, prologue};
-    GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-      if (prologue != 0) token_step_kernel<T, G, true><<<unsigned(blocks), kTokThreads, 0, stream>>>(p);
-      else token_step_kernel<T, G, false><<<unsigned(blocks), kTokThreads, 0, stream>>>(p);
-    });
-    return check_launch();
+  // Token by token up to 8 tokens: the spans of token_span.cu cost nearly as much for one token as for 16
+  // (B32 H32, 2 tokens: 73 us there, 32 here; 8 tokens: 87 there, 77 here).
+  const int64_t tokens = t_end - t_begin;
+  if (tokens >= 1 && tokens <= kStepTokens) {
+    const TokenStepParams p{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), 0, scale, prologue};
+    const int most = T == 1 && bnd == nullptr ? 1 : tokens <= 4 ? 4 : kStepTokens;
+    return launch_steps(p, UniformSeqs{t_begin, T, int(tokens), 1, int(B)}, blocks, most, dtype, g_dtype, stream);
   }
   return launch_span_forward(q, k, v, g, beta, w, s_in, out, s_out, bnd, B, T, H, t_begin, t_end, dtype, g_dtype,
                              scale, prologue, stream);
+}
+
+// the sequences from `first` on, none of more than kStepTokens tokens
+int launch_packed_steps(const PackedSpans& table, int first, const void* q, const void* k, const void* v, const void* g,
+                        const void* beta, const void* w, const float* s_in, void* out, float* s_out, float* bnd,
+                        int64_t H, int dtype, int g_dtype, float scale, int prologue, cudaStream_t stream) {
+  const TokenStepParams p{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), first, scale, prologue};
+  return launch_steps(p, table, (table.n - first) * H * kTokTiles, table.e[first].len <= 4 ? 4 : kStepTokens, dtype,
+                      g_dtype, stream);
 }
 
 int launch_token_t1_zero(const void* q, const void* k, const void* v, const void* w, void* out,

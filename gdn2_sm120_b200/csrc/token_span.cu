@@ -23,6 +23,9 @@
 
 namespace gdn2 {
 
+int launch_packed_steps(const PackedSpans&, int, const void*, const void*, const void*, const void*, const void*,
+                        const void*, const float*, void*, float*, float*, int64_t, int, int, float, int, cudaStream_t);
+
 namespace {
 
 constexpr int kSpan = kTokenInterval;          // 16
@@ -1028,8 +1031,18 @@ int launch_packed_token_forward(const PackedSpans& table, const void* q, const v
                                 const void* beta, const void* w, const float* s_in, void* out, float* s_out,
                                 float* bnd, int64_t H, int dtype, int g_dtype, float scale, int prologue,
                                 cudaStream_t stream) {
-  return run_forward(table, SpanFwdParams{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), scale, prologue}, dtype,
-                     g_dtype, stream);
+  // longest first: the sequences of a few tokens are the end of the list
+  int spans = 0;
+  while (spans < table.n && table.e[spans].len > kStepTokens) ++spans;
+  if (spans > 0) {
+    PackedSpans longer = table;
+    longer.n = spans;
+    const int st = run_forward(longer, SpanFwdParams{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), scale, prologue},
+                               dtype, g_dtype, stream);
+    if (st != GDN2_OK || spans == table.n) return st;
+  }
+  return launch_packed_steps(table, spans, q, k, v, g, beta, w, s_in, out, s_out, bnd, H, dtype, g_dtype, scale,
+                             prologue, stream);
 }
 
 int launch_packed_token_backward(const PackedSpans& table, const void* q, const void* k, const void* v, const void* g,

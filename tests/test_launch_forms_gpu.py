@@ -109,3 +109,23 @@ def test_token_spans_at_the_grid_where_the_form_changes(batch, heads, time):
     tensors, d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
     full = _step(tensors, d_out, d_fin)
     _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
+
+
+# token by token up to 8 tokens (inputs of 4 read at once), spans from 9 on; the prologue's rows as well
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("time", [2, 4, 5, 8, 9])
+def test_few_tokens_with_and_without_the_prologue(time, raw):
+    make = oracle.make_raw_inputs if raw else oracle.make_inputs
+    cpu = make(3, time, 2, seed=time)
+    state = 0.05 * torch.randn(3, 2, 128, 128, generator=torch.Generator().manual_seed(time))
+    flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
+    with torch.no_grad():
+        out, fin = chunk_gdn2(*[t.to(DEV) for t in cpu[:6]], state.to(DEV), output_final_state=True, **flags)
+    plain = cpu[:6]
+    if raw:
+        q, k, v, g, beta, w = [t.double() for t in cpu[:6]]
+        norm = lambda x: x * torch.rsqrt((x * x).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
+        plain = (norm(q), norm(k), v, -torch.nn.functional.softplus(g), torch.sigmoid(beta), torch.sigmoid(w))
+    ref_out, ref_state = oracle.recurrence(*plain, state)
+    torch.testing.assert_close(out.float().cpu(), ref_out.float(), rtol=2e-2, atol=1e-2)
+    assert oracle.rel_l2(fin, ref_state) < 1e-3
