@@ -129,3 +129,22 @@ def test_few_tokens_with_and_without_the_prologue(time, raw):
     ref_out, ref_state = oracle.recurrence(*plain, state)
     torch.testing.assert_close(out.float().cpu(), ref_out.float(), rtol=2e-2, atol=1e-2)
     assert oracle.rel_l2(fin, ref_state) < 1e-3
+
+
+def test_joint_launch_replays_from_a_cuda_graph():
+    tensors, _, _ = _device_inputs(1, 80 * 64, 16, seed=11)
+    with torch.no_grad():
+        expected = chunk_gdn2(*tensors, output_final_state=True)
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            chunk_gdn2(*tensors, output_final_state=True)
+        torch.cuda.current_stream().wait_stream(stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            got = chunk_gdn2(*tensors, output_final_state=True)
+        for _ in range(2):
+            got[0].zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(got[0], expected[0]) and torch.equal(got[1], expected[1])
