@@ -166,6 +166,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     issue_kqb(at);
   }
   const uint32_t leader = elect_leader();
+  const bool wide_tiles = (reinterpret_cast<uintptr_t>(p.tiles.yt) & 31) == 0;  // (a tile is 32 KiB)
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
   using RawG = typename Raw4<G>::type;
@@ -619,10 +620,18 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     float y[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
+    // (buffers are 16-byte aligned by contract; from an allocator they are 32-byte aligned as well)
+    if (wide_tiles) {
 #pragma unroll
-    for (int j = 0; j < 32; j += 8) {
-      store_global_32b(row_yt + j, make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]),
-                       make_float4(y[j + 4], y[j + 5], y[j + 6], y[j + 7]));
+      for (int j = 0; j < 32; j += 8) {
+        store_global_32b(row_yt + j, make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]),
+                         make_float4(y[j + 4], y[j + 5], y[j + 6], y[j + 7]));
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 32; j += 4) {
+        *reinterpret_cast<float4*>(row_yt + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+      }
     }
   }
   tc_fence_before();  // the next unit's products replace these accumulators, behind two barriers
