@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import gdn2_oracle as oracle
-from gdn2_sm120_b200 import _lib, chunk_kernels
+from gdn2_sm120_b200 import _lib, chunk_gdn2, chunk_kernels
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -41,3 +41,32 @@ def test_chunk_forward_takes_buffers_aligned_to_16_bytes(batch, time, heads, tra
         results.append((out, fin) if bnd is None else (out, fin, bnd))
     for other in results[1:]:
         assert all(torch.equal(a, b) for a, b in zip(results[0], other))
+
+
+# Every term of dg_t holds exp(g_t): a product of at most 16 exponentials of 2 units in the last place each is
+# right to 4e-6, the 16 x 16 solve and the sums over channels as much again: 1e-5 for each token.  "mixed": a
+# third of the decays strong and the others weak; "zeroed": some decays are exactly zero, and so is their dg.
+@pytest.mark.parametrize("decay", [-1.0, -5.0, -10.0, -15.0, -25.0, "mixed", "zeroed"])
+@pytest.mark.parametrize("time", [1, 16, 17, 47])
+def test_log_decay_gradients_of_short_sequences_at_any_decay(time, decay):
+    batch, heads = 2, 2
+    cpu = list(oracle.make_inputs(batch, time, heads, seed=time))
+    gen = torch.Generator().manual_seed(time + 1)
+    u, third = torch.rand(cpu[3].shape, generator=gen), torch.rand(cpu[3].shape, generator=gen) < 0.33
+    if decay == "mixed":
+        cpu[3] = torch.where(third, -20.0 * u, -0.05 * u)
+    elif decay == "zeroed":
+        cpu[3] = torch.where(third, torch.full_like(u, -float("inf")), -0.5 * u)
+    else:
+        cpu[3] = decay * (0.5 + u)
+    d_out = torch.randn(cpu[2].shape, generator=gen).to(cpu[2].dtype)
+    d_fin = torch.randn((batch, heads, 128, 128), generator=gen)
+    _, _, ref = oracle.recurrence_grads(*cpu, d_out, d_fin)
+    leaves = [t.to(DEV).requires_grad_(True) for t in cpu]
+    out, fin = chunk_gdn2(*leaves[:6], leaves[6], output_final_state=True)
+    dg = torch.autograd.grad([out, fin], leaves, [d_out.to(DEV), d_fin.to(DEV)])[3]
+    if decay == "zeroed":
+        assert (dg.cpu()[third] == 0).all()
+    for t in range(time):
+        err = oracle.rel_l2(dg[:, t], ref[3][:, t])
+        assert err < 1e-5, f"token {t}: rel-L2 {err:.3e}"
