@@ -326,7 +326,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
       const int i = i0 + 4 * e;
       if (pro_gate) {
 #pragma unroll
-        for (int f = 0; f < 4; f += 2) prologue_sigmoid2(bb[e][f], bb[e][f + 1]);
+        for (int f = 0; f < 4; ++f) bb[e][f] = prologue_sigmoid(bb[e][f]);
       }
       float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4];
 #pragma unroll
@@ -1085,7 +1085,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         }
         if (p.activate_w) {
 #pragma unroll
-          for (int j = 0; j < 16; j += 2) prologue_sigmoid2(z[j], z[j + 1]);
+          for (int j = 0; j < 16; ++j) z[j] = prologue_sigmoid(z[j]);
         }
         uint32_t zr[16];
 #pragma unroll

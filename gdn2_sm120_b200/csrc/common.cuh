@@ -120,15 +120,6 @@ __device__ __forceinline__ float prologue_sigmoid(float x) {
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + __expf(-x)));
   return r;
 }
-// Two at a time with one reciprocal, 1 / (a b): three special-function results instead of four.  The
-// arguments are held to -43 so that the product stays finite (a sigmoid is 2e-19 there).
-__device__ __forceinline__ void prologue_sigmoid2(float& x, float& y) {
-  const float a = 1.f + __expf(-fmaxf(x, -43.f)), b = 1.f + __expf(-fmaxf(y, -43.f));
-  float r;
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(a * b));
-  x = r * b;
-  y = r * a;
-}
 // log-decay g = -softplus(x) = -log(1 + e^x).  Small e^x: the series e - e^2/2 + e^3/3 (its first
 // dropped term is below 2^-26 of the sum there; lg2 of a number next to 1 would lose the digits);
 // softplus(x) equals x to fp32 precision beyond 20.

@@ -8,6 +8,7 @@ import torch
 
 import gdn2_oracle as oracle
 from gdn2_sm120_b200 import _lib, chunk_gdn2, chunk_kernels
+from gdn2_sm120_b200.varlen import chunk_gdn2_varlen
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda"
@@ -70,3 +71,32 @@ def test_log_decay_gradients_of_short_sequences_at_any_decay(time, decay):
     for t in range(time):
         err = oracle.rel_l2(dg[:, t], ref[3][:, t])
         assert err < 1e-5, f"token {t}: rel-L2 {err:.3e}"
+
+
+RAW = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True}
+
+
+# -inf and the type's lowest value close a gate completely (sigmoid = 0): nothing is written, the state stays zero
+@pytest.mark.parametrize("closed", [-float("inf"), torch.finfo(torch.bfloat16).min])
+@pytest.mark.parametrize("time", [1, 5, 40, 64, 101])
+def test_closed_gates_of_the_fused_prologue_write_nothing(time, closed):
+    cpu = oracle.make_raw_inputs(1, time, 2, seed=time)
+    q, k, v, g, beta, w = [t.to(DEV) for t in cpu[:6]]
+    w[:, :, 1] = closed
+    with torch.no_grad():
+        out, fin = chunk_gdn2(q, k, v, g, beta, w, output_final_state=True, **RAW)
+    assert (out[:, :, 1] == 0).all() and (fin[:, 1] == 0).all()
+    assert (out[:, :, 0] != 0).any() and torch.isfinite(out).all()
+
+
+# the first sequence ends inside a pair of tokens whose second one is the next sequence's
+@pytest.mark.parametrize("first", [100, 101])
+def test_a_nan_behind_the_end_of_a_packed_sequence_stays_there(first):
+    cpu = oracle.make_raw_inputs(1, 200, 2, seed=first)
+    seq = [t.to(DEV) for t in cpu[:6]]
+    with torch.no_grad():
+        expected, _ = chunk_gdn2_varlen(*seq, [0, first, 200], **RAW)
+        for t in seq:
+            t[0, first] = float("nan")
+        out, _ = chunk_gdn2_varlen(*seq, [0, first, 200], **RAW)
+    assert torch.equal(out[:, :first], expected[:, :first])
