@@ -434,8 +434,10 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
           matrix_row(rows.m, i, m);
           float o = (sm.part[0][i][1][col] + sm.part[1][i][1][col]) +
                     (sm.part[2][i][1][col] + sm.part[3][i][1][col]);
+          // tokens up to i alone: what follows must not reach this output, not even as 0 times an infinity
+          static_assert(kThreads / kCols == 4, "rows i of this thread: 4 x + 0..3");
 #pragma unroll
-          for (int j = 0; j < kSpan; ++j) o = fmaf(m[j], u[j], o);
+          for (int j = 0; j < 4 * x + 4; ++j) o = j <= i ? fmaf(m[j], u[j], o) : o;
           stf<T>(p.out, ((row0 + i) * p.H + h) * kDim + tile * kCols + col, o);
         }
       }

@@ -100,3 +100,16 @@ def test_a_nan_behind_the_end_of_a_packed_sequence_stays_there(first):
             t[0, first] = float("nan")
         out, _ = chunk_gdn2_varlen(*seq, [0, first, 200], **RAW)
     assert torch.equal(out[:, :first], expected[:, :first])
+
+
+# spans of 16 tokens: in the middle of the only one, in the second, at the first token of one
+@pytest.mark.parametrize("time,at", [(12, 5), (40, 20), (33, 16), (16, 15)])
+@pytest.mark.parametrize("name,value", [("q", "nan"), ("k", "nan"), ("v", "inf"), ("g", "nan"), ("beta", "nan"), ("w", "nan")])
+def test_outputs_do_not_depend_on_later_tokens(time, at, name, value):
+    seq = dict(zip(("q", "k", "v", "g", "beta", "w"), [t.to(DEV) for t in oracle.make_inputs(2, time, 2, seed=time)]))
+    with torch.no_grad():
+        expected, _ = chunk_gdn2(*seq.values())
+        seq[name][:, at, 1, 7] = float(value)
+        out, _ = chunk_gdn2(*seq.values())
+    assert torch.equal(out[:, :at], expected[:, :at]) and torch.equal(out[:, :, 0], expected[:, :, 0])
+    assert not torch.isfinite(out[:, at, 1]).all()
