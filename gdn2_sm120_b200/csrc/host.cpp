@@ -225,8 +225,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                          : fin_given ? *fin_given
                                      : floats({s.batch, s.heads, kDim, kDim}, *s.t[0]);
   if ((out_given || fin_given || inplace) && !apart(s, init, out, fin, out_given, fin_given || inplace)) return none();
-  // (token path: an exact alias is spelled inplace_final_state, an aliasing final_state_out is refused there)
-  if (!chunked && fin_given && init && Span(fin).meets(Span(*init))) return none();
+  // (an exact alias is spelled inplace_final_state, a final_state_out that meets initial_state is refused)
+  if (fin_given && init && Span(fin).meets(Span(*init))) return none();
   void* stream = at::cuda::getCurrentCUDAStream().stream();
   int status;
   if (chunked) {

@@ -7,7 +7,7 @@ import pytest
 import torch
 
 import gdn2_oracle as oracle
-from gdn2_sm120_b200 import _lib, chunk_gdn2, chunk_kernels
+from gdn2_sm120_b200 import _lib, chunk_gdn2, chunk_kernels, recurrent_gdn2
 from gdn2_sm120_b200.varlen import chunk_gdn2_varlen
 
 pytestmark = pytest.mark.gpu
@@ -113,3 +113,12 @@ def test_outputs_do_not_depend_on_later_tokens(time, at, name, value):
         out, _ = chunk_gdn2(*seq.values())
     assert torch.equal(out[:, :at], expected[:, :at]) and torch.equal(out[:, :, 0], expected[:, :, 0])
     assert not torch.isfinite(out[:, at, 1]).all()
+
+
+@pytest.mark.parametrize("time", [1, 5, 64, 100])
+def test_final_state_out_that_is_the_initial_state_is_refused(time):
+    tensors = [t.to(DEV) for t in oracle.make_inputs(2, time, 2, seed=time)]
+    before = tensors[6].clone()
+    with pytest.raises(ValueError, match="final_state_out must not overlap"):
+        recurrent_gdn2(*tensors, final_state_out=tensors[6])
+    assert torch.equal(tensors[6], before)
