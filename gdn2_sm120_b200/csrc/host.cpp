@@ -188,7 +188,9 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!g_bound || n != 14 || !read_seq(a, &s) || !read_scale(a[7], &scale)) return none();
   const at::Tensor *init = nullptr, *fin_given = nullptr;
   if (read_state(a[6], s, &init) < 0 || read_state(a[9], s, &fin_given) < 0) return none();
-  const bool inplace = a[10] == Py_True, chunk_api = a[12] == Py_True;
+  const int truth = PyObject_IsTrue(a[10]);  // (any object is a flag in Python: 1, a NumPy bool)
+  if (truth < 0) return nullptr;
+  const bool inplace = truth != 0, chunk_api = a[12] == Py_True;
   const int prologue = int(PyLong_AsLong(a[11]));
   const int64_t budget = PyLong_AsLongLong(a[13]);
   if (inplace && (init == nullptr || fin_given != nullptr)) return none();

@@ -3,6 +3,7 @@ non-finite values, strong decays, flags that are no booleans, threads beside a b
 
 from __future__ import annotations
 
+import numpy as np
 import pytest
 import torch
 
@@ -122,3 +123,12 @@ def test_final_state_out_that_is_the_initial_state_is_refused(time):
     with pytest.raises(ValueError, match="final_state_out must not overlap"):
         recurrent_gdn2(*tensors, final_state_out=tensors[6])
     assert torch.equal(tensors[6], before)
+
+
+@pytest.mark.parametrize("flag", [1, np.True_])
+@pytest.mark.parametrize("time", [1, 5, 64])
+def test_inplace_update_with_a_flag_that_is_no_bool(time, flag):
+    tensors = [t.to(DEV) for t in oracle.make_inputs(2, time, 2, seed=time)]
+    expected = recurrent_gdn2(*tensors)
+    out, state = recurrent_gdn2(*tensors, inplace_final_state=flag)
+    assert state is tensors[6] and torch.equal(state, expected[1]) and torch.equal(out, expected[0])
