@@ -125,6 +125,13 @@ bool read_scale(PyObject* o, float* scale) {
   return std::isfinite(value) && std::isfinite(*scale);
 }
 
+// the scratch budget, a module variable that callers set: a float or a huge number is left to Python
+bool read_budget(PyObject* o, int64_t* budget) {
+  int overflow = 1;
+  if (PyLong_Check(o)) *budget = PyLong_AsLongLongAndOverflow(o, &overflow);
+  return overflow == 0;
+}
+
 struct Span {
   uintptr_t lo, hi;
   explicit Span(const at::Tensor& t)
@@ -192,7 +199,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (truth < 0) return nullptr;
   const bool inplace = truth != 0, chunk_api = a[12] == Py_True;
   const int prologue = int(PyLong_AsLong(a[11]));
-  const int64_t budget = PyLong_AsLongLong(a[13]);
+  int64_t budget;
+  if (!read_budget(a[13], &budget)) return none();
   if (inplace && (init == nullptr || fin_given != nullptr)) return none();
   if (chunk_api && c10::GradMode::is_enabled()) {
     bool grad = init != nullptr && init->requires_grad();
@@ -279,7 +287,8 @@ PyObject* train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (!g_bound || n != 9 || !read_seq(a, &s) || !read_scale(a[7], &scale) || read_state(a[6], s, &init) < 0) {
     return none();
   }
-  const int64_t budget = PyLong_AsLongLong(a[8]);
+  int64_t budget;
+  if (!read_budget(a[8], &budget)) return none();
   const bool chunked = s.time >= kChunk;
   const at::Tensor& q = *s.t[0];
   int64_t full = 0, ws_bytes = 0;

@@ -132,3 +132,14 @@ def test_inplace_update_with_a_flag_that_is_no_bool(time, flag):
     expected = recurrent_gdn2(*tensors)
     out, state = recurrent_gdn2(*tensors, inplace_final_state=flag)
     assert state is tensors[6] and torch.equal(state, expected[1]) and torch.equal(out, expected[0])
+
+
+@pytest.mark.parametrize("budget", [1e10, 10 ** 20])
+def test_a_scratch_budget_that_is_no_64_bit_int(monkeypatch, budget):
+    tensors = [t.to(DEV) for t in oracle.make_inputs(2, 130, 2, seed=3)]
+    leaves = [t.clone().requires_grad_(True) for t in tensors]
+    expected = chunk_gdn2(*tensors, output_final_state=True)
+    monkeypatch.setattr(chunk_kernels, "SCRATCH_BUDGET_BYTES", budget)
+    for got in (chunk_gdn2(*tensors, output_final_state=True), chunk_gdn2(*leaves, output_final_state=True),
+                recurrent_gdn2(*tensors)):
+        assert torch.equal(got[0], expected[0]) and torch.equal(got[1], expected[1])
