@@ -160,6 +160,17 @@ void count(long kernels) {
   if (now != nullptr) PyList_SetItem(g_launches, 0, now);
 }
 
+// Other Python threads run while a call allocates and launches: an allocation may go to the driver and a launch
+// waits where the launch queue is full or its kernel is loaded for the first time.
+struct WithoutGil {
+  PyThreadState* state = PyEval_SaveThread();
+  void end() {
+    if (state != nullptr) PyEval_RestoreThread(state);
+    state = nullptr;
+  }
+  ~WithoutGil() { end(); }
+};
+
 // false with a Python exception set when the entry point failed
 bool ok(int status, const char* name, long kernels) {
   if (status == GDN2_OK) { count(kernels); return true; }
@@ -229,17 +240,26 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     sc_bytes = api.chunk_scratch_bytes(s.batch, full, s.heads, 0);
     if (ws_bytes <= 0 || sc_bytes <= 0 || sc_bytes > budget || ws_bytes + sc_bytes >= kCheckedBytes) return none();
   }
-  const c10::cuda::CUDAGuard guard(s.t[0]->device());
-  const at::Tensor out = out_given ? *out_given : at::empty(s.t[0]->sizes(), s.t[0]->options());
-  const at::Tensor fin = inplace     ? *init
-                         : fin_given ? *fin_given
-                                     : floats({s.batch, s.heads, kDim, kDim}, *s.t[0]);
-  if ((out_given || fin_given || inplace) && !apart(s, init, out, fin, out_given, fin_given || inplace)) return none();
-  // (an exact alias is spelled inplace_final_state, a final_state_out that meets initial_state is refused)
-  if (fin_given && init && Span(fin).meets(Span(*init))) return none();
-  void* stream = at::cuda::getCurrentCUDAStream().stream();
+  at::Tensor out, fin;
   int status;
+  const char* name;
+  bool distinct = true;
+  WithoutGil others;
+  const c10::cuda::CUDAGuard guard(s.t[0]->device());
+  out = out_given ? *out_given : at::empty(s.t[0]->sizes(), s.t[0]->options());
+  fin = inplace ? *init : fin_given ? *fin_given : floats({s.batch, s.heads, kDim, kDim}, *s.t[0]);
+  if (out_given || fin_given || inplace) {
+    // (an exact alias is spelled inplace_final_state, a final_state_out that meets initial_state is refused)
+    distinct = apart(s, init, out, fin, out_given, fin_given || inplace) &&
+               !(fin_given && init && Span(fin).meets(Span(*init)));
+  }
+  void* stream = at::cuda::getCurrentCUDAStream().stream();
+  if (!distinct) {
+    others.end();
+    return none();
+  }
   if (chunked) {
+    name = "gdn2_chunk_forward";
     const at::Tensor buffer = bytes(ws_bytes + sc_bytes, *s.t[0]);
     uint8_t* ws = static_cast<uint8_t*>(buffer.data_ptr());
     if (prologue) {
@@ -251,22 +271,23 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                  out.data_ptr(), fptr(&fin), nullptr, ws, ws + ws_bytes, s.batch, s.time, s.heads,
                                  full, 0, s.dtype, s.g_dtype, scale, stream);
     }
-    if (!ok(status, "gdn2_chunk_forward", 2)) return nullptr;
   } else if (s.time == 1 && init == nullptr) {
+    name = "gdn2_token_forward_t1_zero";
     status = prologue ? api.token_forward_t1_zero_fused(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(5), out.data_ptr(),
                                                         fptr(&fin), s.batch, s.heads, s.dtype, scale, prologue, stream)
                       : api.token_forward_t1_zero(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(5), out.data_ptr(), fptr(&fin),
                                                   s.batch, s.heads, s.dtype, scale, stream);
-    if (!ok(status, "gdn2_token_forward_t1_zero", 1)) return nullptr;
   } else {
+    name = "gdn2_token_forward";
     status = prologue ? api.token_forward_fused(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init),
                                                 out.data_ptr(), fptr(&fin), s.batch, s.time, s.heads, 0, s.time,
                                                 s.dtype, s.g_dtype, scale, prologue, stream)
                       : api.token_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init),
                                           out.data_ptr(), fptr(&fin), nullptr, s.batch, s.time, s.heads, 0, s.time,
                                           s.dtype, s.g_dtype, scale, stream);
-    if (!ok(status, "gdn2_token_forward", 1)) return nullptr;
   }
+  others.end();
+  if (!ok(status, name, chunked ? 2 : 1)) return nullptr;
   PyObject* first = out_given ? Py_NewRef(a[8]) : wrap(out);
   PyObject* second = inplace ? Py_NewRef(a[6]) : fin_given ? Py_NewRef(a[9]) : wrap(fin);
   PyObject* result = PyTuple_New(2);
@@ -302,27 +323,28 @@ PyObject* train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                   api.chunk_scratch_bytes(s.batch, full, s.heads, 1) + states);
     if (ws_bytes <= 0 || (wave > budget && s.batch > 1) || ws_bytes + states + wave >= kCheckedBytes) return none();
   }
+  at::Tensor out, fin, boundaries, workspace;
+  int status;
+  WithoutGil others;
   const c10::cuda::CUDAGuard guard(q.device());
-  at::Tensor out = at::empty(q.sizes(), q.options());
-  at::Tensor fin = floats({s.batch, s.heads, kDim, kDim}, q);
+  out = at::empty(q.sizes(), q.options());
+  fin = floats({s.batch, s.heads, kDim, kDim}, q);
   const int64_t slots = chunked ? full / kChunk + 1 : ceil_div(s.time, kInterval) + 1;
-  at::Tensor boundaries = floats({s.batch, slots, s.heads, kDim, kDim}, q);
-  at::Tensor workspace;
+  boundaries = floats({s.batch, slots, s.heads, kDim, kDim}, q);
   void* stream = at::cuda::getCurrentCUDAStream().stream();
   if (chunked) {
     workspace = bytes(ws_bytes, q);
     // (the forward scratch of a training call is reserved, nothing is written there)
-    const int status = api.chunk_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init),
-                                         out.data_ptr(), fptr(&fin), fptr(&boundaries), workspace.data_ptr(),
-                                         workspace.data_ptr(), s.batch, s.time, s.heads, full, 1, s.dtype, s.g_dtype,
-                                         scale, stream);
-    if (!ok(status, "gdn2_chunk_forward", 2)) return nullptr;
+    status = api.chunk_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init), out.data_ptr(),
+                               fptr(&fin), fptr(&boundaries), workspace.data_ptr(), workspace.data_ptr(), s.batch,
+                               s.time, s.heads, full, 1, s.dtype, s.g_dtype, scale, stream);
   } else {
-    const int status = api.token_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init),
-                                         out.data_ptr(), fptr(&fin), fptr(&boundaries), s.batch, s.time, s.heads, 0,
-                                         s.time, s.dtype, s.g_dtype, scale, stream);
-    if (!ok(status, "gdn2_token_forward", 1)) return nullptr;
+    status = api.token_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init), out.data_ptr(),
+                               fptr(&fin), fptr(&boundaries), s.batch, s.time, s.heads, 0, s.time, s.dtype, s.g_dtype,
+                               scale, stream);
   }
+  others.end();
+  if (!ok(status, chunked ? "gdn2_chunk_forward" : "gdn2_token_forward", chunked ? 2 : 1)) return nullptr;
   PyObject* result = PyTuple_New(4);
   PyTuple_SET_ITEM(result, 0, wrap(out));
   PyTuple_SET_ITEM(result, 1, wrap(fin));
@@ -345,58 +367,64 @@ PyObject* train_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const at::Tensor* workspace = chunked ? tensor(a[8]) : nullptr;
   const at::Tensor* boundaries = tensor(a[9]);
   if (boundaries == nullptr || (chunked && (workspace == nullptr || !s.all_aligned))) return none();
+  const at::Tensor *out_given = nullptr, *fin_given = nullptr;
+  if (a[6] != Py_None) {
+    out_given = tensor(a[6]);
+    if (out_given == nullptr || out_given->sizes() != q.sizes() || out_given->scalar_type() != q.scalar_type() ||
+        out_given->device() != q.device()) {
+      return none();
+    }
+  }
+  if (a[7] != Py_None) {
+    fin_given = tensor(a[7]);
+    if (fin_given == nullptr || fin_given->dim() != 4 || fin_given->numel() != s.batch * s.heads * kDim * kDim ||
+        fin_given->scalar_type() != at::kFloat || fin_given->device() != q.device()) {
+      return none();
+    }
+  }
+  const int64_t full = chunked ? ceil_div(s.time, kChunk) * kChunk : 0;
+  const int64_t states = s.batch * (full / kChunk + 1) * s.heads * kStateBytes;
+  if (chunked && boundaries->numel() * 4 != states) return none();
+  at::Tensor grads[6], d_init;
+  int status, scan_status = GDN2_OK;
+  WithoutGil others;
   const c10::cuda::CUDAGuard guard(q.device());
   auto dense = [](const at::Tensor& t) {
     at::Tensor d = t.contiguous();
     return aligned(d) ? d : d.clone();
   };
-  at::Tensor d_out, d_fin;
-  if (a[6] == Py_None) {
-    d_out = at::zeros(q.sizes(), q.options());
-  } else {
-    const at::Tensor* t = tensor(a[6]);
-    if (t == nullptr || t->sizes() != q.sizes() || t->scalar_type() != q.scalar_type() || t->device() != q.device()) {
-      return none();
-    }
-    d_out = dense(*t);
-  }
-  if (a[7] != Py_None) {
-    const at::Tensor* t = tensor(a[7]);
-    if (t == nullptr || t->dim() != 4 || t->numel() != s.batch * s.heads * kDim * kDim ||
-        t->scalar_type() != at::kFloat || t->device() != q.device()) {
-      return none();
-    }
-    d_fin = dense(*t);
-  }
-  at::Tensor grads[6];
+  const at::Tensor d_out = out_given ? dense(*out_given) : at::zeros(q.sizes(), q.options());
+  const at::Tensor d_fin = fin_given ? dense(*fin_given) : at::Tensor();
   for (int i = 0; i < 6; ++i) grads[i] = at::empty(s.t[i]->sizes(), s.t[i]->options());
-  at::Tensor d_init = floats({s.batch, s.heads, kDim, kDim}, q);
+  d_init = floats({s.batch, s.heads, kDim, kDim}, q);
   const float* df = d_fin.defined() ? static_cast<const float*>(d_fin.data_ptr()) : nullptr;
   void* stream = at::cuda::getCurrentCUDAStream().stream();
   void* g[6];
   for (int i = 0; i < 6; ++i) g[i] = grads[i].data_ptr();
   if (chunked) {
-    const int64_t full = ceil_div(s.time, kChunk) * kChunk;
     const int64_t sc_bytes = api.chunk_scratch_bytes(s.batch, full, s.heads, 1);
-    const int64_t states = s.batch * (full / kChunk + 1) * s.heads * kStateBytes;
-    if (boundaries->numel() * 4 != states) return none();
     const at::Tensor buffer = bytes(states + sc_bytes, q);
     uint8_t* base = static_cast<uint8_t*>(buffer.data_ptr());
-    const int status = api.chunk_backward(
+    status = api.chunk_backward(
         s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), d_out.data_ptr(), df, fptr(boundaries),
         reinterpret_cast<float*>(base), workspace->data_ptr(), base + states, g[0], g[1], g[2], g[3], g[4], g[5],
         fptr(&d_init), s.batch, s.time, s.heads, full, s.dtype, s.g_dtype, scale, stream);
-    if (!ok(status, "gdn2_chunk_backward", 2)) return nullptr;
   } else {
     const at::Tensor d_bnd = at::empty(boundaries->sizes(), boundaries->options());
-    int status = api.token_dstate_scan(s.ptr(0), s.ptr(1), s.ptr(3), s.ptr(4), d_out.data_ptr(), df, fptr(&d_bnd),
-                                       fptr(&d_init), s.batch, s.time, s.heads, 0, s.time, s.dtype, s.g_dtype, scale,
-                                       stream);
-    if (!ok(status, "gdn2_token_dstate_scan", 1)) return nullptr;
-    status = api.token_chunk_vjp(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), d_out.data_ptr(),
-                                 fptr(boundaries), fptr(&d_bnd), g[0], g[1], g[2], g[3], g[4], g[5], s.batch, s.time,
-                                 s.heads, 0, s.time, s.dtype, s.g_dtype, scale, stream);
-    if (!ok(status, "gdn2_token_chunk_vjp", 1)) return nullptr;
+    status = scan_status = api.token_dstate_scan(s.ptr(0), s.ptr(1), s.ptr(3), s.ptr(4), d_out.data_ptr(), df,
+                                                 fptr(&d_bnd), fptr(&d_init), s.batch, s.time, s.heads, 0, s.time,
+                                                 s.dtype, s.g_dtype, scale, stream);
+    if (scan_status == GDN2_OK) {
+      status = api.token_chunk_vjp(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), d_out.data_ptr(),
+                                   fptr(boundaries), fptr(&d_bnd), g[0], g[1], g[2], g[3], g[4], g[5], s.batch, s.time,
+                                   s.heads, 0, s.time, s.dtype, s.g_dtype, scale, stream);
+    }
+  }
+  others.end();
+  if (chunked) {
+    if (!ok(status, "gdn2_chunk_backward", 2)) return nullptr;
+  } else if (!ok(scan_status, "gdn2_token_dstate_scan", 1) || !ok(status, "gdn2_token_chunk_vjp", 1)) {
+    return nullptr;
   }
   PyObject* result = PyTuple_New(7);
   for (int i = 0; i < 6; ++i) PyTuple_SET_ITEM(result, i, wrap(grads[i]));
@@ -416,9 +444,11 @@ PyObject* prologue_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   const bool norm = a[5] == Py_True, gate = a[6] == Py_True;
   if (!norm && !gate) return none();
   const at::Tensor& q = *s.t[0];
-  const c10::cuda::CUDAGuard guard(q.device());
   const int which[5] = {0, 1, 3, 4, 5};  // q k g beta w
   at::Tensor out[5], inv[2];
+  int status;
+  WithoutGil others;
+  const c10::cuda::CUDAGuard guard(q.device());
   const void* in[5];
   void* to[5];
   for (int i = 0; i < 5; ++i) {
@@ -431,9 +461,10 @@ PyObject* prologue_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   if (norm) {
     for (int i = 0; i < 2; ++i) inv[i] = floats({s.batch, s.time, s.heads}, q);
   }
-  const int status = api.gate_prologue(in[0], in[1], in[2], in[3], in[4], to[0], to[1], to[2], to[3], to[4],
-                                       norm ? fptr(&inv[0]) : nullptr, norm ? fptr(&inv[1]) : nullptr, s.batch, s.time,
-                                       s.heads, s.dtype, s.g_dtype, at::cuda::getCurrentCUDAStream().stream());
+  status = api.gate_prologue(in[0], in[1], in[2], in[3], in[4], to[0], to[1], to[2], to[3], to[4],
+                             norm ? fptr(&inv[0]) : nullptr, norm ? fptr(&inv[1]) : nullptr, s.batch, s.time, s.heads,
+                             s.dtype, s.g_dtype, at::cuda::getCurrentCUDAStream().stream());
+  others.end();
   if (!ok(status, "gdn2_gate_prologue", 1)) return nullptr;
   PyObject* result = PyTuple_New(7);
   for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(result, i, out[i].defined() ? wrap(out[i]) : Py_NewRef(a[i]));
@@ -465,8 +496,10 @@ PyObject* prologue_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
       return none();
     }
   }
-  const c10::cuda::CUDAGuard guard(s.t[0]->device());
   at::Tensor out[5];
+  int status;
+  WithoutGil others;
+  const c10::cuda::CUDAGuard guard(s.t[0]->device());
   const void *raw[5], *from[5];
   void* to[5];
   for (int i = 0; i < 5; ++i) {
@@ -476,10 +509,10 @@ PyObject* prologue_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     from[i] = on ? in[i]->data_ptr() : nullptr;
     to[i] = on ? out[i].data_ptr() : nullptr;
   }
-  const int status = api.gate_prologue_vjp(raw[0], raw[1], raw[2], raw[3], raw[4], fptr(inv[0]), fptr(inv[1]), from[0],
-                                           from[1], from[2], from[3], from[4], to[0], to[1], to[2], to[3], to[4],
-                                           s.batch, s.time, s.heads, s.dtype, s.g_dtype,
-                                           at::cuda::getCurrentCUDAStream().stream());
+  status = api.gate_prologue_vjp(raw[0], raw[1], raw[2], raw[3], raw[4], fptr(inv[0]), fptr(inv[1]), from[0], from[1],
+                                 from[2], from[3], from[4], to[0], to[1], to[2], to[3], to[4], s.batch, s.time, s.heads,
+                                 s.dtype, s.g_dtype, at::cuda::getCurrentCUDAStream().stream());
+  others.end();
   if (!ok(status, "gdn2_gate_prologue_vjp", 1)) return nullptr;
   PyObject* result = PyTuple_New(5);
   for (int i = 0; i < 5; ++i) PyTuple_SET_ITEM(result, i, out[i].defined() ? wrap(out[i]) : Py_NewRef(a[7 + i]));

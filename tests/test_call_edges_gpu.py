@@ -3,6 +3,9 @@ non-finite values, strong decays, flags that are no booleans, threads beside a b
 
 from __future__ import annotations
 
+import threading
+import time
+
 import numpy as np
 import pytest
 import torch
@@ -143,3 +146,37 @@ def test_a_scratch_budget_that_is_no_64_bit_int(monkeypatch, budget):
     for got in (chunk_gdn2(*tensors, output_final_state=True), chunk_gdn2(*leaves, output_final_state=True),
                 recurrent_gdn2(*tensors)):
         assert torch.equal(got[0], expected[0]) and torch.equal(got[1], expected[1])
+
+
+def test_other_python_threads_run_while_a_launch_waits():
+    """Launches behind a kernel of a second fill the launch queue, and one waits until it is over: a thread that
+    only looks at the clock must go on meanwhile."""
+
+    tensors = [t.to(DEV) for t in oracle.make_inputs(1, 1, 2, seed=1)]
+    recurrent_gdn2(*tensors, inplace_final_state=True)
+    torch.cuda.synchronize()
+    stop, gaps = threading.Event(), []
+
+    def watch():
+        last = time.perf_counter()
+        while not stop.is_set():
+            time.sleep(0.001)
+            now = time.perf_counter()
+            gaps.append(now - last)
+            last = now
+
+    watcher = threading.Thread(target=watch)
+    watcher.start()
+    longest = 0.0
+    torch.cuda._sleep(2_000_000_000)
+    for _ in range(20000):
+        begin = time.perf_counter()
+        recurrent_gdn2(*tensors, inplace_final_state=True)
+        longest = max(longest, time.perf_counter() - begin)
+        if longest > 0.1:
+            break
+    stop.set()
+    watcher.join()
+    torch.cuda.synchronize()
+    assert longest > 0.1, "no launch waited"
+    assert max(gaps) < 0.5 * longest
