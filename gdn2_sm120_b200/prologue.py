@@ -19,9 +19,12 @@ import torch
 from . import _lib, _validate
 
 
-def _launch_forward(q, k, g, beta, w, normalize_qk, activate_gates):
+def _check(q, k, g, beta, w):
     # beta / w / v share the value-shaped layout checks of the primitive; v is not touched here
     _validate.sequence_inputs(q, k, w, g, beta, w, need_alignment=True)
+
+
+def _launch_forward(q, k, g, beta, w, normalize_qk, activate_gates):
     batch, time, heads, _ = q.shape
     rows = (batch, time, heads)
     outs = [torch.empty_like(t) if on else t for t, on in
@@ -48,11 +51,12 @@ class _GatePrologue(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, g, beta, w, normalize_qk: bool, activate_gates: bool):
         done = None
-        if _lib.KERNEL_EVENTS is None:
+        if _lib.KERNEL_EVENTS is None and isinstance(q, torch.Tensor) and q.is_cuda:
             done = _lib.host().prologue_forward(q, k, g, beta, w, normalize_qk, activate_gates)
         if done is not None:
             *outs, inv_q, inv_k = done
         else:
+            _check(q, k, g, beta, w)
             raw = tuple(_validate.detached(t) for t in (q, k, g, beta, w))
             outs, inv_q, inv_k = _launch_forward(*raw, normalize_qk, activate_gates)
         ctx.normalize_qk, ctx.activate_gates = normalize_qk, activate_gates
@@ -115,6 +119,7 @@ def gate_prologue(q, k, g, beta, w, *, normalize_qk: bool = True, activate_gates
         isinstance(t, torch.Tensor) and t.requires_grad for t in (q, k, g, beta, w))
     if wants_grad:
         return _GatePrologue.apply(q, k, g, beta, w, bool(normalize_qk), bool(activate_gates))
+    _check(q, k, g, beta, w)
     raw = tuple(_validate.detached(t) for t in (q, k, g, beta, w))
     outs, _, _ = _launch_forward(*raw, bool(normalize_qk), bool(activate_gates))
     return tuple(outs)

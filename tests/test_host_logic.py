@@ -237,6 +237,27 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
         _lib.lib()
 
 
+@pytest.mark.parametrize("library", ["there", "missing"])
+@pytest.mark.parametrize("training", [False, True])
+def test_gate_prologue_checks_its_arguments_before_anything_else(monkeypatch, tmp_path, training, library):
+    from gdn2_sm120_b200.prologue import gate_prologue
+
+    if library == "missing":
+        monkeypatch.setattr(_lib, "_handle", None)
+        monkeypatch.setattr(_lib, "_host_module", None)
+        monkeypatch.setenv("GDN2_B200_LIB", str(tmp_path / "nope.so"))
+    q, k, _, g, beta, w = _cpu_inputs()[:6]
+    k.requires_grad_(training)
+    with pytest.raises(TypeError, match="must be torch.Tensor objects"):
+        gate_prologue(q, k, g, beta.tolist(), w)
+    with pytest.raises(TypeError, match="must be torch.Tensor objects"):
+        gate_prologue(q.tolist(), k, g, beta, w)
+    with pytest.raises(ValueError, match="rank-4"):
+        gate_prologue(q, k, g[0], beta, w)
+    with pytest.raises(ValueError, match="CUDA"):
+        gate_prologue(q, k, g, beta, w)
+
+
 def test_wave_plan_sizes_training_waves_for_the_backward_transients():
     """The workspace of a wave is what backward consumes, so backward runs over the forward's waves: a
     training plan must keep the backward scratch of a wave (dZ tiles + cotangent checkpoints) inside the
