@@ -14,7 +14,9 @@ import importlib.machinery
 import importlib.util
 import os
 import pathlib
+import sys
 import threading
+import warnings
 
 import torch
 
@@ -99,26 +101,50 @@ def lib() -> ctypes.CDLL:
     return _handle
 
 
+def host_path() -> pathlib.Path:
+    """The native host path is tied to the Python and PyTorch it was built with: its file carries their versions."""
+
+    return _PACKAGE_DIR / f"_host.{sys.implementation.cache_tag}.torch-{torch.__version__}.so"
+
+
+class _PythonWay:
+    """Stands in for the native host path and takes no call: the Python wrappers do the same on the same kernels."""
+
+    forward = train_forward = train_backward = prologue_forward = prologue_backward = staticmethod(lambda *_: None)
+
+
 _host_module = None
 
 
 def host():
-    """The native host path (csrc/host.cpp), bound to the library; raise if it has not been built."""
+    """The native host path (csrc/host.cpp), bound to the library.
+
+    Where it has not been built for this Python and PyTorch, a warning says so once and calls go through the Python
+    wrappers, some 20 us longer each.  Without the library, too, calls go there: they check their arguments first
+    and then raise."""
 
     global _host_module
     if _host_module is not None:
         return _host_module
+    if _handle is None and not library_path().exists():
+        return _PythonWay
     handle = lib()
-    path = _PACKAGE_DIR / "_host.so"
-    if not path.exists():
-        raise RuntimeError(f"{path} is missing: build it with `python -m gdn2_sm120_b200.build`")
-    loader = importlib.machinery.ExtensionFileLoader("_host", str(path))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
-    loader.exec_module(module)
-    addresses = {name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in _PROTOTYPES}
-    module.bind(addresses, check, LAUNCHES, torch.cuda.OutOfMemoryError)
-    _host_module = module
-    return module
+    with _lock:
+        if _host_module is not None:
+            return _host_module
+        path = host_path()
+        if not path.exists():
+            warnings.warn(f"{path} is missing: calls take some 20 us more on the host until "
+                          "`python -m gdn2_sm120_b200.build` has been run", RuntimeWarning, stacklevel=3)
+            _host_module = _PythonWay
+            return _host_module
+        loader = importlib.machinery.ExtensionFileLoader("_host", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_host", loader))
+        loader.exec_module(module)
+        addresses = {name: ctypes.cast(getattr(handle, name), ctypes.c_void_p).value for name in _PROTOTYPES}
+        module.bind(addresses, check, LAUNCHES, torch.cuda.OutOfMemoryError)
+        _host_module = module
+    return _host_module
 
 
 def dtype_code(dtype: torch.dtype) -> int:

@@ -1,5 +1,6 @@
 """Compile the CUDA sources in ``csrc/`` into ``libgdn2_b200.so`` next to this file, and the native host
-path (``csrc/host.cpp``, a CPython extension against PyTorch's headers) into ``_host.so``.
+path (``csrc/host.cpp``, a CPython extension against PyTorch's headers) into ``_host.<Python>.<PyTorch>.so``:
+another version of either finds no file of its own, and a build makes it.
 
 ``nvcc`` cross-compiles for sm_100a without a GPU, so this runs anywhere the CUDA
 toolkit is installed.  The shared object is built in-tree (it is git-ignored) and is
@@ -19,13 +20,15 @@ import sys
 import sysconfig
 import tempfile
 
+from . import _lib
+
 PACKAGE_DIR = pathlib.Path(__file__).resolve().parent
 CSRC = PACKAGE_DIR / "csrc"
 INCLUDE = PACKAGE_DIR.parent / "include"
 LIB_NAME = "libgdn2_b200.so"
 LIB_PATH = PACKAGE_DIR / LIB_NAME
 HOST_SOURCE = CSRC / "host.cpp"
-HOST_PATH = PACKAGE_DIR / "_host.so"
+HOST_PATH = _lib.host_path()
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",

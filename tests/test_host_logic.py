@@ -8,6 +8,7 @@ from __future__ import annotations
 import ctypes
 import pathlib
 import re
+import sys
 
 import pytest
 import torch
@@ -256,6 +257,22 @@ def test_gate_prologue_checks_its_arguments_before_anything_else(monkeypatch, tm
         gate_prologue(q, k, g[0], beta, w)
     with pytest.raises(ValueError, match="CUDA"):
         gate_prologue(q, k, g, beta, w)
+
+
+def test_native_host_path_belongs_to_one_python_and_torch(monkeypatch, tmp_path):
+    from gdn2_sm120_b200 import build
+
+    monkeypatch.setattr(_lib, "_host_module", None)
+    assert torch.__version__ in _lib.host_path().name and sys.implementation.cache_tag in _lib.host_path().name
+    assert _lib.host().forward.__name__ == "forward" and _lib.host() is not _lib._PythonWay
+    # after an upgrade the old file is neither loaded nor taken for up to date
+    monkeypatch.setattr(_lib, "_host_module", None)
+    monkeypatch.setattr(torch, "__version__", "99.0")
+    monkeypatch.setattr(build, "HOST_PATH", _lib.host_path())
+    assert build._stale()
+    with pytest.warns(RuntimeWarning, match="torch-99.0.so is missing"):
+        assert _lib.host() is _lib._PythonWay
+    assert _lib.host().train_forward(1, 2) is None
 
 
 def test_wave_plan_sizes_training_waves_for_the_backward_transients():
