@@ -169,7 +169,9 @@ class _ChunkGDN2Varlen(torch.autograd.Function):
             workspace, chunk_states, span_states = (next(rest) if there else None for there in present)
             scratch = d_chunk_states = None
             if group.chunks:
-                scratch = _bytes(chunk_kernels.scratch_bytes(1, 64 * group.chunks, heads, True), device)
+                size = chunk_kernels.scratch_bytes(1, 64 * group.chunks, heads, True)
+                chunk_kernels.check_memory(size + chunk_states.numel() * 4, device, "packed backward")
+                scratch = _bytes(size, device)
                 d_chunk_states = torch.empty_like(chunk_states)
             d_span_states = None if span_states is None else torch.empty_like(span_states)
             part = slice(group.first, group.last)

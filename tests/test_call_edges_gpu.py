@@ -180,3 +180,15 @@ def test_other_python_threads_run_while_a_launch_waits():
     torch.cuda.synchronize()
     assert longest > 0.1, "no launch waited"
     assert max(gaps) < 0.5 * longest
+
+
+def test_packed_backward_checks_the_free_memory(monkeypatch):
+    leaves = [t.to(DEV).requires_grad_(True) for t in oracle.make_inputs(1, 300, 2, seed=5)[:6]]
+    out, _ = chunk_gdn2_varlen(*leaves, [0, 100, 300])
+    monkeypatch.setattr(chunk_kernels, "CHECK_MEMORY_MIN_BYTES", 0)
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device: (0, 0))
+    monkeypatch.setattr(torch.cuda, "memory_reserved", lambda device: 0)
+    # 2 + 4 chunks of 2 heads: dZ of 36 KiB each, and cotangents of 64 KiB at 6 + 2 checkpoints
+    needed = 12 * 36 * 1024 + 16 * 65536
+    with pytest.raises(ValueError, match=f"packed backward needs {needed} bytes"):
+        torch.autograd.grad(out.float().sum(), leaves)
