@@ -5,7 +5,7 @@ after asking the C ABI for their sizes:
 
   workspace   what a training forward leaves for backward (160 KiB per 64-token chunk and head;
               an inference call's holds the chunk-end decays and a status word only)
-  scratch     tiles that live inside one call (forward 144 KiB, backward 36 KiB per chunk-head)
+  scratch     tiles that live inside one call (inference forward 144 KiB, backward 36 KiB per chunk-head)
   cotangent checkpoints of backward (64 KiB per chunk-head), also dead when the call returns
 
 A large batch is processed as *waves* of consecutive batch rows: every wave is one call of the
@@ -48,8 +48,8 @@ def workspace_bytes(batch: int, full_tokens: int, heads: int, training: bool = F
 
 def scratch_bytes(batch: int, full_tokens: int, heads: int, backward: bool = False, *,
                   training: bool = False) -> int:
-    """Per-call scratch: of a backward pass, or of the forward of an inference / a training call (a
-    training forward keeps the tiles both scans read in its workspace, so its scratch is smaller)."""
+    """Per-call scratch: of a backward pass, or of the forward of an inference / a training call (reserved: a
+    training forward keeps the tiles both scans read in its workspace and takes NULL for its scratch)."""
 
     kind = 1 if backward else (2 if training else 0)
     size = _lib.lib().gdn2_chunk_scratch_bytes(batch, full_tokens, heads, kind)
@@ -72,10 +72,9 @@ def plan_waves(batch: int, full_tokens: int, heads: int, *, backward: bool = Fal
     if backward:
         per_row = _backward_wave_bytes(1, full_tokens, heads)
     elif training:
-        # backward runs over the same waves (a workspace belongs to one wave): the larger of the two
-        # transients, the backward one (dZ tiles and cotangent checkpoints), sets the wave size
-        per_row = max(scratch_bytes(1, full_tokens, heads, False, training=True),
-                      _backward_wave_bytes(1, full_tokens, heads))
+        # backward runs over the same waves (a workspace belongs to one wave): its transients (dZ tiles and
+        # cotangent checkpoints) set the wave size, the forward has none of its own
+        per_row = _backward_wave_bytes(1, full_tokens, heads)
     else:
         per_row = scratch_bytes(1, full_tokens, heads, False)
     rows = max(1, min(batch, budget // per_row))
@@ -116,11 +115,10 @@ def forward(q, k, v, g, beta, w, initial_state, output, final_state, chunk_bound
     if prologue and training:
         raise ValueError("the fused prologue is forward-only")
     waves = plan_waves(batch, full_tokens, heads, training=training)
-    rows = waves[0][1] - waves[0][0]
-    scratch_size = scratch_bytes(rows, full_tokens, heads, False, training=training)
+    scratch_size = 0 if training else scratch_bytes(waves[0][1] - waves[0][0], full_tokens, heads, False)
     needed = scratch_size + sum(workspace_bytes(b1 - b0, full_tokens, heads, training) for b0, b1 in waves)
     check_memory(needed, q.device, "chunk forward")
-    scratch = torch.empty(scratch_size, device=q.device, dtype=torch.uint8)
+    scratch = None if training else torch.empty(scratch_size, device=q.device, dtype=torch.uint8)
     dtype, g_dtype = _lib.dtype_code(q.dtype), _lib.dtype_code(g.dtype)
     stream = _lib.stream_ptr(q.device)
     workspaces = []
@@ -140,7 +138,7 @@ def forward(q, k, v, g, beta, w, initial_state, output, final_state, chunk_bound
             _lib.call(
                 "gdn2_chunk_forward", q.device, *common,
                 None if chunk_boundaries is None else chunk_boundaries[b0:b1].data_ptr(),
-                workspace.data_ptr(), scratch.data_ptr(), b1 - b0, time, heads, full_tokens, int(training),
+                workspace.data_ptr(), _lib.ptr(scratch), b1 - b0, time, heads, full_tokens, int(training),
                 dtype, g_dtype, scale, stream,
             )
         workspaces.append(workspace)

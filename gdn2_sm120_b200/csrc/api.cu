@@ -327,8 +327,8 @@ int chunk_forward_checked(const void* q, const void* k, const void* v, const voi
                           float* chunk_boundaries, void* workspace, void* scratch, int64_t batch, int64_t time,
                           int64_t heads, int64_t full_tokens, int training, int dtype, int g_dtype, float scale,
                           int prologue, void* stream) {
-  if (!q || !k || !v || !g || !beta || !w || !out || !workspace || !scratch) return GDN2_ERR_NULL_POINTER;
-  if (training && !chunk_boundaries) return GDN2_ERR_NULL_POINTER;
+  if (!q || !k || !v || !g || !beta || !w || !out || !workspace) return GDN2_ERR_NULL_POINTER;
+  if (training ? !chunk_boundaries : !scratch) return GDN2_ERR_NULL_POINTER;
   int st = check_shape(batch, time, heads);
   if (st != GDN2_OK) return st;
   // whole chunks only, or rounded up over a partial last chunk (its missing tokens are identity steps)

@@ -30,8 +30,8 @@
 //   workspace  D, a 256-byte status block, and for a training call what backward consumes:
 //              Rn, Q, Kn, Yt, At, Tt
 //   scratch    dead when the call returns: the forward tiles of an inference call (Q, Kn, Yt, At, Tt in
-//              144 KiB per unit; a training call has them in its workspace and leaves its forward
-//              scratch alone); backward dZ
+//              144 KiB per unit; a training call has them in its workspace and no forward scratch);
+//              backward dZ
 #pragma once
 
 #include <cuda.h>
@@ -50,8 +50,8 @@ constexpr int64_t kBlobRn = 32768, kBlobDZ = 8 * 4608;
 constexpr int64_t kStatusBytes = 256;  // word 0: status
 constexpr int kQueueWord = 16;         // joint launch: next unit to prepare
 constexpr float kLog2e = 1.4426950408889634f;  // log-decays are summed in units of ln 2
-// forward scratch per unit, a size callers know: 144 KiB for an inference call (its tiles take 128 of
-// them), 32 KiB for a training call
+// forward scratch per unit, sizes callers know: 144 KiB for an inference call (its tiles take 128 of
+// them), 32 KiB reserved for a training call (NULL will do)
 constexpr int64_t kFwdScratchInference = 147456, kFwdScratchTraining = 32768;
 
 // workspace: what a training forward leaves for backward (inference: D and the status block only)

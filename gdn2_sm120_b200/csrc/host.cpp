@@ -14,7 +14,6 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/python_variable.h>
 
-#include <algorithm>
 #include <cmath>
 #include <cstring>
 
@@ -319,8 +318,7 @@ PyObject* train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     ws_bytes = api.chunk_workspace_bytes(s.batch, full, s.heads, 1);
     const int64_t states = s.batch * (full / kChunk + 1) * s.heads * kStateBytes;
     // one wave: what backward needs for all batch rows fits the budget
-    const int64_t wave = std::max(api.chunk_scratch_bytes(s.batch, full, s.heads, 2),
-                                  api.chunk_scratch_bytes(s.batch, full, s.heads, 1) + states);
+    const int64_t wave = api.chunk_scratch_bytes(s.batch, full, s.heads, 1) + states;
     if (ws_bytes <= 0 || (wave > budget && s.batch > 1) || ws_bytes + states + wave >= kCheckedBytes) return none();
   }
   at::Tensor out, fin, boundaries, workspace;
@@ -334,10 +332,9 @@ PyObject* train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   void* stream = at::cuda::getCurrentCUDAStream().stream();
   if (chunked) {
     workspace = bytes(ws_bytes, q);
-    // (the forward scratch of a training call is reserved, nothing is written there)
     status = api.chunk_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init), out.data_ptr(),
-                               fptr(&fin), fptr(&boundaries), workspace.data_ptr(), workspace.data_ptr(), s.batch,
-                               s.time, s.heads, full, 1, s.dtype, s.g_dtype, scale, stream);
+                               fptr(&fin), fptr(&boundaries), workspace.data_ptr(), nullptr, s.batch, s.time, s.heads,
+                               full, 1, s.dtype, s.g_dtype, scale, stream);
   } else {
     status = api.token_forward(s.ptr(0), s.ptr(1), s.ptr(2), s.ptr(3), s.ptr(4), s.ptr(5), fptr(init), out.data_ptr(),
                                fptr(&fin), fptr(&boundaries), s.batch, s.time, s.heads, 0, s.time, s.dtype, s.g_dtype,

@@ -106,7 +106,7 @@ extern "C" int gdn2_packed_forward(const void* q, const void* k, const void* v, 
   }
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
   if (t.chunks.n > 0) {
-    if (workspace == nullptr || scratch == nullptr || (training && chunk_boundaries == nullptr)) {
+    if (workspace == nullptr || (training ? chunk_boundaries == nullptr : scratch == nullptr)) {
       return GDN2_ERR_NULL_POINTER;
     }
     st = launch_packed_chunk_forward(t.chunks, q, k, v, g, beta, w, initial_state, out, final_state,

@@ -121,10 +121,11 @@ def _packed_forward(seq, state, bounds, scale: float, training: bool, prologue: 
         workspace = scratch = chunk_states = span_states = None
         if tokens:
             size = chunk_kernels.workspace_bytes(1, tokens, heads, training)
-            scratch_size = chunk_kernels.scratch_bytes(1, tokens, heads, False, training=training)
+            scratch_size = 0 if training else chunk_kernels.scratch_bytes(1, tokens, heads, False)
             slots = group.chunk_slots if training else 0
             chunk_kernels.check_memory(size + scratch_size + slots * heads * _DIM * _DIM * 4, device, "packed forward")
-            workspace, scratch = _bytes(size, device), _bytes(scratch_size, device)
+            workspace = _bytes(size, device)
+            scratch = None if training else _bytes(scratch_size, device)
         if training:
             chunk_states = _states(group.chunk_slots, heads, device)
             span_states = _states(group.span_slots, heads, device)

@@ -165,7 +165,7 @@ int gdn2_token_chunk_vjp(const void* q, const void* k, const void* v, const void
  *   scratch    gdn2_chunk_scratch_bytes(batch, full_tokens, heads, kind).  Tiles that only live
  *              inside one call.  kind 0: forward of an inference call (the WY tiles; 144 KiB per
  *              chunk-head); kind 2: forward of a training call (32 KiB per chunk-head, reserved: its
- *              tiles are in the workspace); kind 1: backward (dZ, 36 KiB per chunk-head).
+ *              tiles are in the workspace, NULL is accepted); kind 1: backward (dZ, 36 KiB per chunk-head).
  *              Dead when the call's kernels have run, so one scratch buffer serves every call on a
  *              stream; a large batch can be processed as several calls over batch slices that share it.
  * The kernels address tiles, sequence tensors and state checkpoints through tensor maps, which the
@@ -188,7 +188,7 @@ int64_t gdn2_chunk_scratch_bytes(int64_t batch, int64_t full_tokens, int64_t hea
  *   final_state    fp32 state after token full_tokens-1 (may alias initial_state exactly); or NULL
  *   chunk_boundaries  NULL, or fp32 [B, full_tokens/64 + 1, H,128,128]: state before every
  *                  chunk and after the last one (the activation checkpoints of backward)
- *   workspace, scratch  see above (forward scratch: kind 2 when `training`, else kind 0)
+ *   workspace, scratch  see above (forward scratch: kind 0, or NULL when `training`)
  *   training       non-zero: workspace was sized with training = 1, chunk_boundaries is
  *                  required, and everything backward needs is saved
  * All sequence pointers, states, the workspace and the scratch must be 16-byte aligned.

@@ -231,6 +231,16 @@ def test_entry_points_reject_bad_arguments_without_a_gpu():
     assert handle.gdn2_token_forward(*bad_state, 1, 4, 1, 0, 4, 0, 2, 1.0, null) == -5
 
 
+def test_chunk_forward_needs_a_scratch_for_inference_and_checkpoints_for_training():
+    one = ctypes.c_void_p(256)
+    seq_and_states = [one] * 6 + [None, one, None]
+    for boundaries, scratch, training in ((None, None, 0), (one, None, 0), (None, None, 1), (None, one, 1)):
+        assert _lib.lib().gdn2_chunk_forward(*seq_and_states, boundaries, one, scratch, 1, 64, 1, 64, training, 0, 2,
+                                             1.0, None) == -1
+    # with checkpoints a training call needs no scratch: what is refused here is the range
+    assert _lib.lib().gdn2_chunk_forward(*seq_and_states, one, one, None, 1, 64, 1, 65, 1, 0, 2, 1.0, None) == -4
+
+
 def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_handle", None)
     monkeypatch.setenv("GDN2_B200_LIB", str(tmp_path / "nope.so"))
