@@ -48,6 +48,7 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_chunk_forward": [_P] * 12 + [_I64] * 4 + [_INT, _INT, _INT, _F32, _P],
     "gdn2_chunk_backward": [_P] * 19 + [_I64] * 4 + [_INT, _INT, _F32, _P],
     "gdn2_chunk_backward_f32grads": [_P] * 19 + [_I64] * 4 + [_F32, _P],
+    "gdn2_chunk_forward_kernels": [],
     "gdn2_chunk_read_status": [_P] + [_I64] * 3 + [_P],
     "gdn2_debug_wait_expires": [_P] + [_I64] * 4 + [_P],
     "gdn2_token_forward_fused": [_P] * 9 + [_I64] * 5 + [_INT, _INT, _F32, _INT, _P],
@@ -167,17 +168,19 @@ LAUNCHES = [0]
 KERNEL_EVENTS: dict[str, list] | None = None
 
 
-# kernels launched by one successful call of each entry point (default 1); a chunk forward of few heads, which
-# runs its two kernels as one launch, still counts as two
-_KERNELS_PER_CALL = {"gdn2_chunk_forward": 2, "gdn2_chunk_forward_fused": 2, "gdn2_chunk_backward": 2, "gdn2_chunk_backward_f32grads": 2,
-                     "gdn2_chunk_forward_static": 2}
+# kernels launched by one successful call of each entry point (default 1); a chunk forward says it itself
+_KERNELS_PER_CALL = {"gdn2_chunk_backward": 2, "gdn2_chunk_backward_f32grads": 2}
+_CHUNK_FORWARDS = ("gdn2_chunk_forward", "gdn2_chunk_forward_fused", "gdn2_chunk_forward_static")
 
 
 def check(status: int, what: str, kernels: int | None = None) -> None:
     """Turn a negative gdn2_status into a RuntimeError; count successful launches."""
 
     if status == 0:
-        LAUNCHES[0] += _KERNELS_PER_CALL.get(what, 1) if kernels is None else kernels
+        if kernels is None:
+            kernels = (lib().gdn2_chunk_forward_kernels() if what in _CHUNK_FORWARDS
+                       else _KERNELS_PER_CALL.get(what, 1))
+        LAUNCHES[0] += kernels
         return
     handle = lib()
     text = handle.gdn2_status_string(status).decode()

@@ -1293,6 +1293,8 @@ struct ForwardCall {
   int prologue;
 };
 
+thread_local int t_forward_kernels = 0;  // of this thread's latest chunk forward
+
 // One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation) and 2-3 us per chunk
 // (the scans); together the longer of the two, the first units taking some 35 us and a scan 0.4 us per chunk
 // more beside preparers.  Beyond a quarter of the SMs scanning, the preparation falls behind.
@@ -1314,6 +1316,10 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
     return cudaFuncGetAttributes(&attr, kernel) == cudaSuccess ? attr.numRegs : -1;
   }();
   if (regs != kJointRegs) return GDN2_ERR_UNSUPPORTED;  // (the caller then takes two launches)
+  // the marks of finished units are in D, right before the status block: one fill clears both
+  const WsLayout ws{pp.n_ch, pp.training != 0};
+  err = cudaMemsetAsync(pp.ws + ws.off_d(), 0, size_t(pp.n_ch) * kBlobD + kStatusBytes, stream);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int n_scan = seqs.count() * sp.H;
   // clusters of two CTAs; no more preparers than pairs of units
   const int64_t want = n_scan + (pp.n_ch + 3) / 4;
@@ -1375,15 +1381,15 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   cudaError_t err;
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     if (prefer_joint(n_scan, n_ch, seqs.n_chunks, sm_count)) {
-      // the marks of finished units are in D, right before the status block: one fill clears both
-      err = cudaMemsetAsync(a.workspace + ws.off_d(), 0, size_t(n_ch) * kBlobD + kStatusBytes, stream);
-      if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
       int st = GDN2_OK;
       GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
         st = a.prologue != 0 ? launch_joint<T, G, Seqs, true>(pp, sp, seqs, tm_prep, tm, sm_count, stream)
                              : launch_joint<T, G, Seqs, false>(pp, sp, seqs, tm_prep, tm, sm_count, stream);
       });
-      if (st != GDN2_ERR_UNSUPPORTED) return st;
+      if (st != GDN2_ERR_UNSUPPORTED) {
+        t_forward_kernels = 1;
+        return st;
+      }
     }
   }
   err = cudaMemsetAsync(status, 0, kStatusBytes, stream);
@@ -1410,10 +1416,13 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   kernel<<<grid, kScanThreads, smem, stream>>>(sp, seqs, tm);
   st = check_launch();
   profile_mark(2, stream);
+  t_forward_kernels = 2;
   return st;
 }
 
 }  // namespace
+
+int chunk_forward_kernels() { return t_forward_kernels; }
 
 int launch_chunk_forward(const void* q, const void* k, const void* v, const void* g, const void* beta,
                          const void* w, const float* s_in, void* out, float* s_out, float* bnd,

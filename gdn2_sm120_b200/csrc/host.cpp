@@ -30,6 +30,7 @@ struct Api {
   decltype(&gdn2_token_chunk_vjp) token_chunk_vjp;
   decltype(&gdn2_chunk_forward) chunk_forward;
   decltype(&gdn2_chunk_forward_fused) chunk_forward_fused;
+  decltype(&gdn2_chunk_forward_kernels) chunk_forward_kernels;
   decltype(&gdn2_chunk_backward) chunk_backward;
   decltype(&gdn2_chunk_workspace_bytes) chunk_workspace_bytes;
   decltype(&gdn2_chunk_scratch_bytes) chunk_scratch_bytes;
@@ -286,7 +287,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                           s.dtype, s.g_dtype, scale, stream);
   }
   others.end();
-  if (!ok(status, name, chunked ? 2 : 1)) return nullptr;
+  if (!ok(status, name, chunked ? api.chunk_forward_kernels() : 1)) return nullptr;
   PyObject* first = out_given ? Py_NewRef(a[8]) : wrap(out);
   PyObject* second = inplace ? Py_NewRef(a[6]) : fin_given ? Py_NewRef(a[9]) : wrap(fin);
   PyObject* result = PyTuple_New(2);
@@ -341,7 +342,9 @@ PyObject* train_forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
                                scale, stream);
   }
   others.end();
-  if (!ok(status, chunked ? "gdn2_chunk_forward" : "gdn2_token_forward", chunked ? 2 : 1)) return nullptr;
+  if (!ok(status, chunked ? "gdn2_chunk_forward" : "gdn2_token_forward", chunked ? api.chunk_forward_kernels() : 1)) {
+    return nullptr;
+  }
   PyObject* result = PyTuple_New(4);
   PyTuple_SET_ITEM(result, 0, wrap(out));
   PyTuple_SET_ITEM(result, 1, wrap(fin));
@@ -538,6 +541,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   GDN2_BIND(token_chunk_vjp);
   GDN2_BIND(chunk_forward);
   GDN2_BIND(chunk_forward_fused);
+  GDN2_BIND(chunk_forward_kernels);
   GDN2_BIND(chunk_backward);
   GDN2_BIND(chunk_workspace_bytes);
   GDN2_BIND(chunk_scratch_bytes);

@@ -203,6 +203,12 @@ int gdn2_chunk_forward(const void* q, const void* k, const void* v, const void* 
                        void* stream);
 
 /*
+ * Kernels that the calling thread's latest chunk forward launched (0: it has made none): 2, the preparation of the
+ * chunks and the scan, or 1 where few sequences and heads let one launch do both side by side.
+ */
+int gdn2_chunk_forward_kernels(void);
+
+/*
  * Chunkwise backward over tokens [0, full_tokens): reverse scan of the state cotangent plus
  * the compact-WY chunk VJP, from what gdn2_chunk_forward(training = 1) saved.  Replaces
  * wy_boundary_dstate and compact_wy_chunk_vjp_cute with their kernels

@@ -21,11 +21,12 @@ DEV = "cuda"
 
 # (at most SMs / 4 sequences x heads, and enough chunks: the smallest that qualify at 37, 32 and 16 heads, one
 # chunk less, and ragged ends of 1 and 63 tokens)
-@pytest.mark.parametrize("batch,heads,time", [(1, 37, 21 * 64), (2, 16, 26 * 64), (2, 16, 25 * 64), (2, 16, 26 * 64 + 1),
-                                              (1, 16, 70 * 64 + 63)])
-def test_joint_launch_equals_a_unit_alone_and_the_oracle(batch, heads, time):
+@pytest.mark.parametrize("batch,heads,time,kernels", [(1, 37, 21 * 64, 1), (2, 16, 26 * 64, 1), (2, 16, 25 * 64, 2),
+                                                      (2, 16, 26 * 64 + 1, 1), (1, 16, 70 * 64 + 63, 1)])
+def test_joint_launch_equals_a_unit_alone_and_the_oracle(batch, heads, time, kernels):
     tensors, d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
     full = _step(tensors, d_out, d_fin)
+    assert _lib.lib().gdn2_chunk_forward_kernels() == kernels
     _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
 
 
@@ -36,10 +37,13 @@ def test_joint_launch_equals_two_launches(dtype, g_dtype, raw):
     q, k, v, g, beta, w = [t.to(g_dtype if i == 3 else dtype) for i, t in enumerate(tensors[:6])]
     flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
     with torch.no_grad():
+        launched = _lib.LAUNCHES[0]
         joint = chunk_gdn2(q, k, v, g, beta, w, tensors[6], output_final_state=True, **flags)
+        assert _lib.lib().gdn2_chunk_forward_kernels() == _lib.LAUNCHES[0] - launched == 1
         _lib.profile_enable(True)  # times the kernels one by one: never joint
         try:
             apart = chunk_gdn2(q, k, v, g, beta, w, tensors[6], output_final_state=True, **flags)
+            assert _lib.lib().gdn2_chunk_forward_kernels() == 2
         finally:
             _lib.profile_enable(False)
     assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
@@ -143,6 +147,7 @@ def test_joint_launch_replays_from_a_cuda_graph():
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
             got = chunk_gdn2(*tensors, output_final_state=True)
+        assert _lib.lib().gdn2_chunk_forward_kernels() == 1
         for _ in range(2):
             got[0].zero_()
             graph.replay()
