@@ -11,7 +11,17 @@
 namespace gdn2 {
 
 constexpr int kChunk = GDN2_CHUNK;  // 64
-constexpr int kStepTokens = 8;      // forward calls of sequences up to this long go token by token
+// Forward calls of sequences up to this long go token by token, longer ones in spans of 16 tokens.  The line is one
+// for all grids, so that a sequence gives the same bits alone and in a batch.  us, steps / spans, for sequences x
+// heads of 16, 64, 96, 128, 512, 1024 (at 64 and 128 the spans fill the SMs once and twice):
+//   8 tokens            6.5/7.5   8.4/7.8  10.0/11.3  11.9/11.3  33.8/37.9  75.1/83.6
+//   9 tokens            7.1/8.4   9.1/8.6  11.1/12.7  13.2/12.7  38.2/42.6  82.4/91.8
+//   10 tokens           7.6/8.4   9.9/8.6  11.9/12.7  14.2/12.8  41.1/42.8  88.9/91.8
+//   raw inputs, 7       7.3/8.2   9.3/8.4  11.1/12.0  13.2/12.1  39.5/39.8  80.7/83.4
+//   raw inputs, 8       7.9/8.3  10.1/8.5  12.1/12.1  14.4/12.2  43.5/40.1  88.3/83.9
+//   raw inputs, 9       8.9/9.1  11.2/9.3  13.6/13.5  16.0/13.5  48.9/45.1  99.5/92.8
+constexpr int kStepTokens = 9, kStepTokensRaw = 8;
+inline int step_tokens(int prologue) { return prologue != 0 ? kStepTokensRaw : kStepTokens; }
 
 struct SeqInfo {
   int64_t row0;   // first token row

@@ -1,7 +1,7 @@
 // Token-path kernels for one token or a few: exact fp32 recurrence.
 //
 //   token_step_kernel         one decode step of few heads (or of states that are not 16-byte aligned), and
-//                             sequences of up to 8 tokens
+//                             sequences of up to 9 tokens
 //   token_decode_ring_kernel  one decode step of many heads, persistent
 //   token_t1_zero_kernel      T == 1, zero initial state closed form (write-only state)
 //
@@ -460,7 +460,7 @@ __global__ void __launch_bounds__(kTokThreads) token_t1_zero_kernel(const T1Zero
 
 inline bool grid_fits(int64_t blocks) { return blocks > 0 && blocks <= int64_t(0x7fffffff); }
 
-// `most`: 1 (T == 1 without checkpoints), 4 or 8, the most tokens a sequence has
+// `most`: 1 (T == 1 without checkpoints), 4 or kStepTokens, the most tokens a sequence has
 template <typename Seqs>
 int launch_steps(const TokenStepParams& p, const Seqs& seqs, int64_t blocks, int most, int dtype, int g_dtype,
                  cudaStream_t stream) {
@@ -508,10 +508,10 @@ int launch_token_forward(const void* q, const void* k, const void* v, const void
     });
     return check_launch();
   }
-  // Token by token up to 8 tokens: the spans of token_span.cu cost nearly as much for one token as for 16
-  // (B32 H32, 2 tokens: 73 us there, 32 here; 8 tokens: 87 there, 77 here).
+  // A few tokens one by one (step_tokens says how many): the spans of token_span.cu cost nearly as much for one
+  // token as for 16 (B32 H32, 2 tokens: 73 us there, 32 here).
   const int64_t tokens = t_end - t_begin;
-  if (tokens >= 1 && tokens <= kStepTokens) {
+  if (tokens >= 1 && tokens <= step_tokens(prologue)) {
     const TokenStepParams p{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), 0, scale, prologue};
     const int most = T == 1 && bnd == nullptr ? 1 : tokens <= 4 ? 4 : kStepTokens;
     return launch_steps(p, UniformSeqs{t_begin, T, int(tokens), 1, int(B)}, blocks, most, dtype, g_dtype, stream);
@@ -520,7 +520,7 @@ int launch_token_forward(const void* q, const void* k, const void* v, const void
                              scale, prologue, stream);
 }
 
-// the sequences from `first` on, none of more than kStepTokens tokens
+// the sequences from `first` on, none of more than step_tokens(prologue) tokens
 int launch_packed_steps(const PackedSpans& table, int first, const void* q, const void* k, const void* v, const void* g,
                         const void* beta, const void* w, const float* s_in, void* out, float* s_out, float* bnd,
                         int64_t H, int dtype, int g_dtype, float scale, int prologue, cudaStream_t stream) {

@@ -1050,7 +1050,7 @@ int launch_packed_token_forward(const PackedSpans& table, const void* q, const v
                                 cudaStream_t stream) {
   // longest first: the sequences of a few tokens are the end of the list
   int spans = 0;
-  while (spans < table.n && table.e[spans].len > kStepTokens) ++spans;
+  while (spans < table.n && table.e[spans].len > step_tokens(prologue)) ++spans;
   if (spans > 0) {
     PackedSpans longer = table;
     longer.n = spans;

@@ -96,11 +96,11 @@ def _bytes(size: int, device):
     return torch.empty(size, device=device, dtype=torch.uint8)
 
 
-def _short_kernels(bounds) -> int:
-    """Forward launches for the sequences shorter than a chunk: up to 8 tokens go token by token."""
+def _short_kernels(bounds, prologue: int) -> int:
+    """Forward launches for the sequences shorter than a chunk: up to 9 tokens (raw inputs: 8) go token by token."""
 
-    lengths = [b - a for a, b in zip(bounds, bounds[1:])]
-    return any(8 < n < 64 for n in lengths) + any(n <= 8 for n in lengths)
+    lengths, steps = [b - a for a, b in zip(bounds, bounds[1:])], 8 if prologue else 9
+    return any(steps < n < 64 for n in lengths) + any(n <= steps for n in lengths)
 
 
 def _packed_forward(seq, state, bounds, scale: float, training: bool, prologue: int = 0):
@@ -135,7 +135,7 @@ def _packed_forward(seq, state, bounds, scale: float, training: bool, prologue: 
                   _lib.ptr(chunk_states), _lib.ptr(span_states), _lib.ptr(workspace), _lib.ptr(scratch), group.bounds,
                   group.last - group.first, total, heads, int(training), _lib.dtype_code(q.dtype),
                   _lib.dtype_code(seq[3].dtype), scale, prologue, _lib.stream_ptr(device),
-                  kernels=2 * (group.chunks > 0) + _short_kernels(group.bounds))
+                  kernels=2 * (group.chunks > 0) + _short_kernels(group.bounds, prologue))
         saved.append((workspace, chunk_states, span_states))
     return output, final_state, groups, saved
 

@@ -115,9 +115,9 @@ def test_token_spans_at_the_grid_where_the_form_changes(batch, heads, time):
     _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
 
 
-# token by token up to 8 tokens (inputs of 4 read at once), spans from 9 on; the prologue's rows as well
+# token by token up to 9 tokens (inputs of 4 read at once; raw inputs up to 8), spans from there on
 @pytest.mark.parametrize("raw", [False, True])
-@pytest.mark.parametrize("time", [2, 4, 5, 8, 9])
+@pytest.mark.parametrize("time", [2, 4, 5, 8, 9, 10])
 def test_few_tokens_with_and_without_the_prologue(time, raw):
     make = oracle.make_raw_inputs if raw else oracle.make_inputs
     cpu = make(3, time, 2, seed=time)
@@ -153,3 +153,20 @@ def test_joint_launch_replays_from_a_cuda_graph():
             graph.replay()
             torch.cuda.synchronize()
             assert torch.equal(got[0], expected[0]) and torch.equal(got[1], expected[1])
+
+
+# the longest sequences that go token by token and one token more: alone, in a grid and packed, the same bits
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("time", [8, 9, 10])
+def test_a_few_tokens_alone_in_a_batch_and_packed(time, raw):
+    tensors, _, _ = _device_inputs(24, time, 4, seed=time)
+    flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
+    with torch.no_grad():
+        out, fin = chunk_gdn2(*tensors, output_final_state=True, **flags)
+        alone = chunk_gdn2(*[t[3:4] for t in tensors], output_final_state=True, **flags)
+        rows = [t.reshape(1, 24 * time, 4, 128) for t in tensors[:6]]
+        launched = _lib.LAUNCHES[0]
+        packed = chunk_gdn2_varlen(*rows, [time * i for i in range(25)], tensors[6], output_final_state=True, **flags)
+    assert _lib.LAUNCHES[0] == launched + 1
+    assert torch.equal(alone[0], out[3:4]) and torch.equal(alone[1], fin[3:4])
+    assert torch.equal(packed[0].view_as(out), out) and torch.equal(packed[1], fin)
