@@ -170,3 +170,23 @@ def test_a_few_tokens_alone_in_a_batch_and_packed(time, raw):
     assert _lib.LAUNCHES[0] == launched + 1
     assert torch.equal(alone[0], out[3:4]) and torch.equal(alone[1], fin[3:4])
     assert torch.equal(packed[0].view_as(out), out) and torch.equal(packed[1], fin)
+
+
+# whole chunks only (short sequences beside them do not count), and one sequence that ends in a partial chunk
+@pytest.mark.parametrize("lengths", [(64, 192, 128, 640), (128, 40, 64, 0, 256), (64, 192, 129)])
+def test_packed_gradients_with_and_without_a_partial_chunk(lengths):
+    heads, total = 3, sum(lengths)
+    tensors, d_out, _ = _device_inputs(1, total, heads, seed=total)
+    states = 0.02 * torch.randn(len(lengths), heads, 128, 128, device=DEV)
+    d_fin = 0.01 * torch.randn_like(states)
+    leaves = [t.requires_grad_(True) for t in (*tensors[:6], states)]
+    cu = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    out, fin = chunk_gdn2_varlen(*leaves[:6], cu, leaves[6], output_final_state=True)
+    grads = torch.autograd.grad((out.float() * d_out.float()).sum() + (fin * d_fin).sum(), leaves)
+    for i, (lo, hi) in enumerate(zip(cu, cu[1:])):
+        if lo < hi:
+            single = [t[:, lo:hi].detach() for t in leaves[:6]] + [states[i:i + 1].detach()]
+            o, f, gr = _step(single, d_out[:, lo:hi], d_fin[i:i + 1])
+            assert torch.equal(o, out[:, lo:hi]) and torch.equal(f, fin[i:i + 1])
+            assert all(torch.equal(a, b[:, lo:hi]) for a, b in zip(gr[:6], grads[:6]))
+            assert torch.equal(gr[6], grads[6][i:i + 1])
