@@ -371,6 +371,7 @@ def _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, b, h, full):
     cpu = [t.cpu() for t in sub]
     ref_out, ref_state, ref = oracle.recurrence_grads(*cpu, sub_do.cpu(), sub_df.cpu())
     torch.testing.assert_close(out_s.float().cpu(), ref_out.float(), rtol=2e-2, atol=1e-2)
+    check_gradient("out", out_s, ref_out)  # (relative: the outputs are of the order of atol above)
     assert oracle.rel_l2(fin_s, ref_state) < FP32_REL
     for name, got, want in zip(("dq", "dk", "dv", "dg", "dbeta", "dw", "dS0"), grads_s, ref):
         check_gradient(name, got, want)

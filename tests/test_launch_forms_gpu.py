@@ -1,7 +1,7 @@
 """GPU tests of what a dispatch rule chooses between: the joint launch of prep and scan, packed batches that
 take several launches, the token spans' loads of unaligned tensors, and calls from threads that have made no
 CUDA call yet.  The forms run the same arithmetic in the same order, so results are compared bit for bit; one
-unit of each joint case is held against the oracle with the tolerances of test_autograd_gpu.py."""
+unit of each case is held against the oracle with the tolerances of test_autograd_gpu.py."""
 
 from __future__ import annotations
 
@@ -131,8 +131,11 @@ def test_few_tokens_with_and_without_the_prologue(time, raw):
         norm = lambda x: x * torch.rsqrt((x * x).sum(-1, keepdim=True) + 1e-6)  # noqa: E731
         plain = (norm(q), norm(k), v, -torch.nn.functional.softplus(g), torch.sigmoid(beta), torch.sigmoid(w))
     ref_out, ref_state = oracle.recurrence(*plain, state)
-    torch.testing.assert_close(out.float().cpu(), ref_out.float(), rtol=2e-2, atol=1e-2)
-    assert oracle.rel_l2(fin, ref_state) < 1e-3
+    # exact fp32, one rounding to bf16 of at most 2^-9 = 1.95e-3 of a value: each token by itself, so that a wrong row
+    # cannot hide among the others
+    for t in range(time):
+        assert oracle.rel_l2(out[:, t], ref_out[:, t]) < 2.2e-3, t
+    assert oracle.rel_l2(fin, ref_state) < 1e-5
 
 
 def test_joint_launch_replays_from_a_cuda_graph():
