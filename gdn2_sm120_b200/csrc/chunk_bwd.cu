@@ -407,8 +407,8 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
 // =============================================================================================
 // chunk VJP
 // =============================================================================================
-// 512 threads.  Elementwise phases: warp = 4-token group tg, lane = 4-channel group c4 (as in the
-// forward prep kernel).  TMEM phases: warp & 3 = lane quadrant, warp >> 2 = share of the columns.
+// 512 threads.  Elementwise phases: warp = 4-token group tg, lane = 4-channel group c4.  TMEM phases:
+// warp & 3 = lane quadrant, warp >> 2 = share of the columns.
 // Final chain: thread = (key channel, 16-token block).
 constexpr int kVjpThreads = 512;
 constexpr int kCsN = 144;              // natural 128-column tiles: padded chunk stride
@@ -466,8 +466,6 @@ __device__ __forceinline__ uint32_t d6_col(int I) { return (I == 3) ? 0u : (I ==
 struct VjpParams {
   const void *q, *k, *v, *g, *beta, *w, *d_out;
   const uint8_t* sc;    // scratch: dZ written by the reverse scan
-  const float* bnd;     // [B, n_chunks+1, H,128,128] forward states
-  const float* d_bnd;   // same shape, cotangents
   void *dq, *dk, *dv, *dg, *dbeta, *dw;
   int* status;
   int64_t n_ch;
@@ -480,24 +478,8 @@ struct VjpInputMaps {
 };
 
 template <typename T>
-__device__ __forceinline__ void load4v(const void* base, int64_t idx, float (&out)[4]);
-template <>
-__device__ __forceinline__ void load4v<__nv_bfloat16>(const void* base, int64_t idx, float (&out)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __nv_bfloat16*>(base) + idx);
-  out[0] = __uint_as_float(raw.x << 16); out[1] = __uint_as_float(raw.x & 0xffff0000u);
-  out[2] = __uint_as_float(raw.y << 16); out[3] = __uint_as_float(raw.y & 0xffff0000u);
-}
-template <>
-__device__ __forceinline__ void load4v<__half>(const void* base, int64_t idx, float (&out)[4]) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(static_cast<const __half*>(base) + idx);
-  const __half2* h = reinterpret_cast<const __half2*>(&raw);
-  const float2 a = __half22float2(h[0]), b = __half22float2(h[1]);
-  out[0] = a.x; out[1] = a.y; out[2] = b.x; out[3] = b.y;
-}
-template <>
-__device__ __forceinline__ void load4v<float>(const void* base, int64_t idx, float (&out)[4]) {
-  const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx);
-  out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
+__device__ __forceinline__ void load4v(const void* base, int64_t idx, float (&out)[4]) {
+  unpack4<T>(load4_raw<T>(base, idx), out);
 }
 
 template <typename T>
@@ -1248,7 +1230,7 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
       !encode_sequence_map(&m.in.d_out, a.d_out, a.rows, a.H, a.dtype)) {
     return GDN2_ERR_LAUNCH;
   }
-  const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.bnd, a.d_bnd, a.dq, a.dk, a.dv, a.dg,
+  const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.dq, a.dk, a.dv, a.dg,
                      a.dbeta, a.dw, status, n_ch, int(a.H), a.scale};
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     if (a.grads_f32) {

@@ -149,38 +149,6 @@ __device__ __forceinline__ bool marked(const float* p) {
   return (x >> 31) != 0;
 }
 
-// load 8 consecutive sequence elements (16-bit type: one 16-byte load; fp32: two)
-template <typename T>
-__device__ __forceinline__ void load8(const void* base, int64_t idx, float (&out)[8]);
-template <>
-__device__ __forceinline__ void load8<__nv_bfloat16>(const void* base, int64_t idx, float (&out)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(base) + idx);
-  const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    out[2 * i] = __uint_as_float(wv[i] << 16);
-    out[2 * i + 1] = __uint_as_float(wv[i] & 0xffff0000u);
-  }
-}
-template <>
-__device__ __forceinline__ void load8<__half>(const void* base, int64_t idx, float (&out)[8]) {
-  const uint4 raw = *reinterpret_cast<const uint4*>(static_cast<const __half*>(base) + idx);
-  const __half2* h = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 f = __half22float2(h[i]);
-    out[2 * i] = f.x;
-    out[2 * i + 1] = f.y;
-  }
-}
-template <>
-__device__ __forceinline__ void load8<float>(const void* base, int64_t idx, float (&out)[8]) {
-  const float4 a = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx);
-  const float4 b = *reinterpret_cast<const float4*>(static_cast<const float*>(base) + idx + 4);
-  out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w;
-  out[4] = b.x; out[5] = b.y; out[6] = b.z; out[7] = b.w;
-}
-
 // ---- tensor maps (host) -------------------------------------------------------------------------
 // cuTensorMapEncodeTiled through the runtime's driver entry point query: the library does not link
 // against the driver API for this one call.

@@ -1,22 +1,24 @@
-// Tensor-core chunk forward (64-token chunks, compact-WY form), two kernels:
+// Tensor-core chunk forward (64-token chunks, compact-WY form), two kernels or one that does the work of both:
 //
-//   chunk_prep_kernel   persistent, one CTA per SM walking over the (batch, chunk, head) units, all
+//   chunk_prep_kernel   persistent, two CTAs per SM walking over the (sequence, chunk, head) units, all
 //                       chunks independent.  The raw inputs of the next unit arrive by tiled TMA
 //                       loads under the tail of the current one (a CTA that starts a unit with
 //                       per-thread loads spends a quarter of its time issuing them: the load/store
 //                       unit's queue, not HBM, is the limit).  Builds the WY factors of the chunk
 //                       and writes them as row-major tiles:
 //                       cumulative log-decay, block-anchored Gram products on tf32 tcgen05 MMAs,
-//                       blocked inverse of the unit lower-triangular system on CUDA cores (fp32),
-//                       Y = T E and U^T = Z^T T^T on tf32 tcgen05 MMAs.
-//   chunk_scan_kernel   one CTA per (batch, head), chunks in order.  The state lives transposed
+//                       blocked inverse T of the unit lower-triangular system on CUDA cores (fp32),
+//                       Y = T E on tf32 tcgen05 MMAs.
+//   chunk_scan_kernel   one CTA per (sequence, head), chunks in order.  The state lives transposed
 //                       (S^T: value rows x key columns) in TMEM as the fp32 accumulator and is fed
 //                       back as the tf32 A operand of the next MMAs without leaving TMEM:
-//                           R^T  = U^T - S^T Y^T
+//                           R^T  = Z^T T^T - S^T Y^T           (Z = w v)
 //                           O^T  = S^T Qg^T + R^T Aqk^T
 //                           S^T <- S^T diag(d) + R^T Kt
 //                       The B operands are the prep kernel's row-major tiles, brought in by tiled
 //                       TMA loads in the swizzled layout of their role (chunk_common.cuh).
+//   chunk_joint_kernel  where few sequences and heads leave most SMs without a scan: some CTAs scan
+//                       while the others prepare, chunk by chunk.
 //
 // Math per chunk (reference: src/gdn2_sm120/reference.py:149-172, chunk.py:188-331, with the
 // chunk length re-chosen as 64 and the decay normalisation anchored per 16-token block so that
@@ -24,7 +26,7 @@
 //   G_i = sum_{t<=i} g_t,  a_I = G at the start of block I = i / 16
 //   L[i][j]   = sum_k beta k_i exp(G_i - a_I) * k_j exp(a_I - G_j)      (j < i)
 //   Aqk[i][j] = sum_k scale q_i exp(G_i - a_I) * k_j exp(a_I - G_j)     (j <= i)
-//   T = (I + L)^-1,  Y = T (beta k exp(G)),  U = T (w v)
+//   T = (I + L)^-1,  Y = T (beta k exp(G)),  R = T (w v) - Y S
 //   Qg = scale q exp(G),  Kt = k exp(G_end - G),  d = exp(G_end)
 
 #include <type_traits>

@@ -102,14 +102,6 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const void* tmap, int c0, int
       "r"(c2), "r"(leader)
       : "memory");
 }
-__device__ __forceinline__ void tma_prefetch_l2_4d(const void* tmap, int c0, int c1, int c2, int c3,
-                                                   uint32_t leader = 1) {
-  asm volatile(
-      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
-      "@q cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n\t}" ::"l"(tmap), "r"(c0), "r"(c1),
-      "r"(c2), "r"(c3), "r"(leader)
-      : "memory");
-}
 // Tiled TMA loads global -> shared; completion (bytes) on an mbarrier.  `tmap` points at a
 // CUtensorMap in kernel-parameter space.  c0 must keep c0 * element size a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar,
@@ -302,9 +294,8 @@ __device__ __forceinline__ uint32_t blk_off(int r, int c, int rs, int cs) {
   return uint32_t((r >> 3) * rs + (c / CH) * cs + (r & 7) * 16 + (c % CH) * ES);
 }
 
-// 32-byte global store (sm_100: 256-bit vector access; the address must be 32-byte aligned).  Two
-// neighbouring 16-byte chunks of a blocked tile leave in one instruction, which halves the cache lines
-// a warp's store instructions touch in total.
+// 32-byte global store (sm_100: 256-bit vector access; the address must be 32-byte aligned): a whole sector
+// per lane where each lane writes a row of its own.
 __device__ __forceinline__ void store_global_32b(void* ptr, float4 lo, float4 hi) {
   asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(ptr), "f"(lo.x), "f"(lo.y), "f"(lo.z),
                "f"(lo.w), "f"(hi.x), "f"(hi.y), "f"(hi.z), "f"(hi.w)
