@@ -41,14 +41,20 @@ constexpr int64_t kStateElems = int64_t(kDim) * kDim;
 // =============================================================================================
 // Warp-specialised like the forward scan (chunk_fwd.cu), for the same reason: the MMAs of a chunk are issued
 // back to back by one warp, the rest runs beside them.
-//   warp 0       tiled TMA loads, each buffer refilled as soon as its MMA has read it
-//   warp 1       MMAs, per chunk:  dR^T += dS^T Kt^T | dS'^T += dO^T Qg | dS'^T -= dR^T Y | dZ^T = dR^T T |
+//   warp 16      tiled TMA loads, each buffer refilled as soon as its MMA has read it
+//   warp 18      MMAs, per chunk:  dR^T += dS^T Kt^T | dS'^T += dO^T Qg | dS'^T -= dR^T Y | dZ^T = dR^T T |
 //                dR'^T = dO'^T Aqk of the next chunk, the dependences between accumulators waited for
-//   warps 2..9   decay: dS' <- dS diag(d) into the other of two buffers; the cotangent checkpoints, staged
-//   warps 10..17 dO of the next chunk (the one before it in time) into tensor memory, dZ out (staged)
+//   warps 0..7   decay: dS' <- dS diag(d) into the other of two buffers; the cotangent checkpoints, staged
+//   warps 8..15  dO of the next chunk (the one before it in time) into tensor memory, dZ out (staged)
 // Tensor memory (columns): dS 2 x 128, dR 2 x 64, dZ 64, dO 64 = all 512.
-constexpr int kBScanThreads = 576;
-constexpr int kBScanDecay0 = 2, kBScanDo0 = 10;  // first warps of the groups
+// (With a half or a quarter of the value rows two or one warp of four has work; the loads and the MMAs then take the
+// places of others, see ScanWarps in chunk_fwd.cu.)
+template <int kParts>
+struct BScanWarps {
+  static constexpr int kDo0 = 8, kLoads = kParts > 1 ? 2 : 16, kMma = kParts > 1 ? 3 : 18;
+  static constexpr int kThreads = kParts > 1 ? 512 : 608;
+  static __device__ __forceinline__ bool works(int warp) { return warp < 16 && (warp & 3) < 4 / kParts; }
+};
 constexpr int kCsZ = 144, kRsZ = 32 * kCsZ;  // dZ tile: the padded strides of the VJP kernel's [dZ ; dO] stack
 
 struct BScanSmem {
@@ -87,15 +93,18 @@ struct BScanMaps {
   CUtensorMap at, tt, kn, q, yt, d_out;
 };
 
-template <typename T, typename Seqs>
-__global__ void __launch_bounds__(kBScanThreads, 1)
+template <typename T, typename Seqs, int kParts>
+__global__ void __launch_bounds__(BScanWarps<kParts>::kThreads, 1)
 chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   BScanSmem& sm = *reinterpret_cast<BScanSmem*>(smem_raw);
   BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
+  using W = BScanWarps<kParts>;
+  constexpr int kRows = kDim / kParts;  // value rows of this CTA: lanes 0 .. kRows - 1 of tensor memory
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int s = int(blockIdx.x) / p.H, h = int(blockIdx.x) - s * p.H;
+  const int unit = int(blockIdx.x) / kParts, v0 = (int(blockIdx.x) - unit * kParts) * kRows;
+  const int s = unit / p.H, h = unit - s * p.H;
   const SeqInfo sq = seqs.at(s);
   const int n_chunks = sq.n_chunks;
   constexpr uint32_t kColS = 0, kColR = 256, kColZ = 384, kColDo = 448;
@@ -103,7 +112,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
   auto chunk_of = [&](int it) { return n_chunks - 1 - it; };
   auto ch_of = [&](int it) { return int64_t(sq.chunk0 + chunk_of(it)) * p.H + h; };
 
-  if (warp == 1) {
+  if (warp == W::kMma) {
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
@@ -112,16 +121,16 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
                        &sm.z_done, &sm.do_done, &sm.s_done};
 #pragma unroll
     for (int i = 0; i < 10; ++i) mbar_init(one[i], 1);
-    mbar_init(&sm.go_a, 1 + 8);
-    mbar_init(&sm.go_q, 1 + 8);
-    mbar_init(&sm.go_z, 1 + 8);
-    mbar_init(&sm.do_read, 8);
+    mbar_init(&sm.go_a, 1 + 8 / kParts);
+    mbar_init(&sm.go_q, 1 + 8 / kParts);
+    mbar_init(&sm.go_z, 1 + 8 / kParts);
+    mbar_init(&sm.do_read, 8 / kParts);
     // a wait that ran out earlier (forward or backward) left garbage behind: results become NaN
     sm.failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
     fence_mbar_init();
   }
   // lines 32..63 of the first slab of At and Tt (j >= 32, i < 32) are never loaded: zero, once
-  for (int e = tid; e < 4096 / 16; e += kBScanThreads) {
+  for (int e = tid; e < 4096 / 16; e += W::kThreads) {
     reinterpret_cast<float4*>(sm.at + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
     reinterpret_cast<float4*>(sm.tt + 4096)[e] = make_float4(0.f, 0.f, 0.f, 0.f);
   }
@@ -137,12 +146,12 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
     if (lane == 0) mbar_arrive(bar);
   };
 
-  if (warp == 0) {
+  if (warp == W::kLoads) {
     // ---------------------------------------------------------------- loads
     const uint32_t leader = elect_leader();
     auto load_o = [&](int it) {
-      mbar_arrive_expect_tx(&sm.full_o, 16384u, leader);
-      tma_load_3d(sm.d_out, &tm.d_out, 0, h, int(sq.row0) + chunk_of(it) * kChunk, &sm.full_o, leader);
+      mbar_arrive_expect_tx(&sm.full_o, 16384u / kParts, leader);
+      tma_load_3d(sm.d_out, &tm.d_out, v0, h, int(sq.row0) + chunk_of(it) * kChunk, &sm.full_o, leader);
     };
     // At and Tt are zero for j >= 32, i < 32: three 32-row boxes each, the fourth quadrant stays zero
     auto load_tri = [&](uint8_t* dst, const CUtensorMap* map, int it, uint64_t* bar) {
@@ -184,10 +193,10 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       waiter.wait(&sm.z_done, par);
       load_tri(sm.tt, &tm.tt, it, &sm.go_z);
     }
-  } else if (warp == 1) {
+  } else if (warp == W::kMma) {
     // ---------------------------------------------------------------- MMAs
     // (the terminal cotangent must be in tensor memory: barrier 1, decay group and this warp)
-    asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(2 * kRows + 32) : "memory");
     tc_fence_after();
     const uint32_t leader = elect_leader();
     const uint32_t a0 = smem_u32(sm.at), kn0 = smem_u32(sm.kn), tt0 = smem_u32(sm.tt);
@@ -248,14 +257,17 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       mma_commit(&sm.z_done, leader);
       if (it + 1 < n_chunks) issue_a(it + 1);
     }
-  } else if (warp < kBScanDo0) {
+  } else if (!W::works(warp)) {
+    // (nothing to do in this form)
+  } else if (warp < W::kDo0) {
     // ---------------------------------------------------------------- decay of the cotangent
     // thread = value row of the transposed cotangent (TMEM lane) x one half of the 128 key columns
-    const int q4 = warp & 3, half = (warp - kBScanDecay0) >> 2;
+    const int q4 = warp & 3, half = warp >> 2;
     const int vrow = 32 * q4 + lane, k0 = 64 * half;
+    const int64_t my_row = v0 + vrow;
     const uint32_t lane_base = 32u * q4;
     const int64_t state = (int64_t(sq.sid) * p.H + h) * kStateElems;
-    const bool sender = lane == 0 && ((warp - kBScanDecay0) & 3) == 0;  // sends this half's staged rows
+    const bool sender = lane == 0 && q4 == 0;  // sends this half's staged rows
     uint32_t lo[32], hi[32];
     auto half_barrier = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory"); };
     auto load_state = [&](uint32_t col) {
@@ -283,7 +295,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       }
     };
     {
-      const float* src = (p.ds_final != nullptr) ? p.ds_final + state + vrow : nullptr;
+      const float* src = (p.ds_final != nullptr) ? p.ds_final + state + my_row : nullptr;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         lo[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
@@ -291,7 +303,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       }
       store_state(kColS);
       tc_fence_before();
-      asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(2 * kRows + 32) : "memory");
     }
     for (int it = 0; it < n_chunks; ++it) {
       const uint32_t par = uint32_t(it) & 1u;
@@ -319,15 +331,24 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       // the cotangent at the end of this chunk, off the chain: it is still in its buffer, which this group
       // alone overwrites, one step later
       load_state(kColS + 128u * par);
-      send_rows(lo, chunk_of(it), k0);
-      send_rows(hi, chunk_of(it), k0 + 32);
+      if (kParts == 1) {
+        send_rows(lo, chunk_of(it), k0);
+        send_rows(hi, chunk_of(it), k0 + 32);
+      } else {  // (a part of a row is not contiguous: plain stores)
+        float* ck = p.d_bnd + ((int64_t(sq.slot0 + chunk_of(it) + 1) * p.H + h) * kDim + k0) * kDim + my_row;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+          ck[j * kDim] = __uint_as_float(lo[j]);
+          ck[(32 + j) * kDim] = __uint_as_float(hi[j]);
+        }
+      }
     }
     // ---- cotangent of the initial state: slot 0 and d_initial_state ----------------------------------
     waiter.wait(&sm.s_done, uint32_t(n_chunks - 1) & 1u);
     tc_fence_after();
     load_state(kColS + 128u * (uint32_t(n_chunks) & 1u));
-    float* slot = p.d_bnd + (int64_t(sq.slot0) * p.H + h) * kStateElems + vrow;
-    float* init = (p.ds_init != nullptr) ? p.ds_init + state + vrow : nullptr;
+    float* slot = p.d_bnd + (int64_t(sq.slot0) * p.H + h) * kStateElems + my_row;
+    float* init = (p.ds_init != nullptr) ? p.ds_init + state + my_row : nullptr;
     const bool failed = sm.failed != 0;
 #pragma unroll
     for (int j = 0; j < 64; ++j) {
@@ -339,17 +360,17 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
   } else {
     // ---------------------------------------------------------------- dO in, dZ out
     // thread = value row (TMEM lane) x one half of the 64 tokens
-    const int q4 = warp & 3, half = (warp - kBScanDo0) >> 2;
+    const int q4 = warp & 3, half = (warp - W::kDo0) >> 2;
     const int vrow = 32 * q4 + lane, i0 = 32 * half;
     const uint32_t lane_base = 32u * q4;
-    const bool sender = tid == kBScanDo0 * 32;
-    auto group_barrier = [&] { asm volatile("bar.sync 4, 256;" ::: "memory"); };
-    const T* src = reinterpret_cast<const T*>(sm.d_out) + i0 * kDim + vrow;
+    const bool sender = lane == 0 && q4 == 0 && half == 0;
+    auto group_barrier = [&] { asm volatile("bar.sync 4, %0;" ::"n"(2 * kRows) : "memory"); };
+    const T* src = reinterpret_cast<const T*>(sm.d_out) + i0 * kRows + vrow;
     auto build_do = [&](int it) {
       waiter.wait(&sm.full_o, uint32_t(it) & 1u);
       uint32_t x[32];
 #pragma unroll
-      for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(to_float(src[j * kDim]));
+      for (int j = 0; j < 32; ++j) x[j] = __float_as_uint(to_float(src[j * kRows]));
       __syncwarp();
       if (lane == 0) mbar_arrive(&sm.do_read);
       const int n_valid = sq.len - chunk_of(it) * kChunk;
@@ -367,7 +388,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
     };
     arrive(&sm.go_z);  // no earlier step holds up the first dZ
     build_do(0);
-    uint8_t* col = sm.dz + (vrow >> 2) * kCsZ + (vrow & 3) * 4;
+    uint8_t* col = sm.dz + ((v0 + vrow) >> 2) * kCsZ + (vrow & 3) * 4;
     for (int it = 0; it < n_chunks; ++it) {
       if (it + 1 < n_chunks) build_do(it + 1);
       waiter.wait(&sm.z_done, uint32_t(it) & 1u);
@@ -389,7 +410,16 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       fence_async_smem();
       group_barrier();
       if (sender) {
-        bulk_s2g(p.dz + ch_of(it) * kBlobDZ, sm.dz, uint32_t(kBlobDZ));
+        uint8_t* dst = p.dz + ch_of(it) * kBlobDZ;
+        if (kParts == 1) {
+          bulk_s2g(dst, sm.dz, uint32_t(kBlobDZ));
+        } else {  // this CTA's columns of each group of eight rows
+#pragma unroll
+          for (int jg = 0; jg < 8; ++jg) {
+            const int at = jg * kRsZ + (v0 >> 2) * kCsZ;
+            bulk_s2g(dst + at, sm.dz + at, uint32_t(kRows / 4 * kCsZ));
+          }
+        }
         bulk_commit();
       }
     }
@@ -397,7 +427,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == W::kMma) {
     tc_fence_after();
     tmem_dealloc(tb, 512);
   }
@@ -1176,6 +1206,19 @@ int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStrea
   return check_launch();
 }
 
+template <typename T, typename Seqs>
+int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, int64_t n_scan, int parts,
+                 cudaStream_t stream) {
+  auto kernel = parts == 4 ? chunk_bwd_scan_kernel<T, Seqs, 4>
+              : parts == 2 ? chunk_bwd_scan_kernel<T, Seqs, 2> : chunk_bwd_scan_kernel<T, Seqs, 1>;
+  const int smem = int(sizeof(BScanSmem));
+  const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  const int threads = parts > 1 ? BScanWarps<2>::kThreads : BScanWarps<1>::kThreads;
+  kernel<<<unsigned(n_scan * parts), threads, smem, stream>>>(p, seqs, tm);
+  return check_launch();
+}
+
 template <typename Seqs>
 int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream) {
   if (a.grads_f32 && !(a.dtype == GDN2_BF16 && a.g_dtype == GDN2_FP32)) return GDN2_ERR_UNSUPPORTED;
@@ -1188,6 +1231,10 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
   int* status = reinterpret_cast<int*>(const_cast<uint8_t*>(a.workspace) + ws.off_status());
 
   profile_mark(3, stream);
+  int sm_count = 0;
+  if (int err = multiprocessors(&sm_count); err != GDN2_OK) return err;
+  const int64_t n_scan = int64_t(seqs.count()) * a.H;
+  const int parts = value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 4);
   // the reverse scan's operands: the forward's tiles, each in the swizzle of the role backward reads it in
   BScanMaps tm;
   if (!encode_tile_map(&tm.at, a.workspace + ws.off_at(), n_ch, kChunk, kChunk, false, 32, 1) ||
@@ -1195,20 +1242,13 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
       !encode_tile_map(&tm.kn, a.workspace + ws.off_kn(), n_ch, kChunk, kDim, false) ||
       !encode_tile_map(&tm.q, a.workspace + ws.off_q(), n_ch, kChunk, kDim, true) ||
       !encode_tile_map(&tm.yt, a.workspace + ws.off_yt(), n_ch, kDim, kChunk, false) ||
-      !encode_sequence_map(&tm.d_out, a.d_out, a.rows, a.H, a.dtype)) {
+      !encode_sequence_map(&tm.d_out, a.d_out, a.rows, a.H, a.dtype, kChunk, kDim / parts)) {
     return GDN2_ERR_LAUNCH;
   }
   const BScanParams sp{a.workspace + ws.off_d(), a.scratch + sc.off_dz(), a.ds_final, a.d_bnd, a.ds_init, status,
                        int(a.H)};
-  {
-    const int smem = int(sizeof(BScanSmem));
-    auto kernel = a.dtype == GDN2_BF16 ? chunk_bwd_scan_kernel<__nv_bfloat16, Seqs>
-                                       : chunk_bwd_scan_kernel<__half, Seqs>;
-    cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-    if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-    kernel<<<unsigned(seqs.count() * a.H), kBScanThreads, smem, stream>>>(sp, seqs, tm);
-  }
-  int st = check_launch();
+  int st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)
+                                : launch_bscan<__half>(sp, seqs, tm, n_scan, parts, stream);
   if (st != GDN2_OK) return st;
   profile_mark(4, stream);
 

@@ -227,17 +227,17 @@ inline bool encode_cached(CUtensorMap* tm, int rank, CUtensorMapDataType type, c
 
 // A contiguous [rows, H, 128] sequence tensor (rows = batch * time, or the packed length) seen as
 // (channel, head, row): a box (128, 1, 64) is one head's 64-token chunk, landing in shared memory as dense
-// [64][128] rows (`box_rows` tokens instead of 64 when given).  A partial chunk reads on into the rows of
+// [64][128] rows (`box_rows` tokens and `box_cols` channels when given).  A partial chunk reads on into the rows of
 // the next sequence (zeros past the end of the tensor): the kernels mask what is not theirs.
 inline bool encode_sequence_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t heads, int dtype,
-                                int box_rows = kChunk) {
+                                int box_rows = kChunk, int box_cols = kDim) {
   const cuuint64_t es = (dtype == GDN2_FP32) ? 4 : 2;
   const CUtensorMapDataType type = (dtype == GDN2_FP32)   ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
                                    : (dtype == GDN2_BF16) ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                           : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   const cuuint64_t dims[4] = {cuuint64_t(kDim), cuuint64_t(heads), cuuint64_t(rows), 1};
   const cuuint64_t strides[3] = {cuuint64_t(kDim) * es, cuuint64_t(heads) * kDim * es, 0};  // bytes, dimensions 1..2
-  const cuuint32_t box[4] = {cuuint32_t(kDim), 1, cuuint32_t(box_rows), 1};
+  const cuuint32_t box[4] = {cuuint32_t(box_cols), 1, cuuint32_t(box_rows), 1};
   return encode_cached(tm, 3, type, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
@@ -265,6 +265,22 @@ inline bool encode_tile_map(CUtensorMap* tm, const uint8_t* base, int64_t n_ch, 
                              cuuint32_t(box_slabs > 0 ? box_slabs : cols / 32), 1};
   return encode_cached(tm, 4, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, base, dims, strides, box,
                        mn_major ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// CTAs that share the value rows of one (sequence, head) in a scan.  A value row of the state never meets another
+// one, so a scan may have 64 or 32 of the 128 rows (its MMAs still have 128; the lanes behind are idle) and gives
+// the same bits.  What an SM takes in and puts out goes through a port of 48-50 bytes a clock (a probe that only
+// copies: 48.2 in, 50 both ways), and a chunk of a training scan is 284 KB forward and 236 KB back, 2.9 and 2.5 us
+// of its 3.0 and 2.6: halves of the rows move 212 and 178 KB each, quarters 176 and 149.  Scan times, us, with 1 / 2 /
+// 4 parts: training B1 T2048 H16 100 / 70 / 73 forward, 86 / 64 / 60 back; B2 T4096 H16 193 / 143 / 152 and
+// 162 / 128 / 123; inference B1 T2048 H32 70 / 68 / 73, B1 T32768 H16 971 / 866 / 920 (hence 2 at most forward).
+// As many as leave the longest sequence the longest part of the call: with 128 sequences x heads of one length,
+// where every SM has a scan as it is, halves take 749 -> 758 us (training B4 T8192 H32) and 221 -> 293 (inference
+// B8 T4096); packed training of 911, 2300, 150, 1640, 77, 1202, 514, 1398 tokens, H16, 133 -> 114 and 109 -> 97.
+inline int value_parts(int64_t units, int64_t longest, int sm_count, int most) {
+  int parts = 1;
+  while (parts < most && 2 * parts * units <= longest * sm_count) parts *= 2;
+  return parts;
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {

@@ -678,11 +678,11 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 // the tensor cores and the tensor cores for every phase).  Here the MMAs of a chunk are issued back to
 // back by one warp and everything else runs beside them:
 //   warp 0       tiled TMA loads, each buffer refilled as soon as its MMA has read it (one lane)
-//   warp 1       MMAs, per chunk:  R^T -= S^T Y^T | O^T = S^T Qg^T | S'^T += R^T Kt | O^T += R^T Aqk^T |
+//   warp 3       MMAs, per chunk:  R^T -= S^T Y^T | O^T = S^T Qg^T | S'^T += R^T Kt | O^T += R^T Aqk^T |
 //                R'^T = Z'^T T^T of the next chunk.  MMAs of one shape on one accumulator run in order; every
 //                other dependence (R -> S', S' -> R') is waited for, with independent MMAs in the queue meanwhile
 //   warp 2       loads of v and w, whose buffer frees at another time than the others
-//   warp 3       joint launch: watches the marks of prepared chunks (a look at one takes most of a microsecond)
+//   warp 1       joint launch: watches the marks of prepared chunks (a look at one takes most of a microsecond)
 //   warps 4..11  decay: S' <- S diag(d) into the other of two state buffers while R is formed (the output
 //                still reads S); training: the chunk-start state, staged and sent by bulk stores
 //   warps 12..19 Z = w v of the next chunk into tensor memory; training: R out
@@ -692,8 +692,20 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 // A passed mbarrier wait costs ~150 clocks, so what an MMA group needs arrives on one barrier: the bytes of
 // its tiles, the threads that wrote its other operand and those that freed its accumulator.
 // Tensor memory (columns): S 2 x 128, R 2 x 64, O 64, Z 64 = all 512.
-constexpr int kScanThreads = 768, kScanThreadsJoint = 640;
-constexpr int kScanVw = 2, kScanWatch = 3, kScanDecay0 = 4, kScanZ0 = 12, kScanOut0 = 20;  // first warps of the groups
+// Where a CTA has only the first 64 value rows, a group has work for the two warps of four that reach them, and the
+// four single warps take the places of two others: the MMA warp is then alone on its scheduler (3300 -> 2940 clocks a
+// chunk; with working warps beside it an MMA is issued in 50 clocks instead of 25).
+constexpr int kScanThreadsJoint = 640;
+template <int kParts>
+struct ScanWarps {  // (first) warps of the groups
+  static constexpr int kLoads = 0, kWatch = 1, kVw = 2, kMma = 3, kDecay0 = 4, kZ0 = 12, kOut0 = 20, kThreads = 768;
+  static __device__ __forceinline__ bool works(int warp) { return warp >= kDecay0; }
+};
+template <>
+struct ScanWarps<2> {
+  static constexpr int kLoads = 2, kWatch = 7, kVw = 6, kMma = 3, kDecay0 = 0, kZ0 = 8, kOut0 = 16, kThreads = 576;
+  static __device__ __forceinline__ bool works(int warp) { return (warp & 3) < 2; }
+};
 
 struct ScanSmem {
   // swizzled operand tiles, slabs of 32 columns (tc05.cuh): Q is read K-major, the others MN-major
@@ -710,7 +722,8 @@ struct ScanSmem {
   alignas(16) float d[2][kDim];
   alignas(8) uint64_t full_vw, full_d[2];
   uint64_t go_u;      // Tt, Z written (and the R before the last read):          1 load + 8 warps
-  uint64_t go_r;      // Yt, Q, the state of the last chunk, its O read:          2 loads + 1 commit + the warps of O
+  uint64_t go_r;      // Yt, the state of the last chunk:                         1 load + 1 commit
+  uint64_t go_o;      // Q, the O of the last chunk read:                         1 load + the warps of O
   uint64_t go_s;      // Kn, At, decayed state, R:                                2 loads + 8 warps + 1 commit
   uint64_t vw_read;   // v, w are in registers:                                   8 warps
   uint64_t u_done, r_done, q_done, s_done, o_done, all_done;  // MMA commits
@@ -735,22 +748,25 @@ struct ScanMaps {
   CUtensorMap yt, q, kn, at, tt, v, w, out;
 };
 
-// One sequence and head, by a whole CTA.  kJoint: the prep groups run beside in the same launch, and a chunk's
+// One sequence and head, or a half of its value rows (kParts = 2: value_parts), by a whole CTA.  kJoint: the prep groups run beside in the same launch, and a chunk's
 // tiles are loaded once its mark is there.
-template <typename T, typename Seqs, bool kJoint>
+template <typename T, typename Seqs, bool kJoint, int kParts>
 __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& seqs, const ScanMaps& tm, ScanSmem& sm,
                                               const int item) {
-  constexpr int kThreads = kJoint ? kScanThreadsJoint : kScanThreads;
+  constexpr int kRows = kDim / kParts;  // value rows of this CTA: lanes 0 .. kRows - 1 of tensor memory
+  using W = ScanWarps<kParts>;
+  constexpr int kThreads = kJoint ? kScanThreadsJoint : W::kThreads;
   BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int s = item / p.H, h = item - s * p.H;
+  const int unit = item / kParts, v0 = (item - unit * kParts) * kRows;
+  const int s = unit / p.H, h = unit - s * p.H;
   const SeqInfo sq = seqs.at(s);
   const int n_chunks = sq.n_chunks;
   constexpr uint32_t kColS = 0, kColR = 256, kColO = 384, kColZ = 448;
   auto ch_of = [&](int c) { return int64_t(sq.chunk0 + c) * p.H + h; };
 
-  if (warp == 1) {
+  if (warp == W::kMma) {
     tmem_alloc(&sm.tmem_base, 512);
     tmem_relinquish();
   }
@@ -758,10 +774,11 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
     mbar_init(&sm.full_vw, 1);
     mbar_init(&sm.full_d[0], 1);
     mbar_init(&sm.full_d[1], 1);
-    mbar_init(&sm.go_u, 1 + 8);
-    mbar_init(&sm.go_r, 2 + 1 + (kJoint ? 8 : 4));
-    mbar_init(&sm.go_s, 2 + 8 + 1);
-    mbar_init(&sm.vw_read, 8);
+    mbar_init(&sm.go_u, 1 + 8 / kParts);
+    mbar_init(&sm.go_r, 1 + 1);
+    mbar_init(&sm.go_o, 1 + (kJoint ? 8 : 4) / kParts);
+    mbar_init(&sm.go_s, 2 + 8 / kParts + 1);
+    mbar_init(&sm.vw_read, 8 / kParts);
     mbar_init(&sm.u_done, 1); mbar_init(&sm.r_done, 1); mbar_init(&sm.q_done, 1);
     mbar_init(&sm.s_done, 1); mbar_init(&sm.o_done, 1); mbar_init(&sm.all_done, 1);
     mbar_arrive(&sm.go_r);  // no earlier chunk holds up the first one
@@ -789,7 +806,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
   // O of a chunk out, by whole sets of four warps (one per lane quadrant of tensor memory), each `kTokens` of
   // the 64 tokens from i0 on
   auto emit_o = [&](auto tokens, int c, int i0, int group0) {
-    constexpr int kTokens = decltype(tokens)::value, kGroup = 128 * (kChunk / kTokens);
+    constexpr int kTokens = decltype(tokens)::value, kGroup = kRows * (kChunk / kTokens);
     const int vrow = 32 * (warp & 3) + lane;
     const bool sender = tid == group0 * 32;
     waiter.wait(&sm.o_done, uint32_t(c) & 1u);
@@ -800,36 +817,38 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       tmem_ld32(tmem_addr(tb, 32u * (warp & 3), kColO + i0 + j), *reinterpret_cast<uint32_t(*)[32]>(&x[j]));
     }
     tmem_wait_ld();
-    if (c + 1 < n_chunks) arrive(&sm.go_r);
+    if (c + 1 < n_chunks) arrive(&sm.go_o);
     const bool failed = sm.failed != 0;
     if (sender) bulk_wait_read_all();  // the previous chunk's rows have left the buffer
     asm volatile("bar.sync 4, %0;" ::"n"(kGroup) : "memory");
-    T* tile = reinterpret_cast<T*>(sm.o) + i0 * kDim + vrow;
+    T* tile = reinterpret_cast<T*>(sm.o) + i0 * kRows + vrow;
 #pragma unroll
     for (int j = 0; j < kTokens; j += 2) {
       typename Pair<T>::type y = Pair<T>::make(__uint_as_float(x[j]), __uint_as_float(x[j + 1]));
       if (failed) y = Pair<T>::make(poison_nan(), poison_nan());
-      tile[j * kDim] = y.x;
-      tile[(j + 1) * kDim] = y.y;
+      tile[j * kRows] = y.x;
+      tile[(j + 1) * kRows] = y.y;
     }
     fence_async_smem();
     asm volatile("bar.sync 4, %0;" ::"n"(kGroup) : "memory");
     const int row = int(sq.row0) + c * kChunk, n_valid = min(kChunk, sq.len - c * kChunk);
     if (n_valid == kChunk) {
       if (sender) {
-        tma_store_3d(&tm.out, 0, h, row, sm.o);
+        tma_store_3d(&tm.out, v0, h, row, sm.o);
         bulk_commit();
       }
     } else {  // the rows behind a partial chunk (the last one) belong to somebody else
-      for (int e = tid - group0 * 32; e < n_valid * 16; e += kGroup) {
-        *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + (int64_t(row + (e >> 4)) * p.H + h) * kDim + 8 * (e & 15)) =
-            *reinterpret_cast<const uint4*>(sm.o + e * 16);
+      constexpr int kPieces = kRows / 8;  // 16-byte pieces of a row
+      const int first = (kTokens == kChunk ? 0 : (i0 / kTokens) * kRows) + vrow;
+      for (int e = first; e < n_valid * kPieces; e += kGroup) {
+        *reinterpret_cast<uint4*>(static_cast<T*>(p.out) + (int64_t(row + e / kPieces) * p.H + h) * kDim + v0 +
+                                  8 * (e % kPieces)) = *reinterpret_cast<const uint4*>(sm.o + e * 16);
       }
     }
     if (sender && c + 1 == n_chunks) bulk_wait_all();  // the last rows are in global memory before the CTA retires
   };
 
-  if (warp == 0) {
+  if (warp == W::kLoads) {
     // ---------------------------------------------------------------- loads
     const uint32_t leader = elect_leader();
     // Tt and At are zero for j >= 32, i < 32: three 32-row boxes, the fourth quadrant of the tile stays zero
@@ -855,8 +874,8 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       tma_load_4d(sm.kn, &tm.kn, 0, 0, 0, int(ch_of(c)), &sm.go_s, leader);
     };
     auto load_q = [&](int c) {
-      mbar_arrive_expect_tx(&sm.go_r, uint32_t(kTileQ), leader);
-      tma_load_4d(sm.q, &tm.q, 0, 0, 0, int(ch_of(c)), &sm.go_r, leader);
+      mbar_arrive_expect_tx(&sm.go_o, uint32_t(kTileQ), leader);
+      tma_load_4d(sm.q, &tm.q, 0, 0, 0, int(ch_of(c)), &sm.go_o, leader);
     };
     auto load_a = [&](int c) {
       mbar_arrive_expect_tx(&sm.go_s, uint32_t(kTileAt - 4096), leader);
@@ -892,10 +911,10 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       waiter.wait(&sm.o_done, par);
       load_a(c);
     }
-  } else if (warp == 1) {
+  } else if (warp == W::kMma) {
     // ---------------------------------------------------------------- MMAs
     // (the initial state must be in tensor memory: barrier 1, decay group and this warp)
-    asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(2 * kRows + 32) : "memory");
     tc_fence_after();
     const uint32_t leader = elect_leader();
     const uint32_t y0 = smem_u32(sm.yt), q0 = smem_u32(sm.q), a0 = smem_u32(sm.at);
@@ -929,6 +948,8 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       }
       mma_commit(&sm.r_done, leader);
       mma_commit(&sm.go_s, leader);
+      waiter.wait(&sm.go_o, par);
+      tc_fence_after();
       // O^T = S^T Qg^T   (B = Q[i][k] read K-major)
 #pragma unroll
       for (int ks = 0; ks < 16; ++ks) {
@@ -953,15 +974,52 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       if (c + 1 < n_chunks) issue_u(c + 1);
     }
     mma_commit(&sm.all_done, leader);
-  } else if (warp >= kScanDecay0 && warp < kScanZ0) {
+  } else if (warp == W::kVw) {
+    // ---------------------------------------------------------------- v and w
+    const uint32_t leader = elect_leader();
+    auto load_vw = [&](int c) {
+      const int row = int(sq.row0) + c * kChunk;
+      mbar_arrive_expect_tx(&sm.full_vw, 2u * 16384u / kParts, leader);
+      tma_load_3d(sm.v, &tm.v, v0, h, row, &sm.full_vw, leader);
+      tma_load_3d(sm.w, &tm.w, v0, h, row, &sm.full_vw, leader);
+    };
+    load_vw(0);
+    for (int c = 1; c < n_chunks; ++c) {
+      waiter.wait(&sm.vw_read, uint32_t(c - 1) & 1u);
+      load_vw(c);
+    }
+  } else if (kJoint && warp == W::kWatch) {
+    // ---------------------------------------------------------------- marks of prepared chunks
+    for (int c = 0; c < n_chunks;) {
+      const int mine = min(c + lane, n_chunks - 1);
+      const uint32_t missing = ~__ballot_sync(0xffffffffu, marked(reinterpret_cast<const float*>(p.d + ch_of(mine) * kBlobD)));
+      const int there = missing == 0 ? 32 : __ffs(int(missing)) - 1;
+      if (there == 0) {
+        if (!waiter.look_again()) c = n_chunks;
+        __nanosleep(200);
+      } else {
+        c = min(c + there, n_chunks);
+      }
+      // (a wait of a preparer that ran out, or this one's own: results become NaN)
+      if (*static_cast<volatile const int*>(p.status) != kStatusOk) sm.failed = 1;
+      __syncwarp();
+      if (lane == 0 && c > 0) {
+        __threadfence_block();
+        sm.prepared = c;
+      }
+    }
+  } else if (!W::works(warp)) {
+    // (nothing to do in this form)
+  } else if (warp < W::kZ0) {
     // ---------------------------------------------------------------- decay of the state
     // thread = value row of the transposed state (TMEM lane) x one half of the 128 key columns
-    const int q4 = warp & 3, half = (warp - kScanDecay0) >> 2;
+    const int q4 = warp & 3, half = (warp - W::kDecay0) >> 2;
     const int vrow = 32 * q4 + lane, k0 = 64 * half;
     const uint32_t lane_base = 32u * q4;
     const int64_t state = (int64_t(sq.sid) * p.H + h) * int64_t(kDim * kDim);
-    const bool sender = lane == 0 && ((warp - kScanDecay0) & 3) == 0;  // sends this half's staged rows
+    const bool sender = lane == 0 && q4 == 0;  // sends this half's staged rows
     uint32_t lo[32], hi[32];
+    const int64_t my_row = v0 + vrow;
     auto half_barrier = [&] { asm volatile("bar.sync %0, 128;" ::"r"(2 + half) : "memory"); };
     auto load_state = [&](uint32_t col) {
       tmem_ld32(tmem_addr(tb, lane_base, col + k0), lo);
@@ -988,7 +1046,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       }
     };
     {
-      const float* src = (p.s_in != nullptr) ? p.s_in + state + vrow : nullptr;
+      const float* src = (p.s_in != nullptr) ? p.s_in + state + my_row : nullptr;
 #pragma unroll
       for (int j = 0; j < 32; ++j) {
         lo[j] = (src != nullptr) ? __float_as_uint(src[(k0 + j) * kDim]) : 0u;
@@ -996,7 +1054,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       }
       store_state(kColS);
       tc_fence_before();
-      asm volatile("bar.sync 1, %0;" ::"n"(256 + 32) : "memory");
+      asm volatile("bar.sync 1, %0;" ::"n"(2 * kRows + 32) : "memory");
     }
     for (int c = 0; c < n_chunks; ++c) {
       const uint32_t par = uint32_t(c) & 1u;
@@ -1005,7 +1063,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         tc_fence_after();
         load_state(kColS + 128u * par);
       }
-      if (p.bnd != nullptr) send_rows(lo, c, k0);
+      if (kParts == 1 && p.bnd != nullptr) send_rows(lo, c, k0);
       waiter.wait(&sm.full_d[par], uint32_t(c >> 1) & 1u);
 #pragma unroll
       for (int j4 = 0; j4 < 8; ++j4) {
@@ -1027,19 +1085,25 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         // the other rows, off the chain: the chunk-start state is still in its buffer, which this group alone
         // overwrites, one chunk later.  They leave by plain stores: the copy engine has 200 KB of a chunk to
         // move as it is (with these rows staged too, a chunk waited 2000 clocks for its buffer)
+        float* ck = p.bnd + ((int64_t(sq.slot0 + c) * p.H + h) * kDim + k0) * kDim + my_row;
+        if (kParts > 1) {  // (a part of a row is not contiguous: all of it in this way)
+          tmem_ld32(tmem_addr(tb, lane_base, kColS + 128u * par + k0), lo);
+          tmem_wait_ld();
+#pragma unroll
+          for (int j = 0; j < 32; ++j) ck[j * kDim] = __uint_as_float(lo[j]);
+        }
         tmem_ld32(tmem_addr(tb, lane_base, kColS + 128u * par + k0 + 32), hi);
         tmem_wait_ld();
-        float* ck = p.bnd + ((int64_t(sq.slot0 + c) * p.H + h) * kDim + k0 + 32) * kDim + vrow;
 #pragma unroll
-        for (int j = 0; j < 32; ++j) ck[j * kDim] = __uint_as_float(hi[j]);
+        for (int j = 0; j < 32; ++j) ck[(32 + j) * kDim] = __uint_as_float(hi[j]);
       }
     }
     // ---- final state ---------------------------------------------------------------------------------
     waiter.wait(&sm.s_done, uint32_t(n_chunks - 1) & 1u);
     tc_fence_after();
     load_state(kColS + 128u * (uint32_t(n_chunks) & 1u));
-    float* fin = (p.s_out != nullptr) ? p.s_out + state + vrow : nullptr;
-    float* ck = (p.bnd != nullptr) ? p.bnd + (int64_t(sq.slot0 + n_chunks) * p.H + h) * int64_t(kDim * kDim) + vrow
+    float* fin = (p.s_out != nullptr) ? p.s_out + state + my_row : nullptr;
+    float* ck = (p.bnd != nullptr) ? p.bnd + (int64_t(sq.slot0 + n_chunks) * p.H + h) * int64_t(kDim * kDim) + my_row
                                    : nullptr;
     const bool failed = sm.failed != 0;
 #pragma unroll
@@ -1049,14 +1113,14 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       if (ck != nullptr) ck[(k0 + j) * kDim] = x;
     }
     if (sender) bulk_wait_all();  // the last staged rows are in global memory before the CTA retires
-  } else if (warp >= kScanZ0 && (kJoint || warp < kScanOut0)) {
+  } else if (kJoint || warp < W::kOut0) {
     // ---------------------------------------------------------------- Z = w v (and in a joint launch O out)
     // thread = value row (TMEM lane) x one half of the 64 tokens
-    const int q4 = warp & 3, half = (warp - kScanZ0) >> 2;
+    const int q4 = warp & 3, half = (warp - W::kZ0) >> 2;
     const int vrow = 32 * q4 + lane, i0 = 32 * half;
     const uint32_t lane_base = 32u * q4;
-    const T* vs = reinterpret_cast<const T*>(sm.v) + i0 * kDim + vrow;
-    const T* wsrc = reinterpret_cast<const T*>(sm.w) + i0 * kDim + vrow;
+    const T* vs = reinterpret_cast<const T*>(sm.v) + i0 * kRows + vrow;
+    const T* wsrc = reinterpret_cast<const T*>(sm.w) + i0 * kRows + vrow;
     uint32_t a[32];
     // R of chunk c for backward, row-major R[j][v]: the 32 lanes of a warp fill one 128-byte line per token
     auto load_residual = [&](int c) {
@@ -1064,7 +1128,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       tmem_wait_ld();
     };
     auto store_residual = [&](int c) {
-      float* rn = p.rn + ch_of(c) * (kBlobRn / 4) + i0 * kDim + vrow;
+      float* rn = p.rn + ch_of(c) * (kBlobRn / 4) + i0 * kDim + v0 + vrow;
 #pragma unroll
       for (int j = 0; j < 32; ++j) rn[j * kDim] = to_tf32(__uint_as_float(a[j]));
     };
@@ -1078,8 +1142,8 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         float z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          z[j] = to_float(wsrc[(16 * part + j) * kDim]);
-          vr[j] = vs[(16 * part + j) * kDim];
+          z[j] = to_float(wsrc[(16 * part + j) * kRows]);
+          vr[j] = vs[(16 * part + j) * kRows];
         }
         if (part == 1) {
           __syncwarp();
@@ -1107,11 +1171,11 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       arrive(&sm.go_u);
       if (p.rn != nullptr && c > 1) store_residual(c - 2);
     };
-    if constexpr (kJoint) arrive(&sm.go_r);  // no earlier chunk holds up the first output
+    if constexpr (kJoint) arrive(&sm.go_o);  // no earlier chunk holds up the first output
     build_z(0);
     for (int c = 0; c < n_chunks; ++c) {
       if (c + 1 < n_chunks) build_z(c + 1);
-      if constexpr (kJoint) emit_o(std::integral_constant<int, 32>{}, c, i0, kScanZ0);
+      if constexpr (kJoint) emit_o(std::integral_constant<int, 32>{}, c, i0, W::kZ0);
     }
     if (p.rn != nullptr) {
       waiter.wait(&sm.all_done, 0);
@@ -1121,58 +1185,24 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         store_residual(c);
       }
     }
-  } else if (!kJoint && warp >= kScanOut0) {
+  } else {
     // ---------------------------------------------------------------- O out
-    arrive(&sm.go_r);  // no earlier chunk holds up the first output
-    for (int c = 0; c < n_chunks; ++c) emit_o(std::integral_constant<int, 64>{}, c, 0, kScanOut0);
-  } else if (warp == kScanVw) {
-    // ---------------------------------------------------------------- v and w
-    const uint32_t leader = elect_leader();
-    auto load_vw = [&](int c) {
-      const int row = int(sq.row0) + c * kChunk;
-      mbar_arrive_expect_tx(&sm.full_vw, 2u * 16384u, leader);
-      tma_load_3d(sm.v, &tm.v, 0, h, row, &sm.full_vw, leader);
-      tma_load_3d(sm.w, &tm.w, 0, h, row, &sm.full_vw, leader);
-    };
-    load_vw(0);
-    for (int c = 1; c < n_chunks; ++c) {
-      waiter.wait(&sm.vw_read, uint32_t(c - 1) & 1u);
-      load_vw(c);
-    }
-  } else if (kJoint && warp == kScanWatch) {
-    // ---------------------------------------------------------------- marks of prepared chunks
-    for (int c = 0; c < n_chunks;) {
-      const int mine = min(c + lane, n_chunks - 1);
-      const uint32_t missing = ~__ballot_sync(0xffffffffu, marked(reinterpret_cast<const float*>(p.d + ch_of(mine) * kBlobD)));
-      const int there = missing == 0 ? 32 : __ffs(int(missing)) - 1;
-      if (there == 0) {
-        if (!waiter.look_again()) c = n_chunks;
-        __nanosleep(200);
-      } else {
-        c = min(c + there, n_chunks);
-      }
-      // (a wait of a preparer that ran out, or this one's own: results become NaN)
-      if (*static_cast<volatile const int*>(p.status) != kStatusOk) sm.failed = 1;
-      __syncwarp();
-      if (lane == 0 && c > 0) {
-        __threadfence_block();
-        sm.prepared = c;
-      }
-    }
+    arrive(&sm.go_o);  // no earlier chunk holds up the first output
+    for (int c = 0; c < n_chunks; ++c) emit_o(std::integral_constant<int, 64>{}, c, 0, W::kOut0);
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 1) {
+  if (warp == W::kMma) {
     tc_fence_after();
     tmem_dealloc(tb, 512);
   }
 }
 
-template <typename T, typename Seqs>
-__global__ void __launch_bounds__(kScanThreads, 1)
+template <typename T, typename Seqs, int kParts>
+__global__ void __launch_bounds__(ScanWarps<kParts>::kThreads, 1)
 chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ ScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  scan_sequence<T, Seqs, false>(p, seqs, tm, *reinterpret_cast<ScanSmem*>(smem_raw), int(blockIdx.x));
+  scan_sequence<T, Seqs, false, kParts>(p, seqs, tm, *reinterpret_cast<ScanSmem*>(smem_raw), int(blockIdx.x));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1199,7 +1229,7 @@ chunk_joint_kernel(const PrepParams pp, const ScanParams sp, const __grid_consta
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const int n_scan = seqs.count() * sp.H, pair = int(blockIdx.x) >> 1, mate = int(blockIdx.x) & 1;
   if (pair < n_scan && mate == 0) {
-    scan_sequence<T, Seqs, true>(sp, seqs, tm_scan, *reinterpret_cast<ScanSmem*>(smem_raw), pair);
+    scan_sequence<T, Seqs, true, 1>(sp, seqs, tm_scan, *reinterpret_cast<ScanSmem*>(smem_raw), pair);
     return;
   }
   if (pair < n_scan && !mates) return;
@@ -1347,11 +1377,29 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   return GDN2_OK;
 }
 
+template <typename T, typename Seqs>
+int launch_scan(const ScanParams& p, const Seqs& seqs, const ScanMaps& tm, int64_t n_scan, int parts,
+                cudaStream_t stream) {
+  auto kernel = parts == 2 ? chunk_scan_kernel<T, Seqs, 2> : chunk_scan_kernel<T, Seqs, 1>;
+  const int smem = int(sizeof(ScanSmem));
+  const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  const int threads = parts == 2 ? ScanWarps<2>::kThreads : ScanWarps<1>::kThreads;
+  kernel<<<unsigned(n_scan * parts), threads, smem, stream>>>(p, seqs, tm);
+  return check_launch();
+}
+
 template <typename Seqs>
 int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) {
   const int64_t n_ch = int64_t(seqs.total_chunks()) * a.H;
   // units, token rows and the grids of the scans are 31-bit numbers
   if (n_ch <= 0 || n_ch > int64_t(0x7fffffff) || a.rows > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
+  int sm_count = 0;
+  if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
+  const int64_t n_scan = int64_t(seqs.count()) * a.H;
+  bool joint = false;
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, sm_count);
+  const int parts = joint ? 1 : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 2);
   const WsLayout ws{n_ch, a.training != 0};
   int* status = reinterpret_cast<int*>(a.workspace + ws.off_status());
   const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
@@ -1362,9 +1410,9 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
       !encode_round_map(&tm_prep.k, a.k, a.rows, a.H, a.dtype) ||
       !encode_round_map(&tm_prep.q, a.q, a.rows, a.H, a.dtype) ||
       !encode_round_map(&tm_prep.beta, a.beta, a.rows, a.H, a.dtype) ||
-      !encode_sequence_map(&tm.v, a.v, a.rows, a.H, a.dtype) ||
-      !encode_sequence_map(&tm.w, a.w, a.rows, a.H, a.dtype) ||
-      !encode_sequence_map(&tm.out, a.out, a.rows, a.H, a.dtype) ||
+      !encode_sequence_map(&tm.v, a.v, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||
+      !encode_sequence_map(&tm.w, a.w, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||
+      !encode_sequence_map(&tm.out, a.out, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||
       !encode_tile_map(&tm.yt, tiles.yt, n_ch, kDim, kChunk, true) ||
       !encode_tile_map(&tm.q, tiles.q, n_ch, kChunk, kDim, false) ||
       !encode_tile_map(&tm.kn, tiles.kn, n_ch, kChunk, kDim, true) ||
@@ -1372,17 +1420,13 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
       !encode_tile_map(&tm.tt, tiles.tt, n_ch, kChunk, kChunk, true, 32, 1)) {
     return GDN2_ERR_LAUNCH;
   }
-  int sm_count = 0;
-  if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
-
   const PrepParams pp{a.workspace, tiles, n_ch, int(a.H), a.scale, a.training, a.prologue};
   const ScanParams sp{a.workspace + ws.off_d(), a.s_in, a.out, a.s_out, a.bnd,
                       a.training ? reinterpret_cast<float*>(a.workspace + ws.off_rn()) : nullptr,
                       status, int(a.H), (a.prologue & kPrologueGate) != 0};
-  const int64_t n_scan = int64_t(seqs.count()) * a.H;
   cudaError_t err;
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
-    if (prefer_joint(n_scan, n_ch, seqs.n_chunks, sm_count)) {
+    if (joint) {
       int st = GDN2_OK;
       GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
         st = a.prologue != 0 ? launch_joint<T, G, Seqs, true>(pp, sp, seqs, tm_prep, tm, sm_count, stream)
@@ -1410,13 +1454,8 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (st != GDN2_OK) return st;
   profile_mark(1, stream);
 
-  const int smem = int(sizeof(ScanSmem));
-  const unsigned grid = unsigned(n_scan);
-  auto kernel = a.dtype == GDN2_BF16 ? chunk_scan_kernel<__nv_bfloat16, Seqs> : chunk_scan_kernel<__half, Seqs>;
-  err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  kernel<<<grid, kScanThreads, smem, stream>>>(sp, seqs, tm);
-  st = check_launch();
+  st = a.dtype == GDN2_BF16 ? launch_scan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)
+                            : launch_scan<__half>(sp, seqs, tm, n_scan, parts, stream);
   profile_mark(2, stream);
   t_forward_kernels = 2;
   return st;

@@ -30,6 +30,49 @@ def test_joint_launch_equals_a_unit_alone_and_the_oracle(batch, heads, time, ker
     _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
 
 
+# One head has its scans' value rows split over two CTAs forward and four back, 37, 38 and 74 heads over two (or four
+# and two) and 75 over none: one chunk, a partial one of a token, and several with a ragged end
+@pytest.mark.parametrize("time", [64, 65, 200])
+@pytest.mark.parametrize("heads", [37, 38, 74, 75])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_scans_of_split_value_rows_equal_whole_ones(heads, time, dtype):
+    tensors, d_out, d_fin = _device_inputs(2, time, 75, seed=time)
+    tensors, d_out = [t.to(dtype) if t.dtype == torch.bfloat16 else t for t in tensors], d_out.to(dtype)
+    out, fin, grads = _step(tensors, d_out, d_fin)  # 150 sequences x heads: never split
+    h = slice(75 - heads, 75)
+    part = [t[1:2, :, h].contiguous() for t in tensors[:6]] + [tensors[6][1:2, h].contiguous()]
+    for single in (part, [t[:, :, :1].contiguous() for t in part[:6]] + [part[6][:, :1].contiguous()]):
+        n = single[6].shape[1]
+        at = slice(75 - heads, 75 - heads + n)
+        o, f, gr = _step(single, d_out[1:2, :, at].contiguous(), d_fin[1:2, at].contiguous())
+        assert torch.equal(o, out[1:2, :, at]) and torch.equal(f, fin[1:2, at])
+        for a, b in zip(gr[:6], grads[:6]):
+            assert torch.equal(a, b[1:2, :, at])
+        assert torch.equal(gr[6], grads[6][1:2, at])
+
+
+# four sequences of which one is long: split at 16 heads (2 * 56 units a head <= 41 * 148), not in the sequences alone
+def test_packed_scans_of_split_value_rows_equal_single_sequences():
+    lengths, heads = [2600, 64, 70, 700], 16
+    cu = [0]
+    for n in lengths:
+        cu.append(cu[-1] + n)
+    tensors, d_out, _ = _device_inputs(1, cu[-1], heads, seed=5)
+    torch.manual_seed(5)
+    states = 0.02 * torch.randn(len(lengths), heads, 128, 128, device=DEV)
+    d_fin = 0.01 * torch.randn_like(states)
+    leaves = [t.requires_grad_(True) for t in (*tensors[:6], states)]
+    out, fin = chunk_gdn2_varlen(*leaves[:6], cu, leaves[6], output_final_state=True)
+    grads = torch.autograd.grad((out.float() * d_out.float()).sum() + (fin * d_fin).sum(), leaves)
+    for i, (lo, hi) in enumerate(zip(cu, cu[1:])):
+        single = [t[:, lo:hi].detach().clone() for t in leaves[:6]] + [states[i:i + 1].detach().clone()]
+        o, f, gr = _step(single, d_out[:, lo:hi], d_fin[i:i + 1])
+        assert torch.equal(o, out[:, lo:hi]) and torch.equal(f, fin[i:i + 1])
+        for a, b in zip(gr[:6], grads[:6]):
+            assert torch.equal(a, b[:, lo:hi])
+        assert torch.equal(gr[6], grads[6][i:i + 1])
+
+
 @pytest.mark.parametrize("dtype,g_dtype", [(torch.bfloat16, torch.float32), (torch.float16, torch.float16)])
 @pytest.mark.parametrize("raw", [False, True])
 def test_joint_launch_equals_two_launches(dtype, g_dtype, raw):
