@@ -29,6 +29,7 @@
 //   T = (I + L)^-1,  Y = T (beta k exp(G)),  R = T (w v) - Y S
 //   Qg = scale q exp(G),  Kt = k exp(G_end - G),  d = exp(G_end)
 
+#include <algorithm>
 #include <type_traits>
 
 #include "chunk_common.cuh"
@@ -52,6 +53,7 @@ namespace {
 // A thread owns 2 tokens x 4 channels of each round: tokens 8 warp + lane / 8 and 4 further on, channels
 // 4 (lane % 8): one 16-byte chunk of every tile row.  The eight lanes of a store phase fill one 128-byte line.
 constexpr int kPrepThreads = 256;
+constexpr int kJointParts = 2;
 constexpr int kRound = 32, kRounds = kDim / kRound;  // channels per round
 constexpr int kLd = 68;           // leading dimension of the fp32 64x64 scratch matrices (16-byte rows, banks shift by 4)
 constexpr int kLdW = 20;          // leading dimension of the transposed 16x16 block products
@@ -108,12 +110,12 @@ struct PrepMaps {
 // The units of one group of 256 threads (`tid` within it): first, first + stride, ..., or in a joint launch
 // `first` and then whatever the queue gives; tensor memory columns tb .. tb + 255.  kPro: the instantiation
 // that can apply the layer prologue to raw inputs (p.prologue says which parts); the plain instantiation
-// carries none of that code.  kJoint: units are taken in the order in which the scans running beside need
+// carries none of that code.  kJoint: `quota` (0: all there are) units are taken in the order in which the scans running beside need
 // them (chunk by chunk through all sequences), and a finished one is marked in its D array.
 template <typename T, typename G, typename Seqs, bool kPro, bool kJoint>
 __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs, const PrepMaps& tm, PrepSmem& sm,
                                            const int tid, const uint32_t tb, const int first, const int stride,
-                                           const int barrier, int* queue) {
+                                           const int barrier, int* queue, int quota) {
   uint8_t* const R = sm.region;
   const WsLayout ws{p.n_ch, p.training != 0};
   int* status = reinterpret_cast<int*>(p.ws + ws.off_status());
@@ -180,7 +182,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   // the pace of the others, and the scans wait for the slowest
   unit_next = unit + stride;
   if constexpr (kJoint) {
-    if (tid == 32) sm.next[par] = unit_next = stride + atomicAdd(queue, 1);
+    if (tid == 32) sm.next[par] = unit_next = --quota != 0 ? stride + atomicAdd(queue, 1) : n_ch;
   }
   // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
   // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
@@ -664,7 +666,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tb = sm.tmem_base;
-  prep_units<T, G, Seqs, kPro, false>(p, seqs, tm, sm, threadIdx.x, tb, int(blockIdx.x), int(gridDim.x), 0, nullptr);
+  prep_units<T, G, Seqs, kPro, false>(p, seqs, tm, sm, threadIdx.x, tb, int(blockIdx.x), int(gridDim.x), 0, nullptr, 0);
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x < 32) tmem_dealloc(tb, 256);
@@ -695,7 +697,6 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 // Where a CTA has only the first 64 value rows, a group has work for the two warps of four that reach them, and the
 // four single warps take the places of two others: the MMA warp is then alone on its scheduler (3300 -> 2940 clocks a
 // chunk; with working warps beside it an MMA is issued in 50 clocks instead of 25).
-constexpr int kScanThreadsJoint = 640;
 template <int kParts>
 struct ScanWarps {  // (first) warps of the groups
   static constexpr int kLoads = 0, kWatch = 1, kVw = 2, kMma = 3, kDecay0 = 4, kZ0 = 12, kOut0 = 20, kThreads = 768;
@@ -714,18 +715,18 @@ struct ScanSmem {
   alignas(1024) uint8_t kn[32768];   // Kn[j][k]: 4 slabs of 64 lines
   alignas(1024) uint8_t at[16384];   // At[j][i]: 2 slabs of 64 lines
   alignas(1024) uint8_t tt[16384];   // Tt[j][i]: 2 slabs of 64 lines
-  alignas(128) uint8_t v[16384];     // raw v, w of the chunk, [64][128] 16-bit rows
+  alignas(128) uint8_t v[16384];     // raw v, w of the chunk, [64][128] 16-bit rows (halves of two chunks)
   alignas(128) uint8_t w[16384];
   alignas(128) uint8_t o[16384];     // output rows [64][128] on their way out (one TMA store: 64-byte pieces
                                      // stored by threads at the stride of a token row drain at 2 bytes per clock)
   alignas(128) float ck[2][32 * kDim];  // training: 32 rows of the chunk-start state per half of the decay group
   alignas(16) float d[2][kDim];
-  alignas(8) uint64_t full_vw, full_d[2];
+  alignas(8) uint64_t full_vw[2], full_d[2];
   uint64_t go_u;      // Tt, Z written (and the R before the last read):          1 load + 8 warps
   uint64_t go_r;      // Yt, the state of the last chunk:                         1 load + 1 commit
   uint64_t go_o;      // Q, the O of the last chunk read:                         1 load + the warps of O
   uint64_t go_s;      // Kn, At, decayed state, R:                                2 loads + 8 warps + 1 commit
-  uint64_t vw_read;   // v, w are in registers:                                   8 warps
+  uint64_t vw_read[2];  // v, w are in registers:                                   8 warps
   uint64_t u_done, r_done, q_done, s_done, o_done, all_done;  // MMA commits
   volatile int failed;
   volatile int prepared;  // chunks whose tiles may be loaded
@@ -754,8 +755,9 @@ template <typename T, typename Seqs, bool kJoint, int kParts>
 __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& seqs, const ScanMaps& tm, ScanSmem& sm,
                                               const int item) {
   constexpr int kRows = kDim / kParts;  // value rows of this CTA: lanes 0 .. kRows - 1 of tensor memory
+  constexpr int kVwSlots = kParts;      // halves of v and w leave room for those of the next chunk
   using W = ScanWarps<kParts>;
-  constexpr int kThreads = kJoint ? kScanThreadsJoint : W::kThreads;
+  constexpr int kThreads = kJoint ? 32 * W::kOut0 : W::kThreads;
   BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -771,14 +773,16 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
     tmem_relinquish();
   }
   if (tid == 0) {
-    mbar_init(&sm.full_vw, 1);
+    for (int i = 0; i < kVwSlots; ++i) {
+      mbar_init(&sm.full_vw[i], 1);
+      mbar_init(&sm.vw_read[i], 8 / kParts);
+    }
     mbar_init(&sm.full_d[0], 1);
     mbar_init(&sm.full_d[1], 1);
     mbar_init(&sm.go_u, 1 + 8 / kParts);
     mbar_init(&sm.go_r, 1 + 1);
     mbar_init(&sm.go_o, 1 + (kJoint ? 8 : 4) / kParts);
     mbar_init(&sm.go_s, 2 + 8 / kParts + 1);
-    mbar_init(&sm.vw_read, 8 / kParts);
     mbar_init(&sm.u_done, 1); mbar_init(&sm.r_done, 1); mbar_init(&sm.q_done, 1);
     mbar_init(&sm.s_done, 1); mbar_init(&sm.o_done, 1); mbar_init(&sm.all_done, 1);
     mbar_arrive(&sm.go_r);  // no earlier chunk holds up the first one
@@ -881,13 +885,13 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       mbar_arrive_expect_tx(&sm.go_s, uint32_t(kTileAt - 4096), leader);
       load_tri(sm.at, &tm.at, int(ch_of(c)), &sm.go_s);
     };
+    int prepared = 0;  // chunks known to be prepared: a fence for each of them held up its first load by 1000 clocks
     auto ready = [&](int c) {
-      if constexpr (kJoint) {
-        // (the watching warp gives up by itself and then lets everything pass)
-        for (uint32_t looks = 0; sm.prepared <= c && looks < (1u << 27); ++looks) __nanosleep(20);
-        __threadfence_block();
-        fence_async_all();
-      }
+      if (!kJoint || c < prepared) return;
+      // (the watching warp gives up by itself and then lets everything pass)
+      for (uint32_t looks = 0; (prepared = sm.prepared) <= c && looks < (1u << 27); ++looks) __nanosleep(20);
+      __threadfence_block();
+      fence_async_all();
     };
     ready(0);
     load_t(0);
@@ -978,14 +982,13 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
     // ---------------------------------------------------------------- v and w
     const uint32_t leader = elect_leader();
     auto load_vw = [&](int c) {
-      const int row = int(sq.row0) + c * kChunk;
-      mbar_arrive_expect_tx(&sm.full_vw, 2u * 16384u / kParts, leader);
-      tma_load_3d(sm.v, &tm.v, v0, h, row, &sm.full_vw, leader);
-      tma_load_3d(sm.w, &tm.w, v0, h, row, &sm.full_vw, leader);
+      const int row = int(sq.row0) + c * kChunk, slot = c % kVwSlots, at = slot * (16384 / kVwSlots);
+      mbar_arrive_expect_tx(&sm.full_vw[slot], 2u * 16384u / kParts, leader);
+      tma_load_3d(sm.v + at, &tm.v, v0, h, row, &sm.full_vw[slot], leader);
+      tma_load_3d(sm.w + at, &tm.w, v0, h, row, &sm.full_vw[slot], leader);
     };
-    load_vw(0);
-    for (int c = 1; c < n_chunks; ++c) {
-      waiter.wait(&sm.vw_read, uint32_t(c - 1) & 1u);
+    for (int c = 0; c < n_chunks; ++c) {
+      if (c >= kVwSlots) waiter.wait(&sm.vw_read[c % kVwSlots], uint32_t(c / kVwSlots - 1) & 1u);
       load_vw(c);
     }
   } else if (kJoint && warp == W::kWatch) {
@@ -1133,7 +1136,8 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       for (int j = 0; j < 32; ++j) rn[j * kDim] = to_tf32(__uint_as_float(a[j]));
     };
     auto build_z = [&](int c) {
-      waiter.wait(&sm.full_vw, uint32_t(c) & 1u);
+      const int slot = c % kVwSlots, at = slot * (kChunk * kDim / kVwSlots);
+      waiter.wait(&sm.full_vw[slot], uint32_t(c / kVwSlots) & 1u);
       const int n_valid = sq.len - c * kChunk;
       // 16 tokens at a time: more with their activations in flight would not fit the registers
 #pragma unroll
@@ -1142,12 +1146,12 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         float z[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) {
-          z[j] = to_float(wsrc[(16 * part + j) * kRows]);
-          vr[j] = vs[(16 * part + j) * kRows];
+          z[j] = to_float(wsrc[at + (16 * part + j) * kRows]);
+          vr[j] = vs[at + (16 * part + j) * kRows];
         }
         if (part == 1) {
           __syncwarp();
-          if (lane == 0) mbar_arrive(&sm.vw_read);
+          if (lane == 0) mbar_arrive(&sm.vw_read[slot]);
         }
         if (p.activate_w) {
 #pragma unroll
@@ -1208,56 +1212,59 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
 // ---------------------------------------------------------------------------------------------
 // prep and scan in one launch
 // ---------------------------------------------------------------------------------------------
-// With few sequences and heads the scan is a serial chain on a few SMs (1.85 us per chunk) while the others
+// With few sequences and heads the scan is a serial chain on a few SMs (1.6-2 us per chunk) while the others
 // idle, and it starts when the last prep unit is done.  Here some CTAs scan and the others prepare, chunk by
 // chunk; the tiles are still in L2 when the scan reads them.  The scans wait for the preparers, which wait
 // for nobody; the launch is cooperative, so that all CTAs are resident together.
-// The two SMs of a pair share their way to L2: with a preparer beside it a scan took 3.3 us per chunk.  So the
-// CTAs come in clusters of two, the first n_scan clusters scan with one CTA and leave the other idle unless
-// (`mates`) the preparation would be the longer part.
-// Registers: 640 threads x 96 at launch; a preparing CTA gives its two groups of 256 threads 112 each and the
-// four warps left 32 (16 * 112 + 4 * 32 = 20 * 96).
-constexpr int kJointRegs = 96;
+// The two SMs of a pair share their way to L2 (with a preparer beside it a scan took 3.3 us per chunk): the CTAs
+// come in clusters of two, and those of a scanning pair take half of the value rows each.  512 threads leave a
+// preparing group the 128 registers a thread that it has in a launch of its own.  us, against one scanning CTA a
+// pair and 96 registers: B1 T8192 H16 364 -> 233, B1 T32768 H16 1521 -> 820 (raw 1112 -> 960), training B2 T4133
+// H16 329 -> 238, training B1 T2048 H32 170 -> 136.
+constexpr int kJointThreads = 512;
 struct JointSmem {
   PrepSmem prep[2];
 };
 template <typename T, typename G, typename Seqs, bool kPro>
-__global__ void __launch_bounds__(kScanThreadsJoint, 1) __cluster_dims__(2, 1, 1)
+__global__ void __launch_bounds__(kJointThreads, 1) __cluster_dims__(2, 1, 1)
 chunk_joint_kernel(const PrepParams pp, const ScanParams sp, const __grid_constant__ Seqs seqs,
                    const __grid_constant__ PrepMaps tm_prep, const __grid_constant__ ScanMaps tm_scan,
-                   const int mates) {
+                   const int quota) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  const int n_scan = seqs.count() * sp.H, pair = int(blockIdx.x) >> 1, mate = int(blockIdx.x) & 1;
-  if (pair < n_scan && mate == 0) {
-    scan_sequence<T, Seqs, true, 1>(sp, seqs, tm_scan, *reinterpret_cast<ScanSmem*>(smem_raw), pair);
-    return;
+  const int tid = threadIdx.x, n_scan = kJointParts * seqs.count() * sp.H;
+  const bool scans = int(blockIdx.x) < n_scan;
+  if (!scans || quota > 0) {
+    // number of this CTA among those that prepare from the start
+    const int nr = quota > 0 ? int(blockIdx.x) : int(blockIdx.x) - n_scan;
+    const int n_groups = 2 * (quota > 0 ? int(gridDim.x) : int(gridDim.x) - n_scan);
+    JointSmem& sm = *reinterpret_cast<JointSmem*>(smem_raw);
+    if (tid < 32) {
+      tmem_alloc(&sm.prep[0].tmem_base, 512);
+      if (!scans) tmem_relinquish();
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tb = sm.prep[0].tmem_base;
+    const int group = tid >> 8;
+    prep_units<T, G, Seqs, kPro, true>(pp, seqs, tm_prep, sm.prep[group], tid & 255, tb + 256u * group,
+                                       group * (n_groups / 2) + nr, n_groups, 1 + group, sp.status + kQueueWord,
+                                       scans ? quota : 0);
+    tc_fence_before();
+    __syncthreads();
+    if (tid < 32) {
+      tc_fence_after();
+      tmem_dealloc(tb, 512);
+    }
+    if (!scans) return;
+    if ((tid & 255) == 0) {  // the scan's shared memory lies over these
+      for (uint64_t* bar : {&sm.prep[group].bar[0], &sm.prep[group].bar[1], &sm.prep[group].bar_ld[0], &sm.prep[group].bar_ld[1]}) {
+        mbar_inval(bar);
+      }
+    }
+    __syncthreads();
   }
-  if (pair < n_scan && !mates) return;
-  // number of this CTA among those that prepare: whole pairs first
-  const int n_whole = int(gridDim.x) - 2 * n_scan;
-  const int nr = pair < n_scan ? n_whole + pair : int(blockIdx.x) - 2 * n_scan;
-  const int n_groups = 2 * (n_whole + (mates ? n_scan : 0));
-  JointSmem& sm = *reinterpret_cast<JointSmem*>(smem_raw);
-  const int tid = threadIdx.x;
-  if (tid < 32) {
-    tmem_alloc(&sm.prep[0].tmem_base, 512);
-    tmem_relinquish();
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const uint32_t tb = sm.prep[0].tmem_base;
-  if (tid >= 512) {  // (nothing may follow for these warps: code behind a join is compiled for the others' registers)
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 32;");
-    return;
-  }
-  asm volatile("setmaxnreg.inc.sync.aligned.u32 112;");
-  const int group = tid >> 8;
-  prep_units<T, G, Seqs, kPro, true>(pp, seqs, tm_prep, sm.prep[group], tid & 255, tb + 256u * group,
-                                     group * (n_groups / 2) + nr, n_groups, 1 + group, sp.status + kQueueWord);
-  tc_fence_before();
-  asm volatile("bar.sync 3, 512;" ::: "memory");
-  if (tid < 32) tmem_dealloc(tb, 512);
+  scan_sequence<T, Seqs, true, kJointParts>(sp, seqs, tm_scan, *reinterpret_cast<ScanSmem*>(smem_raw), int(blockIdx.x));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1327,11 +1334,17 @@ struct ForwardCall {
 
 thread_local int t_forward_kernels = 0;  // of this thread's latest chunk forward
 
-// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation) and 2-3 us per chunk
-// (the scans); together the longer of the two, the first units taking some 35 us and a scan 0.4 us per chunk
-// more beside preparers.  Beyond a quarter of the SMs scanning, the preparation falls behind.
-bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, int sm_count) {
-  return 4 * n_scan <= sm_count && 83 * n_ch > (350 + 4 * n_chunks) * sm_count && !profiling();
+// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation) and 1.6-2 us per chunk
+// (the scans); together, where the preparers keep the scans' pace or nearly so, the scans' time and some 20 us; with
+// more to scan about n_ch * 8.3 us / SMs and 1 us per chunk, 35 us and what uneven ends cost.  Two launches / one, us:
+//   H16 T1024 53.5/53.8   H16 T2048 95.8/81.3, training 108.9/101.6   H16 T3072 137/108, training 152/136
+//   H8 T4096 140/126, training 164/164   H4 T8192 231/218   H4 T16384 training 517/559 (a training scan beside
+//   preparers takes 2.1 us a chunk, not 1.9)   H24 T1344 training 90/82   H32 T1664 110/111, training 121/116
+// Beyond a quarter of the SMs scanning, the preparation falls behind.
+bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, bool training, int sm_count) {
+  if (4 * n_scan > sm_count || profiling()) return false;
+  if (6 * n_scan <= sm_count) return n_ch >= 400 && (!training || n_scan >= 8);
+  return 83 * n_ch > (350 + 4 * n_chunks) * sm_count;
 }
 
 template <typename T, typename G, typename Seqs, bool kPro>
@@ -1342,25 +1355,24 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   auto kernel = chunk_joint_kernel<T, G, Seqs, kPro>;
   cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  // the register split of the kernel is only valid for the launch allocation it was written for
-  static const int regs = [&] {
-    cudaFuncAttributes attr;
-    return cudaFuncGetAttributes(&attr, kernel) == cudaSuccess ? attr.numRegs : -1;
-  }();
-  if (regs != kJointRegs) return GDN2_ERR_UNSUPPORTED;  // (the caller then takes two launches)
   // the marks of finished units are in D, right before the status block: one fill clears both
   const WsLayout ws{pp.n_ch, pp.training != 0};
   err = cudaMemsetAsync(pp.ws + ws.off_d(), 0, size_t(pp.n_ch) * kBlobD + kStatusBytes, stream);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  const int n_scan = seqs.count() * sp.H;
-  // clusters of two CTAs; no more preparers than pairs of units
-  const int64_t want = n_scan + (pp.n_ch + 3) / 4;
-  const int clusters = int(want < sm_count / 2 ? want : sm_count / 2);
-  // per chunk the scans take 2 us (3 with a preparer beside them), a unit 9.5 us on one SM
-  const int mates = 95 * n_scan > 20 * (2 * (clusters - n_scan)) || clusters == n_scan;
+  const int pairs = seqs.count() * sp.H;
+  // Clusters of two CTAs.  No more preparers than pairs of units, nor than keep ahead of the scans: a unit takes an
+  // SM 9.4 us (raw 12) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way (B1 T32768 H16 817
+  // us with 96, 867 with 116; raw 964 with 104, 1031 with 116).
+  const int64_t paced = (int64_t(pairs) * (pp.prologue != 0 ? 66 : 60) + 19) / 20;
+  const int64_t want = pairs + std::min((pp.n_ch + 3) / 4, paced);
+  const int clusters = int(std::min(want, int64_t(sm_count / 2)));
+  // Where the preparers alone would not keep up, the scanning CTAs first prepare `quota` units for each group of
+  // theirs, so that everybody is done at the same time.
+  const int64_t in_time = int64_t(2 * (clusters - pairs)) * seqs.n_chunks * 28 / 100;
+  const int quota = pp.n_ch > in_time ? int((pp.n_ch - in_time + 2 * clusters) / (4 * clusters)) : 0;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(unsigned(2 * clusters));
-  config.blockDim = dim3(kScanThreadsJoint);
+  config.blockDim = dim3(kJointThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
   cudaLaunchAttribute together;
@@ -1368,7 +1380,7 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   together.val.cooperative = 1;
   config.attrs = &together;
   config.numAttrs = 1;
-  err = cudaLaunchKernelEx(&config, kernel, pp, sp, seqs, tm_prep, tm_scan, mates);
+  err = cudaLaunchKernelEx(&config, kernel, pp, sp, seqs, tm_prep, tm_scan, quota);
   if (err == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs than the device
     (void)cudaGetLastError();
     return GDN2_ERR_UNSUPPORTED;
@@ -1398,8 +1410,10 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
   const int64_t n_scan = int64_t(seqs.count()) * a.H;
   bool joint = false;
-  if constexpr (std::is_same<Seqs, UniformSeqs>::value) joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, sm_count);
-  const int parts = joint ? 1 : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 2);
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
+    joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, a.training != 0, sm_count);
+  }
+  const int parts = joint ? kJointParts : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 2);
   const WsLayout ws{n_ch, a.training != 0};
   int* status = reinterpret_cast<int*>(a.workspace + ws.off_status());
   const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
