@@ -49,6 +49,7 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_chunk_backward": [_P] * 19 + [_I64] * 4 + [_INT, _INT, _F32, _P],
     "gdn2_chunk_backward_f32grads": [_P] * 19 + [_I64] * 4 + [_F32, _P],
     "gdn2_chunk_forward_kernels": [],
+    "gdn2_chunk_backward_kernels": [],
     "gdn2_chunk_read_status": [_P] + [_I64] * 3 + [_P],
     "gdn2_debug_wait_expires": [_P] + [_I64] * 4 + [_P],
     "gdn2_token_forward_fused": [_P] * 9 + [_I64] * 5 + [_INT, _INT, _F32, _INT, _P],
@@ -168,9 +169,9 @@ LAUNCHES = [0]
 KERNEL_EVENTS: dict[str, list] | None = None
 
 
-# kernels launched by one successful call of each entry point (default 1); a chunk forward says it itself
-_KERNELS_PER_CALL = {"gdn2_chunk_backward": 2, "gdn2_chunk_backward_f32grads": 2}
+# kernels launched by one successful call of each entry point: 1, or what a chunk call says itself
 _CHUNK_FORWARDS = ("gdn2_chunk_forward", "gdn2_chunk_forward_fused", "gdn2_chunk_forward_static")
+_CHUNK_BACKWARDS = ("gdn2_chunk_backward", "gdn2_chunk_backward_f32grads")
 
 
 def check(status: int, what: str, kernels: int | None = None) -> None:
@@ -179,7 +180,7 @@ def check(status: int, what: str, kernels: int | None = None) -> None:
     if status == 0:
         if kernels is None:
             kernels = (lib().gdn2_chunk_forward_kernels() if what in _CHUNK_FORWARDS
-                       else _KERNELS_PER_CALL.get(what, 1))
+                       else lib().gdn2_chunk_backward_kernels() if what in _CHUNK_BACKWARDS else 1)
         LAUNCHES[0] += kernels
         return
     handle = lib()

@@ -51,7 +51,7 @@ constexpr int64_t kStateElems = int64_t(kDim) * kDim;
 // places of others, see ScanWarps in chunk_fwd.cu.)
 template <int kParts>
 struct BScanWarps {
-  static constexpr int kDo0 = 8, kLoads = kParts > 1 ? 2 : 16, kMma = kParts > 1 ? 3 : 18;
+  static constexpr int kDo0 = 8, kLoads = kParts > 1 ? 2 : 16, kMma = kParts > 1 ? 3 : 18, kMark = 6;
   static constexpr int kThreads = kParts > 1 ? 512 : 608;
   static __device__ __forceinline__ bool works(int warp) { return warp < 16 && (warp & 3) < 4 / kParts; }
 };
@@ -76,9 +76,23 @@ struct BScanSmem {
   uint64_t do_read;   // dO is in registers:                                 8 warps
   uint64_t a_done, k_done, z_done, do_done, s_done;  // MMA commits
   volatile int failed;
+  volatile int stored[4], sent;  // joint launch: steps whose cotangents (by warp) and dZ are in memory
   uint32_t tmem_base;
 };
 static_assert(sizeof(BScanSmem) <= 232448, "reverse scan exceeds the 227 KiB shared-memory limit");
+
+// Joint launch: the last 16 bytes of a dZ tile, behind its last row, belong to nobody.  Word 0 counts the CTAs
+// of the scan that have left in memory what the VJP reads of the unit; the first unit's word 1 is the queue of units.
+constexpr int64_t kMarkOffset = kBlobDZ - 16;
+struct Marks {
+  uint8_t* dz;
+  __device__ __forceinline__ unsigned* of(int64_t ch) const {
+    return reinterpret_cast<unsigned*>(dz + ch * kBlobDZ + kMarkOffset);
+  }
+  __device__ __forceinline__ void arrive(int64_t ch) const {
+    asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(of(ch)) : "memory");
+  }
+};
 
 struct BScanParams {
   const uint8_t* d;         // chunk-end decays, 512 bytes per unit
@@ -88,22 +102,23 @@ struct BScanParams {
   float* ds_init;           // [sequences,H,128,128] or null
   int* status;
   int H;
+  Marks marks;              // joint launch
 };
 struct BScanMaps {
   CUtensorMap at, tt, kn, q, yt, d_out;
 };
 
-template <typename T, typename Seqs, int kParts>
-__global__ void __launch_bounds__(BScanWarps<kParts>::kThreads, 1)
-chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  BScanSmem& sm = *reinterpret_cast<BScanSmem*>(smem_raw);
+// One sequence and head, or a part of its value rows (value_parts), by a whole CTA.  kJoint: the VJP of finished
+// chunks runs beside in the same launch, and this CTA joins it afterwards.
+template <typename T, typename Seqs, bool kJoint, int kParts>
+__device__ __forceinline__ void reverse_sequence(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm,
+                                                 BScanSmem& sm, const int item) {
   BoundedWaiter waiter(p.status, 1u << 20, &sm.failed);
 
   using W = BScanWarps<kParts>;
   constexpr int kRows = kDim / kParts;  // value rows of this CTA: lanes 0 .. kRows - 1 of tensor memory
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int unit = int(blockIdx.x) / kParts, v0 = (int(blockIdx.x) - unit * kParts) * kRows;
+  const int unit = item / kParts, v0 = (item - unit * kParts) * kRows;
   const int s = unit / p.H, h = unit - s * p.H;
   const SeqInfo sq = seqs.at(s);
   const int n_chunks = sq.n_chunks;
@@ -114,7 +129,7 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
 
   if (warp == W::kMma) {
     tmem_alloc(&sm.tmem_base, 512);
-    tmem_relinquish();
+    if (!kJoint) tmem_relinquish();
   }
   if (tid == 0) {
     uint64_t* one[] = {&sm.full_o, &sm.full_d[0], &sm.full_d[1], &sm.full_k, &sm.full_y, &sm.a_done, &sm.k_done,
@@ -125,6 +140,8 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
     mbar_init(&sm.go_q, 1 + 8 / kParts);
     mbar_init(&sm.go_z, 1 + 8 / kParts);
     mbar_init(&sm.do_read, 8 / kParts);
+    for (int i = 0; i < 4; ++i) sm.stored[i] = 0;
+    sm.sent = 0;
     // a wait that ran out earlier (forward or backward) left garbage behind: results become NaN
     sm.failed = *static_cast<volatile const int*>(p.status) != kStatusOk;
     fence_mbar_init();
@@ -257,6 +274,18 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       mma_commit(&sm.z_done, leader);
       if (it + 1 < n_chunks) issue_a(it + 1);
     }
+  } else if (kJoint && warp == W::kMark) {
+    // ---------------------------------------------------------------- marks of finished units
+    // a warp of its own: what a mark has to wait for would hold up the others for half of a chunk's time
+    for (int it = 0; it < n_chunks; ++it) {
+      const volatile int* mine = lane < 4 ? &sm.stored[lane] : &sm.sent;
+      // (the other warps of the scan give up by themselves)
+      for (uint32_t looks = 0; !__all_sync(0xffffffffu, *mine > it) && looks < (1u << 27); ++looks) __nanosleep(40);
+      __threadfence_block();
+      // (the VJP reads through the copy engine, another proxy than the stores)
+      fence_async_all();
+      if (lane == 0) p.marks.arrive(ch_of(it));
+    }
   } else if (!W::works(warp)) {
     // (nothing to do in this form)
   } else if (warp < W::kDo0) {
@@ -341,6 +370,11 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
           ck[j * kDim] = __uint_as_float(lo[j]);
           ck[(32 + j) * kDim] = __uint_as_float(hi[j]);
         }
+        if constexpr (kJoint) {
+          __threadfence_block();
+          __syncwarp();
+          if (lane == 0) sm.stored[2 * half + q4] = it + 1;
+        }
       }
     }
     // ---- cotangent of the initial state: slot 0 and d_initial_state ----------------------------------
@@ -399,7 +433,15 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
       if (it + 1 < n_chunks) arrive(&sm.go_z);
       // dZ out: 32 token columns of value row v into the staging tile X[r = j][c = v], one bulk store
       const bool failed = sm.failed != 0;
-      if (sender) bulk_wait_read_all();  // the previous tile has left the staging buffer
+      if (sender) {
+        if constexpr (kJoint) {
+          bulk_wait_all();  // the previous tile is in memory, long since
+          __threadfence_block();
+          sm.sent = it;
+        } else {
+          bulk_wait_read_all();  // the previous tile has left the staging buffer
+        }
+      }
       group_barrier();
 #pragma unroll
       for (int jj = 0; jj < 32; ++jj) {
@@ -417,13 +459,19 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
 #pragma unroll
           for (int jg = 0; jg < 8; ++jg) {
             const int at = jg * kRsZ + (v0 >> 2) * kCsZ;
-            bulk_s2g(dst + at, sm.dz + at, uint32_t(kRows / 4 * kCsZ));
+            bulk_s2g(dst + at, sm.dz + at, uint32_t(kRows / 4 * kCsZ - 16));
           }
         }
         bulk_commit();
       }
     }
-    if (sender) bulk_wait_all();  // the last dZ tile is in global memory before the CTA retires
+    if (sender) {
+      bulk_wait_all();  // the last dZ tile is in global memory before the CTA retires
+      if constexpr (kJoint) {
+        __threadfence_block();
+        sm.sent = n_chunks;
+      }
+    }
   }
   tc_fence_before();
   __syncthreads();
@@ -431,6 +479,16 @@ chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, co
     tc_fence_after();
     tmem_dealloc(tb, 512);
   }
+  if (kJoint && tid == 0) {  // other shared memory lies over these from here on
+    for (uint64_t* bar = &sm.full_o; bar <= &sm.s_done; ++bar) mbar_inval(bar);
+  }
+}
+
+template <typename T, typename Seqs, int kParts>
+__global__ void __launch_bounds__(BScanWarps<kParts>::kThreads, 1)
+chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  reverse_sequence<T, Seqs, false, kParts>(p, seqs, tm, *reinterpret_cast<BScanSmem*>(smem_raw), int(blockIdx.x));
 }
 
 
@@ -483,6 +541,9 @@ struct VjpMisc {
   float xt[4][kDim];      // partial sums of dd = sum_v dS_1 * S_0, then the per-block sums of dG
   alignas(8) uint64_t bar_a, bar_s, bar_r, bar_m, bar_d;
   uint32_t tmem_base;
+  int next[2], ready[2];  // joint launch: the unit after this one, and whether the scan is done with it (two slots:
+                          // one may still be read)
+  int failed;             // joint launch: a wait of the scan ran out, or the wait for it
 };
 constexpr int kVjpSmemBytes = kOffMisc + int(sizeof(VjpMisc));
 static_assert(kVjpSmemBytes <= 232448, "VJP kernel exceeds the 227 KiB shared-memory limit");
@@ -501,6 +562,8 @@ struct VjpParams {
   int64_t n_ch;
   int H;
   float scale;
+  Marks marks;          // joint launch
+  unsigned marks_full;  // CTAs that mark a unit
 };
 // tensor maps of the seven sequence tensors the VJP kernel reads (for L2 prefetches only)
 struct VjpInputMaps {
@@ -577,14 +640,17 @@ __device__ __forceinline__ void tmem_ld4x2(uint32_t taddr, float2 (&x)[4]) {
 // their final rounding; used by tests to judge the arithmetic apart from the 16-bit cast).
 // kRagged: some sequence length is not a multiple of 64, its last chunk is partial; only this
 // instantiation carries the guards (they cost the others 6 %; a packed step of H16, 8192 tokens 1 %).
-template <typename T, typename G, typename Seqs, bool kF32Grads = false, bool kRagged = false>
-__global__ void __launch_bounds__(kVjpThreads, 1)
-chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ CUtensorMap tm_s0,
-                     const __grid_constant__ CUtensorMap tm_ds, const __grid_constant__ CUtensorMap tm_rn,
-                     const __grid_constant__ CUtensorMap tm_dq, const __grid_constant__ CUtensorMap tm_dk,
-                     const __grid_constant__ CUtensorMap tm_dbeta, const __grid_constant__ VjpInputMaps tm_in) {
+// kJoint: units come from a queue in the order in which the scans that run beside finish them, and what the scans
+// write of a unit is loaded once their marks are there.
+struct VjpMaps {
+  CUtensorMap s0, ds, rn, dq, dk, dbeta;
+  VjpInputMaps in;
+};
+template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged, bool kJoint>
+__device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, const VjpMaps& tm, uint8_t* smem) {
   using O = typename std::conditional<kF32Grads, float, T>::type;  // element type of dq, dk, dv, dbeta, dw
-  extern __shared__ __align__(1024) uint8_t smem[];
+  const CUtensorMap &tm_s0 = tm.s0, &tm_ds = tm.ds, &tm_rn = tm.rn, &tm_dq = tm.dq, &tm_dk = tm.dk, &tm_dbeta = tm.dbeta;
+  const VjpInputMaps& tm_in = tm.in;
   VjpMisc& ms = *reinterpret_cast<VjpMisc*>(smem + kOffMisc);
   const ScratchLayout sc{p.n_ch};
   BoundedWaiter waiter(p.status);
@@ -638,20 +704,63 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
     tma_load_4d(smem + kOffS0, &tm_s0, 0, 0, 0, slot_, &ms.bar_s);
     mbar_arrive_expect_tx(&ms.bar_a, uint32_t(kBlobDZ + kBlobRn));
     tma_load_4d(smem + kOffRn, &tm_rn, 0, 0, 0, int(ch_), &ms.bar_a);
+  };
+  auto issue_dz = [&](int64_t ch_) {
     bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + ch_ * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
   };
   auto issue_ds1 = [&](int slot_) {
     tma_load_4d(smem + kOffDs1, &tm_ds, 0, 0, 0, slot_ + p.H, &ms.bar_s);
   };
-  if (tid == 0 && int64_t(blockIdx.x) < p.n_ch) {
-    const int slot_ = locate(blockIdx.x).slot;
-    issue_loads(blockIdx.x, slot_);
+  // joint launch: the next unit of the queue, last chunks first; have the scans finished it (a look, or a wait)
+  auto pop = [&] {
+    const unsigned u = atomicAdd(p.marks.of(0) + 1, 1u);
+    if (u >= unsigned(p.n_ch)) return int(p.n_ch);
+    const unsigned per_chunk = unsigned(seqs.count()) * unsigned(p.H), step = u / per_chunk, r = u - step * per_chunk;
+    const SeqInfo sq = seqs.at(int(r / unsigned(p.H)));
+    return (sq.chunk0 + sq.n_chunks - 1 - int(step)) * p.H + int(r % unsigned(p.H));
+  };
+  auto finished = [&](int64_t ch_) {
+    unsigned x;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p.marks.of(ch_)) : "memory");
+    if (x != p.marks_full) return false;
+    fence_async_all();
+    // (a wait of the scan that ran out: gradients become NaN)
+    if (*static_cast<volatile const int*>(p.status) != kStatusOk) ms.failed = 1;
+    return true;
+  };
+  auto await = [&](int64_t ch_) {
+    while (!finished(ch_)) {
+      if (!waiter.look_again()) {
+        ms.failed = 1;
+        break;
+      }
+      __nanosleep(100);
+    }
+  };
+  int64_t first = blockIdx.x;
+  if constexpr (kJoint) {
+    if (tid == 0) {
+      ms.failed = 0;
+      ms.next[0] = pop();
+    }
+    __syncthreads();
+    first = ms.next[0];
+    __syncthreads();
+  }
+  if (tid == 0 && first < p.n_ch) {
+    const int slot_ = locate(first).slot;
+    issue_loads(first, slot_);
+    if constexpr (kJoint) await(first);
+    issue_dz(first);
     issue_ds1(slot_);
   }
 
   uint32_t iter = 0;
-  for (int64_t ch = blockIdx.x; ch < p.n_ch; ch += gridDim.x, ++iter) {
+  for (int64_t ch = first, ch_next; ch < p.n_ch; ch = ch_next, ++iter) {
   const uint32_t par = iter & 1u;
+  ch_next = ch + gridDim.x;
+  int popped = 0;
+  if (kJoint && tid == 96) popped = pop();
   const Place at = locate(ch);
   const int h = at.h;
   auto seq_idx = [&](int tok) { return (int64_t(at.row + tok) * p.H + h) * int64_t(kDim); };
@@ -721,12 +830,14 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
     }
   }
   *reinterpret_cast<float4*>(&ms.part[tg][kc0]) = make_float4(Gc[3][0], Gc[3][1], Gc[3][2], Gc[3][3]);
+  if (kJoint && tid == 96) ms.next[par] = popped;
   waiter.wait(&ms.bar_a, par);
   waiter.wait(&ms.bar_s, par);
   dd_half(0);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
+  if constexpr (kJoint) ch_next = ms.next[par];
   // ---- first MMA batch: M4 (first half) dKt^T = dS_1[:, v < 64] R[:, v < 64]^T ;
   //      M2 [-dL ; dA] = [dZ ; dO] R^T ;  M3 [-dE ; dQg]^T = S_0 [dZ ; dO]^T ------------------------------
   if (warp == 0) {
@@ -801,7 +912,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
       for (int e = 0; e < 4; ++e) {
         const int j = 4 * tg + e;
         float4 dz = *reinterpret_cast<const float4*>(smem + kOffStack + (j >> 3) * kRsN + c4 * kCsN + (j & 7) * 16);
-        if (upstream_failed || waiter.dead) dz = make_float4(poison_nan(), poison_nan(), poison_nan(), poison_nan());
+        if (upstream_failed || waiter.dead || (kJoint && ms.failed != 0)) dz = make_float4(poison_nan(), poison_nan(), poison_nan(), poison_nan());
         const int64_t idx = seq_idx(j) + kc0;
         float wv[4], vv[4];
         unpack4<T>(wr[e], wv);
@@ -819,13 +930,15 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   // bytes in flight over the latency: have its seven [64][128] tiles brought into L2, the four that are read
   // first from here on and the others with the tile copies.  (All behind the tile copies they wait for those
   // in the copy engine: B4 T8192 H32 1.72 ms against 1.63; all from here, ragged lengths lose 2 %.)
-  if (tid == 64 && ch + gridDim.x < p.n_ch) {
-    const Place nx = locate(ch + gridDim.x);
+  if (tid == 64 && ch_next < p.n_ch) {
+    const Place nx = locate(ch_next);
     tma_prefetch_l2_3d(&tm_in.d_out, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.g, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.w, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.v, 0, nx.h, nx.row);
   }
+  // (where all wait for the tensor cores anyway: a look takes 1500 clocks)
+  if (kJoint && tid == 96) ms.ready[par] = ch_next < p.n_ch && finished(ch_next);
   // ---- M4 (second half) once the second half of dS_1 has landed -----------------------------------------
   waiter.wait(&ms.bar_d, par);
   dd_half(1);
@@ -973,9 +1086,14 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   ++mma_phase;
   tc_fence_after();
   // shared memory (all but the small arrays of VjpMisc) is dead from here on: fetch the next chunk-head
-  if (tid == 0 && ch + gridDim.x < p.n_ch) issue_loads(ch + gridDim.x, locate(ch + gridDim.x).slot);
-  if (tid == 64 && ch + gridDim.x < p.n_ch) {  // (see the other prefetches above)
-    const Place nx = locate(ch + gridDim.x);
+  bool pending = false;  // (what the scan writes of the next unit is not there yet)
+  if (tid == 0 && ch_next < p.n_ch) {
+    issue_loads(ch_next, locate(ch_next).slot);
+    pending = kJoint && ms.ready[par] == 0;
+    if (!pending) issue_dz(ch_next);
+  }
+  if (tid == 64 && ch_next < p.n_ch) {  // (see the other prefetches above)
+    const Place nx = locate(ch_next);
     tma_prefetch_l2_3d(&tm_in.k, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.q, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.beta, 0, nx.h, nx.row);
@@ -1001,7 +1119,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   // the row and column contributions of the Gram products to dG then cancel as they do exactly.
   {
     const int kc = tid & 127, blk = part;
-    const bool failed = upstream_failed || waiter.dead;
+    const bool failed = upstream_failed || waiter.dead || (kJoint && ms.failed != 0);
     const float gend = ms.gend[kc];
     // dd[k] = sum_v dS_1[k][v] S_0[k][v]: read here, before xt is reused for the block sums of dG
     const float dd_k = (ms.xt[0][kc] + ms.xt[1][kc]) + (ms.xt[2][kc] + ms.xt[3][kc]);
@@ -1162,11 +1280,50 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
       bulk_commit();
     }
     // the G tile is dead: the dS_1 half of the next chunk-head may land on it
-    if (ch + gridDim.x < p.n_ch) issue_ds1(locate(ch + gridDim.x).slot);
+    if (ch_next < p.n_ch) {
+      if (pending) {
+        await(ch_next);
+        issue_dz(ch_next);
+      }
+      issue_ds1(locate(ch_next).slot);
+    }
   }
   }  // chunk-head loop
   if (tid == 0) bulk_wait_all();  // the last dq / dk tiles are in global memory before the CTA retires
   if (warp == 0) tmem_dealloc(tb, 512);
+}
+
+template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
+__global__ void __launch_bounds__(kVjpThreads, 1)
+chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ VjpMaps tm) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  vjp_units<T, G, Seqs, kF32Grads, kRagged, false>(p, seqs, tm, smem_raw);
+}
+
+// =============================================================================================
+// reverse scan and VJP in one launch
+// =============================================================================================
+// With few sequences and heads the reverse scan keeps a few SMs busy, 1.9-2.2 us per chunk, and the VJP of a chunk
+// needs nothing but that chunk's share of it.  Here the scans run on pairs of CTAs (a half of the value rows each) and
+// all other CTAs, and at last these too, take the units from a queue, last chunks first, waiting for the scans'
+// marks.  The scans wait for nobody; the launch is cooperative, so that all CTAs are resident together.  A unit's
+// scratch tiles and cotangents are still in L2 when the VJP reads them.  Whatever waits for memory on behalf of a mark
+// is kept off the scan's chain and the VJP's: by the scanning warps themselves it cost a chunk 1.2 us, by the thread
+// that issues the VJP's copies a unit 1500 clocks.
+constexpr int kJointParts = 2;
+template <typename T, typename G, bool kRagged>
+__global__ void __launch_bounds__(kVjpThreads, 1) __cluster_dims__(2, 1, 1)
+chunk_bwd_joint_kernel(const BScanParams sp, const VjpParams vp, const __grid_constant__ UniformSeqs seqs,
+                       const __grid_constant__ BScanMaps tm_scan, const __grid_constant__ VjpMaps tm_vjp) {
+  static_assert(BScanWarps<kJointParts>::kThreads == kVjpThreads, "a scanning CTA goes on with the VJP");
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if (int(blockIdx.x) < kJointParts * seqs.count() * sp.H) {
+    reverse_sequence<T, UniformSeqs, true, kJointParts>(sp, seqs, tm_scan, *reinterpret_cast<BScanSmem*>(smem_raw),
+                                                        int(blockIdx.x));
+    fence_async_smem();
+    __syncthreads();
+  }
+  vjp_units<T, G, UniformSeqs, false, kRagged, true>(vp, seqs, tm_vjp, smem_raw);
 }
 
 }  // namespace
@@ -1189,11 +1346,6 @@ struct BackwardCall {
   bool ragged;      // some last chunk is partial
 };
 
-struct VjpMaps {
-  CUtensorMap s0, ds, rn, dq, dk, dbeta;
-  VjpInputMaps in;
-};
-
 template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
 int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStream_t stream) {
   auto kernel = chunk_bwd_vjp_kernel<T, G, Seqs, kF32Grads, kRagged>;
@@ -1202,7 +1354,7 @@ int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStrea
   int sm_count = 0;
   if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
   const unsigned grid = unsigned(p.n_ch < int64_t(sm_count) ? p.n_ch : int64_t(sm_count));
-  kernel<<<grid, kVjpThreads, kVjpSmemBytes, stream>>>(p, seqs, m.s0, m.ds, m.rn, m.dq, m.dk, m.dbeta, m.in);
+  kernel<<<grid, kVjpThreads, kVjpSmemBytes, stream>>>(p, seqs, m);
   return check_launch();
 }
 
@@ -1217,6 +1369,46 @@ int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, in
   const int threads = parts > 1 ? BScanWarps<2>::kThreads : BScanWarps<1>::kThreads;
   kernel<<<unsigned(n_scan * parts), threads, smem, stream>>>(p, seqs, tm);
   return check_launch();
+}
+
+thread_local int t_backward_kernels = 0;  // of this thread's latest chunk backward
+
+// One launch for both where it gains: at most a quarter of the SMs with a scan, as in the forward, and sequences long
+// enough for the VJP to run behind it.  Training steps with two launches / one, us: H16 T1024 157/154, T2048 228/210,
+// T8192 719/624; H8 T4096 336/309; H4 T8192 537/521; H24 T4096 467/445; H32 T2048 318/312, B2 T4133 H16 (fp16)
+// 619/581; H37 T1024 201/209.  With one or two scans all that the launch could hide is a few units, and quarters of
+// the value rows, which only the scan kernel has, are worth more.
+bool prefer_joint_backward(int64_t n_scan, int64_t n_chunks, int sm_count) {
+  return 4 * n_scan <= sm_count && n_scan >= 4 && n_chunks >= 32 && !profiling();
+}
+
+template <typename T, typename G, bool kRagged>
+int launch_joint(const BScanParams& sp, const VjpParams& vp, const UniformSeqs& seqs, const BScanMaps& tm_scan,
+                 const VjpMaps& tm_vjp, int sm_count, cudaStream_t stream) {
+  constexpr int smem = int(sizeof(BScanSmem)) > kVjpSmemBytes ? int(sizeof(BScanSmem)) : kVjpSmemBytes;
+  auto kernel = chunk_bwd_joint_kernel<T, G, kRagged>;
+  cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  err = cudaMemset2DAsync(vp.marks.dz + kMarkOffset, kBlobDZ, 0, 16, size_t(vp.n_ch), stream);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  const int64_t want = int64_t(seqs.count()) * sp.H + (vp.n_ch + 1) / 2;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(2 * unsigned(want < sm_count / 2 ? want : sm_count / 2));
+  config.blockDim = dim3(kVjpThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute together;
+  together.id = cudaLaunchAttributeCooperative;
+  together.val.cooperative = 1;
+  config.attrs = &together;
+  config.numAttrs = 1;
+  err = cudaLaunchKernelEx(&config, kernel, sp, vp, seqs, tm_scan, tm_vjp);
+  if (err == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs than the device
+    (void)cudaGetLastError();
+    return GDN2_ERR_UNSUPPORTED;
+  }
+  if (err != cudaSuccess) { (void)cudaGetLastError(); record_cuda_error(err); return GDN2_ERR_LAUNCH; }
+  return GDN2_OK;
 }
 
 template <typename Seqs>
@@ -1234,7 +1426,11 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
   int sm_count = 0;
   if (int err = multiprocessors(&sm_count); err != GDN2_OK) return err;
   const int64_t n_scan = int64_t(seqs.count()) * a.H;
-  const int parts = value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 4);
+  bool joint = false;
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
+    joint = !a.grads_f32 && prefer_joint_backward(n_scan, seqs.n_chunks, sm_count);
+  }
+  const int parts = joint ? kJointParts : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 4);
   // the reverse scan's operands: the forward's tiles, each in the swizzle of the role backward reads it in
   BScanMaps tm;
   if (!encode_tile_map(&tm.at, a.workspace + ws.off_at(), n_ch, kChunk, kChunk, false, 32, 1) ||
@@ -1245,13 +1441,9 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
       !encode_sequence_map(&tm.d_out, a.d_out, a.rows, a.H, a.dtype, kChunk, kDim / parts)) {
     return GDN2_ERR_LAUNCH;
   }
+  const Marks marks{a.scratch + sc.off_dz()};
   const BScanParams sp{a.workspace + ws.off_d(), a.scratch + sc.off_dz(), a.ds_final, a.d_bnd, a.ds_init, status,
-                       int(a.H)};
-  int st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)
-                                : launch_bscan<__half>(sp, seqs, tm, n_scan, parts, stream);
-  if (st != GDN2_OK) return st;
-  profile_mark(4, stream);
-
+                       int(a.H), marks};
   // dq, dk and dbeta leave the VJP kernel through tiled TMA stores; the maps of the inputs serve prefetches
   VjpMaps m;
   const int grad_dtype = a.grads_f32 ? GDN2_FP32 : a.dtype;
@@ -1271,7 +1463,24 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
     return GDN2_ERR_LAUNCH;
   }
   const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.dq, a.dk, a.dv, a.dg,
-                     a.dbeta, a.dw, status, n_ch, int(a.H), a.scale};
+                     a.dbeta, a.dw, status, n_ch, int(a.H), a.scale, marks, kJointParts};
+  int st = GDN2_ERR_UNSUPPORTED;
+  if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
+    if (joint) {
+      GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
+        st = a.ragged ? launch_joint<T, G, true>(sp, vp, seqs, tm, m, sm_count, stream)
+                      : launch_joint<T, G, false>(sp, vp, seqs, tm, m, sm_count, stream);
+      });
+      if (st != GDN2_ERR_UNSUPPORTED) {
+        t_backward_kernels = 1;
+        return st;
+      }
+    }
+  }
+  st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)
+                            : launch_bscan<__half>(sp, seqs, tm, n_scan, parts, stream);
+  if (st != GDN2_OK) return st;
+  profile_mark(4, stream);
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     if (a.grads_f32) {
       st = a.ragged ? launch_vjp<__nv_bfloat16, float, Seqs, true, true>(vp, seqs, m, stream)
@@ -1285,10 +1494,13 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
     });
   }
   profile_mark(5, stream);
+  t_backward_kernels = 2;
   return st;
 }
 
 }  // namespace
+
+int chunk_backward_kernels() { return t_backward_kernels; }
 
 int launch_chunk_backward(const void* q, const void* k, const void* v, const void* g, const void* beta,
                           const void* w, const void* d_out, const float* ds_final, const float* bnd,

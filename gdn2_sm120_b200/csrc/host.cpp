@@ -32,6 +32,7 @@ struct Api {
   decltype(&gdn2_chunk_forward_fused) chunk_forward_fused;
   decltype(&gdn2_chunk_forward_kernels) chunk_forward_kernels;
   decltype(&gdn2_chunk_backward) chunk_backward;
+  decltype(&gdn2_chunk_backward_kernels) chunk_backward_kernels;
   decltype(&gdn2_chunk_workspace_bytes) chunk_workspace_bytes;
   decltype(&gdn2_chunk_scratch_bytes) chunk_scratch_bytes;
   decltype(&gdn2_gate_prologue) gate_prologue;
@@ -422,7 +423,7 @@ PyObject* train_backward(PyObject*, PyObject* const* a, Py_ssize_t n) {
   }
   others.end();
   if (chunked) {
-    if (!ok(status, "gdn2_chunk_backward", 2)) return nullptr;
+    if (!ok(status, "gdn2_chunk_backward", api.chunk_backward_kernels())) return nullptr;
   } else if (!ok(scan_status, "gdn2_token_dstate_scan", 1) || !ok(status, "gdn2_token_chunk_vjp", 1)) {
     return nullptr;
   }
@@ -543,6 +544,7 @@ PyObject* bind(PyObject*, PyObject* const* a, Py_ssize_t n) {
   GDN2_BIND(chunk_forward_fused);
   GDN2_BIND(chunk_forward_kernels);
   GDN2_BIND(chunk_backward);
+  GDN2_BIND(chunk_backward_kernels);
   GDN2_BIND(chunk_workspace_bytes);
   GDN2_BIND(chunk_scratch_bytes);
   GDN2_BIND(gate_prologue);

@@ -208,6 +208,9 @@ int gdn2_chunk_forward(const void* q, const void* k, const void* v, const void* 
  */
 int gdn2_chunk_forward_kernels(void);
 
+/* The same of its latest chunk backward: 2, the reverse scan and the VJP, or 1. */
+int gdn2_chunk_backward_kernels(void);
+
 /*
  * Chunkwise backward over tokens [0, full_tokens): reverse scan of the state cotangent plus
  * the compact-WY chunk VJP, from what gdn2_chunk_forward(training = 1) saved.  Replaces

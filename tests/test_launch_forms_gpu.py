@@ -92,6 +92,31 @@ def test_joint_launch_equals_two_launches(dtype, g_dtype, raw):
     assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
 
 
+# (four scans at least, a quarter of the SMs at most, 32 chunks: the smallest and widest grids, one chunk less, and
+# ragged ends of 1 and 63 tokens)
+@pytest.mark.parametrize("batch,heads,time,kernels", [(1, 4, 32 * 64, 1), (1, 3, 32 * 64, 2), (2, 16, 31 * 64, 2),
+                                                      (2, 16, 32 * 64 + 1, 1), (1, 37, 32 * 64 + 63, 1)])
+@pytest.mark.parametrize("dtype,g_dtype", [(torch.bfloat16, torch.float32), (torch.float16, torch.float16)])
+def test_joint_backward_equals_two_launches_and_the_oracle(batch, heads, time, kernels, dtype, g_dtype):
+    tensors, d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
+    tensors = [t.to(g_dtype if i == 3 else dtype) for i, t in enumerate(tensors[:6])] + [tensors[6]]
+    d_out = d_out.to(dtype)
+    launched = _lib.LAUNCHES[0]
+    full = _step(tensors, d_out, d_fin)
+    assert _lib.LAUNCHES[0] - launched == _lib.lib().gdn2_chunk_forward_kernels() + kernels
+    again = _step(tensors, d_out, d_fin)  # (a second call finds other memory, or the first one's marks)
+    _lib.profile_enable(True)  # times the kernels one by one: never joint
+    try:
+        apart = _step(tensors, d_out, d_fin)
+    finally:
+        _lib.profile_enable(False)
+    for other in (again, apart):
+        assert torch.equal(full[0], other[0]) and torch.equal(full[1], other[1])
+        assert all(torch.equal(a, b) for a, b in zip(full[2], other[2]))
+    if dtype == torch.bfloat16:
+        _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
+
+
 # 255 .. 257 and 513: around one and two launch tables of 256 sequences
 @pytest.mark.parametrize("count", [255, 256, 257, 513])
 def test_packed_batches_around_the_table_size(count):
