@@ -9,7 +9,7 @@
 //                       cumulative log-decay, block-anchored Gram products on tf32 tcgen05 MMAs,
 //                       blocked inverse T of the unit lower-triangular system on CUDA cores (fp32),
 //                       Y = T E on tf32 tcgen05 MMAs.
-//   chunk_scan_kernel   one CTA per (sequence, head), chunks in order.  The state lives transposed
+//   chunk_scan_kernel   one CTA per (sequence, head) or half of its value rows, chunks in order.  The state lives transposed
 //                       (S^T: value rows x key columns) in TMEM as the fp32 accumulator and is fed
 //                       back as the tf32 A operand of the next MMAs without leaving TMEM:
 //                           R^T  = Z^T T^T - S^T Y^T           (Z = w v)
@@ -18,7 +18,7 @@
 //                       The B operands are the prep kernel's row-major tiles, brought in by tiled
 //                       TMA loads in the swizzled layout of their role (chunk_common.cuh).
 //   chunk_joint_kernel  where few sequences and heads leave most SMs without a scan: some CTAs scan
-//                       while the others prepare, chunk by chunk.
+//                       (after helping to prepare) while the others prepare, chunk by chunk.
 //
 // Math per chunk (reference: src/gdn2_sm120/reference.py:149-172, chunk.py:188-331, with the
 // chunk length re-chosen as 64 and the decay normalisation anchored per 16-token block so that
@@ -412,14 +412,17 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   float* Tc = reinterpret_cast<float*>(R + kOffTc);           // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
   float* Ln = reinterpret_cast<float*>(R + kOffLn);           // [64][kLd]   L
   float* Wt = reinterpret_cast<float*>(R + kOffWt);           // [2][16][kLdW] block products, transposed
+  // L (rows 0..63) goes into fp32 scratch, A_qk (rows 64..127) into the workspace; the two warps of a quadrant take 32
+  // columns each.  A_qk is stored behind the barrier, beside the first step of the inverse, which its warps have no
+  // part in: the stores queue behind those of the rounds, and the inverse would wait for them.  (With the diagonal
+  // blocks column by column, below: B8 T4096 H16 455 -> 450 us, B4 T8192 H32 training 892 -> 881.)
+  const int gram_row = 32 * q4 + lane;  // TMEM lane = row of [E_a ; Q_a]
+  float a_qk[2][16];
   {
-    // pull L (rows 0..63) into fp32 scratch and A_qk (rows 64..127) into the workspace;
-    // the two warps of a quadrant take 32 columns each
-    const int r = 32 * q4 + lane;  // TMEM lane = row of [E_a ; Q_a]
+    const int r = gram_row;
     const int i = r & 63;
     const int I_lo = (q4 & 1) * 2;
     const int my_I = I_lo + (lane >> 4);
-    float* tile_at = reinterpret_cast<float*>(p.tiles.at + int64_t(ch) * kTileAt);
 #pragma unroll
     for (int sub = 0; sub < 2; ++sub) {
       const int c0 = 32 * part + 16 * sub;
@@ -428,7 +431,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
       if (need_lo) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo) + c0), lo);
       if (need_hi) tmem_ld16(tmem_addr(tb, 32 * q4, gram_col(I_lo + 1) + c0), hi);
       tmem_wait_ld();
-      float vals[16];
+      float (&vals)[16] = a_qk[sub];
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         const bool mine_lo = (my_I == I_lo);
@@ -442,16 +445,20 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
           *reinterpret_cast<float4*>(Ln + i * kLd + c0 + 4 * j4) =
               make_float4(vals[4 * j4], vals[4 * j4 + 1], vals[4 * j4 + 2], vals[4 * j4 + 3]);
         }
-      } else if (!(c0 >= 32 && i < 32)) {
-        // A_qk leaves transposed, At[j][i]: the 32 lanes of a warp (rows i) fill one 128-byte line per column j;
-        // the quadrant j >= 32, i < 32 is zero and stays unwritten (nobody reads it)
-#pragma unroll
-        for (int j = 0; j < 16; ++j) tile_at[(c0 + j) * kChunk + i] = vals[j];
       }
     }
   }
   tc_fence_before();
   sync();
+  if (gram_row >= 64) {
+    // A_qk leaves transposed, At[j][i]: the 32 lanes of a warp (rows i) fill one 128-byte line per column j;
+    // the quadrant j >= 32, i < 32 is zero and stays unwritten (nobody reads it)
+    float* tile_at = reinterpret_cast<float*>(p.tiles.at + int64_t(ch) * kTileAt) + gram_row - 64;
+    if (part == 0 || gram_row >= 96) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) tile_at[(32 * part + j) * kChunk] = a_qk[j >> 4][j & 15];
+    }
+  }
 
   // ---- T = (I + L)^-1, blocked: 16x16 diagonal blocks by substitution, the rest by block products.
   // T is kept in both orientations (Tn row-major, Tc column-major) and the block products W transposed,
@@ -460,19 +467,24 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   auto ld4 = [](const float* ptr) { return *reinterpret_cast<const float4*>(ptr); };
   if (tid < 64) {
     const int I = tid >> 4, cc = tid & 15;
+    // (column by column: what a finished entry contributes to all later ones is independent, so that the chain is 16
+    // multiply-adds long and not 120; each entry sums in the same order)
     float x[16];
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-      float s = (r == cc) ? 1.f : 0.f;
+    for (int r = 0; r < 16; ++r) x[r] = (r == cc) ? 1.f : 0.f;
 #pragma unroll
-      for (int m4 = 0; m4 < (r + 3) / 4; ++m4) {
-        const float4 l = ld4(Ln + (16 * I + r) * kLd + 16 * I + 4 * m4);
-        if (4 * m4 + 0 < r) s = fmaf(-l.x, x[4 * m4 + 0], s);
-        if (4 * m4 + 1 < r) s = fmaf(-l.y, x[4 * m4 + 1], s);
-        if (4 * m4 + 2 < r) s = fmaf(-l.z, x[4 * m4 + 2], s);
-        if (4 * m4 + 3 < r) s = fmaf(-l.w, x[4 * m4 + 3], s);
-      }
-      x[r] = s;
+    for (int m4 = 0; m4 < 4; ++m4) {
+      float4 l[16];
+#pragma unroll
+      for (int r = 4 * m4 + 1; r < 16; ++r) l[r] = ld4(Ln + (16 * I + r) * kLd + 16 * I + 4 * m4);
+#pragma unroll
+      for (int r = 4 * m4 + 1; r < 16; ++r) x[r] = fmaf(-l[r].x, x[4 * m4], x[r]);
+#pragma unroll
+      for (int r = 4 * m4 + 2; r < 16; ++r) x[r] = fmaf(-l[r].y, x[4 * m4 + 1], x[r]);
+#pragma unroll
+      for (int r = 4 * m4 + 3; r < 16; ++r) x[r] = fmaf(-l[r].z, x[4 * m4 + 2], x[r]);
+#pragma unroll
+      for (int r = 4 * m4 + 4; r < 16; ++r) x[r] = fmaf(-l[r].w, x[4 * m4 + 3], x[r]);
     }
 #pragma unroll
     for (int r = 0; r < 16; ++r) Tn[(16 * I + r) * kLd + 16 * I + cc] = x[r];
