@@ -3,7 +3,7 @@
 // tiles the forward scan read, through tiled TMA loads in the other swizzle: what the forward
 // contracted over columns it contracts over rows (K-major <-> MN-major operands, tc05.cuh).
 //
-//   chunk_bwd_scan_kernel  one CTA per (batch, head), chunks in reverse order.  The state
+//   chunk_bwd_scan_kernel  one CTA per (batch, head) or part of its value rows, chunks in reverse order.  The state
 //                          cotangent lives transposed (dS^T: value rows x key columns) in TMEM:
 //                              dR^T  = dO^T Aqk + dS^T Kt^T        dZ^T = dR^T T
 //                              dS^T <- dS^T diag(d) + dO^T Qg - dR^T Y
@@ -17,6 +17,7 @@
 //                          then the Gram products' VJP with the same 16-token block anchors as the
 //                          forward, and a per-channel chain (one thread = one key channel) that
 //                          forms dq, dk, dbeta and the reverse cumulative sum for dg.
+//   chunk_bwd_joint_kernel the work of both in one launch, where few sequences and heads scan.
 // A ragged length ends in a partial chunk: tokens past T - 1 carry no cotangent and get no gradient.
 //
 // Reference counterparts: boundary scan  src/gdn2_sm120/backward_parallel.py:721-1049,
