@@ -117,31 +117,6 @@ def test_joint_backward_equals_two_launches_and_the_oracle(batch, heads, time, k
         _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
 
 
-def test_joint_training_step_inside_a_cuda_graph():
-    tensors, d_out, d_fin = _device_inputs(1, 32 * 64 + 5, 13, seed=11)
-    leaves = [t.clone().requires_grad_(True) for t in tensors]
-
-    def step():
-        out, fin = chunk_gdn2(*leaves[:6], leaves[6], output_final_state=True)
-        return [out, fin, *torch.autograd.grad([out, fin], leaves, [d_out, d_fin])]
-
-    expected = [t.clone() for t in step()]
-    stream = torch.cuda.Stream()
-    stream.wait_stream(torch.cuda.current_stream())
-    with torch.cuda.stream(stream):
-        step()
-    torch.cuda.current_stream().wait_stream(stream)
-    graph = torch.cuda.CUDAGraph()
-    with torch.cuda.graph(graph):
-        captured = step()
-    for _ in range(3):  # (each replay clears the marks of the one before)
-        for t in captured:
-            t.detach().zero_()
-        graph.replay()
-        torch.cuda.synchronize()
-        assert all(torch.equal(a, b) for a, b in zip(captured, expected))
-
-
 # 255 .. 257 and 513: around one and two launch tables of 256 sequences
 @pytest.mark.parametrize("count", [255, 256, 257, 513])
 def test_packed_batches_around_the_table_size(count):
