@@ -285,6 +285,7 @@ __device__ __forceinline__ void reverse_sequence(const BScanParams& p, const Seq
       __threadfence_block();
       // (the VJP reads through the copy engine, another proxy than the stores)
       fence_async_all();
+      __syncwarp();  // what each lane saw is ordered before lane 0's release (a vote orders no memory)
       if (lane == 0) p.marks.arrive(ch_of(it));
     }
   } else if (!W::works(warp)) {

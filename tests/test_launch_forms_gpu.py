@@ -11,7 +11,8 @@ import pytest
 import torch
 
 import gdn2_oracle as oracle
-from gdn2_sm120_b200 import _lib, chunk_gdn2
+from gdn2_sm120_b200 import _lib, chunk_gdn2, chunk_kernels
+from gdn2_sm120_b200.chunk import chunk_forward
 from gdn2_sm120_b200.varlen import chunk_gdn2_varlen
 from test_autograd_gpu import _check_unit_alone_and_against_oracle, _device_inputs, _step
 
@@ -115,6 +116,31 @@ def test_joint_backward_equals_two_launches_and_the_oracle(batch, heads, time, k
         assert all(torch.equal(a, b) for a, b in zip(full[2], other[2]))
     if dtype == torch.bfloat16:
         _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
+
+
+# a unit whose mark is seen before its cotangent rows or its dZ tile are in memory reads what lay there before: NaN
+# here, in the fewest and the most scans and with a partial chunk
+@pytest.mark.parametrize("batch,heads,time", [(1, 4, 40 * 64), (1, 37, 32 * 64 + 5)])
+def test_joint_backward_never_reads_ahead_of_a_mark(batch, heads, time):
+    (q, k, v, g, beta, w, s0), d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
+    scale, full = 128 ** -0.5, -(-time // 64) * 64
+    _, _, aux = chunk_forward(q, k, v, g, beta, w, s0, scale=scale, return_aux=True)
+    slots = torch.empty((batch, full // 64 + 1, heads, 128, 128), device=DEV)
+    scratch = torch.empty(chunk_kernels.scratch_bytes(batch, full, heads, True) // 4, device=DEV)
+    first = None
+    for _ in range(25):
+        slots.fill_(float("nan"))
+        scratch.fill_(float("nan"))
+        grads = [torch.full_like(x, float("nan")) for x in (q, k, v, g, beta, w, s0)]
+        _lib.call("gdn2_chunk_backward", q.device, *[x.data_ptr() for x in (q, k, v, g, beta, w, d_out, d_fin)],
+                  aux.chunk_boundaries.data_ptr(), slots.data_ptr(), aux.workspace[0].data_ptr(), scratch.data_ptr(),
+                  *[x.data_ptr() for x in grads], batch, time, heads, full, _lib.dtype_code(q.dtype),
+                  _lib.dtype_code(g.dtype), scale, _lib.stream_ptr(q.device))
+        assert _lib.lib().gdn2_chunk_backward_kernels() == 1
+        if first is None:
+            first = grads
+            assert all(torch.isfinite(x.float()).all() for x in grads)
+        assert all(torch.equal(a, b) for a, b in zip(grads, first))
 
 
 # 255 .. 257 and 513: around one and two launch tables of 256 sequences
