@@ -50,6 +50,7 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_chunk_backward_f32grads": [_P] * 19 + [_I64] * 4 + [_F32, _P],
     "gdn2_chunk_forward_kernels": [],
     "gdn2_chunk_backward_kernels": [],
+    "gdn2_tensor_maps_encoded": [],
     "gdn2_chunk_read_status": [_P] + [_I64] * 3 + [_P],
     "gdn2_debug_wait_expires": [_P] + [_I64] * 4 + [_P],
     "gdn2_token_forward_fused": [_P] * 9 + [_I64] * 5 + [_INT, _INT, _F32, _INT, _P],
@@ -66,7 +67,8 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_profile_chunk_kernels": [_P] * 4,
 }
 _RESTYPES = {"gdn2_status_string": ctypes.c_char_p, "gdn2_last_cuda_error": ctypes.c_char_p,
-             "gdn2_chunk_workspace_bytes": ctypes.c_int64, "gdn2_chunk_scratch_bytes": ctypes.c_int64}
+             "gdn2_chunk_workspace_bytes": ctypes.c_int64, "gdn2_chunk_scratch_bytes": ctypes.c_int64,
+             "gdn2_tensor_maps_encoded": ctypes.c_int64}
 
 
 def library_path() -> pathlib.Path:

@@ -36,6 +36,7 @@
 
 #include <cuda.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -171,7 +172,8 @@ inline EncodeTiledFn encode_tiled_fn() {
 
 // Encoding a tensor map costs the host some 20 microseconds and a call needs a dozen of them; the
 // maps depend only on addresses and shapes, which repeat from call to call (allocators hand the same
-// blocks out again), so the last few hundred are kept.  Direct-mapped, one mutex.
+// blocks out again), so the last few hundred are kept.  Four ways a set, the oldest of a set leaves; one mutex.
+// (One map a set is not enough: a training step has some thirty, of which one pair in two steps met in 512 places.)
 struct TensorMapKey {
   uintptr_t base;
   cuuint64_t dims[4], strides[3];
@@ -183,27 +185,39 @@ struct TensorMapKey {
     for (int i = 0; i < 3; ++i) same = same && strides[i] == o.strides[i];
     return same;
   }
+  // every field counts: scans of split value rows and the VJP have maps of one tensor that differ in box[0] alone
+  uint64_t hash() const {
+    uint64_t h = base;
+    auto mix = [&h](uint64_t x) { h = (h ^ x) * 0x9E3779B97F4A7C15ull; h ^= h >> 32; };
+    for (int i = 0; i < 4; ++i) { mix(dims[i]); mix(box[i]); }
+    for (int i = 0; i < 3; ++i) mix(strides[i]);
+    mix(uint64_t(rank) << 32 | uint64_t(type) << 16 | uint64_t(swizzle));
+    return h;
+  }
 };
+
+inline std::atomic<int64_t> g_tensor_maps_encoded{0};  // by this process: those that were not kept
 
 // rank 3 or 4; unused trailing entries of dims / strides / box are 1 / 0 / 1
 inline bool encode_cached(CUtensorMap* tm, int rank, CUtensorMapDataType type, const void* base,
                           const cuuint64_t (&dims)[4], const cuuint64_t (&strides)[3], const cuuint32_t (&box)[4],
                           CUtensorMapSwizzle swizzle) {
-  constexpr int kSlots = 512;
-  struct Slot { bool used = false; TensorMapKey key; CUtensorMap map; };
-  static Slot slots[kSlots];
+  constexpr int kSets = 128, kWays = 4;
+  struct Set {
+    struct { bool used = false; TensorMapKey key; CUtensorMap map; } way[kWays];
+    int oldest = 0;
+  };
+  static Set sets[kSets];
   static std::mutex mutex;
-  TensorMapKey key{reinterpret_cast<uintptr_t>(base), {dims[0], dims[1], dims[2], dims[3]},
-                   {strides[0], strides[1], strides[2]}, {box[0], box[1], box[2], box[3]}, rank, int(type),
-                   int(swizzle)};
-  uint64_t h = key.base * 0x9E3779B97F4A7C15ull;
-  h ^= (key.dims[2] + 0x632BE59BD9B4E019ull * key.strides[1]) + (uint64_t(key.box[1]) << 7) + (uint64_t(key.box[2]) << 17) +
-       uint64_t(key.swizzle) * 31 + uint64_t(key.type) + uint64_t(rank) * 131 + key.dims[3] * 0x2545F4914F6CDD1Dull;
-  h ^= h >> 29;
-  Slot& slot = slots[h % kSlots];
+  const TensorMapKey key{reinterpret_cast<uintptr_t>(base), {dims[0], dims[1], dims[2], dims[3]},
+                         {strides[0], strides[1], strides[2]}, {box[0], box[1], box[2], box[3]}, rank, int(type),
+                         int(swizzle)};
+  Set& set = sets[key.hash() % kSets];
   {
     std::lock_guard<std::mutex> lock(mutex);
-    if (slot.used && slot.key == key) { *tm = slot.map; return true; }
+    for (const auto& way : set.way) {
+      if (way.used && way.key == key) { *tm = way.map; return true; }
+    }
   }
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return false;
@@ -220,8 +234,14 @@ inline bool encode_cached(CUtensorMap* tm, int rank, CUtensorMapDataType type, c
     int device = 0;
     if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(device) != cudaSuccess || !attempt()) return false;
   }
+  g_tensor_maps_encoded.fetch_add(1, std::memory_order_relaxed);
   std::lock_guard<std::mutex> lock(mutex);
-  slot.used = true; slot.key = key; slot.map = *tm;
+  for (const auto& way : set.way) {
+    if (way.used && way.key == key) return true;  // (another thread was first)
+  }
+  auto& way = set.way[set.oldest];
+  set.oldest = (set.oldest + 1) % kWays;
+  way.used = true; way.key = key; way.map = *tm;
   return true;
 }
 

@@ -1490,6 +1490,7 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
 }  // namespace
 
 int chunk_forward_kernels() { return t_forward_kernels; }
+int64_t tensor_maps_encoded() { return g_tensor_maps_encoded.load(std::memory_order_relaxed); }
 
 int launch_chunk_forward(const void* q, const void* k, const void* v, const void* g, const void* beta,
                          const void* w, const float* s_in, void* out, float* s_out, float* bnd,

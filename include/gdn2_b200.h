@@ -212,6 +212,12 @@ int gdn2_chunk_forward_kernels(void);
 int gdn2_chunk_backward_kernels(void);
 
 /*
+ * Test aid: TMA tensor maps that this process has encoded so far (some 20 us of host time each).  The chunk calls keep
+ * the last few hundred, so a call that repeats the addresses and sizes of an earlier one encodes none.
+ */
+int64_t gdn2_tensor_maps_encoded(void);
+
+/*
  * Chunkwise backward over tokens [0, full_tokens): reverse scan of the state cotangent plus
  * the compact-WY chunk VJP, from what gdn2_chunk_forward(training = 1) saved.  Replaces
  * wy_boundary_dstate and compact_wy_chunk_vjp_cute with their kernels

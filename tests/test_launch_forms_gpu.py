@@ -118,6 +118,25 @@ def test_joint_backward_equals_two_launches_and_the_oracle(batch, heads, time, k
         _check_unit_alone_and_against_oracle(tensors, d_out, d_fin, batch - 1, heads - 1, full)
 
 
+# The scans' maps of v, w, the output and its cotangent differ from those of the other kernels in the width of the box
+# alone where value rows are split (halves, quarters), and are the same where they are not
+@pytest.mark.parametrize("batch,heads,time", [(1, 16, 2048), (1, 2, 192), (2, 38, 130)])
+def test_a_repeated_training_step_encodes_no_tensor_map(batch, heads, time):
+    tensors, d_out, _ = _device_inputs(batch, time, heads, seed=2)
+    leaves = [t.requires_grad_(True) for t in tensors]
+
+    def step():
+        out, _ = chunk_gdn2(*leaves)
+        torch.autograd.grad(out, leaves, d_out)
+
+    for _ in range(4):  # until the allocator hands out the same blocks
+        step()
+    before = _lib.lib().gdn2_tensor_maps_encoded()
+    for _ in range(3):
+        step()
+    assert _lib.lib().gdn2_tensor_maps_encoded() == before > 0
+
+
 # a unit whose mark is seen before its cotangent rows or its dZ tile are in memory reads what lay there before: NaN
 # here, in the fewest and the most scans and with a partial chunk
 @pytest.mark.parametrize("batch,heads,time", [(1, 4, 40 * 64), (1, 37, 32 * 64 + 5)])
