@@ -17,7 +17,7 @@
 //                          then the Gram products' VJP with the same 16-token block anchors as the
 //                          forward, and a per-channel chain (one thread = one key channel) that
 //                          forms dq, dk, dbeta and the reverse cumulative sum for dg.
-//   chunk_bwd_joint_kernel the work of both in one launch, where few sequences and heads scan.
+//                          Its joint form does the work of both, where few sequences and heads scan.
 // A ragged length ends in a partial chunk: tokens past T - 1 carry no cotangent and get no gradient.
 //
 // Reference counterparts: boundary scan  src/gdn2_sm120/backward_parallel.py:721-1049,
@@ -564,8 +564,6 @@ struct VjpParams {
   int64_t n_ch;
   int H;
   float scale;
-  Marks marks;          // joint launch
-  unsigned marks_full;  // CTAs that mark a unit
 };
 // tensor maps of the seven sequence tensors the VJP kernel reads (for L2 prefetches only)
 struct VjpInputMaps {
@@ -642,15 +640,84 @@ __device__ __forceinline__ void tmem_ld4x2(uint32_t taddr, float2 (&x)[4]) {
 // their final rounding; used by tests to judge the arithmetic apart from the 16-bit cast).
 // kRagged: some sequence length is not a multiple of 64, its last chunk is partial; only this
 // instantiation carries the guards (they cost the others 6 %; a packed step of H16, 8192 tokens 1 %).
-// kJoint: units come from a queue in the order in which the scans that run beside finish them, and what the scans
-// write of a unit is loaded once their marks are there.
+// kJoint: the reverse scans run in the same launch (below).  Units come from a queue in the order in which the scans
+// finish them, and what the scans write of a unit is loaded once their marks are there.  The plain form carries none
+// of that, and the body is the kernel's own: bound by instruction issue and short of registers, the plain kernel
+// depends on how the compiler places what is nobody's business here.  As a function that both kernels called, with
+// the next unit kept in a register and the flag of a failed scan in the plain form's condition as a constant, B4 T8192
+// H32 took 1615 us; without these three 1585.
 struct VjpMaps {
   CUtensorMap s0, ds, rn, dq, dk, dbeta;
   VjpInputMaps in;
 };
+
+// Reverse scan and VJP in one launch.  With few sequences and heads the reverse scan keeps a few SMs busy, 1.9-2.2 us
+// per chunk, and the VJP of a chunk needs nothing but that chunk's share of it.  Here the scans run on pairs of CTAs (a
+// half of the value rows each) and all other CTAs, and at last these too, take the units from a queue, last chunks
+// first, waiting for the scans' marks.  The scans wait for nobody; the launch is cooperative, so that all CTAs are
+// resident together.  A unit's scratch tiles and cotangents are still in L2 when the VJP reads them.  Whatever waits for
+// memory on behalf of a mark is kept off the scan's chain and the VJP's: by the scanning warps themselves it cost a
+// chunk 1.2 us, by the thread that issues the VJP's copies a unit 1500 clocks.
+constexpr int kJointParts = 2;
+template <bool kJoint>
+struct JointScan {
+  BScanParams p;
+  BScanMaps tm;
+};
+template <>
+struct JointScan<false> {};
+
+// The queue of units of a joint launch, and the marks of those that the scans have finished.
+template <typename Seqs>
+struct JointUnits {
+  const VjpParams& p;
+  const Seqs& seqs;
+  const Marks marks;
+  VjpMisc& ms;
+  // the next unit of the queue, last chunks first
+  __device__ __forceinline__ int pop() const {
+    const unsigned u = atomicAdd(marks.of(0) + 1, 1u);
+    if (u >= unsigned(p.n_ch)) return int(p.n_ch);
+    const unsigned per_chunk = unsigned(seqs.count()) * unsigned(p.H), step = u / per_chunk, r = u - step * per_chunk;
+    const SeqInfo sq = seqs.at(int(r / unsigned(p.H)));
+    return (sq.chunk0 + sq.n_chunks - 1 - int(step)) * p.H + int(r % unsigned(p.H));
+  }
+  // have the scans finished a unit: a look, or a wait
+  __device__ __forceinline__ bool finished(int64_t ch) const {
+    unsigned x;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(marks.of(ch)) : "memory");
+    if (x != unsigned(kJointParts)) return false;
+    fence_async_all();
+    // (a wait of the scan that ran out: gradients become NaN)
+    if (*static_cast<volatile const int*>(p.status) != kStatusOk) ms.failed = 1;
+    return true;
+  }
+  __device__ __forceinline__ void await(int64_t ch, BoundedWaiter& waiter) const {
+    while (!finished(ch)) {
+      if (!waiter.look_again()) {
+        ms.failed = 1;
+        break;
+      }
+      __nanosleep(100);
+    }
+  }
+};
+
 template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged, bool kJoint>
-__device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, const VjpMaps& tm, uint8_t* smem) {
+__global__ void __launch_bounds__(kVjpThreads, 1)
+chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ VjpMaps tm,
+                     const __grid_constant__ JointScan<kJoint> scan) {
   using O = typename std::conditional<kF32Grads, float, T>::type;  // element type of dq, dk, dv, dbeta, dw
+  extern __shared__ __align__(1024) uint8_t smem[];
+  if constexpr (kJoint) {
+    static_assert(BScanWarps<kJointParts>::kThreads == kVjpThreads, "a scanning CTA goes on with the VJP");
+    if (int(blockIdx.x) < kJointParts * seqs.count() * p.H) {
+      reverse_sequence<T, Seqs, true, kJointParts>(scan.p, seqs, scan.tm, *reinterpret_cast<BScanSmem*>(smem),
+                                                   int(blockIdx.x));
+      fence_async_smem();
+      __syncthreads();
+    }
+  }
   const CUtensorMap &tm_s0 = tm.s0, &tm_ds = tm.ds, &tm_rn = tm.rn, &tm_dq = tm.dq, &tm_dk = tm.dk, &tm_dbeta = tm.dbeta;
   const VjpInputMaps& tm_in = tm.in;
   VjpMisc& ms = *reinterpret_cast<VjpMisc*>(smem + kOffMisc);
@@ -706,44 +773,16 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
     tma_load_4d(smem + kOffS0, &tm_s0, 0, 0, 0, slot_, &ms.bar_s);
     mbar_arrive_expect_tx(&ms.bar_a, uint32_t(kBlobDZ + kBlobRn));
     tma_load_4d(smem + kOffRn, &tm_rn, 0, 0, 0, int(ch_), &ms.bar_a);
-  };
-  auto issue_dz = [&](int64_t ch_) {
-    bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + ch_ * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
+    if constexpr (!kJoint) bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + ch_ * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
   };
   auto issue_ds1 = [&](int slot_) {
     tma_load_4d(smem + kOffDs1, &tm_ds, 0, 0, 0, slot_ + p.H, &ms.bar_s);
   };
-  // joint launch: the next unit of the queue, last chunks first; have the scans finished it (a look, or a wait)
-  auto pop = [&] {
-    const unsigned u = atomicAdd(p.marks.of(0) + 1, 1u);
-    if (u >= unsigned(p.n_ch)) return int(p.n_ch);
-    const unsigned per_chunk = unsigned(seqs.count()) * unsigned(p.H), step = u / per_chunk, r = u - step * per_chunk;
-    const SeqInfo sq = seqs.at(int(r / unsigned(p.H)));
-    return (sq.chunk0 + sq.n_chunks - 1 - int(step)) * p.H + int(r % unsigned(p.H));
-  };
-  auto finished = [&](int64_t ch_) {
-    unsigned x;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(p.marks.of(ch_)) : "memory");
-    if (x != p.marks_full) return false;
-    fence_async_all();
-    // (a wait of the scan that ran out: gradients become NaN)
-    if (*static_cast<volatile const int*>(p.status) != kStatusOk) ms.failed = 1;
-    return true;
-  };
-  auto await = [&](int64_t ch_) {
-    while (!finished(ch_)) {
-      if (!waiter.look_again()) {
-        ms.failed = 1;
-        break;
-      }
-      __nanosleep(100);
-    }
-  };
-  int64_t first = blockIdx.x;
+  int64_t first = blockIdx.x, joint_next = 0;
   if constexpr (kJoint) {
     if (tid == 0) {
       ms.failed = 0;
-      ms.next[0] = pop();
+      ms.next[0] = JointUnits<Seqs>{p, seqs, scan.p.marks, ms}.pop();
     }
     __syncthreads();
     first = ms.next[0];
@@ -752,17 +791,20 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
   if (tid == 0 && first < p.n_ch) {
     const int slot_ = locate(first).slot;
     issue_loads(first, slot_);
-    if constexpr (kJoint) await(first);
-    issue_dz(first);
+    if constexpr (kJoint) {
+      JointUnits<Seqs>{p, seqs, scan.p.marks, ms}.await(first, waiter);
+      bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + first * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
+    }
     issue_ds1(slot_);
   }
 
   uint32_t iter = 0;
-  for (int64_t ch = first, ch_next; ch < p.n_ch; ch = ch_next, ++iter) {
+  for (int64_t ch = first; ch < p.n_ch; ch = kJoint ? joint_next : ch + gridDim.x, ++iter) {
   const uint32_t par = iter & 1u;
-  ch_next = ch + gridDim.x;
-  int popped = 0;
-  if (kJoint && tid == 96) popped = pop();
+  [[maybe_unused]] int popped = 0;
+  if constexpr (kJoint) {
+    if (tid == 96) popped = JointUnits<Seqs>{p, seqs, scan.p.marks, ms}.pop();
+  }
   const Place at = locate(ch);
   const int h = at.h;
   auto seq_idx = [&](int tok) { return (int64_t(at.row + tok) * p.H + h) * int64_t(kDim); };
@@ -832,14 +874,16 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
     }
   }
   *reinterpret_cast<float4*>(&ms.part[tg][kc0]) = make_float4(Gc[3][0], Gc[3][1], Gc[3][2], Gc[3][3]);
-  if (kJoint && tid == 96) ms.next[par] = popped;
+  if constexpr (kJoint) {
+    if (tid == 96) ms.next[par] = popped;
+  }
   waiter.wait(&ms.bar_a, par);
   waiter.wait(&ms.bar_s, par);
   dd_half(0);
   fence_async_smem();
   tc_fence_before();
   __syncthreads();
-  if constexpr (kJoint) ch_next = ms.next[par];
+  if constexpr (kJoint) joint_next = ms.next[par];
   // ---- first MMA batch: M4 (first half) dKt^T = dS_1[:, v < 64] R[:, v < 64]^T ;
   //      M2 [-dL ; dA] = [dZ ; dO] R^T ;  M3 [-dE ; dQg]^T = S_0 [dZ ; dO]^T ------------------------------
   if (warp == 0) {
@@ -914,7 +958,10 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
       for (int e = 0; e < 4; ++e) {
         const int j = 4 * tg + e;
         float4 dz = *reinterpret_cast<const float4*>(smem + kOffStack + (j >> 3) * kRsN + c4 * kCsN + (j & 7) * 16);
-        if (upstream_failed || waiter.dead || (kJoint && ms.failed != 0)) dz = make_float4(poison_nan(), poison_nan(), poison_nan(), poison_nan());
+        if (upstream_failed || waiter.dead) dz = make_float4(poison_nan(), poison_nan(), poison_nan(), poison_nan());
+        if constexpr (kJoint) {
+          if (ms.failed != 0) dz = make_float4(poison_nan(), poison_nan(), poison_nan(), poison_nan());
+        }
         const int64_t idx = seq_idx(j) + kc0;
         float wv[4], vv[4];
         unpack4<T>(wr[e], wv);
@@ -932,15 +979,19 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
   // bytes in flight over the latency: have its seven [64][128] tiles brought into L2, the four that are read
   // first from here on and the others with the tile copies.  (All behind the tile copies they wait for those
   // in the copy engine: B4 T8192 H32 1.72 ms against 1.63; all from here, ragged lengths lose 2 %.)
-  if (tid == 64 && ch_next < p.n_ch) {
-    const Place nx = locate(ch_next);
+  if (tid == 64 && (kJoint ? joint_next : ch + gridDim.x) < p.n_ch) {
+    const Place nx = locate(kJoint ? joint_next : ch + gridDim.x);
     tma_prefetch_l2_3d(&tm_in.d_out, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.g, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.w, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.v, 0, nx.h, nx.row);
   }
   // (where all wait for the tensor cores anyway: a look takes 1500 clocks)
-  if (kJoint && tid == 96) ms.ready[par] = ch_next < p.n_ch && finished(ch_next);
+  if constexpr (kJoint) {
+    if (tid == 96) {
+      ms.ready[par] = joint_next < p.n_ch && JointUnits<Seqs>{p, seqs, scan.p.marks, ms}.finished(joint_next);
+    }
+  }
   // ---- M4 (second half) once the second half of dS_1 has landed -----------------------------------------
   waiter.wait(&ms.bar_d, par);
   dd_half(1);
@@ -1088,14 +1139,16 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
   ++mma_phase;
   tc_fence_after();
   // shared memory (all but the small arrays of VjpMisc) is dead from here on: fetch the next chunk-head
-  bool pending = false;  // (what the scan writes of the next unit is not there yet)
-  if (tid == 0 && ch_next < p.n_ch) {
-    issue_loads(ch_next, locate(ch_next).slot);
-    pending = kJoint && ms.ready[par] == 0;
-    if (!pending) issue_dz(ch_next);
+  [[maybe_unused]] bool pending = false;  // (what the scan writes of the next unit is not there yet)
+  if (tid == 0 && (kJoint ? joint_next : ch + gridDim.x) < p.n_ch) issue_loads((kJoint ? joint_next : ch + gridDim.x), locate(kJoint ? joint_next : ch + gridDim.x).slot);
+  if constexpr (kJoint) {
+    if (tid == 0 && joint_next < p.n_ch) {
+      pending = ms.ready[par] == 0;
+      if (!pending) bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + joint_next * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
+    }
   }
-  if (tid == 64 && ch_next < p.n_ch) {  // (see the other prefetches above)
-    const Place nx = locate(ch_next);
+  if (tid == 64 && (kJoint ? joint_next : ch + gridDim.x) < p.n_ch) {  // (see the other prefetches above)
+    const Place nx = locate(kJoint ? joint_next : ch + gridDim.x);
     tma_prefetch_l2_3d(&tm_in.k, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.q, 0, nx.h, nx.row);
     tma_prefetch_l2_3d(&tm_in.beta, 0, nx.h, nx.row);
@@ -1121,7 +1174,8 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
   // the row and column contributions of the Gram products to dG then cancel as they do exactly.
   {
     const int kc = tid & 127, blk = part;
-    const bool failed = upstream_failed || waiter.dead || (kJoint && ms.failed != 0);
+    bool failed = upstream_failed || waiter.dead;
+    if constexpr (kJoint) failed = failed || ms.failed != 0;
     const float gend = ms.gend[kc];
     // dd[k] = sum_v dS_1[k][v] S_0[k][v]: read here, before xt is reused for the block sums of dG
     const float dd_k = (ms.xt[0][kc] + ms.xt[1][kc]) + (ms.xt[2][kc] + ms.xt[3][kc]);
@@ -1282,50 +1336,17 @@ __device__ __forceinline__ void vjp_units(const VjpParams& p, const Seqs& seqs, 
       bulk_commit();
     }
     // the G tile is dead: the dS_1 half of the next chunk-head may land on it
-    if (ch_next < p.n_ch) {
+    if constexpr (kJoint) {
       if (pending) {
-        await(ch_next);
-        issue_dz(ch_next);
+        JointUnits<Seqs>{p, seqs, scan.p.marks, ms}.await(joint_next, waiter);
+        bulk_g2s(smem + kOffStack, p.sc + sc.off_dz() + joint_next * kBlobDZ, uint32_t(kBlobDZ), &ms.bar_a);
       }
-      issue_ds1(locate(ch_next).slot);
     }
+    if ((kJoint ? joint_next : ch + gridDim.x) < p.n_ch) issue_ds1(locate(kJoint ? joint_next : ch + gridDim.x).slot);
   }
   }  // chunk-head loop
   if (tid == 0) bulk_wait_all();  // the last dq / dk tiles are in global memory before the CTA retires
   if (warp == 0) tmem_dealloc(tb, 512);
-}
-
-template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
-__global__ void __launch_bounds__(kVjpThreads, 1)
-chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ VjpMaps tm) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  vjp_units<T, G, Seqs, kF32Grads, kRagged, false>(p, seqs, tm, smem_raw);
-}
-
-// =============================================================================================
-// reverse scan and VJP in one launch
-// =============================================================================================
-// With few sequences and heads the reverse scan keeps a few SMs busy, 1.9-2.2 us per chunk, and the VJP of a chunk
-// needs nothing but that chunk's share of it.  Here the scans run on pairs of CTAs (a half of the value rows each) and
-// all other CTAs, and at last these too, take the units from a queue, last chunks first, waiting for the scans'
-// marks.  The scans wait for nobody; the launch is cooperative, so that all CTAs are resident together.  A unit's
-// scratch tiles and cotangents are still in L2 when the VJP reads them.  Whatever waits for memory on behalf of a mark
-// is kept off the scan's chain and the VJP's: by the scanning warps themselves it cost a chunk 1.2 us, by the thread
-// that issues the VJP's copies a unit 1500 clocks.
-constexpr int kJointParts = 2;
-template <typename T, typename G, bool kRagged>
-__global__ void __launch_bounds__(kVjpThreads, 1) __cluster_dims__(2, 1, 1)
-chunk_bwd_joint_kernel(const BScanParams sp, const VjpParams vp, const __grid_constant__ UniformSeqs seqs,
-                       const __grid_constant__ BScanMaps tm_scan, const __grid_constant__ VjpMaps tm_vjp) {
-  static_assert(BScanWarps<kJointParts>::kThreads == kVjpThreads, "a scanning CTA goes on with the VJP");
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (int(blockIdx.x) < kJointParts * seqs.count() * sp.H) {
-    reverse_sequence<T, UniformSeqs, true, kJointParts>(sp, seqs, tm_scan, *reinterpret_cast<BScanSmem*>(smem_raw),
-                                                        int(blockIdx.x));
-    fence_async_smem();
-    __syncthreads();
-  }
-  vjp_units<T, G, UniformSeqs, false, kRagged, true>(vp, seqs, tm_vjp, smem_raw);
 }
 
 }  // namespace
@@ -1350,13 +1371,13 @@ struct BackwardCall {
 
 template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
 int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStream_t stream) {
-  auto kernel = chunk_bwd_vjp_kernel<T, G, Seqs, kF32Grads, kRagged>;
+  auto kernel = chunk_bwd_vjp_kernel<T, G, Seqs, kF32Grads, kRagged, false>;
   cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kVjpSmemBytes);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   int sm_count = 0;
   if (int st = multiprocessors(&sm_count); st != GDN2_OK) return st;
   const unsigned grid = unsigned(p.n_ch < int64_t(sm_count) ? p.n_ch : int64_t(sm_count));
-  kernel<<<grid, kVjpThreads, kVjpSmemBytes, stream>>>(p, seqs, m);
+  kernel<<<grid, kVjpThreads, kVjpSmemBytes, stream>>>(p, seqs, m, JointScan<false>{});
   return check_launch();
 }
 
@@ -1388,10 +1409,10 @@ template <typename T, typename G, bool kRagged>
 int launch_joint(const BScanParams& sp, const VjpParams& vp, const UniformSeqs& seqs, const BScanMaps& tm_scan,
                  const VjpMaps& tm_vjp, int sm_count, cudaStream_t stream) {
   constexpr int smem = int(sizeof(BScanSmem)) > kVjpSmemBytes ? int(sizeof(BScanSmem)) : kVjpSmemBytes;
-  auto kernel = chunk_bwd_joint_kernel<T, G, kRagged>;
+  auto kernel = chunk_bwd_vjp_kernel<T, G, UniformSeqs, false, kRagged, true>;
   cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  err = cudaMemset2DAsync(vp.marks.dz + kMarkOffset, kBlobDZ, 0, 16, size_t(vp.n_ch), stream);
+  err = cudaMemset2DAsync(sp.marks.dz + kMarkOffset, kBlobDZ, 0, 16, size_t(vp.n_ch), stream);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int64_t want = int64_t(seqs.count()) * sp.H + (vp.n_ch + 1) / 2;
   cudaLaunchConfig_t config = {};
@@ -1399,12 +1420,15 @@ int launch_joint(const BScanParams& sp, const VjpParams& vp, const UniformSeqs& 
   config.blockDim = dim3(kVjpThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute together;
-  together.id = cudaLaunchAttributeCooperative;
-  together.val.cooperative = 1;
-  config.attrs = &together;
-  config.numAttrs = 1;
-  err = cudaLaunchKernelEx(&config, kernel, sp, vp, seqs, tm_scan, tm_vjp);
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeCooperative;
+  attributes[0].val.cooperative = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = 2;
+  attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
+  err = cudaLaunchKernelEx(&config, kernel, vp, seqs, tm_vjp, JointScan<true>{sp, tm_scan});
   if (err == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs than the device
     (void)cudaGetLastError();
     return GDN2_ERR_UNSUPPORTED;
@@ -1465,7 +1489,7 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
     return GDN2_ERR_LAUNCH;
   }
   const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.dq, a.dk, a.dv, a.dg,
-                     a.dbeta, a.dw, status, n_ch, int(a.H), a.scale, marks, kJointParts};
+                     a.dbeta, a.dw, status, n_ch, int(a.H), a.scale};
   int st = GDN2_ERR_UNSUPPORTED;
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     if (joint) {
