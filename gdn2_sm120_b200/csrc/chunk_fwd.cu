@@ -1379,8 +1379,13 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   const int64_t want = pairs + std::min((pp.n_ch + 3) / 4, paced);
   const int clusters = int(std::min(want, int64_t(sm_count / 2)));
   // Where the preparers alone would not keep up, the scanning CTAs first prepare `quota` units for each group of
-  // theirs, so that everybody is done at the same time.
-  const int64_t in_time = int64_t(2 * (clusters - pairs)) * seqs.n_chunks * 28 / 100;
+  // theirs, so that everybody is done at the same time.  While a scan advances by a chunk a preparing SM makes
+  // `pace` / 100 units: 1.7 us to 9.4, 1.9 to 12 with the prologue, 2.0 to 10 where the states are written out.  us, with
+  // 28 for all / with these: inference T8192 H24 318/297, H32 432/391, H37 502/454, T32768 H24 1152/1098; raw T8192
+  // H24 383/361, H32 531/472, H37 621/537, T32768 H24 1450/1349, B2 T4133 H16 282/260; training T4096 H24 440/433, T8192
+  // H28 930/922.  (One unit in a hundred more or less moves these by 1 %, four by 5.)
+  const int64_t pace = pp.training != 0 ? 20 : pp.prologue != 0 ? 16 : 18;
+  const int64_t in_time = int64_t(2 * (clusters - pairs)) * seqs.n_chunks * pace / 100;
   const int quota = pp.n_ch > in_time ? int((pp.n_ch - in_time + 2 * clusters) / (4 * clusters)) : 0;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(unsigned(2 * clusters));

@@ -93,6 +93,23 @@ def test_joint_launch_equals_two_launches(dtype, g_dtype, raw):
     assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
 
 
+# scanning CTAs that prepare none, some and nearly all of the units that the others could not have ready in time
+@pytest.mark.parametrize("heads,time", [(16, 30 * 64), (24, 48 * 64), (28, 33 * 64 + 9), (37, 21 * 64), (37, 64 * 64)])
+@pytest.mark.parametrize("raw", [False, True])
+def test_joint_launches_whose_scans_prepare_first_equal_two_launches(heads, time, raw):
+    tensors, _, _ = _device_inputs(1, time, heads, seed=heads + time)
+    flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
+    with torch.no_grad():
+        joint = chunk_gdn2(*tensors, output_final_state=True, **flags)
+        assert _lib.lib().gdn2_chunk_forward_kernels() == 1
+        _lib.profile_enable(True)  # times the kernels one by one: never joint
+        try:
+            apart = chunk_gdn2(*tensors, output_final_state=True, **flags)
+        finally:
+            _lib.profile_enable(False)
+    assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
+
+
 # (four scans at least, a quarter of the SMs at most, 32 chunks: the smallest and widest grids, one chunk less, and
 # ragged ends of 1 and 63 tokens)
 @pytest.mark.parametrize("batch,heads,time,kernels", [(1, 4, 32 * 64, 1), (1, 3, 32 * 64, 2), (2, 16, 31 * 64, 2),
