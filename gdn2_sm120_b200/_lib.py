@@ -51,6 +51,7 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_chunk_forward_kernels": [],
     "gdn2_chunk_backward_kernels": [],
     "gdn2_tensor_maps_encoded": [],
+    "gdn2_chunk_value_parts": [_I64] * 3 + [_INT] * 2,
     "gdn2_chunk_read_status": [_P] + [_I64] * 3 + [_P],
     "gdn2_debug_wait_expires": [_P] + [_I64] * 4 + [_P],
     "gdn2_token_forward_fused": [_P] * 9 + [_I64] * 5 + [_INT, _INT, _F32, _INT, _P],

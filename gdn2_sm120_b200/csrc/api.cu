@@ -30,6 +30,7 @@ int64_t chunk_scratch_bytes(int64_t, int64_t, int64_t, int);
 int chunk_forward_kernels();
 int chunk_backward_kernels();
 int64_t tensor_maps_encoded();
+int chunk_value_parts(int64_t, int64_t, int64_t, int, int);
 int64_t chunk_status_offset(int64_t, int64_t, int64_t);
 int launch_chunk_forward(const void*, const void*, const void*, const void*, const void*, const void*,
                          const float*, void*, float*, float*, uint8_t*, uint8_t*, int64_t, int64_t, int64_t,
@@ -423,6 +424,11 @@ int gdn2_chunk_backward_f32grads(const void* q, const void* k, const void* v, co
 int gdn2_chunk_forward_kernels(void) { return chunk_forward_kernels(); }
 int gdn2_chunk_backward_kernels(void) { return chunk_backward_kernels(); }
 int64_t gdn2_tensor_maps_encoded(void) { return tensor_maps_encoded(); }
+
+int gdn2_chunk_value_parts(int64_t chunks, int64_t scans, int64_t longest, int multiprocessors, int most) {
+  if (chunks <= 0 || scans <= 0 || longest <= 0 || multiprocessors <= 0 || most <= 0) return GDN2_ERR_BAD_SHAPE;
+  return chunk_value_parts(chunks, scans, longest, multiprocessors, most);
+}
 
 int gdn2_chunk_read_status(const void* workspace, int64_t batch, int64_t full_tokens, int64_t heads,
                            void* stream) {

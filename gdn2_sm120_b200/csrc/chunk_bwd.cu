@@ -1456,7 +1456,7 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     joint = !a.grads_f32 && prefer_joint_backward(n_scan, seqs.n_chunks, sm_count);
   }
-  const int parts = joint ? kJointParts : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 4);
+  const int parts = joint ? kJointParts : value_parts(n_ch, n_scan, seqs.at(0).n_chunks, sm_count, 4);
   // the reverse scan's operands: the forward's tiles, each in the swizzle of the role backward reads it in
   BScanMaps tm;
   if (!encode_tile_map(&tm.at, a.workspace + ws.off_at(), n_ch, kChunk, kChunk, false, 32, 1) ||

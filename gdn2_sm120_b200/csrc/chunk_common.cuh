@@ -297,9 +297,13 @@ inline bool encode_tile_map(CUtensorMap* tm, const uint8_t* base, int64_t n_ch, 
 // As many as leave the longest sequence the longest part of the call: with 128 sequences x heads of one length,
 // where every SM has a scan as it is, halves take 749 -> 758 us (training B4 T8192 H32) and 221 -> 293 (inference
 // B8 T4096); packed training of 911, 2300, 150, 1640, 77, 1202, 514, 1398 tokens, H16, 133 -> 114 and 109 -> 97.
-inline int value_parts(int64_t units, int64_t longest, int sm_count, int most) {
+// A CTA counts for five chunks more than it scans: it takes that long to start, to read its state and to end (a scan of
+// one to four chunks takes 15-17 us).  Without them packed inference of 100, 200, 300 tokens, H32, was split into 192
+// CTAs for 148 SMs: 51.8 -> 56.0 us, and 300, 300, 600 80.7 -> 84.1; 64, 128, 192, 256 at H24 39.0 -> 41.1.
+constexpr int kScanOverhead = 5;
+inline int value_parts(int64_t units, int64_t scans, int64_t longest, int sm_count, int most) {
   int parts = 1;
-  while (parts < most && 2 * parts * units <= longest * sm_count) parts *= 2;
+  while (parts < most && 2 * parts * (units + kScanOverhead * scans) <= (longest + kScanOverhead) * sm_count) parts *= 2;
   return parts;
 }
 

@@ -1430,7 +1430,7 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, a.training != 0, sm_count);
   }
-  const int parts = joint ? kJointParts : value_parts(n_ch, seqs.at(0).n_chunks, sm_count, 2);
+  const int parts = joint ? kJointParts : value_parts(n_ch, n_scan, seqs.at(0).n_chunks, sm_count, 2);
   const WsLayout ws{n_ch, a.training != 0};
   int* status = reinterpret_cast<int*>(a.workspace + ws.off_status());
   const ForwardTiles tiles = forward_tiles(a.workspace, a.scratch, n_ch, a.training != 0);
@@ -1495,6 +1495,9 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
 }  // namespace
 
 int chunk_forward_kernels() { return t_forward_kernels; }
+int chunk_value_parts(int64_t units, int64_t scans, int64_t longest, int sm_count, int most) {
+  return value_parts(units, scans, longest, sm_count, most);
+}
 int64_t tensor_maps_encoded() { return g_tensor_maps_encoded.load(std::memory_order_relaxed); }
 
 int launch_chunk_forward(const void* q, const void* k, const void* v, const void* g, const void* beta,

@@ -218,6 +218,12 @@ int gdn2_chunk_backward_kernels(void);
 int64_t gdn2_tensor_maps_encoded(void);
 
 /*
+ * Test aid: into how many CTAs the value rows of a scan are split (1, 2, or where `most` = 4 up to 4), for `chunks`
+ * chunks of all sequences and heads, `scans` sequences x heads, `longest` chunks of the longest sequence.  Host only.
+ */
+int gdn2_chunk_value_parts(int64_t chunks, int64_t scans, int64_t longest, int multiprocessors, int most);
+
+/*
  * Chunkwise backward over tokens [0, full_tokens): reverse scan of the state cotangent plus
  * the compact-WY chunk VJP, from what gdn2_chunk_forward(training = 1) saved.  Replaces
  * wy_boundary_dstate and compact_wy_chunk_vjp_cute with their kernels

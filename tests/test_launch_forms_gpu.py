@@ -52,6 +52,19 @@ def test_scans_of_split_value_rows_equal_whole_ones(heads, time, dtype):
         assert torch.equal(gr[6], grads[6][1:2, at])
 
 
+# Scans of value rows are split while the longest sequence stays the longest part of the call: equal lengths up to half
+# (a quarter) of the SMs whatever their length, packed ones by their chunks and the cost of a CTA.  (The rule only: no
+# launch.)
+@pytest.mark.parametrize("lengths,heads,most,parts", [
+    ([64], 74, 2, 2), ([64], 75, 2, 1), ([4096], 74, 4, 2), ([4096], 37, 4, 4), ([4096], 38, 4, 2), ([64], 1, 2, 2),
+    ([100, 200, 300], 32, 2, 1), ([100, 200, 300], 24, 2, 2), ([64, 128, 192, 256], 24, 2, 1),
+    ([300, 300, 600], 32, 2, 1), ([300, 300, 600], 24, 2, 2), ([1400, 700, 350, 175], 32, 2, 2),
+    ([911, 2300, 150, 1640, 77, 1202, 514, 1398], 16, 4, 2), ([2600, 64, 70, 700], 16, 4, 4)])
+def test_rule_that_splits_value_rows(lengths, heads, most, parts):
+    chunks = [-(-n // 64) for n in lengths]
+    assert _lib.lib().gdn2_chunk_value_parts(sum(chunks) * heads, len(chunks) * heads, max(chunks), 148, most) == parts
+
+
 # four sequences of which one is long: split at 16 heads (2 * 56 units a head <= 41 * 148), not in the sequences alone
 def test_packed_scans_of_split_value_rows_equal_single_sequences():
     lengths, heads = [2600, 64, 70, 700], 16
