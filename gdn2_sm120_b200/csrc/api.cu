@@ -41,6 +41,7 @@ int launch_chunk_backward(const void*, const void*, const void*, const void*, co
                           void*, void*, void*, void*, void*, float*, int64_t, int64_t, int64_t, int64_t, int,
                           int, float, int, cudaStream_t);
 int launch_debug_wait_expires(int* status, uint32_t max_polls, cudaStream_t stream);
+int launch_debug_looks(int* status, uint32_t limit, uint32_t looks, uint32_t waits, cudaStream_t stream);
 int launch_gate_prologue(const void*, const void*, const void*, const void*, const void*, void*, void*, void*,
                          void*, void*, float*, float*, int64_t, int, int, cudaStream_t);
 int launch_gate_prologue_vjp(const void*, const void*, const void*, const void*, const void*, const float*,
@@ -502,6 +503,18 @@ int gdn2_debug_wait_expires(void* workspace, int64_t batch, int64_t full_tokens,
   int* status = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) +
                                        chunk_status_offset(batch, full_tokens, heads));
   return launch_debug_wait_expires(status, uint32_t(polls), static_cast<cudaStream_t>(stream));
+}
+
+int gdn2_debug_looks(void* workspace, int64_t batch, int64_t full_tokens, int64_t heads, int64_t limit, int64_t looks,
+                     int64_t waits, void* stream) {
+  if (!workspace) return GDN2_ERR_NULL_POINTER;
+  if (batch <= 0 || heads <= 0 || full_tokens <= 0 || full_tokens % GDN2_CHUNK != 0) return GDN2_ERR_BAD_SHAPE;
+  if (limit < 1 || looks < 0 || waits < 0 || limit > 4096 || looks > 4096 || waits > 4096) return GDN2_ERR_BAD_SHAPE;
+  if (check_shape(batch, full_tokens, heads) != GDN2_OK) return GDN2_ERR_TOO_LARGE;
+  if (!aligned(workspace, 16)) return GDN2_ERR_ALIGNMENT;
+  int* status = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) +
+                                       chunk_status_offset(batch, full_tokens, heads));
+  return launch_debug_looks(status, uint32_t(limit), uint32_t(looks), uint32_t(waits), static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

@@ -693,6 +693,7 @@ struct JointUnits {
     return true;
   }
   __device__ __forceinline__ void await(int64_t ch, BoundedWaiter& waiter) const {
+    waiter.look_anew();
     while (!finished(ch)) {
       if (!waiter.look_again()) {
         ms.failed = 1;

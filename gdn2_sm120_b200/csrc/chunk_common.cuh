@@ -127,11 +127,14 @@ struct BoundedWaiter {
     if (dead) return;
     if (!tc::mbar_wait(bar, parity, limit)) expire();
   }
-  // for loops that look at something other than an mbarrier: false once `limit` looks were in vain
+  // for loops that look at something other than an mbarrier: false once `limit` looks in a row were in vain.  What was
+  // looked for has a count of its own, from look_anew on: a launch may look any number of times, and mbarrier waits
+  // keep their limit.
+  uint32_t looks = 0;
+  __device__ __forceinline__ void look_anew() { looks = 0; }
   __device__ __forceinline__ bool look_again() {
-    if (limit > 0) --limit;
-    if (limit == 0 && !dead) expire();
-    return limit > 0;
+    if (!dead && ++looks >= limit) expire();
+    return !dead;
   }
   __device__ __forceinline__ void expire() {
     dead = true;

@@ -1014,6 +1014,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
         __nanosleep(200);
       } else {
         c = min(c + there, n_chunks);
+        waiter.look_anew();
       }
       // (a wait of a preparer that ran out, or this one's own: results become NaN)
       if (*static_cast<volatile const int*>(p.status) != kStatusOk) sm.failed = 1;
@@ -1306,7 +1307,28 @@ __global__ void __launch_bounds__(128, 1) debug_wait_expires_kernel(int* status,
   if (warp == 0) tmem_dealloc(tmem_base, 32);
 }
 
+// One thread looks `looks` times in vain for each of `waits` things and then waits on an mbarrier that is complete: the
+// status word tells whether any of it ran out.
+__global__ void __launch_bounds__(32, 1) debug_looks_kernel(int* status, uint32_t limit, uint32_t looks, uint32_t waits) {
+  __shared__ alignas(8) uint64_t bar;
+  if (threadIdx.x != 0) return;
+  mbar_init(&bar, 1);
+  fence_mbar_init();
+  mbar_arrive(&bar);
+  BoundedWaiter waiter(status, limit);
+  for (uint32_t i = 0; i < waits; ++i) {
+    waiter.look_anew();
+    for (uint32_t j = 0; j < looks && waiter.look_again(); ++j) {}
+  }
+  waiter.wait(&bar, 0);
+}
+
 }  // namespace
+
+int launch_debug_looks(int* status, uint32_t limit, uint32_t looks, uint32_t waits, cudaStream_t stream) {
+  debug_looks_kernel<<<1, 32, 0, stream>>>(status, limit, looks, waits);
+  return check_launch();
+}
 
 int launch_debug_wait_expires(int* status, uint32_t max_polls, cudaStream_t stream) {
   debug_wait_expires_kernel<<<1, 128, 0, stream>>>(status, max_polls);

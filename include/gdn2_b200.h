@@ -285,6 +285,14 @@ int gdn2_debug_wait_expires(void* workspace, int64_t batch, int64_t full_tokens,
                             int64_t max_polls, void* stream);
 
 /*
+ * Test aid for the waits of a joint launch, which look at marks in global memory: one thread looks `looks` times in vain
+ * for each of `waits` marks, with the kernels' own bounded waiter (`limit` looks for one mark; each at most 4096), and
+ * then waits on an mbarrier that is complete.  Status 1 in the workspace's status word if any of it ran out.
+ */
+int gdn2_debug_looks(void* workspace, int64_t batch, int64_t full_tokens, int64_t heads, int64_t limit,
+                     int64_t looks, int64_t waits, void* stream);
+
+/*
  * ---- fused input prologue of a layer (next to the primitive, not inside it) ----------------
  *
  * One pass over the [B, T, H, 128] sequence tensors that does what a Gated DeltaNet-2 layer does to

@@ -79,6 +79,18 @@ def test_a_failure_recorded_in_the_workspace_turns_the_gradients_into_nan():
     assert all(torch.isnan(x.float()).all() for x in backward())
 
 
+# one look short of the limit for each of many marks: none runs out, and neither does the mbarrier wait behind them
+@pytest.mark.parametrize("limit,looks,waits,expired", [(64, 63, 1, 0), (64, 63, 200, 0), (64, 64, 1, 1), (64, 0, 5, 0),
+                                                       (1, 1, 1, 1), (4096, 4095, 3, 0)])
+def test_looks_at_marks_are_counted_for_one_mark_at_a_time(limit, looks, waits, expired):
+    batch, time, heads = 1, 64, 1
+    workspace = torch.zeros(chunk_kernels.workspace_bytes(batch, time, heads, False), device=DEV, dtype=torch.uint8)
+    status = _lib.lib().gdn2_debug_looks(workspace.data_ptr(), batch, time, heads, limit, looks, waits,
+                                         torch.cuda.current_stream().cuda_stream)
+    assert status == 0
+    assert chunk_kernels.read_status(workspace, batch, time, heads) == expired
+
+
 def test_debug_wait_entry_validates_its_arguments():
     handle = _lib.lib()
     stream = torch.cuda.current_stream().cuda_stream
