@@ -293,6 +293,12 @@ int gdn2_debug_looks(void* workspace, int64_t batch, int64_t full_tokens, int64_
                      int64_t looks, int64_t waits, void* stream);
 
 /*
+ * Test aid: keeps `pairs` pairs of SMs busy for `microseconds` (at most a second), one CTA each that leaves no room for
+ * another kernel's large CTAs, so that a test can see what a call does on the SMs that are left.
+ */
+int gdn2_debug_occupy(int pairs, int64_t microseconds, void* stream);
+
+/*
  * ---- fused input prologue of a layer (next to the primitive, not inside it) ----------------
  *
  * One pass over the [B, T, H, 128] sequence tensors that does what a Gated DeltaNet-2 layer does to
