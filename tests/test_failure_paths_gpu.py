@@ -79,6 +79,30 @@ def test_a_failure_recorded_in_the_workspace_turns_the_gradients_into_nan():
     assert all(torch.isnan(x.float()).all() for x in backward())
 
 
+def test_a_recorded_failure_turns_the_gradients_of_a_joint_backward_into_nan():
+    """The same where reverse scan and VJP share a launch, whose VJP learns of a failure from the status word when it
+    starts and with every mark of the scans; a partial chunk at the end."""
+
+    batch, time, heads, scale = 1, 32 * 64 + 5, 4, 128 ** -0.5
+    full = 33 * 64
+    q, k, v, g, beta, w, s0 = (t.to(DEV) for t in oracle.make_inputs(batch, time, heads, seed=72))
+    _, _, aux = chunk_forward(q, k, v, g, beta, w, s0, scale=scale, return_aux=True)
+
+    def backward():
+        grads = tuple(torch.zeros_like(x) for x in (q, k, v, g, beta, w))
+        d_s0 = torch.zeros_like(s0)
+        chunk_kernels.backward(q, k, v, g, beta, w, aux.workspace, aux.chunk_boundaries, torch.ones_like(v),
+                               torch.ones_like(s0), grads, d_s0, batch, time, heads, full, scale)
+        assert _lib.lib().gdn2_chunk_backward_kernels() == 1
+        torch.cuda.synchronize()
+        return (*grads, d_s0)
+
+    assert all(torch.isfinite(x.float()).all() for x in backward())
+    _expire_a_wait(aux.workspace[0], batch, full, heads)
+    assert chunk_kernels.read_status(aux.workspace, batch, full, heads) == 1
+    assert all(torch.isnan(x.float()).all() for x in backward())
+
+
 # one look short of the limit for each of many marks: none runs out, and neither does the mbarrier wait behind them
 @pytest.mark.parametrize("limit,looks,waits,expired", [(64, 63, 1, 0), (64, 63, 200, 0), (64, 64, 1, 1), (64, 0, 5, 0),
                                                        (1, 1, 1, 1), (4096, 4095, 3, 0)])

@@ -372,3 +372,61 @@ def test_packed_gradients_with_and_without_a_partial_chunk(lengths):
             assert torch.equal(o, out[:, lo:hi]) and torch.equal(f, fin[i:i + 1])
             assert all(torch.equal(a, b[:, lo:hi]) for a, b in zip(gr[:6], grads[:6]))
             assert torch.equal(gr[6], grads[6][i:i + 1])
+
+
+# The queues of units and of scans and the marks lie in scratch that a replay finds as the one before left it: a replay
+# that did not clear them would find every unit taken, or finished before it is.  (The leaves are made on the capturing
+# stream: the autograd engine runs a leaf's last step where the leaf was made.)
+@pytest.mark.parametrize("batch,heads,time", [(1, 16, 40 * 64), (2, 16, 33 * 64 + 7)])
+def test_joint_training_step_replays_from_a_cuda_graph(batch, heads, time):
+    tensors, d_out, _ = _device_inputs(batch, time, heads, seed=12)
+    others, other_d_out, _ = _device_inputs(batch, time, heads, seed=13)
+    expected = []
+    for values, cotangent in ((tensors, d_out), (others, other_d_out)):
+        leaves = [t.clone().requires_grad_(True) for t in values]
+        out, _ = chunk_gdn2(*leaves)
+        expected.append([out.detach(), *torch.autograd.grad(out, leaves, cotangent)])
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        leaves = [t.clone().requires_grad_(True) for t in tensors]
+        cotangent = d_out.clone()
+
+        def step():
+            out, _ = chunk_gdn2(*leaves)
+            return [out, *torch.autograd.grad(out, leaves, cotangent)]
+
+        step()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            launched = _lib.LAUNCHES[0]
+            got = step()
+            assert _lib.lib().gdn2_chunk_forward_kernels() == 1 and _lib.LAUNCHES[0] - launched == 2
+        for turn in (0, 1, 1, 0):
+            with torch.no_grad():
+                for leaf, value in zip(leaves, (tensors, others)[turn]):
+                    leaf.copy_(value)
+                cotangent.copy_((d_out, other_d_out)[turn])
+                for t in got:
+                    t.fill_(float("nan"))
+            graph.replay()
+            stream.synchronize()
+            assert all(torch.equal(a, b) for a, b in zip(got, expected[turn]))
+
+
+# the fewest scans and units that a joint forward has (400 units), and what is its smallest number of preparing CTAs
+@pytest.mark.parametrize("heads,time", [(1, 400 * 64), (3, 134 * 64 + 1), (7, 58 * 64)])
+@pytest.mark.parametrize("raw", [False, True])
+def test_joint_forward_of_few_scans_equals_two_launches(heads, time, raw):
+    tensors, _, _ = _device_inputs(1, time, heads, seed=heads)
+    flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
+    with torch.no_grad():
+        joint = chunk_gdn2(*tensors, output_final_state=True, **flags)
+        assert _lib.lib().gdn2_chunk_forward_kernels() == 1
+        _lib.profile_enable(True)  # times the kernels one by one: never joint
+        try:
+            apart = chunk_gdn2(*tensors, output_final_state=True, **flags)
+            assert _lib.lib().gdn2_chunk_forward_kernels() == 2
+        finally:
+            _lib.profile_enable(False)
+    assert torch.equal(joint[0], apart[0]) and torch.equal(joint[1], apart[1])
