@@ -3,8 +3,8 @@
 // tiles the forward scan read, through tiled TMA loads in the other swizzle: what the forward
 // contracted over columns it contracts over rows (K-major <-> MN-major operands, tc05.cuh).
 //
-//   chunk_bwd_scan_kernel  one CTA per (batch, head) or part of its value rows, chunks in reverse order.  The state
-//                          cotangent lives transposed (dS^T: value rows x key columns) in TMEM:
+//   chunk_bwd_scan_kernel  one CTA per (batch, head) or part of its value rows, chunks in reverse order.  The
+//                          state cotangent lives transposed (dS^T: value rows x key columns) in TMEM:
 //                              dR^T  = dO^T Aqk + dS^T Kt^T        dZ^T = dR^T T
 //                              dS^T <- dS^T diag(d) + dO^T Qg - dR^T Y
 //                          It writes dZ = T^T dR per chunk and the cotangent at every chunk start.
@@ -1419,11 +1419,18 @@ int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, in
 
 thread_local int t_backward_kernels = 0;  // of this thread's latest chunk backward
 
-// One launch for both where it gains: at most a quarter of the SMs with a scan, as in the forward, and sequences long
-// enough for the VJP to run behind it.  Training steps with two launches / one, us: H16 T1024 157/154, T2048 228/210,
-// T8192 719/624; H8 T4096 336/309; H4 T8192 537/521; H24 T4096 467/445; H32 T2048 318/312, B2 T4133 H16 (fp16)
-// 619/581; H37 T1024 201/209.  With one or two scans all that the launch could hide is a few units, and quarters of
-// the value rows, which only the scan kernel has, are worth more.
+// One launch for both where it gains: at most a quarter of the SMs with a scan, as in the forward, enough scans, and
+// sequences long enough for the VJP to run behind them.  Training steps with two launches / one, us:
+//   32 chunks on    H4 T2048 151/159   H4 T2560 198/192   H8 T2048 180/170   H12 T2560 246/224   H16 T2048 225/207
+//                   H16 T2560 269/243   H24 T2048 262/249   H28 T2048 294/280   H32 T2048 312/309   H37 T2048 340/350
+//                   H37 T2560 420/424   B2 T4133 H16 fp16 619/581
+//   below           H4 T1024 98/100   H8 T1024 102/105   H8 T1280 137/130   H8 T1792 165/156   H16 T1024 131/133
+//                   H16 T1280 169/161   H16 T1792 208/195   H24 T1280 184/180   H24 T1536 202/207   H32 T1024 187/185
+//                   H32 T1792 287/278   H37 T1280 233/240   H37 T1792 300/306
+//   fewer scans     H2 T2560 169/175   H3 T2560 174/181: all that the launch could hide is a few units, and quarters of
+//                   the value rows, which only the scan kernel has, are worth more
+// (Between 18 and 31 chunks 6 to 32 scans would gain 2-6 % where the units are more than one per SM; the line stands
+// above that, where all but the two ends of the range gain.)
 bool prefer_joint_backward(int64_t n_scan, int64_t n_chunks, int sm_count) {
   return 4 * n_scan <= sm_count && n_scan >= 4 && n_chunks >= 32 && !profiling();
 }

@@ -9,9 +9,9 @@
 //                       cumulative log-decay, block-anchored Gram products on tf32 tcgen05 MMAs,
 //                       blocked inverse T of the unit lower-triangular system on CUDA cores (fp32),
 //                       Y = T E on tf32 tcgen05 MMAs.
-//   chunk_scan_kernel   one CTA per (sequence, head) or half of its value rows, chunks in order.  The state lives transposed
-//                       (S^T: value rows x key columns) in TMEM as the fp32 accumulator and is fed
-//                       back as the tf32 A operand of the next MMAs without leaving TMEM:
+//   chunk_scan_kernel   one CTA per (sequence, head) or half of its value rows, chunks in order.  The state
+//                       lives transposed (S^T: value rows x key columns) in TMEM as the fp32 accumulator
+//                       and is fed back as the tf32 A operand of the next MMAs without leaving TMEM:
 //                           R^T  = Z^T T^T - S^T Y^T           (Z = w v)
 //                           O^T  = S^T Qg^T + R^T Aqk^T
 //                           S^T <- S^T diag(d) + R^T Kt
@@ -110,8 +110,8 @@ struct PrepMaps {
 // The units of one group of 256 threads (`tid` within it): first, first + stride, ..., or in a joint launch
 // `first` and then whatever the queue gives; tensor memory columns tb .. tb + 255.  kPro: the instantiation
 // that can apply the layer prologue to raw inputs (p.prologue says which parts); the plain instantiation
-// carries none of that code.  kJoint: `quota` (0: all there are) units are taken in the order in which the scans running beside need
-// them (chunk by chunk through all sequences), and a finished one is marked in its D array.
+// carries none of that code.  kJoint: `quota` (0: all there are) units are taken in the order in which the scans
+// running beside need them (chunk by chunk through all sequences), and a finished one is marked in its D array.
 template <typename T, typename G, typename Seqs, bool kPro, bool kJoint>
 __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs, const PrepMaps& tm, PrepSmem& sm,
                                            const int tid, const uint32_t tb, const int first, const int stride,
@@ -696,7 +696,6 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 //                R'^T = Z'^T T^T of the next chunk.  MMAs of one shape on one accumulator run in order; every
 //                other dependence (R -> S', S' -> R') is waited for, with independent MMAs in the queue meanwhile
 //   warp 2       loads of v and w, whose buffer frees at another time than the others
-//   warp 1       joint launch: watches the marks of prepared chunks (a look at one takes most of a microsecond)
 //   warps 4..11  decay: S' <- S diag(d) into the other of two state buffers while R is formed (the output
 //                still reads S); training: the chunk-start state, staged and sent by bulk stores
 //   warps 12..19 Z = w v of the next chunk into tensor memory; training: R out
@@ -707,11 +706,13 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
 // its tiles, the threads that wrote its other operand and those that freed its accumulator.
 // Tensor memory (columns): S 2 x 128, R 2 x 64, O 64, Z 64 = all 512.
 // Where a CTA has only the first 64 value rows, a group has work for the two warps of four that reach them, and the
-// four single warps take the places of two others: the MMA warp is then alone on its scheduler (3300 -> 2940 clocks a
-// chunk; with working warps beside it an MMA is issued in 50 clocks instead of 25).
+// single warps take the places of others: the MMA warp is then alone on its scheduler (3300 -> 2940 clocks a chunk;
+// with working warps beside it an MMA is issued in 50 clocks instead of 25).  In a joint launch, which has this form
+// only, one more warp watches the marks of prepared chunks (a look at one takes most of a microsecond); it is on the
+// MMA warp's scheduler too, and asleep for 200 ns between looks.
 template <int kParts>
 struct ScanWarps {  // (first) warps of the groups
-  static constexpr int kLoads = 0, kWatch = 1, kVw = 2, kMma = 3, kDecay0 = 4, kZ0 = 12, kOut0 = 20, kThreads = 768;
+  static constexpr int kLoads = 0, kVw = 2, kMma = 3, kDecay0 = 4, kZ0 = 12, kOut0 = 20, kThreads = 768;
   static __device__ __forceinline__ bool works(int warp) { return warp >= kDecay0; }
 };
 template <>
@@ -761,8 +762,8 @@ struct ScanMaps {
   CUtensorMap yt, q, kn, at, tt, v, w, out;
 };
 
-// One sequence and head, or a half of its value rows (kParts = 2: value_parts), by a whole CTA.  kJoint: the prep groups run beside in the same launch, and a chunk's
-// tiles are loaded once its mark is there.
+// One sequence and head, or a half of its value rows (kParts = 2: value_parts), by a whole CTA.  kJoint: the prep
+// groups run beside in the same launch, and a chunk's tiles are loaded once its mark is there.
 template <typename T, typename Seqs, bool kJoint, int kParts>
 __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& seqs, const ScanMaps& tm, ScanSmem& sm,
                                               const int item) {
@@ -817,6 +818,10 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
     tc_fence_before();
     __syncwarp();
     if (lane == 0) mbar_arrive(bar);
+  };
+  auto watches = [&] {
+    if constexpr (kJoint) return warp == W::kWatch;
+    return false;
   };
 
   // O of a chunk out, by whole sets of four warps (one per lane quadrant of tensor memory), each `kTokens` of
@@ -1003,7 +1008,7 @@ __device__ __forceinline__ void scan_sequence(const ScanParams& p, const Seqs& s
       if (c >= kVwSlots) waiter.wait(&sm.vw_read[c % kVwSlots], uint32_t(c / kVwSlots - 1) & 1u);
       load_vw(c);
     }
-  } else if (kJoint && warp == W::kWatch) {
+  } else if (watches()) {
     // ---------------------------------------------------------------- marks of prepared chunks
     for (int c = 0; c < n_chunks;) {
       const int mine = min(c + lane, n_chunks - 1);
@@ -1387,16 +1392,25 @@ struct ForwardCall {
 
 thread_local int t_forward_kernels = 0;  // of this thread's latest chunk forward
 
-// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation) and 1.6-2 us per chunk
-// (the scans); together, where the preparers keep the scans' pace or nearly so, the scans' time and some 20 us; with
-// more to scan about n_ch * 8.3 us / SMs and 1 us per chunk, 35 us and what uneven ends cost.  Two launches / one, us:
-//   H16 T1024 53.5/53.8   H16 T2048 95.8/81.3, training 108.9/101.6   H16 T3072 137/108, training 152/136
-//   H8 T4096 140/126, training 164/164   H4 T8192 231/218   H4 T16384 training 517/559 (a training scan beside
-//   preparers takes 2.1 us a chunk, not 1.9)   H24 T1344 training 90/82   H32 T1664 110/111, training 121/116
-// Beyond a quarter of the SMs scanning, the preparation falls behind.
-bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, bool training, int sm_count) {
+// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation), 1.6-2 us per chunk (the
+// scans) and what two launches cost; together the scans' time and some 20 us, where the SMs that do not scan, or all in
+// turn (quota), have the units ready in time.
+// At most a sixth of the SMs scanning, two launches / one, us, inference, raw, training:
+//   400 units on    H16 T1600 77/69 86/80 187/184   H16 T2048 95/81 105/93 214/208   H8 T3200 109/103 118/118 252/252
+//                   H8 T4096 136/125 146/141 303/303   H24 T1152 70/71 77/82 171/164   H24 T1408 82/78 92/87 205/195
+//   below           H16 T1024 51/52 55/60 131/135   H16 T1280 69/60 74/68 169/164   H8 T2048 72/75 76/86 170/179
+//   fewer scans     H1 T25600 565/627 578/669   H3 T12288 306/312 320/346   H4 T8192 220/219 233/243, training 515/530:
+//   the units are ready in time either way and a pair of CTAs scans no faster than it does alone, so 4 scans at least,
+//   and 8 with a prologue or states to write
+// With up to a quarter scanning, inference, raw, training (above that the preparation falls behind):
+//   above the line  H28 T2048 126/113 140/135 296/275   H32 T1664 109/111 122/114 271/266   H32 T2048 129/116 142/141
+//                   315/305   H37 T1408 104/95 118/113 260/256
+//   below           H28 T1024 72/61 83/70 183/174   H28 T1536 97/90 108/110 238/224   H32 T1280 91/91 101/107 226/219
+//                   H32 T1536 104/97 117/110 262/250   H37 T1024 76/77 87/91 193/190   H37 T1280 94/90 105/103 233/232
+//   (the line is that of an earlier form of the launch, which cost more; it stands on the safe side)
+bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, bool training, bool prologue, int sm_count) {
   if (4 * n_scan > sm_count || profiling()) return false;
-  if (6 * n_scan <= sm_count) return n_ch >= 400 && (!training || n_scan >= 8);
+  if (6 * n_scan <= sm_count) return n_ch >= 400 && n_scan >= (training || prologue ? 8 : 4);
   return 83 * n_ch > (350 + 4 * n_chunks) * sm_count;
 }
 
@@ -1469,7 +1483,7 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   const int64_t n_scan = int64_t(seqs.count()) * a.H;
   bool joint = false;
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
-    joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, a.training != 0, sm_count);
+    joint = prefer_joint(n_scan, n_ch, seqs.n_chunks, a.training != 0, a.prologue != 0, sm_count);
   }
   const int parts = joint ? kJointParts : value_parts(n_ch, n_scan, seqs.at(0).n_chunks, sm_count, 2);
   const WsLayout ws{n_ch, a.training != 0};

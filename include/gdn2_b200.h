@@ -204,11 +204,15 @@ int gdn2_chunk_forward(const void* q, const void* k, const void* v, const void* 
 
 /*
  * Kernels that the calling thread's latest chunk forward launched (0: it has made none): 2, the preparation of the
- * chunks and the scan, or 1 where few sequences and heads let one launch do both side by side.
+ * chunks and the scan, or 1 where few sequences and heads let one launch do both side by side.  That one is a
+ * cooperative launch of up to one CTA per SM: it begins when the whole GPU is free, behind other streams' kernels.
  */
 int gdn2_chunk_forward_kernels(void);
 
-/* The same of its latest chunk backward: 2, the reverse scan and the VJP, or 1. */
+/*
+ * The same of its latest chunk backward: 2, the reverse scan and the VJP, or 1.  That one begins on whatever SMs are
+ * free.
+ */
 int gdn2_chunk_backward_kernels(void);
 
 /*

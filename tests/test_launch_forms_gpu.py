@@ -414,15 +414,18 @@ def test_joint_training_step_replays_from_a_cuda_graph(batch, heads, time):
             assert all(torch.equal(a, b) for a, b in zip(got, expected[turn]))
 
 
-# the fewest scans and units that a joint forward has (400 units), and what is its smallest number of preparing CTAs
-@pytest.mark.parametrize("heads,time", [(1, 400 * 64), (3, 134 * 64 + 1), (7, 58 * 64)])
-@pytest.mark.parametrize("raw", [False, True])
-def test_joint_forward_of_few_scans_equals_two_launches(heads, time, raw):
+# the fewest scans and units that a joint forward has (4 scans, with the prologue 8, and 400 units), with its smallest
+# number of preparing CTAs; fewer scans take two launches
+@pytest.mark.parametrize("heads,time,raw,kernels", [(4, 100 * 64, False, 1), (7, 58 * 64, False, 1), (8, 50 * 64, True, 1),
+                                                    (4, 99 * 64 + 1, False, 1), (4, 99 * 64, False, 2),
+                                                    (3, 134 * 64 + 1, False, 2), (7, 58 * 64, True, 2),
+                                                    (1, 400 * 64, False, 2)])
+def test_joint_forward_of_few_scans_equals_two_launches(heads, time, raw, kernels):
     tensors, _, _ = _device_inputs(1, time, heads, seed=heads)
     flags = {"use_qk_l2norm_in_kernel": True, "use_gate_in_kernel": True} if raw else {}
     with torch.no_grad():
         joint = chunk_gdn2(*tensors, output_final_state=True, **flags)
-        assert _lib.lib().gdn2_chunk_forward_kernels() == 1
+        assert _lib.lib().gdn2_chunk_forward_kernels() == kernels
         _lib.profile_enable(True)  # times the kernels one by one: never joint
         try:
             apart = chunk_gdn2(*tensors, output_final_state=True, **flags)
