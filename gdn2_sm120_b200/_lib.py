@@ -55,7 +55,6 @@ _PROTOTYPES: dict[str, list] = {
     "gdn2_chunk_read_status": [_P] + [_I64] * 3 + [_P],
     "gdn2_debug_wait_expires": [_P] + [_I64] * 4 + [_P],
     "gdn2_debug_looks": [_P] + [_I64] * 6 + [_P],
-    "gdn2_debug_occupy": [_INT, _I64, _P],
     "gdn2_token_forward_fused": [_P] * 9 + [_I64] * 5 + [_INT, _INT, _F32, _INT, _P],
     "gdn2_token_forward_t1_zero_fused": [_P] * 6 + [_I64] * 2 + [_INT, _F32, _INT, _P],
     "gdn2_chunk_forward_fused": [_P] * 11 + [_I64] * 4 + [_INT, _INT, _F32, _INT, _P],

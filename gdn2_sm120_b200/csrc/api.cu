@@ -42,7 +42,6 @@ int launch_chunk_backward(const void*, const void*, const void*, const void*, co
                           int, float, int, cudaStream_t);
 int launch_debug_wait_expires(int* status, uint32_t max_polls, cudaStream_t stream);
 int launch_debug_looks(int* status, uint32_t limit, uint32_t looks, uint32_t waits, cudaStream_t stream);
-int launch_debug_occupy(int pairs, int64_t us, cudaStream_t stream);
 int launch_gate_prologue(const void*, const void*, const void*, const void*, const void*, void*, void*, void*,
                          void*, void*, float*, float*, int64_t, int, int, cudaStream_t);
 int launch_gate_prologue_vjp(const void*, const void*, const void*, const void*, const void*, const float*,
@@ -516,11 +515,6 @@ int gdn2_debug_looks(void* workspace, int64_t batch, int64_t full_tokens, int64_
   int* status = reinterpret_cast<int*>(static_cast<uint8_t*>(workspace) +
                                        chunk_status_offset(batch, full_tokens, heads));
   return launch_debug_looks(status, uint32_t(limit), uint32_t(looks), uint32_t(waits), static_cast<cudaStream_t>(stream));
-}
-
-int gdn2_debug_occupy(int pairs, int64_t microseconds, void* stream) {
-  if (pairs < 1 || pairs > 512 || microseconds < 0 || microseconds > 1000000) return GDN2_ERR_BAD_SHAPE;
-  return launch_debug_occupy(pairs, microseconds, static_cast<cudaStream_t>(stream));
 }
 
 }  // extern "C"

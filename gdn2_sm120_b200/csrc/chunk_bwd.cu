@@ -25,7 +25,6 @@
 
 #include <cuda.h>
 
-#include <cstddef>
 #include <type_traits>
 
 #include "chunk_common.cuh"
@@ -84,8 +83,7 @@ struct BScanSmem {
 static_assert(sizeof(BScanSmem) <= 232448, "reverse scan exceeds the 227 KiB shared-memory limit");
 
 // Joint launch: the last 16 bytes of a dZ tile, behind its last row, belong to nobody.  Word 0 counts the CTAs
-// of the scan that have left in memory what the VJP reads of the unit; the first unit's word 1 is the queue of units,
-// its word 2 the queue of scans.
+// of the scan that have left in memory what the VJP reads of the unit; the first unit's word 1 is the queue of units.
 constexpr int64_t kMarkOffset = kBlobDZ - 16;
 struct Marks {
   uint8_t* dz;
@@ -112,7 +110,7 @@ struct BScanMaps {
 };
 
 // One sequence and head, or a part of its value rows (value_parts), by a whole CTA.  kJoint: the VJP of finished
-// chunks runs beside in the same launch, and this CTA scans again or joins it afterwards.
+// chunks runs beside in the same launch, and this CTA joins it afterwards.
 template <typename T, typename Seqs, bool kJoint, int kParts>
 __device__ __forceinline__ void reverse_sequence(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm,
                                                  BScanSmem& sm, const int item) {
@@ -550,7 +548,6 @@ struct VjpMisc {
   int failed;             // joint launch: a wait of the scan ran out, or the wait for it
 };
 constexpr int kVjpSmemBytes = kOffMisc + int(sizeof(VjpMisc));
-static_assert(kOffMisc + offsetof(VjpMisc, next) >= sizeof(BScanSmem), "a slot beside the scans");
 static_assert(kVjpSmemBytes <= 232448, "VJP kernel exceeds the 227 KiB shared-memory limit");
 
 __device__ __forceinline__ int kit_rs(int I) { return 512 * (I + 1) + 16; }
@@ -657,12 +654,12 @@ struct VjpMaps {
 // Reverse scan and VJP in one launch.  With few sequences and heads the reverse scan keeps a few SMs busy, 1.9-2.2 us
 // per chunk, and the VJP of a chunk needs nothing but that chunk's share of it.  Here the scans run on pairs of CTAs (a
 // half of the value rows each) and all other CTAs, and at last these too, take the units from a queue, last chunks
-// first, waiting for the scans' marks.  The scans wait for nobody, and a pair draws one scan after the other until all
-// are drawn before it goes on with the VJP: whoever waits for a mark waits for a CTA that runs, so that the launch may
-// begin on whatever SMs are free beside another stream's work.  (As a cooperative launch it began when the whole GPU
-// was free.)  A unit's scratch tiles and cotangents are still in L2 when the VJP reads them.  Whatever waits for memory
-// on behalf of a mark is kept off the scan's chain and the VJP's: by the scanning warps themselves it cost a chunk 1.2
-// us, by the thread that issues the VJP's copies a unit 1500 clocks.
+// first, waiting for the scans' marks.  The scans wait for nobody; the launch is cooperative, so that all CTAs are
+// resident together: it begins when every SM is free.  (Pairs that draw scans from a queue, and need no others beside
+// them, can begin on the SMs that are free; every step took 10-12 us more, B1 T2048 H16 207 -> 218, H32 T8192 1046 ->
+// 1059.)  A unit's scratch tiles and cotangents are still in L2 when the VJP reads them.  Whatever waits for memory on
+// behalf of a mark is kept off the scan's chain and the VJP's: by the scanning warps themselves it cost a chunk 1.2 us,
+// by the thread that issues the VJP's copies a unit 1500 clocks.
 constexpr int kJointParts = 2;
 template <bool kJoint>
 struct JointScan {
@@ -671,22 +668,6 @@ struct JointScan {
 };
 template <>
 struct JointScan<false> {};
-
-// The next number of a queue for a cluster of two.
-__device__ __forceinline__ int draw(unsigned* queue, int* slot) {
-  uint32_t rank, first_slot;
-  int number;
-  auto cluster_sync = [] {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-  };
-  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  if (rank == 0 && threadIdx.x == 0) *slot = int(atomicAdd(queue, 1u));
-  cluster_sync();
-  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(first_slot) : "r"(smem_u32(slot)));
-  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(number) : "r"(first_slot) : "memory");
-  cluster_sync();  // the slot is read: it may become something else
-  return 2 * number + int(rank);
-}
 
 // The queue of units of a joint launch, and the marks of those that the scans have finished.
 template <typename Seqs>
@@ -733,10 +714,9 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
   extern __shared__ __align__(1024) uint8_t smem[];
   if constexpr (kJoint) {
     static_assert(BScanWarps<kJointParts>::kThreads == kVjpThreads, "a scanning CTA goes on with the VJP");
-    static_assert(kJointParts == 2, "a cluster of two shares a scan");
-    int* const slot = &reinterpret_cast<VjpMisc*>(smem + kOffMisc)->next[0];
-    for (int item; (item = draw(scan.p.marks.of(0) + 2, slot)) < kJointParts * seqs.count() * p.H;) {
-      reverse_sequence<T, Seqs, true, kJointParts>(scan.p, seqs, scan.tm, *reinterpret_cast<BScanSmem*>(smem), item);
+    if (int(blockIdx.x) < kJointParts * seqs.count() * p.H) {
+      reverse_sequence<T, Seqs, true, kJointParts>(scan.p, seqs, scan.tm, *reinterpret_cast<BScanSmem*>(smem),
+                                                   int(blockIdx.x));
       fence_async_smem();
       __syncthreads();
     }
@@ -1450,13 +1430,19 @@ int launch_joint(const BScanParams& sp, const VjpParams& vp, const UniformSeqs& 
   config.blockDim = dim3(kVjpThreads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  cudaLaunchAttribute pairs;
-  pairs.id = cudaLaunchAttributeClusterDimension;
-  pairs.val.clusterDim.x = 2;
-  pairs.val.clusterDim.y = pairs.val.clusterDim.z = 1;
-  config.attrs = &pairs;
-  config.numAttrs = 1;
+  cudaLaunchAttribute attributes[2];
+  attributes[0].id = cudaLaunchAttributeCooperative;
+  attributes[0].val.cooperative = 1;
+  attributes[1].id = cudaLaunchAttributeClusterDimension;
+  attributes[1].val.clusterDim.x = 2;
+  attributes[1].val.clusterDim.y = attributes[1].val.clusterDim.z = 1;
+  config.attrs = attributes;
+  config.numAttrs = 2;
   err = cudaLaunchKernelEx(&config, kernel, vp, seqs, tm_vjp, JointScan<true>{sp, tm_scan});
+  if (err == cudaErrorCooperativeLaunchTooLarge) {  // a context with fewer SMs than the device
+    (void)cudaGetLastError();
+    return GDN2_ERR_UNSUPPORTED;
+  }
   if (err != cudaSuccess) { (void)cudaGetLastError(); record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   return GDN2_OK;
 }
@@ -1514,15 +1500,17 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
   }
   const VjpParams vp{a.q, a.k, a.v, a.g, a.beta, a.w, a.d_out, a.scratch, a.dq, a.dk, a.dv, a.dg,
                      a.dbeta, a.dw, status, n_ch, int(a.H), a.scale};
-  int st = GDN2_OK;
+  int st = GDN2_ERR_UNSUPPORTED;
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
     if (joint) {
       GDN2_DISPATCH_TYPES(a.dtype, a.g_dtype, {
         st = a.ragged ? launch_joint<T, G, true>(sp, vp, seqs, tm, m, sm_count, stream)
                       : launch_joint<T, G, false>(sp, vp, seqs, tm, m, sm_count, stream);
       });
-      t_backward_kernels = 1;
-      return st;
+      if (st != GDN2_ERR_UNSUPPORTED) {
+        t_backward_kernels = 1;
+        return st;
+      }
     }
   }
   st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)

@@ -26,7 +26,7 @@
 //   dZ   X[r = token j (64)][c = value v (128)] RS = 4608, CS = 144   36 KiB   dZ = T^T dR
 //        (reverse scan -> VJP kernel; the padded strides are those of the tile it is copied into.  The 16 bytes
 //        behind the last row are padding too: where the two share a launch they hold the unit's mark and, in the
-//        first tile, the queues of units and of scans)
+//        first tile, the queue of units)
 //
 // Buffers (caller-provided, struct of arrays, each array n_ch entries long):
 //   workspace  D, a 256-byte status block, and for a training call what backward consumes:

@@ -1328,26 +1328,7 @@ __global__ void __launch_bounds__(32, 1) debug_looks_kernel(int* status, uint32_
   waiter.wait(&bar, 0);
 }
 
-// Pairs of CTAs that take a whole SM each and leave after `us` microseconds (or 2^24 looks at the clock).
-__global__ void __launch_bounds__(32, 1) __cluster_dims__(2, 1, 1) debug_occupy_kernel(uint64_t us) {
-  auto now = [] {
-    uint64_t t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-  };
-  const uint64_t start = now();
-  for (uint32_t looks = 0; looks < (1u << 24) && now() - start < 1000 * us; ++looks) __nanosleep(1000);
-}
-
 }  // namespace
-
-int launch_debug_occupy(int pairs, int64_t us, cudaStream_t stream) {
-  const int smem = 200 * 1024;
-  const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(debug_occupy_kernel), smem);
-  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  debug_occupy_kernel<<<unsigned(2 * pairs), 32, smem, stream>>>(uint64_t(us));
-  return check_launch();
-}
 
 int launch_debug_looks(int* status, uint32_t limit, uint32_t looks, uint32_t waits, cudaStream_t stream) {
   debug_looks_kernel<<<1, 32, 0, stream>>>(status, limit, looks, waits);

@@ -209,10 +209,7 @@ int gdn2_chunk_forward(const void* q, const void* k, const void* v, const void* 
  */
 int gdn2_chunk_forward_kernels(void);
 
-/*
- * The same of its latest chunk backward: 2, the reverse scan and the VJP, or 1.  That one begins on whatever SMs are
- * free.
- */
+/* The same of its latest chunk backward: 2, the reverse scan and the VJP, or 1, cooperative like the forward's. */
 int gdn2_chunk_backward_kernels(void);
 
 /*
@@ -295,12 +292,6 @@ int gdn2_debug_wait_expires(void* workspace, int64_t batch, int64_t full_tokens,
  */
 int gdn2_debug_looks(void* workspace, int64_t batch, int64_t full_tokens, int64_t heads, int64_t limit,
                      int64_t looks, int64_t waits, void* stream);
-
-/*
- * Test aid: keeps `pairs` pairs of SMs busy for `microseconds` (at most a second), one CTA each that leaves no room for
- * another kernel's large CTAs, so that a test can see what a call does on the SMs that are left.
- */
-int gdn2_debug_occupy(int pairs, int64_t microseconds, void* stream);
 
 /*
  * ---- fused input prologue of a layer (next to the primitive, not inside it) ----------------

@@ -6,7 +6,6 @@ unit of each case is held against the oracle with the tolerances of test_autogra
 from __future__ import annotations
 
 import threading
-import time as time_module
 
 import pytest
 import torch
@@ -193,41 +192,6 @@ def test_joint_backward_never_reads_ahead_of_a_mark(batch, heads, time):
         assert all(torch.equal(a, b) for a, b in zip(grads, first))
 
 
-# One pair of SMs, half of them or all but three busy for half a second with another stream's kernel: the backward goes
-# on beside it, with room for all of its scans at once or for a few.
-@pytest.mark.parametrize("batch,heads,time", [(1, 4, 32 * 64), (1, 37, 32 * 64 + 9)])
-@pytest.mark.parametrize("busy_pairs", [1, 37, 71])
-def test_joint_backward_runs_beside_another_kernel(batch, heads, time, busy_pairs):
-    (q, k, v, g, beta, w, s0), d_out, d_fin = _device_inputs(batch, time, heads, seed=time)
-    scale, full = 128 ** -0.5, -(-time // 64) * 64
-    _, _, aux = chunk_forward(q, k, v, g, beta, w, s0, scale=scale, return_aux=True)
-    slots = torch.empty((batch, full // 64 + 1, heads, 128, 128), device=DEV)
-    scratch = torch.empty(chunk_kernels.scratch_bytes(batch, full, heads, True), device=DEV, dtype=torch.uint8)
-
-    def backward(grads):
-        _lib.call("gdn2_chunk_backward", q.device, *[x.data_ptr() for x in (q, k, v, g, beta, w, d_out, d_fin)],
-                  aux.chunk_boundaries.data_ptr(), slots.data_ptr(), aux.workspace[0].data_ptr(), scratch.data_ptr(),
-                  *[x.data_ptr() for x in grads], batch, time, heads, full, _lib.dtype_code(q.dtype),
-                  _lib.dtype_code(g.dtype), scale, _lib.stream_ptr(q.device))
-        assert _lib.lib().gdn2_chunk_backward_kernels() == 1
-
-    expected, grads = ([torch.zeros_like(x) for x in (q, k, v, g, beta, w, s0)] for _ in range(2))
-    backward(expected)
-    torch.cuda.synchronize()
-    other, busy, done = torch.cuda.Stream(), torch.cuda.Event(), torch.cuda.Event()
-    with torch.cuda.stream(other):
-        assert _lib.lib().gdn2_debug_occupy(busy_pairs, 500_000, other.cuda_stream) == 0
-        busy.record()
-    time_module.sleep(0.05)  # until they are all there
-    assert not busy.query()
-    backward(grads)
-    done.record()
-    done.synchronize()
-    assert not busy.query()
-    torch.cuda.synchronize()
-    assert all(torch.equal(a, b) for a, b in zip(grads, expected))
-
-
 # 255 .. 257 and 513: around one and two launch tables of 256 sequences
 @pytest.mark.parametrize("count", [255, 256, 257, 513])
 def test_packed_batches_around_the_table_size(count):
@@ -374,7 +338,7 @@ def test_packed_gradients_with_and_without_a_partial_chunk(lengths):
             assert torch.equal(gr[6], grads[6][i:i + 1])
 
 
-# The queues of units and of scans and the marks lie in scratch that a replay finds as the one before left it: a replay
+# The queue of units and the marks lie in scratch that a replay finds as the one before left it: a replay
 # that did not clear them would find every unit taken, or finished before it is.  (The leaves are made on the capturing
 # stream: the autograd engine runs a leaf's last step where the leaf was made.)
 @pytest.mark.parametrize("batch,heads,time", [(1, 16, 40 * 64), (2, 16, 33 * 64 + 7)])
