@@ -592,34 +592,7 @@ __device__ __forceinline__ void store4v<__half>(void* base, int64_t idx, float a
       make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
 }
 
-// Two fp32 operations per instruction (each rounded like the scalar one): the VJP kernel's elementwise phases
-// are bound by instruction issue.
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-  return d;
-}
-__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
-  float2 d;
-  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-      "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
-      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
-  return d;
-}
-__device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
-__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return fma2(b, twice(-1.f), a); }
-__device__ __forceinline__ float2 exp2_2(float2 x) { return make_float2(exp2_approx(x.x), exp2_approx(x.y)); }
 __device__ __forceinline__ float2 tf32_2(float2 x) { return make_float2(to_tf32(x.x), to_tf32(x.y)); }
-__device__ __forceinline__ float2 tf32_operand_2(float2 x) { return make_float2(to_tf32_operand(x.x), to_tf32_operand(x.y)); }
 
 // The value of k times its anchored decay, `decay` alone or `decay * far` for row blocks beyond the next one:
 // the chain calls this with the factors of the tile build, so that it multiplies the Gram cotangents by

@@ -266,14 +266,14 @@ inline bool encode_sequence_map(CUtensorMap* tm, const void* base, int64_t rows,
   return encode_cached(tm, 3, type, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
 }
 
-// The same tensor (16-bit) seen as (channel within 32, row, group of 32 channels, head): a box (32, 64, 4, 1) is
-// one head's chunk, landing as [group][64][32].
-inline bool encode_round_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t heads, int dtype) {
-  const cuuint64_t dims[4] = {32, cuuint64_t(rows), kDim / 32, cuuint64_t(heads)};
-  const cuuint64_t strides[3] = {cuuint64_t(heads) * kDim * 2, 64, kDim * 2};
-  const cuuint32_t box[4] = {32, kChunk, kDim / 32, 1};
+// The same tensor (16-bit) seen as (channel within 64, row, half of the channels, head): a box (64, 64, 2, 1) is one
+// head's chunk, landing as [half][64] lines of 128 bytes whose 16-byte pieces are permuted by the line.
+inline bool encode_half_map(CUtensorMap* tm, const void* base, int64_t rows, int64_t heads, int dtype) {
+  const cuuint64_t dims[4] = {64, cuuint64_t(rows), kDim / 64, cuuint64_t(heads)};
+  const cuuint64_t strides[3] = {cuuint64_t(heads) * kDim * 2, 128, kDim * 2};
+  const cuuint32_t box[4] = {64, kChunk, kDim / 64, 1};
   return encode_cached(tm, 4, dtype == GDN2_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16,
-                       base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_NONE);
+                       base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
 // An array of n_ch row-major fp32 tiles [rows][cols] seen as (column within a slab, row, slab of 32

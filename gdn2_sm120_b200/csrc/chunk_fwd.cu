@@ -50,40 +50,47 @@ namespace {
 // 32 channels at a time, and everything else shares their place.  (In two rounds of 64 channels the inputs
 // waiting for the second spilled: 115 KB a unit through L2, as much as the tiles themselves.)
 //
-// A thread owns 2 tokens x 4 channels of each round: tokens 8 warp + lane / 8 and 4 further on, channels
-// 4 (lane % 8): one 16-byte chunk of every tile row.  The eight lanes of a store phase fill one 128-byte line.
+// What a unit takes is what passes through the load/store unit of shared memory (10 thousand wavefronts of 128 bytes a
+// unit in an earlier form, where a unit took 14 thousand clocks of an SM), so the layouts below are chosen for few of
+// them.  A thread owns 4 consecutive tokens x 2 channels of each round: tokens 8 warp + 4 (lane / 16), channels
+// 2 (lane % 16).  Sums along the tokens need no shuffles, a 16-lane row of a store phase fills a 128-byte line, and what
+// depends on a channel alone is read once for four tokens.
 constexpr int kPrepThreads = 256;
 constexpr int kJointParts = 2;
 constexpr int kRound = 32, kRounds = kDim / kRound;  // channels per round
-constexpr int kLd = 68;           // leading dimension of the fp32 64x64 scratch matrices (16-byte rows, banks shift by 4)
-constexpr int kLdW = 20;          // leading dimension of the transposed 16x16 block products
+constexpr int kLdQ = 36;          // leading dimension of a transposed 32 x 32 block (16-byte rows, banks shift by 4)
 
 // One region, by phase (bytes):
-//   inputs       g at 0 (16 or 32 KiB), dense rows; k, q, beta (16 KiB each) by rounds, [round][64][32]
+//   inputs       g at 0 (16 or 32 KiB), dense rows; k, q, beta (16 KiB each), 2 slabs of 64 lines of 64 channels,
+//                16-byte pieces permuted by the line: the rows of both halves of a warp are then in other banks
+//                (lines of 32 channels would be too, but the copy engine is paid by the line)
 //   rounds       A operand [E_anchored ; Q_anchored], 128 lines of 32 channels, B operands K^I, 16 (I + 1) lines
 //                each (K-major, 128-byte swizzle); E[j][k], tf32, MN-major operand, 4 swizzled slabs of 32
 //                channels x 64 lines (tc05.cuh) over k and q: slab r is written once rounds r and r + 1 have
 //                been read, hence the order 0, 2, 1, 3
-//   inverse      fp32 T and T^T over the Gram operands, L over beta, block products over the decay table; the
-//                tf32 T tile replaces L
-// The next unit's g arrives over T and T^T under the last MMA, its k, q and beta after it.
+//   inverse      -L^T over beta, T's diagonal blocks behind the next unit's g, T^T as a tf32 tile
+//   last product Y^T on its way out, over -L^T and T^T
+// The next unit's g arrives over the Gram operands under the inverse, its k and q after the last product, its beta
+// once Y^T has left.
 constexpr int kOffGramA = 0, kOffGramB = 16384;                         // + 20480
 constexpr int kOffTable = 36864;                                        // decay table, 13 rows of 128
-constexpr int kOffInG = 0, kOffInK = 47104, kOffInQ = kOffInK + 16384, kOffInBeta = kOffInQ + 16384;
+constexpr int kOffInG = 0, kOffInK = 44032, kOffInQ = kOffInK + 16384, kOffInBeta = kOffInQ + 16384;
 constexpr int kOffE = kOffInK;
-constexpr int kOffTn = 0, kOffTc = kOffTn + 64 * kLd * 4;               // 17408 each
-constexpr int kOffLn = kOffInBeta, kOffTmat = kOffLn;
-constexpr int kOffWt = kOffTable;
-constexpr int kPrepRegion = kOffLn + 64 * kLd * 4;                      // 97280
-static_assert(kOffTc + 64 * kLd * 4 <= kOffTable && kOffWt + 2 * 16 * kLdW * 4 <= kOffE && kOffTable + 13 * 512 <= kOffE,
-              "prep region");
-static_assert(kOffE % 1024 == 0 && kOffGramB % 1024 == 0, "swizzled tiles are 1024-byte aligned");
+constexpr int kOffLt = kOffInBeta;                                      // -L^T, [64][64]
+constexpr int kOffW = kOffLt + 32 * 64 * 4;                             // over its lines 32.., columns ..32: the block product
+constexpr int kOffP = 32768, kOffQt = kOffP + 4096;                     // T[..32][..32], T[32..][32..] transposed
+constexpr int kOffTt = kOffLt + 16384;                                  // T^T[j][i], MN-major operand, 2 swizzled slabs of 64 lines
+constexpr int kOffY = kOffLt;                                           // Y^T[k][i], 2 swizzled slabs of 128 lines
+constexpr int kPrepRegion = kOffTt + 16384;                             // 109568
+static_assert(kOffTable + 13 * 512 <= kOffE && kOffQt + 32 * kLdQ * 4 <= kOffE && kOffY + 32768 <= kPrepRegion, "prep region");
+static_assert(kOffE % 1024 == 0 && kOffGramB % 1024 == 0 && kOffTt % 1024 == 0 && kOffY % 1024 == 0,
+              "swizzled tiles are 1024-byte aligned");
 
 struct PrepSmem {
   alignas(1024) uint8_t region[kPrepRegion];
-  float part[8][kDim];                 // per 8-token group sums -> exclusive prefixes
+  float part[8][kDim];                 // sums of g over groups of 8 tokens, then what precedes them in their block
   float gend[kDim];
-  alignas(8) uint64_t bar[2];          // MMA commits
+  alignas(8) uint64_t bar[2];          // MMA commits (the second one: and T^T has left)
   alignas(8) uint64_t bar_ld[2];       // raw inputs: {g} and {k, q, beta}
   int next[2];                         // joint launch: the unit after this one (two slots: one may still be read)
   uint32_t tmem_base;
@@ -105,6 +112,7 @@ __device__ __forceinline__ int gram_col(int I) { return (I == 0) ? 0 : (I == 1) 
 
 struct PrepMaps {
   CUtensorMap g, k, q, beta;
+  CUtensorMap out_tt, out_yt;  // tiles that leave by tiled stores
 };
 
 // The units of one group of 256 threads (`tid` within it): first, first + stride, ..., or in a joint launch
@@ -127,12 +135,13 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   };
   if (tid == 0) {
     mbar_init(&sm.bar[0], 1);
-    mbar_init(&sm.bar[1], 1);
+    mbar_init(&sm.bar[1], 2);
     mbar_init(&sm.bar_ld[0], 1);
     mbar_init(&sm.bar_ld[1], 1);
     fence_mbar_init();
   }
-  const int i0 = 8 * warp + (lane >> 3), cl = lane & 7;  // tokens i0 and i0 + 4
+  constexpr int kMmaWarp = 6, kCopyWarp = 7;  // (the first warps have more to write)
+  const int i0 = 8 * warp + 4 * (lane >> 4), cl = lane & 15;  // tokens i0 .. i0 + 3
   const int mb = warp >> 1;                   // 16-token block of this warp's tokens
   const int q4 = warp & 3, part = warp >> 2;  // TMEM lane quadrant of this warp, and its half of the columns
 
@@ -153,36 +162,48 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
       return Place{unit, unit - chunk * heads, int(sq.row0) + t_, min(kChunk, sq.len - t_)};
     }
   };
+  const uint32_t leader = elect_leader();
   auto issue_g = [&](const Place& at) {
-    mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)));
-    tma_load_3d(R + kOffInG, &tm.g, 0, at.h, at.row, &sm.bar_ld[0]);
+    mbar_arrive_expect_tx(&sm.bar_ld[0], uint32_t(kChunk * kDim * sizeof(G)), leader);
+    tma_load_3d(R + kOffInG, &tm.g, 0, at.h, at.row, &sm.bar_ld[0], leader);
   };
-  auto issue_kqb = [&](const Place& at) {
-    mbar_arrive_expect_tx(&sm.bar_ld[1], 3 * kStageTile16);
-    tma_load_4d(R + kOffInK, &tm.k, 0, at.row, 0, at.h, &sm.bar_ld[1]);
-    tma_load_4d(R + kOffInQ, &tm.q, 0, at.row, 0, at.h, &sm.bar_ld[1]);
-    tma_load_4d(R + kOffInBeta, &tm.beta, 0, at.row, 0, at.h, &sm.bar_ld[1]);
+  auto issue_kq = [&](const Place& at) {
+    mbar_arrive_expect_tx(&sm.bar_ld[1], 3 * kStageTile16, leader);  // (beta among them)
+    tma_load_4d(R + kOffInK, &tm.k, 0, at.row, 0, at.h, &sm.bar_ld[1], leader);
+    tma_load_4d(R + kOffInQ, &tm.q, 0, at.row, 0, at.h, &sm.bar_ld[1], leader);
   };
+  auto issue_b = [&](const Place& at) { tma_load_4d(R + kOffInBeta, &tm.beta, 0, at.row, 0, at.h, &sm.bar_ld[1], leader); };
   sync();
-  if (tid == 0 && first < n_ch) {
+  if (warp == kCopyWarp && first < n_ch) {
     const Place at = locate(first);
     issue_g(at);
-    issue_kqb(at);
+    issue_kq(at);
+    issue_b(at);
   }
-  const uint32_t leader = elect_leader();
-  const bool wide_tiles = (reinterpret_cast<uintptr_t>(p.tiles.yt) & 31) == 0;  // (a tile is 32 KiB)
+  [[maybe_unused]] const bool wide_tiles = (reinterpret_cast<uintptr_t>(p.tiles.yt) & 31) == 0;  // (a tile is 32 KiB)
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
-  using RawG = typename Raw4<G>::type;
-  using RawT = typename Raw4<T>::type;
-
+  using RawG = typename Raw2<G>::type;
+  using RawT = typename Raw2<T>::type;
   uint32_t par = 0;
+  // joint launch, the copying warp: the unit after this one, and one whose tiles are on their way out, with its mark
+  [[maybe_unused]] int popped = 0, leaving = -1;
+  [[maybe_unused]] float mark = 0.f;
+  auto set_mark = [&] {
+    if constexpr (kJoint) {
+      bulk_wait_all();
+      fence_async_all();
+      if (lane == 0 && leaving >= 0) {
+        store_release(reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(leaving) * kBlobD), mark);
+      }
+    }
+  };
   for (int unit = first, unit_next; unit < n_ch; unit = unit_next, par ^= 1u) {
   // a queue and not a stride: an SM that shares its way to L2 with a scan prepares at little more than half
   // the pace of the others, and the scans wait for the slowest
   unit_next = unit + stride;
   if constexpr (kJoint) {
-    if (tid == 32) sm.next[par] = unit_next = --quota != 0 ? stride + atomicAdd(queue, 1) : n_ch;
+    if (warp == kCopyWarp && lane == 0) popped = --quota != 0 ? stride + atomicAdd(queue, 1) : n_ch;
   }
   // tokens of this chunk that exist: 64, fewer in the last chunk of a sequence.  The rest of the tile
   // belongs to somebody else and is replaced by the identity step (no decay, no key, no query).
@@ -190,116 +211,113 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   const int ch = here.ch, n_valid = here.valid;
   const bool partial = n_valid < kChunk;
   // ---- log-decays, in units of ln 2 (a decay is one ex2): sums from the start of the 16-token block ----------
-  float Gc[kRounds][2][4];
+  float2 Gc[kRounds][4];
   waiter.wait(&sm.bar_ld[0], par);
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
-    float gv[2][4];
+    RawG raw[4];
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int i = i0 + 4 * e;
-      unpack4<G>(*reinterpret_cast<const RawG*>(R + kOffInG + (i * kDim + kRound * r + 4 * cl) * sizeof(G)), gv[e]);
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        if (pro_gate) gv[e][f] = prologue_log_decay(gv[e][f]);
-        gv[e][f] = (partial && i >= n_valid) ? 0.f : gv[e][f] * kLog2e;
-      }
+    for (int t = 0; t < 4; ++t) {
+      raw[t] = *reinterpret_cast<const RawG*>(R + kOffInG + ((i0 + t) * kDim + kRound * r + 2 * cl) * sizeof(G));
     }
-    // inclusive sums over the eight tokens of this warp: four lanes of one channel, first tokens, then the others
-    float total[4];
 #pragma unroll
-    for (int f = 0; f < 4; ++f) {
-#pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float x = __shfl_up_sync(0xffffffffu, gv[e][f], 8);
-        if (lane >= 8) gv[e][f] += x;
-        x = __shfl_up_sync(0xffffffffu, gv[e][f], 16);
-        if (lane >= 16) gv[e][f] += x;
-      }
-      gv[1][f] += __shfl_sync(0xffffffffu, gv[0][f], 24 + cl);
-      total[f] = gv[1][f];
-#pragma unroll
-      for (int e = 0; e < 2; ++e) Gc[r][e][f] = gv[e][f];
+    for (int t = 0; t < 4; ++t) {
+      float2 x = unpack2<G>(raw[t]);
+      if (pro_gate) x = make_float2(prologue_log_decay(x.x), prologue_log_decay(x.y));
+      x = (partial && i0 + t >= n_valid) ? twice(0.f) : mul2(x, twice(kLog2e));
+      Gc[r][t] = t > 0 ? add2(Gc[r][t - 1], x) : x;
     }
-    if (lane >= 24) {
-      *reinterpret_cast<float4*>(&sm.part[warp][kRound * r + 4 * cl]) = make_float4(total[0], total[1], total[2], total[3]);
+    // the upper half of the warp goes on from the lower one
+    const float2 x = make_float2(__shfl_up_sync(0xffffffffu, Gc[r][3].x, 16), __shfl_up_sync(0xffffffffu, Gc[r][3].y, 16));
+    if (lane >= 16) {
+#pragma unroll
+      for (int t = 0; t < 4; ++t) Gc[r][t] = add2(Gc[r][t], x);
+      *reinterpret_cast<float2*>(&sm.part[warp][kRound * r + 2 * cl]) = Gc[r][3];
     }
   }
+  if (warp == kCopyWarp) {
+    bulk_wait_read_all();  // the last unit's Y^T has left
+    if (unit != first) issue_b(here);
+  }
   sync();
-  // A thread per channel: prefixes of the eight groups, and the decay table, row by row:
+  // A thread per channel: what precedes each group in its block, and the decay table, row by row:
   //   0..3 exp(a_I), a_I = sum up to block I   4..7 exp(a_{I+1} - a_I)   8..11 exp(a_end - a_{I+1})   12 exp(a_3 - a_1)
   float* const table = reinterpret_cast<float*>(R + kOffTable);
   if (tid < kDim) {
-    float a[9];
-    a[0] = 0.f;
+    float x[8], block[4];
 #pragma unroll
-    for (int t = 0; t < 8; ++t) a[t + 1] = sm.part[t][tid];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) a[t + 1] += a[t];
-#pragma unroll
-    for (int t = 0; t < 8; ++t) sm.part[t][tid] = a[t] - a[t & ~1];  // from the start of the block
-    sm.gend[tid] = a[8];
-    // (element 0 of D doubles as the mark of a finished unit: see the end of the loop)
-    if (!kJoint || tid > 0) reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(a[8]);
+    for (int t = 0; t < 8; ++t) x[t] = sm.part[t][tid];
 #pragma unroll
     for (int I = 0; I < 4; ++I) {
-      table[I * kDim + tid] = exp2_approx(a[2 * I]);
-      table[(4 + I) * kDim + tid] = exp2_approx(a[2 * I + 2] - a[2 * I]);
-      table[(8 + I) * kDim + tid] = exp2_approx(a[8] - a[2 * I + 2]);
+      sm.part[2 * I][tid] = 0.f;
+      sm.part[2 * I + 1][tid] = x[2 * I];
+      block[I] = x[2 * I] + x[2 * I + 1];
     }
-    table[12 * kDim + tid] = exp2_approx(a[6] - a[2]);
+    const float a1 = block[0], a2 = a1 + block[1], a3 = a2 + block[2], end = a3 + block[3];
+    sm.gend[tid] = end;
+    // (element 0 of D doubles as the mark of a finished unit: see the end of the loop)
+    if (!kJoint || tid > 0) reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD)[tid] = exp2_approx(end);
+    table[tid] = 1.f;
+    table[kDim + tid] = exp2_approx(a1);
+    table[2 * kDim + tid] = exp2_approx(a2);
+    table[3 * kDim + tid] = exp2_approx(a3);
+#pragma unroll
+    for (int I = 0; I < 4; ++I) table[(4 + I) * kDim + tid] = exp2_approx(block[I]);
+    table[8 * kDim + tid] = exp2_approx(block[1] + block[2] + block[3]);
+    table[9 * kDim + tid] = exp2_approx(block[2] + block[3]);
+    table[10 * kDim + tid] = exp2_approx(block[3]);
+    table[11 * kDim + tid] = 1.f;
+    table[12 * kDim + tid] = exp2_approx(block[1] + block[2]);
   }
   waiter.wait(&sm.bar_ld[1], par);
-  RawT rk[2], rq[2], rb[2];
+  RawT rk[4], rq[4], rb[4];
   auto read_raw = [&](int r) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int at = r * 4096 + (i0 + 4 * e) * 64 + cl * 8;
-      rk[e] = *reinterpret_cast<const RawT*>(R + kOffInK + at);
-      rq[e] = *reinterpret_cast<const RawT*>(R + kOffInQ + at);
-      rb[e] = *reinterpret_cast<const RawT*>(R + kOffInBeta + at);
-      if (partial && i0 + 4 * e >= n_valid) rk[e] = rq[e] = rb[e] = RawT{};
+    for (int t = 0; t < 4; ++t) {
+      const int i = i0 + t, at = (r >> 1) * 8192 + i * 128 + ((((r & 1) * 4 + (cl >> 2)) ^ (i & 7)) << 4) + (cl & 3) * 4;
+      rk[t] = *reinterpret_cast<const RawT*>(R + kOffInK + at);
+      rq[t] = *reinterpret_cast<const RawT*>(R + kOffInQ + at);
+      rb[t] = *reinterpret_cast<const RawT*>(R + kOffInBeta + at);
+      if (partial && i0 + t >= n_valid) rk[t] = rq[t] = rb[t] = RawT{};
     }
   };
-  float inv_q[2] = {1.f, 1.f}, inv_k[2] = {1.f, 1.f};
+  float inv_q[4], inv_k[4];
+#pragma unroll
+  for (int t = 0; t < 4; ++t) inv_q[t] = inv_k[t] = 1.f;
   if (pro_norm) {
-    // sums of q^2 and k^2 over the channels: this thread's, then the eight lanes of a token
-    float sq[2] = {0.f, 0.f}, sk[2] = {0.f, 0.f};
+    // sums of q^2 and k^2 over the channels: this thread's, then the sixteen lanes of a token
+    float sq[4] = {}, sk[4] = {};
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
       read_raw(r);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        float x[4];
-        unpack4<T>(rq[e], x);
-        sq[e] += (x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]);
-        unpack4<T>(rk[e], x);
-        sk[e] += (x[0] * x[0] + x[1] * x[1]) + (x[2] * x[2] + x[3] * x[3]);
+      for (int t = 0; t < 4; ++t) {
+        const float2 x = unpack2<T>(rq[t]), y = unpack2<T>(rk[t]);
+        sq[t] += x.x * x.x + x.y * x.y;
+        sk[t] += y.x * y.x + y.y * y.y;
       }
     }
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
+    for (int t = 0; t < 4; ++t) {
 #pragma unroll
-      for (int off = 1; off < 8; off <<= 1) {
-        sq[e] += __shfl_xor_sync(0xffffffffu, sq[e], off);
-        sk[e] += __shfl_xor_sync(0xffffffffu, sk[e], off);
+      for (int off = 1; off < 16; off <<= 1) {
+        sq[t] += __shfl_xor_sync(0xffffffffu, sq[t], off);
+        sk[t] += __shfl_xor_sync(0xffffffffu, sk[t], off);
       }
-      inv_q[e] = rsqrtf(sq[e] + kPrologueEps);
-      inv_k[e] = rsqrtf(sk[e] + kPrologueEps);
+      inv_q[t] = rsqrtf(sq[t] + kPrologueEps);
+      inv_k[t] = rsqrtf(sk[t] + kPrologueEps);
     }
   }
   read_raw(0);
   sync();
 #pragma unroll
   for (int r = 0; r < kRounds; ++r) {
-    float base[4];
-    load4(&sm.part[warp][kRound * r + 4 * cl], true, base);
+    const float2 base = *reinterpret_cast<const float2*>(&sm.part[warp][kRound * r + 2 * cl]);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-#pragma unroll
-      for (int f = 0; f < 4; ++f) Gc[r][e][f] += base[f];
-    }
+    for (int t = 0; t < 4; ++t) Gc[r][t] = add2(Gc[r][t], base);
   }
+
+  if (warp == kCopyWarp) set_mark();
 
   // ---- Gram products P_I = [E_a ; Q_a] (K^I)^T on the tensor cores, 32 channels at a time ------------------
   float* const tile_q = reinterpret_cast<float*>(p.tiles.q + int64_t(ch) * kTileQ);
@@ -308,76 +326,71 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   // compiler's moves across the rounds cost more registers than there are)
 #pragma unroll 1
   for (int r = 0; r < kRounds; ++r) {
-    const int kc0 = kRound * r + 4 * cl;
-    float e_amb[4], c_nx[4], t_end[4], far0[4], far1[4];
-    load4(table + mb * kDim + kc0, true, e_amb);
-    load4(table + (4 + mb) * kDim + kc0, true, c_nx);         // decay over the whole 16-token block (<= 1)
-    load4(table + (8 + mb) * kDim + kc0, true, t_end);
-    load4(table + (mb < 2 ? 5 + mb : 4) * kDim + kc0, true, far0);  // (mb < 2) on to the block after the next one
-    load4(table + 12 * kDim + kc0, true, far1);                     // (mb < 1) ... and the one after that
-    float kk[2][4], bb[2][4], qq[2][4];
+    const int kc0 = kRound * r + 2 * cl;
+    auto row = [&](int t) { return *reinterpret_cast<const float2*>(table + t * kDim + kc0); };
+    const float2 e_amb = row(mb);
+    // before their rounding: beta k and scale q decayed from the block's anchor, k decayed to it and to the next one
+    float2 ba[4], qa[4], ko[4], nb[4];
+    {
+      const float2 c_nx = row(4 + mb);  // decay over the whole 16-token block (<= 1)
+      const float2 t_end = row(8 + mb);
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      unpack4<T>(rk[e], kk[e]);
-      unpack4<T>(rb[e], bb[e]);
-      unpack4<T>(rq[e], qq[e]);
+      for (int t = 0; t < 4; ++t) {
+        const float2 G2 = Gc[0][t];
+        const float2 anchored = exp2_2(G2);                    // <= 1
+        const float2 own = exp2_2(make_float2(-G2.x, -G2.y));  // >= 1, bounded by the 16-token contract
+        float2 k = unpack2<T>(rk[t]), b = unpack2<T>(rb[t]), q = mul2(unpack2<T>(rq[t]), twice(p.scale));
+        if (pro_gate) b = make_float2(prologue_sigmoid(b.x), prologue_sigmoid(b.y));
+        if (pro_norm) {
+          k = mul2(k, twice(inv_k[t]));
+          q = mul2(q, twice(inv_q[t]));
+        }
+        ba[t] = mul2(mul2(b, k), anchored);
+        qa[t] = mul2(q, anchored);
+        ko[t] = mul2(k, own);
+        nb[t] = mul2(k, mul2(own, c_nx));
+        // token-major tiles Q[i][k] and Kn[i][k]: 16 lanes write 128 consecutive bytes
+        *reinterpret_cast<float2*>(tile_q + (i0 + t) * kDim + kc0) = tf32_operand_2(mul2(qa[t], e_amb));
+        *reinterpret_cast<float2*>(tile_kn + (i0 + t) * kDim + kc0) = tf32_operand_2(mul2(nb[t], t_end));
+      }
     }
     if (r + 1 < kRounds) read_raw(r + 1);
     if (r > 0) waiter.wait(&sm.bar[0], (r - 1) & 1);  // the last round's operands have been multiplied
-    float eb[2][4];
+    {
+      // 8 bytes of a 128-byte line, whose 16-byte pieces are permuted by the line (the row numbers of K^I start at
+      // multiples of 16: one permutation for all)
+      auto put = [&](int line0, const float2 (&x)[4]) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int i = i0 + 4 * e;
-      if (pro_gate) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) bb[e][f] = prologue_sigmoid(bb[e][f]);
-      }
-      float ea[4], qa[4], kown[4], knb[4], qgam[4], ktail[4];
-#pragma unroll
-      for (int f = 0; f < 4; ++f) {
-        const float anchored = exp2_approx(Gc[0][e][f]);   // <= 1
-        const float own = exp2_approx(-Gc[0][e][f]);       // >= 1, bounded by the 16-token contract
-        const float nb = own * c_nx[f];                    // <= 1: decay from token i to the next block start
-        const float k = kPro ? kk[e][f] * inv_k[e] : kk[e][f];
-        const float bk = bb[e][f] * k;
-        const float sq = p.scale * (kPro ? qq[e][f] * inv_q[e] : qq[e][f]);
-        ea[f] = to_tf32_operand(bk * anchored);
-        qa[f] = to_tf32_operand(sq * anchored);
-        eb[e][f] = to_tf32_operand(bk * anchored * e_amb[f]);
-        qgam[f] = to_tf32_operand(sq * anchored * e_amb[f]);
-        kown[f] = to_tf32_operand(k * own);
-        knb[f] = k * nb;
-        ktail[f] = to_tf32_operand(knb[f] * t_end[f]);
-      }
-      // 16-byte chunk cl of a 128-byte line, permuted by the line (the row numbers of K^I start at multiples
-      // of 16: one permutation for all)
-      const uint32_t at = i * 128 + ((cl ^ (i & 7)) << 4);
-      *reinterpret_cast<float4*>(R + kOffGramA + at) = make_float4(ea[0], ea[1], ea[2], ea[3]);
-      *reinterpret_cast<float4*>(R + kOffGramA + 64 * 128 + at) = make_float4(qa[0], qa[1], qa[2], qa[3]);
+        for (int t = 0; t < 4; ++t) {
+          const int i = i0 + t;
+          *reinterpret_cast<float2*>(R + line0 * 128 + i * 128 + (((cl >> 1) ^ (i & 7)) << 4) + (cl & 1) * 8) =
+              tf32_operand_2(x[t]);
+        }
+      };
+      put(kOffGramA / 128, ba);
+      put(kOffGramA / 128 + 64, qa);
       // token i is a row of every K^I, I >= its own block
-      *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb) * 128 + at) = make_float4(kown[0], kown[1], kown[2], kown[3]);
-      if (mb < 3) {
-        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb + 1) * 128 + at) =
-            make_float4(to_tf32_operand(knb[0]), to_tf32_operand(knb[1]), to_tf32_operand(knb[2]), to_tf32_operand(knb[3]));
-      }
+      put(kOffGramB / 128 + gram_col(mb), ko);
+      if (mb < 3) put(kOffGramB / 128 + gram_col(mb + 1), nb);
       if (mb < 2) {
-        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(mb + 2) * 128 + at) =
-            make_float4(to_tf32_operand(knb[0] * far0[0]), to_tf32_operand(knb[1] * far0[1]),
-                        to_tf32_operand(knb[2] * far0[2]), to_tf32_operand(knb[3] * far0[3]));
+        const float2 far = row(5 + mb);  // on over the next block
+        float2 y[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) y[t] = mul2(nb[t], far);
+        put(kOffGramB / 128 + gram_col(mb + 2), y);
       }
       if (mb < 1) {
-        *reinterpret_cast<float4*>(R + kOffGramB + gram_col(3) * 128 + at) =
-            make_float4(to_tf32_operand(knb[0] * far1[0]), to_tf32_operand(knb[1] * far1[1]),
-                        to_tf32_operand(knb[2] * far1[2]), to_tf32_operand(knb[3] * far1[3]));
+        const float2 far = row(12);      // ... and the one after that
+        float2 y[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) y[t] = mul2(nb[t], far);
+        put(kOffGramB / 128 + gram_col(3), y);
       }
-      // token-major tiles Q[i][k] and Kn[i][k]: the 8 lanes of a token write 128 consecutive bytes
-      *reinterpret_cast<float4*>(tile_q + i * kDim + kc0) = make_float4(qgam[0], qgam[1], qgam[2], qgam[3]);
-      *reinterpret_cast<float4*>(tile_kn + i * kDim + kc0) = make_float4(ktail[0], ktail[1], ktail[2], ktail[3]);
     }
     fence_async_smem();
     tc_fence_before();
     sync();
-    if (warp == 0) {
+    if (warp == kMmaWarp) {
       tc_fence_after();
       // the four anchored copies K^0 .. K^3 are stacked (16 + 32 + 48 + 64 = 160 rows) and their products
       // sit side by side in TMEM, so one N = 160 instruction per k-step reads the A tile once for all four
@@ -389,33 +402,28 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
       }
       mma_commit(&sm.bar[0], leader);
     }
-    // E[i][channels of this thread]: 16 bytes of line i of a slab, 32-byte pieces permuted by the line
+    // E[i][channels of this thread]: 8 bytes of line i of a slab, 32-byte pieces permuted by the line
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const int i = i0 + 4 * e, slab = (r >> 1) | ((r & 1) << 1);
-      *reinterpret_cast<float4*>(R + kOffE + slab * 8192 + i * 128 + (((cl >> 1) ^ (i & 3)) << 5) + (cl & 1) * 16) =
-          make_float4(eb[e][0], eb[e][1], eb[e][2], eb[e][3]);
+    for (int t = 0; t < 4; ++t) {
+      const int i = i0 + t, slab = (r >> 1) | ((r & 1) << 1);
+      *reinterpret_cast<float2*>(R + kOffE + slab * 8192 + i * 128 + (((cl >> 2) ^ (i & 3)) << 5) + (cl & 3) * 8) =
+          tf32_operand_2(mul2(ba[t], e_amb));
     }
 #pragma unroll
     for (int n = 0; n + 1 < kRounds; ++n) {
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) Gc[n][e][f] = Gc[n + 1][e][f];
-      }
+      for (int t = 0; t < 4; ++t) Gc[n][t] = Gc[n + 1][t];
     }
   }
   waiter.wait(&sm.bar[0], 1);
   tc_fence_after();
-  // the Gram operands are dead: the region becomes fp32 scratch
-  float* Tn = reinterpret_cast<float*>(R + kOffTn);           // [64][kLd]   T
-  float* Tc = reinterpret_cast<float*>(R + kOffTc);           // [64][kLd]   T transposed: Tc[j][i] = T[i][j]
-  float* Ln = reinterpret_cast<float*>(R + kOffLn);           // [64][kLd]   L
-  float* Wt = reinterpret_cast<float*>(R + kOffWt);           // [2][16][kLdW] block products, transposed
-  // L (rows 0..63) goes into fp32 scratch, A_qk (rows 64..127) into the workspace; the two warps of a quadrant take 32
+  float* const Lt = reinterpret_cast<float*>(R + kOffLt);     // [64][64]    -L transposed: Lt[m][r] = -L[r][m]
+  float* const P = reinterpret_cast<float*>(R + kOffP);       // [32][32]    T[..32][..32]
+  float* const Qt = reinterpret_cast<float*>(R + kOffQt);     // [32][kLdQ]  Qt[m][r] = T[32 + r][32 + m]
+  float* const W = reinterpret_cast<float*>(R + kOffW);       // [32][64]    -L[32.., ..32) T[..32][..32]
+  // -L (rows 0..63) goes into fp32 scratch, A_qk (rows 64..127) into the workspace; the two warps of a quadrant take 32
   // columns each.  A_qk is stored behind the barrier, beside the first step of the inverse, which its warps have no
-  // part in: the stores queue behind those of the rounds, and the inverse would wait for them.  (With the diagonal
-  // blocks column by column, below: B8 T4096 H16 455 -> 450 us, B4 T8192 H32 training 892 -> 881.)
+  // part in: the stores queue behind those of the rounds, and the inverse would wait for them.
   const int gram_row = 32 * q4 + lane;  // TMEM lane = row of [E_a ; Q_a]
   float a_qk[2][16];
   {
@@ -437,19 +445,27 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
         const bool mine_lo = (my_I == I_lo);
         const float x = mine_lo ? (need_lo ? __uint_as_float(lo[j]) : 0.f) : (need_hi ? __uint_as_float(hi[j]) : 0.f);
         const int col = c0 + j;
-        vals[j] = (r < 64) ? ((col < i) ? x : 0.f) : ((col <= i) ? to_tf32_operand(x) : 0.f);
+        vals[j] = (r < 64) ? ((col < i) ? -x : 0.f) : ((col <= i) ? to_tf32_operand(x) : 0.f);
       }
-      if (r < 64) {
+      if (r < 64 && need_hi) {  // (nobody reads the block of zeros)
 #pragma unroll
-        for (int j4 = 0; j4 < 4; ++j4) {
-          *reinterpret_cast<float4*>(Ln + i * kLd + c0 + 4 * j4) =
-              make_float4(vals[4 * j4], vals[4 * j4 + 1], vals[4 * j4 + 2], vals[4 * j4 + 3]);
-        }
+        for (int j = 0; j < 16; ++j) Lt[(c0 + j) * kChunk + i] = vals[j];
       }
     }
   }
   tc_fence_before();
   sync();
+  // the Gram operands are dead: the next unit's g may have their place
+  if (warp == kCopyWarp) {
+    if constexpr (kJoint) {
+      unit_next = __shfl_sync(0xffffffffu, popped, 0);
+      if (lane == 0) sm.next[par] = unit_next;
+    }
+    if (unit_next < n_ch) {
+      const Place at = locate(unit_next);
+      issue_g(at);
+    }
+  }
   if (gram_row >= 64) {
     // A_qk leaves transposed, At[j][i]: the 32 lanes of a warp (rows i) fill one 128-byte line per column j;
     // the quadrant j >= 32, i < 32 is zero and stays unwritten (nobody reads it)
@@ -460,209 +476,176 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     }
   }
 
-  // ---- T = (I + L)^-1, blocked: 16x16 diagonal blocks by substitution, the rest by block products.
-  // T is kept in both orientations (Tn row-major, Tc column-major) and the block products W transposed,
-  // so that both factors of every inner product are read as 16-byte vectors along the summed index.  Blocks
-  // above the diagonal are not stored, except the two that the 32 x 32 products read as zeros.
+  // ---- T = (I + L)^-1 ----------------------------------------------------------------------------------------
+  // The two 32 x 32 diagonal blocks by substitution, a warp each and a lane per column: what a finished entry adds to
+  // all later ones is independent, and the factor L is the same for all lanes, four rows of it a broadcast.  Then
+  // T[32.., ..32) = -T[32.., 32..) (L[32.., ..32) T[..32, ..32)) in two products of four warps, a lane 4 rows x 2
+  // columns.  (16 x 16 blocks, whose products read both factors lane by lane, were a third of all wavefronts, 6 barriers
+  // and 6.4 thousand clocks a unit.)
   auto ld4 = [](const float* ptr) { return *reinterpret_cast<const float4*>(ptr); };
-  if (tid < 64) {
-    const int I = tid >> 4, cc = tid & 15;
-    // (column by column: what a finished entry contributes to all later ones is independent, so that the chain is 16
-    // multiply-adds long and not 120; each entry sums in the same order)
-    float x[16];
-#pragma unroll
-    for (int r = 0; r < 16; ++r) x[r] = (r == cc) ? 1.f : 0.f;
-#pragma unroll
-    for (int m4 = 0; m4 < 4; ++m4) {
-      float4 l[16];
-#pragma unroll
-      for (int r = 4 * m4 + 1; r < 16; ++r) l[r] = ld4(Ln + (16 * I + r) * kLd + 16 * I + 4 * m4);
-#pragma unroll
-      for (int r = 4 * m4 + 1; r < 16; ++r) x[r] = fmaf(-l[r].x, x[4 * m4], x[r]);
-#pragma unroll
-      for (int r = 4 * m4 + 2; r < 16; ++r) x[r] = fmaf(-l[r].y, x[4 * m4 + 1], x[r]);
-#pragma unroll
-      for (int r = 4 * m4 + 3; r < 16; ++r) x[r] = fmaf(-l[r].z, x[4 * m4 + 2], x[r]);
-#pragma unroll
-      for (int r = 4 * m4 + 4; r < 16; ++r) x[r] = fmaf(-l[r].w, x[4 * m4 + 3], x[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < 16; ++r) Tn[(16 * I + r) * kLd + 16 * I + cc] = x[r];
-#pragma unroll
-    for (int r4 = 0; r4 < 4; ++r4) {
-      *reinterpret_cast<float4*>(Tc + (16 * I + cc) * kLd + 16 * I + 4 * r4) =
-          make_float4(x[4 * r4], x[4 * r4 + 1], x[4 * r4 + 2], x[4 * r4 + 3]);
-    }
-  } else if (tid < 192) {
-    const int e = tid & 63, r = e >> 2, c4 = 4 * (e & 3);
-    *reinterpret_cast<float4*>((tid < 128 ? Tc + (16 + r) * kLd : Tn + (32 + r) * kLd + 48) + c4) =
-        make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-  sync();
-  // inner product of 4 `quads` values, in four independent chains (latency-bound otherwise)
-  auto dot = [&](const float* a, const float* b, int quads) {
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int m4 = 0; m4 < quads; ++m4) {
-      const float4 x = ld4(a + 4 * m4), y = ld4(b + 4 * m4);
-      acc.x = fmaf(x.x, y.x, acc.x); acc.y = fmaf(x.y, y.y, acc.y);
-      acc.z = fmaf(x.z, y.z, acc.z); acc.w = fmaf(x.w, y.w, acc.w);
-    }
-    return (acc.x + acc.y) + (acc.z + acc.w);
+  // T^T[j][i .. i + 3]: lines of 32 tokens i, two slabs, 32-byte pieces permuted by the line
+  auto put_t = [&](int j, int i, float2 lo, float2 hi) {
+    lo = tf32_operand_2(lo);
+    hi = tf32_operand_2(hi);
+    *reinterpret_cast<float4*>(R + kOffTt + (i >> 5) * 8192 + j * 128 + ((((i & 31) >> 3) ^ (j & 3)) << 5) + (i & 4) * 4) =
+        make_float4(lo.x, lo.y, hi.x, hi.y);
   };
-  // Two levels of 2 x 2 blocking instead of one block row at a time (four barriers fewer):
-  // level 1: the 16 x 16 blocks (1,0) and (3,2) complete the two 32 x 32 diagonal inverses P and Q,
-  // level 2: T[32.., ..32) = -Q (L[32.., ..32) P).
-  // level 1, W = L_IJ T_JJ for (I, J) = (1, 0), (3, 2)
-  {
-    const int r = tid >> 4, cc = tid & 15;
-    float w[2];
+  if (warp < 2) {
+    const float* l0 = Lt + 32 * warp * (kChunk + 1);
+    float2 x[16];
 #pragma unroll
-    for (int pair = 0; pair < 2; ++pair) {
-      const int J = 2 * pair, I = J + 1;
-      w[pair] = dot(Ln + (16 * I + r) * kLd + 16 * J, Tc + (16 * J + cc) * kLd + 16 * J, 4);
+    for (int r = 0; r < 16; ++r) x[r] = make_float2(lane == 2 * r ? 1.f : 0.f, lane == 2 * r + 1 ? 1.f : 0.f);
+#pragma unroll
+    for (int m = 0; m < 31; ++m) {
+      const float2 xm = twice((m & 1) ? x[m >> 1].y : x[m >> 1].x);
+#pragma unroll
+      for (int r4 = (m + 1) / 4; r4 < 8; ++r4) {  // (entries up to m meet zeros)
+        const float4 l = ld4(l0 + m * kChunk + 4 * r4);
+        x[2 * r4] = fma2(make_float2(l.x, l.y), xm, x[2 * r4]);
+        x[2 * r4 + 1] = fma2(make_float2(l.z, l.w), xm, x[2 * r4 + 1]);
+      }
     }
+    if (warp == 0) {
 #pragma unroll
-    for (int pair = 0; pair < 2; ++pair) Wt[(pair * 16 + cc) * kLdW + r] = w[pair];
-  }
-  sync();
-  // level 1, T_IJ = -T_II W
-  {
-    const int r = tid >> 4, cc = tid & 15;
-    float s[2];
+      for (int r = 0; r < 16; ++r) {
+        P[2 * r * 32 + lane] = x[r].x;
+        P[(2 * r + 1) * 32 + lane] = x[r].y;
+      }
+    } else {
 #pragma unroll
-    for (int pair = 0; pair < 2; ++pair) {
-      const int I = 2 * pair + 1;
-      s[pair] = dot(Tn + (16 * I + r) * kLd + 16 * I, Wt + (pair * 16 + cc) * kLdW, 4);
-    }
-#pragma unroll
-    for (int pair = 0; pair < 2; ++pair) {
-      const int J = 2 * pair, I = J + 1;
-      Tn[(16 * I + r) * kLd + 16 * J + cc] = -s[pair];
-      Tc[(16 * J + cc) * kLd + 16 * I + r] = -s[pair];
-    }
-  }
-  sync();
-  // level 2, W2 = L[32.., ..32) P, stored transposed over the (now dead) first 32 rows of L
-  // A thread forms four entries of a column (rows r, r + 8, r + 16, r + 24): the column of the right factor is
-  // the expensive read (a different 16-byte piece per lane, four shared-memory wavefronts), the rows of the
-  // left factor are broadcasts; the column is read once for all.
-  auto four_rows = [&](const float* rows, const float* col, float (&out)[4]) {
-    float4 acc[4];
-#pragma unroll
-    for (int x = 0; x < 4; ++x) acc[x] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int m4 = 0; m4 < 8; ++m4) {
-      const float4 b = ld4(col + 4 * m4);
-#pragma unroll
-      for (int x = 0; x < 4; ++x) {
-        const float4 a = ld4(rows + 8 * x * kLd + 4 * m4);
-        acc[x].x = fmaf(a.x, b.x, acc[x].x); acc[x].y = fmaf(a.y, b.y, acc[x].y);
-        acc[x].z = fmaf(a.z, b.z, acc[x].z); acc[x].w = fmaf(a.w, b.w, acc[x].w);
+      for (int r = 0; r < 16; r += 2) {
+        *reinterpret_cast<float4*>(Qt + lane * kLdQ + 2 * r) = make_float4(x[r].x, x[r].y, x[r + 1].x, x[r + 1].y);
       }
     }
 #pragma unroll
-    for (int x = 0; x < 4; ++x) out[x] = (acc[x].x + acc[x].y) + (acc[x].z + acc[x].w);
+    for (int r = 0; r < 16; r += 2) put_t(32 * warp + lane, 32 * warp + 2 * r, x[r], x[r + 1]);
+  } else if (warp < 6) {
+    // the block of zeros, j >= 32, i < 32 (it does not leave)
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      *reinterpret_cast<float4*>(R + kOffTt + 4096 + (tid - 64 + 128 * x) * 16) = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+  }
+  sync();
+  // rows r0 .. r0 + 3, columns c0, c0 + 1 of a product: the sum over m of rows[m][r0 ..] cols[m][c0 ..], in two chains
+  const int r0 = 8 * (warp - 2) + 4 * (lane >> 4), c0 = 2 * (lane & 15);
+  auto product = [&](const float* rows, int ld_rows, const float* cols, int ld_cols, float2 (&out)[2][2]) {
+    float2 acc[2][2][2] = {};
+#pragma unroll
+    for (int m = 0; m < 32; ++m) {
+      const float4 a = ld4(rows + m * ld_rows + r0);
+      const float2 b = *reinterpret_cast<const float2*>(cols + m * ld_cols + c0);
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {
+        const float2 bc = twice(c ? b.y : b.x);
+        acc[m & 1][c][0] = fma2(make_float2(a.x, a.y), bc, acc[m & 1][c][0]);
+        acc[m & 1][c][1] = fma2(make_float2(a.z, a.w), bc, acc[m & 1][c][1]);
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x) out[c][x] = add2(acc[0][c][x], acc[1][c][x]);
+    }
   };
-  float* W2t = Ln;  // W2t[c][r] = W2[r][c], leading dimension kLd
-  {
-    const int r = tid >> 5, cc = tid & 31;
-    float w[4];
-    // rows 32.. of L are read here, W2t lives in rows 0..31, which nobody reads any more
-    four_rows(Ln + (32 + r) * kLd, Tc + cc * kLd, w);
+  const bool multiplies = warp >= 2 && warp < 6;
+  if (multiplies) {
+    float2 w[2][2];
+    product(Lt + 32, kChunk, P, 32, w);
 #pragma unroll
-    for (int x = 0; x < 4; ++x) W2t[cc * kLd + r + 8 * x] = w[x];
-  }
-  sync();
-  // level 2, T[32 + r][c] = -sum_m Q[r][m] W2[m][c]
-  {
-    const int r = tid >> 5, cc = tid & 31;
-    float s[4];
-    four_rows(Tn + (32 + r) * kLd + 32, W2t + cc * kLd, s);
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      Tn[(32 + r + 8 * x) * kLd + cc] = -s[x];
-      Tc[cc * kLd + 32 + r + 8 * x] = -s[x];
+    for (int x = 0; x < 2; ++x) {
+      *reinterpret_cast<float2*>(W + (r0 + 2 * x) * kChunk + c0) = make_float2(w[0][x].x, w[1][x].x);
+      *reinterpret_cast<float2*>(W + (r0 + 2 * x + 1) * kChunk + c0) = make_float2(w[0][x].y, w[1][x].y);
     }
   }
   sync();
-  // T as tf32 tile X[r = i][c = j] over L (MMA operand), and T^T[j][i] for the scans
-  {
-    float* tile_tt = reinterpret_cast<float*>(p.tiles.tt + int64_t(ch) * kTileTt);
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int e = tid + x * kPrepThreads, i = e & 63, c4t = e >> 6;  // consecutive rows: contiguous 16-byte chunks
-      const float4 tn = (c4t >> 2) <= (i >> 4) ? ld4(Tn + i * kLd + 4 * c4t) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(R + kOffTmat + blk_off<4>(i, 4 * c4t, 2048, 128)) =
-          make_float4(to_tf32_operand(tn.x), to_tf32_operand(tn.y), to_tf32_operand(tn.z), to_tf32_operand(tn.w));
-    }
-#pragma unroll
-    for (int x = 0; x < 4; ++x) {
-      const int e = tid + x * kPrepThreads, j = e >> 4, c4t = e & 15;  // consecutive 16-byte pieces of a row
-      if (j >= 32 && c4t < 8) continue;    // the zero quadrant j >= 32, i < 32 stays unwritten
-      const float4 tc = (j >> 4) <= (c4t >> 2) ? ld4(Tc + j * kLd + 4 * c4t) : make_float4(0.f, 0.f, 0.f, 0.f);
-      *reinterpret_cast<float4*>(tile_tt + j * kChunk + 4 * c4t) =
-          make_float4(to_tf32_operand(tc.x), to_tf32_operand(tc.y), to_tf32_operand(tc.z), to_tf32_operand(tc.w));
-    }
+  if (multiplies) {
+    float2 t[2][2];
+    product(Qt, kLdQ, W, kChunk, t);
+    put_t(c0, 32 + r0, t[0][0], t[0][1]);
+    put_t(c0 + 1, 32 + r0, t[1][0], t[1][1]);
   }
   fence_async_smem();
   tc_fence_before();
   sync();
 
-  // ---- Y^T = E^T T^T (A = E[j][k] read MN-major) ------------------------------------------------------------------------------------
-  if (warp == 0) {
+  // ---- Y^T = E^T T^T (both read MN-major), while T^T leaves -----------------------------------------------------
+  if (warp == kMmaWarp) {
     tc_fence_after();
-    const uint32_t t0a = smem_u32(R + kOffTmat), e0 = smem_u32(R + kOffE);
-    const uint32_t id_y = idesc(128, 64, kFmtTF32, kMajorMN, kMajorK);
+    const uint32_t t0a = smem_u32(R + kOffTt), e0 = smem_u32(R + kOffE);
+    const uint32_t id_y = idesc(128, 64, kFmtTF32, kMajorMN, kMajorMN);
 #pragma unroll
     for (int ks = 0; ks < 8; ++ks) {
-      mma_tf32_ss(tb, smem_desc_sw128_mn(e0, 8192, ks), smem_desc(t0a + ks * 256, 128, 2048), id_y,
-                  ks > 0 ? 1u : 0u, leader);
+      mma_tf32_ss(tb, smem_desc_sw128_mn(e0, 8192, ks), smem_desc_sw128_mn(t0a, 8192, ks), id_y, ks > 0 ? 1u : 0u, leader);
     }
     mma_commit(&sm.bar[1], leader);
   }
-  if (tid == 32 && unit_next < n_ch) issue_g(locate(unit_next));
+  if (warp == kCopyWarp) {
+    tma_store_4d(&tm.out_tt, 0, 0, 0, ch, R + kOffTt, leader);
+    tma_store_4d(&tm.out_tt, 0, 0, 1, ch, R + kOffTt + 8192, leader);
+    tma_store_4d(&tm.out_tt, 0, 32, 1, ch, R + kOffTt + 8192 + 4096, leader);
+    bulk_commit();
+    bulk_wait_read_all();
+    mbar_arrive(&sm.bar[1], leader);
+  }
   waiter.wait(&sm.bar[1], par);
   tc_fence_after();
-  if (tid == 32 && unit_next < n_ch) issue_kqb(locate(unit_next));
+  if (warp == kCopyWarp && unit_next < n_ch) issue_kq(locate(unit_next));
   {
-    // lanes = key channels k, columns = tokens i: each warp takes 32 tokens of its quadrant, a lane 128
-    // consecutive bytes of row k of Yt[k][i]
-    const int kr = 32 * ((q4 >> 1) | ((q4 & 1) << 1)) + lane, c0 = 32 * part;  // (slabs in the order 0, 2, 1, 3)
-    float* row_yt = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + c0;
+    // lanes = key channels k, columns = tokens i: each warp takes 32 tokens of its quadrant, a lane 128 bytes of a row of
+    // Yt[k][i].  They leave through shared memory, lines whose 16-byte pieces are permuted by their number: rows of their
+    // own stored by the lanes take five times the wavefronts.  Not so in a joint launch, where the scans beside are held
+    // up more than that is worth (B1 T32768 H16 805 us by the lanes, 861 through shared memory; T16384 416 and 440).
+    const int kr = 32 * ((q4 >> 1) | ((q4 & 1) << 1)) + lane;  // (slabs in the order 0, 2, 1, 3)
     uint32_t r[32];
-    tmem_ld32(tmem_addr(tb, 32 * q4, c0), r);
+    tmem_ld32(tmem_addr(tb, 32 * q4, 32 * part), r);
     tmem_wait_ld();
     float y[32];
 #pragma unroll
     for (int j = 0; j < 32; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
-    // (buffers are 16-byte aligned by contract; from an allocator they are 32-byte aligned as well)
-    if (wide_tiles) {
+    if constexpr (kJoint) {
+      float* row = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + 32 * part;
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
-        store_global_32b(row_yt + j, make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]),
-                         make_float4(y[j + 4], y[j + 5], y[j + 6], y[j + 7]));
+        const float4 lo = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+        const float4 hi = make_float4(y[j + 4], y[j + 5], y[j + 6], y[j + 7]);
+        // (buffers are 16-byte aligned by contract; from an allocator they are 32-byte aligned as well)
+        if (wide_tiles) {
+          store_global_32b(row + j, lo, hi);
+        } else {
+          *reinterpret_cast<float4*>(row + j) = lo;
+          *reinterpret_cast<float4*>(row + j + 4) = hi;
+        }
       }
     } else {
 #pragma unroll
       for (int j = 0; j < 32; j += 4) {
-        *reinterpret_cast<float4*>(row_yt + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+        *reinterpret_cast<float4*>(R + kOffY + part * 16384 + kr * 128 + (((j >> 2) ^ (kr & 7)) << 4)) =
+            make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
       }
     }
   }
-  tc_fence_before();  // the next unit's products replace these accumulators, behind two barriers
+  // (what the scan of a joint launch reads through the copy engine, another proxy than these stores)
+  if constexpr (kJoint) fence_async_all();
+  else fence_async_smem();
+  tc_fence_before();  // the next unit's products replace these accumulators
+  sync();
+  if (!kJoint && warp == kCopyWarp) {
+    tma_store_4d(&tm.out_yt, 0, 0, 0, ch, R + kOffY, leader);
+    bulk_commit();
+  }
   if constexpr (kJoint) {
-    // every thread's stores, then the mark: the sign of D[0] (a decay is never negative).  The scan reads the
-    // tiles through the copy engine, another proxy than the stores.
-    fence_async_all();
-    sync();
+    // A finished unit is marked by the sign of D[0] (a decay is never negative) once its tiles are in memory: the
+    // copying warp looks to that when it has the next unit's sums.
     unit_next = sm.next[par];
-    if (tid == 0) {
-      float* d = reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(ch) * kBlobD);
-      store_release(d, __uint_as_float(__float_as_uint(exp2_approx(sm.gend[0])) | 0x80000000u));
-    }
+    leaving = ch;
+    mark = __uint_as_float(__float_as_uint(exp2_approx(sm.gend[0])) | 0x80000000u);
   }
   }  // units of this group
+  if (warp == kCopyWarp) {
+    bulk_wait_all();  // the last tiles are in memory before the CTA goes on
+    set_mark();
+  }
 }
 
 template <typename T, typename G, typename Seqs, bool kPro = false>
@@ -1373,21 +1356,22 @@ struct ForwardCall {
 
 thread_local int t_forward_kernels = 0;  // of this thread's latest chunk forward
 
-// One launch for both where it gains.  Apart they take n_ch * 8.3 us / SMs (the preparation), 1.6-2 us per chunk (the
+// One launch for both where it gains.  Apart they take n_ch * 7.1 us / SMs (the preparation), 1.6-2 us per chunk (the
 // scans) and what two launches cost; together the scans' time and some 20 us, where the SMs that do not scan, or all in
 // turn (quota), have the units ready in time.
 // At most a sixth of the SMs scanning, two launches / one, us, inference, raw, training:
-//   400 units on    H16 T1600 77/69 86/80 187/184   H16 T2048 95/81 105/93 214/208   H8 T3200 109/103 118/118 252/252
-//                   H8 T4096 136/125 146/141 303/303   H24 T1152 70/71 77/82 171/164   H24 T1408 82/78 92/87 205/195
-//   below           H16 T1024 51/52 55/60 131/135   H16 T1280 69/60 74/68 169/164   H8 T2048 72/75 76/86 170/179
-//   fewer scans     H1 T25600 565/627 578/669   H3 T12288 306/312 320/346   H4 T8192 220/219 233/243, training 515/530:
+//   400 units on    H16 T1600 71/67 80/80 182/180   H16 T2048 86/78 97/92 207/204   H8 T3200 103/102 111/119 242/246
+//                   H8 T4096 126/122 137/142 298/298   H24 T1152 62/64 72/76 163/159   H24 T1408 74/70 85/79 195/189
+//   below           H16 T1024 46/51 54/61 128/133   H16 T1280 62/58 71/69 163/162   H8 T2048 66/73 74/87 166/176
+//   fewer scans     H1 T25600 535/563 551/665   H3 T12288 288/291 302/344   H4 T8192 206/216 218/243, training 511/523
+//                   H6 T8192 228/213 243/243, training 535/532
 //   the units are ready in time either way and a pair of CTAs scans no faster than it does alone, so 4 scans at least,
 //   and 8 with a prologue or states to write
 // With up to a quarter scanning, inference, raw, training (above that the preparation falls behind):
-//   above the line  H28 T2048 126/113 140/135 296/275   H32 T1664 109/111 122/114 271/266   H32 T2048 129/116 142/141
-//                   315/305   H37 T1408 104/95 118/113 260/256
-//   below           H28 T1024 72/61 83/70 183/174   H28 T1536 97/90 108/110 238/224   H32 T1280 91/91 101/107 226/219
-//                   H32 T1536 104/97 117/110 262/250   H37 T1024 76/77 87/91 193/190   H37 T1280 94/90 105/103 233/232
+//   above the line  H28 T2048 114/100 127/124 281/261   H32 T1664 99/99 113/105 259/252   H32 T2048 118/104 130/127
+//                   303/295   H37 T1408 95/87 108/103 249/248
+//   below           H28 T1024 62/56 73/66 173/169   H28 T1536 89/80 99/101 229/217   H32 T1280 84/80 93/100 217/209
+//                   H32 T1536 94/87 108/101 251/238   H37 T1024 68/70 79/84 184/180   H37 T1280 86/82 98/95 225/224
 //   (the line is that of an earlier form of the launch, which cost more; it stands on the safe side)
 bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, bool training, bool prologue, int sm_count) {
   if (4 * n_scan > sm_count || profiling()) return false;
@@ -1409,18 +1393,19 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int pairs = seqs.count() * sp.H;
   // Clusters of two CTAs.  No more preparers than pairs of units, nor than keep ahead of the scans: a unit takes an
-  // SM 9.4 us (raw 12) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way (B1 T32768 H16 817
-  // us with 96, 867 with 116; raw 964 with 104, 1031 with 116).
-  const int64_t paced = (int64_t(pairs) * (pp.prologue != 0 ? 66 : 60) + 19) / 20;
+  // SM 8.7 us (raw 11) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way.  us with 82 / 88 / 96
+  // SMs that prepare, H16: T32768 869/806/865, T16384 436/418/444, T8192 229/226/233; raw with 88 / 98 / 104: T32768
+  // 969/917/942, T8192 271/256/257.
+  const int64_t paced = (int64_t(pairs) * (pp.prologue != 0 ? 62 : 55) + 19) / 20;
   const int64_t want = pairs + std::min((pp.n_ch + 3) / 4, paced);
   const int clusters = int(std::min(want, int64_t(sm_count / 2)));
   // Where the preparers alone would not keep up, the scanning CTAs first prepare `quota` units for each group of
   // theirs, so that everybody is done at the same time.  While a scan advances by a chunk a preparing SM makes
-  // `pace` / 100 units: 1.7 us to 9.4, 1.9 to 12 with the prologue, 2.0 to 10 where the states are written out.  us, with
-  // 28 for all / with these: inference T8192 H24 318/297, H32 432/391, H37 502/454, T32768 H24 1152/1098; raw T8192
-  // H24 383/361, H32 531/472, H37 621/537, T32768 H24 1450/1349, B2 T4133 H16 282/260; training T4096 H24 440/433, T8192
-  // H28 930/922.  (One unit in a hundred more or less moves these by 1 %, four by 5.)
-  const int64_t pace = pp.training != 0 ? 20 : pp.prologue != 0 ? 16 : 18;
+  // `pace` / 100 units: 1.7 us to 8.5, 1.9 to 12 with the prologue, 1.8 to 9 where the states are written out.  us, with
+  // 18 / 20 / 21: T32768 H20 942/925/927, H24 1157/1142/1138, H32 1530/1535/1536, T8192 H32 391/386/400, H37
+  // 445/448/462, training T4096 H32 (18 / 20 / 22) 233/220/221; raw, with 15 / 16 / 18: T8192 H32 441/447/467, H37
+  // 510/515/533, T32768 H24 1341/1316/1320, B2 T4133 H16 238/236/238.
+  const int64_t pace = pp.prologue != 0 && pp.training == 0 ? 16 : 20;
   const int64_t in_time = int64_t(2 * (clusters - pairs)) * seqs.n_chunks * pace / 100;
   const int quota = pp.n_ch > in_time ? int((pp.n_ch - in_time + 2 * clusters) / (4 * clusters)) : 0;
   cudaLaunchConfig_t config = {};
@@ -1474,9 +1459,11 @@ int launch_forward(const Seqs& seqs, const ForwardCall& a, cudaStream_t stream) 
   ScanMaps tm;
   // the sequence tensors, and the scan's operands: the prep kernel's tiles in the swizzle of their role
   if (!encode_sequence_map(&tm_prep.g, a.g, a.rows, a.H, a.g_dtype) ||
-      !encode_round_map(&tm_prep.k, a.k, a.rows, a.H, a.dtype) ||
-      !encode_round_map(&tm_prep.q, a.q, a.rows, a.H, a.dtype) ||
-      !encode_round_map(&tm_prep.beta, a.beta, a.rows, a.H, a.dtype) ||
+      !encode_half_map(&tm_prep.k, a.k, a.rows, a.H, a.dtype) ||
+      !encode_half_map(&tm_prep.q, a.q, a.rows, a.H, a.dtype) ||
+      !encode_half_map(&tm_prep.beta, a.beta, a.rows, a.H, a.dtype) ||
+      !encode_tile_map(&tm_prep.out_tt, tiles.tt, n_ch, kChunk, kChunk, true, 32, 1) ||
+      !encode_tile_map(&tm_prep.out_yt, tiles.yt, n_ch, kDim, kChunk, false) ||
       !encode_sequence_map(&tm.v, a.v, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||
       !encode_sequence_map(&tm.w, a.w, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||
       !encode_sequence_map(&tm.out, a.out, a.rows, a.H, a.dtype, kChunk, kDim / parts) ||

@@ -99,11 +99,54 @@ __device__ __forceinline__ void unpack4<float>(float4 raw, float (&out)[4]) {
   out[0] = raw.x; out[1] = raw.y; out[2] = raw.z; out[3] = raw.w;
 }
 
+// two of them
+template <typename T> struct Raw2 { using type = uint32_t; };
+template <> struct Raw2<float> { using type = float2; };
+template <typename T>
+__device__ __forceinline__ float2 unpack2(typename Raw2<T>::type raw);
+template <>
+__device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t raw) {
+  return make_float2(__uint_as_float(raw << 16), __uint_as_float(raw & 0xffff0000u));
+}
+template <>
+__device__ __forceinline__ float2 unpack2<__half>(uint32_t raw) {
+  return __half22float2(*reinterpret_cast<const __half2*>(&raw));
+}
+template <>
+__device__ __forceinline__ float2 unpack2<float>(float2 raw) { return raw; }
+
 __device__ __forceinline__ float exp2_approx(float x) {  // one special-function result
   float r;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
 }
+
+// Two fp32 operations per instruction (each rounded like the scalar one): the elementwise phases of the chunk kernels
+// are bound by instruction issue.
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mul.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "add.rn.f32x2 rd, ra, rb;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+  return d;
+}
+__device__ __forceinline__ float2 fma2(float2 a, float2 b, float2 c) {
+  float2 d;
+  asm("{\n\t.reg .b64 ra, rb, rc, rd;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+      "mov.b64 rc, {%6, %7};\n\tfma.rn.f32x2 rd, ra, rb, rc;\n\tmov.b64 {%0, %1}, rd;\n\t}"
+      : "=f"(d.x), "=f"(d.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+  return d;
+}
+__device__ __forceinline__ float2 twice(float x) { return make_float2(x, x); }
+__device__ __forceinline__ float2 minus2(float2 a, float2 b) { return fma2(b, twice(-1.f), a); }
+__device__ __forceinline__ float2 exp2_2(float2 x) { return make_float2(exp2_approx(x.x), exp2_approx(x.y)); }
 
 // ---- layer prologue (optional, fused into the forward kernels) ------------------------------
 // bit flags of the `prologue` argument of the *_fused entry points

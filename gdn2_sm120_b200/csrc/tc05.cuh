@@ -53,8 +53,11 @@ __device__ __forceinline__ void mbar_arrive_expect_tx(uint64_t* bar, uint32_t by
       "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(smem_u32(bar)), "r"(bytes), "r"(leader)
       : "memory");
 }
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar, uint32_t leader = 1) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %1, 0;\n\t"
+      "@q mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(leader)
+      : "memory");
 }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -130,6 +133,15 @@ __device__ __forceinline__ void tma_store_3d(const void* tmap, int c0, int c1, i
   asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(tmap),
                "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(smem_src))
                : "memory");
+}
+
+__device__ __forceinline__ void tma_store_4d(const void* tmap, int c0, int c1, int c2, int c3, const void* smem_src,
+                                             uint32_t leader = 1) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %6, 0;\n\t"
+      "@q cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%1, %2, %3, %4}], [%5];\n\t}" ::"l"(tmap),
+      "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(smem_src)), "r"(leader)
+      : "memory");
 }
 
 // 1-D bulk copy shared -> global (bulk async-group completion).
@@ -317,6 +329,7 @@ __device__ __forceinline__ float to_tf32(float x) {
 // tile in the workspace): they ignore the 13 low bits of the container, so adding half a unit is all it
 // takes and the mask can stay away.  Anything the CUDA cores multiply by as well needs to_tf32.
 __device__ __forceinline__ float to_tf32_operand(float x) { return __uint_as_float(__float_as_uint(x) + 0x1000u); }
+__device__ __forceinline__ float2 tf32_operand_2(float2 x) { return make_float2(to_tf32_operand(x.x), to_tf32_operand(x.y)); }
 
 }  // namespace tc
 }  // namespace gdn2
