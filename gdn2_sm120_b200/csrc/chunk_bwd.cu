@@ -876,12 +876,12 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
     mma_commit(&ms.bar_r, leader);  // the dS_1 buffer may be refilled once these have run
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
-      mma_tf32_ss(tb + kColD2, smem_desc(st + ks * 2 * kCsN, kCsN, kRsN), smem_desc_sw128_k(rn, 8192, ks), id64,
+      mma_tf32_ss(tb + kColD2, smem_desc(st, kCsN, kRsN, ks * 2 * kCsN), smem_desc_sw128_k(rn, 8192, ks), id64,
                   ks > 0 ? 1u : 0u, leader);
     }
 #pragma unroll
     for (int ks = 0; ks < 16; ++ks) {
-      mma_tf32_ss(tb + kColD3, smem_desc_sw128_k(s0, 16384, ks), smem_desc(st + ks * 2 * kCsN, kCsN, kRsN), id128,
+      mma_tf32_ss(tb + kColD3, smem_desc_sw128_k(s0, 16384, ks), smem_desc(st, kCsN, kRsN, ks * 2 * kCsN), id128,
                   ks > 0 ? 1u : 0u, leader);
     }
     mma_commit(&ms.bar_m, leader);
@@ -1086,12 +1086,10 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
     // [dEa_I^T | dQa_I^T] (columns 32 I .. 32 I + 31) = (K^I)^T x the 32 stacked rows [dL_I ; dA_I]
 #pragma unroll
     for (int I = 0; I < 4; ++I) {
-      const uint32_t kit = smem_u32(smem + kit_offset(I));
-      const uint32_t rs = uint32_t(kit_rs(I));
 #pragma unroll
       for (int ks = 0; ks < 2 * (I + 1); ++ks) {
-        mma_tf32_ss(tb + kColD5 + 32 * I, smem_desc(kit + ks * 256, 128, rs),
-                    smem_desc(s2 + 4 * I * 2048 + ks * 256, 128, 2048), id32, ks > 0 ? 1u : 0u, leader);
+        mma_tf32_ss(tb + kColD5 + 32 * I, smem_desc(smem_u32(smem), 128, kit_rs(I), kit_offset(I) + ks * 256),
+                    smem_desc(s2, 128, 2048, 4 * I * 2048 + ks * 256), id32, ks > 0 ? 1u : 0u, leader);
       }
     }
     // (dK^I)^T = Ea^T[:, block I] dL[block I, :] + Qa^T[:, block I] dA[block I, :]
@@ -1100,12 +1098,10 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
       const uint32_t idn = idesc(128, 16 * (I + 1), kFmtTF32, kMajorK, kMajorK);
 #pragma unroll
       for (int pt = 0; pt < 2; ++pt) {
-        const uint32_t a_base = (pt ? qat0 : eat0) + 4 * I * 128;
-        const uint32_t b_base = (pt ? dat : dlt) + 4 * I * kCsS;
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {
-          mma_tf32_ss(tb + d6_col(I), smem_desc(a_base + ks * 256, 128, kRsT),
-                      smem_desc(b_base + ks * 2 * kCsS, kCsS, kRsS), idn, (pt | ks) ? 1u : 0u, leader);
+          mma_tf32_ss(tb + d6_col(I), smem_desc(pt ? qat0 : eat0, 128, kRsT, 4 * I * 128 + ks * 256),
+                      smem_desc(pt ? dat : dlt, kCsS, kRsS, 4 * I * kCsS + ks * 2 * kCsS), idn, (pt | ks) ? 1u : 0u, leader);
         }
       }
     }

@@ -185,14 +185,19 @@ __device__ __forceinline__ uint32_t tmem_addr(uint32_t base, uint32_t lane, uint
 }
 
 // ---- descriptors --------------------------------------------------------------------------
-// Shared-memory matrix descriptor, no swizzle, sm_100 descriptor version 1.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes, uint32_t sbo_bytes) {
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((lbo_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>((sbo_bytes >> 4) & 0x3FFFu) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  return d;
+// Shared-memory matrix descriptor, sm_100 descriptor version 1: bits 0-13 address, 16-29 LBO, 32-45 SBO, all in units of
+// 16 bytes, 46 version, 61-63 swizzle.  The address is a tile's plus a step that is a constant where the MMAs of a group
+// are unrolled: one addition per descriptor then (shared memory ends below 2^18, so no sum leaves its field; in a cluster
+// an address has the number of its CTA above that, which does not belong here).
+__device__ __forceinline__ uint64_t smem_desc_at(uint32_t tile, uint32_t step_bytes, uint32_t lbo_bytes,
+                                                 uint32_t sbo_bytes, uint32_t swizzle) {
+  const uint32_t lo = ((tile & 0x3FFFFu) >> 4) + ((step_bytes >> 4) + ((lbo_bytes >> 4) << 16));
+  const uint32_t hi = (sbo_bytes >> 4) | (1u << 14) | (swizzle << 29);
+  return (uint64_t(hi) << 32) | lo;
+}
+__device__ __forceinline__ uint64_t smem_desc(uint32_t tile, uint32_t lbo_bytes, uint32_t sbo_bytes,
+                                              uint32_t step_bytes = 0) {
+  return smem_desc_at(tile, step_bytes, lbo_bytes, sbo_bytes, 0);
 }
 
 // Swizzled operands, fetched by tiled TMA loads from a row-major fp32 matrix X[rows][cols] in slabs of
@@ -201,27 +206,13 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo_bytes
 //   K-major operand (MN index = row, K index = column), TMA swizzle 128B: 8-line atoms, SBO = 1024;
 //     the K step of 8 tf32 values is 32 bytes inside the line, then the next slab.
 __device__ __forceinline__ uint64_t smem_desc_sw128_k(uint32_t tile, uint32_t slab_bytes, int kstep) {
-  const uint32_t saddr = tile + uint32_t(kstep >> 2) * slab_bytes + uint32_t(kstep & 3) * 32u;
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>(1) << 16;
-  d |= static_cast<uint64_t>(1024u >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(2) << 61;  // 128-byte swizzle
-  return d;
+  return smem_desc_at(tile, uint32_t(kstep >> 2) * slab_bytes + uint32_t(kstep & 3) * 32u, 16, 1024, 2);  // 128-byte swizzle
 }
 //   MN-major operand (K index = row, MN index = column), TMA swizzle 128B with 32-byte atoms: 4-line
 //     atoms, SBO = 512 (next 4 rows of K), LBO = slab stride (next 32 columns of MN); the K step of 8
 //     rows is 1024 bytes.  32-bit operands have no other MN-major form.
 __device__ __forceinline__ uint64_t smem_desc_sw128_mn(uint32_t tile, uint32_t slab_bytes, int kstep) {
-  const uint32_t saddr = tile + uint32_t(kstep) * 1024u;
-  uint64_t d = 0;
-  d |= static_cast<uint64_t>((saddr & 0x3FFFFu) >> 4);
-  d |= static_cast<uint64_t>((slab_bytes >> 4) & 0x3FFFu) << 16;
-  d |= static_cast<uint64_t>(512u >> 4) << 32;
-  d |= static_cast<uint64_t>(1) << 46;
-  d |= static_cast<uint64_t>(1) << 61;  // 128-byte swizzle, 32-byte atoms
-  return d;
+  return smem_desc_at(tile, uint32_t(kstep) * 1024u, slab_bytes, 512, 1);  // 128-byte swizzle, 32-byte atoms
 }
 
 enum : uint32_t { kFmtF16 = 0, kFmtBF16 = 1, kFmtTF32 = 2 };
