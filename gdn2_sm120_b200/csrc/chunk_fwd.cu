@@ -464,6 +464,9 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     if (unit_next < n_ch) {
       const Place at = locate(unit_next);
       issue_g(at);
+      // beta has to wait for Y^T to leave and is needed soon after: 393 -> 373 us (B8 T4096 H16).  In a joint launch, whose
+      // Y^T leaves by itself, it is only in the way (B1 T8192 H16 225 -> 229 us).
+      if (!kJoint) tma_prefetch_l2_4d(&tm.beta, 0, at.row, 0, at.h, leader);
     }
   }
   if (gram_row >= 64) {

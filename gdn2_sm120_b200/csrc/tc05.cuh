@@ -108,6 +108,13 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const void* tmap, int c0, int
       "r"(c2), "r"(leader)
       : "memory");
 }
+__device__ __forceinline__ void tma_prefetch_l2_4d(const void* tmap, int c0, int c1, int c2, int c3, uint32_t leader = 1) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\tsetp.ne.b32 q, %5, 0;\n\t"
+      "@q cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n\t}" ::"l"(tmap), "r"(c0), "r"(c1),
+      "r"(c2), "r"(c3), "r"(leader)
+      : "memory");
+}
 // Tiled TMA loads global -> shared; completion (bytes) on an mbarrier.  `tmap` points at a
 // CUtensorMap in kernel-parameter space.  c0 must keep c0 * element size a multiple of 16 bytes.
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar,
