@@ -1210,6 +1210,7 @@ template <typename T, typename Seqs, int kParts>
 __global__ void __launch_bounds__(ScanWarps<kParts>::kThreads, 1)
 chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ ScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) let_others_begin();  // the token kernels of the short sequences
   scan_sequence<T, Seqs, false, kParts>(p, seqs, tm, *reinterpret_cast<ScanSmem*>(smem_raw), int(blockIdx.x));
 }
 

@@ -181,6 +181,33 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);  // once per (ke
 bool profiling();  // per-kernel timing is on: the kernels of a call then run one by one (api.cu)
 void profile_mark(int index, cudaStream_t stream);  // records timing event `index` when profiling is on (api.cu)
 
+// ---- kernels of one call that overlap -----------------------------------------------
+// The second one is launched `beside` the first: it may begin once all CTAs of the first have begun (let_others_begin, at
+// the start of the first) where those leave room, and has wait_for_others where it needs what the first writes, or at its
+// end where it needs nothing: what follows on the stream waits for the second alone.  Everything before the first is over
+// by then.  (Both do nothing in a launch of their own.)
+__device__ __forceinline__ void let_others_begin() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_others() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... Params, typename... Args>
+inline int launch_beside(void (*kernel)(Params...), unsigned blocks, int threads, int smem, cudaStream_t stream,
+                         bool beside, const Args&... args) {
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(blocks);
+  config.blockDim = dim3(unsigned(threads));
+  config.dynamicSmemBytes = size_t(smem);
+  config.stream = stream;
+  cudaLaunchAttribute attribute;
+  attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attribute.val.programmaticStreamSerializationAllowed = 1;
+  config.attrs = &attribute;
+  config.numAttrs = beside ? 1 : 0;
+  const cudaError_t err = cudaLaunchKernelEx(&config, kernel, args...);
+  if (err == cudaSuccess) return GDN2_OK;
+  (void)cudaGetLastError();
+  record_cuda_error(err);
+  return GDN2_ERR_LAUNCH;
+}
+
 inline bool valid_seq_dtype(int d) { return d == GDN2_BF16 || d == GDN2_FP16; }
 inline bool valid_gate_dtype(int d, int seq) { return d == seq || d == GDN2_FP32; }
 

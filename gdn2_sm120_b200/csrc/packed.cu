@@ -21,7 +21,7 @@ int launch_packed_chunk_backward(const PackedSeqs&, const void*, const void*, co
                                  uint8_t*, void*, void*, void*, void*, void*, void*, float*, int64_t, int64_t, int,
                                  int, float, cudaStream_t);
 int launch_packed_token_forward(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
-                                const void*, const float*, void*, float*, float*, int64_t, int, int, float, int,
+                                const void*, const float*, void*, float*, float*, int64_t, int, int, float, int, bool,
                                 cudaStream_t);
 int launch_packed_token_backward(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
                                  const void*, const void*, const float*, const float*, float*, void*, void*, void*,
@@ -117,8 +117,11 @@ extern "C" int gdn2_packed_forward(const void* q, const void* k, const void* v, 
   }
   if (t.spans.n > 0) {
     if (training && span_boundaries == nullptr) return GDN2_ERR_NULL_POINTER;
+    // Beside the scans, which leave the SMs to one another as they end, and some idle from the start.  (Packed inference
+    // of 16 sequences, H16, 33 and 7 tokens among them: 268 -> 236 us.)
     st = launch_packed_token_forward(t.spans, q, k, v, g, beta, w, initial_state, out, final_state,
-                                     training ? span_boundaries : nullptr, heads, dtype, g_dtype, scale, prologue, cs);
+                                     training ? span_boundaries : nullptr, heads, dtype, g_dtype, scale, prologue,
+                                     t.chunks.n > 0 && !profiling(), cs);
   }
   return st;
 }

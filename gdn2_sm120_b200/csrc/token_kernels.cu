@@ -217,6 +217,7 @@ token_step_kernel(const TokenStepParams p, const __grid_constant__ Seqs seqs) {
       stf<T>(p.out, row_of(t) + vt * kTokVT + tid, ov);
     }
   }
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) wait_for_others();
 }
 
 // ---------------------------------------------------------------------------------
@@ -463,10 +464,19 @@ inline bool grid_fits(int64_t blocks) { return blocks > 0 && blocks <= int64_t(0
 // `most`: 1 (T == 1 without checkpoints), 4 or kStepTokens, the most tokens a sequence has
 template <typename Seqs>
 int launch_steps(const TokenStepParams& p, const Seqs& seqs, int64_t blocks, int most, int dtype, int g_dtype,
-                 cudaStream_t stream) {
+                 cudaStream_t stream, bool beside = false) {
   if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
   auto run = [&](auto tok) {
     constexpr int kTok = decltype(tok)::value;
+    int st = GDN2_OK;
+    if (beside) {
+      GDN2_DISPATCH_TYPES(dtype, g_dtype, {
+        st = launch_beside(p.prologue != 0 ? token_step_kernel<T, G, Seqs, true, kTok>
+                                           : token_step_kernel<T, G, Seqs, false, kTok>,
+                           unsigned(blocks), kTokThreads, 0, stream, true, p, seqs);
+      });
+      return st;
+    }
     GDN2_DISPATCH_TYPES(dtype, g_dtype, {
       if (p.prologue != 0) token_step_kernel<T, G, Seqs, true, kTok><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
       else token_step_kernel<T, G, Seqs, false, kTok><<<unsigned(blocks), kTokThreads, 0, stream>>>(p, seqs);
@@ -523,10 +533,11 @@ int launch_token_forward(const void* q, const void* k, const void* v, const void
 // the sequences from `first` on, none of more than step_tokens(prologue) tokens
 int launch_packed_steps(const PackedSpans& table, int first, const void* q, const void* k, const void* v, const void* g,
                         const void* beta, const void* w, const float* s_in, void* out, float* s_out, float* bnd,
-                        int64_t H, int dtype, int g_dtype, float scale, int prologue, cudaStream_t stream) {
+                        int64_t H, int dtype, int g_dtype, float scale, int prologue, bool beside,
+                        cudaStream_t stream) {
   const TokenStepParams p{q, k, v, g, beta, w, s_in, out, s_out, bnd, int(H), first, scale, prologue};
   return launch_steps(p, table, (table.n - first) * H * kTokTiles, table.e[first].len <= 4 ? 4 : kStepTokens, dtype,
-                      g_dtype, stream);
+                      g_dtype, stream, beside);
 }
 
 int launch_token_t1_zero(const void* q, const void* k, const void* v, const void* w, void* out,

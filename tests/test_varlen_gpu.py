@@ -91,3 +91,44 @@ def test_cu_seqlens_and_group_validation():
     assert torch.equal(wide[:, :, 3], a[:, :, 1])
     (grad,) = torch.autograd.grad(wide.sum(), a)
     assert torch.equal(grad, torch.full_like(a, 3.0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [(200, 33, 7, 130, 3), (64, 9, 10, 1), (700, 48), (65, 2, 4)])
+def test_short_sequences_beside_the_scans(lengths):
+    """The token kernels of a packed forward run beside the chunk scans: what follows on the stream sees every output
+    and state, eagerly and in a replayed graph, bit for bit as from separate calls."""
+    heads, total = 5, sum(lengths)
+    cpu = oracle.make_inputs(1, total, heads, seed=61)
+    args = [t.cuda() for t in cpu[:6]]
+    state = (torch.randn(len(lengths), heads, 128, 128, generator=torch.Generator().manual_seed(62)) * 0.02).cuda()
+    bounds = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    wanted_out, wanted_state = [], []
+    for i, (a, b) in enumerate(zip(bounds, bounds[1:])):
+        out, fin = chunk_gdn2(*(x[:, a:b].contiguous() for x in args), state[i:i + 1], output_final_state=True)
+        wanted_out.append(out)
+        wanted_state.append(fin)
+    wanted_out, wanted_state = torch.cat(wanted_out, 1), torch.cat(wanted_state, 0)
+
+    def call():
+        out, fin = chunk_gdn2_varlen(*args, bounds, state, output_final_state=True)
+        return out.clone(), fin.clone()  # right behind on the stream
+
+    with torch.no_grad():
+        for _ in range(20):
+            out, fin = call()
+            assert torch.equal(out, wanted_out) and torch.equal(fin, wanted_state)
+        stream = torch.cuda.Stream()
+        stream.wait_stream(torch.cuda.current_stream())
+        with torch.cuda.stream(stream):
+            call()
+        torch.cuda.current_stream().wait_stream(stream)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            captured = call()
+    for _ in range(5):
+        for x in captured:
+            x.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(captured[0], wanted_out) and torch.equal(captured[1], wanted_state)
