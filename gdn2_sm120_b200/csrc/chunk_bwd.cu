@@ -491,6 +491,7 @@ __global__ void __launch_bounds__(BScanWarps<kParts>::kThreads, 1)
 chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   reverse_sequence<T, Seqs, false, kParts>(p, seqs, tm, *reinterpret_cast<BScanSmem*>(smem_raw), int(blockIdx.x));
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) wait_for_others();  // the short sequences' reverse kernel
 }
 
 
@@ -685,6 +686,7 @@ chunk_bwd_vjp_kernel(const VjpParams p, const __grid_constant__ Seqs seqs, const
                      const __grid_constant__ JointScan<kJoint> scan) {
   using O = typename std::conditional<kF32Grads, float, T>::type;  // element type of dq, dk, dv, dbeta, dw
   extern __shared__ __align__(1024) uint8_t smem[];
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) let_others_begin();  // the short sequences' VJP
   if constexpr (kJoint) {
     static_assert(BScanWarps<kJointParts>::kThreads == kVjpThreads, "a scanning CTA goes on with the VJP");
     if (int(blockIdx.x) < kJointParts * seqs.count() * p.H) {
@@ -1339,6 +1341,7 @@ struct BackwardCall {
   float scale;
   int grads_f32;
   bool ragged;      // some last chunk is partial
+  bool beside;      // the launch before this call's is of the same backward and independent of it
 };
 
 template <typename T, typename G, typename Seqs, bool kF32Grads, bool kRagged>
@@ -1354,7 +1357,7 @@ int launch_vjp(const VjpParams& p, const Seqs& seqs, const VjpMaps& m, cudaStrea
 }
 
 template <typename T, typename Seqs>
-int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, int64_t n_scan, int parts,
+int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, int64_t n_scan, int parts, bool beside,
                  cudaStream_t stream) {
   auto kernel = parts == 4 ? chunk_bwd_scan_kernel<T, Seqs, 4>
               : parts == 2 ? chunk_bwd_scan_kernel<T, Seqs, 2> : chunk_bwd_scan_kernel<T, Seqs, 1>;
@@ -1362,6 +1365,7 @@ int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, in
   const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int threads = parts > 1 ? BScanWarps<2>::kThreads : BScanWarps<1>::kThreads;
+  if (beside) return launch_beside(kernel, unsigned(n_scan * parts), threads, smem, stream, true, p, seqs, tm);
   kernel<<<unsigned(n_scan * parts), threads, smem, stream>>>(p, seqs, tm);
   return check_launch();
 }
@@ -1482,8 +1486,8 @@ int launch_backward(const Seqs& seqs, const BackwardCall& a, cudaStream_t stream
       }
     }
   }
-  st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, stream)
-                            : launch_bscan<__half>(sp, seqs, tm, n_scan, parts, stream);
+  st = a.dtype == GDN2_BF16 ? launch_bscan<__nv_bfloat16>(sp, seqs, tm, n_scan, parts, a.beside, stream)
+                            : launch_bscan<__half>(sp, seqs, tm, n_scan, parts, a.beside, stream);
   if (st != GDN2_OK) return st;
   profile_mark(4, stream);
   if constexpr (std::is_same<Seqs, UniformSeqs>::value) {
@@ -1517,7 +1521,7 @@ int launch_chunk_backward(const void* q, const void* k, const void* v, const voi
   if (B * T > int64_t(0x7fffffff) || B * n_chunks * H > int64_t(0x7fffffff)) return GDN2_ERR_TOO_LARGE;
   const UniformSeqs seqs{0, T, int(full_tokens < T ? full_tokens : T), int(n_chunks), int(B)};
   const BackwardCall a{q, k, v, g, beta, w, d_out, ds_final, bnd, d_bnd, workspace, scratch, dq, dk, dv, dg, dbeta,
-                       dw, ds_init, B * T, H, dtype, g_dtype, scale, grads_f32, full_tokens > T};
+                       dw, ds_init, B * T, H, dtype, g_dtype, scale, grads_f32, full_tokens > T, false};
   return launch_backward(seqs, a, stream);
 }
 
@@ -1526,11 +1530,11 @@ int launch_packed_chunk_backward(const PackedSeqs& table, const void* q, const v
                                  const void* beta, const void* w, const void* d_out, const float* ds_final,
                                  const float* bnd, float* d_bnd, const uint8_t* workspace, uint8_t* scratch, void* dq,
                                  void* dk, void* dv, void* dg, void* dbeta, void* dw, float* ds_init, int64_t rows,
-                                 int64_t H, int dtype, int g_dtype, float scale, cudaStream_t stream) {
+                                 int64_t H, int dtype, int g_dtype, float scale, bool beside, cudaStream_t stream) {
   bool ragged = false;
   for (int i = 0; i < table.n; ++i) ragged = ragged || table.e[i].len % kChunk != 0;
   const BackwardCall a{q, k, v, g, beta, w, d_out, ds_final, bnd, d_bnd, workspace, scratch, dq, dk, dv, dg, dbeta,
-                       dw, ds_init, rows, H, dtype, g_dtype, scale, 0, ragged};
+                       dw, ds_init, rows, H, dtype, g_dtype, scale, 0, ragged, beside};
   return launch_backward(table, a, stream);
 }
 

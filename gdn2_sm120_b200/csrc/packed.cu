@@ -19,13 +19,15 @@ int launch_packed_chunk_forward(const PackedSeqs&, const void*, const void*, con
 int launch_packed_chunk_backward(const PackedSeqs&, const void*, const void*, const void*, const void*, const void*,
                                  const void*, const void*, const float*, const float*, float*, const uint8_t*,
                                  uint8_t*, void*, void*, void*, void*, void*, void*, float*, int64_t, int64_t, int,
-                                 int, float, cudaStream_t);
+                                 int, float, bool, cudaStream_t);
 int launch_packed_token_forward(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
                                 const void*, const float*, void*, float*, float*, int64_t, int, int, float, int, bool,
                                 cudaStream_t);
-int launch_packed_token_backward(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
-                                 const void*, const void*, const float*, const float*, float*, void*, void*, void*,
-                                 void*, void*, void*, float*, int64_t, int, int, float, cudaStream_t);
+int launch_packed_token_reverse(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
+                                const float*, float*, float*, int64_t, int, int, float, cudaStream_t);
+int launch_packed_token_vjp(const PackedSpans&, const void*, const void*, const void*, const void*, const void*,
+                            const void*, const void*, const float*, const float*, void*, void*, void*, void*, void*,
+                            void*, int64_t, int, int, float, bool, cudaStream_t);
 
 namespace {
 
@@ -142,21 +144,28 @@ extern "C" int gdn2_packed_backward(const void* q, const void* k, const void* v,
     return st;
   }
   const cudaStream_t cs = static_cast<cudaStream_t>(stream);
+  if (t.chunks.n > 0 &&
+      (workspace == nullptr || scratch == nullptr || chunk_boundaries == nullptr || d_chunk_boundaries == nullptr)) {
+    return GDN2_ERR_NULL_POINTER;
+  }
+  // The reverse scans run beside the short sequences' reverse kernel, and the short sequences' VJP beside the other one.
+  const bool beside = t.chunks.n > 0 && t.spans.n > 0 && !profiling();
+  if (t.spans.n > 0) {
+    if (span_boundaries == nullptr || d_span_boundaries == nullptr) return GDN2_ERR_NULL_POINTER;
+    st = launch_packed_token_reverse(t.spans, q, k, g, beta, d_out, d_final_state, d_span_boundaries, d_initial_state,
+                                     heads, dtype, g_dtype, scale, cs);
+    if (st != GDN2_OK) return st;
+  }
   if (t.chunks.n > 0) {
-    if (workspace == nullptr || scratch == nullptr || chunk_boundaries == nullptr || d_chunk_boundaries == nullptr) {
-      return GDN2_ERR_NULL_POINTER;
-    }
     st = launch_packed_chunk_backward(t.chunks, q, k, v, g, beta, w, d_out, d_final_state, chunk_boundaries,
                                       d_chunk_boundaries, static_cast<const uint8_t*>(workspace),
                                       static_cast<uint8_t*>(scratch), dq, dk, dv, dg, dbeta, dw, d_initial_state,
-                                      total, heads, dtype, g_dtype, scale, cs);
+                                      total, heads, dtype, g_dtype, scale, beside, cs);
     if (st != GDN2_OK) return st;
   }
   if (t.spans.n > 0) {
-    if (span_boundaries == nullptr || d_span_boundaries == nullptr) return GDN2_ERR_NULL_POINTER;
-    st = launch_packed_token_backward(t.spans, q, k, v, g, beta, w, d_out, d_final_state, span_boundaries,
-                                      d_span_boundaries, dq, dk, dv, dg, dbeta, dw, d_initial_state, heads, dtype,
-                                      g_dtype, scale, cs);
+    st = launch_packed_token_vjp(t.spans, q, k, v, g, beta, w, d_out, span_boundaries, d_span_boundaries, dq, dk, dv, dg,
+                                 dbeta, dw, heads, dtype, g_dtype, scale, beside, cs);
   }
   return st;
 }

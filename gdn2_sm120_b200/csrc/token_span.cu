@@ -480,6 +480,7 @@ __global__ void __launch_bounds__(kSplit ? 2 * kThreads : kThreads)
 token_span_reverse_kernel(const SpanRevParams p, const __grid_constant__ Seqs seqs) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RevSmem<kSplit>& sm = *reinterpret_cast<RevSmem<kSplit>*>(smem_raw);
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) let_others_begin();  // the reverse scans of the longer sequences
   const int tid = threadIdx.x % kThreads, tile = int(blockIdx.x) % kTiles;
   const bool preparer = kSplit && threadIdx.x >= kThreads;
   const TileThread t(tid, tile);
@@ -933,6 +934,7 @@ token_span_vjp_kernel(const SpanVjpParams p, const __grid_constant__ Seqs seqs) 
     const int i = half + x;
     if (i < n) stf<G>(p.dg, ((row0 + i) * p.H + h) * kDim + c, sum[x] + run);
   }
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) wait_for_others();
 }
 
 inline int64_t spans_for(int64_t tokens) { return (tokens + kSpan - 1) / kSpan; }
@@ -1004,11 +1006,12 @@ int run_reverse(const Seqs& seqs, const SpanRevParams& p, int dtype, int g_dtype
   return (split ? run_reverse<true, Seqs> : run_reverse<false, Seqs>)(seqs, p, dtype, g_dtype, stream);
 }
 template <typename Seqs>
-int run_vjp(const Seqs& seqs, const SpanVjpParams& p, int dtype, int g_dtype, cudaStream_t stream) {
+int run_vjp(const Seqs& seqs, const SpanVjpParams& p, int dtype, int g_dtype, cudaStream_t stream,
+            bool beside = false) {
   const int64_t blocks = int64_t(seqs.total_chunks()) * p.H;
   int st = GDN2_OK;
   GDN2_DISPATCH_TYPES(dtype, g_dtype, {
-    st = launch(token_span_vjp_kernel<T, G, Seqs>, blocks, kVjpThreads, int(sizeof(VjpSmem)), p, seqs, stream);
+    st = launch(token_span_vjp_kernel<T, G, Seqs>, blocks, kVjpThreads, int(sizeof(VjpSmem)), p, seqs, stream, beside);
   });
   return st;
 }
@@ -1068,16 +1071,20 @@ int launch_packed_token_forward(const PackedSpans& table, const void* q, const v
                              prologue, beside, stream);
 }
 
-int launch_packed_token_backward(const PackedSpans& table, const void* q, const void* k, const void* v, const void* g,
-                                 const void* beta, const void* w, const void* d_out, const float* ds_final,
-                                 const float* bnd, float* d_bnd, void* dq, void* dk, void* dv, void* dg, void* dbeta,
-                                 void* dw, float* ds_init, int64_t H, int dtype, int g_dtype, float scale,
-                                 cudaStream_t stream) {
-  const int st = run_reverse(table, SpanRevParams{q, k, g, beta, d_out, ds_final, d_bnd, ds_init, int(H), scale},
-                             dtype, g_dtype, stream);
-  if (st != GDN2_OK || table.chunks == 0) return st;
+int launch_packed_token_reverse(const PackedSpans& table, const void* q, const void* k, const void* g, const void* beta,
+                                const void* d_out, const float* ds_final, float* d_bnd, float* ds_init, int64_t H,
+                                int dtype, int g_dtype, float scale, cudaStream_t stream) {
+  return run_reverse(table, SpanRevParams{q, k, g, beta, d_out, ds_final, d_bnd, ds_init, int(H), scale}, dtype, g_dtype,
+                     stream);
+}
+
+int launch_packed_token_vjp(const PackedSpans& table, const void* q, const void* k, const void* v, const void* g,
+                            const void* beta, const void* w, const void* d_out, const float* bnd, const float* d_bnd,
+                            void* dq, void* dk, void* dv, void* dg, void* dbeta, void* dw, int64_t H, int dtype,
+                            int g_dtype, float scale, bool beside, cudaStream_t stream) {
+  if (table.chunks == 0) return GDN2_OK;
   return run_vjp(table, SpanVjpParams{q, k, v, g, beta, w, d_out, bnd, d_bnd, dq, dk, dv, dg, dbeta, dw, int(H), scale},
-                 dtype, g_dtype, stream);
+                 dtype, g_dtype, stream, beside);
 }
 
 }  // namespace gdn2

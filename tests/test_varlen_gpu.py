@@ -132,3 +132,48 @@ def test_short_sequences_beside_the_scans(lengths):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(captured[0], wanted_out) and torch.equal(captured[1], wanted_state)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("lengths", [(200, 33, 7, 130, 3), (64, 9, 10, 1), (700, 63)])
+def test_short_sequences_beside_the_backward_of_the_others(lengths):
+    """The reverse scans run beside the short sequences' reverse kernel and their VJP beside the other one: gradients
+    read right behind on the stream, eagerly and from a replayed graph, are those of separate calls bit for bit."""
+    heads, total = 5, sum(lengths)
+    cpu = oracle.make_inputs(1, total, heads, seed=71)
+    leaves = [t.cuda().requires_grad_(True) for t in cpu[:6]]
+    gen = torch.Generator().manual_seed(72)
+    state = (torch.randn(len(lengths), heads, 128, 128, generator=gen) * 0.02).cuda().requires_grad_(True)
+    d_out = torch.randn(leaves[2].shape, generator=gen).to(leaves[2].dtype).cuda()
+    d_fin = torch.randn(state.shape, generator=gen).cuda()
+    bounds = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+    wanted = [[] for _ in range(7)]
+    for i, (a, b) in enumerate(zip(bounds, bounds[1:])):
+        parts = [x.detach()[:, a:b].contiguous().requires_grad_(True) for x in leaves]
+        start = state.detach()[i:i + 1].clone().requires_grad_(True)
+        out, fin = chunk_gdn2(*parts, start, output_final_state=True)
+        grads = torch.autograd.grad([out, fin], [*parts, start], [d_out[:, a:b].contiguous(), d_fin[i:i + 1]])
+        for w, g in zip(wanted, grads):
+            w.append(g)
+    wanted = [torch.cat(w, 1) for w in wanted[:6]] + [torch.cat(wanted[6], 0)]
+
+    def step():
+        out, fin = chunk_gdn2_varlen(*leaves, bounds, state, output_final_state=True)
+        return [g.clone() for g in torch.autograd.grad([out, fin], [*leaves, state], [d_out, d_fin])]
+
+    for _ in range(10):
+        assert all(torch.equal(g, w) for g, w in zip(step(), wanted))
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(stream):
+        step()
+    torch.cuda.current_stream().wait_stream(stream)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = step()
+    for _ in range(5):
+        for x in captured:
+            x.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert all(torch.equal(g, w) for g, w in zip(captured, wanted))
