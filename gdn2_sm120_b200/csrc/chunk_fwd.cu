@@ -193,7 +193,9 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     if constexpr (kJoint) {
       bulk_wait_all();
       fence_async_all();
-      if (lane == 0 && leaving >= 0) {
+      // (the lane that committed the copies of T^T: a wait for copies is one for the thread's own, and which lane is
+      // elected is not promised)
+      if (leader && leaving >= 0) {
         store_release(reinterpret_cast<float*>(p.ws + ws.off_d() + int64_t(leaving) * kBlobD), mark);
       }
     }

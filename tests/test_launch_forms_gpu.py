@@ -192,6 +192,46 @@ def test_joint_backward_never_reads_ahead_of_a_mark(batch, heads, time):
         assert all(torch.equal(a, b) for a, b in zip(grads, first))
 
 
+# a unit whose mark is seen before one of its tiles is in memory gives a scan what lay there before: NaN here, where the
+# scans wait for the preparing CTAs alone (8 and 16 heads) and where they prepare units themselves first
+@pytest.mark.parametrize("heads,time", [(8, 50 * 64), (16, 40 * 64 + 17), (37, 21 * 64)])
+@pytest.mark.parametrize("training,prologue", [(False, 0), (False, 3), (True, 0)])
+def test_joint_forward_never_reads_ahead_of_a_mark(heads, time, training, prologue):
+    tensors, _, _ = _device_inputs(1, time, heads, seed=time)
+    full = -(-time // 64) * 64
+    workspace = torch.empty(chunk_kernels.workspace_bytes(1, full, heads, training) // 4, device=DEV)
+    scratch = torch.empty(0 if training else chunk_kernels.scratch_bytes(1, full, heads) // 4, device=DEV)
+    slots = torch.empty((1, full // 64 + 1, heads, 128, 128), device=DEV) if training else None
+    out, fin = torch.empty_like(tensors[2]), torch.empty_like(tensors[6])
+    codes = _lib.dtype_code(tensors[0].dtype), _lib.dtype_code(tensors[3].dtype)
+
+    def call():
+        workspace.fill_(float("nan"))
+        scratch.fill_(float("nan"))
+        common = [x.data_ptr() for x in (*tensors, out, fin)]
+        buffers = [workspace.data_ptr(), scratch.data_ptr() or None]
+        sizes, last = (1, time, heads, full), (128 ** -0.5,)
+        if prologue:
+            _lib.call("gdn2_chunk_forward_fused", out.device, *common, *buffers, *sizes, *codes, *last, prologue,
+                      _lib.stream_ptr(out.device))
+        else:
+            _lib.call("gdn2_chunk_forward", out.device, *common, slots.data_ptr() if training else None, *buffers, *sizes,
+                      int(training), *codes, *last, _lib.stream_ptr(out.device))
+
+    _lib.profile_enable(True)  # times the kernels one by one: never joint
+    try:
+        call()
+        assert _lib.lib().gdn2_chunk_forward_kernels() == 2
+    finally:
+        _lib.profile_enable(False)
+    wanted = out.clone(), fin.clone()
+    assert all(torch.isfinite(x.float()).all() for x in wanted)
+    for _ in range(20):
+        call()
+        assert _lib.lib().gdn2_chunk_forward_kernels() == 1
+        assert torch.equal(out, wanted[0]) and torch.equal(fin, wanted[1])
+
+
 # 255 .. 257 and 513: around one and two launch tables of 256 sequences
 @pytest.mark.parametrize("count", [255, 256, 257, 513])
 def test_packed_batches_around_the_table_size(count):
