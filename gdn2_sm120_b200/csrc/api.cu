@@ -97,7 +97,8 @@ void profile_mark(int index, cudaStream_t stream) {
 // stream's behalf, which keeps the entry points usable under stream capture).
 namespace {
 struct SmemOptIn { const void* kernel; uint64_t devices; int bytes; };
-SmemOptIn g_smem_opt_in[128];
+constexpr int kSmemOptIns = 192;  // (142 kernels ask)
+SmemOptIn g_smem_opt_in[kSmemOptIns];
 int g_smem_opt_in_count = 0;
 std::mutex g_smem_opt_in_mutex;
 }  // namespace
@@ -115,7 +116,7 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
   if (entry != nullptr && (entry->devices & bit) != 0 && entry->bytes >= bytes) return cudaSuccess;
   err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err != cudaSuccess) return err;
-  if (entry == nullptr && g_smem_opt_in_count < 128) {
+  if (entry == nullptr && g_smem_opt_in_count < kSmemOptIns) {
     entry = &g_smem_opt_in[g_smem_opt_in_count++];
     *entry = SmemOptIn{kernel, 0, bytes};
   }

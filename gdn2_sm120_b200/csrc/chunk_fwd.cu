@@ -119,8 +119,9 @@ struct PrepMaps {
 // `first` and then whatever the queue gives; tensor memory columns tb .. tb + 255.  kPro: the instantiation
 // that can apply the layer prologue to raw inputs (p.prologue says which parts); the plain instantiation
 // carries none of that code.  kJoint: `quota` (0: all there are) units are taken in the order in which the scans
-// running beside need them (chunk by chunk through all sequences), and a finished one is marked in its D array.
-template <typename T, typename G, typename Seqs, bool kPro, bool kJoint>
+// running beside need them (chunk by chunk through all sequences), and a finished one is marked in its D array: at
+// once with kSoon, else when the next unit's inputs are in registers.
+template <typename T, typename G, typename Seqs, bool kPro, bool kJoint, bool kSoon>
 __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs, const PrepMaps& tm, PrepSmem& sm,
                                            const int tid, const uint32_t tb, const int first, const int stride,
                                            const int barrier, int* queue, int quota) {
@@ -319,7 +320,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     for (int t = 0; t < 4; ++t) Gc[r][t] = add2(Gc[r][t], base);
   }
 
-  if (warp == kCopyWarp) set_mark();
+  if (!kSoon && warp == kCopyWarp) set_mark();
 
   // ---- Gram products P_I = [E_a ; Q_a] (K^I)^T on the tensor cores, 32 channels at a time ------------------
   float* const tile_q = reinterpret_cast<float*>(p.tiles.q + int64_t(ch) * kTileQ);
@@ -641,15 +642,16 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
   }
   if constexpr (kJoint) {
     // A finished unit is marked by the sign of D[0] (a decay is never negative) once its tiles are in memory: the
-    // copying warp looks to that when it has the next unit's sums.
+    // copying warp looks to that here or when it has the next unit's sums.
     unit_next = sm.next[par];
     leaving = ch;
     mark = __uint_as_float(__float_as_uint(exp2_approx(sm.gend[0])) | 0x80000000u);
+    if (kSoon && warp == kCopyWarp) set_mark();
   }
   }  // units of this group
   if (warp == kCopyWarp) {
     bulk_wait_all();  // the last tiles are in memory before the CTA goes on
-    set_mark();
+    set_mark();       // (with kSoon once more the same)
   }
 }
 
@@ -666,7 +668,7 @@ chunk_prep_kernel(const PrepParams p, const __grid_constant__ Seqs seqs, const _
   __syncthreads();
   tc_fence_after();
   const uint32_t tb = sm.tmem_base;
-  prep_units<T, G, Seqs, kPro, false>(p, seqs, tm, sm, threadIdx.x, tb, int(blockIdx.x), int(gridDim.x), 0, nullptr, 0);
+  prep_units<T, G, Seqs, kPro, false, false>(p, seqs, tm, sm, threadIdx.x, tb, int(blockIdx.x), int(gridDim.x), 0, nullptr, 0);
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x < 32) tmem_dealloc(tb, 256);
@@ -1232,7 +1234,7 @@ constexpr int kJointThreads = 512;
 struct JointSmem {
   PrepSmem prep[2];
 };
-template <typename T, typename G, typename Seqs, bool kPro>
+template <typename T, typename G, typename Seqs, bool kPro, bool kSoon>
 __global__ void __launch_bounds__(kJointThreads, 1) __cluster_dims__(2, 1, 1)
 chunk_joint_kernel(const PrepParams pp, const ScanParams sp, const __grid_constant__ Seqs seqs,
                    const __grid_constant__ PrepMaps tm_prep, const __grid_constant__ ScanMaps tm_scan,
@@ -1254,7 +1256,7 @@ chunk_joint_kernel(const PrepParams pp, const ScanParams sp, const __grid_consta
     tc_fence_after();
     const uint32_t tb = sm.prep[0].tmem_base;
     const int group = tid >> 8;
-    prep_units<T, G, Seqs, kPro, true>(pp, seqs, tm_prep, sm.prep[group], tid & 255, tb + 256u * group,
+    prep_units<T, G, Seqs, kPro, true, kSoon>(pp, seqs, tm_prep, sm.prep[group], tid & 255, tb + 256u * group,
                                        group * (n_groups / 2) + nr, n_groups, 1 + group, sp.status + kQueueWord,
                                        scans ? quota : 0);
     tc_fence_before();
@@ -1390,12 +1392,9 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
                  const ScanMaps& tm_scan, int sm_count, cudaStream_t stream) {
   constexpr int smem = int(sizeof(JointSmem) > sizeof(ScanSmem) ? sizeof(JointSmem) : sizeof(ScanSmem));
   static_assert(smem <= 232448, "joint kernel exceeds the 227 KiB shared-memory limit");
-  auto kernel = chunk_joint_kernel<T, G, Seqs, kPro>;
-  cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
-  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   // the marks of finished units are in D, right before the status block: one fill clears both
   const WsLayout ws{pp.n_ch, pp.training != 0};
-  err = cudaMemsetAsync(pp.ws + ws.off_d(), 0, size_t(pp.n_ch) * kBlobD + kStatusBytes, stream);
+  cudaError_t err = cudaMemsetAsync(pp.ws + ws.off_d(), 0, size_t(pp.n_ch) * kBlobD + kStatusBytes, stream);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int pairs = seqs.count() * sp.H;
   // Clusters of two CTAs.  No more preparers than pairs of units, nor than keep ahead of the scans: a unit takes an
@@ -1414,6 +1413,14 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   const int64_t pace = pp.prologue != 0 && pp.training == 0 ? 16 : 20;
   const int64_t in_time = int64_t(2 * (clusters - pairs)) * seqs.n_chunks * pace / 100;
   const int quota = pp.n_ch > in_time ? int((pp.n_ch - in_time + 2 * clusters) / (4 * clusters)) : 0;
+  // Where the preparers keep ahead by themselves a unit is marked at once; where the scanning CTAs have to help, the
+  // microsecond that a release waits for the unit's stores is taken from the next unit, and the mark waits until that one
+  // has its inputs.  us, at once / later: raw H8 T3200 115/119, T5000 163/167, H16 T2048 90/94, plain H16 T2048 75/78,
+  // T32768 781/801; with a quota raw H24 T8192 332/327, H32 T4096 235/232, plain H24 T8192 278/271.  (Two kernels: with
+  // both forms in one the raw calls that have a quota take 331 and 235.)
+  auto kernel = quota == 0 ? chunk_joint_kernel<T, G, Seqs, kPro, true> : chunk_joint_kernel<T, G, Seqs, kPro, false>;
+  err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
+  if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(unsigned(2 * clusters));
   config.blockDim = dim3(kJointThreads);
