@@ -1398,10 +1398,14 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int pairs = seqs.count() * sp.H;
   // Clusters of two CTAs.  No more preparers than pairs of units, nor than keep ahead of the scans: a unit takes an
-  // SM 8.7 us (raw 11) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way.  us with 82 / 88 / 96
-  // SMs that prepare, H16: T32768 869/806/865, T16384 436/418/444, T8192 229/226/233; raw with 88 / 98 / 104: T32768
-  // 969/917/942, T8192 271/256/257.
-  const int64_t paced = (int64_t(pairs) * (pp.prologue != 0 ? 62 : 55) + 19) / 20;
+  // SM 8.7 us (raw 11) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way: three clusters a pair
+  // up to eight pairs, then less, as the scans slow down themselves; raw, two more than three a pair.  us at T32768, with
+  // one cluster less than the rule gives / the rule / one more:
+  //   H4 760/728/729   H6 743/729/739   H8 734/734/754   H10 755/734/755   H11 752/735/767   H12 770/748/762
+  //   H14 781/762/804  H15 797/780/813  H16 817/814/851  H17 847/836/869   H18 865/891/910
+  //   raw  H8 897/893/894   H10 903/895/897   H12 914/900/902   H14 914/903/907   H16 933/918/916   H18 1003/982/-
+  // (T8192 lies flatter and at the same places: H8 204/204/204, H12 212/208/209, H16 219/220/224, raw H16 255/255/255.)
+  const int64_t paced = pp.prologue != 0 ? 3 * pairs + 2 : std::min(3 * pairs, (49 * pairs + 102) / 20);
   const int64_t want = pairs + std::min((pp.n_ch + 3) / 4, paced);
   const int clusters = int(std::min(want, int64_t(sm_count / 2)));
   // Where the preparers alone would not keep up, the scanning CTAs first prepare `quota` units for each group of
