@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(BScanWarps<kParts>::kThreads, 1)
 chunk_bwd_scan_kernel(const BScanParams p, const __grid_constant__ Seqs seqs, const __grid_constant__ BScanMaps tm) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   reverse_sequence<T, Seqs, false, kParts>(p, seqs, tm, *reinterpret_cast<BScanSmem*>(smem_raw), int(blockIdx.x));
-  if constexpr (std::is_same<Seqs, PackedSeqs>::value) wait_for_others();  // the short sequences' reverse kernel
+  if constexpr (std::is_same<Seqs, PackedSeqs>::value) outlast_others();  // the short sequences' reverse kernel
 }
 
 

@@ -217,7 +217,7 @@ token_step_kernel(const TokenStepParams p, const __grid_constant__ Seqs seqs) {
       stf<T>(p.out, row_of(t) + vt * kTokVT + tid, ov);
     }
   }
-  if constexpr (std::is_same<Seqs, PackedSpans>::value) wait_for_others();
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) outlast_others();
 }
 
 // ---------------------------------------------------------------------------------

@@ -456,7 +456,7 @@ token_span_forward_kernel(const SpanFwdParams p, const __grid_constant__ Seqs se
   if (preparer) return;
   if (p.bnd != nullptr) store_tile(p.bnd + (int64_t(sq.slot0 + sq.n_chunks) * p.H + h) * kStateElems, t, S);
   if (p.s_out != nullptr) store_tile(p.s_out + state, t, S);
-  if constexpr (std::is_same<Seqs, PackedSpans>::value) wait_for_others();
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) outlast_others();
 }
 
 // ---- reverse scan of the state cotangent -------------------------------------------------------------
@@ -934,7 +934,7 @@ token_span_vjp_kernel(const SpanVjpParams p, const __grid_constant__ Seqs seqs) 
     const int i = half + x;
     if (i < n) stf<G>(p.dg, ((row0 + i) * p.H + h) * kDim + c, sum[x] + run);
   }
-  if constexpr (std::is_same<Seqs, PackedSpans>::value) wait_for_others();
+  if constexpr (std::is_same<Seqs, PackedSpans>::value) outlast_others();
 }
 
 inline int64_t spans_for(int64_t tokens) { return (tokens + kSpan - 1) / kSpan; }

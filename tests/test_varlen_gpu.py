@@ -177,3 +177,45 @@ def test_short_sequences_beside_the_backward_of_the_others(lengths):
         graph.replay()
         torch.cuda.synchronize()
         assert all(torch.equal(g, w) for g, w in zip(captured, wanted))
+
+
+# several waves of CTAs in every kernel that runs beside another one: 12 sequences of spans, 14 of a few tokens
+@pytest.mark.gpu
+@pytest.mark.parametrize("raw", [False, True])
+@pytest.mark.parametrize("dtype,g_dtype", [(torch.bfloat16, torch.float32), (torch.float16, torch.float32),
+                                           (torch.float16, torch.float16), (torch.bfloat16, torch.bfloat16)])
+def test_many_short_sequences_beside_two_long_ones(dtype, g_dtype, raw):
+    lengths, heads = [37, 5] * 6 + [300] + [3, 8, 1, 6] * 2 + [130] + [20, 63] * 3, 16
+    make = oracle.make_raw_inputs if raw else oracle.make_inputs
+    cpu = make(1, sum(lengths), heads, seed=81, dtype=dtype, g_dtype=g_dtype)
+    leaves = [x.to(DEV).requires_grad_(True) for x in cpu[:6]]
+    gen = torch.Generator().manual_seed(82)
+    state = (torch.randn(len(lengths), heads, 128, 128, generator=gen) * 0.02).to(DEV).requires_grad_(True)
+    d_out = torch.randn(leaves[2].shape, generator=gen).to(DEV, dtype)
+    d_fin = torch.randn(state.shape, generator=gen).to(DEV)
+    flags = {"use_qk_l2norm_in_kernel": raw, "use_gate_in_kernel": raw}
+    bounds = [sum(lengths[:i]) for i in range(len(lengths) + 1)]
+
+    def step(*inputs, call, d):
+        results = call(*inputs)
+        return [*results, *torch.autograd.grad(results, inputs, d)]
+
+    wanted, wanted_plain = [], []
+    for i, (a, b) in enumerate(zip(bounds, bounds[1:])):
+        parts = [x.detach()[:, a:b].contiguous().requires_grad_(True) for x in leaves]
+        parts.append(state.detach()[i:i + 1].clone().requires_grad_(True))
+        single = lambda *x: chunk_gdn2(*x[:6], x[6], output_final_state=True, **flags)  # noqa: E731
+        wanted.append(step(*parts, call=single, d=[d_out[:, a:b].contiguous(), d_fin[i:i + 1]]))
+        with torch.no_grad():
+            wanted_plain.append(single(*parts))
+    join = lambda rows, i: torch.cat([r[i] for r in rows], 0 if i in (1, 8) else 1)  # noqa: E731
+
+    packed = lambda *x: chunk_gdn2_varlen(*x[:6], bounds, x[6], output_final_state=True, **flags)  # noqa: E731
+    for _ in range(5):
+        got = [x.clone() for x in step(*leaves, state, call=packed, d=[d_out, d_fin])]  # right behind on the stream
+        for i, x in enumerate(got):
+            assert torch.equal(x, join(wanted, i)), i
+        with torch.no_grad():
+            plain = [x.clone() for x in packed(*leaves, state)]
+        for i, x in enumerate(plain):
+            assert torch.equal(x, join(wanted_plain, i)), i
