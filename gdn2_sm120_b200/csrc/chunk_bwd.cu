@@ -1365,7 +1365,7 @@ int launch_bscan(const BScanParams& p, const Seqs& seqs, const BScanMaps& tm, in
   const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
   const int threads = parts > 1 ? BScanWarps<2>::kThreads : BScanWarps<1>::kThreads;
-  if (beside) return launch_beside(kernel, unsigned(n_scan * parts), threads, smem, stream, true, p, seqs, tm);
+  if (beside) return launch_beside(kernel, unsigned(n_scan * parts), threads, smem, stream, p, seqs, tm);
   kernel<<<unsigned(n_scan * parts), threads, smem, stream>>>(p, seqs, tm);
   return check_launch();
 }

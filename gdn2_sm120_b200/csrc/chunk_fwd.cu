@@ -181,7 +181,6 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     issue_kq(at);
     issue_b(at);
   }
-  [[maybe_unused]] const bool wide_tiles = (reinterpret_cast<uintptr_t>(p.tiles.yt) & 31) == 0;  // (a tile is 32 KiB)
   const bool pro_norm = kPro && (p.prologue & kPrologueNorm) != 0;
   const bool pro_gate = kPro && (p.prologue & kPrologueGate) != 0;
   using RawG = typename Raw2<G>::type;
@@ -611,6 +610,7 @@ __device__ __forceinline__ void prep_units(const PrepParams& p, const Seqs& seqs
     for (int j = 0; j < 32; ++j) y[j] = to_tf32_operand(__uint_as_float(r[j]));
     if constexpr (kJoint) {
       float* row = reinterpret_cast<float*>(p.tiles.yt + int64_t(ch) * kTileYt) + kr * kChunk + 32 * part;
+      const bool wide_tiles = (reinterpret_cast<uintptr_t>(p.tiles.yt) & 31) == 0;  // (a tile is 32 KiB)
 #pragma unroll
       for (int j = 0; j < 32; j += 8) {
         const float4 lo = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);

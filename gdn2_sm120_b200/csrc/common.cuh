@@ -194,7 +194,7 @@ __device__ __forceinline__ void outlast_others() {
 }
 template <typename... Params, typename... Args>
 inline int launch_beside(void (*kernel)(Params...), unsigned blocks, int threads, int smem, cudaStream_t stream,
-                         bool beside, const Args&... args) {
+                         const Args&... args) {
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(blocks);
   config.blockDim = dim3(unsigned(threads));
@@ -204,7 +204,7 @@ inline int launch_beside(void (*kernel)(Params...), unsigned blocks, int threads
   attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attribute.val.programmaticStreamSerializationAllowed = 1;
   config.attrs = &attribute;
-  config.numAttrs = beside ? 1 : 0;
+  config.numAttrs = 1;
   const cudaError_t err = cudaLaunchKernelEx(&config, kernel, args...);
   if (err == cudaSuccess) return GDN2_OK;
   (void)cudaGetLastError();

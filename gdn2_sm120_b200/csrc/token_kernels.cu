@@ -473,7 +473,7 @@ int launch_steps(const TokenStepParams& p, const Seqs& seqs, int64_t blocks, int
       GDN2_DISPATCH_TYPES(dtype, g_dtype, {
         st = launch_beside(p.prologue != 0 ? token_step_kernel<T, G, Seqs, true, kTok>
                                            : token_step_kernel<T, G, Seqs, false, kTok>,
-                           unsigned(blocks), kTokThreads, 0, stream, true, p, seqs);
+                           unsigned(blocks), kTokThreads, 0, stream, p, seqs);
       });
       return st;
     }

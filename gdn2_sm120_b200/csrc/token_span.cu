@@ -957,7 +957,7 @@ int launch(Kernel kernel, int64_t blocks, int threads, int smem, const Params& p
   if (!grid_fits(blocks)) return GDN2_ERR_TOO_LARGE;
   const cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), smem);
   if (err != cudaSuccess) { record_cuda_error(err); return GDN2_ERR_LAUNCH; }
-  if (beside) return launch_beside(kernel, unsigned(blocks), threads, smem, stream, true, p, seqs);
+  if (beside) return launch_beside(kernel, unsigned(blocks), threads, smem, stream, p, seqs);
   kernel<<<unsigned(blocks), threads, smem, stream>>>(p, seqs);
   return check_launch();
 }
