@@ -1400,12 +1400,15 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   // Clusters of two CTAs.  No more preparers than pairs of units, nor than keep ahead of the scans: a unit takes an
   // SM 8.7 us (raw 11) and a chunk of a scan 1.6 us (1.8), and more of them get in the scans' way: three clusters a pair
   // up to eight pairs, then less, as the scans slow down themselves; raw, two more than three a pair.  us at T32768, with
-  // one cluster less than the rule gives / the rule / one more:
-  //   H4 760/728/729   H6 743/729/739   H8 734/734/754   H10 755/734/755   H11 752/735/767   H12 770/748/762
-  //   H14 781/762/804  H15 797/780/813  H16 817/814/851  H17 847/836/869   H18 865/891/910
-  //   raw  H8 897/893/894   H10 903/895/897   H12 914/900/902   H14 914/903/907   H16 933/918/916   H18 1003/982/-
-  // (T8192 lies flatter and at the same places: H8 204/204/204, H12 212/208/209, H16 219/220/224, raw H16 255/255/255.)
-  const int64_t paced = pp.prologue != 0 ? 3 * pairs + 2 : std::min(3 * pairs, (49 * pairs + 102) / 20);
+  // one cluster less than the rule gives / the rule / one more, and from H16 on the same on a second and a third GPU, on
+  // which the step up lies elsewhere by a cluster:
+  //   H4 761/734/736   H6 744/738/745   H8 740/742/761   H10 759/745/763   H11 757/746/777   H12 773/755/785
+  //   H14 785/769/814  H15 802/785/814  H16 816/800/816, 818/802/787, 818/849/861  H17 828/812/843, 833/814/837, 830/843/871
+  //   H18 841/824/865, 845/827/861, 843/855/886   H19 853/837/869, 855/839/873, 855/886/902   H20 861/869/910, 865/849/894
+  //   raw  H8 900/886/886   H10 904/890/892   H12 914/898/900   H14 912/904/900   H16 919/918/908   H18 941/935/933
+  // (T8192 lies flatter and at the same places: H8 206/206/206, H12 214/212/212, H16 226/224/226, raw H16 259/257/257;
+  // training within 1 %.)
+  const int64_t paced = pp.prologue != 0 ? 3 * pairs + 2 : std::min({3 * pairs, (49 * pairs + 102) / 20, 2 * pairs + 11});
   const int64_t want = pairs + std::min((pp.n_ch + 3) / 4, paced);
   const int clusters = int(std::min(want, int64_t(sm_count / 2)));
   // Where the preparers alone would not keep up, the scanning CTAs first prepare `quota` units for each group of
