@@ -2,13 +2,15 @@
 //
 //   chunk_prep_kernel   persistent, two CTAs per SM walking over the (sequence, chunk, head) units, all
 //                       chunks independent.  The raw inputs of the next unit arrive by tiled TMA
-//                       loads under the tail of the current one (a CTA that starts a unit with
-//                       per-thread loads spends a quarter of its time issuing them: the load/store
-//                       unit's queue, not HBM, is the limit).  Builds the WY factors of the chunk
-//                       and writes them as row-major tiles:
+//                       loads as their places become free, g under the inverse of the current one,
+//                       k and q after its last product, beta behind its last store (a CTA that
+//                       starts a unit with per-thread loads spends a quarter of its time issuing
+//                       them: the load/store unit's queue, not HBM, is the limit).  Builds the WY
+//                       factors of the chunk and writes them as row-major tiles:
 //                       cumulative log-decay, block-anchored Gram products on tf32 tcgen05 MMAs,
-//                       blocked inverse T of the unit lower-triangular system on CUDA cores (fp32),
-//                       Y = T E on tf32 tcgen05 MMAs.
+//                       the inverse T of the unit lower-triangular system on CUDA cores (fp32; two
+//                       32 x 32 blocks by substitution, the third by products), Y = T E on tf32
+//                       tcgen05 MMAs.
 //   chunk_scan_kernel   one CTA per (sequence, head) or half of its value rows, chunks in order.  The state
 //                       lives transposed (S^T: value rows x key columns) in TMEM as the fp32 accumulator
 //                       and is fed back as the tf32 A operand of the next MMAs without leaving TMEM:
@@ -44,7 +46,7 @@ namespace {
 // prep kernel
 // ---------------------------------------------------------------------------------------------
 // Persistent, two CTAs of 256 threads per SM.  A unit is a chain of a dozen phases of about a microsecond,
-// each waiting for the one before (loads, exponentials, tensor cores, the blocked inverse, stores): with one
+// each waiting for the one before (loads, exponentials, tensor cores, the inverse, stores): with one
 // CTA per SM the issue slots were 35 % busy and a unit took 10.5 us.  Two CTAs fill each other's waits; for
 // that a CTA has to live in 113 KB and 128 registers per thread, so the Gram operands are built and multiplied
 // 32 channels at a time, and everything else shares their place.  (In two rounds of 64 channels the inputs
@@ -1228,8 +1230,8 @@ chunk_scan_kernel(const ScanParams p, const __grid_constant__ Seqs seqs, const _
 // The two SMs of a pair share their way to L2 (with a preparer beside it a scan took 3.3 us per chunk): the CTAs
 // come in clusters of two, and those of a scanning pair take half of the value rows each.  512 threads leave a
 // preparing group the 128 registers a thread that it has in a launch of its own.  us, against one scanning CTA a
-// pair and 96 registers: B1 T8192 H16 364 -> 233, B1 T32768 H16 1521 -> 820 (raw 1112 -> 960), training B2 T4133
-// H16 329 -> 238, training B1 T2048 H32 170 -> 136.
+// pair and 96 registers, when this form was made: B1 T8192 H16 364 -> 233, B1 T32768 H16 1521 -> 820 (raw 1112 -> 960).
+// With a faster preparation and other numbers of CTAs it takes 224 and 802 (raw 921).
 constexpr int kJointThreads = 512;
 struct JointSmem {
   PrepSmem prep[2];
@@ -1364,23 +1366,28 @@ struct ForwardCall {
 
 thread_local int t_forward_kernels = 0;  // of this thread's latest chunk forward
 
-// One launch for both where it gains.  Apart they take n_ch * 7.1 us / SMs (the preparation), 1.6-2 us per chunk (the
+// One launch for both where it gains.  Apart they take n_ch * 6.7 us / SMs (the preparation), 1.6-2 us per chunk (the
 // scans) and what two launches cost; together the scans' time and some 20 us, where the SMs that do not scan, or all in
 // turn (quota), have the units ready in time.
-// At most a sixth of the SMs scanning, two launches / one, us, inference, raw, training:
-//   400 units on    H16 T1600 71/67 80/80 182/180   H16 T2048 86/78 97/92 207/204   H8 T3200 103/102 111/119 242/246
-//                   H8 T4096 126/122 137/142 298/298   H24 T1152 62/64 72/76 163/159   H24 T1408 74/70 85/79 195/189
-//   below           H16 T1024 46/51 54/61 128/133   H16 T1280 62/58 71/69 163/162   H8 T2048 66/73 74/87 166/176
-//   fewer scans     H1 T25600 535/563 551/665   H3 T12288 288/291 302/344   H4 T8192 206/216 218/243, training 511/523
-//                   H6 T8192 228/213 243/243, training 535/532
+// At most a sixth of the SMs scanning, two launches / one, us, inference, raw, forward of a training step:
+//   400 units on    H16 T1792 84/73 94/87 98/91   H16 T2048 90/79 100/95 105/97   H16 T8192 295/226 324/261 338/296
+//                   H8 T3200 109/101 117/120 131/132   H8 T4096 131/120 141/144 162/161   H8 T8192 248/210 262/249 301/290
+//                   H12 T3200 123/103 133/124 145/134   H24 T1280 76/69 86/79 84/77   H24 T2048 111/91 123/110 121/105
+//   below           H16 T1024 55/54 61/65 61/65   H16 T1280 70/60 76/73 78/73   H8 T2048 76/75 82/91 90/95   H8 T2560
+//                   94/87 102/103 113/112   H24 T832 61/54 68/65 66/60
+//   fewer scans     H1 T12288 279/292 287/349 354/413   H3 T12288 295/292 307/351 393/413   H4 T8192 211/206 225/247 272/286
+//                   H6 T8192 231/208 246/249 293/288
 //   the units are ready in time either way and a pair of CTAs scans no faster than it does alone, so 4 scans at least,
 //   and 8 with a prologue or states to write
-// With up to a quarter scanning, inference, raw, training (above that the preparation falls behind):
-//   above the line  H28 T2048 114/100 127/124 281/261   H32 T1664 99/99 113/105 259/252   H32 T2048 118/104 130/127
-//                   303/295   H37 T1408 95/87 108/103 249/248
-//   below           H28 T1024 62/56 73/66 173/169   H28 T1536 89/80 99/101 229/217   H32 T1280 84/80 93/100 217/209
-//                   H32 T1536 94/87 108/101 251/238   H37 T1024 68/70 79/84 184/180   H37 T1280 86/82 98/95 225/224
-//   (the line is that of an earlier form of the launch, which cost more; it stands on the safe side)
+// With up to a quarter scanning (above that the preparation falls behind):
+//   above the line  H25 T2560 133/108 145/134 146/122   H28 T2048 121/103 133/128 131/108   H32 T1792 115/105 127/118
+//                   125/108   H32 T8192 397/368 455/431 447/425   H37 T2048 130/126 145/151 143/132   H37 T8192 430/423
+//                   496/497 485/486
+//   below           H25 T1536 90/83 100/91 102/87   H28 T1024 70/62 78/73 78/69   H28 T1792 106/91 119/112 115/97
+//                   H32 T1280 88/85 98/103 96/87   H37 T1024 74/73 84/89 82/77   H37 T1280 94/87 102/103 102/95
+// The lines were drawn for a form of the launch that cost more.  Above them it is the better one or within 3 %, but for raw
+// calls of 35 to 37 scans and some 1100 units (145/151, 143/153).  Below them it would gain in most calls of more units
+// than the preparing kernel takes at once, two an SM: they stand on the safe side.
 bool prefer_joint(int64_t n_scan, int64_t n_ch, int64_t n_chunks, bool training, bool prologue, int sm_count) {
   if (4 * n_scan > sm_count || profiling()) return false;
   if (6 * n_scan <= sm_count) return n_ch >= 400 && n_scan >= (training || prologue ? 8 : 4);

@@ -120,7 +120,7 @@ extern "C" int gdn2_packed_forward(const void* q, const void* k, const void* v, 
   if (t.spans.n > 0) {
     if (training && span_boundaries == nullptr) return GDN2_ERR_NULL_POINTER;
     // Beside the scans, which leave the SMs to one another as they end, and some idle from the start.  (Packed inference
-    // of 16 sequences, H16, 33 and 7 tokens among them: 268 -> 236 us.)
+    // of 16 sequences, H16, 33 and 7 tokens among them: 268 -> 242 us.)
     st = launch_packed_token_forward(t.spans, q, k, v, g, beta, w, initial_state, out, final_state,
                                      training ? span_boundaries : nullptr, heads, dtype, g_dtype, scale, prologue,
                                      t.chunks.n > 0 && !profiling(), cs);
