@@ -1429,7 +1429,7 @@ int launch_joint(const PrepParams& pp, const ScanParams& sp, const Seqs& seqs, c
   const int quota = pp.n_ch > in_time ? int((pp.n_ch - in_time + 2 * clusters) / (4 * clusters)) : 0;
   // Where the preparers keep ahead by themselves, or nearly so, a unit is marked at once; elsewhere the microsecond that a
   // release waits for the unit's stores is taken from the next unit, and the mark waits until that one has its inputs.
-  // us, at once / later: raw H8 T3200 115/119, T5000 163/167, H16 T2048 90/94, plain H16 T2048 75/78, T32768 781/801.  By
+  // us, at once / later: raw H8 T3200 115/119, T5000 163/167, H16 T2048 90/94, plain H16 T2048 75/78, H15 T32768 783/806.  By
   // the units that are in time: all but 1 % raw H18 T1472 74.3/77.7; 94 % plain H22 T1344 64.7/65.9; 93 % raw H19 T1600
   // 79.6/82.3; 86 % raw H20 T1600 82.9/83.2; 83 % plain H24 T1088 61.5/60.3; 81 % raw H21 T1600 85.1/84.4; 71 % raw H23
   // T1344 82.8/80.2; with a quota raw H24 T8192 332/327, H32 T4096 235/232, plain H24 T8192 278/271.  (Two kernels: with
